@@ -479,6 +479,14 @@ int pgk_p2p_destroy(void);
 int pgk_gemm_rows_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
                       float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows,
                       int epilogue, float scale, float cap, void* stream);
+/* the same with a bound on the groups' rows together, total_rows >= group_off[groups] (-1: not known; no groups: M counts).
+ * bfloat16 weights run on tcgen05 when K is a multiple of 8, W and w_group_stride keep 16-byte boundaries and the rows are
+ * known or bounded; their work memory (a bfloat16 copy of the rows) is allocated in stream order. */
+int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
+                        float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows, int total_rows,
+                        int epilogue, float scale, float cap, void* stream);
+/* 1 in *out when a bounded wait inside those products ever ran out on this device (their outputs are then not valid) */
+int pgk_gemm_rows_wait_error(int* out);
 /* the same product for few rows (decoding): blocks of rows_per_block (<= 8) consecutive rows share the matrix
  * row_group[first row of the block] (NULL: matrix 0); the weights are streamed once per block of rows */
 int pgk_gemm_few_rows_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,

@@ -48,6 +48,7 @@ SOURCES = {
     "init.cu": [],
     "quant_nvf4.cu": ["--use_fast_math"],
     "seq_gemm.cu": [],
+    "seq_gemm_tc.cu": [],
     "seq_attention.cu": [],
     "seq_layers.cu": [],
     "seq_latent.cu": [],
@@ -61,7 +62,7 @@ SOURCES = {
 COMPONENTS = {
     "core": ["runtime.cu"],
     # token-major float32-activation models on the paged cache (llm/models/layered.py)
-    "seq": ["runtime.cu", "seq_gemm.cu", "seq_attention.cu", "seq_layers.cu", "seq_latent.cu", "seq_recurrent.cu",
+    "seq": ["runtime.cu", "seq_gemm.cu", "seq_gemm_tc.cu", "seq_attention.cu", "seq_layers.cu", "seq_latent.cu", "seq_recurrent.cu",
             "seq_gated.cu", "seq_mlstm.cu", "seq_gla.cu"],
 }
 

@@ -39,6 +39,11 @@ bool p2p_gemv_xchg(GemvXchg* x);     // p2p.cu: false until the peer buffers are
 void fp8_codes_forget(const void* base);
 void set_free_hook(void (*fn)(const void*));   // runtime.cu: called by pgk_free() with the pointer being released
 
+// Work memory of one call, in stream order: allocated before the call's first launch and given back behind its last on the same
+// stream, so that calls on other streams and threads never share it.  Capturable (the graph then owns the memory).
+int  scratch_alloc(void** ptr, size_t bytes, cudaStream_t st);
+int  scratch_free(void* ptr, cudaStream_t st);
+
 
 #define PGK_CUDA(call)                                                        \
     do {                                                                      \

@@ -52,6 +52,58 @@ int sm_count() {
     return g_sm_count;
 }
 
+// ---- stream-ordered work memory: a pool of the library's own per device.  Up to kScratchKeep bytes stay with the pool across
+// synchronisations (a fresh mapping costs tens of microseconds); pgk_malloc gives them back when the device runs out.
+static const uint64_t kScratchKeep = 256ull << 20;
+static std::mutex g_scratch_mu;
+static cudaMemPool_t g_scratch[64] = {};
+
+static cudaError_t scratch_pool(cudaMemPool_t* out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    if (!g_scratch[dev]) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // making the pool is no part of a capture
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        e = cudaMemPoolCreate(&pool, &props);
+        if (e == cudaSuccess) {
+            uint64_t keep = kScratchKeep;
+            e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (e != cudaSuccess) return e;
+        g_scratch[dev] = pool;
+    }
+    *out = g_scratch[dev];
+    return cudaSuccess;
+}
+
+int scratch_alloc(void** ptr, size_t bytes, cudaStream_t st) {
+    *ptr = nullptr;
+    cudaMemPool_t pool;
+    PGK_CUDA(scratch_pool(&pool));
+    PGK_CUDA(cudaMallocFromPoolAsync(ptr, bytes ? bytes : 1, pool, st));
+    return 0;
+}
+int scratch_free(void* ptr, cudaStream_t st) {
+    if (ptr) PGK_CUDA(cudaFreeAsync(ptr, st));
+    return 0;
+}
+static bool scratch_trim() {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    bool any = false;
+    for (cudaMemPool_t p : g_scratch)
+        if (p) any = cudaMemPoolTrimTo(p, 0) == cudaSuccess || any;
+    return any;
+}
+
 }  // namespace pgk
 
 using namespace pgk;
@@ -102,7 +154,12 @@ int pgk_mem_info(size_t* free_bytes, size_t* total_bytes) {
 int pgk_malloc(void** ptr, size_t bytes) {
     *ptr = nullptr;
     if (bytes == 0) bytes = 1;
-    PGK_CUDA(cudaMalloc(ptr, bytes));
+    cudaError_t e = cudaMalloc(ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && scratch_trim()) {       // idle work memory counts as free
+        cudaGetLastError();
+        e = cudaMalloc(ptr, bytes);
+    }
+    PGK_CUDA(e);
     return 0;
 }
 int pgk_free(void* ptr) {

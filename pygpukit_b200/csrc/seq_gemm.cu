@@ -1,9 +1,9 @@
 // seq_gemm.cu -- C[m, n] = sum_k A[row(m), k] * W[g][n, k] for the token-major ("ragged batch") models: float32
 // activations, weights [N, K] K-contiguous in bfloat16 or float32, float32 accumulation and output.
 //
-//   * many rows (prompts): 64 x 64 x 32 tiles, four warps; bfloat16 weights run on the tensor cores (mma.sync m16n8k16,
-//     the activation tile is rounded to bfloat16 while it is staged), float32 weights on FMAs with no reduced-precision
-//     mode anywhere;
+//   * many rows (prompts): bfloat16 weights run in seq_gemm_tc.cu (tcgen05) wherever its copies can fetch the operands; the
+//     64 x 64 x 32 tiles here (four warps, mma.sync m16n8k16, the activation tile rounded to bfloat16 while it is staged) serve
+//     the rest, and float32 weights on FMAs with no reduced-precision mode anywhere;
 //   * few rows (decoding): a warp per output column streams its weight row once with 128-bit loads and serves up to
 //     eight rows of A held in shared memory;
 //   * groups: `group_off` [E + 1] cuts the rows into E consecutive runs, run e uses weight matrix e (mixture of experts:
@@ -16,40 +16,12 @@
 //   * batches: grid.z can also walk `batch` independent products whose A columns, matrices and C columns are a fixed number
 //     of elements apart (one product per attention head on slices of the same rows).
 #include "common.cuh"
+#include "seq_gemm.cuh"
 #include "../../include/pgk_b200.h"
 
 using namespace pgk;
 
 namespace {
-
-struct GemmArgs {
-    const float* A;
-    const int* a_rows;
-    const void* W;
-    float* C;
-    const int* group_off;
-    const int* row_group;     // few-row form: weight matrix of every row (NULL: matrix 0)
-    long long w_stride;       // elements between the weight matrices of consecutive groups
-    int lda, ldc, M, N, K;
-    float scale, cap;
-    const float* colv;        // epilogue 4: [N] factors of the accumulated product
-    const void* aux;          // epilogue 5: table [*, aux_ld] (float32 or bfloat16), entry (aux_rows[m], aux_off + n);
-                              // epilogue 10: float32 gate rows, element (m, aux_off + C column)
-    const int* aux_rows;
-    int aux_ld, aux_off, aux_dt;
-    long long a_z, c_z;       // batches: elements between the A columns / C columns of consecutive products
-};
-
-__device__ __forceinline__ float gelu_tanh_f(float z) {
-    return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
-__device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.f + erff(z * 0.7071067811865476f)); }
-__device__ __forceinline__ float aux_at(const GemmArgs& a, int row, int col) {
-    const size_t i = (size_t)a.aux_rows[row] * a.aux_ld + a.aux_off + col;
-    return a.aux_dt == 2 ? bf16_bits_to_f32(((const uint16_t*)a.aux)[i]) : ((const float*)a.aux)[i];
-}
-
-__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
 
 template <int EPI>
 __device__ __forceinline__ void store_pair(const GemmArgs& a, int row, int col, float c0, float c1) {
@@ -420,8 +392,16 @@ __global__ void __launch_bounds__(FEW_MAX_WARPS * 32) gemm_few_rows_kernel(GemmA
     }
 }
 
+// bfloat16 weights go to the tcgen05 form (seq_gemm_tc.cu) whenever its copies can fetch the operands; `rows` bounds the rows of
+// A (-1: the groups' total is not known here).  The tiles below serve what is left: K no multiple of 8, matrices off
+// 16-byte boundaries, products of a few k steps, groups without a bound.
 template <int EPI>
-int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream_t st) {
+int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream_t st, int rows = -1) {
+    if (wdt == 2 && rows >= 0) {
+        bool served = false;
+        if (const int rc = gemm_rows_tc(a, EPI, groups, rows, max_rows, st, &served)) return rc;
+        if (served) return 0;
+    }
     dim3 grid((a.N + BN - 1) / BN, (max_rows + BM - 1) / BM, groups);
     if (wdt == 2) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI>, grid, dim3(128), 0, st, a));
     else PGK_CUDA(launch(gemm_rows_f32_kernel<EPI>, grid, dim3(128), 0, st, a));
@@ -494,6 +474,13 @@ extern "C" {
 int pgk_gemm_rows_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
                       float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows,
                       int epilogue, float scale, float cap, void* stream) {
+    return pgk_gemm_groups_f32(A, lda, a_rows, W, wdt, w_group_stride, C, ldc, M, N, K, group_off, groups, max_rows, -1, epilogue, scale,
+                               cap, stream);
+}
+
+int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
+                        float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows, int total_rows,
+                        int epilogue, float scale, float cap, void* stream) {
     PGK_REQUIRE(wdt == 0 || wdt == 2, "gemm_rows_f32 failed: weights must be float32 (0) or bfloat16 (2), got %d", wdt);
     PGK_REQUIRE(N > 0 && K > 0 && M >= 0, "gemm_rows_f32 failed: invalid shape M=%d N=%d K=%d", M, N, K);
     PGK_REQUIRE((epilogue >= 0 && epilogue <= 2) || (epilogue >= 6 && epilogue <= 9), "gemm_rows_f32 failed: unknown epilogue %d", epilogue);
@@ -507,13 +494,14 @@ int pgk_gemm_rows_f32(const float* A, int lda, const int32_t* a_rows, const void
         PGK_CUDA(launch(gemm_skinny_f32_kernel, dim3((M + SK_WARPS * SKM - 1) / (SK_WARPS * SKM)), dim3(SK_WARPS * 32), 0, st, a));
         return 0;
     }
-    if (epilogue == 0) return launch_many<0>(a, wdt, G, rows, st);
-    if (epilogue == 1) return launch_many<1>(a, wdt, G, rows, st);
-    if (epilogue == 6) return launch_many<6>(a, wdt, G, rows, st);
-    if (epilogue == 7) return launch_many<7>(a, wdt, G, rows, st);
-    if (epilogue == 8) return launch_many<8>(a, wdt, G, rows, st);
-    if (epilogue == 9) return launch_many<9>(a, wdt, G, rows, st);
-    return launch_many<2>(a, wdt, G, rows, st);
+    const int bound = group_off ? total_rows : M;
+    if (epilogue == 0) return launch_many<0>(a, wdt, G, rows, st, bound);
+    if (epilogue == 1) return launch_many<1>(a, wdt, G, rows, st, bound);
+    if (epilogue == 6) return launch_many<6>(a, wdt, G, rows, st, bound);
+    if (epilogue == 7) return launch_many<7>(a, wdt, G, rows, st, bound);
+    if (epilogue == 8) return launch_many<8>(a, wdt, G, rows, st, bound);
+    if (epilogue == 9) return launch_many<9>(a, wdt, G, rows, st, bound);
+    return launch_many<2>(a, wdt, G, rows, st, bound);
 }
 
 /* Few rows (decoding): every block of `rows_per_block` (<= 8) consecutive rows shares one weight matrix; row_group
@@ -575,17 +563,17 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
         }
     }
     switch (epilogue) {
-        case 0: return launch_many<0>(a, wdt, batch, M, st);
-        case 1: return launch_many<1>(a, wdt, batch, M, st);
-        case 2: return launch_many<2>(a, wdt, batch, M, st);
-        case 3: return launch_many<3>(a, wdt, batch, M, st);
-        case 4: return launch_many<4>(a, wdt, batch, M, st);
-        case 5: return launch_many<5>(a, wdt, batch, M, st);
-        case 6: return launch_many<6>(a, wdt, batch, M, st);
-        case 7: return launch_many<7>(a, wdt, batch, M, st);
-        case 8: return launch_many<8>(a, wdt, batch, M, st);
-        case 9: return launch_many<9>(a, wdt, batch, M, st);
-        default: return launch_many<10>(a, wdt, batch, M, st);
+        case 0: return launch_many<0>(a, wdt, batch, M, st, M);
+        case 1: return launch_many<1>(a, wdt, batch, M, st, M);
+        case 2: return launch_many<2>(a, wdt, batch, M, st, M);
+        case 3: return launch_many<3>(a, wdt, batch, M, st, M);
+        case 4: return launch_many<4>(a, wdt, batch, M, st, M);
+        case 5: return launch_many<5>(a, wdt, batch, M, st, M);
+        case 6: return launch_many<6>(a, wdt, batch, M, st, M);
+        case 7: return launch_many<7>(a, wdt, batch, M, st, M);
+        case 8: return launch_many<8>(a, wdt, batch, M, st, M);
+        case 9: return launch_many<9>(a, wdt, batch, M, st, M);
+        default: return launch_many<10>(a, wdt, batch, M, st, M);
     }
 }
 

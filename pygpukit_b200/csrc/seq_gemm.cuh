@@ -1,0 +1,42 @@
+// seq_gemm.cuh -- what the products of the token-major models share: their argument block, the activations of the epilogues,
+// and the entry of the tcgen05 form (seq_gemm_tc.cu).
+#pragma once
+#include "common.cuh"
+
+namespace pgk {
+
+struct GemmArgs {
+    const float* A;
+    const int* a_rows;
+    const void* W;
+    float* C;
+    const int* group_off;
+    const int* row_group;     // few-row form: weight matrix of every row (NULL: matrix 0)
+    long long w_stride;       // elements between the weight matrices of consecutive groups
+    int lda, ldc, M, N, K;
+    float scale, cap;
+    const float* colv;        // epilogue 4: [N] factors of the accumulated product
+    const void* aux;          // epilogue 5: table [*, aux_ld] (float32 or bfloat16), entry (aux_rows[m], aux_off + n);
+                              // epilogue 10: float32 gate rows, element (m, aux_off + C column)
+    const int* aux_rows;
+    int aux_ld, aux_off, aux_dt;
+    long long a_z, c_z;       // batches: elements between the A columns / C columns of consecutive products
+};
+
+__device__ __forceinline__ float gelu_tanh_f(float z) {
+    return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
+}
+__device__ __forceinline__ float gelu_erf_f(float z) { return 0.5f * z * (1.f + erff(z * 0.7071067811865476f)); }
+__device__ __forceinline__ float aux_at(const GemmArgs& a, int row, int col) {
+    const size_t i = (size_t)a.aux_rows[row] * a.aux_ld + a.aux_off + col;
+    return a.aux_dt == 2 ? bf16_bits_to_f32(((const uint16_t*)a.aux)[i]) : ((const float*)a.aux)[i];
+}
+
+__device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); }
+
+// The tcgen05 form of the many-row product (bfloat16 weights).  `batch`: independent products a.a_z / a.w_stride / a.c_z apart
+// (a.group_off NULL), or the number of row groups; `rows`: rows of A (groups: an upper bound of group_off[groups]), `max_rows`:
+// bound of the longest group.  *served is false, and nothing is launched, when the operands do not fit its copies.
+int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_rows, cudaStream_t st, bool* served);
+
+}  // namespace pgk

@@ -1,0 +1,460 @@
+// seq_gemm_tc.cu -- the many-row products of the token-major models on tcgen05: C[m, n] = sum_k bf16(A[row(m), k]) W[g][n, k]
+// with float32 activations, bfloat16 weights, float32 accumulators in TMEM and every epilogue of seq_gemm.cu.
+//
+// What bounds it: at prompt sizes the tensor pipe and, just behind it, the operand stream from L2; at a few dozen rows the
+// weights' way from HBM.  What follows from that:
+//   * the activations are rounded to bfloat16 ONCE (rows_to_bf16_kernel, 6 bytes per element, L2-resident for the product)
+//     instead of in every tile: the float32 tile would be twice the operand bytes of the bfloat16 one, per tile that reads it;
+//   * the tile is computed transposed, 128 weight rows (TMEM lanes) x up to 256 activation rows (accumulator columns), so
+//     that a warp's lanes hold neighbouring output columns of one row -- stores are whole 128-byte lines without a pass
+//     through shared memory -- and so that the tile's height follows the rows there are (16 ... 256): experts with 13 rows and
+//     prompts with 2000 run the same code;
+//   * TMA brings both operands (128-byte swizzle) into a ring of stages, one thread issues the MMAs, two accumulators in TMEM
+//     let eight epilogue warps drain a tile while the next one is multiplied, and one block per SM walks the tiles;
+//   * few tiles: a cluster of 2 ... 8 blocks shares a tile, each with a part of k, and the partial sums meet in shared memory
+//     (distributed loads, added in the order of the ranks), so that all SMs pull on the weights.
+// Measured on B200, 2000 x 9216 x 2048: 573 us on the 64 x 64 tiles of seq_gemm.cu (132 TFLOP/s), 6 + 76 us here (0.99 PFLOP/s in
+// the product); 8000 gathered rows over 16 experts, 4096 x 2048 and 2048 x 2048: 1510 -> 262 us for both.
+#include "seq_gemm.cuh"
+#include "tc_common.cuh"
+#include "tma.cuh"
+#include "../../include/pgk_b200.h"
+
+namespace pgk {
+
+namespace {
+
+constexpr int TBK = 64;                    // k per stage: one 128-byte swizzle row of bfloat16
+constexpr int TC_THREADS = 320;            // TMA warp, MMA warp, eight epilogue warps
+constexpr int TC_ROWS_MAX = 256;           // activation rows per tile = accumulator columns
+constexpr int TC_MAX_GROUPS = 512;
+constexpr uint32_t TC_W_BYTES = kTcRows * TBK * 2;
+constexpr uint32_t TC_RING_BYTES = 200 * 1024;
+constexpr int TC_MAX_STAGES = 10;
+
+struct TcArgs {
+    GemmArgs g;
+    int epi;
+    int bn;              // rows of a tile at most (multiple of 16)
+    int abox;            // rows per activation copy
+    int mt, nt, nkb;     // row tiles (no groups), column tiles, k blocks
+    int batch;           // products, or row groups
+    int stages;
+    uint32_t stage_bytes;
+    int splits;          // blocks per tile (cluster size)
+};
+
+__device__ int g_tc_wait_error = 0;        // a bounded wait ran out (never, unless a copy or a product is lost)
+
+// ---------------------------------------------------------------- activations -> bfloat16 rows [r][batch][K]
+// Memory: reads 4 and writes 2 bytes per element; 16-byte accesses both ways.  2000 x 2048: 4.0 us warm, 6.0 us from HBM.
+__global__ void __launch_bounds__(256) rows_to_bf16_kernel(GemmArgs a, uint16_t* out, int batch, int kpr, bool vec) {
+    griddep_wait();
+    griddep_launch();
+    const int r = blockIdx.x;
+    if (a.group_off && r >= a.group_off[batch]) return;
+    const float* src = a.A + (size_t)(a.a_rows ? a.a_rows[r] : r) * a.lda;
+    const int nb = a.group_off ? 1 : batch, chunks = nb * kpr;                 // chunks of eight elements
+    for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < chunks; c += gridDim.y * blockDim.x) {
+        const int b = nb == 1 ? 0 : c / kpr, k = (c - b * kpr) * 8;
+        const float* p = src + (size_t)b * a.a_z + k;
+        float v[8];
+        if (vec) {
+            *(float4*)&v[0] = *(const float4*)p;
+            *(float4*)&v[4] = *(const float4*)(p + 4);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[j] = p[j];
+        }
+        uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+        *(uint4*)(out + ((size_t)r * nb + b) * a.K + k) = o;
+    }
+}
+
+// ---------------------------------------------------------------- small pieces
+__device__ __forceinline__ void cluster_arrive_wait() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ float ld_cluster(uint32_t local_addr, uint32_t rank) {
+    uint32_t ra;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(ra) : "memory");
+    return v;
+}
+
+struct Tile { int z, n0, m0, rows; };
+
+// tile t of the launch: row tiles fastest, so that the blocks running at one time read few weight tiles
+__device__ __forceinline__ Tile tile_at(const TcArgs& p, const int* pre, int t) {
+    Tile w;
+    if (!p.g.group_off) {
+        const int mi = t % p.mt, r = t / p.mt;
+        w.z = r / p.nt;
+        w.n0 = (r - w.z * p.nt) * kTcRows;
+        w.m0 = mi * p.bn;
+        w.rows = min(p.bn, p.g.M - w.m0);
+        return w;
+    }
+    int lo = 0, hi = p.batch;                    // pre[lo] <= t < pre[hi]
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pre[mid] <= t) lo = mid; else hi = mid;
+    }
+    const int begin = p.g.group_off[lo], R = p.g.group_off[lo + 1] - begin;
+    const int mte = (R + p.bn - 1) / p.bn, h = ((R + mte - 1) / mte + 15) & ~15, loc = t - pre[lo], mi = loc % mte;
+    w.z = lo;
+    w.n0 = loc / mte * kTcRows;
+    w.m0 = begin + mi * h;
+    w.rows = min(h, R - mi * h);
+    return w;
+}
+
+// ---------------------------------------------------------------- epilogue: 16 rows of one output column per lane
+template <typename F>
+__device__ __forceinline__ void store16(const GemmArgs& a, const float (&v)[16], int row, int left, int col, F f) {
+    if (col >= a.N) return;
+    float* p = a.C + (size_t)row * a.ldc + col;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+        if (j < left) p[(size_t)j * a.ldc] = f(v[j], j);
+}
+// pairs (2j, 2j + 1) of columns sit in neighbouring lanes: the even lane finishes the even rows, the odd lane the odd ones
+template <typename F>
+__device__ __forceinline__ void store16_pairs(const GemmArgs& a, const float (&v)[16], int row, int left, int col, int lane, F f) {
+    const bool odd = lane & 1;
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+        const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+        const float first = odd ? got : v[j], second = odd ? v[j + 1] : got;
+        const int jj = odd ? j + 1 : j;
+        if ((col | 1) < a.N && jj < left) a.C[(size_t)(row + jj) * a.ldc + (col >> 1)] = f(first, second);
+    }
+}
+
+__device__ __forceinline__ void epilogue16(const GemmArgs& a, int epi, const float (&v)[16], int row, int left, int col, int lane) {
+    switch (epi) {
+        case 1: store16_pairs(a, v, row, left, col, lane, [](float g, float u) { return silu_f(g) * u; }); return;
+        case 7: store16_pairs(a, v, row, left, col, lane, [](float g, float u) { return gelu_tanh_f(g) * u; }); return;
+        case 3:          // scale = alpha, cap = limit
+            store16_pairs(a, v, row, left, col, lane, [&](float c0, float c1) {
+                const float g = fminf(c0, a.cap), u = fminf(fmaxf(c1, -a.cap), a.cap);
+                return g / (1.f + expf(-a.scale * g)) * (u + 1.f);
+            });
+            return;
+        case 2:
+            store16(a, v, row, left, col, [&](float c, int) {
+                c *= a.scale;
+                return a.cap > 0.f ? a.cap * tanhf(c / a.cap) : c;
+            });
+            return;
+        case 4: {
+            if (col >= a.N) return;
+            const float s = a.colv[col];
+            float old[16];
+            const float* p = a.C + (size_t)row * a.ldc + col;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) old[j] = j < left ? p[(size_t)j * a.ldc] : 0.f;
+            store16(a, v, row, left, col, [&](float c, int j) { return fmaf(s, c, old[j]); });
+            return;
+        }
+        case 5:
+            store16(a, v, row, left, col, [&](float c, int j) { return gelu_tanh_f(c) * aux_at(a, row + j, col); });
+            return;
+        case 6:
+            store16(a, v, row, left, col, [](float c, int) { c = fmaxf(c, 0.f); return c * c; });
+            return;
+        case 8: store16(a, v, row, left, col, [](float c, int) { return gelu_erf_f(c); }); return;
+        case 9: store16(a, v, row, left, col, [](float c, int) { return gelu_tanh_f(c); }); return;
+        case 10:         // the gate's columns are as far apart as the output's: `aux` moves with C from batch to batch
+            store16(a, v, row, left, col, [&](float c, int j) {
+                return c * (1.f / (1.f + expf(-((const float*)a.aux)[(size_t)(row + j) * a.aux_ld + a.aux_off + col])));
+            });
+            return;
+        default: store16(a, v, row, left, col, [](float c, int) { return c; });
+    }
+}
+
+// ---------------------------------------------------------------- the product
+__global__ void __launch_bounds__(TC_THREADS, 1)
+gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap amap, const __grid_constant__ TcArgs p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t full_bar[TC_MAX_STAGES], empty_bar[TC_MAX_STAGES], done_bar[2], drained_bar[2];
+    __shared__ uint32_t tmem_base_s;
+    __shared__ int pre[TC_MAX_GROUPS + 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u;
+
+    if (warp == 1) tmem_alloc(&tmem_base_s, 512);
+    if (tid == 0) {
+        for (int s = 0; s < p.stages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&done_bar[b], 1); mbar_init(&drained_bar[b], 8); }
+        mbar_fence_init();
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&amap) : "memory");
+    }
+    griddep_wait();
+    if (p.g.group_off && warp == 2) {            // tiles before every group
+        int run = 0;
+        for (int e0 = 0; e0 < p.batch; e0 += 32) {
+            const int e = e0 + lane;
+            int n = 0;
+            if (e < p.batch) n = (p.g.group_off[e + 1] - p.g.group_off[e] + p.bn - 1) / p.bn * p.nt;
+            int inc = n;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += up;
+            }
+            if (e < p.batch) pre[e] = run + inc - n;
+            run += __shfl_sync(0xffffffffu, inc, 31);
+        }
+        if (lane == 0) pre[p.batch] = run;
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_s;
+    const int total = p.g.group_off ? pre[p.batch] : p.batch * p.mt * p.nt;
+    const int rank = p.splits > 1 ? (int)cluster_rank() : 0;
+    const int first = (int)blockIdx.x / p.splits, step = (int)gridDim.x / p.splits;
+    const int per = (p.nkb + p.splits - 1) / p.splits, kb0 = rank * per, kb1 = min(p.nkb, kb0 + per);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int i = 0;                            // stages filled so far
+            bool ok = true;
+            for (int t = first; ok && t < total; t += step) {
+                const Tile w = tile_at(p, pre, t);
+                const int boxes = (w.rows + p.abox - 1) / p.abox, az = p.g.group_off ? 0 : w.z;
+                const uint32_t bytes = TC_W_BYTES + (uint32_t)(boxes * p.abox) * (TBK * 2);
+                for (int kb = kb0; kb < kb1; ++kb, ++i) {
+                    const int s = i % p.stages;
+                    const uint32_t fb = smem_u32(&full_bar[s]), dst = ring + (uint32_t)s * p.stage_bytes;
+                    if (!bar_wait(&g_tc_wait_error, smem_u32(&empty_bar[s]), (uint32_t)(((i / p.stages) & 1) ^ 1))) { ok = false; break; }
+                    mbar_expect_tx(fb, bytes);
+                    tma_load_3d(dst, &wmap, kb * TBK, w.n0, w.z, fb);
+                    for (int b = 0; b < boxes; ++b)
+                        tma_load_3d(dst + TC_W_BYTES + (uint32_t)(b * p.abox) * (TBK * 2), &amap, kb * TBK, az, w.m0 + b * p.abox, fb);
+                }
+            }
+            if (!ok)                              // do not leave with copies in flight
+                for (int j = max(0, i - p.stages); j < i; ++j) bar_wait(&g_tc_wait_error, smem_u32(&full_bar[j % p.stages]), (uint32_t)((j / p.stages) & 1));
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            int i = 0, u = 0;
+            bool ok = true;
+            for (int t = first; ok && t < total; t += step, ++u) {
+                const Tile w = tile_at(p, pre, t);
+                const uint32_t idesc = umma_idesc_bf16((w.rows + 15) & ~15), acc = tmem + (uint32_t)(u & 1) * TC_ROWS_MAX;
+                if (!bar_wait(&g_tc_wait_error, smem_u32(&drained_bar[u & 1]), (uint32_t)(((u >> 1) & 1) ^ 1))) break;
+                tc_fence_after();
+                for (int kb = kb0; kb < kb1; ++kb, ++i) {
+                    const int s = i % p.stages;
+                    if (!bar_wait(&g_tc_wait_error, smem_u32(&full_bar[s]), (uint32_t)((i / p.stages) & 1))) { ok = false; break; }
+                    tc_fence_after();
+                    const uint32_t addr = ring + (uint32_t)s * p.stage_bytes;
+                    const uint64_t dw = desc_sw128(addr), da = desc_sw128(addr + TC_W_BYTES);
+#pragma unroll
+                    for (int ks = 0; ks < TBK / 16; ++ks)         // 32 bytes of k per MMA: +2 in the descriptor's 16-byte units
+                        umma_bf16(acc, dw + (uint64_t)(ks * 2), da + (uint64_t)(ks * 2), idesc, (kb > kb0 || ks > 0) ? 1u : 0u);
+                    umma_commit(&empty_bar[s]);
+                }
+                if (ok) umma_commit(&done_bar[u & 1]);
+            }
+        }
+        __syncwarp();
+    } else {
+        const int ew = warp - 2, quad = warp & 3, half = ew >> 2;
+        int u = 0;
+        for (int t = first; t < total; t += step, ++u) {
+            const Tile w = tile_at(p, pre, t);
+            if (!bar_wait(&g_tc_wait_error, smem_u32(&done_bar[u & 1]), (uint32_t)((u >> 1) & 1))) break;
+            tc_fence_after();
+            const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(u & 1) * TC_ROWS_MAX;
+            const int col = w.n0 + quad * 32 + lane;
+            if (p.splits == 1) {
+                GemmArgs a = p.g;
+                if (!a.group_off) {
+                    a.C += (size_t)w.z * a.c_z;
+                    if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)w.z * a.c_z;
+                }
+                for (int c = half * 16; c < w.rows; c += 32) {
+                    float v[16];
+                    tmem_ld16(acc + c, v);
+                    epilogue16(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
+                    __syncwarp();
+                }
+            } else {                              // this block's share of k: row c of the partial tile, 128 columns
+                for (int c = half * 16; c < w.rows; c += 32) {
+                    float v[16];
+                    tmem_ld16(acc + c, v);
+#pragma unroll
+                    for (int j = 0; j < 16; ++j)
+                        asm volatile("st.shared.f32 [%0], %1;" :: "r"(ring + (uint32_t)((c + j) * kTcRows + quad * 32 + lane) * 4u), "f"(v[j]) : "memory");
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&drained_bar[u & 1]);
+        }
+    }
+    if (p.splits > 1) {
+        __syncthreads();
+        cluster_arrive_wait();
+        if (warp >= 2 && first < total) {         // one tile per cluster: block `rank` finishes every splits-th group of 16 rows
+            const Tile w = tile_at(p, pre, first);
+            const int ew = warp - 2, quad = warp & 3, half = ew >> 2, col = w.n0 + quad * 32 + lane;
+            GemmArgs a = p.g;
+            if (!a.group_off) {
+                a.C += (size_t)w.z * a.c_z;
+                if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)w.z * a.c_z;
+            }
+            const int parts = (p.nkb + per - 1) / per;            // blocks that had any k
+            for (int c = (rank * 2 + half) * 16; c < w.rows; c += p.splits * 32) {
+                float v[16];
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                for (int s = 0; s < parts; ++s)
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) v[j] += ld_cluster(ring + (uint32_t)((c + j) * kTcRows + quad * 32 + lane) * 4u, (uint32_t)s);
+                epilogue16(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
+            }
+        }
+        cluster_arrive_wait();                    // the others may still read this block's partial sums
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------- how a product is cut
+// Costs in cycles per SM, of one k block of a tile: the MMAs take 2 per row, the operands 16 KB + 128 bytes per row at the rate
+// an SM draws from L2.  Among the tile heights and cluster sizes the cheapest wins: whole waves of 148 blocks against tiles
+// so low that the weights are read too often, and k cut over a cluster only where the tiles alone would leave SMs idle.
+constexpr double TC_L2_BYTES_PER_CLK = 48.0;
+
+struct Plan { int bn, mt, splits; };
+
+Plan tc_plan(int M, long long ntz, int nkb) {
+    Plan best{16, 1, 1};
+    double best_cost = 1e30;
+    const int sms = sm_count();
+    for (int want = 16; want <= TC_ROWS_MAX; want += 16) {
+        const int mt = (M + want - 1) / want, bn = ((M + mt - 1) / mt + 15) & ~15;
+        const double block = fmax(2.0 * bn, (TC_W_BYTES + 128.0 * bn) / TC_L2_BYTES_PER_CLK);
+        for (int s = 1; s <= 8; s *= 2) {
+            if (s > 1 && (nkb < 4 * s || (long long)mt * ntz * s > 2LL * sms)) break;
+            const long long blocks = (long long)mt * ntz * s;
+            const double waves = (double)((blocks + sms - 1) / sms), k = (double)((nkb + s - 1) / s);
+            const double cost = s == 1 ? waves * fmax(k * block, 12.0 * bn) + 12.0 * bn + 3000.0
+                                       : waves * (k * block + 3000.0 + 20.0 * bn + 3000.0);
+            if (cost < best_cost) { best_cost = cost; best = {bn, mt, s}; }
+        }
+    }
+    return best;
+}
+
+}  // namespace
+
+int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_rows, cudaStream_t st, bool* served) {
+    *served = false;
+    // what the copies can fetch: k rows of a multiple of 16 bytes, matrices on 16-byte boundaries
+    if (a.K % 8 || a.K < TBK || (uintptr_t)a.W % 16 || (batch > 1 && (a.w_stride % 8 || a.w_stride <= 0)) || !tma_encode_fn()) return 0;
+    if (a.group_off && batch > TC_MAX_GROUPS) return 0;
+    if (rows <= 0) return 0;
+    const bool grouped = a.group_off != nullptr;
+    TcArgs p{};
+    p.g = a;
+    p.epi = epilogue;
+    p.batch = batch;
+    p.nt = (a.N + kTcRows - 1) / kTcRows;
+    p.nkb = (a.K + TBK - 1) / TBK;
+    if (grouped) {
+        // rows per group are known on the device only; aim at the mean
+        const int mean = (rows + batch - 1) / batch, most = max_rows < rows ? max_rows : rows;
+        const int cap = 2 * mean < most ? 2 * mean : most;
+        p.bn = cap >= 192 ? 256 : (cap >= 96 ? 128 : (cap >= 48 ? 64 : 32));
+        p.abox = p.bn >= 64 ? 64 : 32;
+        p.mt = 0;
+        p.splits = 1;
+    } else {
+        const Plan plan = tc_plan(a.M, (long long)p.nt * batch, p.nkb);
+        p.bn = plan.bn; p.mt = plan.mt; p.splits = plan.splits;
+        p.abox = p.bn;
+    }
+    const int held = (p.bn + p.abox - 1) / p.abox * p.abox;
+    p.stage_bytes = (TC_W_BYTES + (uint32_t)held * (TBK * 2) + 1023u) & ~1023u;
+    p.stages = (int)(TC_RING_BYTES / p.stage_bytes);
+    if (p.stages > TC_MAX_STAGES) p.stages = TC_MAX_STAGES;
+
+    const int nb = grouped ? 1 : batch;
+    void* abuf = nullptr;
+    const size_t bytes = (size_t)rows * nb * a.K * 2;
+    if (scratch_alloc(&abuf, bytes, st)) {        // no room for the copy: the tiles of seq_gemm.cu need none
+        set_error("");
+        return 0;
+    }
+    CUtensorMap wmap, amap;
+    const uint64_t wd[3] = {(uint64_t)a.K, (uint64_t)a.N, (uint64_t)batch};
+    const uint64_t ws[2] = {(uint64_t)a.K * 2, (uint64_t)(batch > 1 ? a.w_stride : (long long)a.N * a.K) * 2};
+    const uint32_t wb[3] = {TBK, kTcRows, 1};
+    const uint64_t ad[3] = {(uint64_t)a.K, (uint64_t)nb, (uint64_t)rows};
+    const uint64_t as[2] = {(uint64_t)a.K * 2, (uint64_t)nb * a.K * 2};
+    const uint32_t ab[3] = {TBK, 1, (uint32_t)p.abox};
+    if (!tma_map_bf16_3d(&wmap, a.W, wd, ws, wb) || !tma_map_bf16_3d(&amap, abuf, ad, as, ab)) {
+        scratch_free(abuf, st);
+        set_error("gemm_rows failed: the copies of a %d x %d x %d product cannot be described", rows, a.N, a.K);
+        return 1;
+    }
+    static bool configured = false;
+    if (!configured) {
+        PGK_CUDA(cudaFuncSetAttribute(gemm_rows_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_RING_BYTES + 1024));
+        configured = true;
+    }
+    const int kpr = a.K / 8, chunks = nb * kpr;
+    const bool vec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
+    int gy = (chunks + 255) / 256;
+    if (gy > 8) gy = 8;
+    cudaError_t e = launch(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, a, (uint16_t*)abuf, batch, kpr, vec);
+    if (e == cudaSuccess) {
+        const int sms = sm_count();
+        const long long tiles = (long long)batch * p.mt * p.nt;
+        const int grid = grouped ? sms : (p.splits > 1 ? (int)(tiles * p.splits) : (int)(tiles < sms ? tiles : sms));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TC_RING_BYTES + 1024; cfg.stream = st;
+        cudaLaunchAttribute at[2];
+        int n = 0;
+        at[n].id = cudaLaunchAttributeClusterDimension;
+        at[n].val.clusterDim.x = p.splits; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+        ++n;
+        if (pdl_enabled()) {
+            at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+            at[n].val.programmaticStreamSerializationAllowed = 1;
+            ++n;
+        }
+        cfg.attrs = at; cfg.numAttrs = n;
+        count_launch();
+        e = cudaLaunchKernelEx(&cfg, gemm_rows_tc_kernel, wmap, amap, p);
+    }
+    const int rc = scratch_free(abuf, st);
+    if (e != cudaSuccess) return cuda_fail(e, "gemm_rows_tc", __FILE__, __LINE__);
+    *served = rc == 0;
+    return rc;
+}
+
+}  // namespace pgk
+
+extern "C" int pgk_gemm_rows_wait_error(int* out) {
+    int v = 0;
+    PGK_CUDA(cudaMemcpyFromSymbol(&v, pgk::g_tc_wait_error, sizeof(int)));
+    *out = v;
+    return 0;
+}

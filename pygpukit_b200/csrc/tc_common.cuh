@@ -48,5 +48,39 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
 }
 
+// Bounded wait: false, and *error set, when the phase never completes (a lost copy or product) -- the caller then leaves its loop.
+__device__ __forceinline__ bool bar_wait(int* error, uint32_t bar, uint32_t parity) {
+    for (int spin = 0; spin < (1 << 22); ++spin) {
+        uint32_t ok;
+        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                     : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+        if (ok) return true;
+    }
+    atomicExch(error, 1);
+    return false;
+}
+// K-major rows of 128 bytes with the 128-byte swizzle, 8-row groups 1024 bytes apart
+__device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+// MN-major operands: every k is a row of 128 bytes = 64 elements (64 bytes = 32 elements), 8-row groups 1024 (512) bytes apart,
+// the next 64 (32) elements `group` bytes on
+__device__ __forceinline__ uint64_t desc_mn_sw128(uint32_t smem_addr, uint32_t group) {
+    return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(group >> 4) << 16) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ uint64_t desc_mn_sw64(uint32_t smem_addr, uint32_t group) {
+    return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(group >> 4) << 16) | ((uint64_t)(512u >> 4) << 32) | (1ull << 46) | (4ull << 61);
+}
+__host__ __device__ constexpr uint32_t umma_idesc_bf16_mn(int n) {        // both operands MN-major
+    return umma_idesc_bf16(n) | (1u << 15) | (1u << 16);
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float (&v)[16]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+                 :: "r"(taddr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])),
+                    "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])), "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7])),
+                    "r"(__float_as_uint(v[8])), "r"(__float_as_uint(v[9])), "r"(__float_as_uint(v[10])), "r"(__float_as_uint(v[11])),
+                    "r"(__float_as_uint(v[12])), "r"(__float_as_uint(v[13])), "r"(__float_as_uint(v[14])), "r"(__float_as_uint(v[15])) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
 
 }  // namespace pgk

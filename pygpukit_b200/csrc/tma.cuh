@@ -1,0 +1,43 @@
+// tma.cuh -- tensor-map copies (cp.async.bulk.tensor) for the kernels of the token-major models: host-side description of
+// bfloat16 operands and the device-side load.
+#pragma once
+#include "common.cuh"
+
+#include <cuda.h>
+
+namespace pgk {
+
+typedef CUresult (*TmaEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+// the driver's encoder (no link-time dependency on it), NULL when it is not exported
+inline TmaEncodeFn tma_encode_fn() {
+    static TmaEncodeFn fn = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        return (TmaEncodeFn)f;
+    }();
+    return fn;
+}
+
+// dims / box innermost first, strides (bytes) of dimensions 1 and 2; 128-byte swizzle, zeros outside
+inline bool tma_map_bf16_3d(CUtensorMap* m, const void* base, const uint64_t (&dims)[3], const uint64_t (&strides)[2], const uint32_t (&box)[3]) {
+    const cuuint64_t d[3] = {dims[0], dims[1], dims[2]}, s[2] = {strides[0], strides[1]};
+    const cuuint32_t b[3] = {box[0], box[1], box[2]}, one[3] = {1, 1, 1};
+    return tma_encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), d, s, b, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+#ifdef __CUDACC__
+__device__ __forceinline__ void tma_load_3d(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+                 :: "r"(smem_dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+}
+#endif
+
+}  // namespace pgk

@@ -302,11 +302,12 @@ class LinearRows:
                          ax[0], ax[1], ax[2], ax[3], ax[4], per_block, _st())
 
     def forward_grouped(self, x_ptr: int, ldx: int, out_ptr: int, ldo: int, a_rows: int | None, group_off: int,
-                        max_rows: int) -> None:
-        """Rows sorted by group: run g = rows group_off[g] .. group_off[g + 1] uses matrix g."""
+                        max_rows: int, rows: int = -1) -> None:
+        """Rows sorted by group: run g = rows group_off[g] .. group_off[g + 1] uses matrix g.  rows: a bound on all groups'
+        rows together (-1: not known; the product then runs on the general tiles)."""
         N, K = self.out_features, self.in_features
-        api.gemm_rows_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt, N * K, out_ptr, ldo, 0, N, K, group_off,
-                          self.groups, max_rows, self.epilogue, self.scale, self.cap, _st())
+        api.gemm_groups_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt, N * K, out_ptr, ldo, 0, N, K, group_off,
+                            self.groups, max_rows, rows, self.epilogue, self.scale, self.cap, _st())
 
     def forward_per_row(self, x_ptr: int, ldx: int, rows: int, out_ptr: int, ldo: int, a_rows: int | None,
                         row_group: int) -> None:

@@ -74,8 +74,8 @@ class GroupedRouterMoE:
             api.moe_row_lists(b.moe_counts.device_ptr, b.moe_off.device_ptr, b.moe_idx.device_ptr, b.moe_rank.device_ptr,
                               b.moe_perm.device_ptr, b.moe_inv.device_ptr, self.stack, T, top, _st())
             self.gate_up.forward_grouped(x.device_ptr, W, b.moe_act.device_ptr, ff, b.moe_perm.device_ptr,
-                                         b.moe_off.device_ptr, T)
-            self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T)
+                                         b.moe_off.device_ptr, T, T * top)
+            self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T, T * top)
             inv = b.moe_inv.device_ptr
         base = None
         if self.shared_gate_up is not None:
@@ -160,8 +160,8 @@ class BiasedRouterMoE:
                               b.moe_perm.device_ptr, b.moe_inv.device_ptr, max(R, self.stack), T, top, _st())
             if sp.experts > 0:
                 self.gate_up.forward_grouped(x.device_ptr, W, b.moe_act.device_ptr, ff, b.moe_perm.device_ptr,
-                                             b.moe_off.device_ptr, T)
-                self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T)
+                                             b.moe_off.device_ptr, T, T * top)
+                self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T, T * top)
             inv = b.moe_inv.device_ptr
         shared = None
         if self.shared_gate_up is not None:

@@ -1,0 +1,196 @@
+"""The many-row products of the token-major family at the sizes where their tiles end: row counts around the tile heights and
+the MMA's granularity, columns and k that are no multiple of a tile, k cut over a cluster, every epilogue, row gathers, groups
+of unequal length (empty, one row, several tiles) and batches -- against float64 products of the bfloat16-rounded operands.
+
+Tolerance: a product of K bfloat16 pairs is exact per pair; the sums are formed in float32 in blocks of 16, at most K / 16 + 8
+roundings of half a unit or truncations of one, so |error| <= (K / 16 + 8) 2^-23 sum |a w|.  An activation f changes that by its
+slope (at most 2 here, for pairs times the other factor), and adds a few units of its own value."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import pygpukit_b200 as gk
+from pygpukit_b200 import llm
+from pygpukit_b200._lib import api
+
+pytestmark = pytest.mark.gpu
+
+
+def bf16(a):
+    u = np.ascontiguousarray(a, np.float32).view(np.uint32)
+    return (((u + 0x7FFF + ((u >> 16) & 1)) >> 16) << 16).astype(np.uint32).view(np.float32)
+
+
+def dev_w(a):
+    a = np.ascontiguousarray(a, np.float32)
+    return gk.from_numpy((a.view(np.uint32) >> 16).astype(np.uint16).reshape(a.shape))
+
+
+def operands(seed, M, N, K, groups=1):
+    rng = np.random.default_rng(seed)
+    A = rng.standard_normal((M, K)).astype(np.float32)
+    W = bf16(rng.standard_normal((groups, N, K)).astype(np.float32) / np.sqrt(K))
+    return A, W
+
+
+def product(A, W):
+    a, w = bf16(A).astype(np.float64), W.astype(np.float64)
+    return a @ w.T, (K_ROUND(A.shape[1]) * (np.abs(a) @ np.abs(w).T))
+
+
+def K_ROUND(K):
+    return (K / 16 + 8) * 2.0 ** -23
+
+
+def no_wait_error():
+    v = C.c_int(7)
+    api.gemm_rows_wait_error(C.byref(v))
+    assert v.value == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 128, 64), (16, 130, 72), (17, 7, 128), (33, 257, 136), (64, 2048, 2048), (100, 96, 4096), (127, 129, 520),
+                                   (255, 384, 192), (256, 128, 64), (257, 640, 320), (300, 1000, 1000), (513, 2049, 264), (2000, 272, 128)])
+def test_rows(M, N, K):
+    A, W = operands(M + N, M, N, K)
+    ref, tol = product(A, W[0])
+    a, w = gk.from_numpy(A), dev_w(W[0])
+    c = gk.from_numpy(np.full((M, N + 3), 7.0, np.float32))
+    api.gemm_rows_f32(a.device_ptr, K, None, w.device_ptr, 2, 0, c.device_ptr, N + 3, M, N, K, None, 1, M, 0, 1.0, 0.0, None)
+    out = c.to_numpy()
+    assert (np.abs(out[:, :N] - ref) <= tol + 1e-6).all()
+    assert (out[:, N:] == 7.0).all()
+    no_wait_error()
+
+
+def gelu_tanh(z):
+    return 0.5 * z * (1 + np.tanh(np.sqrt(2 / np.pi) * (z + 0.044715 * z ** 3)))
+
+
+def sigmoid(z):
+    return 1 / (1 + np.exp(-z))
+
+
+@pytest.mark.parametrize("M,F,K", [(20, 66, 80), (130, 131, 256), (48, 64, 2048)])
+@pytest.mark.parametrize("epi", [1, 2, 3, 4, 5, 6, 7, 8, 9, 10])
+def test_epilogues(M, F, K, epi):
+    from math import erf
+    N = 2 * F if epi in (1, 3, 7) else F
+    A, W = operands(M + epi, M, N, K)
+    z, tol = product(A, W[0])
+    rng = np.random.default_rng(epi)
+    g, u = (z[:, 0::2], z[:, 1::2]) if epi in (1, 3, 7) else (z, None)
+    old = rng.standard_normal((M, F)).astype(np.float32)
+    colv = rng.standard_normal(F).astype(np.float32)
+    table = rng.standard_normal((11, F + 5)).astype(np.float32)
+    rows = rng.integers(0, 11, M).astype(np.int32)
+    gate = rng.standard_normal((M, F + 2)).astype(np.float32)
+    p0, p1, aux = 0.0, 0.0, (None, 0, None, 0, 0)
+    if epi == 1:
+        ref = g * sigmoid(g) * u
+    elif epi == 2:
+        p0, p1 = 1.3, 2.0
+        ref = 2.0 * np.tanh(1.3 * z / 2.0)
+    elif epi == 3:
+        p0, p1 = 1.702, 0.9
+        gg, uu = np.minimum(g, 0.9), np.clip(u, -0.9, 0.9)
+        ref = gg * sigmoid(1.702 * gg) * (uu + 1)
+    elif epi == 4:
+        ref = old + colv * z
+    elif epi == 5:
+        ref = gelu_tanh(z) * table[rows, 3:3 + F]
+    elif epi == 6:
+        ref = np.maximum(z, 0) ** 2
+    elif epi == 7:
+        ref = gelu_tanh(g) * u
+    elif epi == 8:
+        ref = 0.5 * z * (1 + np.vectorize(erf)(z / np.sqrt(2)))
+    elif epi == 9:
+        ref = gelu_tanh(z)
+    else:
+        ref = z * sigmoid(gate[:, 1:1 + F])
+    a, w, c = gk.from_numpy(A), dev_w(W[0]), gk.from_numpy(old)
+    dt, dr, dg, dc = gk.from_numpy(table), gk.from_numpy(rows), gk.from_numpy(gate), gk.from_numpy(colv)
+    if epi == 5:
+        aux = (dt.device_ptr, 0, dr.device_ptr, F + 5, 3)
+    if epi == 10:
+        aux = (dg.device_ptr, 0, None, F + 2, 1)
+    api.gemm_seq_f32(a.device_ptr, K, 0, w.device_ptr, 2, 0, c.device_ptr, F, 0, M, N, K, 1, epi, p0, p1, dc.device_ptr, aux[0], aux[1], aux[2],
+                     aux[3], aux[4], 0, None)
+    t = tol if epi not in (1, 3, 7) else np.maximum(tol[:, 0::2], tol[:, 1::2])
+    slope = 4.0 * (1.0 + (np.abs(u) + np.abs(g) if u is not None else np.abs(z)) + np.abs(table[rows, 3:3 + F]) + np.abs(colv))
+    assert (np.abs(c.to_numpy() - ref) <= slope * t + 1e-5 * (1 + np.abs(ref))).all()
+    no_wait_error()
+
+
+@pytest.mark.parametrize("counts,N,K", [([30, 0, 70, 1, 9], 130, 72), ([300, 16, 0, 17, 257, 1], 256, 128), ([0, 0, 5], 64, 200),
+                                        ([1] * 40, 96, 64), ([0] * 7, 96, 64), ([3, 129] * 20, 64, 96)])
+@pytest.mark.parametrize("extra", [0, 50])
+def test_groups(counts, N, K, extra):
+    E, R = len(counts), sum(counts)
+    T = max(R, 8)
+    A, W = operands(R + N, T, N, K, E)
+    rng = np.random.default_rng(R)
+    src = rng.integers(0, T, R + extra).astype(np.int32)
+    src[R:] = 1 << 30                                    # rows behind the last group name nothing
+    off = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    a, w, o, s = gk.from_numpy(A), dev_w(W), gk.from_numpy(off), gk.from_numpy(src if len(src) else np.zeros(1, np.int32))
+    c = gk.from_numpy(np.full((R + extra + 1, N), 7.0, np.float32))
+    lin = llm.LinearRows(w)
+    lin.forward_grouped(a.device_ptr, K, c.device_ptr, N, s.device_ptr, o.device_ptr, max(counts + [1]), R + extra)
+    out = c.to_numpy()
+    grp = np.repeat(np.arange(E), counts)
+    for e in range(E):
+        if counts[e]:
+            ref, tol = product(A[src[:R]][grp == e], W[e])
+            assert (np.abs(out[:R][grp == e] - ref) <= tol + 1e-6).all()
+    assert (out[R:] == 7.0).all()
+    no_wait_error()
+
+
+@pytest.mark.parametrize("M,H,N,K,pad", [(40, 3, 96, 64, 0), (70, 5, 512, 128, 8), (260, 2, 130, 72, 4), (33, 4, 64, 128, 3)])
+def test_batches(M, H, N, K, pad):
+    """products on slices of the same rows, K + pad columns apart (pad 3: off the 16-byte grid)"""
+    rng = np.random.default_rng(M)
+    A = rng.standard_normal((M, H * (K + pad))).astype(np.float32)
+    W = bf16(rng.standard_normal((H, N, K)).astype(np.float32) / np.sqrt(K))
+    a, w, c = gk.from_numpy(A), dev_w(W), gk.zeros((M, H * (N + 1)), gk.float32)
+    api.gemm_seq_f32(a.device_ptr, H * (K + pad), K + pad, w.device_ptr, 2, N * K, c.device_ptr, H * (N + 1), N + 1, M, N, K, H, 0, 0.0, 0.0, None,
+                     None, 0, None, 0, 0, 0, None)
+    out = c.to_numpy().reshape(M, H, N + 1)
+    for h in range(H):
+        ref, tol = product(A[:, h * (K + pad):h * (K + pad) + K], W[h])
+        assert (np.abs(out[:, h, :N] - ref) <= tol + 1e-6).all()
+    no_wait_error()
+
+
+def test_nan_stays_in_its_row_and_batch():
+    """a batch's k tail reads nothing of the next batch's columns"""
+    M, H, N, K = 20, 2, 64, 72
+    A = np.ones((M, H * K), np.float32)
+    A[:, K:] = np.nan
+    W = np.ones((H, N, K), np.float32)
+    a, w, c = gk.from_numpy(A), dev_w(W), gk.zeros((M, H * N), gk.float32)
+    api.gemm_seq_f32(a.device_ptr, H * K, K, w.device_ptr, 2, N * K, c.device_ptr, H * N, N, M, N, K, H, 0, 0.0, 0.0, None, None, 0, None, 0, 0, 0, None)
+    out = c.to_numpy()
+    assert (out[:, :N] == K).all() and np.isnan(out[:, N:]).all()
+
+
+def test_captured_and_replayed():
+    """work memory is part of a captured graph; replays follow new inputs"""
+    M, N, K = 50, 256, 512
+    A, W = operands(5, M, N, K)
+    a, w, c = gk.from_numpy(A), dev_w(W[0]), gk.zeros((M, N), gk.float32)
+    from pygpukit_b200.core.stream import CudaGraph, Stream
+    st, g = Stream(), CudaGraph()
+    lin = llm.LinearRows(w)
+    with g.capture(st):
+        lin.forward(a.device_ptr, K, M, c.device_ptr, N)
+        lin.forward(a.device_ptr, K, M, c.device_ptr, N)
+    for _ in range(3):
+        a.copy_from_numpy(A)
+        g.replay(st)
+        st.synchronize()
+        ref, tol = product(A, W[0])
+        assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6).all()
+        A = A[::-1].copy()
