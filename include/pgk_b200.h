@@ -780,6 +780,9 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
                      long long c_batch, int M, int N, int K, int batch, int epilogue, float p0, float p1, const float* col_scale,
                      const void* aux, int aux_dtype, const int32_t* aux_rows, int aux_ld, int aux_off, int rows_per_block,
                      void* stream);
+/* 1 in *out when a bounded wait of the tensor-core prompt attention ever ran out on this device (2: its shared memory was not
+ * where it needs it); its outputs are then not valid */
+int pgk_seq_attention_wait_error(int* out);
 int pgk_seq_decode_heads_per_block(void);
 int pgk_seq_heads_per_block(int heads, int kv_heads);
 int pgk_seq_queries_per_tile(int heads, int kv_heads);

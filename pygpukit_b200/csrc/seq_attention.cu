@@ -22,6 +22,7 @@
 //   mixer_prep_all: the form whose q / k norm runs over the WHOLE projection (all heads at once), with projection
 //                biases and values that are the keys before the norm.
 #include "common.cuh"
+#include "seq_attention.cuh"
 #include "../../include/pgk_b200.h"
 
 using namespace pgk;
@@ -263,42 +264,8 @@ __global__ void __launch_bounds__(256) mixer_prep_all_kernel(PrepAllArgs a) {
     }
 }
 
-struct AttnArgs {
-    const float* proj; int ld, q_off, g_off;
-    float* out; int ldo;
-    const void* kc; const void* vc; const int* table; int max_pages, PS;
-    const float* gsrc; int ldg;         // rows the gate is read from (gate 1: g_off + h * Dv + dv, gate 2: g_off + h)
-    const float* sinks;                 // [H] or NULL: a score per head that joins the denominator and has no value
-    int window;                         // > 0: key j is visible from i only when i - j < window
-    int kld, vld;                       // elements between consecutive positions' rows in the K / V arrays
-    int valias;                         // the value rows are the first Dv elements of the key rows (one staging)
-    const int4* tiles;                  // (first token row, queries, slot, first position)
-    const float* slopes;                // [H] or NULL
-    const float* slopes2;               // [H] or NULL: the distance term is slopes[h] * ln(1 + slopes2[h] * (i - j)) instead
-    int keep;                           // with a window: the first `keep` positions stay visible beyond it
-    int prob;                           // 0: softmax over the visible keys; 1: weight sigmoid(score + pbias[h]), not normalised
-    const float* pbias;                 // [H] or NULL
-    float out_mult;                     // constant factor on the output
-    int H, G, D, Dv, chunk, HB, gate;
-    float scale, cap;
-    int splits; float* ws;              // splits > 1: partial (m, l, acc[Dv]) records [row][H][splits][Dv + 2]
-    unsigned* tickets;                  // one arrival counter per (tile, head block), zero between launches
-    int pool, pool_rows;                // pool > 0 (with a window): means of blocks of `pool` positions, rows per page of pk / pv
-    const void* pk; const void* pv;     // [pages][G][pool_rows][D] / [Dv], dense rows
-    const double* o_inv_freq;           // [Dv / 2] or NULL: pair m of an output (elements m and m + Dv / 2, or 2m and 2m + 1
-    int o_pairs;                        // with o_pairs) turns by -position * o_inv_freq[m]
-};
-
 constexpr int KT = 32;                  // keys per tile = one per lane
 
-__device__ __forceinline__ float gate_logit(const AttnArgs& a, size_t t, int h, int dv) {
-    return a.gsrc[t * a.ldg + a.g_off + (a.gate == 2 ? (size_t)h : (size_t)h * a.Dv + dv)];
-}
-__device__ __forceinline__ int first_key(const AttnArgs& a, int pos) {
-    int lo = a.chunk > 0 ? (pos / a.chunk) * a.chunk : 0;
-    if (a.window > 0) lo = max(lo, pos - a.window + 1);
-    return lo;
-}
 // The keys of a tile whose lowest window start is jlo come in two runs: the kept first positions below jlo, [0, kept), and
 // [jlo, jhi].  Key tile ti covers KT positions from tile_first(); positions past tile_last() are padding.
 // With pooled blocks the first run is the blocks instead, [0, blocks_seen(last query)), a row of pk / pv each.
@@ -329,11 +296,6 @@ __device__ __forceinline__ float turn_back(const AttnArgs& a, int pos, int dv, f
     rope_angle_sincos(pos, a.o_inv_freq[a.o_pairs ? dv >> 1 : (second ? dv - half : dv)], sn, cs);
     return second ? fmaf(o, cs, -partner * sn) : fmaf(o, cs, partner * sn);
 }
-__device__ __forceinline__ float distance_term(float slope, float slope2, bool log_form, int dist) {
-    const float d = (float)max(dist, 0);
-    return log_form ? slope * log1pf(slope2 * d) : slope * d;
-}
-
 // KT cache rows of n elements -> shared memory as float32 (row stride ld), 16 bytes per load when the rows allow it;
 // rows with offset < 0 (past the last key) are zero-filled
 template <typename TC>
@@ -1087,6 +1049,11 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
     if (single_query)       // every tile holds one query: the decoding kernel
         return cache_dtype == 2 ? launch_attn_decode_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
                                 : launch_attn_decode_nv<float>(a, n_tiles, (cudaStream_t)stream);
+    if (cache_dtype == 2 && !extended(a)) {      // the tensor cores serve what they can fetch; the kernel below the rest
+        bool served = false;
+        if (const int rc = seq_attention_tc(a, n_tiles, (cudaStream_t)stream, &served)) return rc;
+        if (served) return 0;
+    }
     return cache_dtype == 2 ? launch_attn_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
                             : launch_attn_nv<float>(a, n_tiles, (cudaStream_t)stream);
 }

@@ -276,7 +276,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         int u = 0;
         for (int t = first; t < total; t += step, ++u) {
             const Tile w = tile_at(p, pre, t);
-            if (!bar_wait(&g_tc_wait_error, smem_u32(&done_bar[u & 1]), (uint32_t)((u >> 1) & 1))) break;
+            if (!__all_sync(0xffffffffu, bar_wait(&g_tc_wait_error, smem_u32(&done_bar[u & 1]), (uint32_t)((u >> 1) & 1)))) break;
             tc_fence_after();
             const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(u & 1) * TC_ROWS_MAX;
             const int col = w.n0 + quad * 32 + lane;
