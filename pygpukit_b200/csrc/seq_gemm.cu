@@ -423,8 +423,24 @@ int launch_few_t(const GemmArgs& a, int rows_per_block, cudaStream_t st, int bat
     return 0;
 }
 
+// Few rows, bfloat16 weights: the tcgen05 form (gemm_few_tc) reads the weights at the rate of HBM whatever the rows, but takes 7 us
+// from its first barrier to its last store; a warp per column pair starts faster and then costs time per row.  The line lies where
+// the two meet, rows^2 N K (matrices) = 2^24 (us, warp per pair -> tcgen05): one row of 2048 x 2048 7.4 -> 8.3, of 8192 x 2048
+// 11 -> 11, of 32768 x 2048 35 -> 25; eight rows of 512 x 2048 14.4 -> 8.0, 2048 x 8192 37 -> 14.5, 24576 x 4096 158 -> 37; eight
+// rows with matrices of their own, 4096 x 2048, 37 -> 14.5.
+inline bool few_tc_pays(const GemmArgs& a, int rows_per_block, int batch) {
+    const double rows = a.row_group ? rows_per_block : a.M;
+    const double matrices = a.row_group ? (a.M + rows_per_block - 1) / rows_per_block : batch;
+    return rows * rows * matrices * (double)a.N * (double)a.K >= 16777216.0;
+}
+
 template <int EPI>
 int launch_few(const GemmArgs& a, int wdt, int rows_per_block, cudaStream_t st, int batch = 1) {
+    if (wdt == 2 && few_tc_pays(a, rows_per_block, batch)) {
+        bool served = false;
+        if (const int rc = gemm_few_tc(a, EPI, batch, rows_per_block, st, &served)) return rc;
+        if (served) return 0;
+    }
     if (wdt == 2) return launch_few_t<uint16_t, EPI, true>(a, rows_per_block, st, batch);
     return launch_few_t<float, EPI, false>(a, rows_per_block, st, batch);
 }

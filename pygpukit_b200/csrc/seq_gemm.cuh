@@ -39,4 +39,8 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 // bound of the longest group.  *served is false, and nothing is launched, when the operands do not fit its copies.
 int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_rows, cudaStream_t st, bool* served);
 
+// The same for at most 16 rows, in one launch without work memory: `batch` products over the same rows, or blocks of rows_per_block
+// rows that share the matrix a.row_group names.
+int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, cudaStream_t st, bool* served);
+
 }  // namespace pgk

@@ -12,8 +12,9 @@
 //   * TMA brings both operands (128-byte swizzle) into a ring of stages, one thread issues the MMAs, two accumulators in TMEM
 //     let eight epilogue warps drain a tile while the next one is multiplied, and one block per SM walks the tiles;
 //   * few tiles: a cluster of 2 ... 8 blocks shares a tile, each with a part of k, and the partial sums meet in shared memory
-//     (distributed loads, added in the order of the ranks), so that all SMs pull on the weights.
-// Measured on B200, 2000 x 9216 x 2048: 573 us on the 64 x 64 tiles of seq_gemm.cu (132 TFLOP/s), 6 + 76 us here (0.99 PFLOP/s in
+//     (distributed loads, added in the order of the ranks), so that all SMs pull on the weights;
+//   * up to 16 rows (decoding): a kernel of its own (gemm_few_tc_kernel), one launch without work memory.
+// Measured on B200, 2000 x 9216 x 2048: 573 us on the 64 x 64 tiles of seq_gemm.cu (132 TFLOP/s), 6 + 59 us here (1.27 PFLOP/s in
 // the product); 8000 gathered rows over 16 experts, 4096 x 2048 and 2048 x 2048: 1510 -> 262 us for both.
 #include "seq_gemm.cuh"
 #include "tc_common.cuh"
@@ -31,6 +32,10 @@ constexpr int TC_MAX_GROUPS = 512;
 constexpr uint32_t TC_W_BYTES = kTcRows * TBK * 2;
 constexpr uint32_t TC_RING_BYTES = 200 * 1024;
 constexpr int TC_MAX_STAGES = 10;
+constexpr int TC_DIRECT_ROWS = 16;         // rows whose activations the kernel rounds itself
+constexpr int FEW_STAGES = 5;
+constexpr uint32_t FEW_STAGE_BYTES = TC_W_BYTES + TC_DIRECT_ROWS * TBK * 2;
+constexpr uint32_t FEW_SMEM = FEW_STAGES * FEW_STAGE_BYTES + 1024;      // with 16 KB of partial rows: two blocks per SM
 
 struct TcArgs {
     GemmArgs g;
@@ -115,40 +120,47 @@ __device__ __forceinline__ Tile tile_at(const TcArgs& p, const int* pre, int t) 
     return w;
 }
 
-// ---------------------------------------------------------------- epilogue: 16 rows of one output column per lane
-template <typename F>
-__device__ __forceinline__ void store16(const GemmArgs& a, const float (&v)[16], int row, int left, int col, F f) {
+// ---------------------------------------------------------------- epilogue: R rows of one output column per lane
+template <int R, typename F>
+__device__ __forceinline__ void store_rows(const GemmArgs& a, const float (&v)[R], int row, int left, int col, F f) {
     if (col >= a.N) return;
     float* p = a.C + (size_t)row * a.ldc + col;
 #pragma unroll
-    for (int j = 0; j < 16; ++j)
+    for (int j = 0; j < R; ++j)
         if (j < left) p[(size_t)j * a.ldc] = f(v[j], j);
 }
 // pairs (2j, 2j + 1) of columns sit in neighbouring lanes: the even lane finishes the even rows, the odd lane the odd ones
-template <typename F>
-__device__ __forceinline__ void store16_pairs(const GemmArgs& a, const float (&v)[16], int row, int left, int col, int lane, F f) {
+template <int R, typename F>
+__device__ __forceinline__ void store_pairs(const GemmArgs& a, const float (&v)[R], int row, int left, int col, int lane, F f) {
     const bool odd = lane & 1;
+    if constexpr (R == 1) {
+        const float second = __shfl_xor_sync(0xffffffffu, v[0], 1);
+        if (!odd && col + 1 < a.N && left > 0) a.C[(size_t)row * a.ldc + (col >> 1)] = f(v[0], second);
+        return;
+    } else {
 #pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-        const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
-        const float first = odd ? got : v[j], second = odd ? v[j + 1] : got;
-        const int jj = odd ? j + 1 : j;
-        if ((col | 1) < a.N && jj < left) a.C[(size_t)(row + jj) * a.ldc + (col >> 1)] = f(first, second);
+        for (int j = 0; j < R; j += 2) {
+            const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
+            const float first = odd ? got : v[j], second = odd ? v[j + 1] : got;
+            const int jj = odd ? j + 1 : j;
+            if ((col | 1) < a.N && jj < left) a.C[(size_t)(row + jj) * a.ldc + (col >> 1)] = f(first, second);
+        }
     }
 }
 
-__device__ __forceinline__ void epilogue16(const GemmArgs& a, int epi, const float (&v)[16], int row, int left, int col, int lane) {
+template <int R>
+__device__ __forceinline__ void epilogue_rows(const GemmArgs& a, int epi, const float (&v)[R], int row, int left, int col, int lane) {
     switch (epi) {
-        case 1: store16_pairs(a, v, row, left, col, lane, [](float g, float u) { return silu_f(g) * u; }); return;
-        case 7: store16_pairs(a, v, row, left, col, lane, [](float g, float u) { return gelu_tanh_f(g) * u; }); return;
+        case 1: store_pairs<R>(a, v, row, left, col, lane, [](float g, float u) { return silu_f(g) * u; }); return;
+        case 7: store_pairs<R>(a, v, row, left, col, lane, [](float g, float u) { return gelu_tanh_f(g) * u; }); return;
         case 3:          // scale = alpha, cap = limit
-            store16_pairs(a, v, row, left, col, lane, [&](float c0, float c1) {
+            store_pairs<R>(a, v, row, left, col, lane, [&](float c0, float c1) {
                 const float g = fminf(c0, a.cap), u = fminf(fmaxf(c1, -a.cap), a.cap);
                 return g / (1.f + expf(-a.scale * g)) * (u + 1.f);
             });
             return;
         case 2:
-            store16(a, v, row, left, col, [&](float c, int) {
+            store_rows<R>(a, v, row, left, col, [&](float c, int) {
                 c *= a.scale;
                 return a.cap > 0.f ? a.cap * tanhf(c / a.cap) : c;
             });
@@ -156,27 +168,27 @@ __device__ __forceinline__ void epilogue16(const GemmArgs& a, int epi, const flo
         case 4: {
             if (col >= a.N) return;
             const float s = a.colv[col];
-            float old[16];
+            float old[R];
             const float* p = a.C + (size_t)row * a.ldc + col;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) old[j] = j < left ? p[(size_t)j * a.ldc] : 0.f;
-            store16(a, v, row, left, col, [&](float c, int j) { return fmaf(s, c, old[j]); });
+            for (int j = 0; j < R; ++j) old[j] = j < left ? p[(size_t)j * a.ldc] : 0.f;
+            store_rows<R>(a, v, row, left, col, [&](float c, int j) { return fmaf(s, c, old[j]); });
             return;
         }
         case 5:
-            store16(a, v, row, left, col, [&](float c, int j) { return gelu_tanh_f(c) * aux_at(a, row + j, col); });
+            store_rows<R>(a, v, row, left, col, [&](float c, int j) { return gelu_tanh_f(c) * aux_at(a, row + j, col); });
             return;
         case 6:
-            store16(a, v, row, left, col, [](float c, int) { c = fmaxf(c, 0.f); return c * c; });
+            store_rows<R>(a, v, row, left, col, [](float c, int) { c = fmaxf(c, 0.f); return c * c; });
             return;
-        case 8: store16(a, v, row, left, col, [](float c, int) { return gelu_erf_f(c); }); return;
-        case 9: store16(a, v, row, left, col, [](float c, int) { return gelu_tanh_f(c); }); return;
+        case 8: store_rows<R>(a, v, row, left, col, [](float c, int) { return gelu_erf_f(c); }); return;
+        case 9: store_rows<R>(a, v, row, left, col, [](float c, int) { return gelu_tanh_f(c); }); return;
         case 10:         // the gate's columns are as far apart as the output's: `aux` moves with C from batch to batch
-            store16(a, v, row, left, col, [&](float c, int j) {
+            store_rows<R>(a, v, row, left, col, [&](float c, int j) {
                 return c * (1.f / (1.f + expf(-((const float*)a.aux)[(size_t)(row + j) * a.aux_ld + a.aux_off + col])));
             });
             return;
-        default: store16(a, v, row, left, col, [](float c, int) { return c; });
+        default: store_rows<R>(a, v, row, left, col, [](float c, int) { return c; });
     }
 }
 
@@ -188,7 +200,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     __shared__ uint32_t tmem_base_s;
     __shared__ int pre[TC_MAX_GROUPS + 1];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u;
+    const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
 
     if (warp == 1) tmem_alloc(&tmem_base_s, 512);
     if (tid == 0) {
@@ -226,17 +238,17 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     const int per = (p.nkb + p.splits - 1) / p.splits, kb0 = rank * per, kb1 = min(p.nkb, kb0 + per);
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
+            RingPos r;
             int i = 0;                            // stages filled so far
             bool ok = true;
             for (int t = first; ok && t < total; t += step) {
                 const Tile w = tile_at(p, pre, t);
                 const int boxes = (w.rows + p.abox - 1) / p.abox, az = p.g.group_off ? 0 : w.z;
                 const uint32_t bytes = TC_W_BYTES + (uint32_t)(boxes * p.abox) * (TBK * 2);
-                for (int kb = kb0; kb < kb1; ++kb, ++i) {
-                    const int s = i % p.stages;
-                    const uint32_t fb = smem_u32(&full_bar[s]), dst = ring + (uint32_t)s * p.stage_bytes;
-                    if (!bar_wait(&g_tc_wait_error, smem_u32(&empty_bar[s]), (uint32_t)(((i / p.stages) & 1) ^ 1))) { ok = false; break; }
+                for (int kb = kb0; kb < kb1; ++kb, ++i, r.next(p.stages)) {
+                    const uint32_t fb = full + 8u * r.s, dst = ring + r.s * p.stage_bytes;
+                    if (!bar_wait(&g_tc_wait_error, empty + 8u * r.s, r.round ^ 1u)) { ok = false; break; }
                     mbar_expect_tx(fb, bytes);
                     tma_load_3d(dst, &wmap, kb * TBK, w.n0, w.z, fb);
                     for (int b = 0; b < boxes; ++b)
@@ -248,24 +260,24 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {
-            int i = 0, u = 0;
+        if (elect_one()) {
+            RingPos r;
+            int u = 0;
             bool ok = true;
             for (int t = first; ok && t < total; t += step, ++u) {
                 const Tile w = tile_at(p, pre, t);
                 const uint32_t idesc = umma_idesc_bf16((w.rows + 15) & ~15), acc = tmem + (uint32_t)(u & 1) * TC_ROWS_MAX;
                 if (!bar_wait(&g_tc_wait_error, smem_u32(&drained_bar[u & 1]), (uint32_t)(((u >> 1) & 1) ^ 1))) break;
                 tc_fence_after();
-                for (int kb = kb0; kb < kb1; ++kb, ++i) {
-                    const int s = i % p.stages;
-                    if (!bar_wait(&g_tc_wait_error, smem_u32(&full_bar[s]), (uint32_t)((i / p.stages) & 1))) { ok = false; break; }
+                for (int kb = kb0; kb < kb1; ++kb, r.next(p.stages)) {
+                    if (!bar_wait(&g_tc_wait_error, full + 8u * r.s, r.round)) { ok = false; break; }
                     tc_fence_after();
-                    const uint32_t addr = ring + (uint32_t)s * p.stage_bytes;
+                    const uint32_t addr = ring + r.s * p.stage_bytes;
                     const uint64_t dw = desc_sw128(addr), da = desc_sw128(addr + TC_W_BYTES);
 #pragma unroll
                     for (int ks = 0; ks < TBK / 16; ++ks)         // 32 bytes of k per MMA: +2 in the descriptor's 16-byte units
                         umma_bf16(acc, dw + (uint64_t)(ks * 2), da + (uint64_t)(ks * 2), idesc, (kb > kb0 || ks > 0) ? 1u : 0u);
-                    umma_commit(&empty_bar[s]);
+                    umma_commit(&empty_bar[r.s]);
                 }
                 if (ok) umma_commit(&done_bar[u & 1]);
             }
@@ -289,7 +301,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 for (int c = half * 16; c < w.rows; c += 32) {
                     float v[16];
                     tmem_ld16(acc + c, v);
-                    epilogue16(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
+                    epilogue_rows<16>(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
                     __syncwarp();
                 }
             } else {                              // this block's share of k: row c of the partial tile, 128 columns
@@ -325,7 +337,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 for (int s = 0; s < parts; ++s)
 #pragma unroll
                     for (int j = 0; j < 16; ++j) v[j] += ld_cluster(ring + (uint32_t)((c + j) * kTcRows + quad * 32 + lane) * 4u, (uint32_t)s);
-                epilogue16(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
+                epilogue_rows<16>(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
             }
         }
         cluster_arrive_wait();                    // the others may still read this block's partial sums
@@ -333,6 +345,170 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem, 512);
+}
+
+// ---------------------------------------------------------------- at most 16 rows
+// One tile of `th` weight rows (or a share of its k) per block, two blocks per SM: the next block's start -- barriers, TMEM,
+// the first copies' way from HBM, 5000 cycles -- hides behind the other's stream.  No work memory: the epilogue warps, idle until
+// the tile is done, round the float32 rows into the stages, eight k blocks per fence (a fence also waits for loads in flight).
+// A cluster that shares a tile along k pushes its partial rows to their owners' shared memory, one barrier, and every block
+// finishes its rows.  Measured at 8 rows, against a warp per column pair (gemm_few_rows_kernel): see few_tc_pays.
+struct FewArgs {
+    GemmArgs g;
+    int epi, th, nkb, kper, splits, rpb, avec;
+};
+
+__device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* row, int k, bool vec) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (row && k < a.K) {                        // K is a multiple of eight
+        if (vec) v = *(const float4*)(row + k);
+        else { v.x = row[k]; v.y = row[k + 1]; v.z = row[k + 2]; v.w = row[k + 3]; }
+    }
+    return v;
+}
+
+__global__ void __launch_bounds__(TC_THREADS, 2)
+gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ FewArgs p) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t full_bar[FEW_STAGES], empty_bar[FEW_STAGES], done_bar;
+    __shared__ uint32_t tmem_base_s;
+    __shared__ float part[TC_DIRECT_ROWS * 2 * kTcRows];               // partial rows: [rank][row slot][128], at most 16 + 7 rows
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
+    const int rank = blockIdx.x, n0 = blockIdx.y * p.th, kb0 = rank * p.kper, kb1 = min(p.nkb, kb0 + p.kper);
+
+    if (warp == 1) tmem_alloc(&tmem_base_s, 32);
+    if (tid == 0) {
+        for (int s = 0; s < FEW_STAGES; ++s) { mbar_init(&full_bar[s], 9); mbar_init(&empty_bar[s], 1); }
+        mbar_init(&done_bar, 1);
+        mbar_fence_init();
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
+    }
+    griddep_wait();
+    const int m0 = p.rpb ? (int)blockIdx.z * p.rpb : 0, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z;
+    const int rows = z < 0 ? 0 : min(p.rpb ? p.rpb : TC_DIRECT_ROWS, p.g.M - m0);      // no matrix: nothing to do, the same in the cluster
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base_s;
+    if (p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // this block runs
+    float v[16];
+
+    if (rows > 0 && warp == 0) {
+        if (elect_one()) {
+            RingPos r;
+            const uint32_t bytes = (uint32_t)p.th * (TBK * 2);
+            for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
+                if (!bar_wait(&g_tc_wait_error, empty + 8u * r.s, r.round ^ 1u)) break;
+                mbar_expect_tx(full + 8u * r.s, bytes);
+                tma_load_3d(ring + r.s * FEW_STAGE_BYTES, &wmap, kb * TBK, n0, z, full + 8u * r.s);
+            }
+        }
+        __syncwarp();
+    } else if (rows > 0 && warp == 1) {
+        if (elect_one()) {
+            RingPos r;
+            constexpr uint32_t idesc = umma_idesc_bf16(TC_DIRECT_ROWS);
+            for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
+                if (!bar_wait(&g_tc_wait_error, full + 8u * r.s, r.round)) break;
+                tc_fence_after();
+                const uint32_t addr = ring + r.s * FEW_STAGE_BYTES;
+                const uint64_t dw = desc_sw128(addr), da = desc_sw128(addr + TC_W_BYTES);
+#pragma unroll
+                for (int ks = 0; ks < TBK / 16; ++ks)
+                    umma_bf16(tmem, dw + (uint64_t)(ks * 2), da + (uint64_t)(ks * 2), idesc, (kb > kb0 || ks > 0) ? 1u : 0u);
+                umma_commit(&empty_bar[r.s]);
+            }
+            umma_commit(&done_bar);
+        }
+        __syncwarp();
+    } else if (rows > 0) {
+        // this thread's row and four columns of every k block
+        constexpr int DEPTH = 8;
+        const int et = tid - 64, r = et >> 4, c4 = et & 15;
+        const float* row = nullptr;
+        if (r < rows) row = p.g.A + (size_t)(p.rpb ? 0 : z) * p.g.a_z + (size_t)(p.g.a_rows ? p.g.a_rows[m0 + r] : m0 + r) * p.g.lda;
+        const uint32_t at = ring + TC_W_BYTES + (uint32_t)r * 128u + (uint32_t)(((c4 >> 1) ^ (r & 7)) << 4) + (uint32_t)(c4 & 1) * 8u;
+        RingPos f;
+        bool ok = true;
+        for (int kb = kb0; kb < kb1; kb += DEPTH) {
+            const int nb = min(DEPTH, kb1 - kb);
+            float4 v[DEPTH];
+#pragma unroll
+            for (int d = 0; d < DEPTH; ++d) v[d] = direct_load(p.g, d < nb ? row : nullptr, (kb + d) * TBK + c4 * 4, p.avec);
+            // hand over in groups that the ring can hold: a group's stages are free before any of them is written
+#pragma unroll
+            for (int d0 = 0; d0 < DEPTH; d0 += 4) {
+                if (d0 >= nb) break;
+                RingPos h = f;
+#pragma unroll
+                for (int d = d0; d < d0 + 4; ++d) {
+                    if (d >= nb) break;
+                    ok = ok && bar_wait(&g_tc_wait_error, empty + 8u * f.s, f.round ^ 1u);
+                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(at + f.s * FEW_STAGE_BYTES), "r"(pack_bf16x2(v[d].x, v[d].y)),
+                                 "r"(pack_bf16x2(v[d].z, v[d].w)) : "memory");
+                    f.next(FEW_STAGES);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0)
+                    for (int d = d0; d < min(d0 + 4, nb); ++d, h.next(FEW_STAGES)) mbar_arrive(&full_bar[h.s]);
+            }
+        }
+        const int quad = warp & 3, col = n0 + quad * 32 + lane;
+        if (warp < 6) {                                   // four warps drain: lane = output column, v = the rows
+            bar_wait(&g_tc_wait_error, smem_u32(&done_bar), 0);
+            __syncwarp();
+            tc_fence_after();
+            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16), v);
+            if (p.splits == 1) {
+                GemmArgs a = p.g;
+                a.N = min(a.N, n0 + p.th);
+                if (!p.rpb) {
+                    a.C += (size_t)z * a.c_z;
+                    if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)z * a.c_z;
+                }
+                epilogue_rows<16>(a, p.epi, v, m0, rows, col, lane);
+            }
+        }
+    }
+    if (p.splits > 1) {
+        const int quad = warp & 3, col = n0 + quad * 32 + lane, slots = (rows + p.splits - 1) / p.splits;
+        __syncwarp();
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");                       // so do the others
+        if (rows > 0 && warp >= 2 && warp < 6) {          // row j belongs to block j % splits
+            int owner = 0, slot = 0;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                if (j < rows) {
+                    const uint32_t to = smem_u32(part) + (uint32_t)((rank * slots + slot) * kTcRows + quad * 32 + lane) * 4u;
+                    uint32_t remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(to), "r"(owner));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(remote), "f"(v[j]) : "memory");
+                }
+                if (++owner == p.splits) { owner = 0; ++slot; }
+            }
+        }
+        __syncwarp();
+        cluster_arrive_wait();
+        if (rows > 0 && warp >= 2 && warp < 6) {
+            const int parts = (p.nkb + p.kper - 1) / p.kper;          // blocks that had any k
+            GemmArgs a = p.g;
+            a.N = min(a.N, n0 + p.th);
+            if (!p.rpb) {
+                a.C += (size_t)z * a.c_z;
+                if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)z * a.c_z;
+            }
+            for (int j = rank, slot = 0; j < rows; j += p.splits, ++slot) {
+                float sum[1] = {0.f};
+                for (int s = 0; s < parts; ++s) sum[0] += part[(s * slots + slot) * kTcRows + quad * 32 + lane];
+                epilogue_rows<1>(a, p.epi, sum, m0 + j, 1, col, lane);
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) tmem_dealloc(tmem, 32);
 }
 
 // ---------------------------------------------------------------- how a product is cut
@@ -361,8 +537,106 @@ Plan tc_plan(int M, long long ntz, int nkb) {
     }
     return best;
 }
+// clusters of s blocks of the few-row kernel that the device holds at one time: clusters do not cross its processing clusters, whose
+// SMs are no multiple of s
+int clusters_held(int s) {
+    static int held[9] = {};
+    if (held[s] == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(s, 64); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = FEW_SMEM;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = s; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(gemm_few_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FEW_SMEM) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, gemm_few_tc_kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        held[s] = n > 0 ? n : -1;
+    }
+    return held[s];
+}
+struct FewPlan { int th, splits; };
+// Tile height and blocks per tile.  An SM draws 24 bytes of weights per cycle when all do (HBM), a copy takes 300 cycles at
+// least; a block's start and end cost 6000 cycles, half hidden where two blocks share an SM, a shared tile 1500 more.
+FewPlan few_plan(int N, int zs, int nkb) {
+    FewPlan best{kTcRows, 1};
+    double best_cost = 1e30;
+    const int sms = sm_count();
+    for (int s = 1; s <= 8; ++s) {
+        if (s > 1 && (nkb < 2 * s || s > 1 && clusters_held(s) <= 0)) continue;
+        for (int th = 16; th <= kTcRows; th += 8) {
+            const long long tiles = (long long)((N + th - 1) / th) * zs, blocks = tiles * s;
+            const int held = s == 1 ? 2 * sms : clusters_held(s) * s;
+            const double rounds = (double)((blocks + held - 1) / held), per_sm = blocks <= sms ? 1.0 : fmin(2.0, (double)blocks / sms);
+            const double block = (double)((nkb + s - 1) / s) * fmax(per_sm * th * (TBK * 2) / 24.0, 300.0);
+            const double cost = rounds * block + 6000.0 + (rounds - 1.0) * 3000.0 + (s > 1 ? 1500.0 : 0.0);
+            if (cost < best_cost * 0.999) { best_cost = cost; best = {th, s}; }
+        }
+    }
+    return best;
+}
+
+cudaError_t launch_clustered(const void* kernel, dim3 grid, size_t smem, int cluster, cudaStream_t st, void** args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    int n = 0;
+    at[n].id = cudaLaunchAttributeClusterDimension;
+    at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
+    ++n;
+    if (pdl_enabled()) {
+        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[n].val.programmaticStreamSerializationAllowed = 1;
+        ++n;
+    }
+    cfg.attrs = at; cfg.numAttrs = n;
+    count_launch();
+    return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
+bool weight_map(CUtensorMap* m, const GemmArgs& a, uint64_t matrices, bool many, int height) {
+    const uint64_t wd[3] = {(uint64_t)a.K, (uint64_t)a.N, matrices};
+    const uint64_t ws[2] = {(uint64_t)a.K * 2, (uint64_t)(many ? a.w_stride : (long long)a.N * a.K) * 2};
+    const uint32_t wb[3] = {TBK, (uint32_t)height, 1};
+    return tma_map_bf16_3d(m, a.W, wd, ws, wb);
+}
 
 }  // namespace
+
+int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, cudaStream_t st, bool* served) {
+    *served = false;
+    const bool own = a.row_group != nullptr, many = own || batch > 1;
+    if (a.K % 8 || a.K < TBK || (uintptr_t)a.W % 16 || (many && (a.w_stride % 8 || a.w_stride <= 0)) || !tma_encode_fn()) return 0;
+    if (a.group_off || (own ? rows_per_block : a.M) > TC_DIRECT_ROWS || (own && batch > 1) || a.M <= 0) return 0;
+    const int zs = own ? (a.M + rows_per_block - 1) / rows_per_block : batch;
+    if (zs > 65535) return 0;
+    FewArgs p{};
+    p.g = a;
+    p.epi = epilogue;
+    p.nkb = (a.K + TBK - 1) / TBK;
+    const FewPlan plan = few_plan(a.N, zs, p.nkb);
+    if ((a.N + plan.th - 1) / plan.th > 65535) return 0;
+    p.th = plan.th;
+    p.splits = plan.splits;
+    p.kper = (p.nkb + p.splits - 1) / p.splits;
+    p.rpb = own ? rows_per_block : 0;
+    p.avec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
+    CUtensorMap wmap;
+    if (!weight_map(&wmap, a, own ? 1u << 20 : (uint64_t)batch, many, p.th)) return 0;      // row groups name matrices that exist
+    static bool configured = false;
+    if (!configured) {
+        PGK_CUDA(cudaFuncSetAttribute(gemm_few_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FEW_SMEM));
+        configured = true;
+    }
+    void* args[] = {&wmap, &p};
+    const cudaError_t e = launch_clustered((const void*)gemm_few_tc_kernel, dim3(p.splits, (a.N + p.th - 1) / p.th, zs), FEW_SMEM, p.splits, st, args);
+    if (e != cudaSuccess) return cuda_fail(e, "gemm_few_tc", __FILE__, __LINE__);
+    *served = true;
+    return 0;
+}
 
 int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_rows, cudaStream_t st, bool* served) {
     *served = false;
@@ -371,6 +645,7 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
     if (a.group_off && batch > TC_MAX_GROUPS) return 0;
     if (rows <= 0) return 0;
     const bool grouped = a.group_off != nullptr;
+    if (!grouped && a.M <= TC_DIRECT_ROWS) return gemm_few_tc(a, epilogue, batch, a.M, st, served);
     TcArgs p{};
     p.g = a;
     p.epi = epilogue;
@@ -403,21 +678,13 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
         return 0;
     }
     CUtensorMap wmap, amap;
-    const uint64_t wd[3] = {(uint64_t)a.K, (uint64_t)a.N, (uint64_t)batch};
-    const uint64_t ws[2] = {(uint64_t)a.K * 2, (uint64_t)(batch > 1 ? a.w_stride : (long long)a.N * a.K) * 2};
-    const uint32_t wb[3] = {TBK, kTcRows, 1};
     const uint64_t ad[3] = {(uint64_t)a.K, (uint64_t)nb, (uint64_t)rows};
     const uint64_t as[2] = {(uint64_t)a.K * 2, (uint64_t)nb * a.K * 2};
     const uint32_t ab[3] = {TBK, 1, (uint32_t)p.abox};
-    if (!tma_map_bf16_3d(&wmap, a.W, wd, ws, wb) || !tma_map_bf16_3d(&amap, abuf, ad, as, ab)) {
+    if (!weight_map(&wmap, a, (uint64_t)batch, batch > 1, kTcRows) || !tma_map_bf16_3d(&amap, abuf, ad, as, ab)) {
         scratch_free(abuf, st);
         set_error("gemm_rows failed: the copies of a %d x %d x %d product cannot be described", rows, a.N, a.K);
         return 1;
-    }
-    static bool configured = false;
-    if (!configured) {
-        PGK_CUDA(cudaFuncSetAttribute(gemm_rows_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_RING_BYTES + 1024));
-        configured = true;
     }
     const int kpr = a.K / 8, chunks = nb * kpr;
     const bool vec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
@@ -428,21 +695,13 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
         const int sms = sm_count();
         const long long tiles = (long long)batch * p.mt * p.nt;
         const int grid = grouped ? sms : (p.splits > 1 ? (int)(tiles * p.splits) : (int)(tiles < sms ? tiles : sms));
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(grid); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = TC_RING_BYTES + 1024; cfg.stream = st;
-        cudaLaunchAttribute at[2];
-        int n = 0;
-        at[n].id = cudaLaunchAttributeClusterDimension;
-        at[n].val.clusterDim.x = p.splits; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
-        ++n;
-        if (pdl_enabled()) {
-            at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[n].val.programmaticStreamSerializationAllowed = 1;
-            ++n;
+        static bool configured = false;
+        if (!configured) {
+            e = cudaFuncSetAttribute(gemm_rows_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_RING_BYTES + 1024);
+            configured = e == cudaSuccess;
         }
-        cfg.attrs = at; cfg.numAttrs = n;
-        count_launch();
-        e = cudaLaunchKernelEx(&cfg, gemm_rows_tc_kernel, wmap, amap, p);
+        void* args[] = {&wmap, &amap, &p};
+        if (e == cudaSuccess) e = launch_clustered((const void*)gemm_rows_tc_kernel, dim3(grid), TC_RING_BYTES + 1024, p.splits, st, args);
     }
     const int rc = scratch_free(abuf, st);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_rows_tc", __FILE__, __LINE__);

@@ -7,6 +7,15 @@ namespace pgk {
 
 constexpr int kTcRows = 128;      // weight rows per CTA = MMA M (one TMEM lane per weight row)
 
+// One lane of a converged warp, for MMAs and tensor copies: their operands are warp-uniform registers, and elect.sync tells the
+// compiler that a single lane is active.  What such a thread does between two instructions is serial time -- an MMA of 96 columns
+// takes 56 cycles, one of 256 128, a division by a run-time number 40 ... 60 -- so ring positions are counted, not divided
+// (2000 x 9216 x 2048, the product of seq_gemm_tc.cu: 76 -> 59 us when lane == 0 became elect.sync).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t e;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(e));
+    return e != 0;
+}
 // ---- tcgen05 / TMEM primitives (raw PTX)
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" :: "r"(smem_u32(smem_dst)), "r"(ncols) : "memory");
@@ -59,6 +68,13 @@ __device__ __forceinline__ bool bar_wait(int* error, uint32_t bar, uint32_t pari
     atomicExch(error, 1);
     return false;
 }
+// position in a ring of stages and the parity of its round
+struct RingPos {
+    uint32_t s = 0, round = 0;
+    __device__ __forceinline__ void next(uint32_t stages) {
+        if (++s == stages) { s = 0; round ^= 1u; }
+    }
+};
 // K-major rows of 128 bytes with the 128-byte swizzle, 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3fffu) | ((uint64_t)(1024u >> 4) << 32) | (1ull << 46) | (2ull << 61);

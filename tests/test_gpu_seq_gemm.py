@@ -194,3 +194,79 @@ def test_captured_and_replayed():
         ref, tol = product(A, W[0])
         assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6).all()
         A = A[::-1].copy()
+
+
+# ---------------------------------------------------------------- at most 16 rows: the rounding in the kernel
+@pytest.mark.parametrize("M", [1, 3, 8, 12, 16])
+@pytest.mark.parametrize("N,K", [(128, 64), (130, 72), (7, 200), (2048, 2048), (300, 1000), (96, 8192), (20000, 128)])
+def test_few_rows(M, N, K):
+    A, W = operands(M + N, M + 3, N, K)
+    rows = np.random.default_rng(M).permutation(M + 3)[:M].astype(np.int32)
+    ref, tol = product(A[rows], W[0])
+    lda = K + (1 if M == 3 else 0)                       # rows off the 16-byte grid
+    wide = np.zeros((M + 3, lda), np.float32)
+    wide[:, :K] = A
+    a, w, r = gk.from_numpy(wide), dev_w(W[0]), gk.from_numpy(rows)
+    c = gk.from_numpy(np.full((M, N + 1), 7.0, np.float32))
+    if M <= 8:
+        api.gemm_few_rows_f32(a.device_ptr, lda, r.device_ptr, w.device_ptr, 2, 0, c.device_ptr, N + 1, M, N, K, None, min(M, max(1, 40960 // K)), 0, 1.0,
+                              0.0, None)
+    else:
+        api.gemm_rows_f32(a.device_ptr, lda, r.device_ptr, w.device_ptr, 2, 0, c.device_ptr, N + 1, M, N, K, None, 1, M, 0, 1.0, 0.0, None)
+    out = c.to_numpy()
+    assert (np.abs(out[:, :N] - ref) <= tol + 1e-6).all()
+    assert (out[:, N:] == 7.0).all()
+    no_wait_error()
+
+
+@pytest.mark.parametrize("groups,per", [([0], 1), ([2, 0, -1, 2, 4], 1), ([-1, -1], 1), ([3, 1], 4), (list(range(5)) * 9, 1)])
+@pytest.mark.parametrize("epi", [0, 1, 6])
+def test_few_rows_with_their_own_matrices(groups, per, epi):
+    E, N, K, M = 5, 140, 136, len(groups) * per
+    A, W = operands(M, M, N, K, E)
+    grp = np.repeat(groups, per).astype(np.int32)
+    cols = N // 2 if epi == 1 else N
+    a, w, g = gk.from_numpy(A), dev_w(W), gk.from_numpy(grp)
+    c = gk.from_numpy(np.full((M, cols), 7.0, np.float32))
+    api.gemm_few_rows_f32(a.device_ptr, K, None, w.device_ptr, 2, N * K, c.device_ptr, cols, M, N, K, g.device_ptr, per, epi, 1.0, 0.0, None)
+    out = c.to_numpy()
+    for m in range(M):
+        if grp[m] < 0:
+            assert (out[m] == 7.0).all()
+            continue
+        z, tol = product(A[m:m + 1], W[grp[m]])
+        z, tol = z[0], tol[0]
+        if epi == 1:
+            u = z[1::2]
+            z = z[0::2] * sigmoid(z[0::2]) * u
+            tol = 2.0 * (1.0 + np.abs(u) + np.abs(z)) * np.maximum(tol[0::2], tol[1::2])
+        if epi == 6:
+            tol = 2.0 * (np.maximum(z, 0) + tol) * tol
+            z = np.maximum(z, 0) ** 2
+        assert (np.abs(out[m] - z) <= tol + 1e-6).all()
+    no_wait_error()
+
+
+@pytest.mark.parametrize("M", [1, 8])
+@pytest.mark.parametrize("epi", [0, 4, 10])
+def test_few_rows_batches(M, epi):
+    H, N, K = 6, 200, 72
+    A, W = operands(M, M, N, H * K)
+    W = bf16(np.random.default_rng(1).standard_normal((H, N, K)).astype(np.float32) / np.sqrt(K))
+    old = np.random.default_rng(2).standard_normal((M, H * N)).astype(np.float32)
+    gate = np.random.default_rng(3).standard_normal((M, H * N)).astype(np.float32)
+    cs = np.random.default_rng(4).standard_normal(N).astype(np.float32)
+    a, w, c, g, s = gk.from_numpy(A), dev_w(W), gk.from_numpy(old), gk.from_numpy(gate), gk.from_numpy(cs)
+    aux = (g.device_ptr, 0, None, H * N, 0) if epi == 10 else (None, 0, None, 0, 0)
+    api.gemm_seq_f32(a.device_ptr, H * K, K, w.device_ptr, 2, N * K, c.device_ptr, H * N, N, M, N, K, H, epi, 0.0, 0.0, s.device_ptr, aux[0], aux[1],
+                     aux[2], aux[3], aux[4], M, None)
+    out = c.to_numpy()
+    for h in range(H):
+        z, tol = product(A[:, h * K:(h + 1) * K], W[h])
+        sl = slice(h * N, (h + 1) * N)
+        if epi == 4:
+            z, tol = old[:, sl] + cs * z, tol * np.abs(cs)
+        if epi == 10:
+            z = z * sigmoid(gate[:, sl])
+        assert (np.abs(out[:, sl] - z) <= tol + 1e-6).all()
+    no_wait_error()
