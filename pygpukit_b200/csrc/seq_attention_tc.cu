@@ -19,9 +19,9 @@
 //   * heads of 128: 113 KB of shared memory and 256 TMEM columns, two blocks per SM hide each other's chains; ten warps leave
 //     96 registers a thread; the forms of the score are template parameters, since a tile's straight-line code is long enough
 //     for instruction fetch to show.
-// Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 240 us; 16 heads over latent rows
-// of 576 / 512 5097 -> 570 us.  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
-// 128; two terms per weight instead of three would give 2e-6).
+// Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 232 us; 16 heads over latent rows
+// of 576 / 512 5097 -> 494 us.  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
+// 128).
 #include "seq_attention.cuh"
 #include "tc_common.cuh"
 #include "tma.cuh"
@@ -173,32 +173,30 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
         // ---------------- copies
         int k = 0;                                        // slots issued
         bool ok = true;
-        if (p.bp) {                                       // TMA: lane l fetches positions l bp ... of a tile
+        if (p.bp) {                                       // TMA: piece l is positions l bp ... of a tile
             const int pieces = AK / p.bp;
             uint32_t phase = 0;
-            int c1[2] = {0, 0}, c2[2] = {-1, -1};         // row in the page, page row: of tiles i and i + 1 by turns
+            // lane l: the cache row of tile ti's piece l, and how many pieces there are (tiles i and i + 1 by turns)
+            int row0 = 0, row1 = 0, have0 = 0, have1 = 0;
             auto where = [&](int ti, int u) {
                 const bool early = ti < nkept;
-                const int j = (early ? ti * AK : jal + (ti - nkept) * AK) + lane * p.bp, jmax = early ? kept - 1 : jhi;
-                int row = -1, at = 0;
+                const int j0 = early ? ti * AK : jal + (ti - nkept) * AK, j = j0 + lane * p.bp, jmax = early ? kept - 1 : jhi;
+                int row = 0;
                 if (lane < pieces && j <= jmax) {
                     const int pg = j / a.PS;
-                    at = j - pg * a.PS;
-                    row = a.table[(size_t)slot * a.max_pages + pg] * a.G + g;
+                    row = (a.table[(size_t)slot * a.max_pages + pg] * a.G + g) * a.PS + j - pg * a.PS;
                 }
-                if (u) { c1[1] = at; c2[1] = row; } else { c1[0] = at; c2[0] = row; }
+                const int have = __popc(__ballot_sync(0xffffffffu, lane < pieces && j <= jmax));
+                if (u) { row1 = row; have1 = have; } else { row0 = row; have0 = have; }
             };
+            // every lane waits for the slot and fetches its piece at once: the ring is short, its round trip is what counts
             auto issue = [&](const CUtensorMap* map, int c, int u, bool pad, bool edge) {
-                const uint32_t sl = (uint32_t)(k & (A_RING - 1)), dst = ring + sl * A_CHUNK;
-                ok = ok && __all_sync(0xffffffffu, bar_wait(err, empty_bar + 8u * sl, (uint32_t)(((k / A_RING) & 1) ^ 1)));
-                if (ok) {
-                    const uint32_t bar = edge ? land_bar : full_bar + 8u * sl;
-                    const int row = u ? c2[1] : c2[0], at = u ? c1[1] : c1[0];
-                    const unsigned have = __ballot_sync(0xffffffffu, !pad && row >= 0);
-                    if (lane == 0) mbar_expect_tx(bar, (uint32_t)(__popc(have) * p.bp) * 128u);
-                    __syncwarp();
-                    if ((have >> lane) & 1) tma_load_3d(dst + (uint32_t)(lane * p.bp) * 128u, map, c * 64, at, row, bar);
-                }
+                const uint32_t sl = (uint32_t)(k & (A_RING - 1)), dst = ring + sl * A_CHUNK + (uint32_t)(lane * p.bp) * 128u;
+                const uint32_t bar = edge ? land_bar : full_bar + 8u * sl;
+                const int have = pad ? 0 : (u ? have1 : have0), row = u ? row1 : row0;
+                ok = ok && bar_wait(err, empty_bar + 8u * sl, (uint32_t)(((k / A_RING) & 1) ^ 1));
+                if (ok && lane < have) tma_load_2d(dst, map, c * 64, row, bar);
+                if (ok && lane == 0) mbar_expect_tx(bar, (uint32_t)(have * p.bp) * 128u);
                 ++k;
             };
             if (n > 0) {
@@ -219,7 +217,8 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                     issue(&vmap, c, u, false, edge);
                     issue(&vmap, c + 1, u, (c + 1) * 64 >= Dv, edge);
                     if (!edge) continue;
-                    ok = ok && __all_sync(0xffffffffu, bar_wait(err, land_bar, phase));
+                    __syncwarp();
+                    bar_wait(err, land_bar, phase);
                     phase ^= 1u;
                     const uint32_t pair = ring + (uint32_t)((k - 2) & (A_RING - 1)) * A_CHUNK;
                     for (int r = lane >> 3; r < AK; r += 4) {
@@ -296,7 +295,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
         }
     } else if (warp == A_SOFT + 1) {
         // ---------------- MMAs
-        if (lane == 0) {
+        if (elect_one()) {
             constexpr uint32_t id_s = umma_idesc_bf16(AN), id_o = umma_idesc_bf16_mn(AN);
             int k = 0;
             bool ok = true;
@@ -621,11 +620,9 @@ int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served
     int bp = a.PS & -a.PS;
     if (bp > AK) bp = AK;
     if (bp >= 8 && tma_encode_fn()) {
-        const uint64_t rows = (uint64_t)a.G << 22;        // page rows: the table names only those that exist
-        const uint64_t kd[3] = {(uint64_t)a.D, (uint64_t)a.PS, rows}, ks[2] = {(uint64_t)a.kld * 2, (uint64_t)a.PS * a.kld * 2};
-        const uint64_t vd[3] = {(uint64_t)a.Dv, (uint64_t)a.PS, rows}, vs[2] = {(uint64_t)a.vld * 2, (uint64_t)a.PS * a.vld * 2};
-        const uint32_t box[3] = {64, (uint32_t)bp, 1};
-        if (tma_map_bf16_3d(&kmap, a.kc, kd, ks, box) && tma_map_bf16_3d(&vmap, a.vc, vd, vs, box)) p.bp = bp;
+        const uint64_t rows = 1ull << 31;                 // cache rows: the table names only pages that exist
+        if (tma_map_bf16_2d(&kmap, a.kc, (uint64_t)a.D, rows, (uint64_t)a.kld * 2, 64, (uint32_t)bp) &&
+            tma_map_bf16_2d(&vmap, a.vc, (uint64_t)a.Dv, rows, (uint64_t)a.vld * 2, 64, (uint32_t)bp)) p.bp = bp;
     }
     *served = true;
     switch ((a.cap > 0.f ? 1 : 0) + (a.slopes2 ? 4 : (a.slopes ? 2 : 0)) + (a.prob ? 6 : 0)) {
