@@ -523,7 +523,8 @@ int pgk_seq_mixer_prep(float* proj, int ld, int tokens, int heads, int kv_heads,
  * into that many slices over grid.z; their partial (max, sum, P.V) records go through workspace
  * [rows][heads][splits][vdim + 2] and the block that arrives last at the tile's ticket (tickets [n_tiles x head blocks],
  * zero between launches) folds them.  single_query != 0 promises one query per tile (decoding) and selects the kernel
- * without shared-memory K/V tiles: every warp takes 32 keys at a time for up to pgk_seq_decode_heads_per_block heads. */
+ * without shared-memory K/V tiles: every warp takes 32 keys at a time for up to pgk_seq_decode_heads_per_block heads;
+ * 2: the tensor-core kernel instead, where it can serve (a bfloat16 cache whose rows it can fetch). */
 int pgk_seq_attention(const float* proj, int ld, int q_off, int gate_off, float* out, int ldo, const void* k_cache,
                       const void* v_cache, int cache_dtype, const int32_t* table, int max_pages, int page_size,
                       const int32_t* tiles, int n_tiles, const float* slopes, int heads, int kv_heads, int dim, int vdim,

@@ -1046,7 +1046,7 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
     a.scale = scale; a.cap = softcap; a.splits = splits; a.ws = workspace; a.tickets = tickets;
     a.pool = pool; a.pool_rows = pool_rows; a.pk = k_pool; a.pv = v_pool; a.o_inv_freq = out_inv_freq; a.o_pairs = out_pairs;
     PGK_REQUIRE(!a.valias || pool == 0, "seq_attention failed: pooled blocks keep their values in an array of their own");
-    if (single_query)       // every tile holds one query: the decoding kernel
+    if (single_query && single_query != 2)  // every tile holds one query: the decoding kernel (2: the tensor cores where they can serve)
         return cache_dtype == 2 ? launch_attn_decode_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
                                 : launch_attn_decode_nv<float>(a, n_tiles, (cudaStream_t)stream);
     if (cache_dtype == 2 && !extended(a)) {      // the tensor cores serve what they can fetch; the kernel below the rest
@@ -1054,6 +1054,9 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
         if (const int rc = seq_attention_tc(a, n_tiles, (cudaStream_t)stream, &served)) return rc;
         if (served) return 0;
     }
+    if (single_query)
+        return cache_dtype == 2 ? launch_attn_decode_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
+                                : launch_attn_decode_nv<float>(a, n_tiles, (cudaStream_t)stream);
     return cache_dtype == 2 ? launch_attn_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
                             : launch_attn_nv<float>(a, n_tiles, (cudaStream_t)stream);
 }

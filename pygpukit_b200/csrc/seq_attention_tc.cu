@@ -19,8 +19,12 @@
 //   * heads of 128: 113 KB of shared memory and 256 TMEM columns, two blocks per SM hide each other's chains; ten warps leave
 //     96 registers a thread; the forms of the score are template parameters, since a tile's straight-line code is long enough
 //     for instruction fetch to show.
-// Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 232 us; 16 heads over latent rows
-// of 576 / 512 5097 -> 494 us.  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
+//   * the copies start beside the queries' conversion, an edge tile's zeros are written while the next pair of chunks arrives, the
+//     outputs leave four rows at a time in a short loop (code that runs once per block costs its fetch), and rows that no query
+//     has are left out: what decoding, one tile per block, spends its time on.
+// Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 191 us; 16 heads over latent rows
+// of 576 / 512 5097 -> 471 us.  Decoding, 8 requests: latent rows over 2000 keys 129 -> 50 us, 16 / 4
+// heads of 128 over 1024 65 -> 24 us.  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
 // 128).
 #include "seq_attention.cuh"
 #include "tc_common.cuh"
@@ -41,7 +45,7 @@ constexpr uint32_t A_CHUNK = AK * 128;     // 128 keys x 64 elements
 constexpr uint32_t A_QCHUNK = AN * 128;
 constexpr uint32_t A_PTERM = AK * AR * 2;
 constexpr uint32_t A_PBYTES = 3 * A_PTERM;
-constexpr uint32_t A_TAIL = 128 + 512 + 256;         // barriers and TMEM address, row maxima, what a row knows
+constexpr uint32_t A_TAIL = 128 + 512 + 256 + 128;   // barriers and TMEM address, row maxima, what a row knows, its output
 constexpr float LOG2E = 1.4426950408889634f;
 constexpr float LAZY = 8.f;
 
@@ -100,11 +104,12 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t q_s = smem_u32(smem), p_s = q_s + (uint32_t)p.nd * A_QCHUNK, ring = p_s + A_PBYTES, tail = ring + A_RING * A_CHUNK;
     const uint32_t full_bar = tail, empty_bar = tail + 32, s_full = tail + 64, s_read = tail + 72, p_ready = tail + 80, pv_done = tail + 88,
-                   land_bar = tail + 96;
+                   land_bar = tail + 96;                  // and at + 112: pairs of an edge tile by turns
     unsigned char* tail_p = smem + (tail - q_s);
     uint32_t* tmem_slot = (uint32_t*)(tail_p + 104);
     float* wmax = (float*)(tail_p + 128);                // [32 rows][4]
     float2* rowi = (float2*)(tail_p + 640);              // [32 rows] position, slope
+    int* rowo = (int*)(tail_p + 896);                    // [32 rows] query << 16 | head of the row, -1: nobody's
     if (q_s & 1023u) {                                   // the layout relies on it (uniform over the grid)
         if (tid == 0) atomicExch(&g_attn_wait_error, 2);
         return;
@@ -114,52 +119,20 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     if (tid == 0) {
         uint64_t* b = (uint64_t*)tail_p;
         for (int s = 0; s < A_RING; ++s) { mbar_init(b + s, 1); mbar_init(b + A_RING + s, 1); }
-        mbar_init(b + 8, 1); mbar_init(b + 9, A_SOFT); mbar_init(b + 10, A_SOFT); mbar_init(b + 11, 1); mbar_init(b + 12, 2);
+        mbar_init(b + 8, 1); mbar_init(b + 9, A_SOFT); mbar_init(b + 10, A_SOFT); mbar_init(b + 11, 1); mbar_init(b + 12, 2); mbar_init(b + 14, 2);
         mbar_fence_init();
     }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
     griddep_wait();
     const int4 tile = a.tiles[blockIdx.x];
     const int t0 = tile.x, nq = tile.y, slot = tile.z, pos0 = tile.w, D = a.D, Dv = a.Dv, HB = a.HB;
     const int rep = a.H / a.G, hsplit = (rep + HB - 1) / HB;
     const int g = blockIdx.y / hsplit, hpart = blockIdx.y - g * hsplit;
     const int hb0 = g * rep + hpart * HB, nh = min(HB, rep - hpart * HB);
-
-    if (tid < AR) {
-        const int qi = tid / HB, hh = tid - qi * HB;
-        rowi[tid] = make_float2((float)(pos0 + qi), SLOPE && qi < nq && hh < nh ? a.slopes[hb0 + hh] : 0.f);
-    }
-    // queries: rows 32 t + r of chunk c hold term t of row r's elements 64 c ... 64 c + 63
-    for (int i = tid; i < AR * p.nd * 8; i += A_THREADS) {
-        const int r = i / (p.nd * 8), k8 = i - r * p.nd * 8, d = k8 * 8, qi = r / HB, hh = r - qi * HB;
-        float x[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (qi < nq && hh < nh && d < D) {
-            const float* src = a.proj + (size_t)(t0 + qi) * a.ld + a.q_off + (size_t)(hb0 + hh) * D + d;
-            if (p.qvec) {
-                *(float4*)&x[0] = *(const float4*)src;
-                *(float4*)&x[4] = *(const float4*)(src + 4);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) x[e] = src[e];
-            }
-        }
-#pragma unroll
-        for (int t = 0; t < 3; ++t) {                    // three terms that together hold all 24 bits
-            uint32_t v[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                v[e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
-                x[2 * e] -= bf16lo(v[e]);
-                x[2 * e + 1] -= bf16hi(v[e]);
-            }
-            const int row = AR * t + r;
-            sts128(q_s + (uint32_t)(k8 >> 3) * A_QCHUNK + (uint32_t)row * 128u + (uint32_t)(((k8 & 7) ^ (row & 7)) << 4), v);
-        }
-    }
-    fence_proxy_async();
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const int live = min(AR, nq * HB);                   // rows that a query has
 
     // the block's key tiles: the kept first positions below the window, then [jlo, jhi] from a copy's boundary on
     const int jlo = first_key(a, pos0), jhi = pos0 + nq - 1, jal = p.bp ? jlo & ~(p.bp - 1) : jlo;
@@ -169,6 +142,57 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     const int nv2 = 2 * p.ndv;
     int* const err = &g_attn_wait_error;
 
+    if (warp != A_SOFT) {
+        // ---------------- queries, beside the first copies: rows 32 t + r of chunk c hold term t of row r's elements 64 c ... 64 c + 63
+        if (tid < AR) {
+            const int qi = tid / HB, hh = tid - qi * HB;
+            const bool has = qi < nq && hh < nh;
+            rowi[tid] = make_float2((float)(pos0 + qi), SLOPE && has ? a.slopes[hb0 + hh] : 0.f);
+            rowo[tid] = has ? qi << 16 | hh : -1;
+        }
+        if (warp < A_SOFT) {
+            const int items = AR * p.nd * 8;
+            auto fetch = [&](int i, float (&x)[8]) {
+                const int r = i / (p.nd * 8), d = (i - r * p.nd * 8) * 8, qi = r / HB, hh = r - qi * HB;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = 0.f;
+                if (i < items && qi < nq && hh < nh && d < D) {
+                    const float* src = a.proj + (size_t)(t0 + qi) * a.ld + a.q_off + (size_t)(hb0 + hh) * D + d;
+                    if (p.qvec) {
+                        *(float4*)&x[0] = *(const float4*)src;
+                        *(float4*)&x[4] = *(const float4*)(src + 4);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) x[e] = src[e];
+                    }
+                }
+            };
+            float next[8];
+            fetch(tid, next);
+#pragma unroll 1
+            for (int i = tid; i < items; i += A_SOFT * 32) {
+                float x[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) x[e] = next[e];
+                fetch(i + A_SOFT * 32, next);
+                const int r = i / (p.nd * 8), k8 = i - r * p.nd * 8;
+#pragma unroll
+                for (int t = 0; t < 3; ++t) {            // three terms that together hold all 24 bits
+                    uint32_t v[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        v[e] = pack_bf16x2(x[2 * e], x[2 * e + 1]);
+                        x[2 * e] -= bf16lo(v[e]);
+                        x[2 * e + 1] -= bf16hi(v[e]);
+                    }
+                    const int row = AR * t + r;
+                    sts128(q_s + (uint32_t)(k8 >> 3) * A_QCHUNK + (uint32_t)row * 128u + (uint32_t)(((k8 & 7) ^ (row & 7)) << 4), v);
+                }
+            }
+            fence_proxy_async();
+        }
+        asm volatile("bar.sync 3, %0;" :: "n"((A_SOFT + 1) * 32) : "memory");
+    }
     if (warp == A_SOFT) {
         // ---------------- copies
         int k = 0;                                        // slots issued
@@ -189,10 +213,29 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                 const int have = __popc(__ballot_sync(0xffffffffu, lane < pieces && j <= jmax));
                 if (u) { row1 = row; have1 = have; } else { row0 = row; have0 = have; }
             };
+            // the pair of slots from `at` on has arrived: rows outside the run become zeros, then the MMAs may have it
+            auto clear = [&](int at, int below, int above) {
+                __syncwarp();
+                bar_wait(err, land_bar + 8u * (uint32_t)(at & 2), (phase >> (at & 2)) & 1u);
+                phase ^= 1u << (at & 2);
+                const uint32_t pair = ring + (uint32_t)(at & (A_RING - 1)) * A_CHUNK;
+                for (int r = lane >> 3; r < AK; r += 4) {
+                    if (r >= below && r < above) continue;
+                    const uint32_t z[4] = {0u, 0u, 0u, 0u};
+                    sts128(pair + (uint32_t)r * 128u + (uint32_t)(lane & 7) * 16u, z);
+                    sts128(pair + A_CHUNK + (uint32_t)r * 128u + (uint32_t)(lane & 7) * 16u, z);
+                }
+                fence_proxy_async();
+                __syncwarp();
+                if (lane == 0) {
+                    mbar_arrive((uint64_t*)(tail_p + 8 * (at & (A_RING - 1))));
+                    mbar_arrive((uint64_t*)(tail_p + 8 * ((at + 1) & (A_RING - 1))));
+                }
+            };
             // every lane waits for the slot and fetches its piece at once: the ring is short, its round trip is what counts
             auto issue = [&](const CUtensorMap* map, int c, int u, bool pad, bool edge) {
                 const uint32_t sl = (uint32_t)(k & (A_RING - 1)), dst = ring + sl * A_CHUNK + (uint32_t)(lane * p.bp) * 128u;
-                const uint32_t bar = edge ? land_bar : full_bar + 8u * sl;
+                const uint32_t bar = edge ? land_bar + 8u * (sl & 2u) : full_bar + 8u * sl;
                 const int have = pad ? 0 : (u ? have1 : have0), row = u ? row1 : row0;
                 ok = ok && bar_wait(err, empty_bar + 8u * sl, (uint32_t)(((k / A_RING) & 1) ^ 1));
                 if (ok && lane < have) tma_load_2d(dst, map, c * 64, row, bar);
@@ -217,22 +260,8 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                     issue(&vmap, c, u, false, edge);
                     issue(&vmap, c + 1, u, (c + 1) * 64 >= Dv, edge);
                     if (!edge) continue;
-                    __syncwarp();
-                    bar_wait(err, land_bar, phase);
-                    phase ^= 1u;
-                    const uint32_t pair = ring + (uint32_t)((k - 2) & (A_RING - 1)) * A_CHUNK;
-                    for (int r = lane >> 3; r < AK; r += 4) {
-                        if (r >= below && r < above) continue;
-                        const uint32_t z[4] = {0u, 0u, 0u, 0u};
-                        sts128(pair + (uint32_t)r * 128u + (uint32_t)(lane & 7) * 16u, z);
-                        sts128(pair + A_CHUNK + (uint32_t)r * 128u + (uint32_t)(lane & 7) * 16u, z);
-                    }
-                    fence_proxy_async();
-                    __syncwarp();
-                    if (lane == 0) {
-                        mbar_arrive((uint64_t*)(tail_p + 8 * ((k - 2) & (A_RING - 1))));
-                        mbar_arrive((uint64_t*)(tail_p + 8 * ((k - 1) & (A_RING - 1))));
-                    }
+                    if (c) clear(k - 4, below, above);    // a pair is cleared while the next one arrives
+                    if (c + 2 >= nv2) clear(k - 2, below, above);
                 }
             }
             if (!ok)                                      // do not leave with copies in flight
@@ -368,6 +397,16 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
             l[r] = ((PROB && blockIdx.z == 0) || has_sink) && quad == 0 && lane == 0 ? 1.f : 0.f;
         }
         bool ok = true;
+        if (r0 >= live) {                                 // nobody's rows (decoding): keep the barriers' count
+            for (int i = 0; i < n; ++i) {
+                ok = ok && bar_wait(err, s_full, (uint32_t)(i & 1));
+                __syncwarp();
+                if (lane == 0) mbar_arrive((uint64_t*)(tail_p + 72));
+                if (i > 0) ok = ok && bar_wait(err, pv_done, (uint32_t)((i - 1) & 1));
+                __syncwarp();
+                if (lane == 0) mbar_arrive((uint64_t*)(tail_p + 80));
+            }
+        } else
         for (int i = 0; i < n; ++i) {
             const int ti = tend - 1 - i;
             const bool early = ti < nkept;
@@ -498,38 +537,48 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                 }
             }
             const float inv_r = a.splits > 1 ? 1.f : (l_r > 0.f ? 1.f / l_r : 0.f) * a.out_mult;
-            for (int c = 0; c < p.ndv; ++c) {
-                const int dv = c * 128 + quad * 32 + lane;
-                float o[16], gz[16];
-                int qi = r0 / HB, hh = r0 - qi * HB;
-                if (a.gate && a.splits == 1) {            // all loads at once
+            // four rows at a time and only a query's: what runs once costs its fetch, 16 rows in a row 7000 cycles per 128 elements
+            const int steps = 4 * p.ndv;
+            const bool gated = a.gate && a.splits == 1;
+            float gz[4], go[4] = {0.f, 0.f, 0.f, 0.f};
+            auto gates = [&](int u) {
+                const int dv = (u >> 2) * 128 + quad * 32 + lane, rr = r0 + (u & 3) * 4;
 #pragma unroll
-                    for (int r = 0; r < 16; ++r) {
-                        gz[r] = dv < Dv && qi < nq && hh < nh ? gate_logit(a, (size_t)(t0 + qi), hb0 + hh, dv) : 0.f;
-                        if (++hh == HB) { hh = 0; ++qi; }
-                    }
+                for (int e = 0; e < 4; ++e) {
+                    const int ro = rowo[rr + e];
+                    go[e] = u < steps && dv < Dv && ro >= 0 ? gate_logit(a, (size_t)(t0 + (ro >> 16)), hb0 + (ro & 0xffff), dv) : 0.f;
                 }
+            };
+            if (gated) gates(0);
+#pragma unroll 1
+            for (int u = 0; u < steps; ++u) {
+                const int rr = r0 + (u & 3) * 4, dv = (u >> 2) * 128 + quad * 32 + lane;
+                float o[4] = {0.f, 0.f, 0.f, 0.f}, x[4], y[4];
+                if (gated) {                              // the next step's loads go out before this one's use
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) gz[e] = go[e];
+                    gates(u + 1);
+                }
+                if (rr >= live) continue;
                 if (n > 0) {
-                    const uint32_t at = lanes + AN + (uint32_t)c * AN + (uint32_t)r0;
-                    tmem_sum3(at, at + AR, at + 2 * AR, o);
-                } else {
+                    const uint32_t at = lanes + AN + (uint32_t)(u >> 2) * AN + (uint32_t)rr;
+                    tmem_ld4x3(at, at + AR, at + 2 * AR, o, x, y);
 #pragma unroll
-                    for (int r = 0; r < 16; ++r) o[r] = 0.f;
+                    for (int e = 0; e < 4; ++e) o[e] += x[e] + y[e];
                 }
-                qi = r0 / HB; hh = r0 - qi * HB;
 #pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    float x = o[r] * __shfl_sync(0xffffffffu, inv_r, r);
-                    if (a.gate && a.splits == 1) x *= 1.f / (1.f + expf(-gz[r]));
-                    if (dv < Dv && qi < nq && hh < nh) {
-                        const size_t t = t0 + qi;
-                        const int h = hb0 + hh;
-                        if (a.splits > 1) a.ws[((t * a.H + h) * a.splits + blockIdx.z) * (Dv + 2) + 2 + dv] = x;
-                        else a.out[t * a.ldo + (size_t)h * Dv + dv] = x;
+                for (int e = 0; e < 4; ++e) {
+                    float v = o[e] * __shfl_sync(0xffffffffu, inv_r, rr - r0 + e);
+                    const int ro = rowo[rr + e];
+                    if (dv >= Dv || ro < 0) continue;
+                    const size_t t = t0 + (ro >> 16);
+                    const int h = hb0 + (ro & 0xffff);
+                    if (a.splits > 1) a.ws[((t * a.H + h) * a.splits + blockIdx.z) * (Dv + 2) + 2 + dv] = v;
+                    else {
+                        if (gated) v *= 1.f / (1.f + expf(-gz[e]));
+                        a.out[t * a.ldo + (size_t)h * Dv + dv] = v;
                     }
-                    if (++hh == HB) { hh = 0; ++qi; }
                 }
-                __syncwarp();
             }
         }
     }
@@ -574,17 +623,42 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
             if (lane + 32 * u < a.splits) wsl[r * 64 + lane + 32 * u] = e[u] * inv;
     }
     __syncthreads();
-    for (int i = tid; i < AR * Dv; i += A_THREADS) {
-        const int r = i / Dv, dv = i - r * Dv, qi = r / HB, hh = r - qi * HB;
-        if (qi >= nq || hh >= nh) continue;
-        const size_t t = t0 + qi;
-        const int h = hb0 + hh;
-        const float* rec = a.ws + ((t * a.H + h) * a.splits) * (Dv + 2) + 2 + dv;
-        float o = 0.f;
-#pragma unroll 8
-        for (int sp = 0; sp < a.splits; ++sp) o = fmaf(wsl[r * 64 + sp], __ldcg(rec + (size_t)sp * (Dv + 2)), o);
-        if (a.gate) o *= 1.f / (1.f + expf(-gate_logit(a, t, h, dv)));
-        a.out[t * a.ldo + (size_t)h * Dv + dv] = o * a.out_mult;
+    // pairs of elements (records start on 8 bytes), four per thread and round: one at a time, the loads' latency is all it does
+    const int half_dv = Dv / 2, total = live * half_dv;
+    for (int i0 = tid; i0 < total; i0 += 4 * A_THREADS) {
+        const float2* src[4];
+        float2 o[4];
+        int row[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = i0 + q * A_THREADS, r = i / half_dv, ro = i < total ? rowo[r] : -1;
+            row[q] = ro >= 0 ? r : -1;
+            o[q] = make_float2(0.f, 0.f);
+            src[q] = (const float2*)(a.ws + ((size_t)(t0 + (max(ro, 0) >> 16)) * a.H + hb0 + (max(ro, 0) & 0xffff)) * a.splits * (Dv + 2) + 2) +
+                     (ro >= 0 ? i - r * half_dv : 0);
+        }
+#pragma unroll 4
+        for (int sp = 0; sp < a.splits; ++sp)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const float w = wsl[max(row[q], 0) * 64 + sp];
+                const float2 v = __ldcg(src[q] + (size_t)sp * (half_dv + 1));
+                o[q].x = fmaf(w, v.x, o[q].x);
+                o[q].y = fmaf(w, v.y, o[q].y);
+            }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (row[q] < 0) continue;
+            const int ro = rowo[row[q]], dv = 2 * (i0 + q * A_THREADS - row[q] * half_dv), h = hb0 + (ro & 0xffff);
+            const size_t t = t0 + (ro >> 16);
+            float* dst = a.out + t * a.ldo + (size_t)h * Dv + dv;
+            if (a.gate) {
+                o[q].x *= 1.f / (1.f + expf(-gate_logit(a, t, h, dv)));
+                o[q].y *= 1.f / (1.f + expf(-gate_logit(a, t, h, dv + 1)));
+            }
+            dst[0] = o[q].x * a.out_mult;
+            dst[1] = o[q].y * a.out_mult;
+        }
     }
 }
 
@@ -606,6 +680,7 @@ int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served
     *served = false;
     // copies of 16 bytes from rows of the cache; at most 512 value elements (TMEM) and 704 key elements (shared memory)
     if (a.D % 8 || a.Dv % 8 || a.kld % 8 || a.vld % 8 || (uintptr_t)a.kc % 16 || (uintptr_t)a.vc % 16 || a.Dv > 512 || a.HB > AR) return 0;
+    if (a.splits > 1 && (uintptr_t)a.ws % 8) return 0;    // the fold reads pairs
     TcAttnArgs p{};
     p.a = a;
     p.nd = (a.D + 63) / 64;

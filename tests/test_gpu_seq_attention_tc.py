@@ -29,7 +29,7 @@ class Case:
     """portions [(first position, tokens), ...] of sequences whose earlier keys are in the cache"""
 
     def __init__(self, portions, H, G, D, Dv, PS=64, chunk=0, window=0, keep=0, cap=0.0, slopes=0, sinks=False, gate=0, prob=False,
-                 splits=1, alias=False, seed=0, q_gain=1.0):
+                 splits=1, alias=False, seed=0, q_gain=1.0, single=0):
         self.__dict__.update({k: v for k, v in locals().items() if k != "self"})
         rng = np.random.default_rng(seed + H * 100 + D)
         self.scale = D ** -0.5
@@ -54,7 +54,7 @@ class Case:
         qt = int(api.seq_queries_per_tile(self.H, self.G))
         tiles, row = [], 0
         for s, (p, n) in enumerate(self.portions):
-            tiles += [(row + i, min(qt, n - i), s, p + i) for i in range(0, n, qt)]
+            tiles += [(row + i, 1 if self.single else min(qt, n - i), s, p + i) for i in range(0, n, 1 if self.single else qt)]
             row += n
         assert hb * qt <= 32
         up = gk.from_numpy if f32_cache else dev16
@@ -70,7 +70,7 @@ class Case:
                               v.device_ptr, self.D, self.D if self.alias else self.Dv, 0 if f32_cache else 2, t.device_ptr, self.table.shape[1],
                               self.PS, tl.device_ptr, len(tiles), ptr["sl"], ptr["sl2"], ptr["sink"], self.H, self.G, self.D, self.Dv, self.chunk,
                               self.window, self.keep, self.scale, self.cap, 1 if self.prob else 0, ptr["pb"], 0.75, 0, 0, None, None, None, 0,
-                              self.splits, ws.device_ptr, tk.device_ptr, 0, None)
+                              self.splits, ws.device_ptr, tk.device_ptr, self.single, None)
         r = out.to_numpy()
         assert (tk.to_numpy() == 0).all()
         err = C.c_int(7)
@@ -155,6 +155,26 @@ def test_forms(form):
     print(f"form {form}: max {worst_old:.2e} -> {worst_new:.2e}, rms {rms_old:.2e} -> {rms_new:.2e}, top {top:.2f}")
     assert worst_new <= 2 * worst_old + 2 * 2.0 ** -23 * top
     assert rms_new <= 1.5 * rms_old + 2.0 ** -24 * top
+
+
+DECODE = [
+    dict(H=16, G=4, D=128, Dv=128, window=90, gate=1),
+    dict(H=16, G=1, D=576, Dv=512, alias=True, sinks=True),
+    dict(H=8, G=8, D=64, Dv=80, slopes=1, cap=20.0, PS=7),
+    dict(H=40, G=1, D=40, Dv=256, chunk=100, gate=2, PS=16),
+    dict(H=6, G=2, D=100, Dv=128),                               # rows that the copies cannot fetch: the float32 kernel
+]
+
+
+@pytest.mark.parametrize("splits", [1, 2, 8, 64])
+@pytest.mark.parametrize("form", range(len(DECODE)))
+def test_decoding(form, splits):
+    """one query per request, over contexts that end at and beside a tile of keys: the bounds of the portions above"""
+    c = Case([(p, 1) for p in (0, 59, 126, 127, 128, 300, 1030)], splits=splits, single=2, **DECODE[form])
+    ref = c.exact()
+    old, new = c.run(True), c.run(False)
+    top = np.abs(ref).max()
+    assert np.abs(new - ref).max() <= 2 * np.abs(old - ref).max() + 2 * 2.0 ** -23 * top
 
 
 def test_late_maximum():
