@@ -353,6 +353,8 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
 // the tile is done, round the float32 rows into the stages, eight k blocks per fence (a fence also waits for loads in flight).
 // A cluster that shares a tile along k pushes its partial rows to their owners' shared memory, one barrier, and every block
 // finishes its rows.  Measured at 8 rows, against a warp per column pair (gemm_few_rows_kernel): see few_tc_pays.
+// The weights are marked first to leave L2: at the default they push out what the small kernels in between keep reading (norm
+// weights, page tables, rows), which then cost 4 us more each: a decode step of 0.5 GB of weights 598 -> 536 us.
 struct FewArgs {
     GemmArgs g;
     int epi, th, nkb, kper, splits, rpb, avec;
@@ -398,10 +400,11 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         if (elect_one()) {
             RingPos r;
             const uint32_t bytes = (uint32_t)p.th * (TBK * 2);
+            const uint64_t once = l2_evict_first();
             for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
                 if (!bar_wait(&g_tc_wait_error, empty + 8u * r.s, r.round ^ 1u)) break;
                 mbar_expect_tx(full + 8u * r.s, bytes);
-                tma_load_3d(ring + r.s * FEW_STAGE_BYTES, &wmap, kb * TBK, n0, z, full + 8u * r.s);
+                tma_load_3d_hint(ring + r.s * FEW_STAGE_BYTES, &wmap, kb * TBK, n0, z, full + 8u * r.s, once);
             }
         }
         __syncwarp();
