@@ -96,14 +96,16 @@ int pgk_gemv_fp8_swiglu_bf16(const void* A, const void* Wg_nk, const void* Sg, c
 
 /* Decode batch 5..64 on the tensor cores (tcgen05.mma kind::f16, BF16 x BF16 -> F32 in TMEM): same operands
  * and epilogues as pgk_gemv_fp8_bf16_ex; the weights are read ONCE for all M rows, converted exactly to BF16
- * on the way into shared memory, the 128x128 block scale is folded into the activation slab (rounded to BF16
- * where the reference rounds weight*scale, w8a16_gemm.cu:104-339).  Needs 1 <= M <= 64 (rows up to the MMA
+ * on the way into tensor memory, the 128x128 block scale multiplies the float32 sums of its 128 products (the
+ * reference rounds weight*scale to BF16, w8a16_gemm.cu:104-339).  Needs 1 <= M <= 64 (rows up to the MMA
  * width 16/32/64 are zero-filled), K % 128 == 0, N % 128 == 0.  pgk_gemv_fp8_bf16(_ex) dispatch here by
  * themselves for M >= 5 (measured crossover against the CUDA-core slab GEMV; env PGK_TC_MIN_M) when the shape
  * allows (replaces gemv_fp8_bf16_batched, fp8_opt.cuh:220-295, and w8a16_gemm_sm120's mma.sync path). */
 int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void* S, void* C, int M, int K, int N,
                          const void* bias, const void* residual, void* stream);
 
+/* 1 once a wait of the FP8 tensor-core GEMM ran out (its results are then undefined), else 0. */
+int pgk_gemm_fp8_wait_error(int* out);
 /* The same contract with NO CUDA-core work on the weight stream: raw E4M3 tiles by TMA (cp.async.bulk.tensor, 2-D tensor
  * map over the [N,K] matrix, 128-byte swizzle) straight into tcgen05.mma.kind::f8f6f4; the activations are split once
  * (pre-kernel) into two exact E4M3 terms a' = t0 + t1/16 after a per-row power-of-two shift; the 128x128 block scale is

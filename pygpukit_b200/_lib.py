@@ -117,7 +117,7 @@ _SIGS = {
     # token-major models (seq_gemm.cu, seq_attention.cu, seq_layers.cu)
     "pgk_gemm_rows_f32": [vp, i32, vp, vp, i32, C.c_longlong, vp, i32, i32, i32, i32, vp, i32, i32, i32, f32, f32, vp],
     "pgk_gemm_groups_f32": [vp, i32, vp, vp, i32, C.c_longlong, vp, i32, i32, i32, i32, vp, i32, i32, i32, i32, f32, f32, vp],
-    "pgk_gemm_rows_wait_error": [C.POINTER(i32)], "pgk_seq_attention_wait_error": [C.POINTER(i32)],
+    "pgk_gemm_rows_wait_error": [C.POINTER(i32)], "pgk_gemm_fp8_wait_error": [C.POINTER(i32)], "pgk_seq_attention_wait_error": [C.POINTER(i32)],
     "pgk_gemm_few_rows_f32": [vp, i32, vp, vp, i32, C.c_longlong, vp, i32, i32, i32, i32, vp, i32, i32, f32, f32, vp],
     "pgk_embed_rows_f32": [vp, i32, vp, vp, i32, i32, i32, vp],
     "pgk_combine_layernorm_f32": [vp, vp, vp, vp, vp, i32, vp, vp, f32, vp, i32, i32, i32, vp],

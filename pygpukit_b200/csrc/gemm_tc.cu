@@ -1,52 +1,56 @@
-// gemm_tc.cu -- W8A16 skinny GEMM for decode batch 16..64 on the 5th-gen tensor cores (tcgen05 + TMEM).
+// gemm_tc.cu -- W8A16 GEMM for a few dozen rows on the 5th-gen tensor cores (tcgen05 + TMEM + TMA).
 //
-//   C[M,N] = A[M,K] . dequant(B[N,K])^T     B = FP8-E4M3 codes [N,K], S = bf16 [N/128, K/128], 1 <= M <= 64 (used for M >= 5)
+//   C[M,N] = A[M,K] . dequant(B[N,K])^T     B = FP8-E4M3 codes [N,K], S = bf16 [N/128, K/128]
 //
 // replaces gemv_fp8_warp_reduce_vec4_batched_kernel (fp8_opt.cuh:220-295, re-reads the weights M times) and
 // the M >= 16 tensor-core path of pygpukit_w8a16_gemm_sm120 (w8a16_gemm.cu:104-339: dequantise to BF16 in
 // shared memory, mma.sync m16n8k16, unpipelined).
 //
-// Design (DESIGN.md "gemm_fp8_tc"): the problem is still weight-streaming bound (M <= 64 rows share one read
-// of N*K bytes), so the kernel is organised around the HBM stream and hands the arithmetic to tcgen05:
-//   * the GEMM is computed transposed, D^T[n, m] = W[n, :] . A[m, :]: a CTA owns 128 weight rows (the MMA's
-//     M = 128 -> one TMEM lane per weight row) and the batch is the MMA's N (16 / 32 / 64 f32 TMEM columns);
-//     split-K over gridDim.y fills the 148 SMs when N/128 tiles are too few.
-//   * per 128-wide k block (= one FP8 scale block; the 128-row tile lies inside one scale row, so the CTA sees
-//     ONE scale per k block): 16 KB of E4M3 codes stream global -> shared memory with cp.async (a ring of
-//     four raw blocks = 64 KB in flight per SM, requested before the dependency wait), are converted exactly to BF16
-//     (cvt e4m3x2 -> f16x2 -> f32 -> BF16x2 pack; E4M3 fits BF16) and stored to shared memory in the
-//     canonical no-swizzle K-major core-matrix layout; the [M,128] activation slab is multiplied by the block
-//     scale in f32 and split into TWO BF16 terms, hi = bf16(a*s) and lo = bf16(a*s - hi), stored in the same
-//     layout: with exact BF16 weights the two MMAs reproduce the f32 product a*s*w to ~2^-17, i.e. the
-//     FP32-accumulate class of the CUDA-core GEMV (the reference's tensor-core path rounds weight*scale to BF16
-//     once, a 2^-9 step).  The second MMA is free: the kernel is bound by the weight stream, not the tensor pipe.
-//   * one elected thread issues 2 x 8 x tcgen05.mma.kind::f16 (128 x NB x 16, BF16 in, F32 accumulate in TMEM)
-//     per k block from shared-memory descriptors, then tcgen05.commit -> mbarrier releases the stage; two
-//     BF16 operand stages per CTA, one CTA per SM.
-//   * epilogue: tcgen05.ld 32x32b -> registers, [split-K partials folded in split order by the last-arriving
-//     CTA], bias / residual with the reference's rounding points, BF16 store (lanes = consecutive n: coalesced).
+// What bounds it: the weights' way from HBM, and close behind it what an SM does per 128 x 128 block of them: the conversion of
+// 16384 codes and the traffic through its shared memory.  What follows from that:
+//   * the GEMM is computed transposed, D^T[n, m] = W[n, :] . A[m, :]: a block owns 128 weight rows (MMA M, a TMEM lane per row), the
+//     batch is the MMA's N (16 / 32 / 64 columns; more rows take further blocks);
+//   * TMA brings codes and activations as they are (128-byte swizzle) into a ring; eight warps turn the codes into BF16 exactly and
+//     store them to TENSOR MEMORY, from where the MMA takes its A operand: through shared memory the BF16 form would be written
+//     and read once more, 128 KB per block of weights instead of 64, which alone is 1000 cycles against 680 for the HBM stream;
+//   * the block scale multiplies the partial sums of its 128 products in float32 (two accumulators by turns): products are exact and
+//     the activations need no second term that holds their product with the scale;
+//   * the same eight warps add the partial sums of the block before while the tensor cores multiply; MMAs and copies have a warp each;
+//   * a stage holds a block's codes and rows together (rings of their own left too few slots for the rows: 65 -> 72 us);
+//   * two blocks per SM (256 TMEM columns, 100 KB each) hide each other's start and end; K is cut over a cluster that pushes
+//     its partial rows to their owners' shared memory and adds them in the order of the ranks: no work memory.
+// Measured on B200 (us, cp.async and conversion through shared memory -> here), M = 5 / 64: 14336 x 4096 35 / 43 -> 20.7 / 24.5,
+// 4096 x 4096 16.5 / 26.8 -> 10.5 / 13.9, 1024 x 4096 10.9 / 21.3 -> 8.3 / 10.4, 14336 x 14336 103 / 134 -> 55 / 65 (3.7 / 3.2 TB/s).
 #include "common.cuh"
 #include "tc_common.cuh"
+#include "tma.cuh"
 #include "../../include/pgk_b200.h"
 
 namespace pgk {
 
 constexpr int kTcBK = 128;        // k block = FP8 scale block
-constexpr int kTcThreads = 512;    // 16 converter warps (+ one MMA-issuing warp per CTA): the FP8 -> BF16 conversion is CUDA-core work and needs the warps to hide its latencies
-constexpr int kTcMaxKb = 256;     // k blocks per CTA (K <= 32768)
-constexpr int kTcStages = 2;      // BF16 operand stages (tensor-core side)
-// raw FP8 weight blocks / activation slabs in flight per CTA (cp.async rings): as deep as 227 KB of shared memory
-// allows next to the two BF16 operand stages -- the ring depth is what keeps HBM requests in flight while the CTA converts
-__host__ __device__ constexpr int tc_raw_depth(int nb) { return nb <= 16 ? 6 : (nb <= 32 ? 5 : 3); }
+constexpr int kTcMaxKb = 256;     // k blocks (K <= 32768)
+constexpr int kTcMaxTiles = 8192;
 
-struct TcParams {
-    const uint16_t* A; const uint8_t* B; const uint16_t* S; uint16_t* C;
+namespace {
+
+constexpr int F_WARPS = 8;                        // conversion, partial sums, output; one more for the copies, one for the MMAs
+constexpr int F_THREADS = (F_WARPS + 2) * 32;
+constexpr uint32_t F_W_BYTES = kTcRows * kTcBK;   // codes of a stage
+__host__ __device__ constexpr int f_stages(int nb) { return nb <= 16 ? 5 : (nb <= 32 ? 4 : 3); }
+__host__ __device__ constexpr uint32_t f_stage_bytes(int nb) { return F_W_BYTES + (uint32_t)nb * kTcBK * 2; }
+__host__ __device__ constexpr size_t f_smem(int nb) { return (size_t)f_stages(nb) * f_stage_bytes(nb) + 1024; }
+
+struct F8TcParams {
+    const uint16_t* S; uint16_t* C;
     const uint16_t* bias; const uint16_t* residual;
-    int M, K, N, splits;
-    float* ws; unsigned* counters;
+    int M, K, N, splits, kper, once;              // once: nobody reads the weights again
 };
 
-// four e4m3 codes (one 32-bit word) -> four bf16 (two packed words), exact
+__device__ int g_f8tc_wait_error = 0;
+
+// four e4m3 codes (one 32-bit word) -> four bf16 (two packed words), exact.  (The bits moved by integer instructions and a product
+// with 2^120 for the bias are slower, 55 -> 63 us at 14336 x 14336; with no conversion at all it would be 43.)
 __device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
     const uint32_t h0 = e4m3x2_to_f16x2_lo(w), h1 = e4m3x2_to_f16x2_hi(w);
     const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
@@ -56,288 +60,282 @@ __device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t& lo, uint3
 }
 
 template <int NB>
-__global__ void __launch_bounds__(kTcThreads + 32, 1)
-gemm_fp8_tc_kernel(TcParams p) {
-    constexpr int NW = kTcThreads / 32;
-    constexpr int kTcRaw = tc_raw_depth(NB);
-    constexpr int WI = 32 / NW;                   // weight items per thread per k block (8 rows x 64 B each per warp)
-    constexpr int AI = (NB / 2 + NW - 1) / NW;    // activation items per thread per k block (copy: 2 rows per warp)
-    constexpr uint32_t A_STAGE = kTcRows * kTcBK * 2;      // 32 KB of BF16 weights
-    constexpr uint32_t B_HALF = NB * kTcBK * 2;            // one BF16 activation tile (<= 16 KB)
-    constexpr uint32_t B_STAGE = 2 * B_HALF;               // hi + lo terms of activation * block scale
-    constexpr uint32_t TMEM_COLS = NB < 32 ? 32 : NB;
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mma_bar[kTcStages];
+__global__ void __launch_bounds__(F_THREADS, 2)
+gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap amap, const __grid_constant__ F8TcParams p) {
+    constexpr int STAGES = f_stages(NB), COLS = NB / 2;          // columns of a warp
+    constexpr uint32_t STAGE = f_stage_bytes(NB), TMEM_COLS = 2 * NB + 128 <= 256 ? 256 : 512;
+    static_assert(TMEM_COLS == 256, "two blocks per SM");
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], w_bar[2], d_bar[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ unsigned s_ticket;
-    __shared__ float sc_s[kTcMaxKb];              // this CTA's block scales (one per k block), staged once
+    __shared__ float sc_s[kTcMaxKb];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
+    const uint32_t wb = smem_u32(w_bar), db = smem_u32(d_bar);
+    int* const err = &g_f8tc_wait_error;
+    const int rank = blockIdx.x, n0 = blockIdx.y * kTcRows, m0 = blockIdx.z * NB, nkb_total = p.K / kTcBK;
+    const int kb0 = rank * p.kper, nkb = max(0, min(nkb_total, kb0 + p.kper) - kb0);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tile = blockIdx.x, split = blockIdx.y;
-    const int n0 = tile * kTcRows;
-    const int nkb_total = p.K / kTcBK;
-    const int per = (nkb_total + p.splits - 1) / p.splits;
-    const int kb0 = split * per, kb1 = min(nkb_total, kb0 + per);
-    const int nkb = max(0, kb1 - kb0);
-    const int SK = nkb_total;                     // scale row length (K % 128 == 0)
-    const int rr = lane & 7, piece = lane >> 3;
-
-    // block scales are weights: staged before the dependency wait, off the per-block critical path
-    for (int i = tid; i < nkb; i += blockDim.x) sc_s[i] = bf16_bits_to_f32(__ldg(p.S + (size_t)(n0 >> 7) * SK + kb0 + i));
-    if (warp == 0) tmem_alloc(&tmem_base_s, TMEM_COLS);
+    // the block's scales are weights: staged before the dependency wait
+    for (int i = tid; i < nkb; i += F_THREADS) sc_s[i] = bf16_bits_to_f32(__ldg(p.S + (size_t)blockIdx.y * nkb_total + kb0 + i));
+    if (warp == F_WARPS + 1) tmem_alloc(&tmem_base_s, TMEM_COLS);
     if (tid == 0) {
-#pragma unroll
-        for (int s = 0; s < kTcStages; ++s) mbar_init(&mma_bar[s], 1);
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&w_bar[b], F_WARPS); mbar_init(&d_bar[b], 1); }
         mbar_fence_init();
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&amap) : "memory");
     }
-
-    // ---- raw rings (cp.async): global -> shared in FULL 128-byte lines (8 lanes per weight row, 16 lanes
-    // per activation row), stored row-major with the 16-byte pieces of a row XOR-swizzled by (row & 7) so that
-    // both the line-wise copy and the core-matrix-wise read-back (8 rows x one piece per quarter warp) are
-    // bank-conflict free.  Weights never depend on the previous kernel: their first kTcRaw blocks are requested
-    // before the dependency wait, the activation slabs after it.  Group order: W0..W(D-1) | A0..A(D-1) |
-    // (W_D, A_D) | ...: block `b` is complete for a thread once at most D-1 of its groups are pending, and
-    // visible to the CTA after the next barrier -- iteration `it` therefore waits for block it+1 before its barrier.
-    unsigned char* raw_w = smem + (size_t)kTcStages * (A_STAGE + B_STAGE);
-    unsigned char* raw_a = raw_w + (size_t)kTcRaw * kTcRows * kTcBK;
-    auto issue_weights = [&](int kb, int rs) {
-#pragma unroll
-        for (int i = 0; i < WI; ++i) {
-            const int r = (i * NW + warp) * 4 + (lane >> 3), pc = lane & 7;     // 4 rows x 128 B per warp request
-            const uint8_t* src = p.B + (size_t)(n0 + r) * p.K + (size_t)kb * kTcBK + pc * 16;
-            const uint32_t dst = smem_u32(raw_w + (size_t)rs * (kTcRows * kTcBK) + r * 128 + ((pc ^ (r & 7)) * 16));
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst), "l"(src) : "memory");
-        }
-    };
-    auto issue_acts = [&](int kb, int rs) {
-#pragma unroll
-        for (int i = 0; i < AI; ++i) {
-            const int m = (i * NW + warp) * 2 + (lane >> 4), pc = lane & 15;    // 2 rows x 256 B per warp request
-            if (m < NB) {
-                const bool ok = m < p.M;                       // rows past the batch are zero-filled (src-size 0)
-                const uint16_t* src = p.A + (ok ? (size_t)m * p.K + (size_t)kb * kTcBK + pc * 8 : 0);
-                const uint32_t dst = smem_u32(raw_a + (size_t)rs * (NB * kTcBK * 2) + m * 256 + ((pc ^ (m & 7)) * 16));
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
-            }
-        }
-    };
-#pragma unroll
-    const bool conv = warp < NW;                  // 16 converter warps; warp NW only issues the MMAs
-    for (int d = 0; d < kTcRaw; ++d) {
-        if (conv && d < nkb) issue_weights(kb0 + d, d);
-        asm volatile("cp.async.commit_group;" ::: "memory");   // one group per block, empty ones included
-    }
-    griddep_wait();
-    griddep_launch();
-#pragma unroll
-    for (int d = 0; d < kTcRaw; ++d) {
-        if (conv && d < nkb) issue_acts(kb0 + d, d);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    asm volatile("cp.async.wait_group %0;" :: "n"(kTcRaw - 1) : "memory");       // block 0 (weights + slab) landed
-
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem_d = tmem_base_s;
-    constexpr uint32_t idesc = umma_idesc_bf16(NB);
+    const uint32_t tmem = tmem_base_s, tmem_w = tmem + 2 * NB;   // accumulators, then two k blocks of weights (64 columns each)
+    float acc[COLS];
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) acc[j] = 0.f;
 
-    for (int it = 0; it < nkb; ++it) {
-        const int st = it & 1, kb = kb0 + it, rs = it % kTcRaw;
-        unsigned char* a_s = smem + (size_t)st * (A_STAGE + B_STAGE);
-        unsigned char* b_s = a_s + A_STAGE;
-        const unsigned char* rw = raw_w + (size_t)rs * (kTcRows * kTcBK);
-        const unsigned char* ra = raw_a + (size_t)rs * (NB * kTcBK * 2);
-        const float sc = sc_s[it];
-        if (conv) {
-            uint4 wq[WI], aq[AI];
-#pragma unroll
-            for (int i = 0; i < WI; ++i) {
-                const int q = i * NW + warp;                      // 32 items: row group q>>1, 64-byte half q&1
-                const int r = 8 * (q >> 1) + rr, pc = (q & 1) * 4 + piece;
-                wq[i] = *reinterpret_cast<const uint4*>(rw + r * 128 + ((pc ^ rr) * 16));
+    if (warp == F_WARPS) {
+        // ---------------- copies; the first weights leave before the dependency wait
+        if (elect_one()) {
+            const uint64_t once = l2_evict_first();
+            auto weights = [&](int it, uint32_t s) {
+                mbar_expect_tx(full + 8u * s, STAGE);
+                if (p.once) tma_load_2d_hint(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s, once);
+                else tma_load_2d(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s);
+            };
+            auto rows = [&](int it, uint32_t s) {
+                const uint32_t at = ring + s * STAGE + F_W_BYTES;
+                tma_load_2d(at, &amap, (kb0 + it) * kTcBK, m0, full + 8u * s);
+                tma_load_2d(at + NB * 128u, &amap, (kb0 + it) * kTcBK + 64, m0, full + 8u * s);
+            };
+            const int first = min(nkb, STAGES);
+            for (int it = 0; it < first; ++it) weights(it, (uint32_t)it);
+            griddep_wait();
+            griddep_launch();
+            for (int it = 0; it < first; ++it) rows(it, (uint32_t)it);
+            RingPos r;
+            r.round = 1;
+            int it = first;
+            for (; it < nkb; ++it, r.next(STAGES)) {
+                if (!bar_wait(err, empty + 8u * r.s, r.round ^ 1u)) break;
+                weights(it, r.s);
+                rows(it, r.s);
             }
-#pragma unroll
-            for (int i = 0; i < AI; ++i) {
-                const int q = i * NW + warp;                      // NB/2 items: row group q>>2, 64-byte quarter q&3
-                if (q < NB / 2) {
-                    const int m = 8 * (q >> 2) + rr, pc = (q & 3) * 4 + piece;
-                    aq[i] = *reinterpret_cast<const uint4*>(ra + m * 256 + ((pc ^ rr) * 16));
-                }
-            }
-            // the MMAs that read this BF16 stage two iterations ago must have completed
-            if (it >= kTcStages) mbar_wait(&mma_bar[st], (uint32_t)(((it >> 1) - 1) & 1));
-            // weights: 16 codes -> 16 bf16 = k chunks c0, c0 + 1 of row r
-#pragma unroll
-            for (int i = 0; i < WI; ++i) {
-                const int q = i * NW + warp;
-                const int c0 = (q & 1) * 8 + piece * 2;
-                unsigned char* dst = a_s + (size_t)c0 * (kTcRows * 16) + (size_t)(q >> 1) * 128 + rr * 16;
-                uint4 o0, o1;
-                e4m3x4_to_bf16x4(wq[i].x, o0.x, o0.y); e4m3x4_to_bf16x4(wq[i].y, o0.z, o0.w);
-                e4m3x4_to_bf16x4(wq[i].z, o1.x, o1.y); e4m3x4_to_bf16x4(wq[i].w, o1.z, o1.w);
-                *reinterpret_cast<uint4*>(dst) = o0;
-                *reinterpret_cast<uint4*>(dst + kTcRows * 16) = o1;
-            }
-            // activations: 8 bf16 x block scale -> bf16, k chunk c of batch row m
-#pragma unroll
-            for (int i = 0; i < AI; ++i) {
-                const int q = i * NW + warp;
-                if (q < NB / 2) {
-                    const int c = (q & 3) * 4 + piece;
-                    unsigned char* dst = b_s + (size_t)c * (NB * 16) + (size_t)(q >> 2) * 128 + rr * 16;
-                    const uint32_t aw[4] = {aq[i].x, aq[i].y, aq[i].z, aq[i].w};
-                    uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float v0 = bf16lo(aw[j]) * sc, v1 = bf16hi(aw[j]) * sc;   // exact-ish f32 (8 x 8 bit product)
-                        hi[j] = pack_bf16x2(v0, v1);
-                        lo[j] = pack_bf16x2(v0 - bf16lo(hi[j]), v1 - bf16hi(hi[j]));    // residual of the BF16 rounding
-                    }
-                    *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                    *reinterpret_cast<uint4*>(dst + B_HALF) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-                }
-            }
-            fence_proxy_async();          // generic-proxy smem writes -> visible to the tensor core (async proxy)
-            asm volatile("cp.async.wait_group %0;" :: "n"(kTcRaw - 2) : "memory");   // this thread's part of block it+1 landed
+            if (it < nkb)                                     // given up: do not leave with copies in flight
+                for (int j = max(0, it - STAGES); j < it; ++j) bar_wait(err, full + 8u * (uint32_t)(j % STAGES), (uint32_t)((j / STAGES) & 1));
+        } else {
+            griddep_wait();
+            griddep_launch();
         }
-        __syncthreads();                  // BF16 stage complete; raw slot `rs` fully read; block it+1 visible to all
-        if (conv) {
-            // refill the raw slot that every thread has finished reading, keep the group count uniform
-            if (it + kTcRaw < nkb) { issue_weights(kb + kTcRaw, rs); issue_acts(kb + kTcRaw, rs); }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        } else if (lane == 0) {           // the MMA warp: off the converters' critical path
+        __syncwarp();
+    } else if (warp == F_WARPS + 1) {
+        // ---------------- MMAs
+        griddep_wait();
+        griddep_launch();
+        if (elect_one()) {
+            constexpr uint32_t idesc = umma_idesc_bf16(NB);
+            RingPos r;
+            for (int it = 0; it < nkb; ++it, r.next(STAGES)) {
+                const uint32_t b = (uint32_t)it & 1u;
+                if (!bar_wait(err, full + 8u * r.s, r.round) || !bar_wait(err, wb + 8u * b, (uint32_t)(it >> 1) & 1u)) break;
+                tc_fence_after();
+                const uint32_t a_s = ring + r.s * STAGE + F_W_BYTES;
+#pragma unroll
+                for (int ks = 0; ks < kTcBK / 16; ++ks)
+                    umma_bf16_ta(tmem + b * NB, tmem_w + b * 64u + (uint32_t)ks * 8u, desc_sw128(a_s + (uint32_t)(ks >> 2) * (NB * 128u)) + (uint64_t)((ks & 3) * 2),
+                                 idesc, ks > 0 ? 1u : 0u);
+                umma_commit(&d_bar[b]);
+                umma_commit(&empty_bar[r.s]);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------- codes -> TMEM, and the partial sums of the block before
+        griddep_wait();
+        griddep_launch();
+        const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
+        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+        bool ok = true;
+        auto add = [&](int it) {                              // acc += scale x the products of block it
+            const uint32_t b = (uint32_t)it & 1u;
+            ok = ok && bar_wait(err, db + 8u * b, (uint32_t)(it >> 1) & 1u);
+            __syncwarp();
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(a_s), b_addr = smem_u32(b_s);
+            const float sc = sc_s[it];
+            const uint32_t at = tmem + lanes + b * NB + (uint32_t)half * COLS;
+            if constexpr (COLS == 8) {
+                float v[8];
+                tmem_ld8(at, v);
 #pragma unroll
-            for (int ks = 0; ks < kTcBK / 16; ++ks) {
-                const uint64_t da = umma_desc(a_addr + ks * 2 * (kTcRows * 16), kTcRows * 16, 128);
-                const uint64_t db = umma_desc(b_addr + ks * 2 * (NB * 16), NB * 16, 128);
-                const uint64_t dl = umma_desc(b_addr + B_HALF + ks * 2 * (NB * 16), NB * 16, 128);
-                umma_bf16(tmem_d, da, db, idesc, (it > 0 || ks > 0) ? 1u : 0u);
-                umma_bf16(tmem_d, da, dl, idesc, 1u);
-            }
-            umma_commit(&mma_bar[st]);    // arrives when every MMA issued so far has completed
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // ---- epilogue
-    if (nkb > 0) {
-        const int last = nkb - 1;
-        mbar_wait(&mma_bar[last & 1], (uint32_t)((last >> 1) & 1));
-    }
-    tc_fence_after();
-    const int row = 32 * (warp & 3) + lane;                 // TMEM lane = weight row of the tile
-    const int n = n0 + row;
-    const size_t tile_ws = ((size_t)tile * p.splits + split) * (size_t)NB * kTcRows;
-    if (warp < 4) {
+                for (int j = 0; j < 8; ++j) acc[j] = fmaf(sc, v[j], acc[j]);
+            } else {
 #pragma unroll
-        for (int c = 0; c < NB; c += 16) {
-            float v[16];
-            if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(32 * warp) << 16) + c, v);
-            else {
+                for (int c = 0; c < COLS; c += 16) {
+                    float v[16];
+                    tmem_ld16(at + c, v);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = 0.f;
-            }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int m = c + j;
-                if (m >= p.M) continue;
-                if (p.splits == 1) {
-                    float x = v[j];
-                    const size_t o = (size_t)m * p.N + n;
-                    if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[n]);
-                    p.C[o] = p.residual ? hadd_bf16_bits(x, p.residual[o]) : f32_to_bf16_bits(x);
-                } else {
-                    __stcg(p.ws + tile_ws + (size_t)m * kTcRows + row, v[j]);
+                    for (int j = 0; j < 16; ++j) acc[c + j] = fmaf(sc, v[j], acc[c + j]);
                 }
+            }
+            tc_fence_before();
+        };
+        RingPos r;
+        for (int it = 0; it < nkb; ++it, r.next(STAGES)) {
+            const uint32_t b = (uint32_t)it & 1u, src = ring + r.s * STAGE + (uint32_t)row * 128u;
+            ok = ok && bar_wait(err, full + 8u * r.s, r.round);
+            __syncwarp();
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {                     // 32 codes: 16 columns
+                uint32_t o[16];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    uint4 w;
+                    const uint32_t at = src + (uint32_t)(((half * 4 + h * 2 + i) ^ (row & 7)) << 4);
+                    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(w.x), "=r"(w.y), "=r"(w.z), "=r"(w.w) : "r"(at) : "memory");
+                    e4m3x4_to_bf16x4(w.x, o[8 * i], o[8 * i + 1]);
+                    e4m3x4_to_bf16x4(w.y, o[8 * i + 2], o[8 * i + 3]);
+                    e4m3x4_to_bf16x4(w.z, o[8 * i + 4], o[8 * i + 5]);
+                    e4m3x4_to_bf16x4(w.w, o[8 * i + 6], o[8 * i + 7]);
+                }
+                tmem_st16u(tmem_w + lanes + b * 64u + (uint32_t)(half * 32 + h * 16), o);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&w_bar[b]);
+            if (it > 0) add(it - 1);                          // ... before block it + 1 takes its place
+        }
+        if (nkb > 0) add(nkb - 1);
+    }
+
+    // ---------------- outputs
+    const int rows_here = min(NB, p.M - m0);
+    auto store = [&](float x, int m, int n) {
+        const size_t o = (size_t)(m0 + m) * p.N + n;
+        if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[n]);
+        p.C[o] = p.residual ? hadd_bf16_bits(x, p.residual[o]) : f32_to_bf16_bits(x);
+    };
+    const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
+    if (p.splits == 1) {
+        if (warp < F_WARPS) {
+#pragma unroll
+            for (int j = 0; j < COLS; ++j)
+                if (half * COLS + j < rows_here) store(acc[j], half * COLS + j, n0 + row);
+        }
+    } else {                                                  // column m belongs to block m % splits
+        const int slots = (rows_here + p.splits - 1) / p.splits;
+        __syncthreads();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");     // every ring is free
+        if (warp < F_WARPS) {
+            int owner = half * COLS % p.splits, slot = half * COLS / p.splits;
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) {
+                if (half * COLS + j < rows_here) {
+                    const uint32_t to = ring + (uint32_t)((rank * slots + slot) * kTcRows + row) * 4u;
+                    uint32_t remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(to), "r"(owner));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(remote), "f"(acc[j]) : "memory");
+                }
+                if (++owner == p.splits) { owner = 0; ++slot; }
+            }
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (warp < F_WARPS) {
+            const int parts = (nkb_total + p.kper - 1) / p.kper;              // blocks that had any k
+            const float* part = (const float*)(smem + (ring - smem_u32(smem)));
+            for (int slot = half; slot * p.splits + rank < rows_here; slot += 2) {
+                float x = 0.f;
+                for (int s = 0; s < parts; ++s) x += part[(s * slots + slot) * kTcRows + row];
+                store(x, slot * p.splits + rank, n0 + row);
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_d, TMEM_COLS);
-    if (p.splits == 1) return;
-    if (tid == 0) {
-        __threadfence();
-        s_ticket = atomicAdd(p.counters + tile, 1u);
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_ticket != (unsigned)(p.splits - 1)) return;
-    // last CTA of the tile: fold the split-K partials in split order (deterministic), then the epilogue.
-    // thread = (weight row, half of the batch rows); the loads of eight splits are issued together.
-    if (conv) {
-        const int r = tid & (kTcRows - 1), half = tid >> 7;      // four batch-row phases with 512 threads
-        const float* base = p.ws + (size_t)tile * p.splits * NB * kTcRows;
-        const int nn = n0 + r;
-        for (int m = half; m < p.M; m += kTcThreads / kTcRows) {
-            float x = 0.f;
-            for (int s0 = 0; s0 < p.splits; s0 += 8) {
-                float v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    v[u] = (s0 + u < p.splits) ? __ldcg(base + ((size_t)(s0 + u) * NB + m) * kTcRows + r) : 0.f;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) x += v[u];
-            }
-            const size_t o = (size_t)m * p.N + nn;
-            if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[nn]);
-            p.C[o] = p.residual ? hadd_bf16_bits(x, p.residual[o]) : f32_to_bf16_bits(x);
-        }
-    }
-    if (tid == 0) p.counters[tile] = 0;
+    if (warp == F_WARPS + 1) tmem_dealloc(tmem, TMEM_COLS);
 }
 
-static float* g_tc_ws = nullptr;
-static unsigned* g_tc_cnt = nullptr;
-static const size_t kTcWsBytes = 96ull << 20;
-static const int kTcMaxTiles = 8192;
+template <int NB>
+cudaError_t f8tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int splits) {
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f_smem(NB));
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    cfg->blockDim = dim3(F_THREADS);
+    cfg->dynamicSmemBytes = f_smem(NB);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+    return cudaSuccess;
+}
+
+// blocks that the device holds at one time in clusters of s (clusters do not cross its processing clusters)
+int f8tc_held(int s) {
+    static int held[9] = {};
+    if (held[s] == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[2];
+        int n = 0;
+        cfg.gridDim = dim3(s, 64);
+        if (f8tc_config<64>(&cfg, at, s) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_fp8_tc_kernel<64>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        held[s] = n > 0 ? n * s : -1;
+    }
+    return held[s];
+}
+
+// Blocks per tile: an SM draws 24 bytes of weights per cycle when all do (HBM), and needs 600 cycles at least from one k block of a
+// block to its next; start and end cost 6000 cycles, half of it hidden where two blocks share an SM, an exchange 2000 more.
+int f8tc_splits(long long tiles, int nkb) {
+    const int sms = sm_count();
+    int best = 1;
+    double best_cost = 1e30;
+    for (int s = 1; s <= 8; ++s) {
+        if (s > 1 && (nkb < 2 * s || f8tc_held(s) <= 0)) continue;
+        const long long blocks = tiles * s;
+        const int held = s == 1 ? 2 * sms : f8tc_held(s);
+        const double rounds = (double)((blocks + held - 1) / held), per_sm = blocks <= sms ? 1.0 : fmin(2.0, (double)blocks / sms);
+        const double cost = rounds * ((nkb + s - 1) / s) * fmax(per_sm * F_W_BYTES / 24.0, 600.0) + 6000.0 + (rounds - 1.0) * 3000.0 + (s > 1 ? 2000.0 : 0.0);
+        if (cost < best_cost * 0.999) { best_cost = cost; best = s; }
+    }
+    return best;
+}
 
 template <int NB>
-static int launch_tc(TcParams p, cudaStream_t st) {
-    const int tiles = p.N / kTcRows, nkb = p.K / kTcBK;
-    // one CTA per SM: pick the split-K count that fills whole waves of the 148 SMs best (ties -> fewer splits,
-    // i.e. fewer partials through L2); every split keeps at least two k blocks
-    const int sms = sm_count();
-    int splits = 1;
-    double best = -1.0;
-    for (int s = 1; s <= 12 && s * 2 <= (nkb < 2 ? 2 : nkb); ++s) {
-        const long ctas = (long)tiles * s;
-        const long waves = (ctas + sms - 1) / sms;
-        const int per = (nkb + s - 1) / s;
-        // time ~ waves * (k blocks per CTA + fixed cost of ~2 blocks): lower is better
-        const double t = (double)waves * (per + 2.0);
-        const double score = 1.0 / t - 1e-6 * s;
-        if (score > best) { best = score; splits = s; }
+int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
+    const int tiles = p.N / kTcRows, mt = (p.M + NB - 1) / NB, nkb = p.K / kTcBK;
+    p.splits = f8tc_splits((long long)tiles * mt, nkb);
+    p.kper = (nkb + p.splits - 1) / p.splits;
+    p.once = mt == 1;
+    PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8_tc failed: the driver does not export cuTensorMapEncodeTiled");
+    CUtensorMap wmap, amap;
+    PGK_REQUIRE(tma_map_bytes_2d(&wmap, B, (uint64_t)p.K, (uint64_t)p.N, kTcBK, kTcRows) &&
+                tma_map_bf16_2d(&amap, A, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)p.K * 2, 64, NB), "gemm_fp8_tc failed: cuTensorMapEncodeTiled refused the operands");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    PGK_CUDA(f8tc_config<NB>(&cfg, at, p.splits));
+    cfg.gridDim = dim3(p.splits, tiles, mt);
+    cfg.stream = st;
+    if (pdl_enabled()) {
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
-    while (splits > 1 && (size_t)tiles * splits * NB * kTcRows * sizeof(float) > kTcWsBytes) --splits;
-    if (!g_tc_ws) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(st, &cs);
-        PGK_REQUIRE(cs == cudaStreamCaptureStatusNone,
-                    "gemm_fp8_tc failed: first call must happen outside graph capture (workspace allocation)");
-        PGK_CUDA(cudaMalloc(&g_tc_ws, kTcWsBytes));
-        PGK_CUDA(cudaMalloc(&g_tc_cnt, kTcMaxTiles * sizeof(unsigned)));
-        PGK_CUDA(cudaMemset(g_tc_cnt, 0, kTcMaxTiles * sizeof(unsigned)));
-    }
-    p.splits = splits;
-    p.ws = g_tc_ws;
-    p.counters = g_tc_cnt;
-    constexpr size_t kSmem = (size_t)kTcStages * (kTcRows * kTcBK * 2 + 2 * NB * kTcBK * 2) +
-                             (size_t)tc_raw_depth(NB) * (kTcRows * kTcBK + NB * kTcBK * 2);
-    static bool attr_set = false;
-    if (!attr_set) {
-        PGK_CUDA(cudaFuncSetAttribute(gemm_fp8_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-        attr_set = true;
-    }
-    PGK_CUDA(launch(gemm_fp8_tc_kernel<NB>, dim3(tiles, splits), dim3(kTcThreads + 32), kSmem, st, p));
+    count_launch();
+    PGK_CUDA(cudaLaunchKernelEx(&cfg, gemm_fp8_tc_kernel<NB>, wmap, amap, p));
     return 0;
 }
 
+}  // namespace
+
 bool gemm_fp8_tc_shape_ok(int M, int K, int N, const void* A, const void* B);
 
-// Smallest batch sent to the tensor cores.  The kernel zero-fills rows M..NB-1, so any M >= 1 works; the crossover
+// Smallest batch sent to the tensor cores.  The copies zero-fill rows M..NB-1, so any M >= 1 works; the crossover
 // against the CUDA-core slab GEMV (whose time grows linearly with M: dequant + M FMAs per weight) measured on
 // B200 is between M = 4 (15.9 us GEMV vs ~16 us here, qkv shape) and M = 5.  PGK_TC_MIN_M overrides (A/B timing).
 int gemm_fp8_tc_min_m() {
@@ -360,13 +358,13 @@ int gemm_fp8_tc(const void* A, const void* B_nk, const void* S, void* C, int M, 
     PGK_REQUIRE(gemm_fp8_tc_shape_ok(M, K, N, A, B_nk),
                 "gemm_fp8_tc failed: needs 1 <= M <= 64, K %% 128 == 0, N %% 128 == 0 and 16-byte aligned pointers "
                 "(M=%d K=%d N=%d)", M, K, N);
-    TcParams p = {};
-    p.A = (const uint16_t*)A; p.B = (const uint8_t*)B_nk; p.S = (const uint16_t*)S; p.C = (uint16_t*)C;
+    F8TcParams p = {};
+    p.S = (const uint16_t*)S; p.C = (uint16_t*)C;
     p.bias = (const uint16_t*)bias; p.residual = (const uint16_t*)residual;
     p.M = M; p.K = K; p.N = N;
-    if (M <= 16) return launch_tc<16>(p, st);
-    if (M <= 32) return launch_tc<32>(p, st);
-    return launch_tc<64>(p, st);
+    if (M <= 16) return launch_f8tc<16>(p, A, B_nk, st);
+    if (M <= 32) return launch_f8tc<32>(p, A, B_nk, st);
+    return launch_f8tc<64>(p, A, B_nk, st);
 }
 
 }  // namespace pgk
@@ -378,4 +376,11 @@ extern "C" int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void*
     PGK_REQUIRE(clean, "gemm_fp8_bf16_tc failed: the weights hold E4M3 codes 0x7F/0xFF (+-480 in the reference's tables, "
                 "NaN for the tensor-core conversion); use pgk_gemv_fp8_bf16, which serves them exactly");
     return pgk::gemm_fp8_tc(A, B_nk, S, C, M, K, N, bias, residual, (cudaStream_t)stream);
+}
+
+extern "C" int pgk_gemm_fp8_wait_error(int* out) {
+    int v = 0;
+    PGK_CUDA(cudaMemcpyFromSymbol(&v, pgk::g_f8tc_wait_error, sizeof(int)));
+    *out = v;
+    return 0;
 }

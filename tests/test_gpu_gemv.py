@@ -463,3 +463,30 @@ def test_gemm_fp8_f8mma_wide_dynamic_range():
     out, gA, gB, gS = gk.zeros((M, N), gk.bfloat16), gk.from_numpy(A), gk.from_numpy(codes), gk.from_numpy(scale)
     api.gemm_fp8_bf16_f8mma(gA.device_ptr, gB.device_ptr, gS.device_ptr, out.device_ptr, M, K, N, None, None, None)
     assert f32acc_mismatch(out.to_numpy(), ref, TOL) == 0
+
+
+@pytest.mark.parametrize("M", [1, 16, 17, 33, 64])
+@pytest.mark.parametrize("K,N", [(128, 128), (384, 256), (1152, 1024), (4096, 384), (4096, 19072)])
+def test_gemm_fp8_tc_against_float64(K, N, M):
+    """Every width of the batch, k ranges that blocks of a cluster share unevenly, tiles over several waves, block scales far apart: exact
+    products, 128 of them summed and scaled in float32, so the sums carry K float32 roundings of their magnitude at most and
+    the output one BF16 rounding."""
+    import ctypes
+    from pygpukit_b200._lib import api
+    rng = np.random.default_rng(K + N + M)
+    codes, _ = rand_fp8_weights(rng, N, K)
+    scale = bf16(np.exp2(rng.integers(-9, 3, (N // 128, K // 128))).astype(np.float32) * 1.5)
+    A = rand_bf16(rng, (M, K))
+    e, m = (codes >> 3) & 15, codes & 7
+    W = np.where(e > 0, np.exp2(e.astype(np.float64) - 7) * (1 + m / 8), np.exp2(-6.0) * m / 8) * np.where(codes & 128, -1, 1)
+    W *= np.repeat(np.repeat(f32(scale).astype(np.float64), 128, 0), 128, 1)
+    a = f32(A).astype(np.float64)
+    ref, size = a @ W.T, np.abs(a) @ np.abs(W).T
+    out = gk.zeros((M, N), gk.bfloat16)
+    gA, gB, gS = gk.from_numpy(A), gk.from_numpy(codes), gk.from_numpy(scale)
+    api.gemm_fp8_bf16_tc(gA.device_ptr, gB.device_ptr, gS.device_ptr, out.device_ptr, M, K, N, None, None, None)
+    got = f32(out.to_numpy()).astype(np.float64)
+    assert (np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + 2.0 ** -24 * (128 + K / 128) * size + 1e-30).all()
+    err = ctypes.c_int(7)
+    api.gemm_fp8_wait_error(ctypes.byref(err))
+    assert err.value == 0
