@@ -1,0 +1,87 @@
+"""Row kernels of the token-major models in the forms that many rows take: a causal convolution of several rows per thread, the
+weighted sum of expert rows by four elements, router logits by pairs of rows, rotary angles shared by a token's heads."""
+import numpy as np
+import pytest
+
+import pygpukit_b200 as gk
+from pygpukit_b200._lib import api
+
+pytestmark = pytest.mark.gpu
+
+
+def f32(a):
+    return gk.from_numpy(np.ascontiguousarray(a, np.float32))
+
+
+def i32(a):
+    return gk.from_numpy(np.ascontiguousarray(a, np.int32))
+
+
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("rows,twice", [((256,), False), ((1, 258, 2, 3), True), ((130, 131), True), ((5, 1, 1, 300), False)])
+def test_convolution_over_many_rows_equals_portions(rows, twice, taps):
+    """one launch of 256 rows and more against the same rows in launches of fewer (the kernel of a row per block): the same bits in
+    rows and rings, sequences that start, continue and end anywhere in a thread's four rows"""
+    W, S = 300, len(rows)
+    rng = np.random.default_rng(sum(rows) + taps)
+    ring, first = max(1, taps - 1), [0 if s % 2 == 0 else 7 for s in range(S)]
+    h, w = rng.standard_normal((sum(rows), W)), f32(rng.standard_normal((W, taps)))
+    start = rng.standard_normal((S, (2 if twice else 1) * ring * W)).astype(np.float32)
+    at = np.concatenate([[0], np.cumsum(rows)])
+
+    def run(parts):
+        state, steps, got = f32(start), [0] * S, [[] for _ in rows]
+        for part in parts:                                       # [(sequence, first, end)]
+            x = np.concatenate([h[at[s] + lo:at[s] + hi] for s, lo, hi in part])
+            slot = np.concatenate([[s] * (hi - lo) for s, lo, hi in part])
+            pos = np.concatenate([first[s] + np.arange(lo, hi) for s, lo, hi in part])
+            par = np.concatenate([[steps[s] & 1] * (hi - lo) for s, lo, hi in part])
+            seqs, row = [], 0
+            for s, lo, hi in part:
+                seqs.append((row, hi - lo, s, first[s] + lo))
+                row += hi - lo
+            xd, u, sl, ps, pr, sq = f32(x), gk.zeros(x.shape, gk.float32), i32(slot), i32(pos), i32(par), i32(seqs)
+            api.causal_conv_rows_f32(xd.device_ptr, u.device_ptr, w.device_ptr, state.device_ptr, sl.device_ptr, ps.device_ptr,
+                                     pr.device_ptr if twice else None, len(x), W, taps, None)
+            if not twice:
+                api.causal_conv_state_f32(xd.device_ptr, state.device_ptr, sq.device_ptr, len(seqs), W, taps, None)
+            out, row = u.to_numpy(), 0
+            for s, lo, hi in part:
+                got[s].append(out[row:row + hi - lo])
+                row += hi - lo
+                steps[s] += 1
+        return np.concatenate([np.concatenate(g) for g in got])
+
+    whole = run([[(s, 0, n) for s, n in enumerate(rows)]])
+    cut = run([[(s, lo, min(lo + 100, n))] for s, n in enumerate(rows) for lo in range(0, n, 100)])
+    assert np.array_equal(whole, cut)
+
+
+@pytest.mark.parametrize("top,W", [(1, 4), (4, 2048), (8, 516), (9, 64), (3, 30), (64, 12)])
+def test_weighted_sum_of_expert_rows(top, W):
+    rng = np.random.default_rng(top + W)
+    T = 37
+    parts, own, shared = (rng.standard_normal((n, W)).astype(np.float32) for n in (T * top, T, T))
+    wt = rng.random((T, top)).astype(np.float32)
+    inv = rng.permutation(T * top).reshape(T, top)
+    mat = np.where(rng.random((T, top)) < 0.2, -1, 0)
+    gate = rng.standard_normal((T, 3)).astype(np.float32)
+    keep = [f32(parts), i32(inv), i32(mat), f32(wt), f32(own), f32(shared), f32(gate)]
+    out = gk.from_numpy(np.full((T, W), 7.0, np.float32))
+    p = [k.device_ptr for k in keep]
+    api.moe_combine_rows_f32(p[0], p[1], p[2], p[3], top, p[4], p[5], p[6], 3, 1, out.device_ptr, T, W, None)
+    x = np.where((mat < 0)[..., None], own[:, None].astype(np.float64), parts.astype(np.float64)[inv])
+    terms = np.concatenate([wt[..., None].astype(np.float64) * x, (shared / (1 + np.exp(-gate[:, 1:2].astype(np.float64))))[:, None]], 1)
+    assert (np.abs(out.to_numpy() - terms.sum(1)) <= 2.0 ** -23 * (top + 4) * np.abs(terms).sum(1) + 1e-30).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 1, 32), (10, 8, 33), (17, 9, 100), (300, 16, 2048), (2001, 64, 31), (1000, 63, 520)])
+def test_router_logits(M, N, K):
+    rng = np.random.default_rng(M + N)
+    A, W = rng.standard_normal((M, K + 1)).astype(np.float32), rng.standard_normal((N, K)).astype(np.float32)
+    a, w, c = f32(A), f32(W), gk.from_numpy(np.full((M, N + 1), 7.0, np.float32))
+    api.gemm_rows_f32(a.device_ptr, K + 1, None, w.device_ptr, 0, 0, c.device_ptr, N + 1, M, N, K, None, 1, M, 0, 1.0, 0.0, None)
+    x, y = A[:, :K].astype(np.float64), W.astype(np.float64)
+    out = c.to_numpy()
+    assert (np.abs(out[:, :N] - x @ y.T) <= 2.0 ** -24 * (K / 32 + 6) * (np.abs(x) @ np.abs(y).T)).all()
+    assert (out[:, N:] == 7.0).all()
