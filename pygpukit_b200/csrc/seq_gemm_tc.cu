@@ -340,6 +340,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 epilogue_rows<16>(a, p.epi, v, w.m0 + c, w.rows - c, col, lane);
             }
         }
+        __syncwarp();                             // lanes beyond N left the epilogue early; the barrier's arrival takes whole warps
         cluster_arrive_wait();                    // the others may still read this block's partial sums
     }
     tc_fence_before();

@@ -270,3 +270,26 @@ def test_few_rows_batches(M, epi):
             z = z * sigmoid(gate[:, sl])
         assert (np.abs(out[:, sl] - z) <= tol + 1e-6).all()
     no_wait_error()
+
+
+@pytest.mark.parametrize("M", [24, 40, 200])
+@pytest.mark.parametrize("N,K", [(140, 1024), (1090, 2056), (2, 4096)])
+@pytest.mark.parametrize("epi", [1, 4])
+def test_rows_beyond_n_with_shared_k(M, N, K, epi):
+    """k shared by a cluster and a last column tile that is not full: lanes beyond N skip their stores, and the block still meets the
+    others at the closing barrier as whole warps"""
+    A, W = operands(M + N, M, N, K)
+    z, tol = product(A, W[0])
+    cols = N // 2 if epi == 1 else N
+    old = np.random.default_rng(1).standard_normal((M, cols)).astype(np.float32)
+    cs = np.random.default_rng(2).standard_normal(N).astype(np.float32)
+    a, w, c, s = gk.from_numpy(A), dev_w(W[0]), gk.from_numpy(old), gk.from_numpy(cs)
+    api.gemm_seq_f32(a.device_ptr, K, 0, w.device_ptr, 2, 0, c.device_ptr, cols, 0, M, N, K, 1, epi, 0.0, 0.0, s.device_ptr, None, 0, None, 0, 0, 0, None)
+    if epi == 1:
+        g, u = z[:, 0::2], z[:, 1::2]
+        ref = g * sigmoid(g) * u
+        tol = 2.0 * (1.0 + np.abs(u) + np.abs(g)) * np.maximum(tol[:, 0::2], tol[:, 1::2])
+    else:
+        ref, tol = old + cs * z, tol * np.abs(cs)
+    assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6 * (1 + np.abs(ref))).all()
+    no_wait_error()
