@@ -62,7 +62,10 @@ __device__ int g_attn_wait_error = 0;
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, 128;" :: "r"(1 + half) : "memory"); }
+__device__ __forceinline__ void half_sync(int half) {
+    __syncwarp();                                         // bar.sync takes whole warps, and a few lanes' stores come before it
+    asm volatile("bar.sync %0, 128;" :: "r"(1 + half) : "memory");
+}
 __device__ __forceinline__ void sts128(uint32_t addr, const uint32_t (&v)[4]) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(addr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]) : "memory");
 }
@@ -191,6 +194,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
             }
             fence_proxy_async();
         }
+        __syncwarp();
         asm volatile("bar.sync 3, %0;" :: "n"((A_SOFT + 1) * 32) : "memory");
     }
     if (warp == A_SOFT) {
@@ -560,6 +564,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                     gates(u + 1);
                 }
                 if (rr >= live) continue;
+                __syncwarp();                             // lanes beyond the row's end skipped the last stores; the load takes whole warps
                 if (n > 0) {
                     const uint32_t at = lanes + AN + (uint32_t)(u >> 2) * AN + (uint32_t)rr;
                     tmem_ld4x3(at, at + AR, at + 2 * AR, o, x, y);

@@ -209,3 +209,12 @@ def test_nan_query_stays_in_its_row():
     out = c.run(False)
     keep = np.arange(90) != 40
     assert (out[keep] == clean[keep]).all() and np.isnan(out[40]).all()
+
+
+@pytest.mark.parametrize("Dv", [8, 72, 136, 264])
+@pytest.mark.parametrize("gate", [0, 1])
+def test_value_rows_off_the_chunks(Dv, gate):
+    """lanes beyond the value row skip their stores between one load of the accumulators and the next"""
+    c = Case([(0, 130), (140, 1)], 24, 1, 64, Dv, gate=gate, seed=6)
+    ref, old, new = c.exact(), c.run(True), c.run(False)
+    assert np.abs(new - ref).max() <= 2 * np.abs(old - ref).max() + 2 * 2.0 ** -23 * np.abs(ref).max()
