@@ -418,10 +418,12 @@ struct RopeSdpaParams {
 // contexts and the multi-sequence batches.  Here a warp owns 16 positions of a 64-position tile:
 //     S[8 heads (+8 zero rows), 16 pos]  = Q[16, 128] . K^T      16 MMAs, B fragments by ldmatrix from the swizzled tile
 //     online softmax on the 4 scores a thread holds (row = lane / 4), quad shuffles only
-//     O[16, 128] += P[16, 16] . V[16, 128]                       16 MMAs, V fragments by ldmatrix.trans
-// The probabilities go to the tensor cores as TWO bf16 terms, p = hi + lo, hi in rows 0..7 and lo in rows 8..15 of the
-// A fragment (the rows the <= 8 query heads leave empty), so one MMA accumulates both and O = O[0..7] + O[8..15] carries
-// 16 bits of p: the products q.k are exact and p.v is as accurate as the f32 loop it replaces.
+//     O[16, 128] += P[16, 16] . V[16, 128]                       32 MMAs, V fragments by ldmatrix.trans
+// The probabilities go to the tensor cores as FOUR bf16 terms in two A fragments: two halves of p in rows 0..7, the rest in rows
+// 8..15 (the rows the <= 8 query heads leave empty); together they hold all 24 bits, and O = O[0..7] + O[8..15].  The
+// products q.k are exact, p.v is what float32 would give.  With 16 bits of p one output in 2^9 rounds to the other bf16
+// neighbour: 570 of 1024 logits moved on the first decoded token of a two-layer model, none with 24 (context 4096, 32 / 8
+// heads, the attention layer: 30.7 us before and after).
 // One CTA = 4 consumer warps + 1 TMA producer warp, 2 CTAs per SM; up to 8 query heads per CTA, so a GQA group of 8
 // (Llama-3-70B, Qwen3-30B-A3B) reads its K/V once instead of twice.  Stages: 2 x 32 KB for one sequence -- measured:
 // with 3 stages the two CTAs need 202 KB of shared memory, the SM is switched to its largest carve-out, and the GEMVs
@@ -465,6 +467,9 @@ __device__ __forceinline__ void mbar_wait_bounded(uint64_t* bar, uint32_t parity
     }
     __trap();
 }
+// the product's leading terms and the smaller ones: an infinite value row makes the leading ones infinite (or NaN) as float32 would
+// have it, and the smaller ones, whose signs vary, say nothing then
+__device__ __forceinline__ float join_terms(float hi, float lo) { return fabsf(hi) < INFINITY ? hi + lo : hi; }
 // [RMSNorm] + NeoX rotation of one 128-wide head row already in registers (x[i] = row[lane + 32 i]); same arithmetic
 // and rounding points as norm_rope_head128 above
 __device__ __forceinline__ void norm_rope_regs(float (&x)[4], bool use_gamma, const float (&g)[4], float eps, const float (&c)[2],
@@ -591,7 +596,7 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
     }
     __syncthreads();   // q_s / new_s visible; also orders the mbarrier init before every wait
 
-    float o[16][4];                                            // [dim tile of 8][c0 c1: hi rows | c2 c3: lo rows]
+    float o[16][4];                                            // [dim tile of 8][c0 c1: halves of p | c2 c3: the rest]
     float m_run = kNegBig, l_run = 0.f;
     if (warp == kMW) {
         // ---- producer: refill a stage as soon as the four consumer warps have released it
@@ -676,21 +681,27 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
 #pragma unroll
                         for (int e = 0; e < 4; ++e) o[nt][e] *= corr;
                 }
-                // p = hi + lo as two bf16 terms: hi in rows 0..7, lo in rows 8..15 of the A fragment
-                float lo[4];
-                uint32_t hb[4];
+                // p as four bf16 terms that hold all 24 bits, in two A fragments: halves h1, h2 in rows 0..7, what they leave, l1 and l2, in
+                // rows 8..15.  Both halves of a positive p are positive: an infinite value row gives that infinity.
+                float rem[4];
+                uint32_t h1[4];
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { hb[j] = f32_to_bf16_bits(pr[j]); lo[j] = pr[j] - bf16_bits_to_f32(hb[j]); }
-                const uint32_t a0 = hb[0] | (hb[1] << 16), a2 = hb[2] | (hb[3] << 16);
-                const uint32_t a1 = pack_bf16x2(lo[0], lo[1]), a3 = pack_bf16x2(lo[2], lo[3]);
+                for (int j = 0; j < 4; ++j) { h1[j] = __float_as_uint(0.5f * pr[j]) & 0xffff0000u; rem[j] = pr[j] - __uint_as_float(h1[j]); }
+                const uint32_t a0 = (h1[0] >> 16) | h1[1], a2 = (h1[2] >> 16) | h1[3];
+                const uint32_t b0 = pack_bf16x2(rem[0], rem[1]), b2 = pack_bf16x2(rem[2], rem[3]);
+                rem[0] -= bf16lo(b0); rem[1] -= bf16hi(b0); rem[2] -= bf16lo(b2); rem[3] -= bf16hi(b2);
+                const uint32_t a1 = pack_bf16x2(rem[0], rem[1]), a3 = pack_bf16x2(rem[2], rem[3]);
+                const uint32_t b1 = pack_bf16x2(rem[0] - bf16lo(a1), rem[1] - bf16hi(a1)), b3 = pack_bf16x2(rem[2] - bf16lo(a3), rem[3] - bf16hi(a3));
                 // ---- O += P . V
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {
                     const uint32_t ch = (uint32_t)(q * 2 + (lj >> 1));
-                    uint32_t b[4];
-                    ldsm_x4_t(tile + (ch >> 3) * kMBox + v_off + (((ch & 7) ^ v_sw) << 4), b);
-                    mma_bf16_16816(o[2 * q], a0, a1, a2, a3, b[0], b[1]);
-                    mma_bf16_16816(o[2 * q + 1], a0, a1, a2, a3, b[2], b[3]);
+                    uint32_t v[4];
+                    ldsm_x4_t(tile + (ch >> 3) * kMBox + v_off + (((ch & 7) ^ v_sw) << 4), v);
+                    mma_bf16_16816(o[2 * q], a0, a1, a2, a3, v[0], v[1]);
+                    mma_bf16_16816(o[2 * q + 1], a0, a1, a2, a3, v[2], v[3]);
+                    mma_bf16_16816(o[2 * q], b0, b1, b2, b3, v[0], v[1]);
+                    mma_bf16_16816(o[2 * q + 1], b0, b1, b2, b3, v[2], v[3]);
                 }
             }
             if (t + kMStages < ntiles) {                        // hand the stage back to the producer
@@ -708,7 +719,7 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
         const int qrow = lane >> 2, kk = (lane & 3) * 2;
 #pragma unroll
         for (int nt = 0; nt < 16; ++nt)
-            *reinterpret_cast<float2*>(&sm_part[warp][qrow][nt * 8 + kk]) = make_float2(o[nt][0] + o[nt][2], o[nt][1] + o[nt][3]);
+            *reinterpret_cast<float2*>(&sm_part[warp][qrow][nt * 8 + kk]) = make_float2(join_terms(o[nt][0], o[nt][2]), join_terms(o[nt][1], o[nt][3]));
         if ((lane & 3) == 0) { sm_part[warp][qrow][HD] = m_run; sm_part[warp][qrow][HD + 1] = l_run; }
     }
     __syncthreads();

@@ -490,3 +490,57 @@ def test_grouped_gemm_fp8():
         o2 = gk.empty((M, N), gk.bfloat16)
         refcuda.grouped_gemm(gk.from_numpy(A), gk.from_numpy(B), gk.from_numpy(S), o2, gk.from_numpy(ids), M, N, K)
         assert rel_err(o2.to_numpy(), ref) < 1e-5
+
+
+def _exact_decode_attention(q, k, v, ctx, hd):
+    """float64 attention of bf16 rows [Hq, hd] over [Hkv, S, hd] and the sum of |p v| that its rounding is measured by"""
+    G = q.shape[0] // k.shape[0]
+    K, V = (np.repeat(f32(a)[:, :ctx].astype(np.float64), G, 0) for a in (k, v))
+    z = np.einsum("hd,hjd->hj", f32(q).astype(np.float64), K) / np.sqrt(hd)
+    e = np.exp(z - z.max(1, keepdims=True))
+    p = e / e.sum(1, keepdims=True)
+    return np.einsum("hj,hjd->hd", p, V), np.einsum("hj,hjd->hd", p, np.abs(V))
+
+
+@pytest.mark.parametrize("Hq,Hkv,S,ctx", [(32, 8, 256, 3), (32, 4, 256, 20), (16, 16, 256, 60), (64, 8, 4096, 300)])
+def test_rope_sdpa_decode_weights_are_float32(Hq, Hkv, S, ctx):
+    """The key weights enter P.V with all their 24 bits.  Scores below 1 carry a float32 error of 2^-23 or less into a weight, the
+    exponential and the sums some 2^-22 more, so an output is the bf16 rounding of a number within 2^-21 sum |p v| of the exact one; weights of 16 bits
+    (2^-18) put some of these thousands of outputs beyond that."""
+    rng = np.random.default_rng(900 + ctx)
+    hd, pos = 128, ctx - 1
+    width = (Hq + 2 * Hkv) * hd
+    k, v = rand_bf16(rng, (Hkv, S, hd), 0.5), rand_bf16(rng, (Hkv, S, hd), 0.5)
+    qkv = rand_bf16(rng, (1, width), 0.3)
+    qkv[0, Hq * hd:(Hq + Hkv) * hd] = k[:, pos].reshape(-1)
+    qkv[0, (Hq + Hkv) * hd:] = v[:, pos].reshape(-1)
+    one, zero = gk.from_numpy(np.ones((S, hd), np.float32)), gk.from_numpy(np.zeros((S, hd), np.float32))      # no rotation
+    q, gkc, gvc, out = gk.from_numpy(qkv), gk.from_numpy(k), gk.from_numpy(v), gk.zeros((1, Hq * hd), gk.bfloat16)
+    api.rope_sdpa_decode(q.device_ptr, None, None, 1e-6, one.device_ptr, zero.device_ptr, gkc.device_ptr, gvc.device_ptr, out.device_ptr,
+                         Hq, Hkv, hd, S, pos, None, ctx, None, 0.0, None)
+    got = f32(out.to_numpy()).astype(np.float64).reshape(Hq, hd)
+    ref, size = _exact_decode_attention(qkv[0, :Hq * hd].reshape(Hq, hd), k, v, ctx, hd)
+    half_ulp = 2.0 ** (np.floor(np.log2(np.maximum(np.abs(ref), 1e-30))) - 8)
+    assert (np.abs(got - ref) <= half_ulp + 2.0 ** -21 * size).all()
+
+
+@pytest.mark.parametrize("ctx", [5, 70])
+def test_rope_sdpa_decode_infinite_value_rows(ctx):
+    """an infinity in a value row with a weight stays that infinity, whatever the signs of the weight's smaller terms"""
+    rng = np.random.default_rng(950 + ctx)
+    Hq, Hkv, S, hd, pos = 32, 8, 256, 128, ctx - 1
+    k, v = rand_bf16(rng, (Hkv, S, hd), 0.5), rand_bf16(rng, (Hkv, S, hd), 0.5)
+    qkv = rand_bf16(rng, (1, (Hq + 2 * Hkv) * hd), 0.3)
+    v[:, 2, 5::9], v[:, 1, 7::9] = 0x7F80, 0xFF80
+    v[:, 1, 3::9] = v[:, 2, 3::9] = 0x7F80
+    v[:, 1, 4::9], v[:, 2, 4::9] = 0x7F80, 0xFF80                    # of both signs: NaN
+    one, zero = gk.from_numpy(np.ones((S, hd), np.float32)), gk.from_numpy(np.zeros((S, hd), np.float32))
+    q, gkc, gvc, out = gk.from_numpy(qkv), gk.from_numpy(k), gk.from_numpy(v), gk.zeros((1, Hq * hd), gk.bfloat16)
+    api.rope_sdpa_decode(q.device_ptr, None, None, 1e-6, one.device_ptr, zero.device_ptr, gkc.device_ptr, gvc.device_ptr, out.device_ptr,
+                         Hq, Hkv, hd, S, pos, None, ctx, None, 0.0, None)
+    got = f32(out.to_numpy()).reshape(Hq, hd)
+    assert (got[:, 5::9] == np.inf).all() and (got[:, 7::9] == -np.inf).all() and (got[:, 3::9] == np.inf).all() and np.isnan(got[:, 4::9]).all()
+    rest = np.ones(hd, bool)
+    for r in (3, 4, 5, 7):
+        rest[r::9] = False
+    assert np.isfinite(got[:, rest]).all()
