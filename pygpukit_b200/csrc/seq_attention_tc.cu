@@ -87,8 +87,16 @@ __device__ __forceinline__ float ex2(float x) {          // 2^x to 2 units, 0 be
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
+__device__ __forceinline__ float max_nan(float a, float b) {       // NaN if either is
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+// A product whose leading term is infinite or NaN: with an infinite operand that is what float32 gives, while the smaller terms --
+// zeros, of either sign, or infinity minus itself -- make NaN of it.
+__device__ __forceinline__ float leading_or(float lead, float sum) { return fabsf(lead) < INFINITY ? sum : lead; }
 // a + b + c of three accumulators' 16 columns, smallest first
-__device__ __forceinline__ void tmem_sum3(uint32_t t0, uint32_t t1, uint32_t t2, float (&v)[16]) {
+__device__ __forceinline__ void tmem_sum3(uint32_t t0, uint32_t t1, uint32_t t2, float (&v)[16], bool infinities) {
     float x[16], y[16];
     tmem_ld16_async(t2, v);
     tmem_ld16_async(t1, x);
@@ -96,6 +104,10 @@ __device__ __forceinline__ void tmem_sum3(uint32_t t0, uint32_t t1, uint32_t t2,
     tmem_ld_wait(v, x, y);
 #pragma unroll
     for (int r = 0; r < 16; ++r) v[r] = (v[r] + x[r]) + y[r];
+    if (infinities) {
+#pragma unroll
+        for (int r = 0; r < 16; ++r) v[r] = leading_or(y[r], v[r]);
+    }
 }
 
 // CAP: tanh cap; SLOPE: 0 none, 1 per-head slopes, 2 the logarithmic form; PROB: sigmoid weights
@@ -421,41 +433,50 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
             ok = ok && bar_wait(err, s_full, (uint32_t)(i & 1));       // (when a wait runs out the rest runs through without waiting)
             __syncwarp();
             tc_fence_after();
-            float s[16];
-            tmem_sum3(lanes + r0, lanes + AR + r0, lanes + 2 * AR + r0, s);
-#pragma unroll
-            for (int r = 0; r < 16; ++r) {
-                s[r] *= a.scale;
-                if (CAP) s[r] = a.cap * tanhf(s[r] * inv_cap);
-                if (SLOPE) {
-                    const float2 w = rowi[r0 + r];
-                    const float d = fmaxf(w.x - jf, 0.f);
-                    if (SLOPE == 2) s[r] -= w.y * log1pf(__shfl_sync(0xffffffffu, extra_r, r) * d);
-                    else s[r] = fmaf(-w.y, d, s[r]);
-                }
-            }
-            if (!whole) {
+            float s[16], top;
+#pragma unroll 1
+            for (bool again = false;; again = true) {     // a second time only where a score is NaN: an infinite operand?
+                tmem_sum3(lanes + r0, lanes + AR + r0, lanes + 2 * AR + r0, s, again);
 #pragma unroll
                 for (int r = 0; r < 16; ++r) {
-                    const float pi = rowi[r0 + r].x, lo = __shfl_sync(0xffffffffu, lo_r, r);
-                    if (!(j >= jmin && j <= jmax && jf <= pi && (jf >= lo || jf < keep_f))) s[r] = -INFINITY;
+                    s[r] *= a.scale;
+                    if (CAP) s[r] = a.cap * tanhf(s[r] * inv_cap);
+                    if (SLOPE) {
+                        const float2 w = rowi[r0 + r];
+                        const float d = fmaxf(w.x - jf, 0.f);
+                        if (SLOPE == 2) s[r] -= w.y * log1pf(__shfl_sync(0xffffffffu, extra_r, r) * d);
+                        else s[r] = fmaf(-w.y, d, s[r]);
+                    }
                 }
+                if (!whole) {
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const float pi = rowi[r0 + r].x, lo = __shfl_sync(0xffffffffu, lo_r, r);
+                        if (!(j >= jmin && j <= jmax && jf <= pi && (jf >= lo || jf < keep_f))) s[r] = -INFINITY;
+                    }
+                }
+                if (PROB) {
+                    top = 0.f;
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) {
+                        const float z = s[r] + __shfl_sync(0xffffffffu, pb_r, r);
+                        s[r] = s[r] == -INFINITY ? 0.f : 1.f / (1.f + expf(-z));
+                        top = max_nan(top, s[r]);
+                    }
+                } else {
+                    float v[16];
+#pragma unroll
+                    for (int r = 0; r < 16; ++r) v[r] = s[r];
+                    top = reduce16(v, lane, [](float x, float y) { return max_nan(x, y); });
+                }
+                if (again || !__any_sync(0xffffffffu, top != top)) break;
             }
             bool waited = false;
             if (PROB) {
-#pragma unroll
-                for (int r = 0; r < 16; ++r) {
-                    const float z = s[r] + __shfl_sync(0xffffffffu, pb_r, r);
-                    s[r] = s[r] == -INFINITY ? 0.f : 1.f / (1.f + expf(-z));
-                }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive((uint64_t*)(tail_p + 72));
             } else {
-                float v[16];
-#pragma unroll
-                for (int r = 0; r < 16; ++r) v[r] = s[r];
-                const float top = reduce16(v, lane, [](float x, float y) { return fmaxf(x, y); });
                 if (lane < 16) wmax[(r0 + lane) * 4 + quad] = top;
                 half_sync(half);
                 const float4 w = *(const float4*)(wmax + (r0 + (lane & 15)) * 4);
@@ -569,7 +590,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                     const uint32_t at = lanes + AN + (uint32_t)(u >> 2) * AN + (uint32_t)rr;
                     tmem_ld4x3(at, at + AR, at + 2 * AR, o, x, y);
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) o[e] += x[e] + y[e];
+                    for (int e = 0; e < 4; ++e) o[e] = leading_or(o[e], o[e] + (x[e] + y[e]));
                 }
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {

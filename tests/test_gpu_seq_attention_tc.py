@@ -218,3 +218,43 @@ def test_value_rows_off_the_chunks(Dv, gate):
     c = Case([(0, 130), (140, 1)], 24, 1, 64, Dv, gate=gate, seed=6)
     ref, old, new = c.exact(), c.run(True), c.run(False)
     assert np.abs(new - ref).max() <= 2 * np.abs(old - ref).max() + 2 * 2.0 ** -23 * np.abs(ref).max()
+
+
+INFINITE = [
+    dict(portions=[(0, 150)], H=8, G=2, D=64, Dv=64),
+    dict(portions=[(0, 150), (200, 9)], H=8, G=2, D=128, Dv=136, cap=5.0, slopes=1, gate=1, window=90),
+    dict(portions=[(0, 150)], H=16, G=2, D=72, Dv=64, prob=True, PS=5),
+    dict(portions=[(140, 10)], H=8, G=2, D=64, Dv=64, splits=2, sinks=True),
+    dict(portions=[(59, 1), (127, 1), (300, 1)], H=16, G=2, D=128, Dv=128, single=2),
+]
+
+
+@pytest.mark.parametrize("where", ["query", "key", "value"])
+@pytest.mark.parametrize("form", range(len(INFINITE)))
+def test_infinities_follow_float32(form, where):
+    """An infinity in a query, key or value row gives what the float32 kernel gives: an infinite score is a weight of 0 (or a cap, or 0
+    and 1 under the sigmoid) or makes its row NaN, an infinite value with a weight is that infinity.  Where that is finite both
+    are within the sums' float32 error of each other."""
+    c = Case(seed=8, **INFINITE[form])
+    rng = np.random.default_rng(form)
+    if where == "query":                                 # a dimension in which the first half of the groups have keys of one sign
+        c.k[..., 5] = bf16(np.abs(c.k[..., 5]) + 0.01)
+        q = c.q[:, 4:].reshape(c.T, c.H, c.D)
+        q[::3, ::2, 5], q[1::3, 1::2, 5] = np.inf, -np.inf
+        c.q[:, 4:] = q.reshape(c.T, -1)
+        c.q[:, 4:][:, ::7] = bf16(c.q[:, 4:][:, ::7])    # elements whose smaller terms are 0
+    rows = [(0, j) for j in (2, 31, 57)]
+    for n, (s, j) in enumerate(rows):
+        pg, r = c.table[s][j // c.PS], j % c.PS
+        if where == "key":
+            c.k[pg, n % c.G, r, 3] = np.inf if n % 2 else -np.inf
+        if where == "value":
+            c.v[pg, :, r, 5 * n:5 * n + 9] = np.inf if n % 2 else -np.inf
+    new, c.single = c.run(False), 0                      # (the float32 kernel for one query per tile writes 0 for a NaN row)
+    old = c.run(True)
+    assert (np.isnan(old) == np.isnan(new)).all()
+    assert not np.isfinite(old).all() or where == "query" or c.prob or c.cap
+    inf = np.isinf(old)
+    assert (inf == np.isinf(new)).all() and (np.sign(old[inf]) == np.sign(new[inf])).all()
+    fin = np.isfinite(old)
+    assert fin.any() and np.abs(old[fin] - new[fin]).max() <= 2.0 ** -18 * (1 + np.abs(old[fin]).max())
