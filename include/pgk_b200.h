@@ -41,7 +41,12 @@ typedef struct {
     int max_smem_per_block;
 } pgk_device_props_t;
 int pgk_device_props(int device, pgk_device_props_t* out);
+/* The calls that synchronise (pgk_device_sync, pgk_stream_sync, pgk_event_sync) also fail, once each, when a bounded wait inside one of
+ * the library's kernels has run out: the kernel then returned with outputs that are not valid. */
 int pgk_device_sync(void);
+/* launches a kernel whose one wait runs out after limit_us (<= 100000) and writes 0 to *ran_out (device memory): shows that a wait
+ * ends, and that the next call that synchronises fails for it */
+int pgk_wait_probe(int limit_us, int32_t* ran_out, void* stream);
 int pgk_mem_info(size_t* free_bytes, size_t* total_bytes);
 
 int pgk_malloc(void** ptr, size_t bytes);            /* memory.cpp:29 cuMemAlloc */
@@ -104,7 +109,8 @@ int pgk_gemv_fp8_swiglu_bf16(const void* A, const void* Wg_nk, const void* Sg, c
 int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void* S, void* C, int M, int K, int N,
                          const void* bias, const void* residual, void* stream);
 
-/* 1 once a wait of the FP8 tensor-core GEMM ran out (its results are then undefined), else 0. */
+/* 1 in *out once a wait of the FP8 tensor-core GEMM ran out in this process (its results are then undefined), else 0.  The next call
+ * that synchronises (pgk_stream_sync, pgk_device_sync, pgk_event_sync) has failed or fails for it. */
 int pgk_gemm_fp8_wait_error(int* out);
 /* The same contract with NO CUDA-core work on the weight stream: raw E4M3 tiles by TMA (cp.async.bulk.tensor, 2-D tensor
  * map over the [N,K] matrix, 128-byte swizzle) straight into tcgen05.mma.kind::f8f6f4; the activations are split once
@@ -487,7 +493,7 @@ int pgk_gemm_rows_f32(const float* A, int lda, const int32_t* a_rows, const void
 int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
                         float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows, int total_rows,
                         int epilogue, float scale, float cap, void* stream);
-/* 1 in *out when a bounded wait inside those products ever ran out on this device (their outputs are then not valid) */
+/* the same for a bounded wait inside those products */
 int pgk_gemm_rows_wait_error(int* out);
 /* the same product for few rows (decoding): blocks of rows_per_block (<= 8) consecutive rows share the matrix
  * row_group[first row of the block] (NULL: matrix 0); the weights are streamed once per block of rows */
@@ -783,8 +789,7 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
                      long long c_batch, int M, int N, int K, int batch, int epilogue, float p0, float p1, const float* col_scale,
                      const void* aux, int aux_dtype, const int32_t* aux_rows, int aux_ld, int aux_off, int rows_per_block,
                      void* stream);
-/* 1 in *out when a bounded wait of the tensor-core prompt attention ever ran out on this device (2: its shared memory was not
- * where it needs it); its outputs are then not valid */
+/* the same for the tensor-core prompt attention (2: its shared memory was not where it needs it) */
 int pgk_seq_attention_wait_error(int* out);
 int pgk_seq_decode_heads_per_block(void);
 int pgk_seq_heads_per_block(int heads, int kv_heads);

@@ -45,9 +45,8 @@ struct F8TcParams {
     const uint16_t* S; uint16_t* C;
     const uint16_t* bias; const uint16_t* residual;
     int M, K, N, splits, kper, once;              // once: nobody reads the weights again
+    int* err;                                     // raised when a bounded wait runs out
 };
-
-__device__ int g_f8tc_wait_error = 0;
 
 // four e4m3 codes (one 32-bit word) -> four bf16 (two packed words), exact.  (The bits moved by integer instructions and a product
 // with 2^120 for the bias are slower, 55 -> 63 us at 14336 x 14336; with no conversion at all it would be 43.)
@@ -72,7 +71,7 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
     const uint32_t wb = smem_u32(w_bar), db = smem_u32(d_bar);
-    int* const err = &g_f8tc_wait_error;
+    int* const err = p.err;
     const int rank = blockIdx.x, n0 = blockIdx.y * kTcRows, m0 = blockIdx.z * NB, nkb_total = p.K / kTcBK;
     const int kb0 = rank * p.kper, nkb = max(0, min(nkb_total, kb0 + p.kper) - kb0);
 
@@ -313,6 +312,8 @@ int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
     p.splits = f8tc_splits((long long)tiles * mt, nkb);
     p.kper = (nkb + p.splits - 1) / p.splits;
     p.once = mt == 1;
+    p.err = wait_word(kWaitFp8);
+    PGK_REQUIRE(p.err, "gemm_fp8_tc failed: no pinned host memory");
     PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8_tc failed: the driver does not export cuTensorMapEncodeTiled");
     CUtensorMap wmap, amap;
     PGK_REQUIRE(tma_map_bytes_2d(&wmap, B, (uint64_t)p.K, (uint64_t)p.N, kTcBK, kTcRows) &&
@@ -379,8 +380,7 @@ extern "C" int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void*
 }
 
 extern "C" int pgk_gemm_fp8_wait_error(int* out) {
-    int v = 0;
-    PGK_CUDA(cudaMemcpyFromSymbol(&v, pgk::g_f8tc_wait_error, sizeof(int)));
-    *out = v;
+    PGK_CUDA(cudaDeviceSynchronize());
+    *out = pgk::wait_raised(pgk::kWaitFp8);
     return 0;
 }

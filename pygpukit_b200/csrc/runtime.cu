@@ -3,6 +3,7 @@
 // (memory.cpp, stream.cpp, event.cpp, cuda_graph.cpp, device.cpp); no driver-API context
 // juggling: one process = one GPU, CUDA runtime primary context.
 #include "common.cuh"
+#include "tc_common.cuh"
 #include "../../include/pgk_b200.h"
 
 #include <atomic>
@@ -104,6 +105,57 @@ static bool scratch_trim() {
     return any;
 }
 
+// ---- bounded waits
+static std::mutex g_wait_mu;
+static std::atomic<int*> g_wait_words{nullptr};
+static std::atomic<int> g_wait_seen[kWaitKinds];
+
+int* wait_word(WaitKind kind) {
+    int* w = g_wait_words.load(std::memory_order_acquire);
+    if (!w) {
+        std::lock_guard<std::mutex> lk(g_wait_mu);
+        w = g_wait_words.load(std::memory_order_relaxed);
+        if (!w) {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;      // no part of a capture
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            void* p = nullptr;
+            const cudaError_t e = cudaHostAlloc(&p, kWaitKinds * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
+            w = (int*)memset(p, 0, kWaitKinds * sizeof(int));
+            g_wait_words.store(w, std::memory_order_release);
+        }
+    }
+    return w + kind;
+}
+int wait_check() {
+    static const char* const what[kWaitKinds] = {"gemm_rows", "gemm_fp8_tc", "seq_attention", "wait_probe"};
+    int* w = g_wait_words.load(std::memory_order_acquire);
+    if (!w) return 0;
+    for (int k = 0; k < kWaitKinds; ++k) {
+        if (__atomic_load_n(w + k, __ATOMIC_RELAXED) == 0) continue;
+        const int v = __atomic_exchange_n(w + k, 0, __ATOMIC_ACQ_REL);
+        if (v == 0) continue;                                               // another thread reports it
+        g_wait_seen[k].store(v);
+        set_error("%s failed: %s; results since the last synchronisation are not valid", what[k],
+                  v == 2 ? "its shared memory is not where it needs it" : "a wait inside its kernel ran out");
+        return 1;
+    }
+    return 0;
+}
+int wait_raised(WaitKind kind) {
+    int* w = g_wait_words.load(std::memory_order_acquire);
+    const int now = w ? __atomic_load_n(w + kind, __ATOMIC_ACQUIRE) : 0;
+    return now ? now : g_wait_seen[kind].load();
+}
+
+__global__ void wait_probe_kernel(int* err, uint32_t limit_ns, int* out) {
+    __shared__ __align__(8) uint64_t bar;
+    mbar_init(&bar, 1);
+    mbar_fence_init();
+    *out = bar_wait(err, smem_u32(&bar), 0, limit_ns) ? 1 : 0;              // nobody arrives
+}
+
 }  // namespace pgk
 
 using namespace pgk;
@@ -144,6 +196,13 @@ int pgk_device_props(int device, pgk_device_props_t* out) {
 }
 int pgk_device_sync(void) {
     PGK_CUDA(cudaDeviceSynchronize());
+    return wait_check();
+}
+int pgk_wait_probe(int limit_us, int32_t* ran_out, void* stream) {
+    PGK_REQUIRE(limit_us > 0 && limit_us <= 100000, "wait_probe failed: the limit must be 1 ... 100000 us, got %d", limit_us);
+    int* err = wait_word(kWaitProbe);
+    PGK_REQUIRE(err, "wait_probe failed: no pinned host memory");
+    PGK_CUDA(launch(wait_probe_kernel, dim3(1), dim3(1), 0, S(stream), err, 1000u * (uint32_t)limit_us, ran_out));
     return 0;
 }
 int pgk_mem_info(size_t* free_bytes, size_t* total_bytes) {
@@ -206,7 +265,7 @@ int pgk_stream_destroy(void* stream) {
 }
 int pgk_stream_sync(void* stream) {
     PGK_CUDA(cudaStreamSynchronize(S(stream)));
-    return 0;
+    return wait_check();
 }
 int pgk_event_create(void** event) {
     cudaEvent_t e;
@@ -224,7 +283,7 @@ int pgk_event_record(void* event, void* stream) {
 }
 int pgk_event_sync(void* event) {
     PGK_CUDA(cudaEventSynchronize((cudaEvent_t)event));
-    return 0;
+    return wait_check();
 }
 int pgk_event_elapsed_ms(void* start, void* stop, float* ms) {
     PGK_CUDA(cudaEventElapsedTime(ms, (cudaEvent_t)start, (cudaEvent_t)stop));

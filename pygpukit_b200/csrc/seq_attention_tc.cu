@@ -55,9 +55,8 @@ struct TcAttnArgs {
     uint32_t tmem_cols;
     int qvec;                // query rows keep 16-byte boundaries
     int bp;                  // positions per TMA copy (a power of two that divides the page), 0: cp.async
+    int* err;                // raised when a bounded wait runs out
 };
-
-__device__ int g_attn_wait_error = 0;
 
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(bytes) : "memory");
@@ -126,7 +125,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     float2* rowi = (float2*)(tail_p + 640);              // [32 rows] position, slope
     int* rowo = (int*)(tail_p + 896);                    // [32 rows] query << 16 | head of the row, -1: nobody's
     if (q_s & 1023u) {                                   // the layout relies on it (uniform over the grid)
-        if (tid == 0) atomicExch(&g_attn_wait_error, 2);
+        if (tid == 0) *(volatile int*)p.err = 2;
         return;
     }
 
@@ -155,7 +154,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     const int ntile = nkept + (jhi - jal) / AK + 1, per = (ntile + a.splits - 1) / a.splits;
     const int tbeg = (int)blockIdx.z * per, tend = min(ntile, tbeg + per), n = max(0, tend - tbeg);
     const int nv2 = 2 * p.ndv;
-    int* const err = &g_attn_wait_error;
+    int* const err = p.err;
 
     if (warp != A_SOFT) {
         // ---------------- queries, beside the first copies: rows 32 t + r of chunk c hold term t of row r's elements 64 c ... 64 c + 63
@@ -725,6 +724,8 @@ int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served
         if (tma_map_bf16_2d(&kmap, a.kc, (uint64_t)a.D, rows, (uint64_t)a.kld * 2, 64, (uint32_t)bp) &&
             tma_map_bf16_2d(&vmap, a.vc, (uint64_t)a.Dv, rows, (uint64_t)a.vld * 2, 64, (uint32_t)bp)) p.bp = bp;
     }
+    p.err = wait_word(kWaitAttention);
+    PGK_REQUIRE(p.err, "seq_attention failed: no pinned host memory");
     *served = true;
     switch ((a.cap > 0.f ? 1 : 0) + (a.slopes2 ? 4 : (a.slopes ? 2 : 0)) + (a.prob ? 6 : 0)) {
         case 0: return launch_form<false, 0, false>(p, kmap, vmap, tiles, smem, st);
@@ -745,8 +746,7 @@ int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served
 }  // namespace pgk
 
 extern "C" int pgk_seq_attention_wait_error(int* out) {
-    int v = 0;
-    PGK_CUDA(cudaMemcpyFromSymbol(&v, pgk::g_attn_wait_error, sizeof(int)));
-    *out = v;
+    PGK_CUDA(cudaDeviceSynchronize());
+    *out = pgk::wait_raised(pgk::kWaitAttention);
     return 0;
 }

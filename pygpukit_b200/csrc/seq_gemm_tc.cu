@@ -47,9 +47,8 @@ struct TcArgs {
     int stages;
     uint32_t stage_bytes;
     int splits;          // blocks per tile (cluster size)
+    int* err;            // raised when a bounded wait runs out (never, unless a copy or a product is lost)
 };
-
-__device__ int g_tc_wait_error = 0;        // a bounded wait ran out (never, unless a copy or a product is lost)
 
 // ---------------------------------------------------------------- activations -> bfloat16 rows [r][batch][K]
 // Memory: reads 4 and writes 2 bytes per element; 16-byte accesses both ways.  2000 x 2048: 4.0 us warm, 6.0 us from HBM.
@@ -248,7 +247,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 const uint32_t bytes = TC_W_BYTES + (uint32_t)(boxes * p.abox) * (TBK * 2);
                 for (int kb = kb0; kb < kb1; ++kb, ++i, r.next(p.stages)) {
                     const uint32_t fb = full + 8u * r.s, dst = ring + r.s * p.stage_bytes;
-                    if (!bar_wait(&g_tc_wait_error, empty + 8u * r.s, r.round ^ 1u)) { ok = false; break; }
+                    if (!bar_wait(p.err, empty + 8u * r.s, r.round ^ 1u)) { ok = false; break; }
                     mbar_expect_tx(fb, bytes);
                     tma_load_3d(dst, &wmap, kb * TBK, w.n0, w.z, fb);
                     for (int b = 0; b < boxes; ++b)
@@ -256,7 +255,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 }
             }
             if (!ok)                              // do not leave with copies in flight
-                for (int j = max(0, i - p.stages); j < i; ++j) bar_wait(&g_tc_wait_error, smem_u32(&full_bar[j % p.stages]), (uint32_t)((j / p.stages) & 1));
+                for (int j = max(0, i - p.stages); j < i; ++j) bar_wait(p.err, smem_u32(&full_bar[j % p.stages]), (uint32_t)((j / p.stages) & 1));
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -267,10 +266,10 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             for (int t = first; ok && t < total; t += step, ++u) {
                 const Tile w = tile_at(p, pre, t);
                 const uint32_t idesc = umma_idesc_bf16((w.rows + 15) & ~15), acc = tmem + (uint32_t)(u & 1) * TC_ROWS_MAX;
-                if (!bar_wait(&g_tc_wait_error, smem_u32(&drained_bar[u & 1]), (uint32_t)(((u >> 1) & 1) ^ 1))) break;
+                if (!bar_wait(p.err, smem_u32(&drained_bar[u & 1]), (uint32_t)(((u >> 1) & 1) ^ 1))) break;
                 tc_fence_after();
                 for (int kb = kb0; kb < kb1; ++kb, r.next(p.stages)) {
-                    if (!bar_wait(&g_tc_wait_error, full + 8u * r.s, r.round)) { ok = false; break; }
+                    if (!bar_wait(p.err, full + 8u * r.s, r.round)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t addr = ring + r.s * p.stage_bytes;
                     const uint64_t dw = desc_sw128(addr), da = desc_sw128(addr + TC_W_BYTES);
@@ -288,7 +287,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         int u = 0;
         for (int t = first; t < total; t += step, ++u) {
             const Tile w = tile_at(p, pre, t);
-            if (!__all_sync(0xffffffffu, bar_wait(&g_tc_wait_error, smem_u32(&done_bar[u & 1]), (uint32_t)((u >> 1) & 1)))) break;
+            if (!__all_sync(0xffffffffu, bar_wait(p.err, smem_u32(&done_bar[u & 1]), (uint32_t)((u >> 1) & 1)))) break;
             tc_fence_after();
             const uint32_t acc = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(u & 1) * TC_ROWS_MAX;
             const int col = w.n0 + quad * 32 + lane;
@@ -359,6 +358,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
 struct FewArgs {
     GemmArgs g;
     int epi, th, nkb, kper, splits, rpb, avec;
+    int* err;
 };
 
 __device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* row, int k, bool vec) {
@@ -403,7 +403,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             const uint32_t bytes = (uint32_t)p.th * (TBK * 2);
             const uint64_t once = l2_evict_first();
             for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
-                if (!bar_wait(&g_tc_wait_error, empty + 8u * r.s, r.round ^ 1u)) break;
+                if (!bar_wait(p.err, empty + 8u * r.s, r.round ^ 1u)) break;
                 mbar_expect_tx(full + 8u * r.s, bytes);
                 tma_load_3d_hint(ring + r.s * FEW_STAGE_BYTES, &wmap, kb * TBK, n0, z, full + 8u * r.s, once);
             }
@@ -414,7 +414,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             RingPos r;
             constexpr uint32_t idesc = umma_idesc_bf16(TC_DIRECT_ROWS);
             for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
-                if (!bar_wait(&g_tc_wait_error, full + 8u * r.s, r.round)) break;
+                if (!bar_wait(p.err, full + 8u * r.s, r.round)) break;
                 tc_fence_after();
                 const uint32_t addr = ring + r.s * FEW_STAGE_BYTES;
                 const uint64_t dw = desc_sw128(addr), da = desc_sw128(addr + TC_W_BYTES);
@@ -448,7 +448,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
 #pragma unroll
                 for (int d = d0; d < d0 + 4; ++d) {
                     if (d >= nb) break;
-                    ok = ok && bar_wait(&g_tc_wait_error, empty + 8u * f.s, f.round ^ 1u);
+                    ok = ok && bar_wait(p.err, empty + 8u * f.s, f.round ^ 1u);
                     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(at + f.s * FEW_STAGE_BYTES), "r"(pack_bf16x2(v[d].x, v[d].y)),
                                  "r"(pack_bf16x2(v[d].z, v[d].w)) : "memory");
                     f.next(FEW_STAGES);
@@ -461,7 +461,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         }
         const int quad = warp & 3, col = n0 + quad * 32 + lane;
         if (warp < 6) {                                   // four warps drain: lane = output column, v = the rows
-            bar_wait(&g_tc_wait_error, smem_u32(&done_bar), 0);
+            bar_wait(p.err, smem_u32(&done_bar), 0);
             __syncwarp();
             tc_fence_after();
             tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16), v);
@@ -628,6 +628,8 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
     p.kper = (p.nkb + p.splits - 1) / p.splits;
     p.rpb = own ? rows_per_block : 0;
     p.avec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
+    p.err = wait_word(kWaitRows);
+    PGK_REQUIRE(p.err, "gemm_rows failed: no pinned host memory");
     CUtensorMap wmap;
     if (!weight_map(&wmap, a, own ? 1u << 20 : (uint64_t)batch, many, p.th)) return 0;      // row groups name matrices that exist
     static bool configured = false;
@@ -654,6 +656,8 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
     p.g = a;
     p.epi = epilogue;
     p.batch = batch;
+    p.err = wait_word(kWaitRows);
+    PGK_REQUIRE(p.err, "gemm_rows failed: no pinned host memory");
     p.nt = (a.N + kTcRows - 1) / kTcRows;
     p.nkb = (a.K + TBK - 1) / TBK;
     if (grouped) {
@@ -716,8 +720,7 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
 }  // namespace pgk
 
 extern "C" int pgk_gemm_rows_wait_error(int* out) {
-    int v = 0;
-    PGK_CUDA(cudaMemcpyFromSymbol(&v, pgk::g_tc_wait_error, sizeof(int)));
-    *out = v;
+    PGK_CUDA(cudaDeviceSynchronize());
+    *out = pgk::wait_raised(pgk::kWaitRows);
     return 0;
 }

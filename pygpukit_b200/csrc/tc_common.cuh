@@ -63,15 +63,27 @@ __host__ __device__ constexpr uint32_t umma_idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kTcRows >> 4) << 24);
 }
 
-// Bounded wait: false, and *error set, when the phase never completes (a lost copy or product) -- the caller then leaves its loop.
-__device__ __forceinline__ bool bar_wait(int* error, uint32_t bar, uint32_t parity) {
-    for (int spin = 0; spin < (1 << 22); ++spin) {
+// Bounded wait: false, and *error (a wait_word) set, when the phase does not complete within the limit (a lost copy or product) -- the
+// caller then leaves its loop.
+constexpr uint32_t kWaitLimitNs = 1000000000u;
+__device__ __forceinline__ uint32_t global_ns() {         // wraps after 4.3 s: differences only
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+    return t;
+}
+__device__ __forceinline__ bool bar_wait(int* error, uint32_t bar, uint32_t parity, uint32_t limit_ns = kWaitLimitNs) {
+    uint32_t start = 0;
+    for (uint32_t spin = 0; spin < (1u << 30); ++spin) {
         uint32_t ok;
         asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
         if (ok) return true;
+        if ((spin & 255u) == 255u) {                      // the clock is read where a wait is long only
+            if (spin == 255u) start = global_ns();
+            else if (global_ns() - start > limit_ns) break;
+        }
     }
-    atomicExch(error, 1);
+    *(volatile int*)error = 1;
     return false;
 }
 // position in a ring of stages and the parity of its round
