@@ -120,8 +120,8 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
                 weights(it, r.s);
                 rows(it, r.s);
             }
-            if (it < nkb)                                     // given up: do not leave with copies in flight
-                for (int j = max(0, it - STAGES); j < it; ++j) bar_wait(err, full + 8u * (uint32_t)(j % STAGES), (uint32_t)((j / STAGES) & 1));
+            for (int j = max(0, it - STAGES); j < it; ++j)    // whoever gave up: do not leave with copies in flight
+                bar_wait(err, full + 8u * (uint32_t)(j % STAGES), (uint32_t)((j / STAGES) & 1));
         } else {
             griddep_wait();
             griddep_launch();

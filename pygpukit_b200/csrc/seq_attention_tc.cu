@@ -279,8 +279,8 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                     if (c + 2 >= nv2) clear(k - 2, below, above);
                 }
             }
-            if (!ok)                                      // do not leave with copies in flight
-                for (int j = max(0, k - A_RING); j < k; ++j) bar_wait(err, full_bar + 8u * (uint32_t)(j & (A_RING - 1)), (uint32_t)((j / A_RING) & 1));
+            for (int j = max(0, k - A_RING); j < k; ++j)  // whoever gave up: do not leave with copies in flight
+                bar_wait(err, full_bar + 8u * (uint32_t)(j & (A_RING - 1)), (uint32_t)((j / A_RING) & 1));
         } else {                                          // cp.async: eight lanes fetch one key's 128 bytes, zeros outside the run
             const int sub = lane >> 3, col16 = lane & 7;
             int cur[4], nxt[4] = {-1, -1, -1, -1};

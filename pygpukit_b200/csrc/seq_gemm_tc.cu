@@ -254,8 +254,8 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                         tma_load_3d(dst + TC_W_BYTES + (uint32_t)(b * p.abox) * (TBK * 2), &amap, kb * TBK, az, w.m0 + b * p.abox, fb);
                 }
             }
-            if (!ok)                              // do not leave with copies in flight
-                for (int j = max(0, i - p.stages); j < i; ++j) bar_wait(p.err, smem_u32(&full_bar[j % p.stages]), (uint32_t)((j / p.stages) & 1));
+            for (int j = max(0, i - p.stages); j < i; ++j)        // whoever gave up: do not leave with copies in flight
+                bar_wait(p.err, smem_u32(&full_bar[j % p.stages]), (uint32_t)((j / p.stages) & 1));
         }
         __syncwarp();
     } else if (warp == 1) {
@@ -402,11 +402,14 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             RingPos r;
             const uint32_t bytes = (uint32_t)p.th * (TBK * 2);
             const uint64_t once = l2_evict_first();
-            for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
+            int i = 0;                            // stages filled so far
+            for (int kb = kb0; kb < kb1; ++kb, ++i, r.next(FEW_STAGES)) {
                 if (!bar_wait(p.err, empty + 8u * r.s, r.round ^ 1u)) break;
                 mbar_expect_tx(full + 8u * r.s, bytes);
                 tma_load_3d_hint(ring + r.s * FEW_STAGE_BYTES, &wmap, kb * TBK, n0, z, full + 8u * r.s, once);
             }
+            for (int j = max(0, i - FEW_STAGES); j < i; ++j)      // whoever gave up: do not leave with copies in flight
+                bar_wait(p.err, full + 8u * (uint32_t)(j % FEW_STAGES), (uint32_t)((j / FEW_STAGES) & 1));
         }
         __syncwarp();
     } else if (rows > 0 && warp == 1) {
