@@ -9,7 +9,7 @@
 // What bounds it: the weights' way from HBM, and close behind it what an SM does per 128 x 128 block of them: the conversion of
 // 16384 codes and the traffic through its shared memory.  What follows from that:
 //   * the GEMM is computed transposed, D^T[n, m] = W[n, :] . A[m, :]: a block owns 128 weight rows (MMA M, a TMEM lane per row), the
-//     batch is the MMA's N (16 / 32 / 64 columns; more rows take further blocks);
+//     batch is the MMA's N (16 / 32 / 64 columns), so that every weight is read once, marked first to leave L2;
 //   * TMA brings codes and activations as they are (128-byte swizzle) into a ring; eight warps turn the codes into BF16 exactly and
 //     store them to TENSOR MEMORY, from where the MMA takes its A operand: through shared memory the BF16 form would be written
 //     and read once more, 128 KB per block of weights instead of 64, which alone is 1000 cycles against 680 for the HBM stream;
@@ -44,7 +44,7 @@ __host__ __device__ constexpr size_t f_smem(int nb) { return (size_t)f_stages(nb
 struct F8TcParams {
     const uint16_t* S; uint16_t* C;
     const uint16_t* bias; const uint16_t* residual;
-    int M, K, N, splits, kper, once;              // once: nobody reads the weights again
+    int M, K, N, splits, kper;
     int* err;                                     // raised when a bounded wait runs out
 };
 
@@ -72,7 +72,7 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
     const uint32_t wb = smem_u32(w_bar), db = smem_u32(d_bar);
     int* const err = p.err;
-    const int rank = blockIdx.x, n0 = blockIdx.y * kTcRows, m0 = blockIdx.z * NB, nkb_total = p.K / kTcBK;
+    const int rank = blockIdx.x, n0 = blockIdx.y * kTcRows, nkb_total = p.K / kTcBK;
     const int kb0 = rank * p.kper, nkb = max(0, min(nkb_total, kb0 + p.kper) - kb0);
 
     // the block's scales are weights: staged before the dependency wait
@@ -99,13 +99,12 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             const uint64_t once = l2_evict_first();
             auto weights = [&](int it, uint32_t s) {
                 mbar_expect_tx(full + 8u * s, STAGE);
-                if (p.once) tma_load_2d_hint(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s, once);
-                else tma_load_2d(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s);
+                tma_load_2d_hint(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s, once);
             };
             auto rows = [&](int it, uint32_t s) {
                 const uint32_t at = ring + s * STAGE + F_W_BYTES;
-                tma_load_2d(at, &amap, (kb0 + it) * kTcBK, m0, full + 8u * s);
-                tma_load_2d(at + NB * 128u, &amap, (kb0 + it) * kTcBK + 64, m0, full + 8u * s);
+                tma_load_2d(at, &amap, (kb0 + it) * kTcBK, 0, full + 8u * s);
+                tma_load_2d(at + NB * 128u, &amap, (kb0 + it) * kTcBK + 64, 0, full + 8u * s);
             };
             const int first = min(nkb, STAGES);
             for (int it = 0; it < first; ++it) weights(it, (uint32_t)it);
@@ -208,9 +207,9 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     }
 
     // ---------------- outputs
-    const int rows_here = min(NB, p.M - m0);
+    const int rows_here = min(NB, p.M);
     auto store = [&](float x, int m, int n) {
-        const size_t o = (size_t)(m0 + m) * p.N + n;
+        const size_t o = (size_t)m * p.N + n;
         if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[n]);
         p.C[o] = p.residual ? hadd_bf16_bits(x, p.residual[o]) : f32_to_bf16_bits(x);
     };
@@ -291,13 +290,13 @@ int f8tc_held(int s) {
 
 // Blocks per tile: an SM draws 24 bytes of weights per cycle when all do (HBM), and needs 600 cycles at least from one k block of a
 // block to its next; start and end cost 6000 cycles, half of it hidden where two blocks share an SM, an exchange 2000 more.
-int f8tc_splits(long long tiles, int nkb) {
+int f8tc_splits(int tiles, int nkb) {
     const int sms = sm_count();
     int best = 1;
     double best_cost = 1e30;
     for (int s = 1; s <= 8; ++s) {
         if (s > 1 && (nkb < 2 * s || f8tc_held(s) <= 0)) continue;
-        const long long blocks = tiles * s;
+        const int blocks = tiles * s;
         const int held = s == 1 ? 2 * sms : f8tc_held(s);
         const double rounds = (double)((blocks + held - 1) / held), per_sm = blocks <= sms ? 1.0 : fmin(2.0, (double)blocks / sms);
         const double cost = rounds * ((nkb + s - 1) / s) * fmax(per_sm * F_W_BYTES / 24.0, 600.0) + 6000.0 + (rounds - 1.0) * 3000.0 + (s > 1 ? 2000.0 : 0.0);
@@ -308,10 +307,9 @@ int f8tc_splits(long long tiles, int nkb) {
 
 template <int NB>
 int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
-    const int tiles = p.N / kTcRows, mt = (p.M + NB - 1) / NB, nkb = p.K / kTcBK;
-    p.splits = f8tc_splits((long long)tiles * mt, nkb);
+    const int tiles = p.N / kTcRows, nkb = p.K / kTcBK;
+    p.splits = f8tc_splits(tiles, nkb);
     p.kper = (nkb + p.splits - 1) / p.splits;
-    p.once = mt == 1;
     p.err = wait_word(kWaitFp8);
     PGK_REQUIRE(p.err, "gemm_fp8_tc failed: no pinned host memory");
     PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8_tc failed: the driver does not export cuTensorMapEncodeTiled");
@@ -321,7 +319,7 @@ int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
     PGK_CUDA(f8tc_config<NB>(&cfg, at, p.splits));
-    cfg.gridDim = dim3(p.splits, tiles, mt);
+    cfg.gridDim = dim3(p.splits, tiles);
     cfg.stream = st;
     if (pdl_enabled()) {
         at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -336,9 +334,10 @@ int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
 
 bool gemm_fp8_tc_shape_ok(int M, int K, int N, const void* A, const void* B);
 
-// Smallest batch sent to the tensor cores.  The copies zero-fill rows M..NB-1, so any M >= 1 works; the crossover
-// against the CUDA-core slab GEMV (whose time grows linearly with M: dequant + M FMAs per weight) measured on
-// B200 is between M = 4 (15.9 us GEMV vs ~16 us here, qkv shape) and M = 5.  PGK_TC_MIN_M overrides (A/B timing).
+// Smallest batch sent to the tensor cores.  The copies zero-fill rows M..NB-1, so any M >= 1 works.  Up to four rows share one pass of the
+// CUDA-core GEMV and get the bits of one row alone, which batches of that size are promised; from three rows on this kernel would be
+// faster (us, GEMV / here: 4096 x 4096 M = 2 10.5 / 10.5, M = 3 14.1 / 10.5, M = 4 16.3 / 10.5; 14336 x 4096 20.8 / 20.7, 24.9 / 20.7, 30.4 /
+// 20.7), and from five on the GEMV takes a second pass.  PGK_TC_MIN_M overrides (A/B timing).
 int gemm_fp8_tc_min_m() {
     static const int v = [] { const char* e = getenv("PGK_TC_MIN_M"); int m = e ? atoi(e) : 5; return m < 1 ? 1 : m; }();
     return v;
