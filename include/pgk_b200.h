@@ -791,6 +791,9 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
                      void* stream);
 /* the same for the tensor-core prompt attention (2: its shared memory was not where it needs it) */
 int pgk_seq_attention_wait_error(int* out);
+/* 1 when the tensor-core attention serves such rows of an aligned cache whose requests have at most `positions` positions (pages x page
+ * size), else 0: single_query 2 and prompts then take the float32 kernels */
+int pgk_seq_attention_tensor(int dim, int vdim, int k_ld, int v_ld, int heads, int kv_heads, int cache_dtype, long long positions);
 int pgk_seq_decode_heads_per_block(void);
 int pgk_seq_heads_per_block(int heads, int kv_heads);
 int pgk_seq_queries_per_tile(int heads, int kv_heads);

@@ -699,12 +699,19 @@ int launch_form(const TcAttnArgs& p, const CUtensorMap& kmap, const CUtensorMap&
     return 0;
 }
 
+size_t smem_bytes(int D) { return (size_t)((D + 63) / 64) * A_QCHUNK + A_PBYTES + A_RING * A_CHUNK + A_TAIL; }
+
+// Copies of 16 bytes from rows of the cache; at most 512 value elements (TMEM) and 704 key elements (shared memory); positions are
+// compared as float32, which holds whole numbers to 2^24.
+bool sizes_fit(int D, int Dv, int kld, int vld, int HB, long long positions) {
+    return D % 8 == 0 && Dv % 8 == 0 && kld % 8 == 0 && vld % 8 == 0 && Dv <= 512 && HB <= AR && smem_bytes(D) <= 227 * 1024 && positions <= 1 << 24;
+}
+
 }  // namespace
 
 int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served) {
     *served = false;
-    // copies of 16 bytes from rows of the cache; at most 512 value elements (TMEM) and 704 key elements (shared memory)
-    if (a.D % 8 || a.Dv % 8 || a.kld % 8 || a.vld % 8 || (uintptr_t)a.kc % 16 || (uintptr_t)a.vc % 16 || a.Dv > 512 || a.HB > AR) return 0;
+    if (!sizes_fit(a.D, a.Dv, a.kld, a.vld, a.HB, (long long)a.max_pages * a.PS) || (uintptr_t)a.kc % 16 || (uintptr_t)a.vc % 16) return 0;
     if (a.splits > 1 && (uintptr_t)a.ws % 8) return 0;    // the fold reads pairs
     TcAttnArgs p{};
     p.a = a;
@@ -713,8 +720,7 @@ int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served
     p.ndv = (a.Dv + 127) / 128;
     p.tmem_cols = AN + AN * p.ndv <= 256 ? 256 : 512;
     p.qvec = a.ld % 4 == 0 && a.q_off % 4 == 0 && (uintptr_t)a.proj % 16 == 0;
-    const size_t smem = (size_t)p.nd * A_QCHUNK + A_PBYTES + A_RING * A_CHUNK + A_TAIL;
-    if (smem > 227 * 1024) return 0;
+    const size_t smem = smem_bytes(a.D);
     // copies of bp positions: the largest power of two that divides a page
     CUtensorMap kmap{}, vmap{};
     int bp = a.PS & -a.PS;
@@ -745,6 +751,9 @@ int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served
 
 }  // namespace pgk
 
+extern "C" int pgk_seq_attention_tensor(int dim, int vdim, int k_ld, int v_ld, int heads, int kv_heads, int cache_dtype, long long positions) {
+    return cache_dtype == 2 && dim > 0 && vdim > 0 && pgk::sizes_fit(dim, vdim, k_ld, v_ld, pgk_seq_heads_per_block(heads, kv_heads), positions) ? 1 : 0;
+}
 extern "C" int pgk_seq_attention_wait_error(int* out) {
     PGK_CUDA(cudaDeviceSynchronize());
     *out = pgk::wait_raised(pgk::kWaitAttention);

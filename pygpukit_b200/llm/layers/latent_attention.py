@@ -70,7 +70,7 @@ class LatentAttentionMixer:
 
     def key_slices(self, ctx) -> int:
         return key_slices(ctx, self.spec.heads, 1, 0, self.spec.window, self.queries_per_tile, self.heads_per_block, self.decode_heads_per_block,
-                          tensor_dims=(self.row, self.spec.kv_rank))
+                          tensor_dims=(self.row, self.spec.kv_rank, self.row, self.row))
 
     def forward(self, ctx, x: GPUArray, out: GPUArray, cache_index: int | None = None, out_scale: int | None = None) -> None:
         """x [T, W] (the block's normed rows) -> out [T, W]: stored, or out += out_scale * result when out_scale (device

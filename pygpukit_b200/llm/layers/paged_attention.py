@@ -41,12 +41,13 @@ def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_
                decode_heads_per_block: int, keep_first: int = 0, pool: int = 0, tensor_dims: "tuple[int, int] | None" = None) -> int:
     """Few long tiles (decoding over a long context): the key range of every tile is cut into this many slices so that the
     whole GPU reads the cache.  A power of two, so that a decode step's launch shapes change rarely.
-    tensor_dims: (key row, value row) of a mixer that the tensor-core kernel can serve; TENSOR is added where decoding takes it."""
+    tensor_dims: (key, value) elements, then elements from row to row of either, of a mixer whose form of attention the tensor-core
+    kernel has; TENSOR is added where decoding takes it."""
     n_tiles = ctx.tiles(queries_per_tile)[1]
     rep = heads // kv_heads
     keys = ctx.max_keys(chunk, window, keep_first, pool)
     tensor = 0
-    if ctx.decode_only and tensor_dims and _tensor_decode(ctx, n_tiles, heads, keys, *tensor_dims):
+    if ctx.decode_only and tensor_dims and _tensor_decode(ctx, n_tiles, heads, kv_heads, keys, *tensor_dims):
         tensor = TENSOR          # tiles of 128 keys, one block per SM (two shared ones are slower: 24 -> 29 us at 8 x 1024 keys)
         blocks = n_tiles * kv_heads * -(-rep // min(rep, heads_per_block))
         want = max(1, min(64, -(-keys // 128), 148 // max(1, blocks)))
@@ -63,13 +64,14 @@ def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_
     return min(64, 1 << (want - 1).bit_length()) + tensor
 
 
-def _tensor_decode(ctx, n_tiles: int, heads: int, keys: int, dim: int, vdim: int) -> bool:
+def _tensor_decode(ctx, n_tiles: int, heads: int, kv_heads: int, keys: int, dim: int, vdim: int, key_row: int, value_row: int) -> bool:
     """Where one query per request belongs on the tensor cores (bfloat16 caches).  The float32 kernel pays per (head, key) for a
     row's every element, 23 us + heads * keys * (dim + vdim) / 2.5e6; the tensor cores for tiles of 128 keys whatever the heads, and
     for the chunks of a row one after the other.  Rows of 128 (16 heads, 4 groups): 16 us against 23 over 60 keys, 24 against 65 us for
     8 requests over 1024.  Latent rows of 576 / 512: 48 against 37 us for one request over 2000 keys, 50 against 129 for eight, 40 against
     58 for 24 over 200: the line lies at 2^26 element products."""
-    if ctx.cache.dtype_code != 2 or vdim > 512:
+    cache = ctx.cache
+    if not api.seq_attention_tensor(dim, vdim, key_row, value_row, heads, kv_heads, cache.dtype_code, cache.pool.max_pages * cache.page_size):
         return False
     return vdim <= 128 or n_tiles * heads * keys * (dim + vdim) >= 1 << 26
 
@@ -153,7 +155,7 @@ class PagedAttentionMixer:
     def key_slices(self, ctx) -> int:
         s = self.spec
         return key_slices(ctx, s.heads, s.kv_heads, s.chunk, s.window, self.queries_per_tile, self.heads_per_block,
-                          self.decode_heads_per_block, s.keep_first, s.pool, None if s.pool or s.rot_values else (s.dim, s.vdim))
+                          self.decode_heads_per_block, s.keep_first, s.pool, None if s.pool or s.rot_values else (s.dim, s.vdim, s.dim, s.vdim))
 
     def forward(self, ctx, x: GPUArray, out: GPUArray, cache_index: int | None = None, out_scale: int | None = None,
                 state=None) -> None:
