@@ -41,6 +41,7 @@ typedef struct {
     int max_smem_per_block;
 } pgk_device_props_t;
 int pgk_device_props(int device, pgk_device_props_t* out);
+int pgk_sm_count(void);               /* multiprocessors of the current device (148 without one); not an error code */
 /* The calls that synchronise (pgk_device_sync, pgk_stream_sync, pgk_event_sync) also fail, once each, when a bounded wait inside one of
  * the library's kernels has run out: the kernel then returned with outputs that are not valid. */
 int pgk_device_sync(void);

@@ -194,6 +194,7 @@ int pgk_device_props(int device, pgk_device_props_t* out) {
     out->max_smem_per_block = (int)p.sharedMemPerBlockOptin;
     return 0;
 }
+int pgk_sm_count(void) { return sm_count(); }
 int pgk_device_sync(void) {
     PGK_CUDA(cudaDeviceSynchronize());
     return wait_check();

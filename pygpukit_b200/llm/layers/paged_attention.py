@@ -24,6 +24,8 @@ launch reads those rows for everything that lies before the window.
 """
 from __future__ import annotations
 
+from math import isqrt
+
 import numpy as np
 
 from ..._lib import api
@@ -38,7 +40,7 @@ TENSOR = 256                 # added to a number of key slices (at most 64): dec
 
 
 def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_per_tile: int, heads_per_block: int,
-               decode_heads_per_block: int, keep_first: int = 0, pool: int = 0, tensor_dims: "tuple[int, int] | None" = None) -> int:
+               decode_heads_per_block: int, keep_first: int = 0, pool: int = 0, tensor_dims: "tuple[int, int, int, int] | None" = None) -> int:
     """Few long tiles (decoding over a long context): the key range of every tile is cut into this many slices so that the
     whole GPU reads the cache.  A power of two, so that a decode step's launch shapes change rarely.
     tensor_dims: (key, value) elements, then elements from row to row of either, of a mixer whose form of attention the tensor-core
@@ -47,10 +49,19 @@ def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_
     rep = heads // kv_heads
     keys = ctx.max_keys(chunk, window, keep_first, pool)
     tensor = 0
-    if ctx.decode_only and tensor_dims and _tensor_decode(ctx, n_tiles, heads, kv_heads, keys, *tensor_dims):
-        tensor = TENSOR          # tiles of 128 keys, one block per SM (two shared ones are slower: 24 -> 29 us at 8 x 1024 keys)
-        blocks = n_tiles * kv_heads * -(-rep // min(rep, heads_per_block))
-        want = max(1, min(64, -(-keys // 128), 148 // max(1, blocks)))
+    if ctx.decode_only and tensor_dims and _tensor_decode(ctx, n_tiles, heads, kv_heads, min(rep, heads_per_block), keys, *tensor_dims):
+        # Tiles of 128 keys.  Value rows of up to 128: about a block per SM, rounded up to a power of two, since two fit one (us: 48
+        # blocks over 4096 keys in 2 / 4 slices 34.7 / 27.0, 8 blocks over 4096 in 16 / 32 16.1 / 16.8; twice as many are slower, 24 -> 29 at
+        # 8 x 1024 keys).  Longer ones fill an SM's tensor memory: never more blocks than SMs (24 requests of 512 elements over
+        # 1024 keys, 4 / 8 slices: 31.2 / 47.2; 8 over 4096, 16 / 32: 40.6 / 63.9), and a slice costs in the fold what its tiles save:
+        # sqrt(8 tiles) slices (one request, 16 heads, over 2000 keys 8 / 16: 35.2 / 37.1, over 16384 16 / 32 / 64: 64 / 58 / 74).
+        tensor, tiles, sms = TENSOR, -(-keys // 128), api.sm_count()
+        room = sms // max(1, n_tiles * kv_heads * -(-rep // min(rep, heads_per_block)))
+        if tensor_dims[1] > 128:
+            want = max(1, min(64, isqrt(8 * tiles), room)) if tiles > 2 else 1
+            want = 1 << (want.bit_length() - 1)
+        else:
+            want = max(1, min(64, tiles, room))
     elif ctx.decode_only:        # the decoding kernel: eight warps take 32 keys each per round
         blocks = n_tiles * kv_heads * -(-rep // decode_heads_per_block)
         want = max(1, min(64, -(-keys // 256), 592 // max(1, blocks)))
@@ -64,16 +75,17 @@ def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_
     return min(64, 1 << (want - 1).bit_length()) + tensor
 
 
-def _tensor_decode(ctx, n_tiles: int, heads: int, kv_heads: int, keys: int, dim: int, vdim: int, key_row: int, value_row: int) -> bool:
+def _tensor_decode(ctx, n_tiles: int, heads: int, kv_heads: int, rows: int, keys: int, dim: int, vdim: int, key_row: int, value_row: int) -> bool:
     """Where one query per request belongs on the tensor cores (bfloat16 caches).  The float32 kernel pays per (head, key) for a
-    row's every element, 23 us + heads * keys * (dim + vdim) / 2.5e6; the tensor cores for tiles of 128 keys whatever the heads, and
-    for the chunks of a row one after the other.  Rows of 128 (16 heads, 4 groups): 16 us against 23 over 60 keys, 24 against 65 us for
-    8 requests over 1024.  Latent rows of 576 / 512: 48 against 37 us for one request over 2000 keys, 50 against 129 for eight, 40 against
-    58 for 24 over 200: the line lies at 2^26 element products."""
+    row's every element; the tensor cores for tiles of 128 keys whatever the heads, and for the chunks of a row one after the other.
+    Value rows of up to 128: always (us, float32 / tensor: 16 heads in 4 groups, one request over 60 keys 14.7 / 8.7, eight over 1024 28.9 /
+    14.8; 16 heads with keys of their own 18.9 / 8.7 and 83 / 18.8).  Latent rows of 576 / 512: from 2^26 element products on, 2^27 where
+    a block serves more than 16 heads (16 heads, one request over 2000 / 4096 / 8192 keys: 37.3 / 35.2, 39.5 / 39.4, 72 / 47.5; eight over 250 /
+    500: 32.3 / 25, 37.5 / 29.1; 32 heads, one over 2000 / 4096: 37.3 / 44.2, 68 / 53.5)."""
     cache = ctx.cache
     if not api.seq_attention_tensor(dim, vdim, key_row, value_row, heads, kv_heads, cache.dtype_code, cache.pool.max_pages * cache.page_size):
         return False
-    return vdim <= 128 or n_tiles * heads * keys * (dim + vdim) >= 1 << 26
+    return vdim <= 128 or n_tiles * heads * keys * (dim + vdim) >= (1 << 27 if rows > 16 else 1 << 26)
 
 
 class PagedAttentionMixer:

@@ -29,3 +29,21 @@ def test_what_the_tensor_form_refuses_is_cut_for_the_float32_form(requests, keys
 def test_what_it_serves_takes_it(dims):
     assert slices(step(8, 1024), 16, 4, dims) >= TENSOR
     assert slices(step(8, 1024, page_size=1 << 12, max_pages=1 << 12), 16, 4, dims) >= TENSOR
+
+
+@pytest.mark.parametrize("heads,dims", [(16, (576, 512, 576, 576)), (32, (320, 256, 320, 320)), (8, (256, 256, 256, 256))])
+@pytest.mark.parametrize("requests", [1, 2, 7, 10, 24, 73, 75, 148, 200])
+def test_long_value_rows_take_an_sm_each(requests, heads, dims):
+    """blocks that fill an SM's tensor memory never outnumber the SMs because of the slices, and slices are a power of two"""
+    for keys in (300, 1024, 4096, 1 << 15):
+        s = slices(step(requests, keys, max_pages=1 << 10), heads, 1 if dims[0] > 256 else 2, dims)
+        if s >= TENSOR:
+            s -= TENSOR
+            blocks = requests * (1 if dims[0] > 256 else 2)
+            assert s & (s - 1) == 0 and 1 <= s <= 64 and (s == 1 or blocks * s <= 148)
+
+
+def test_few_requests_of_many_latent_heads_stay_in_float32():
+    dims = (576, 512, 576, 576)
+    assert slices(step(1, 2000), 32, 1, dims) < TENSOR <= slices(step(1, 4096), 32, 1, dims)
+    assert slices(step(1, 2000), 16, 1, dims) < TENSOR <= slices(step(2, 2000), 16, 1, dims)
