@@ -293,3 +293,55 @@ def test_rows_beyond_n_with_shared_k(M, N, K, epi):
         ref, tol = old + cs * z, tol * np.abs(cs)
     assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6 * (1 + np.abs(ref))).all()
     no_wait_error()
+
+
+@pytest.fixture
+def programmatic_launch():
+    api.set_pdl(1)
+    yield
+    api.set_pdl(0)
+
+
+def chain(ws, x, bufs, rows):
+    """x -> w0 -> w1 -> ... and back into x's shape, every product reading what the one before wrote"""
+    for _ in range(2):
+        src, k = x, ws[0].shape[1]
+        for w, b in zip(ws, bufs):
+            llm.LinearRows(w).forward(src.device_ptr, k, rows, b.device_ptr, w.shape[0])
+            src, k = b, w.shape[0]
+    return src
+
+
+@pytest.mark.parametrize("rows", [8, 16, 17, 60, 300, 1500])
+def test_chained_products_under_programmatic_launch(rows, programmatic_launch):
+    """the activations' rounding lets its dependents start early, clusters carry the launch attribute, work memory goes from product to
+    product: the bits are those of plain launches, eagerly and in a replayed graph"""
+    from pygpukit_b200.core.stream import CudaGraph, Stream
+    sizes = [512, 2048, 264, 1536, 520, 512]
+    rng = np.random.default_rng(rows)
+    ws = [dev_w(bf16(rng.standard_normal((n, k)) / np.sqrt(k))) for k, n in zip(sizes, sizes[1:])]
+    x = gk.from_numpy(rng.standard_normal((rows, sizes[0])).astype(np.float32))
+
+    def buffers():
+        return [gk.zeros((rows, n), gk.float32) for n in sizes[1:]]
+
+    api.set_pdl(0)
+    plain = buffers()
+    chain(ws, x, plain, rows)
+    ref = [b.to_numpy() for b in plain]
+    api.set_pdl(1)
+    for _ in range(5):
+        got = buffers()
+        chain(ws, x, got, rows)
+        assert all((a == b.to_numpy()).all() for a, b in zip(ref, got))
+    st, g, got = Stream(), CudaGraph(), buffers()
+    with g.capture(st):
+        chain(ws, x, got, rows)
+    for _ in range(3):
+        for b in got:
+            b.copy_from_numpy(np.zeros(b.shape, np.float32))
+        g.replay(st)
+        st.synchronize()
+        assert all((a == b.to_numpy()).all() for a, b in zip(ref, got))
+    assert np.isfinite(ref[-1]).all() and np.abs(ref[-1]).max() > 0
+    no_wait_error()
