@@ -77,7 +77,7 @@ def _run_world(world: int) -> dict:
     err = r.stderr
     i = err.find("Traceback")
     out["_rc"], out["_tail"] = r.returncode, (r.stdout[-1500:] + (err[i:i + 3000] if i >= 0 else err[-2500:]))
-    log = os.path.join(ROOT, "gpurun_out")
+    log = os.environ.get("PGK_TEST_LOGS", "")
     if os.path.isdir(log):
         with open(os.path.join(log, f"tp_worker_{world}gpu.err"), "w") as f:
             f.write(err[-20000:])

@@ -118,7 +118,7 @@ def test_shard_range_rejects_uneven():
 
 def test_shard_plan_rejects_vocabulary_remainder():
     """Equal lm_head shards only: the logits all-gather and the 16-byte (best logit, global index) exchange both assume
-    V / world rows per rank, so a vocabulary that does not divide is refused at plan time (ADVICE round 1, low)."""
+    V / world rows per rank, so a vocabulary that does not divide is refused at plan time."""
     cfg, _ = named_config("small-qwen3", max_seq=64)
     cfg.vocab_size = 2049
     with pytest.raises(ValueError, match="vocab_size"):
