@@ -135,11 +135,13 @@ struct LinPrepArgs {
 
 // units per token: H query heads, H key heads, H value heads; a warp takes every 8 gridDim.y-th of them.  A token's angles (a
 // product in float64 and a sine pair each) are taken once per block instead of once per head (a prompt of 2000 tokens: 41 -> 29 us).
+constexpr int LIN_TURNS = 4096;                           // angles that shared memory holds; longer heads take the rest per head
+
 __global__ void __launch_bounds__(256) linear_prep_kernel(LinPrepArgs a) {
-    extern __shared__ float2 turn[];                      // [rot_dims / 2] (sine, cosine)
+    extern __shared__ float2 turn[];                      // [min(rot_dims / 2, LIN_TURNS)] (sine, cosine)
     const int t = blockIdx.x, lane = threadIdx.x & 31, half = a.rot_dims / 2;
     const int pos = half ? a.pos[t] : 0;
-    for (int i = threadIdx.x; i < half; i += 256) {
+    for (int i = threadIdx.x; i < min(half, LIN_TURNS); i += 256) {
         float sn, cs;
         rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
         turn[i] = make_float2(sn, cs);
@@ -159,7 +161,9 @@ __global__ void __launch_bounds__(256) linear_prep_kernel(LinPrepArgs a) {
         for (int i = lane; i < half; i += 32) {
             float p0 = x[i], p1 = x[i + half];
             if (a.act) { p0 = silu_f(p0); p1 = silu_f(p1); }
-            const float sn = turn[i].x, cs = turn[i].y;
+            float sn, cs;
+            if (i < LIN_TURNS) { sn = turn[i].x; cs = turn[i].y; }
+            else rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
             x[i] = (p0 * cs - p1 * sn) * sc;
             x[i + half] = (p1 * cs + p0 * sn) * sc;
         }
@@ -529,7 +533,7 @@ int pgk_seq_linear_prep(float* proj, int ld, int tokens, int heads, int dim, int
     LinPrepArgs a{proj, ld, heads, dim, vdim, q_off, k_off, v_off, activation ? 1 : 0, rot_dims, inv_freq, k_scale, pos};
     // a unit per warp while that fills the SMs no more than once, then two blocks per token (angles twice instead of six times)
     const int all = (3 * heads + 7) / 8, groups = (long long)tokens * all <= 8 * sm_count() ? all : (all < 2 ? all : 2);
-    PGK_CUDA(launch(linear_prep_kernel, dim3(tokens, groups), dim3(256), (size_t)(rot_dims / 2) * sizeof(float2), (cudaStream_t)stream, a));
+    PGK_CUDA(launch(linear_prep_kernel, dim3(tokens, groups), dim3(256), sizeof(float2) * (rot_dims / 2 < LIN_TURNS ? rot_dims / 2 : LIN_TURNS), (cudaStream_t)stream, a));
     return 0;
 }
 

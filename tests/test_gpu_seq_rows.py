@@ -85,3 +85,26 @@ def test_router_logits(M, N, K):
     out = c.to_numpy()
     assert (np.abs(out[:, :N] - x @ y.T) <= 2.0 ** -24 * (K / 32 + 6) * (np.abs(x) @ np.abs(y).T)).all()
     assert (out[:, N:] == 7.0).all()
+
+
+@pytest.mark.parametrize("H,D,rot", [(1, 16400, 16400), (3, 8200, 8194), (4, 64, 0), (2, 96, 50)])
+def test_turned_heads_of_any_length(H, D, rot):
+    """heads with more pairs than the kernel's table of angles holds: silu and turn of q and k in float32 on float64 angles, two
+    products and a sum of values of about 1 and the table's roundings"""
+    T, Dv = 5, 24
+    rng = np.random.default_rng(D + rot)
+    ld = 2 * H * D + H * Dv
+    x = rng.standard_normal((T, ld)).astype(np.float32)
+    pos = np.array([0, 1, 77, 4095, 100000])
+    freq = 10000.0 ** (-np.arange(max(1, rot // 2)) / max(1, rot // 2))
+    p, fr, ps = f32(x), gk.from_numpy(freq), i32(pos)
+    api.seq_linear_prep(p.device_ptr, ld, T, H, D, Dv, 0, H * D, 2 * H * D, 1, rot, fr.device_ptr, 0.25, ps.device_ptr, None)
+    s = x.astype(np.float64) / (1 + np.exp(-x.astype(np.float64)))
+    qk = s[:, :2 * H * D].reshape(T, 2 * H, D).copy()
+    h = rot // 2
+    a = (pos[:, None] * freq[None, :h])[:, None]
+    lo, hi = qk[..., :h].copy(), qk[..., h:rot].copy()
+    qk[..., :h], qk[..., h:rot] = lo * np.cos(a) - hi * np.sin(a), hi * np.cos(a) + lo * np.sin(a)
+    qk[:, H:] *= 0.25
+    ref = np.concatenate([qk.reshape(T, -1), s[:, 2 * H * D:]], 1)
+    assert np.abs(p.to_numpy() - ref).max() <= 2.0 ** -20 * (1 + np.abs(s).max())
