@@ -392,12 +392,26 @@ __global__ void __launch_bounds__(FEW_MAX_WARPS * 32) gemm_few_rows_kernel(GemmA
     }
 }
 
-// bfloat16 weights go to the tcgen05 form (seq_gemm_tc.cu) whenever its copies can fetch the operands; `rows` bounds the rows of
-// A (-1: the groups' total is not known here).  The tiles below serve what is left: K no multiple of 8, matrices off
-// 16-byte boundaries, products of a few k steps, groups without a bound.
+// The tcgen05 form (seq_gemm_tc.cu) takes 10 us from the rounding of the rows to its last store, little more for more work; the tiles
+// below 4 us and 18 ns per k in a wave, again for every further wave.  Above 16 rows (which need no rounding pass) the line lies
+// where the two meet, by the tiles there are (us, tiles -> tcgen05): K = 64 5.2 -> 10.3 for one tile or 128, 12.4 -> 15.1 for 1024,
+// 42 -> 35 for 4608; K = 256 9.3 -> 10.4 for 128, 11.4 -> 10.5 for 256; K = 320 10.4 -> 10.4 for 32; K = 512 14.4 -> 12.4 for 4.  Groups: by
+// the tiles that have rows, groups of the mean length taken, and a little for the grid's empty ones: 32 tiles K = 384 10.4 -> 12.5, K =
+// 512 12.5 -> 12.5; 512 tiles K = 192 14.7 -> 16.5, K = 256 18.6 -> 16.5.
+inline bool many_tc_pays(const GemmArgs& a, int groups, int max_rows, int rows) {
+    const double nt = (a.N + BN - 1) / BN;
+    if (!a.group_off) return a.M <= 16 || a.K * ((double)groups * ((a.M + BM - 1) / BM) * nt + 512.0) >= 180000.0;
+    const int mean = (rows + groups - 1) / groups;
+    const double live = (double)groups * ((mean + BM - 1) / BM) * nt, grid = (double)groups * ((max_rows + BM - 1) / BM) * nt;
+    return a.K * (2.0 * live + 0.25 * grid + 1000.0) >= 500000.0;
+}
+
+// bfloat16 weights go to the tcgen05 form wherever it is faster and its copies can fetch the operands; `rows` bounds the rows of
+// A (-1: the groups' total is not known here).  The tiles below serve what is left: short k, K no multiple of 8, matrices off
+// 16-byte boundaries, groups without a bound.
 template <int EPI>
 int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream_t st, int rows = -1) {
-    if (wdt == 2 && rows >= 0) {
+    if (wdt == 2 && rows >= 0 && many_tc_pays(a, groups, max_rows, rows)) {
         bool served = false;
         if (const int rc = gemm_rows_tc(a, EPI, groups, rows, max_rows, st, &served)) return rc;
         if (served) return 0;
@@ -427,10 +441,13 @@ int launch_few_t(const GemmArgs& a, int rows_per_block, cudaStream_t st, int bat
 // from its first barrier to its last store; a warp per column pair starts faster and then costs time per row.  The line lies where
 // the two meet, rows^2 N K (matrices) = 2^24 (us, warp per pair -> tcgen05): one row of 2048 x 2048 7.4 -> 8.3, of 8192 x 2048
 // 11 -> 11, of 32768 x 2048 35 -> 25; eight rows of 512 x 2048 14.4 -> 8.0, 2048 x 8192 37 -> 14.5, 24576 x 4096 158 -> 37; eight
-// rows with matrices of their own, 4096 x 2048, 37 -> 14.5.
+// rows with matrices of their own, 4096 x 2048, 37 -> 14.5.  Up to 4096 columns the warps are one wave, whose time is its longest
+// warp's: four rows of 4096 x 512 6.3 -> 8.3, two of 4096 x 1024 6.3 -> 8.2, eight of 2048 x 128 5.2 -> 5.7, but eight of 4096 x 256 7.2 -> 6.0,
+// four of 2048 x 1024 8.3 -> 6.5, two of 4096 x 2048 10.4 -> 9.1: there rows^2 K must reach 2^14 as well, or K 2048 for two rows.
 inline bool few_tc_pays(const GemmArgs& a, int rows_per_block, int batch) {
     const double rows = a.row_group ? rows_per_block : a.M;
     const double matrices = a.row_group ? (a.M + rows_per_block - 1) / rows_per_block : batch;
+    if (matrices * a.N <= 4096.0 && rows * rows * a.K < 16384.0 && (rows < 2.0 || a.K < 2048)) return false;
     return rows * rows * matrices * (double)a.N * (double)a.K >= 16777216.0;
 }
 

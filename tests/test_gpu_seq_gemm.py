@@ -317,7 +317,7 @@ def test_chained_products_under_programmatic_launch(rows, programmatic_launch):
     """the activations' rounding lets its dependents start early, clusters carry the launch attribute, work memory goes from product to
     product: the bits are those of plain launches, eagerly and in a replayed graph"""
     from pygpukit_b200.core.stream import CudaGraph, Stream
-    sizes = [512, 2048, 264, 1536, 520, 512]
+    sizes = [512, 2048, 648, 1536, 520, 512]             # every product on tcgen05
     rng = np.random.default_rng(rows)
     ws = [dev_w(bf16(rng.standard_normal((n, k)) / np.sqrt(k))) for k, n in zip(sizes, sizes[1:])]
     x = gk.from_numpy(rng.standard_normal((rows, sizes[0])).astype(np.float32))
@@ -344,4 +344,33 @@ def test_chained_products_under_programmatic_launch(rows, programmatic_launch):
         st.synchronize()
         assert all((a == b.to_numpy()).all() for a, b in zip(ref, got))
     assert np.isfinite(ref[-1]).all() and np.abs(ref[-1]).max() > 0
+    no_wait_error()
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 7, 648), (33, 257, 520), (64, 128, 456), (128, 129, 392), (129, 1023, 1032), (257, 640, 448), (272, 384, 1000), (1999, 272, 456)])
+def test_rows_of_longer_k(M, N, K):
+    """the tile heights, column tails and k tails of test_rows where the product runs on tcgen05"""
+    test_rows(M, N, K)
+
+
+@pytest.mark.parametrize("counts,N,K", [([30, 0, 70, 1, 9], 130, 712), ([300, 16, 0, 17, 257, 1], 256, 640), ([0, 0, 5], 64, 584),
+                                        ([1] * 40, 96, 640), ([0] * 7, 96, 640), ([3, 129] * 20, 64, 520)])
+@pytest.mark.parametrize("extra", [0, 50])
+def test_groups_of_longer_k(counts, N, K, extra):
+    test_groups(counts, N, K, extra)
+
+
+@pytest.mark.parametrize("M,H,N,K,pad", [(40, 3, 96, 512, 0), (70, 5, 512, 384, 8), (260, 2, 130, 456, 4), (33, 4, 64, 520, 3)])
+def test_batches_of_longer_k(M, H, N, K, pad):
+    test_batches(M, H, N, K, pad)
+
+
+@pytest.mark.parametrize("M,N,K", [(20, 128, 312), (20, 128, 352), (500, 2048, 216), (500, 2048, 240), (4, 4096, 1016), (4, 4096, 1024), (2, 4096, 2048)])
+def test_both_sides_of_the_lines(M, N, K):
+    """sizes just below and above the lines between the two forms: the same product"""
+    A, W = operands(M + K, M, N, K)
+    ref, tol = product(A, W[0])
+    a, w, c = gk.from_numpy(A), dev_w(W[0]), gk.zeros((M, N), gk.float32)
+    llm.LinearRows(w).forward(a.device_ptr, K, M, c.device_ptr, N)
+    assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6).all()
     no_wait_error()
