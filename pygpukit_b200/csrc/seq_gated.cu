@@ -296,15 +296,8 @@ __device__ __forceinline__ void combine_stage(const CombineArgs& a, int t, float
 __device__ __forceinline__ float combine_value(const CombineArgs& a, int t, int i, const float* wk, const long long* pk, float sg) {
     float v = 0.f;
     const int top = a.top, ks = top < CTOP ? top : CTOP;
-    for (int k0 = 0; k0 < ks; k0 += 4) {            // four rows' loads in flight, added in their order
-        float x[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            x[j] = k0 + j >= ks ? 0.f : (pk[k0 + j] < 0 ? a.self_rows[(size_t)t * a.W + i] : a.parts[pk[k0 + j] + i]);
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (k0 + j < ks) v = fmaf(wk[k0 + j], x[j], v);
-    }
+    for (int k = 0; k < ks; ++k)
+        v = fmaf(wk[k], pk[k] < 0 ? a.self_rows[(size_t)t * a.W + i] : a.parts[pk[k] + i], v);
     for (int k = CTOP; k < top; ++k) {
         const size_t o = (size_t)t * top + k;
         const bool self = a.mat && a.mat[o] < 0;
@@ -318,19 +311,21 @@ __device__ __forceinline__ float combine_gate(const CombineArgs& a, int t) {
     return a.shared ? (a.gate ? sigmoid_f(a.gate[(size_t)t * a.ldg + a.gate_off]) : 1.f) : 0.f;
 }
 
-__global__ void __launch_bounds__(256) moe_combine_rows_kernel(CombineArgs a, bool vec) {
+template <bool VEC>
+__global__ void __launch_bounds__(256) moe_combine_rows_kernel(CombineArgs a) {
     __shared__ float wk[CTOP];
     __shared__ long long pk[CTOP];
     const int t = blockIdx.x;
     combine_stage(a, t, wk, pk);
     const float sg = combine_gate(a, t);
     // four elements of eight rows per thread in flight where rows allow it: the expert rows' way from memory is all there is to it
-    // (2000 tokens: 36 -> 28 us)
-    if (vec && a.top <= 8) {
+    // (2000 tokens, eight rows of 2048: 51 -> 31 us, of 256: 8.3 -> 5.6); blocks of a thread per four elements, up to 256.  A kernel of its
+    // own, whose registers the other form does not pay for (ten rows of 2048: 66 us, 91 in one kernel)
+    if constexpr (VEC) {                            // at most eight rows
         float4* out = (float4*)(a.out + (size_t)t * a.W);
         const float4* self = (const float4*)(a.self_rows + (size_t)t * a.W);
         const float4* shared = (const float4*)(a.shared + (size_t)t * a.W);
-        for (int i = threadIdx.x; i < a.W / 4; i += 256) {
+        for (int i = threadIdx.x; i < a.W / 4; i += blockDim.x) {
             float4 x[8], v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int k = 0; k < 8; ++k)
@@ -347,9 +342,9 @@ __global__ void __launch_bounds__(256) moe_combine_rows_kernel(CombineArgs a, bo
             }
             out[i] = v;
         }
-        return;
+    } else {
+        for (int i = threadIdx.x; i < a.W; i += 256) a.out[(size_t)t * a.W + i] = combine_value(a, t, i, wk, pk, sg);
     }
-    for (int i = threadIdx.x; i < a.W; i += 256) a.out[(size_t)t * a.W + i] = combine_value(a, t, i, wk, pk, sg);
 }
 
 // ---------------------------------------------------------------- a sublayer's result joins the residual stream
@@ -768,8 +763,10 @@ int pgk_moe_combine_rows_f32(const float* parts, const int32_t* inv, const int32
     if (rows <= 0) return 0;
     CombineArgs a{parts, inv, mat, weights, top, self_rows, shared_rows, gate_rows, ldg, gate_off, out, width};
     const uintptr_t all = (uintptr_t)a.parts | (uintptr_t)a.self_rows | (uintptr_t)a.shared | (uintptr_t)a.out;
-    const bool vec = a.W % 4 == 0 && all % 16 == 0;
-    PGK_CUDA(launch(moe_combine_rows_kernel, dim3(rows), dim3(256), 0, (cudaStream_t)stream, a, vec));
+    const bool vec = a.W % 4 == 0 && all % 16 == 0 && top <= 8;
+    const int threads = a.W < 1024 ? (a.W / 4 + 31) / 32 * 32 : 256;
+    if (vec) PGK_CUDA(launch(moe_combine_rows_kernel<true>, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, a));
+    else PGK_CUDA(launch(moe_combine_rows_kernel<false>, dim3(rows), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 
