@@ -133,15 +133,42 @@ struct LinPrepArgs {
     const double* inv_freq; float k_scale; const int* pos;
 };
 
-// units per token: H query heads, H key heads, H value heads; a warp takes every 8 gridDim.y-th of them.  A token's angles (a
-// product in float64 and a sine pair each) are taken once per block instead of once per head (a prompt of 2000 tokens: 41 -> 29 us).
-constexpr int LIN_TURNS = 4096;                           // angles that shared memory holds; longer heads take the rest per head
+// units per token: H query heads, H key heads, H value heads; a warp each
+__global__ void __launch_bounds__(128) linear_prep_kernel(LinPrepArgs a) {
+    const int t = blockIdx.x, lane = threadIdx.x & 31, u = blockIdx.y * 4 + (threadIdx.x >> 5);
+    if (u >= 3 * a.H) return;
+    float* row = a.proj + (size_t)t * a.ld;
+    if (u >= 2 * a.H) {
+        if (!a.act) return;
+        float* v = row + a.v_off + (size_t)(u - 2 * a.H) * a.Dv;
+        for (int d = lane; d < a.Dv; d += 32) v[d] = silu_f(v[d]);
+        return;
+    }
+    const bool is_k = u >= a.H;
+    float* x = row + (is_k ? a.k_off + (size_t)(u - a.H) * a.D : a.q_off + (size_t)u * a.D);
+    const float sc = is_k ? a.k_scale : 1.f;
+    const int half = a.rot_dims / 2, pos = a.pos[t];
+    for (int i = lane; i < half; i += 32) {
+        float p0 = x[i], p1 = x[i + half];
+        if (a.act) { p0 = silu_f(p0); p1 = silu_f(p1); }
+        float sn, cs;
+        rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
+        x[i] = (p0 * cs - p1 * sn) * sc;
+        x[i + half] = (p1 * cs + p0 * sn) * sc;
+    }
+    for (int d = 2 * half + lane; d < a.D; d += 32) x[d] = (a.act ? silu_f(x[d]) : x[d]) * sc;
+}
 
-__global__ void __launch_bounds__(256) linear_prep_kernel(LinPrepArgs a) {
-    extern __shared__ float2 turn[];                      // [min(rot_dims / 2, LIN_TURNS)] (sine, cosine)
+// Many heads: the warps of a token's gridDim.y blocks take the units in turn, and the token's angles (a product in float64 and a sine
+// pair each) are taken once per block instead of once per head (2000 tokens, us: 16 heads of 128 36 -> 26, 32 85 -> 57).  With few heads
+// the barrier costs more than that (five 13.6 -> 15.5), and so does a test for the table's end in one kernel for both (32 heads of 64 42 -> 34 instead of 29).
+constexpr int LIN_TURNS = 4096;                           // angles that shared memory holds
+
+__global__ void __launch_bounds__(256) linear_prep_many_kernel(LinPrepArgs a) {
+    extern __shared__ float2 turn[];                      // [rot_dims / 2] (sine, cosine)
     const int t = blockIdx.x, lane = threadIdx.x & 31, half = a.rot_dims / 2;
     const int pos = half ? a.pos[t] : 0;
-    for (int i = threadIdx.x; i < min(half, LIN_TURNS); i += 256) {
+    for (int i = threadIdx.x; i < half; i += 256) {
         float sn, cs;
         rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
         turn[i] = make_float2(sn, cs);
@@ -161,9 +188,7 @@ __global__ void __launch_bounds__(256) linear_prep_kernel(LinPrepArgs a) {
         for (int i = lane; i < half; i += 32) {
             float p0 = x[i], p1 = x[i + half];
             if (a.act) { p0 = silu_f(p0); p1 = silu_f(p1); }
-            float sn, cs;
-            if (i < LIN_TURNS) { sn = turn[i].x; cs = turn[i].y; }
-            else rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
+            const float sn = turn[i].x, cs = turn[i].y;
             x[i] = (p0 * cs - p1 * sn) * sc;
             x[i + half] = (p1 * cs + p0 * sn) * sc;
         }
@@ -531,9 +556,12 @@ int pgk_seq_linear_prep(float* proj, int ld, int tokens, int heads, int dim, int
                 "seq_linear_prep failed: %d rotated dimensions in heads of %d", rot_dims, dim);
     if (tokens <= 0 || (!activation && rot_dims == 0 && k_scale == 1.f)) return 0;
     LinPrepArgs a{proj, ld, heads, dim, vdim, q_off, k_off, v_off, activation ? 1 : 0, rot_dims, inv_freq, k_scale, pos};
-    // a unit per warp while that fills the SMs no more than once, then two blocks per token (angles twice instead of six times)
-    const int all = (3 * heads + 7) / 8, groups = (long long)tokens * all <= 8 * sm_count() ? all : (all < 2 ? all : 2);
-    PGK_CUDA(launch(linear_prep_kernel, dim3(tokens, groups), dim3(256), sizeof(float2) * (rot_dims / 2 < LIN_TURNS ? rot_dims / 2 : LIN_TURNS), (cudaStream_t)stream, a));
+    if (heads > 8 && rot_dims / 2 <= LIN_TURNS) {
+        // a unit per warp while that fills the SMs no more than once, then two blocks per token (angles twice instead of six times)
+        const int all = (3 * heads + 7) / 8, groups = (long long)tokens * all <= 8 * sm_count() ? all : 2;
+        PGK_CUDA(launch(linear_prep_many_kernel, dim3(tokens, groups), dim3(256), (size_t)(rot_dims / 2) * sizeof(float2), (cudaStream_t)stream, a));
+    } else
+        PGK_CUDA(launch(linear_prep_kernel, dim3(tokens, (3 * heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
     return 0;
 }
 

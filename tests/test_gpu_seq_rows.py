@@ -87,7 +87,7 @@ def test_router_logits(M, N, K):
     assert (out[:, N:] == 7.0).all()
 
 
-@pytest.mark.parametrize("H,D,rot", [(1, 16400, 16400), (3, 8200, 8194), (4, 64, 0), (2, 96, 50)])
+@pytest.mark.parametrize("H,D,rot", [(1, 16400, 16400), (9, 8200, 8194), (4, 64, 0), (2, 96, 50), (9, 96, 50), (33, 64, 64)])
 def test_turned_heads_of_any_length(H, D, rot):
     """heads with more pairs than the kernel's table of angles holds: silu and turn of q and k in float32 on float64 angles, two
     products and a sum of values of about 1 and the table's roundings"""
