@@ -464,11 +464,12 @@ int launch_few(const GemmArgs& a, int wdt, int rows_per_block, cudaStream_t st, 
 
 // ---------------------------------------------------------------- many rows, few columns, float32 weights (router logits)
 // A 64 x 64 tile would leave all but one tile column empty and the grid a handful of blocks.  Here a warp owns SKM rows and SKN
-// columns and walks K with a lane per element; the partial sums meet in a warp reduction.  Plain epilogue only.  Latency bounds it:
-// two rows and one column group per warp, for more warps with 40 loads each in flight than four rows and all columns leave
-// (router of the 2000-token expert prompt: 55 -> 50 us).  The sums' order is that of one warp per row.
-constexpr int SKM = 2, SKN = 8, SK_WARPS = 4;
+// columns and walks K with a lane per element; the partial sums meet in a warp reduction.  Plain epilogue only.  Latency bounds it: a
+// warp per column group instead of one for all columns, addresses that need no test (us, one warp per row group -> here: 2000 rows of
+// 2048, 4 / 16 / 64 columns 14.5 / 25.2 / 84 -> 12.8 / 14.5 / 28.8; two rows per warp 16.4 / 22.7 / 45.2).  The sums' order is that of one warp per row.
+constexpr int SKM = 4, SK_WARPS = 4;
 
+template <int SKN>
 __global__ void __launch_bounds__(SK_WARPS * 32) gemm_skinny_f32_kernel(GemmArgs a) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = (blockIdx.x * SK_WARPS + warp) * SKM, n0 = blockIdx.y * SKN;
@@ -529,7 +530,9 @@ int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const vo
     GemmArgs a{A, a_rows, W, C, group_off, nullptr, w_group_stride, lda, ldc, M, N, K, scale, cap, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0};
     cudaStream_t st = (cudaStream_t)stream;
     if (wdt == 0 && epilogue == 0 && !group_off && !a_rows && N <= 64) {        // router logits: few columns, float32 weights
-        PGK_CUDA(launch(gemm_skinny_f32_kernel, dim3((M + SK_WARPS * SKM - 1) / (SK_WARPS * SKM), (N + SKN - 1) / SKN), dim3(SK_WARPS * 32), 0, st, a));
+        const int gx = (M + SK_WARPS * SKM - 1) / (SK_WARPS * SKM);
+        if (N <= 4) PGK_CUDA(launch(gemm_skinny_f32_kernel<4>, dim3(gx), dim3(SK_WARPS * 32), 0, st, a));
+        else PGK_CUDA(launch(gemm_skinny_f32_kernel<8>, dim3(gx, (N + 7) / 8), dim3(SK_WARPS * 32), 0, st, a));
         return 0;
     }
     const int bound = group_off ? total_rows : M;
