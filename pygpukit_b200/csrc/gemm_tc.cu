@@ -14,7 +14,8 @@
 //     store them to TENSOR MEMORY, from where the MMA takes its A operand: through shared memory the BF16 form would be written
 //     and read once more, 128 KB per block of weights instead of 64, which alone is 1000 cycles against 680 for the HBM stream;
 //   * the block scale multiplies the partial sums of its 128 products in float32 (two accumulators by turns): products are exact and
-//     the activations need no second term that holds their product with the scale;
+//     the activations need no second term that holds their product with the scale (128 unscaled products must stay within float32:
+//     activations up to 5e33);
 //   * the same eight warps add the partial sums of the block before while the tensor cores multiply; MMAs and copies have a warp each;
 //   * a stage holds a block's codes and rows together (rings of their own left too few slots for the rows: 65 -> 72 us);
 //   * two blocks per SM (256 TMEM columns, 100 KB each) hide each other's start and end; K is cut over a cluster that pushes
@@ -271,7 +272,9 @@ cudaError_t f8tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int sp
     return cudaSuccess;
 }
 
-// blocks that the device holds at one time in clusters of s (clusters do not cross its processing clusters)
+// Blocks that the device holds at one time in clusters of s, as cudaOccupancyMaxActiveClusters counts them (clusters do not cross its
+// processing clusters).  For kernels that allocate tensor memory it answers with one block per SM, while two were seen to run together:
+// plans of several blocks per tile are charged rounds that they may not take.
 int f8tc_held(int s) {
     static int held[9] = {};
     if (held[s] == 0) {

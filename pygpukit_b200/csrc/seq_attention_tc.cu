@@ -23,8 +23,8 @@
 //     outputs leave four rows at a time in a short loop (code that runs once per block costs its fetch), and rows that no query
 //     has are left out: what decoding, one tile per block, spends its time on.
 // Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 191 us; 16 heads over latent rows
-// of 576 / 512 5097 -> 471 us.  Decoding, 8 requests: latent rows over 2000 keys 129 -> 50 us, 16 / 4
-// heads of 128 over 1024 65 -> 24 us.  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
+// of 576 / 512 5097 -> 471 us.  Decoding, 8 requests: latent rows over 2000 keys 129 -> 50 us, 16 / 4 heads of 128 over 1024 65 -> 24
+// us.  (Weights reach 2^LAZY before their reference moves: sums of values above 2^120 may overflow.)  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
 // 128).
 #include "seq_attention.cuh"
 #include "tc_common.cuh"

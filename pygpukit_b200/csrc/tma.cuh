@@ -48,7 +48,7 @@ __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                  :: "r"(smem_dst), "l"(map), "r"(c0), "r"(c1), "r"(bar) : "memory");
 }
-// bytes that nobody reads again: first to leave L2
+// bytes that nobody reads again, or only blocks that run at the same time: first to leave L2
 __device__ __forceinline__ uint64_t l2_evict_first() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
