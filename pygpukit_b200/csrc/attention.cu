@@ -418,12 +418,11 @@ struct RopeSdpaParams {
 // contexts and the multi-sequence batches.  Here a warp owns 16 positions of a 64-position tile:
 //     S[8 heads (+8 zero rows), 16 pos]  = Q[16, 128] . K^T      16 MMAs, B fragments by ldmatrix from the swizzled tile
 //     online softmax on the 4 scores a thread holds (row = lane / 4), quad shuffles only
-//     O[16, 128] += P[16, 16] . V[16, 128]                       32 MMAs, V fragments by ldmatrix.trans
-// The probabilities go to the tensor cores as FOUR bf16 terms in two A fragments: two halves of p in rows 0..7, the rest in rows
-// 8..15 (the rows the <= 8 query heads leave empty); together they hold all 24 bits, and O = O[0..7] + O[8..15].  The
-// products q.k are exact, p.v is what float32 would give.  With 16 bits of p one output in 2^9 rounds to the other bf16
-// neighbour: 570 of 1024 logits moved on the first decoded token of a two-layer model, none with 24 (context 4096, 32 / 8
-// heads, the attention layer: 30.7 us before and after).
+//     O[16, 128] += P[16, 16] . V[16, 128]                       16 or 32 MMAs, V fragments by ldmatrix.trans
+// The probabilities go to the tensor cores as bf16 terms that together hold all 24 bits, in rows of A fragments that the <= 8 query
+// heads leave empty, and O is the sum of the rows.  Up to four heads (a GQA group of four) sit in two rows each, so that one fragment takes
+// all terms; more take a second one.  The products q.k are exact, p.v is what float32 would give.  With 16 bits of p one output in
+// 2^9 rounds to the other bf16 neighbour: 570 of 1024 logits moved on the first decoded token of a two-layer model, none with 24.
 // One CTA = 4 consumer warps + 1 TMA producer warp, 2 CTAs per SM; up to 8 query heads per CTA, so a GQA group of 8
 // (Llama-3-70B, Qwen3-30B-A3B) reads its K/V once instead of twice.  Stages: 2 x 32 KB for one sequence -- measured:
 // with 3 stages the two CTAs need 202 KB of shared memory, the SM is switched to its largest carve-out, and the GEMVs
@@ -494,7 +493,8 @@ __device__ __forceinline__ void norm_rope_regs(float (&x)[4], bool use_gamma, co
     }
 }
 
-template <int kMStages>
+// TWICE: at most four heads per KV head, each in rows r and r + 4
+template <int kMStages, bool TWICE>
 __global__ void __launch_bounds__(kMThreads, 2)
 rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, RopeSdpaParams p) {
     constexpr int HD = 128, RT = kMRT, REC = kMRec;
@@ -577,7 +577,8 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
         for (int j = 0; j < 2; ++j) {
             const int h = warp + j * kMW;
             if (h < rows) norm_rope_regs(x[j], my_gamma != nullptr, rg, p.eps, rc, rs, lane, q_s[h], nullptr);
-            else for (int d = lane; d < HD; d += 32) q_s[h][d] = 0;
+            else if (!TWICE || h < kMW) for (int d = lane; d < HD; d += 32) q_s[h][d] = 0;
+            else for (int d = lane; d < HD; d += 32) q_s[h][d] = q_s[h - kMW][d];       // this lane's own elements
         }
     } else if (has_new || writer) {
         float x[4];
@@ -681,27 +682,42 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
 #pragma unroll
                         for (int e = 0; e < 4; ++e) o[nt][e] *= corr;
                 }
-                // p as four bf16 terms that hold all 24 bits, in two A fragments: halves h1, h2 in rows 0..7, what they leave, l1 and l2, in
-                // rows 8..15.  Both halves of a positive p are positive: an infinite value row gives that infinity.
-                float rem[4];
-                uint32_t h1[4];
+                // ---- O += P . V, p as bf16 terms that hold all 24 bits
+                if constexpr (TWICE) {                            // hi in rows 0..3, lo in rows 8..11, the rest in rows 4..7
+                    const bool second = lane >= 16;
+                    const uint32_t hi0 = pack_bf16x2(pr[0], pr[1]), hi2 = pack_bf16x2(pr[2], pr[3]);
+                    float rem[4] = {pr[0] - bf16lo(hi0), pr[1] - bf16hi(hi0), pr[2] - bf16lo(hi2), pr[3] - bf16hi(hi2)};
+                    const uint32_t lo0 = pack_bf16x2(rem[0], rem[1]), lo2 = pack_bf16x2(rem[2], rem[3]);
+                    const uint32_t re0 = pack_bf16x2(rem[0] - bf16lo(lo0), rem[1] - bf16hi(lo0)), re2 = pack_bf16x2(rem[2] - bf16lo(lo2), rem[3] - bf16hi(lo2));
+                    const uint32_t a0 = second ? re0 : hi0, a2 = second ? re2 : hi2, a1 = second ? 0u : lo0, a3 = second ? 0u : lo2;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { h1[j] = __float_as_uint(0.5f * pr[j]) & 0xffff0000u; rem[j] = pr[j] - __uint_as_float(h1[j]); }
-                const uint32_t a0 = (h1[0] >> 16) | h1[1], a2 = (h1[2] >> 16) | h1[3];
-                const uint32_t b0 = pack_bf16x2(rem[0], rem[1]), b2 = pack_bf16x2(rem[2], rem[3]);
-                rem[0] -= bf16lo(b0); rem[1] -= bf16hi(b0); rem[2] -= bf16lo(b2); rem[3] -= bf16hi(b2);
-                const uint32_t a1 = pack_bf16x2(rem[0], rem[1]), a3 = pack_bf16x2(rem[2], rem[3]);
-                const uint32_t b1 = pack_bf16x2(rem[0] - bf16lo(a1), rem[1] - bf16hi(a1)), b3 = pack_bf16x2(rem[2] - bf16lo(a3), rem[3] - bf16hi(a3));
-                // ---- O += P . V
+                    for (int q = 0; q < 8; ++q) {
+                        const uint32_t ch = (uint32_t)(q * 2 + (lj >> 1));
+                        uint32_t v[4];
+                        ldsm_x4_t(tile + (ch >> 3) * kMBox + v_off + (((ch & 7) ^ v_sw) << 4), v);
+                        mma_bf16_16816(o[2 * q], a0, a1, a2, a3, v[0], v[1]);
+                        mma_bf16_16816(o[2 * q + 1], a0, a1, a2, a3, v[2], v[3]);
+                    }
+                } else {                                          // two fragments: halves in rows 0..7, both positive where p is, so that an
+                    float rem[4];                                 // infinite value row gives that infinity; what they leave in rows 8..15
+                    uint32_t h1[4];
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const uint32_t ch = (uint32_t)(q * 2 + (lj >> 1));
-                    uint32_t v[4];
-                    ldsm_x4_t(tile + (ch >> 3) * kMBox + v_off + (((ch & 7) ^ v_sw) << 4), v);
-                    mma_bf16_16816(o[2 * q], a0, a1, a2, a3, v[0], v[1]);
-                    mma_bf16_16816(o[2 * q + 1], a0, a1, a2, a3, v[2], v[3]);
-                    mma_bf16_16816(o[2 * q], b0, b1, b2, b3, v[0], v[1]);
-                    mma_bf16_16816(o[2 * q + 1], b0, b1, b2, b3, v[2], v[3]);
+                    for (int j = 0; j < 4; ++j) { h1[j] = __float_as_uint(0.5f * pr[j]) & 0xffff0000u; rem[j] = pr[j] - __uint_as_float(h1[j]); }
+                    const uint32_t a0 = (h1[0] >> 16) | h1[1], a2 = (h1[2] >> 16) | h1[3];
+                    const uint32_t b0 = pack_bf16x2(rem[0], rem[1]), b2 = pack_bf16x2(rem[2], rem[3]);
+                    rem[0] -= bf16lo(b0); rem[1] -= bf16hi(b0); rem[2] -= bf16lo(b2); rem[3] -= bf16hi(b2);
+                    const uint32_t a1 = pack_bf16x2(rem[0], rem[1]), a3 = pack_bf16x2(rem[2], rem[3]);
+                    const uint32_t b1 = pack_bf16x2(rem[0] - bf16lo(a1), rem[1] - bf16hi(a1)), b3 = pack_bf16x2(rem[2] - bf16lo(a3), rem[3] - bf16hi(a3));
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) {
+                        const uint32_t ch = (uint32_t)(q * 2 + (lj >> 1));
+                        uint32_t v[4];
+                        ldsm_x4_t(tile + (ch >> 3) * kMBox + v_off + (((ch & 7) ^ v_sw) << 4), v);
+                        mma_bf16_16816(o[2 * q], a0, a1, a2, a3, v[0], v[1]);
+                        mma_bf16_16816(o[2 * q + 1], a0, a1, a2, a3, v[2], v[3]);
+                        mma_bf16_16816(o[2 * q], b0, b1, b2, b3, v[0], v[1]);
+                        mma_bf16_16816(o[2 * q + 1], b0, b1, b2, b3, v[2], v[3]);
+                    }
                 }
             }
             if (t + kMStages < ntiles) {                        // hand the stage back to the producer
@@ -714,16 +730,20 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
         l_run += __shfl_xor_sync(0xffffffffu, l_run, 2);
     }
     __syncthreads();                                           // every stage is consumed: its memory is free for the merge
-    float (*sm_part)[RT][SREC] = reinterpret_cast<float (*)[RT][SREC]>(tiles_g);
+    float (*sm_part)[RT][SREC] = reinterpret_cast<float (*)[RT][SREC]>(tiles_g);      // leading terms, maxima, sums
+    float (*sm_rest)[RT][SREC] = sm_part + kMW;                                      // smaller terms
     if (warp < kMW) {
         const int qrow = lane >> 2, kk = (lane & 3) * 2;
 #pragma unroll
-        for (int nt = 0; nt < 16; ++nt)
-            *reinterpret_cast<float2*>(&sm_part[warp][qrow][nt * 8 + kk]) = make_float2(join_terms(o[nt][0], o[nt][2]), join_terms(o[nt][1], o[nt][3]));
+        for (int nt = 0; nt < 16; ++nt) {
+            *reinterpret_cast<float2*>(&sm_part[warp][qrow][nt * 8 + kk]) = make_float2(o[nt][0], o[nt][1]);
+            *reinterpret_cast<float2*>(&sm_rest[warp][qrow][nt * 8 + kk]) = make_float2(o[nt][2], o[nt][3]);
+        }
         if ((lane & 3) == 0) { sm_part[warp][qrow][HD] = m_run; sm_part[warp][qrow][HD + 1] = l_run; }
     }
     __syncthreads();
     const size_t tile_id = ((size_t)seq * p.n_kv + kvh) * row_tiles + rt;
+    auto part = [&](int w, int r, int d) { return join_terms(sm_part[w][r][d], TWICE ? sm_rest[w][r][d] + sm_part[w][r + kMW][d] : sm_rest[w][r][d]); };
     if (p.splits == 1) {
         for (int idx = threadIdx.x; idx < rows * HD; idx += kMThreads) {
             const int r = idx / HD, d = idx % HD;
@@ -734,7 +754,7 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
 #pragma unroll
             for (int w = 0; w < kMW; ++w) {
                 const float c = exp2f(sm_part[w][r][HD] - mn);
-                ov = fmaf(sm_part[w][r][d], c, ov);
+                ov = fmaf(part(w, r, d), c, ov);
                 lv = fmaf(sm_part[w][r][HD + 1], c, lv);
             }
             p.out[(size_t)(kvh * G + rt * RT + r) * HD + d] = f32_to_bf16_bits(lv > 0.f ? ov / lv : 0.f);
@@ -762,7 +782,7 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
 #pragma unroll
         for (int w = 0; w < kMW; ++w) {
             const float c = exp2f(sm_part[w][r][HD] - mn);
-            ov = fmaf(sm_part[w][r][d], c, ov);
+            ov = fmaf(part(w, r, d), c, ov);
             lv = fmaf(sm_part[w][r][HD + 1], c, lv);
         }
         uint2* rec = ll + ((size_t)split * RT + r) * REC;
@@ -777,7 +797,7 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
     if (n_e <= 0) return;
     const int r0 = e0 / HD, nr = (e0 + n_e - 1) / HD - r0 + 1;   // rows this slice touches
     const int SP = S | 1;                                        // odd stride: conflict-free column walks
-    float* f_o = reinterpret_cast<float*>(tiles_g + 20 * 1024);  // [n_e][SP]
+    float* f_o = reinterpret_cast<float*>(tiles_g + 36 * 1024);  // [n_e][SP]
     float* f_m = f_o + W * SP;                                   // [RT][SP]  (max, then scale factor)
     float* f_l = f_m + RT * SP;                                  // [RT][SP]
     float* f_den = f_l + RT * SP;                                // [RT]
@@ -891,15 +911,15 @@ static int attn_cache_map(const void* cache, int max_seq, int n_kv, int n_seq, l
     return 0;
 }
 
-template <int STAGES>
+template <int STAGES, bool TWICE>
 static int launch_rope_sdpa_stages(const CUtensorMap& kmap, const CUtensorMap& vmap, const RopeSdpaParams& p, dim3 grid, cudaStream_t st) {
     constexpr size_t kSmem = (size_t)STAGES * kMStageB + 1024;
     static bool attr_set = false;
     if (!attr_set) {
-        PGK_CUDA(cudaFuncSetAttribute(rope_sdpa_mma_kernel<STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
+        PGK_CUDA(cudaFuncSetAttribute(rope_sdpa_mma_kernel<STAGES, TWICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
         attr_set = true;
     }
-    PGK_CUDA(launch(rope_sdpa_mma_kernel<STAGES>, grid, dim3(kMThreads), kSmem, st, kmap, vmap, p));
+    PGK_CUDA(launch(rope_sdpa_mma_kernel<STAGES, TWICE>, grid, dim3(kMThreads), kSmem, st, kmap, vmap, p));
     return 0;
 }
 
@@ -939,7 +959,9 @@ static int launch_rope_sdpa(RopeSdpaParams p, cudaStream_t st) {
     p.gen = g_attn_gen;
     p.box_rows = p.max_seq < kMTile ? p.max_seq : kMTile;
     const dim3 grid(splits, row_tiles, p.n_kv * p.n_seq);
-    return p.n_seq > 1 ? launch_rope_sdpa_stages<3>(kmap, vmap, p, grid, st) : launch_rope_sdpa_stages<2>(kmap, vmap, p, grid, st);
+    if (G <= kMRT / 2)
+        return p.n_seq > 1 ? launch_rope_sdpa_stages<3, true>(kmap, vmap, p, grid, st) : launch_rope_sdpa_stages<2, true>(kmap, vmap, p, grid, st);
+    return p.n_seq > 1 ? launch_rope_sdpa_stages<3, false>(kmap, vmap, p, grid, st) : launch_rope_sdpa_stages<2, false>(kmap, vmap, p, grid, st);
 }
 
 }  // namespace pgk
