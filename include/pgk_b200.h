@@ -49,6 +49,8 @@ int pgk_device_sync(void);
  * ends, and that the next call that synchronises fails for it */
 int pgk_wait_probe(int limit_us, int32_t* ran_out, void* stream);
 int pgk_mem_info(size_t* free_bytes, size_t* total_bytes);
+/* gives idle work memory of the library and of destroyed graphs back to the device (pgk_malloc does when it runs out); not during a capture */
+int pgk_mem_trim(void);
 
 int pgk_malloc(void** ptr, size_t bytes);            /* memory.cpp:29 cuMemAlloc */
 int pgk_free(void* ptr);

@@ -27,7 +27,7 @@ class DeviceProps(C.Structure):
 _SIGS = {
     "pgk_version": [],
     "pgk_device_count": [C.POINTER(i32)], "pgk_device_set": [i32], "pgk_device_get": [C.POINTER(i32)],
-    "pgk_device_props": [i32, C.POINTER(DeviceProps)], "pgk_device_sync": [], "pgk_wait_probe": [i32, vp, vp],
+    "pgk_device_props": [i32, C.POINTER(DeviceProps)], "pgk_device_sync": [], "pgk_wait_probe": [i32, vp, vp], "pgk_mem_trim": [],
     "pgk_mem_info": [C.POINTER(sz), C.POINTER(sz)],
     "pgk_malloc": [C.POINTER(vp), sz], "pgk_free": [vp],
     "pgk_host_alloc": [C.POINTER(vp), sz], "pgk_host_free": [vp],

@@ -102,6 +102,9 @@ static bool scratch_trim() {
     bool any = false;
     for (cudaMemPool_t p : g_scratch)
         if (p) any = cudaMemPoolTrimTo(p, 0) == cudaSuccess || any;
+    // work memory of captured products whose graphs are gone stays with the device's graph pool, where no other allocation finds it
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) any = cudaDeviceGraphMemTrim(dev) == cudaSuccess || any;
     return any;
 }
 
@@ -211,6 +214,11 @@ int pgk_mem_info(size_t* free_bytes, size_t* total_bytes) {
     return 0;
 }
 
+int pgk_mem_trim(void) {
+    scratch_trim();
+    cudaGetLastError();
+    return 0;
+}
 int pgk_malloc(void** ptr, size_t bytes) {
     *ptr = nullptr;
     if (bytes == 0) bytes = 1;

@@ -374,3 +374,42 @@ def test_both_sides_of_the_lines(M, N, K):
     llm.LinearRows(w).forward(a.device_ptr, K, M, c.device_ptr, N)
     assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6).all()
     no_wait_error()
+
+
+def free_bytes():
+    f, t = C.c_size_t(), C.c_size_t()
+    api.mem_info(C.byref(f), C.byref(t))
+    return f.value
+
+
+def test_idle_work_memory_goes_back():
+    """256 MB of rounded rows that a captured product allocates, and as many of plain ones: with the device again once they are idle"""
+    from pygpukit_b200.core.stream import CudaGraph, Stream
+    M, N, K = 1 << 16, 256, 2048
+    a, w, c = gk.zeros((M, K), gk.float32), dev_w(np.ones((N, K))), gk.zeros((M, N), gk.float32)
+    lin, st = llm.LinearRows(w), Stream()
+
+    def captured():
+        g = CudaGraph()
+        with g.capture(st):
+            lin.forward(a.device_ptr, K, M, c.device_ptr, N)
+        g.replay(st)
+        st.synchronize()
+        return g
+
+    def plain():
+        lin.forward(a.device_ptr, K, M, c.device_ptr, N)
+        api.device_sync()
+
+    for make in (captured, plain):
+        keep = make()                                    # (whatever the first one keeps for good)
+        del keep
+        api.mem_trim()
+        before = free_bytes()
+        keep = make()
+        assert before - free_bytes() >= 200 << 20
+        del keep
+        api.mem_trim()
+        assert before - free_bytes() <= 32 << 20
+    plain()
+    assert (c.to_numpy() == 0).all()
