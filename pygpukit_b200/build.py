@@ -36,6 +36,7 @@ SOURCES = {
     "gemv_bf16.cu": [],
     "gemm_w8a16.cu": [],
     "gemm_tc.cu": [],
+    "gemm_tc_rows.cu": [],
     "gemm_tc_nvf4.cu": [],
     "gemm_tc_f8.cu": [],
     "elementwise.cu": [],

@@ -70,8 +70,28 @@ class DecodeBuffers:
 
 @dataclass
 class PrefillBuffers:
-    """Kept for API parity (buffers.py:467-621); prefill reuses DecodeBuffers in slabs of rows."""
+    """Work arrays of prompts that go through the layers in portions longer than the decode batch (`for_rows`; the members have
+    DecodeBuffers' names).  `allocate` keeps the signature of buffers.py:467-621; other prompts reuse DecodeBuffers in slabs of rows."""
     max_seq_len: int = 0
+    hidden: GPUArray | None = None
+    norm_out: GPUArray | None = None
+    qkv_proj_out: GPUArray | None = None
+    attn_flat: GPUArray | None = None
+    mlp_act: GPUArray | None = None
+    token_buf: GPUArray | None = None
+
+    @classmethod
+    def for_rows(cls, config: TransformerConfig, rows: int) -> "PrefillBuffers":
+        """One allocation for `rows` tokens of an unsharded model."""
+        H, hd, hq, hkv = config.hidden_size, config.head_dim, config.num_heads, config.num_kv_heads
+        widths = [H, H, (hq + 2 * hkv) * hd, hq * hd, config.intermediate_size]
+        sizes = [-(-rows * w // 128) * 128 for w in widths]                  # 256-byte boundaries
+        whole = GPUArray((sum(sizes) + 2 * rows,), bfloat16)
+        parts, at = [], 0
+        for w, n in zip(widths, sizes):
+            parts.append(GPUArray((rows, w), bfloat16, ptr=whole.device_ptr + 2 * at, source=whole))
+            at += n
+        return cls(rows, *parts, GPUArray((rows,), int32, ptr=whole.device_ptr + 2 * at, source=whole))
 
     @classmethod
     def allocate(cls, config: TransformerConfig, max_seq_len: int, dtype: str = "bfloat16", use_qk_norm: bool = False):

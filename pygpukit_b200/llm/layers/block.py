@@ -32,13 +32,14 @@ class TransformerBlock:
             return b if (b is None or b.shape[0] == M) else b.slice_rows(M)
 
         tp = self.comm is not None and self.comm.world > 1
-        # pre-norms ride inside the qkv / gate-up GEMV launches when the formats allow it
+        # pre-norms ride inside the qkv / gate-up GEMV launches when the formats allow it (the tensor-core products of longer portions
+        # take normed rows)
         if multi:
             fuse = can_fuse_norm(self.attn_norm, hidden.shape[1])
             x = hidden if fuse else self.attn_norm(hidden, out=buf("norm_out"))
             a = self.attn.attend_multi(x, pos_buf, ctx_buf, qkv_buf=buf("qkv_proj_out"), attn_buf=buf("attn_flat"),
                                        norm=self.attn_norm if fuse else None)
-        elif can_fuse_norm(self.attn_norm, hidden.shape[1]):
+        elif can_fuse_norm(self.attn_norm, hidden.shape[1]) and M <= 64:
             a = self.attn.attend(hidden, position, context_len, qkv_buf=buf("qkv_proj_out"), attn_buf=buf("attn_flat"),
                                  pos_buf=pos_buf, ctx_buf=ctx_buf, norm=self.attn_norm)
         else:
@@ -52,7 +53,7 @@ class TransformerBlock:
             self.comm.allreduce_add(part, hidden)
         else:
             self.attn.o_proj.forward(a, out=hidden, residual=hidden)
-        fuse_mlp = isinstance(self.mlp, MLP) and self.mlp.fuses_norm(self.mlp_norm)
+        fuse_mlp = isinstance(self.mlp, MLP) and self.mlp.fuses_norm(self.mlp_norm) and M <= 64
         x, nrm = (hidden, self.mlp_norm) if fuse_mlp else (self.mlp_norm(hidden, out=buf("norm_out")), None)
         kw = {"norm": nrm} if fuse_mlp else {}
         if tp and isinstance(self.mlp, MoELayer):

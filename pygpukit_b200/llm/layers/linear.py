@@ -125,9 +125,9 @@ class LinearFP8:
         self._norm_scratch: dict[int, GPUArray] = {}
 
     def uses_tensor_cores(self, M: int) -> bool:
-        """True when a batch of M rows is served by the tcgen05 skinny GEMM (pgk_gemm_fp8_bf16_tc) instead of
-        the CUDA-core GEMV: TC_MIN_M <= M <= 64 and 128-aligned shapes (every model shape of BASELINE.json)."""
-        return (TC_MIN_M <= M <= 64 and self.in_features % 128 == 0 and self.out_features % 128 == 0
+        """True when a batch of M rows is served by the tcgen05 GEMMs (pgk_gemm_fp8_bf16_tc; above 64 rows the kernel of
+        gemm_tc_rows.cu) instead of the CUDA-core GEMV: M >= TC_MIN_M and 128-aligned shapes."""
+        return (TC_MIN_M <= M <= 65536 and self.in_features % 128 == 0 and self.out_features % 128 == 0
                 and os.environ.get("PGK_TC", "1") != "0")
 
     def _dequantize_cpu(self) -> np.ndarray:

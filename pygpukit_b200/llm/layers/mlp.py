@@ -70,6 +70,10 @@ class MLP:
             self.intermediate_size = (self.gate_up_proj.out_features // 2 if self.gate_up_proj is not None
                                       else self.gate_proj.out_features)
 
+    def _fp8_pair(self) -> bool:
+        return (self.activation == "silu" and self.gate_up_proj is None and isinstance(self.gate_proj, LinearFP8)
+                and isinstance(self.up_proj, LinearFP8) and self.gate_proj.bias is None and self.up_proj.bias is None)
+
     # ---- fused activation( gate/up ) -> act_out [M, I]
     def fuses_norm(self, norm) -> bool:
         """True when `norm` can ride inside the gate/up launch (FP8 / NVF4 fused SwiGLU kernels)."""
@@ -83,6 +87,13 @@ class MLP:
         M, K, I = x.shape[0], x.shape[1], self.intermediate_size
         if out is None:
             out = GPUArray((M, I), bfloat16)
+        if (M > 64 and norm is None and self._fp8_pair() and self.gate_proj.uses_tensor_cores(M)
+                and self.up_proj.uses_tensor_cores(M)):
+            # prompts: both products, silu and mul in one launch, with the layer path's roundings
+            g, u = self.gate_proj, self.up_proj
+            api.gemv_fp8_swiglu_bf16(x.device_ptr, g.weight_fp8.device_ptr, g.scale_inv.device_ptr,
+                                     u.weight_fp8.device_ptr, u.scale_inv.device_ptr, out.device_ptr, M, K, I, _st())
+            return out
         if (self.gate_up_proj is None and isinstance(self.gate_proj, LinearFP8) and isinstance(self.up_proj, LinearFP8)
                 and self.gate_proj.uses_tensor_cores(M) and self.up_proj.uses_tensor_cores(M)):
             # batch >= TC_MIN_M: gate and up on the tcgen05 GEMM, then silu -> mul with the layer path's two roundings

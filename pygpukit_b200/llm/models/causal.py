@@ -24,10 +24,11 @@ from ...core.array import GPUArray
 from ...core.dtypes import bfloat16, int32
 from ...core.factory import from_numpy
 from ...core.stream import CudaGraph, Stream, current_stream_handle as _st, use_stream
-from ..buffers import DecodeBuffers
+from ..buffers import DecodeBuffers, PrefillBuffers
 from ..config import ModelSpec, TransformerConfig
 from ..layers.block import TransformerBlock
-from ..layers.linear import can_fuse_norm
+from ..layers.linear import LinearFP8, can_fuse_norm
+from ..layers.mlp import MLP
 from ..layers.norm import Norm
 from ..decode.accept import accept_jacobi, accept_speculative
 from ..sampling import sample_token
@@ -53,6 +54,7 @@ class CausalTransformerModel:
         self.spec = spec
         self.comm = comm
         self._buffers: DecodeBuffers | None = None
+        self._prompt_bufs: PrefillBuffers | None = None
         self._max_seq = 0
         self._graph: CudaGraph | None = None
         self._graph_stream: Stream | None = None
@@ -102,6 +104,7 @@ class CausalTransformerModel:
         v_local = self._head.shape[0]
         self._buffers = DecodeBuffers.allocate(self.config, "bfloat16", vocab_size=v_local,
                                                max_batch_size=max(max_batch_size, S), num_sequences=S)
+        self._prompt_bufs = None
         self._max_seq = max_seq_len
         self._num_sequences = S
         if self.tp > 1:
@@ -238,10 +241,50 @@ class CausalTransformerModel:
         start = position_ids[0] if position_ids else int(past_key_values or 0)
         hidden = None
         slab = self.buffers.max_batch_size
+        if len(input_ids) > slab and self._long_portions():
+            hidden = self._prompt(list(input_ids), start)
+            return hidden, (start + len(input_ids) if use_cache else None)
         for i in range(0, len(input_ids), slab):
             ids = input_ids[i:i + slab]
             hidden = self._decode_step_fixed_cache_batch(ids, start + i, start + i + len(ids))
         return hidden, (start + len(input_ids) if use_cache else None)
+
+    # ------------------------------------------------------------------ long prompts
+    PROMPT_ROWS = 512                # tokens per portion: the products are near their rate, the buffers 30 ... 60 MB for 8B ... 70B models
+
+    def _long_portions(self) -> bool:
+        """True when every layer serves portions of more than 64 rows on the tensor cores (FP8 projections, silu MLP without biases on
+        gate and up, one GPU); other prompts run in slabs of `max_batch_size` rows."""
+        if self.tp > 1:
+            return False
+        for blk in self.blocks:
+            if type(blk) is not TransformerBlock or blk.comm is not None or type(blk.mlp) is not MLP or not blk.mlp._fp8_pair():
+                return False
+            lin = (blk.attn.qkv_proj, blk.attn.o_proj, blk.mlp.gate_proj, blk.mlp.up_proj, blk.mlp.down_proj)
+            if not all(isinstance(p, LinearFP8) and p.uses_tensor_cores(65) for p in lin):
+                return False
+        return True
+
+    def _prompt(self, ids: list[int], start: int) -> GPUArray:
+        """`ids` through all layers, PROMPT_ROWS rows at a time; returns the final-norm hidden of the last slab of `max_batch_size`
+        rows, like the slabs would."""
+        slab, n = self.buffers.max_batch_size, len(ids)
+        if start + n > self._max_seq:
+            raise ValueError(f"context_len {start + n} exceeds the fixed cache ({self._max_seq})")
+        portion = max(1, self.PROMPT_ROWS // slab) * slab                    # its ends are slabs' ends
+        rows = min(portion, n)
+        if self._prompt_bufs is None or self._prompt_bufs.max_seq_len < rows:
+            self._prompt_bufs = None
+            self._prompt_bufs = PrefillBuffers.for_rows(self.config, rows)
+        b, hidden = self._prompt_bufs, None
+        for i in range(0, n, portion):
+            part = ids[i:i + portion]
+            hidden = self._embed(part, len(part), start + i, b)
+            self._layers(hidden, start + i, start + i + len(part), b)
+        m, last = hidden.shape[0], (n - 1) % slab + 1
+        width = hidden.shape[1]
+        tail = GPUArray((last, width), bfloat16, ptr=hidden.device_ptr + 2 * width * (m - last), source=hidden)
+        return self._final(tail, self.buffers)
 
     # ------------------------------------------------------------------ device-resident step
     def decode_step_device(self) -> None:

@@ -490,3 +490,62 @@ def test_gemm_fp8_tc_against_float64(K, N, M):
     err = ctypes.c_int(7)
     api.gemm_fp8_wait_error(ctypes.byref(err))
     assert err.value == 0
+
+
+def _fp8_case(rng, K, N):
+    codes, _ = rand_fp8_weights(rng, N, K)
+    scale = bf16(np.exp2(rng.integers(-9, 3, (N // 128, K // 128))).astype(np.float32) * 1.5)
+    e, m = (codes >> 3) & 15, codes & 7
+    W = np.where(e > 0, np.exp2(e.astype(np.float64) - 7) * (1 + m / 8), np.exp2(-6.0) * m / 8) * np.where(codes & 128, -1, 1)
+    return codes, scale, W * np.repeat(np.repeat(f32(scale).astype(np.float64), 128, 0), 128, 1)
+
+
+@pytest.mark.parametrize("M", [65, 128, 129, 240, 256, 257, 300, 520])
+@pytest.mark.parametrize("K,N", [(128, 128), (384, 256), (1152, 1024), (4096, 384), (256, 19200)])
+def test_gemm_fp8_many_rows_against_float64(K, N, M):
+    """Prompts' products: last tiles of one and of two products, runs of tiles that mix both, a last launch of its own, k shared by a
+    cluster (unevenly), bias and a residual that is the output.  The bound is that of up to 64 rows."""
+    import ctypes
+    from pygpukit_b200._lib import api
+    if M * N > 300 * 19200:
+        pytest.skip("float64 reference")
+    rng = np.random.default_rng(K + N + M)
+    codes, scale, W = _fp8_case(rng, K, N)
+    A, bias, res = rand_bf16(rng, (M, K)), rand_bf16(rng, (N,), 0.1), rand_bf16(rng, (M, N), 0.5)
+    a = f32(A).astype(np.float64)
+    ref, size = a @ W.T, np.abs(a) @ np.abs(W).T
+    sums = 2.0 ** -24 * (128 + K / 128) * size + 1e-30
+    out, gA, gB, gS = gk.zeros((M, N), gk.bfloat16), gk.from_numpy(A), gk.from_numpy(codes), gk.from_numpy(scale)
+    api.gemv_fp8_bf16(gA.device_ptr, gB.device_ptr, gS.device_ptr, out.device_ptr, M, K, N, None)
+    got = f32(out.to_numpy()).astype(np.float64)
+    assert (np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + sums).all()
+    gb, inout = gk.from_numpy(bias), gk.from_numpy(res)
+    api.gemv_fp8_bf16_ex(gA.device_ptr, gB.device_ptr, gS.device_ptr, inout.device_ptr, M, K, N, gb.device_ptr, inout.device_ptr, None)
+    exp = f32(bf16(f32(out.to_numpy()) + f32(bias)[None, :])).astype(np.float64)      # the product and its sum with the bias are rounded
+    d = np.abs(f32(inout.to_numpy()).astype(np.float64) - (exp + f32(res)))
+    assert (d <= 2.0 ** -7 * (np.abs(exp) + np.abs(f32(res)) + np.abs(ref))).all()
+    err = ctypes.c_int(7)
+    api.gemm_fp8_wait_error(ctypes.byref(err))
+    assert err.value == 0
+
+
+@pytest.mark.parametrize("M,K,N", [(65, 128, 128), (130, 1152, 256), (300, 384, 1280), (200, 256, 9600)])
+def test_gemm_fp8_swiglu_many_rows_against_float64(M, K, N):
+    """Gate and up in one launch: g and u are rounded to BF16 (2^-9 relative beside their sums' error), silu has a slope of at most 1.1,
+    its value, the product and g, u carry one BF16 rounding each."""
+    from pygpukit_b200._lib import api
+    rng = np.random.default_rng(K + N + M)
+    cg, sg, Wg = _fp8_case(rng, K, N)
+    cu, su, Wu = _fp8_case(rng, K, N)
+    A = rand_bf16(rng, (M, K))
+    a = f32(A).astype(np.float64)
+    g, u = a @ Wg.T, a @ Wu.T
+    k = 2.0 ** -24 * (128 + K / 128)
+    eg = 2.0 ** -8 * np.abs(g) + k * (np.abs(a) @ np.abs(Wg).T)
+    eu = 2.0 ** -8 * np.abs(u) + k * (np.abs(a) @ np.abs(Wu).T)
+    s = g / (1 + np.exp(-np.clip(g, -700, 700)))
+    es = 1.1 * eg + 2.0 ** -8 * np.abs(s)
+    out, arrs = gk.zeros((M, N), gk.bfloat16), [gk.from_numpy(x) for x in (A, cg, sg, cu, su)]
+    api.gemv_fp8_swiglu_bf16(*(x.device_ptr for x in arrs), out.device_ptr, M, K, N, None)
+    got = f32(out.to_numpy()).astype(np.float64)
+    assert (np.abs(got - s * u) <= es * np.abs(u) + (np.abs(s) + es) * eu + 2.0 ** -8 * np.abs(s * u) + 1e-30).all()

@@ -385,3 +385,24 @@ def test_multi_sequence_decode_matches_single_sequence_runs(name, fmt, S):
             ulp = 2.0 ** (np.floor(np.log2(max(abs(lg[-1]), 1e-30))) - 7)
             assert lg[-1] - lg[-2] <= ulp, f"sequence {s}: token {same} differs ({together[s][same]} vs {alone[s][same]}), margin {lg[-1] - lg[-2]}"
         assert same >= 8, f"sequence {s}: only {same} identical tokens"
+
+
+@pytest.mark.parametrize("n", [17, 65, 130, 600])
+def test_long_prompt_portions_equal_slabs(n, monkeypatch):
+    """A prompt in portions of up to 512 rows and the same in slabs of 16: the hidden rows that come back are the last slab's (same count),
+    the caches and hidden rows agree within BF16 sums in another order, and decoding goes on from either."""
+    model = llm.build_random_model("tiny-qwen3", "fp8", max_seq=640, seed=7, std=0.05)
+    rng = np.random.default_rng(n)
+    prompt = [int(t) for t in rng.integers(0, model.config.vocab_size, n)]
+    model.init_decode(640, max_batch_size=16)
+    a, past = model(prompt, use_cache=True)
+    a, ka = f32(a.to_numpy()), [f32(k) for kv in model.snapshot_kv_cache() for k in kv]
+    monkeypatch.setattr(type(model), "_long_portions", lambda self: False)
+    model.init_decode(640, max_batch_size=16)
+    b, past2 = model(prompt, use_cache=True)
+    b, kb = f32(b.to_numpy()), [f32(k) for kv in model.snapshot_kv_cache() for k in kv]
+    assert a.shape == b.shape == ((n - 1) % 16 + 1, model.config.hidden_size) and past == past2 == n
+    # two layers, about ten BF16 roundings (2^-9 each) that may fall the other way
+    assert np.linalg.norm(a - b) <= 10 * 2.0 ** -9 * np.linalg.norm(b)
+    for x, y in zip(ka, kb):
+        assert np.linalg.norm(x - y) <= 10 * 2.0 ** -9 * np.linalg.norm(y)
