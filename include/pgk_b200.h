@@ -58,6 +58,9 @@ int pgk_host_alloc(void** host_ptr, size_t bytes);   /* pinned host memory */
 int pgk_host_free(void* host_ptr);
 int pgk_memset(void* ptr, int value, size_t bytes, void* stream);
 int pgk_memcpy_h2d(void* dst, const void* host_src, size_t bytes, void* stream);
+/* host -> device in stream order through pinned memory of the library: returns without waiting for the stream, and the source may
+ * change at once (up to 1 MB; larger copies wait).  Not during a capture. */
+int pgk_upload(void* dst, const void* host_src, size_t bytes, void* stream);
 int pgk_memcpy_d2h(void* host_dst, const void* src, size_t bytes, void* stream);
 int pgk_memcpy_d2d(void* dst, const void* src, size_t bytes, void* stream);
 
@@ -108,7 +111,8 @@ int pgk_gemv_fp8_swiglu_bf16(const void* A, const void* Wg_nk, const void* Sg, c
  * reference rounds weight*scale to BF16, w8a16_gemm.cu:104-339).  Needs 1 <= M <= 64 (rows up to the MMA
  * width 16/32/64 are zero-filled), K % 128 == 0, N % 128 == 0.  pgk_gemv_fp8_bf16(_ex) dispatch here by
  * themselves for M >= 5 (up to four rows keep the bits of the CUDA-core GEMV; env PGK_TC_MIN_M) when the shape
- * allows, and for M > 64, like pgk_gemv_fp8_swiglu_bf16, to a kernel of the same mathematics for many rows, (replaces gemv_fp8_bf16_batched, fp8_opt.cuh:220-295, and w8a16_gemm_sm120's mma.sync path). */
+ * allows, and for M > 64, like pgk_gemv_fp8_swiglu_bf16, to a kernel of the same mathematics for many rows (replaces
+ * gemv_fp8_bf16_batched, fp8_opt.cuh:220-295, and w8a16_gemm_sm120's mma.sync path). */
 int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void* S, void* C, int M, int K, int N,
                          const void* bias, const void* residual, void* stream);
 

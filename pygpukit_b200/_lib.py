@@ -32,7 +32,7 @@ _SIGS = {
     "pgk_malloc": [C.POINTER(vp), sz], "pgk_free": [vp],
     "pgk_host_alloc": [C.POINTER(vp), sz], "pgk_host_free": [vp],
     "pgk_memset": [vp, i32, sz, vp],
-    "pgk_memcpy_h2d": [vp, vp, sz, vp], "pgk_memcpy_d2h": [vp, vp, sz, vp], "pgk_memcpy_d2d": [vp, vp, sz, vp],
+    "pgk_memcpy_h2d": [vp, vp, sz, vp], "pgk_upload": [vp, vp, sz, vp], "pgk_memcpy_d2h": [vp, vp, sz, vp], "pgk_memcpy_d2d": [vp, vp, sz, vp],
     "pgk_stream_create": [C.POINTER(vp)], "pgk_stream_destroy": [vp], "pgk_stream_sync": [vp],
     "pgk_event_create": [C.POINTER(vp)], "pgk_event_destroy": [vp], "pgk_event_record": [vp, vp],
     "pgk_event_sync": [vp], "pgk_event_elapsed_ms": [vp, vp, C.POINTER(f32)],

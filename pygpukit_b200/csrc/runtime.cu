@@ -108,6 +108,77 @@ static bool scratch_trim() {
     return any;
 }
 
+// ---- staged uploads: the caller's bytes go to a pinned slot and from there in stream order, so that neither side waits for the other.
+// (A copy from pageable memory returns once the stream has come to it: a step's description, a few dozen KB, cost the host the whole
+// step before, and the device the 130 ... 200 us until the host had launched enough again.)  Eight slots, used by turns; a slot waits
+// for its last copy.  Copies above kUploadMax take the plain way and wait.
+struct UploadSlot {
+    void* host = nullptr;
+    size_t bytes = 0;
+    cudaEvent_t copied = nullptr;
+    int dev = -1;
+    bool used = false;                                                  // `copied` has been recorded
+};
+static constexpr size_t kUploadMax = 1ull << 20;
+static constexpr int kUploadSlots = 8;
+static UploadSlot g_upload[kUploadSlots];
+static int g_upload_next = 0;
+static std::mutex g_upload_mu;
+
+static int upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PGK_CUDA(cudaStreamIsCapturing(st, &cs));
+    PGK_REQUIRE(cs == cudaStreamCaptureStatusNone, "upload failed: a captured copy would repeat this call's bytes");
+    if (bytes > kUploadMax) {
+        PGK_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+        PGK_CUDA(cudaStreamSynchronize(st));
+        return wait_check();
+    }
+    int dev = 0;
+    PGK_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(g_upload_mu);
+    UploadSlot& s = g_upload[g_upload_next];
+    g_upload_next = (g_upload_next + 1) % kUploadSlots;
+    if (s.used) PGK_CUDA(cudaEventSynchronize(s.copied));
+    s.used = false;
+    if (s.bytes < bytes) {
+        if (s.host) PGK_CUDA(cudaFreeHost(s.host));
+        s.host = nullptr;
+        s.bytes = 0;
+        size_t n = 64 << 10;
+        while (n < bytes) n *= 2;
+        PGK_CUDA(cudaHostAlloc(&s.host, n, cudaHostAllocPortable));
+        s.bytes = n;
+    }
+    if (s.dev != dev) {
+        if (s.copied) PGK_CUDA(cudaEventDestroy(s.copied));
+        s.copied = nullptr;
+        s.dev = -1;
+        PGK_CUDA(cudaEventCreateWithFlags(&s.copied, cudaEventDisableTiming));
+        s.dev = dev;
+    }
+    memcpy(s.host, src, bytes);
+    PGK_CUDA(cudaMemcpyAsync(dst, s.host, bytes, cudaMemcpyHostToDevice, st));
+    const cudaError_t e = cudaEventRecord(s.copied, st);
+    if (e != cudaSuccess) {                                             // the copy may still read the slot
+        cudaStreamSynchronize(st);
+        return cuda_fail(e, "cudaEventRecord", __FILE__, __LINE__);
+    }
+    s.used = true;
+    return 0;
+}
+// slots whose copies are done go back
+static void upload_trim() {
+    std::lock_guard<std::mutex> lk(g_upload_mu);
+    for (UploadSlot& s : g_upload)
+        if (s.host && (!s.used || cudaEventQuery(s.copied) == cudaSuccess)) {
+            cudaFreeHost(s.host);
+            s.host = nullptr;
+            s.bytes = 0;
+            s.used = false;
+        }
+}
+
 // ---- bounded waits
 static std::mutex g_wait_mu;
 static std::atomic<int*> g_wait_words{nullptr};
@@ -216,6 +287,7 @@ int pgk_mem_info(size_t* free_bytes, size_t* total_bytes) {
 
 int pgk_mem_trim(void) {
     scratch_trim();
+    upload_trim();
     cudaGetLastError();
     return 0;
 }
@@ -252,6 +324,10 @@ int pgk_memset(void* ptr, int value, size_t bytes, void* stream) {
 int pgk_memcpy_h2d(void* dst, const void* host_src, size_t bytes, void* stream) {
     PGK_CUDA(cudaMemcpyAsync(dst, host_src, bytes, cudaMemcpyHostToDevice, S(stream)));
     return 0;
+}
+int pgk_upload(void* dst, const void* host_src, size_t bytes, void* stream) {
+    if (bytes == 0) return 0;
+    return pgk::upload(dst, host_src, bytes, S(stream));
 }
 int pgk_memcpy_d2h(void* host_dst, const void* src, size_t bytes, void* stream) {
     PGK_CUDA(cudaMemcpyAsync(host_dst, src, bytes, cudaMemcpyDeviceToHost, S(stream)));

@@ -55,6 +55,7 @@ class CausalTransformerModel:
         self.comm = comm
         self._buffers: DecodeBuffers | None = None
         self._prompt_bufs: PrefillBuffers | None = None
+        self._last_stream: tuple | None = None   # the stream of the last step
         self._max_seq = 0
         self._graph: CudaGraph | None = None
         self._graph_stream: Stream | None = None
@@ -147,8 +148,11 @@ class CausalTransformerModel:
         hidden = b.hidden if b.hidden.shape[0] == M else b.hidden.slice_rows(M)
         if token_ids is not None:
             ids = np.asarray(token_ids, np.int32)
-            api.memcpy_h2d(b.token_buf.device_ptr, ids.ctypes.data_as(C.c_void_p), ids.nbytes, _st())
-            api.stream_sync(_st()) if _st() is not None else api.device_sync()   # ids is pageable
+            stream = _st()
+            if self._last_stream is None or self._last_stream[0] is not stream:
+                api.device_sync()                # the step before ran on another stream, on the same arrays
+                self._last_stream = (stream,)
+            api.upload(b.token_buf.device_ptr, ids.ctypes.data_as(C.c_void_p), ids.nbytes, stream)
         self._embed_rows(hidden, M, start_position, None, b)
         return hidden
 
@@ -291,6 +295,7 @@ class CausalTransformerModel:
         """One greedy token entirely on the device: reads token_buf / position_buf / context_buf,
         writes the sampled token to next_token AND token_buf, then advances position / context."""
         b = self.buffers
+        self._last_stream = (_st(),)
         if getattr(self, "_num_sequences", 1) > 1:
             return self._decode_step_device_multi()
         step = self.step_program()
@@ -387,6 +392,7 @@ class CausalTransformerModel:
         b = self.buffers
         sh = self._graph_stream.handle
         api.memcpy_h2d(b.state_buf.device_ptr, pin, 12 * S, sh)
+        self._last_stream = (sh,)
         self._graph.replay(self._graph_stream)
         api.memcpy_d2h(pin.value + 12 * S, b.next_token.device_ptr, 4 * S, sh)
         api.stream_sync(sh)
@@ -408,6 +414,7 @@ class CausalTransformerModel:
 
     def decode_graph_replay(self) -> None:
         assert self._graph is not None, "Call init_decode_graph first"
+        self._last_stream = (self._graph_stream.handle,)
         self._graph.replay(self._graph_stream)
 
     # ------------------------------------------------------------------ generation

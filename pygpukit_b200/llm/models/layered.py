@@ -35,17 +35,15 @@ class StepContext:
 
     def __init__(self, model: "LayeredCausalModel", entries, tile_sizes: set[int], tops: set[int]):
         cache = model.cache
-        toks, slots, poss, want_rows, seqs, pars = [], [], [], [], [], []
+        toks, want_rows, seqs, pars = [], [], [], []
         row = 0
         for seq_id, tokens, want in entries:
             n = len(tokens)
             if n < 1:
                 raise ValueError(f"request {seq_id!r}: a step needs at least one token")
             slot, pos0 = cache.extend(seq_id, n)
-            toks.extend(int(t) for t in tokens)
-            slots.extend([slot] * n)
-            poss.extend(range(pos0, pos0 + n))
-            pars.extend([(cache.pool.steps(seq_id) - 1) & 1] * n)      # which copy of double-buffered state the step reads
+            toks.extend(tokens)
+            pars.append((cache.pool.steps(seq_id) - 1) & 1)        # which copy of double-buffered state the step reads
             for w in want:
                 if not 0 <= int(w) < n:
                     raise ValueError(f"request {seq_id!r}: wanted place {w} outside its {n} tokens")
@@ -56,8 +54,15 @@ class StepContext:
         self.max_rows = max(n for _, n, _, _ in seqs)          # the longest portion of the step
         self._seqs, self._model = seqs, model
         self.decode_only = all(n == 1 and p0 > 0 for _, n, _, p0 in seqs)
-        parts = [np.asarray(toks, np.int32), np.asarray(slots, np.int32), np.asarray(poss, np.int32),
-                 np.asarray(want_rows, np.int32)]
+        desc = np.asarray(seqs, np.int32)
+        first, rows, slot_of, pos_of = desc.T
+        of_row = np.repeat(np.arange(len(seqs)), rows)          # sequence of every row
+        within = np.arange(row, dtype=np.int32) - first[of_row]
+        try:
+            tok = np.asarray(toks, np.int32)
+        except (TypeError, ValueError):                         # anything else that int() takes
+            tok = np.asarray([int(t) for t in toks], np.int32)
+        parts = [tok, slot_of[of_row], pos_of[of_row] + within, np.asarray(want_rows, np.int32)]
         off = {"tok": 0, "slot": self.T, "pos": 2 * self.T, "want": 3 * self.T}
         cur = 3 * self.T + self.n_want
         self._rows_off = {}
@@ -73,24 +78,25 @@ class StepContext:
             if pad:
                 parts.append(np.zeros(pad, np.int32))
                 cur += pad
-            t = [(r0 + i, min(qt, n - i), slot, p0 + i) for r0, n, slot, p0 in seqs for i in range(0, n, qt)]
-            parts.append(np.asarray(t, np.int32).reshape(-1))
+            starts = within % qt == 0              # rows that open a tile
+            o, i = of_row[starts], within[starts]
+            t = np.stack([first[o] + i, np.minimum(qt, rows[o] - i), slot_of[o], pos_of[o] + i], axis=1)
+            parts.append(t.reshape(-1))
             self._tiles_off[qt] = (cur, len(t))
             cur += 4 * len(t)
         pad = (-cur) % 4                           # one (first row, rows, slot, first position) per sequence, int4 loads
         if pad:
             parts.append(np.zeros(pad, np.int32))
             cur += pad
-        parts.append(np.asarray(seqs, np.int32).reshape(-1))
+        parts.append(desc.reshape(-1))
         self._seqs_off = cur
         cur += 4 * len(seqs)
-        parts.append(np.asarray(pars, np.int32))
+        parts.append(np.asarray(pars, np.int32)[of_row])
         par_off = cur
         cur += self.T
-        meta = np.concatenate(parts)
+        meta = np.concatenate(parts, dtype=np.int32)
         self.meta = model._meta_buffer(meta.size)
-        api.memcpy_h2d(self.meta.device_ptr, meta.ctypes.data, meta.nbytes, _st())
-        api.stream_sync(_st()) if _st() is not None else api.device_sync()
+        api.upload(self.meta.device_ptr, meta.ctypes.data, meta.nbytes, _st())
         base = self.meta.device_ptr
         self.tok_ptr, self.slot_ptr, self.pos_ptr, self.want_ptr = (base + 4 * off[k] for k in ("tok", "slot", "pos", "want"))
         self._base = base
@@ -149,7 +155,8 @@ class LayeredCausalModel:
         self.use_graphs = os.environ.get("PGK_LAYERED_GRAPH", "1") != "0"
         self._graphs: dict = {}
         self._graph_warm: set = set()
-        self._gstream: Stream | None = None
+        self._gstream: Stream | None = None            # captures
+        self._last_stream: tuple | None = None         # the stream of the last step
         self._tile_sizes = {b.mixer.queries_per_tile for b in blocks if b.mixer.queries_per_tile}
         self._tops = {getattr(b.mlp.spec, "slots", b.mlp.spec.top) for b in blocks if b.mlp is not None and b.mlp.spec.kind == "moe"}
 
@@ -160,6 +167,8 @@ class LayeredCausalModel:
         states = [tuple(getattr(self.blocks[li], "state_shapes", ())) for li, _ in self.runs]
         pools = [getattr(self.blocks[li].mixer.spec, "pool", 0) for li, _ in self.runs]
         self.cache = PagedKVCache(shapes, self.dtype, page_size, max_tokens, slots, state_shapes=states, pools=pools)
+        if self._graphs:
+            api.device_sync()
         self._graphs.clear()
         self._graph_warm.clear()
         return self.cache
@@ -233,6 +242,10 @@ class LayeredCausalModel:
             for seq_id in end:
                 self.cache.release(seq_id)
             return None, 0
+        stream = _st()
+        if self._last_stream is None or self._last_stream[0] is not stream:
+            api.device_sync()                          # the step before ran on another stream, on the same arrays
+            self._last_stream = (stream,)
         ctx = StepContext(self, entries, self._tile_sizes, self._tops)
         if self._out is None or self._out.shape[0] < max(ctx.n_want, 1):
             self._out = GPUArray((max(ctx.n_want, 16), V), float32)
@@ -250,15 +263,14 @@ class LayeredCausalModel:
                 if self._gstream is None:
                     self._gstream = Stream()
                 if g is None:
-                    if len(self._graphs) >= 64:
-                        self._graphs.clear()
                     g = CudaGraph()
                     api.device_sync()
+                    if len(self._graphs) >= 64:
+                        self._graphs.clear()
                     with g.capture(self._gstream):
                         self._forward(ctx)
                     self._graphs[key] = g
-                g.replay(self._gstream)
-                self._gstream.synchronize()
+                api.graph_launch(g._exec, stream)      # in the caller's order, like an eager step
         for seq_id in end:
             self.cache.release(seq_id)
         return (self._out if ctx.n_want else None), ctx.n_want

@@ -236,7 +236,7 @@ class PagedKVCache:
         t = self.pool.table
         if self.table_dev.size != t.size:
             self.table_dev = GPUArray((t.size,), int32)
-        self.table_dev.copy_from_numpy(t.reshape(-1))
+        api.upload(self.table_dev.device_ptr, t.ctypes.data, t.nbytes, _st())       # a copy is taken: `t` may change at once
         self.pool.dirty = False
 
     @property

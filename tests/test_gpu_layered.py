@@ -522,3 +522,39 @@ def test_loader_picks_the_family_from_config_json(tmp_path):
         bad = dict(P)
         bad["l0.mix.q"] = P["l0.mix.q"][:-1]
         llm.build_layered_model(layered_config_from_json(cfg), bad, "float32")
+
+
+def test_steps_do_not_wait_and_keep_their_order():
+    """Steps enqueued one after another without a wait -- prompts of several requests, decode steps that replay a graph, a change of stream
+    in between -- give the logits of steps that are each waited for.  A step under capture is refused."""
+    from pygpukit_b200.core.stream import CudaGraph, Stream, current_stream_handle, use_stream
+
+    def run(wait, streams):
+        cfg, _, m = make("mixed_stack")
+        prompts = [tokens(cfg, n, seed=50 + n) for n in (37, 1, 64, 5)]
+        kept = []
+        for i in range(13):
+            with use_stream(streams[i % len(streams)]):
+                if i == 0:
+                    out, n = m.step_device([(r, p, [len(p) - 1]) for r, p in enumerate(prompts)])
+                else:
+                    out, n = m.step_device([(r, [t], [0]) for r, t in enumerate(tokens(cfg, 4, seed=i))])
+                kept.append(gk.empty((n, cfg["vocab"]), gk.float32))
+                api.memcpy_d2d(kept[-1].device_ptr, out.device_ptr, kept[-1].nbytes, current_stream_handle())
+            if wait:
+                api.device_sync()
+        api.device_sync()
+        return [k.to_numpy() for k in kept], m
+
+    a, m = run(True, [None])
+    b, _ = run(False, [None])
+    s1, s2 = Stream(), Stream()
+    c, _ = run(False, [None, None, s1, s1, s2])
+    for x, y, z in zip(a, b, c):
+        assert np.array_equal(x, y) and np.array_equal(x, z)
+    m.step([("warm", [1, 2, 3], [0])])
+    m._last_stream = (s1.handle,)                        # the refusal of the upload itself, not of a wait before it
+    with pytest.raises(RuntimeError, match="capture"):
+        with CudaGraph().capture(s1):
+            m.step_device([("new", [1, 2, 3], [0])])
+    api.device_sync()
