@@ -41,6 +41,7 @@ SOURCES = {
     "gemm_tc_f8.cu": [],
     "elementwise.cu": [],
     "attention.cu": [],
+    "attention_tc.cu": [],
     "moe.cu": [],
     "sampling.cu": [],
     "comm.cu": [],
