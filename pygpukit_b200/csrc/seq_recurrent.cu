@@ -19,6 +19,13 @@
 #include "common.cuh"
 #include "../../include/pgk_b200.h"
 
+namespace pgk {
+// seq_linear_tc.cu: long prompts on the tensor cores
+bool linear_tc_ok(const float* proj, int ld, int q_off, int k_off, int v_off, const float* out, int ldo, const float* state, int D, int Dv, const float* ws);
+int linear_tc(const float* proj, int ld, int q_off, int k_off, int v_off, float* out, int ldo, float* state, const float* decay, const int32_t* seqs, int n_seqs,
+              int H, int D, int Dv, int begin, int end, float* ws, cudaStream_t st);
+}  // namespace pgk
+
 using namespace pgk;
 
 namespace {
@@ -598,6 +605,12 @@ int pgk_seq_linear_attention_chunks(const float* proj, int ld, int q_off, int k_
                                     int chunk_begin, int chunks, float* workspace, void* stream) {
     PGK_REQUIRE(heads > 0 && dim > 0 && vdim > 0 && chunk_begin >= 0 && workspace, "seq_linear_attention_chunks failed: invalid arguments");
     if (n_seqs <= 0 || chunks <= 0) return 0;
+    // Small heads in few chunks do not fill what 128 tokens and 128 x 128 elements take (us, here / there: 16 heads of 64 x 64, 200 tokens 29 / 31,
+    // 400 tokens 35 / 31; 8 heads 400 29.8 / 31, 800 35 / 31; 64 x 128, 130 tokens of two heads 37 / 37, 100 of sixteen 39.7 / 35)
+    const long elements = (long)dim * vdim;
+    if ((elements >= 8192 || (elements >= 4096 && (long)heads * chunks * n_seqs >= 200)) && pgk::linear_tc_ok(proj, ld, q_off, k_off, v_off, out, ldo, state, dim, vdim, workspace))
+        return pgk::linear_tc(proj, ld, q_off, k_off, v_off, out, ldo, state, decay, seqs, n_seqs, heads, dim, vdim, chunk_begin * LC, (chunk_begin + chunks) * LC,
+                              workspace, (cudaStream_t)stream);
     const int D4 = (dim + 3) & ~3, V4 = (vdim + 3) & ~3;
     const size_t smem1 = sizeof(float) * ((size_t)LC * D4 + (size_t)LC * V4);
     const size_t smem3 = sizeof(float) * (2 * (size_t)LC * (dim + 1) + 2 * (size_t)LC * V4 + LC * (LC + 1) + LC + 1);

@@ -108,3 +108,60 @@ def test_turned_heads_of_any_length(H, D, rot):
     qk[:, H:] *= 0.25
     ref = np.concatenate([qk.reshape(T, -1), s[:, 2 * H * D:]], 1)
     assert np.abs(p.to_numpy() - ref).max() <= 2.0 ** -20 * (1 + np.abs(s).max())
+
+
+@pytest.mark.parametrize("lens,heads,dim,vdim", [([128], 2, 128, 128), ([129, 1, 300], 2, 128, 72), ([70, 257], 3, 72, 128), ([640], 20, 64, 64), ([33, 127], 4, 128, 64)])
+@pytest.mark.parametrize("start", [0, 9])
+def test_linear_attention_chunks_against_float64(lens, heads, dim, vdim, start):
+    """Chunks of 128 tokens: ragged sequences that end inside, on and behind a chunk's edge, heads that do not fill a tile, states carried in and
+    from one segment to the next.  Operands keep 24 bits and sums are float32, so errors stay within a few 2^-24 of the sums of magnitudes."""
+    rng = np.random.default_rng(sum(lens) + dim)
+    T, S, ld = sum(lens), len(lens), 2 * heads * dim + heads * vdim + 4
+    proj = rng.standard_normal((T, ld)).astype(np.float32)
+    decay = (1 - 2.0 ** -np.linspace(3, 9, heads)).astype(np.float32)
+    state = rng.standard_normal((S, heads, dim, vdim)).astype(np.float32)
+    rows = np.cumsum([0] + lens)
+    seqs = np.array([(rows[i], n, i, start) for i, n in enumerate(lens)], np.int32)
+    k_off, v_off, chunks = heads * dim, 2 * heads * dim, -(-max(lens) // 32)
+    gp, gs, gd, gq = gk.from_numpy(proj), gk.from_numpy(state), gk.from_numpy(decay), gk.from_numpy(seqs)
+    out, ws = gk.zeros((T, heads * vdim), gk.float32), gk.zeros((chunks * S * heads * dim * vdim,), gk.float32)
+    for c0, n in ((0, 5), (5, chunks - 5)) if chunks > 5 else ((0, chunks),):
+        api.seq_linear_attention_chunks(gp.device_ptr, ld, 0, k_off, v_off, out.device_ptr, heads * vdim, gs.device_ptr, gd.device_ptr, gq.device_ptr, S,
+                                        heads, dim, vdim, c0, n, ws.device_ptr, None)
+    got, after = out.to_numpy().astype(np.float64), gs.to_numpy().astype(np.float64)
+    for i, n in enumerate(lens):
+        x = proj[rows[i]:rows[i + 1]].astype(np.float64)
+        t = np.arange(n)
+        for h in range(heads):
+            q, k, v = x[:, h * dim:(h + 1) * dim], x[:, k_off + h * dim:k_off + (h + 1) * dim], x[:, v_off + h * vdim:v_off + (h + 1) * vdim]
+            a, s0 = float(decay[h]), state[i, h].astype(np.float64) * (start > 0)
+            w = np.where(t[:, None] >= t[None], a ** np.maximum(t[:, None] - t[None], 0), 0.0)
+            fall, rest = (a ** (t + 1.0))[:, None], (a ** (n - 1.0 - t))[:, None]
+            ref, size = (q @ k.T * w) @ v + fall * (q @ s0), (np.abs(q) @ np.abs(k).T * w) @ np.abs(v) + fall * (np.abs(q) @ np.abs(s0))
+            sref, ssize = a ** n * s0 + (k * rest).T @ v, a ** n * np.abs(s0) + (np.abs(k) * rest).T @ np.abs(v)
+            assert (np.abs(got[rows[i]:rows[i + 1], h * vdim:(h + 1) * vdim] - ref) <= 64 * 2.0 ** -24 * size).all()
+            assert (np.abs(after[i, h] - sref) <= 64 * 2.0 ** -24 * ssize).all()
+
+
+def test_linear_attention_chunks_with_an_infinite_value():
+    """float32 semantics: the outputs that see the value are infinite or NaN, all others are untouched."""
+    rng = np.random.default_rng(3)
+    T, heads, dim, vdim = 300, 2, 128, 64
+    ld = 2 * heads * dim + heads * vdim
+    proj = np.abs(rng.standard_normal((T, ld))).astype(np.float32)
+    decay, seqs = np.full(heads, 0.99, np.float32), np.array([(0, T, 0, 0)], np.int32)
+
+    def run(p):
+        bufs = [gk.from_numpy(p), gk.zeros((1, heads, dim, vdim), gk.float32), gk.from_numpy(decay), gk.from_numpy(seqs),
+                gk.zeros((T, heads * vdim), gk.float32), gk.zeros((10 * heads * dim * vdim,), gk.float32)]
+        x, s, d, q, o, w = (b.device_ptr for b in bufs)
+        api.seq_linear_attention_chunks(x, ld, 0, heads * dim, 2 * heads * dim, o, heads * vdim, s, d, q, 1, heads, dim, vdim, 0, 10, w, None)
+        return bufs[4].to_numpy()
+
+    a = run(proj)
+    proj[150, 2 * heads * dim + 7] = np.inf
+    b = run(proj)
+    assert np.isposinf(b[150:, 7]).all()
+    keep = np.ones_like(a, bool)
+    keep[150:, 7] = False
+    assert np.isfinite(b[keep]).all() and np.abs(b - a)[keep].max() <= 1e-5 * np.abs(a).max()
