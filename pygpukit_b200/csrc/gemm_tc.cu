@@ -22,7 +22,10 @@
 //     its partial rows to their owners' shared memory and adds them in the order of the ranks: no work memory.
 // Measured on B200 (us, cp.async and conversion through shared memory -> here), M = 5 / 64: 14336 x 4096 35 / 43 -> 20.7 / 24.5,
 // 4096 x 4096 16.5 / 26.8 -> 10.5 / 13.9, 1024 x 4096 10.9 / 21.3 -> 8.3 / 10.4, 14336 x 14336 103 / 134 -> 55 / 65 (3.7 / 3.2 TB/s).
+// Gate, up and their activation in one launch (PAIR; 64 rows, 14336 x 4096 and back): two products, silu, product and the down projection 85.2 us,
+// with the pair in one launch 57.5, the same bits.
 #include "common.cuh"
+#include "gemv_common.cuh"
 #include "tc_common.cuh"
 #include "tma.cuh"
 #include "../../include/pgk_b200.h"
@@ -43,7 +46,7 @@ __host__ __device__ constexpr uint32_t f_stage_bytes(int nb) { return F_W_BYTES 
 __host__ __device__ constexpr size_t f_smem(int nb) { return (size_t)f_stages(nb) * f_stage_bytes(nb) + 1024; }
 
 struct F8TcParams {
-    const uint16_t* S; uint16_t* C;
+    const uint16_t* S; const uint16_t* S1; uint16_t* C;          // scales (of gate and up), output
     const uint16_t* bias; const uint16_t* residual;
     int M, K, N, splits, kper;
     int* err;                                     // raised when a bounded wait runs out
@@ -59,25 +62,32 @@ __device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t& lo, uint3
     hi = pack_bf16x2(f1.x, f1.y);
 }
 
-template <int NB>
+// PAIR: a tile is 64 rows of a gate and 64 of an up matrix, by turns of 16, so that a lane's partner is 16 lanes on; C = silu(gate) * up
+template <int NB, bool PAIR>
 __global__ void __launch_bounds__(F_THREADS, 2)
-gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap amap, const __grid_constant__ F8TcParams p) {
+gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap umap, const __grid_constant__ CUtensorMap amap,
+                   const __grid_constant__ F8TcParams p) {
     constexpr int STAGES = f_stages(NB), COLS = NB / 2;          // columns of a warp
     constexpr uint32_t STAGE = f_stage_bytes(NB), TMEM_COLS = 2 * NB + 128 <= 256 ? 256 : 512;
     static_assert(TMEM_COLS == 256, "two blocks per SM");
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], w_bar[2], d_bar[2];
     __shared__ uint32_t tmem_base_s;
-    __shared__ float sc_s[kTcMaxKb];
+    __shared__ float sc_s[(PAIR ? 2 : 1) * kTcMaxKb];
+    constexpr int OUT = PAIR ? kTcRows / 2 : kTcRows;            // columns of C per tile
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
     const uint32_t wb = smem_u32(w_bar), db = smem_u32(d_bar);
     int* const err = p.err;
-    const int rank = blockIdx.x, n0 = blockIdx.y * kTcRows, nkb_total = p.K / kTcBK;
+    const int rank = blockIdx.x, n0 = blockIdx.y * OUT, nkb_total = p.K / kTcBK;
     const int kb0 = rank * p.kper, nkb = max(0, min(nkb_total, kb0 + p.kper) - kb0);
 
     // the block's scales are weights: staged before the dependency wait
-    for (int i = tid; i < nkb; i += F_THREADS) sc_s[i] = bf16_bits_to_f32(__ldg(p.S + (size_t)blockIdx.y * nkb_total + kb0 + i));
+    const size_t scales = (size_t)(blockIdx.y >> (PAIR ? 1 : 0)) * nkb_total + kb0;
+    for (int i = tid; i < nkb; i += F_THREADS) {
+        sc_s[i] = bf16_bits_to_f32(__ldg(p.S + scales + i));
+        if (PAIR) sc_s[kTcMaxKb + i] = bf16_bits_to_f32(__ldg(p.S1 + scales + i));
+    }
     if (warp == F_WARPS + 1) tmem_alloc(&tmem_base_s, TMEM_COLS);
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
@@ -100,7 +110,14 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             const uint64_t once = l2_evict_first();
             auto weights = [&](int it, uint32_t s) {
                 mbar_expect_tx(full + 8u * s, STAGE);
-                tma_load_2d_hint(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s, once);
+                if constexpr (PAIR) {
+#pragma unroll 1
+                    for (int q = 0; q < 4; ++q) {
+                        tma_load_2d_hint(ring + s * STAGE + (uint32_t)q * 4096u, &wmap, (kb0 + it) * kTcBK, n0 + q * 16, full + 8u * s, once);
+                        tma_load_2d_hint(ring + s * STAGE + (uint32_t)q * 4096u + 2048u, &umap, (kb0 + it) * kTcBK, n0 + q * 16, full + 8u * s, once);
+                    }
+                } else
+                    tma_load_2d_hint(ring + s * STAGE, &wmap, (kb0 + it) * kTcBK, n0, full + 8u * s, once);
             };
             auto rows = [&](int it, uint32_t s) {
                 const uint32_t at = ring + s * STAGE + F_W_BYTES;
@@ -160,7 +177,7 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             ok = ok && bar_wait(err, db + 8u * b, (uint32_t)(it >> 1) & 1u);
             __syncwarp();
             tc_fence_after();
-            const float sc = sc_s[it];
+            const float sc = sc_s[(PAIR && (lane & 16) ? kTcMaxKb : 0) + it];
             const uint32_t at = tmem + lanes + b * NB + (uint32_t)half * COLS;
             if constexpr (COLS == 8) {
                 float v[8];
@@ -209,6 +226,10 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
 
     // ---------------- outputs
     const int rows_here = min(NB, p.M);
+    auto store_pair = [&](float g, float u, int m, int n) {
+        p.C[(size_t)m * p.N + n] = f32_to_bf16_bits(round_bf16(silu_ref(round_bf16(g))) * round_bf16(u));
+    };
+    const bool up = PAIR && (lane & 16);
     auto store = [&](float x, int m, int n) {
         const size_t o = (size_t)m * p.N + n;
         if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[n]);
@@ -217,9 +238,18 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
     if (p.splits == 1) {
         if (warp < F_WARPS) {
+            if constexpr (PAIR) {
 #pragma unroll
-            for (int j = 0; j < COLS; ++j)
-                if (half * COLS + j < rows_here) store(acc[j], half * COLS + j, n0 + row);
+                for (int j = 0; j < COLS; j += 2) {           // a lane takes its partner's value of every second row for its own of the others
+                    const float got = __shfl_xor_sync(0xffffffffu, up ? acc[j] : acc[j + 1], 16);
+                    const int m = half * COLS + j + (up ? 1 : 0);
+                    if (m < rows_here) store_pair(up ? got : acc[j], up ? acc[j + 1] : got, m, n0 + quad * 16 + (lane & 15));
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < COLS; ++j)
+                    if (half * COLS + j < rows_here) store(acc[j], half * COLS + j, n0 + row);
+            }
         }
     } else {                                                  // column m belongs to block m % splits
         const int slots = (rows_here + p.splits - 1) / p.splits;
@@ -246,7 +276,11 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             for (int slot = half; slot * p.splits + rank < rows_here; slot += 2) {
                 float x = 0.f;
                 for (int s = 0; s < parts; ++s) x += part[(s * slots + slot) * kTcRows + row];
-                store(x, slot * p.splits + rank, n0 + row);
+                if constexpr (PAIR) {
+                    const float u = __shfl_xor_sync(0xffffffffu, x, 16);
+                    if (!up) store_pair(x, u, slot * p.splits + rank, n0 + quad * 16 + lane);
+                } else
+                    store(x, slot * p.splits + rank, n0 + row);
             }
         }
     }
@@ -255,11 +289,11 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     if (warp == F_WARPS + 1) tmem_dealloc(tmem, TMEM_COLS);
 }
 
-template <int NB>
+template <int NB, bool PAIR>
 cudaError_t f8tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int splits) {
     static bool configured = false;
     if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f_smem(NB));
+        const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_tc_kernel<NB, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f_smem(NB));
         if (e != cudaSuccess) return e;
         configured = true;
     }
@@ -282,7 +316,7 @@ int f8tc_held(int s) {
         cudaLaunchAttribute at[2];
         int n = 0;
         cfg.gridDim = dim3(s, 64);
-        if (f8tc_config<64>(&cfg, at, s) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_fp8_tc_kernel<64>, &cfg) != cudaSuccess) {
+        if (f8tc_config<64, false>(&cfg, at, s) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_fp8_tc_kernel<64, false>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
         }
@@ -308,20 +342,21 @@ int f8tc_splits(int tiles, int nkb) {
     return best;
 }
 
-template <int NB>
-int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
-    const int tiles = p.N / kTcRows, nkb = p.K / kTcBK;
+template <int NB, bool PAIR>
+int launch_f8tc(F8TcParams p, const void* A, const void* B, const void* B1, cudaStream_t st) {
+    const int tiles = p.N / (PAIR ? kTcRows / 2 : kTcRows), nkb = p.K / kTcBK;
     p.splits = f8tc_splits(tiles, nkb);
     p.kper = (nkb + p.splits - 1) / p.splits;
     p.err = wait_word(kWaitFp8);
     PGK_REQUIRE(p.err, "gemm_fp8_tc failed: no pinned host memory");
     PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8_tc failed: the driver does not export cuTensorMapEncodeTiled");
-    CUtensorMap wmap, amap;
-    PGK_REQUIRE(tma_map_bytes_2d(&wmap, B, (uint64_t)p.K, (uint64_t)p.N, kTcBK, kTcRows) &&
+    CUtensorMap wmap, umap, amap;
+    const uint32_t box = PAIR ? 16 : kTcRows;
+    PGK_REQUIRE(tma_map_bytes_2d(&wmap, B, (uint64_t)p.K, (uint64_t)p.N, kTcBK, box) && tma_map_bytes_2d(&umap, B1, (uint64_t)p.K, (uint64_t)p.N, kTcBK, box) &&
                 tma_map_bf16_2d(&amap, A, (uint64_t)p.K, (uint64_t)p.M, (uint64_t)p.K * 2, 64, NB), "gemm_fp8_tc failed: cuTensorMapEncodeTiled refused the operands");
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[2];
-    PGK_CUDA(f8tc_config<NB>(&cfg, at, p.splits));
+    PGK_CUDA((f8tc_config<NB, PAIR>(&cfg, at, p.splits)));
     cfg.gridDim = dim3(p.splits, tiles);
     cfg.stream = st;
     if (pdl_enabled()) {
@@ -329,7 +364,7 @@ int launch_f8tc(F8TcParams p, const void* A, const void* B, cudaStream_t st) {
         at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     }
     count_launch();
-    PGK_CUDA(cudaLaunchKernelEx(&cfg, gemm_fp8_tc_kernel<NB>, wmap, amap, p));
+    PGK_CUDA(cudaLaunchKernelEx(&cfg, gemm_fp8_tc_kernel<NB, PAIR>, wmap, umap, amap, p));
     return 0;
 }
 
@@ -365,9 +400,19 @@ int gemm_fp8_tc(const void* A, const void* B_nk, const void* S, void* C, int M, 
     p.S = (const uint16_t*)S; p.C = (uint16_t*)C;
     p.bias = (const uint16_t*)bias; p.residual = (const uint16_t*)residual;
     p.M = M; p.K = K; p.N = N;
-    if (M <= 16) return launch_f8tc<16>(p, A, B_nk, st);
-    if (M <= 32) return launch_f8tc<32>(p, A, B_nk, st);
-    return launch_f8tc<64>(p, A, B_nk, st);
+    if (M <= 16) return launch_f8tc<16, false>(p, A, B_nk, B_nk, st);
+    if (M <= 32) return launch_f8tc<32, false>(p, A, B_nk, B_nk, st);
+    return launch_f8tc<64, false>(p, A, B_nk, B_nk, st);
+}
+
+// silu(A . Wg^T) * (A . Wu^T) with the roundings of the two products, silu and the product (for shapes that gemm_fp8_tc takes)
+int gemm_fp8_tc_pair(const void* A, const void* Wg, const void* Sg, const void* Wu, const void* Su, void* C, int M, int K, int N, cudaStream_t st) {
+    F8TcParams p = {};
+    p.S = (const uint16_t*)Sg; p.S1 = (const uint16_t*)Su; p.C = (uint16_t*)C;
+    p.M = M; p.K = K; p.N = N;
+    if (M <= 16) return launch_f8tc<16, true>(p, A, Wg, Wu, st);
+    if (M <= 32) return launch_f8tc<32, true>(p, A, Wg, Wu, st);
+    return launch_f8tc<64, true>(p, A, Wg, Wu, st);
 }
 
 }  // namespace pgk

@@ -35,6 +35,8 @@ bool gemm_fp8_tc_eligible(int M, int K, int N, const void* A, const void* B);
 int gemm_fp8_tc(const void* A, const void* B_nk, const void* S, void* C, int M, int K, int N, const void* bias,
                 const void* residual, cudaStream_t st);
 
+int gemm_fp8_tc_pair(const void* A, const void* Wg, const void* Sg, const void* Wu, const void* Su, void* C, int M, int K, int N, cudaStream_t st);
+
 // gemm_tc_rows.cu: the same for M > 64; B1: gate and up matrix, silu(gate) * up
 bool gemm_fp8_rows_ok(int M, int K, int N, const void* A, const void* B0, const void* B1);
 int gemm_fp8_rows(const void* A, const void* B0, const void* S0, const void* B1, const void* S1, void* C, int M, int K, int N, const void* bias,
@@ -370,6 +372,8 @@ static int gemv_fp8_dispatch(const void* A, const void* B0, const void* S0, cons
         return gemm_fp8_f8(A, B0, S0, C, M, K, N, bias, residual, st);
     if (tc_on && clean && !swiglu && !gamma && gemm_fp8_tc_eligible(M, K, N, A, B0))
         return gemm_fp8_tc(A, B0, S0, C, M, K, N, bias, residual, st);
+    if (tc_on && clean && swiglu && !gamma && gemm_fp8_tc_eligible(M, K, N, A, B0) && (uintptr_t)B1 % 16 == 0)
+        return gemm_fp8_tc_pair(A, B0, S0, B1, S1, C, M, K, N, st);
     if (tc_on && clean && !gamma && M >= gemm_fp8_tc_min_m() && gemm_fp8_rows_ok(M, K, N, A, B0, B1))
         return gemm_fp8_rows(A, B0, S0, B1, S1, C, M, K, N, bias, residual, st);
     if (!fast) {

@@ -87,16 +87,20 @@ class MLP:
         M, K, I = x.shape[0], x.shape[1], self.intermediate_size
         if out is None:
             out = GPUArray((M, I), bfloat16)
-        if (M > 64 and norm is None and self._fp8_pair() and self.gate_proj.uses_tensor_cores(M)
-                and self.up_proj.uses_tensor_cores(M)):
-            # prompts: both products, silu and mul in one launch, with the layer path's roundings
+        if self._fp8_pair() and self.gate_proj.uses_tensor_cores(M) and self.up_proj.uses_tensor_cores(M):
+            # from TC_MIN_M rows on: both products, silu and mul in one launch, with the layer path's roundings
+            if norm is not None:
+                xs = self._scratch.get(("x", M))
+                if xs is None:
+                    xs = self._scratch[("x", M)] = GPUArray((M, K), bfloat16)
+                x = norm(x, out=xs)
             g, u = self.gate_proj, self.up_proj
             api.gemv_fp8_swiglu_bf16(x.device_ptr, g.weight_fp8.device_ptr, g.scale_inv.device_ptr,
                                      u.weight_fp8.device_ptr, u.scale_inv.device_ptr, out.device_ptr, M, K, I, _st())
             return out
         if (self.gate_up_proj is None and isinstance(self.gate_proj, LinearFP8) and isinstance(self.up_proj, LinearFP8)
                 and self.gate_proj.uses_tensor_cores(M) and self.up_proj.uses_tensor_cores(M)):
-            # batch >= TC_MIN_M: gate and up on the tcgen05 GEMM, then silu -> mul with the layer path's two roundings
+            # products with a bias: gate and up one after the other, then silu -> mul with the layer path's two roundings
             if norm is not None:
                 xs = self._scratch.get(("x", M))
                 if xs is None:

@@ -529,7 +529,8 @@ def test_gemm_fp8_many_rows_against_float64(K, N, M):
     assert err.value == 0
 
 
-@pytest.mark.parametrize("M,K,N", [(65, 128, 128), (130, 1152, 256), (300, 384, 1280), (200, 256, 9600)])
+@pytest.mark.parametrize("M,K,N", [(65, 128, 128), (130, 1152, 256), (300, 384, 1280), (200, 256, 9600), (5, 128, 128), (16, 1152, 256), (17, 4096, 384),
+                                   (33, 384, 1280), (64, 256, 9600)])
 def test_gemm_fp8_swiglu_many_rows_against_float64(M, K, N):
     """Gate and up in one launch: g and u are rounded to BF16 (2^-9 relative beside their sums' error), silu has a slope of at most 1.1,
     its value, the product and g, u carry one BF16 rounding each."""
