@@ -384,7 +384,7 @@ static int launch_sdpa(SdpaParams p, cudaStream_t st) {
         PGK_CUDA(cudaFuncSetAttribute(sdpa_decode_kernel<DT, HD, RT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
         attr_set = true;
     }
-    PGK_CUDA(launch(sdpa_decode_kernel<DT, HD, RT>, dim3(splits, row_tiles, p.n_kv), dim3(kAttnWarps * 32), kSmem, st, p));
+    PGK_CUDA(launch_waiting(sdpa_decode_kernel<DT, HD, RT>, dim3(splits, row_tiles, p.n_kv), dim3(kAttnWarps * 32), kSmem, st, p));
     return 0;
 }
 
@@ -413,6 +413,7 @@ struct RopeSdpaParams {
     float scale_log2;
     int splits;
     uint2* ll; unsigned* gen;                  // LL partial words {f32 bits, exchange number}, per-record generation
+    int ahead;                                 // position, tables and the first tiles are read before the kernel before has finished
     int box_rows;                              // rows of one TMA box = min(64, max_seq)
     // multi-sequence decode (continuous batching, native/ops/batch/continuous_batching.cuh:70-245): n_seq independent
     // sequences, each with its own cache region, position and context length (pos_buf / ctx_buf are then arrays)
@@ -527,6 +528,7 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
     const uint32_t tiles_s = (smem_u32(dyn_raw) + 1023u) & ~1023u;      // the swizzle pattern repeats every 1024 bytes
     unsigned char* tiles_g = dyn_raw + (tiles_s - smem_u32(dyn_raw));
 
+    if (!p.ahead) griddep_wait();
     // ---- independent of the previous kernel: position, barriers, the first K/V tiles, tables
     const int pos = p.pos_buf ? p.pos_buf[seq] : p.pos;
     const int ctx = min(p.ctx_buf ? p.ctx_buf[seq] : p.context_len, p.max_seq);
@@ -928,7 +930,7 @@ static int launch_rope_sdpa_stages(const CUtensorMap& kmap, const CUtensorMap& v
         PGK_CUDA(cudaFuncSetAttribute(rope_sdpa_mma_kernel<STAGES, TWICE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
         attr_set = true;
     }
-    PGK_CUDA(launch(rope_sdpa_mma_kernel<STAGES, TWICE>, grid, dim3(kMThreads), kSmem, st, kmap, vmap, p));
+    PGK_CUDA(launch_waiting(rope_sdpa_mma_kernel<STAGES, TWICE>, grid, dim3(kMThreads), kSmem, st, kmap, vmap, p));
     return 0;
 }
 
@@ -1020,6 +1022,7 @@ int pgk_rope_sdpa_decode(const void* qkv, const void* q_gamma, const void* k_gam
                 "rope_sdpa_decode failed: qkv / K / V must be 16-byte aligned");
     if (scale <= 0.f) scale = 1.0f / sqrtf((float)head_dim);
     RopeSdpaParams p = {};
+    p.ahead = pdl_enabled();
     p.qkv = (const uint16_t*)qkv; p.q_gamma = (const uint16_t*)q_gamma; p.k_gamma = (const uint16_t*)k_gamma; p.eps = eps;
     p.cos_t = cos_table; p.sin_t = sin_table; p.kc = (uint16_t*)k_cache; p.vc = (uint16_t*)v_cache; p.out = (uint16_t*)out;
     p.hq = n_heads_q; p.n_kv = n_kv; p.max_seq = max_seq; p.pos = pos; p.context_len = context_len;
@@ -1041,6 +1044,7 @@ int pgk_rope_sdpa_decode_batch(const void* qkv, const void* q_gamma, const void*
                 "rope_sdpa_decode_batch failed: qkv / K / V must be 16-byte aligned");
     if (scale <= 0.f) scale = 1.0f / sqrtf((float)head_dim);
     RopeSdpaParams p = {};
+    p.ahead = pdl_enabled();
     p.qkv = (const uint16_t*)qkv; p.q_gamma = (const uint16_t*)q_gamma; p.k_gamma = (const uint16_t*)k_gamma; p.eps = eps;
     p.cos_t = cos_table; p.sin_t = sin_table; p.kc = (uint16_t*)k_cache; p.vc = (uint16_t*)v_cache; p.out = (uint16_t*)out;
     p.hq = n_heads_q; p.n_kv = n_kv; p.max_seq = max_seq; p.pos_buf = pos_buf; p.ctx_buf = ctx_buf;

@@ -372,9 +372,9 @@ int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, 
         if (int rc = scratch_alloc(&ws, (size_t)q_len * hq * p.splits * (M_D + 4) * sizeof(float), st)) return rc;
         p.ws = (float*)ws;
     }
-    cudaError_t e = launch(sdpa_prompt_kernel, dim3(qtiles, n_kv * p.hsplit, p.splits), dim3(M_THREADS), M_SMEM, st, kmap, vmap, p);
+    cudaError_t e = launch_waiting(sdpa_prompt_kernel, dim3(qtiles, n_kv * p.hsplit, p.splits), dim3(M_THREADS), M_SMEM, st, kmap, vmap, p);
     if (p.splits > 1) {
-        if (e == cudaSuccess) e = launch(sdpa_prompt_fold_kernel, dim3((q_len * hq + 7) / 8), dim3(256), 0, st, p);
+        if (e == cudaSuccess) e = launch_waiting(sdpa_prompt_fold_kernel, dim3((q_len * hq + 7) / 8), dim3(256), 0, st, p);
         if (int rc = scratch_free(p.ws, st)) return rc;
     }
     PGK_CUDA(e);

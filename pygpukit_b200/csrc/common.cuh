@@ -79,8 +79,8 @@ inline int smem_carveout() {
 }
 
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                          cudaStream_t stream, Args... args) {
+inline cudaError_t launch_as(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -88,7 +88,7 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
     cfg.stream = stream;
     cudaLaunchAttribute attr[2];
     int nattr = 0;
-    if (pdl_enabled()) {
+    if (dependent) {
         attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[0].val.programmaticStreamSerializationAllowed = 1;
         nattr = 1;
@@ -102,6 +102,18 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
     cfg.numAttrs = nattr;
     count_launch();
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_as(pdl_enabled(), kernel, grid, block, smem, stream, args...);
+}
+// For kernels whose every block executes griddep_wait() before it touches global memory: they may always be brought to the SMs while
+// the kernel before them drains, which hides the launch (2 ... 4 us of a kernel with a large block); whoever comes after them finds
+// everything before them finished, since they do not finish earlier themselves.  What a kernel reads AHEAD of its wait (weights, see
+// griddep_wait) it reads ahead only under pdl_enabled(); otherwise its first act is the wait.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_waiting(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_as(true, kernel, grid, block, smem, stream, args...);
 }
 
 // ---------------------------------------------------------------- device helpers

@@ -455,7 +455,7 @@ int pgk_rmsnorm(const void* x, const void* gamma, void* y, int rows, int feature
     int bs = (features + 31) / 32 * 32;          // the reference's block size (rmsnorm.inl:18-19): same partial sums
     if (bs > 256) bs = 256;
     PGK_DISPATCH_DT(dtype, "rmsnorm",
-        PGK_CUDA(launch(rmsnorm_kernel<DT, false>, dim3(rows), dim3(bs), 0, ST(stream), x, (const void*)nullptr, gamma, y, features, eps)));
+        PGK_CUDA(launch_waiting(rmsnorm_kernel<DT, false>, dim3(rows), dim3(bs), 0, ST(stream), x, (const void*)nullptr, gamma, y, features, eps)));
     return 0;
 }
 int pgk_rmsnorm_residual(const void* x, const void* residual, const void* gamma, void* y, int rows, int features,
@@ -463,7 +463,7 @@ int pgk_rmsnorm_residual(const void* x, const void* residual, const void* gamma,
     PGK_REQUIRE(rows >= 0 && features > 0, "rmsnorm_residual failed: invalid shape");
     if (rows == 0) return 0;
     PGK_DISPATCH_DT(dtype, "rmsnorm_residual",
-        PGK_CUDA(launch(rmsnorm_kernel<DT, true>, dim3(rows), dim3(256), 0, ST(stream), x, residual, gamma, y, features, eps)));
+        PGK_CUDA(launch_waiting(rmsnorm_kernel<DT, true>, dim3(rows), dim3(256), 0, ST(stream), x, residual, gamma, y, features, eps)));
     return 0;
 }
 int pgk_layernorm(const void* x, const void* gamma, const void* beta, void* y, int rows, int features, float eps,
@@ -471,7 +471,7 @@ int pgk_layernorm(const void* x, const void* gamma, const void* beta, void* y, i
     PGK_REQUIRE(rows >= 0 && features > 0, "layernorm failed: invalid shape");
     if (rows == 0) return 0;
     PGK_DISPATCH_DT(dtype, "layernorm",
-        PGK_CUDA(launch(layernorm_kernel<DT>, dim3(rows), dim3(256), 0, ST(stream), x, gamma, beta, y, features, eps)));
+        PGK_CUDA(launch_waiting(layernorm_kernel<DT>, dim3(rows), dim3(256), 0, ST(stream), x, gamma, beta, y, features, eps)));
     return 0;
 }
 int pgk_rope_inplace(void* q, void* k, const void* cos, const void* sin, int seq, int n_heads_q, int n_heads_k,
@@ -481,61 +481,61 @@ int pgk_rope_inplace(void* q, void* k, const void* cos, const void* sin, int seq
     if (n == 0) return 0;
     const bool f32tab = (table_dtype == 0);
     PGK_DISPATCH_DT(dtype, "rope_inplace",
-        if (f32tab) PGK_CUDA(launch(rope_kernel<DT, 0>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), q, k, cos, sin, seq, n_heads_q, n_heads_k, head_dim));
-        else        PGK_CUDA(launch(rope_kernel<DT, DT>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), q, k, cos, sin, seq, n_heads_q, n_heads_k, head_dim)));
+        if (f32tab) PGK_CUDA(launch_waiting(rope_kernel<DT, 0>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), q, k, cos, sin, seq, n_heads_q, n_heads_k, head_dim));
+        else        PGK_CUDA(launch_waiting(rope_kernel<DT, DT>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), q, k, cos, sin, seq, n_heads_q, n_heads_k, head_dim)));
     return 0;
 }
 int pgk_silu(const void* x, void* y, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "silu", PGK_CUDA(launch(unary_kernel<DT, OP_SILU>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), x, y, n)));
+    PGK_DISPATCH_DT(dtype, "silu", PGK_CUDA(launch_waiting(unary_kernel<DT, OP_SILU>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), x, y, n)));
     return 0;
 }
 int pgk_gelu(const void* x, void* y, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "gelu", PGK_CUDA(launch(unary_kernel<DT, OP_GELU>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), x, y, n)));
+    PGK_DISPATCH_DT(dtype, "gelu", PGK_CUDA(launch_waiting(unary_kernel<DT, OP_GELU>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), x, y, n)));
     return 0;
 }
 /* y = round(round(silu(gate)) * up): silu + mul_inplace of the layer path (two roundings) in one launch */
 int pgk_silu_mul(const void* gate, const void* up, void* y, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "silu_mul", PGK_CUDA(launch(binary_kernel<DT, OP_SILU_MUL>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), gate, up, y, n)));
+    PGK_DISPATCH_DT(dtype, "silu_mul", PGK_CUDA(launch_waiting(binary_kernel<DT, OP_SILU_MUL>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), gate, up, y, n)));
     return 0;
 }
 int pgk_swiglu(const void* gate, const void* up, void* y, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "swiglu", PGK_CUDA(launch(binary_kernel<DT, OP_SWIGLU>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), gate, up, y, n)));
+    PGK_DISPATCH_DT(dtype, "swiglu", PGK_CUDA(launch_waiting(binary_kernel<DT, OP_SWIGLU>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), gate, up, y, n)));
     return 0;
 }
 int pgk_add(const void* a, const void* b, void* c, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "add", PGK_CUDA(launch(binary_kernel<DT, OP_ADD>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, c, n)));
+    PGK_DISPATCH_DT(dtype, "add", PGK_CUDA(launch_waiting(binary_kernel<DT, OP_ADD>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, c, n)));
     return 0;
 }
 int pgk_mul(const void* a, const void* b, void* c, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "mul", PGK_CUDA(launch(binary_kernel<DT, OP_MUL>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, c, n)));
+    PGK_DISPATCH_DT(dtype, "mul", PGK_CUDA(launch_waiting(binary_kernel<DT, OP_MUL>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, c, n)));
     return 0;
 }
 int pgk_add_inplace(void* a, const void* b, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "add_inplace", PGK_CUDA(launch(binary_inplace_kernel<DT, OP_ADD>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, n)));
+    PGK_DISPATCH_DT(dtype, "add_inplace", PGK_CUDA(launch_waiting(binary_inplace_kernel<DT, OP_ADD>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, n)));
     return 0;
 }
 int pgk_mul_inplace(void* a, const void* b, size_t n, int dtype, void* stream) {
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "mul_inplace", PGK_CUDA(launch(binary_inplace_kernel<DT, OP_MUL>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, n)));
+    PGK_DISPATCH_DT(dtype, "mul_inplace", PGK_CUDA(launch_waiting(binary_inplace_kernel<DT, OP_MUL>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), a, b, n)));
     return 0;
 }
 int pgk_bias_add_inplace(void* x, const void* bias, int rows, int features, int dtype, void* stream) {
     size_t n = (size_t)rows * features;
     if (n == 0) return 0;
-    PGK_DISPATCH_DT(dtype, "bias_add_inplace", PGK_CUDA(launch(bias_add_kernel<DT>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), x, bias, n, features)));
+    PGK_DISPATCH_DT(dtype, "bias_add_inplace", PGK_CUDA(launch_waiting(bias_add_kernel<DT>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), x, bias, n, features)));
     return 0;
 }
 int pgk_cast(const void* src, void* dst, size_t n, int src_dtype, int dst_dtype, void* stream) {
     if (n == 0) return 0;
     unsigned g = blocks_for(n, 256);
-#define PGK_CAST(S, D) if (src_dtype == S && dst_dtype == D) { PGK_CUDA(launch(cast_kernel<S, D>, dim3(g), dim3(256), 0, ST(stream), src, dst, n)); return 0; }
+#define PGK_CAST(S, D) if (src_dtype == S && dst_dtype == D) { PGK_CUDA(launch_waiting(cast_kernel<S, D>, dim3(g), dim3(256), 0, ST(stream), src, dst, n)); return 0; }
     PGK_CAST(0, 1) PGK_CAST(0, 2) PGK_CAST(1, 0) PGK_CAST(2, 0) PGK_CAST(1, 2) PGK_CAST(2, 1)
     PGK_CAST(0, 0) PGK_CAST(1, 1) PGK_CAST(2, 2)
 #undef PGK_CAST
@@ -544,7 +544,7 @@ int pgk_cast(const void* src, void* dst, size_t n, int src_dtype, int dst_dtype,
 }
 int pgk_embedding_lookup(const void* table, void* out, int hidden, int token, int elem_bytes, void* stream) {
     size_t rb = (size_t)hidden * elem_bytes;
-    PGK_CUDA(launch(embedding_kernel, dim3(blocks_for(rb / 16 + 1, 256), 1), dim3(256), 0, ST(stream),
+    PGK_CUDA(launch_waiting(embedding_kernel, dim3(blocks_for(rb / 16 + 1, 256), 1), dim3(256), 0, ST(stream),
                     (const uint8_t*)table, (uint8_t*)out, rb, token, (const int32_t*)nullptr, 1));
     return 0;
 }
@@ -552,7 +552,7 @@ int pgk_embedding_lookup_ptr(const void* table, void* out, int hidden, const int
                              int elem_bytes, void* stream) {
     if (n_tokens <= 0) return 0;
     size_t rb = (size_t)hidden * elem_bytes;
-    PGK_CUDA(launch(embedding_kernel, dim3(blocks_for(rb / 16 + 1, 256), n_tokens > 65535 ? 65535 : n_tokens), dim3(256), 0,
+    PGK_CUDA(launch_waiting(embedding_kernel, dim3(blocks_for(rb / 16 + 1, 256), n_tokens > 65535 ? 65535 : n_tokens), dim3(256), 0,
                     ST(stream), (const uint8_t*)table, (uint8_t*)out, rb, 0, token_buf, n_tokens));
     return 0;
 }
@@ -561,32 +561,32 @@ int pgk_embedding_lookup_pos(const void* wte, const void* wpe, void* out, int hi
     if (n_tokens <= 0) return 0;
     PGK_REQUIRE(token_buf != nullptr, "embedding_lookup_pos failed: token_buf is NULL");
     PGK_DISPATCH_DT(dtype, "embedding_lookup_pos",
-                    PGK_CUDA(launch(embedding_pos_kernel<DT>, dim3(blocks_for(hidden, 256), n_tokens > 65535 ? 65535 : n_tokens),
+                    PGK_CUDA(launch_waiting(embedding_pos_kernel<DT>, dim3(blocks_for(hidden, 256), n_tokens > 65535 ? 65535 : n_tokens),
                                     dim3(256), 0, ST(stream), wte, wpe, out, hidden, token_buf, n_tokens, pos, pos_buf)));
     return 0;
 }
 int pgk_argmax(const void* logits, int32_t* out, int n, int dtype, void* stream) {
     PGK_REQUIRE(n > 0, "argmax failed: empty input");
-    PGK_DISPATCH_DT(dtype, "argmax", PGK_CUDA(launch(argmax_kernel<DT>, dim3(1), dim3(1024), 0, ST(stream), logits, out, n)));
+    PGK_DISPATCH_DT(dtype, "argmax", PGK_CUDA(launch_waiting(argmax_kernel<DT>, dim3(1), dim3(1024), 0, ST(stream), logits, out, n)));
     return 0;
 }
 int pgk_swiglu_interleaved8_bf16(const void* gate_up, void* out, int M, int I, void* stream) {
     PGK_REQUIRE(M >= 1 && I >= 8 && I % 8 == 0, "swiglu_interleaved8 failed: invalid shape M=%d I=%d", M, I);
-    PGK_CUDA(launch(swiglu_interleaved8_kernel, dim3(blocks_for((size_t)M * I, 256)), dim3(256), 0, ST(stream),
+    PGK_CUDA(launch_waiting(swiglu_interleaved8_kernel, dim3(blocks_for((size_t)M * I, 256)), dim3(256), 0, ST(stream),
                     (const uint16_t*)gate_up, (uint16_t*)out, M, I));
     return 0;
 }
 int pgk_argmax_rows(const void* logits, int32_t* out, int32_t* out2, int rows, int n, int dtype, void* stream) {
     PGK_REQUIRE(n > 0 && rows >= 1, "argmax_rows failed: empty input");
-    PGK_DISPATCH_DT(dtype, "argmax_rows", PGK_CUDA(launch(argmax_rows_kernel<DT>, dim3(rows), dim3(1024), 0, ST(stream), logits, out, out2, n)));
+    PGK_DISPATCH_DT(dtype, "argmax_rows", PGK_CUDA(launch_waiting(argmax_rows_kernel<DT>, dim3(rows), dim3(1024), 0, ST(stream), logits, out, out2, n)));
     return 0;
 }
 int pgk_transpose_021(const void* in, void* out, int d0, int d1, int d2, int elem_bytes, void* stream) {
     size_t n = (size_t)d0 * d1 * d2;
     if (n == 0) return 0;
-    if (elem_bytes == 2) PGK_CUDA(launch(transpose021_kernel<uint16_t>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), (const uint16_t*)in, (uint16_t*)out, d0, d1, d2));
-    else if (elem_bytes == 4) PGK_CUDA(launch(transpose021_kernel<uint32_t>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), (const uint32_t*)in, (uint32_t*)out, d0, d1, d2));
-    else if (elem_bytes == 1) PGK_CUDA(launch(transpose021_kernel<uint8_t>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), (const uint8_t*)in, (uint8_t*)out, d0, d1, d2));
+    if (elem_bytes == 2) PGK_CUDA(launch_waiting(transpose021_kernel<uint16_t>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), (const uint16_t*)in, (uint16_t*)out, d0, d1, d2));
+    else if (elem_bytes == 4) PGK_CUDA(launch_waiting(transpose021_kernel<uint32_t>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), (const uint32_t*)in, (uint32_t*)out, d0, d1, d2));
+    else if (elem_bytes == 1) PGK_CUDA(launch_waiting(transpose021_kernel<uint8_t>, dim3(blocks_for(n, 256)), dim3(256), 0, ST(stream), (const uint8_t*)in, (uint8_t*)out, d0, d1, d2));
     else { set_error("transpose_3d_021 failed: unsupported element size %d", elem_bytes); return 1; }
     return 0;
 }
@@ -600,11 +600,11 @@ int pgk_kv_cache_update(const void* new_kv, void* cache, int seq, int n_kv, int 
     bool vec = (rb % 16 == 0) && ((uintptr_t)new_kv % 16 == 0) && ((uintptr_t)cache % 16 == 0);
     if (vec) {
         size_t n = rows * (rb / 16);
-        PGK_CUDA(launch(kv_update_kernel, dim3(blocks_for(n, 256) > 4096 ? 4096 : blocks_for(n, 256)), dim3(256), 0, ST(stream),
+        PGK_CUDA(launch_waiting(kv_update_kernel, dim3(blocks_for(n, 256) > 4096 ? 4096 : blocks_for(n, 256)), dim3(256), 0, ST(stream),
                         (const uint8_t*)new_kv, (uint8_t*)cache, seq, n_kv, num_heads_out, rb, max_seq, pos, pos_buf));
     } else {
         size_t n = rows * rb;
-        PGK_CUDA(launch(kv_update_bytes_kernel, dim3(blocks_for(n, 256) > 4096 ? 4096 : blocks_for(n, 256)), dim3(256), 0, ST(stream),
+        PGK_CUDA(launch_waiting(kv_update_bytes_kernel, dim3(blocks_for(n, 256) > 4096 ? 4096 : blocks_for(n, 256)), dim3(256), 0, ST(stream),
                         (const uint8_t*)new_kv, (uint8_t*)cache, seq, n_kv, num_heads_out, rb, max_seq, pos, pos_buf));
     }
     return 0;
@@ -614,7 +614,7 @@ int pgk_qk_norm_rope_kv_write(void* qkv, const void* q_gamma, const void* k_gamm
                               int head_dim, int max_seq, int pos, const int32_t* pos_buf, void* stream) {
     PGK_REQUIRE(head_dim % 2 == 0 && M >= 1, "qk_norm_rope_kv_write failed: invalid shape");
     long warps = (long)M * (n_heads_q + 2 * n_kv);
-    PGK_CUDA(launch(qk_norm_rope_kv_kernel, dim3(blocks_for((size_t)warps * 32, 128)), dim3(128), 0, ST(stream),
+    PGK_CUDA(launch_waiting(qk_norm_rope_kv_kernel, dim3(blocks_for((size_t)warps * 32, 128)), dim3(128), 0, ST(stream),
                     (uint16_t*)qkv, (const uint16_t*)q_gamma, (const uint16_t*)k_gamma, eps, cos_table, sin_table,
                     (uint16_t*)k_cache, (uint16_t*)v_cache, M, n_heads_q, n_kv, head_dim, max_seq, pos, pos_buf));
     return 0;

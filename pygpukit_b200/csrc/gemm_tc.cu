@@ -49,6 +49,7 @@ struct F8TcParams {
     const uint16_t* S; const uint16_t* S1; uint16_t* C;          // scales (of gate and up), output
     const uint16_t* bias; const uint16_t* residual;
     int M, K, N, splits, kper;
+    int ahead;                                    // scales and the first codes are read before the kernel before has finished
     int* err;                                     // raised when a bounded wait runs out
 };
 
@@ -82,6 +83,7 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     const int rank = blockIdx.x, n0 = blockIdx.y * OUT, nkb_total = p.K / kTcBK;
     const int kb0 = rank * p.kper, nkb = max(0, min(nkb_total, kb0 + p.kper) - kb0);
 
+    if (!p.ahead) griddep_wait();
     // the block's scales are weights: staged before the dependency wait
     const size_t scales = (size_t)(blockIdx.y >> (PAIR ? 1 : 0)) * nkb_total + kb0;
     for (int i = tid; i < nkb; i += F_THREADS) {
@@ -347,6 +349,7 @@ int launch_f8tc(F8TcParams p, const void* A, const void* B, const void* B1, cuda
     const int tiles = p.N / (PAIR ? kTcRows / 2 : kTcRows), nkb = p.K / kTcBK;
     p.splits = f8tc_splits(tiles, nkb);
     p.kper = (nkb + p.splits - 1) / p.splits;
+    p.ahead = pdl_enabled();
     p.err = wait_word(kWaitFp8);
     PGK_REQUIRE(p.err, "gemm_fp8_tc failed: no pinned host memory");
     PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8_tc failed: the driver does not export cuTensorMapEncodeTiled");
@@ -359,10 +362,8 @@ int launch_f8tc(F8TcParams p, const void* A, const void* B, const void* B1, cuda
     PGK_CUDA((f8tc_config<NB, PAIR>(&cfg, at, p.splits)));
     cfg.gridDim = dim3(p.splits, tiles);
     cfg.stream = st;
-    if (pdl_enabled()) {
-        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-    }
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_waiting
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
     count_launch();
     PGK_CUDA(cudaLaunchKernelEx(&cfg, gemm_fp8_tc_kernel<NB, PAIR>, wmap, umap, amap, p));
     return 0;

@@ -50,6 +50,7 @@ struct F8RowsParams {
     int M, K, N;                                   // N: columns of C
     int item0, items, m_tiles, mrows;              // tiles [item0, items), and of how many rows
     int splits, kper;
+    int ahead;                                     // the first codes are read before the kernel before has finished
     int* err;
 };
 
@@ -128,11 +129,12 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
             const uint64_t once = l2_evict_first();
             RingPos c;
             int blk = 0;
-            bool ok = true, waited = false;
+            bool ok = true, waited = !p.ahead;
+            if (waited) { griddep_wait(); griddep_launch(); }
             for (int item = first; ok && item < p.items; item += step) {
                 const int n0 = item / p.m_tiles * OUT;
                 for (int it = 0; it < nkb; ++it, ++blk, c.next(P_CODES)) {
-                    if (blk == P_CODES) { griddep_wait(); griddep_launch(); waited = true; }
+                    if (blk == P_CODES && !waited) { griddep_wait(); griddep_launch(); waited = true; }
                     const uint32_t bar = smem_u32(cfull_bar) + 8u * c.s, at = codes + c.s * P_CODE_BYTES;
                     ok = bar_wait(err, smem_u32(cempty_bar) + 8u * c.s, c.round ^ 1u);
                     if (!ok) break;
@@ -485,6 +487,7 @@ int launch_f8rows(F8RowsParams p, const void* A, const void* B0, const void* B1,
     const F8RowsPlan plan = f8rows_plan(n_tiles, p.M, nkb);
     p.mrows = plan.mrows;
     p.m_tiles = (p.M + p.mrows - 1) / p.mrows;
+    p.ahead = pdl_enabled();
     p.err = wait_word(kWaitFp8);
     PGK_REQUIRE(p.err, "gemm_fp8 failed: no pinned host memory");
     PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8 failed: the driver does not export cuTensorMapEncodeTiled");
@@ -503,10 +506,8 @@ int launch_f8rows(F8RowsParams p, const void* A, const void* B0, const void* B1,
         PGK_CUDA(f8rows_config<PAIR>(&cfg, at, splits));
         cfg.gridDim = dim3(splits, splits > 1 ? items - item0 : min(items - item0, sm_count()));
         cfg.stream = st;
-        if (pdl_enabled()) {
-            at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
-        }
+        at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_waiting
+        at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
         count_launch();
         PGK_CUDA(cudaLaunchKernelEx(&cfg, gemm_fp8_rows_kernel<PAIR>, wmap, umap, amap, q));
         return 0;

@@ -56,6 +56,7 @@ gemv_bf16_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B,
     constexpr int U = 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint16_t* a_s = reinterpret_cast<uint16_t*>(smem_raw);
+    if (!epi.ahead) griddep_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
     // rows dealt round-robin over the warps of the grid (see gemv_fp8.cu)
     const long gwarp = (long)blockIdx.x * wpc + warp;
@@ -198,7 +199,8 @@ static int launch_bf16(const uint16_t* A, const uint16_t* B, uint16_t* C, int K,
         am.key = g_am_scratch;
         am.done = reinterpret_cast<unsigned*>(g_am_scratch + 1);
     }
-    PGK_CUDA(launch(kern, dim3(cfg.ctas), dim3(cfg.warps_per_cta * 32), smem, st, A, B, C, K, N, cfg.rho, epi, am));
+    epi.ahead = pdl_enabled();
+    PGK_CUDA(launch_waiting(kern, dim3(cfg.ctas), dim3(cfg.warps_per_cta * 32), smem, st, A, B, C, K, N, cfg.rho, epi, am));
     return 0;
 }
 
@@ -216,7 +218,7 @@ static int bf16_dispatch(const void* A, const void* B, void* C, int M, int K, in
     if (!fast) {
         GemvEpilogue epi = {(const uint16_t*)bias, (const uint16_t*)residual};
         long warps = (long)N * M;
-        PGK_CUDA(launch(gemv_bf16_generic_kernel<false>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256),
+        PGK_CUDA(launch_waiting(gemv_bf16_generic_kernel<false>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256),
                         0, st, a, b, c, M, K, N, epi));
         return 0;
     }

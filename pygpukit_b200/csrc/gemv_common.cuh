@@ -40,6 +40,7 @@ struct GemvEpilogue {
     const uint16_t* residual;  // [M,N] bf16 or null
     const uint16_t* norm_gamma = nullptr;  // [K] bf16: A <- bf16(rmsnorm(A) * gamma) while staging, or null
     float norm_eps = 0.f;
+    int ahead = 0;                         // the first weights are loaded before the kernel before has finished
     GemvXchg xchg = {};                    // world > 1: all-reduce over the ranks before the residual add (M == 1)
 };
 

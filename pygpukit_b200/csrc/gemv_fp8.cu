@@ -116,6 +116,7 @@ gemv_fp8_sb_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ B
     float* inv_s = reinterpret_cast<float*>(smem_raw + (size_t)M * K * 2);
     uint32_t* red = reinterpret_cast<uint32_t*>(inv_s + 8);
 
+    if (!epi.ahead) griddep_wait();
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     const int wpc = blockDim.x >> 5;
@@ -321,7 +322,8 @@ static int launch_fp8_kern(Kern kern, int maxw, int M, const void* A, const void
         }
         cfg = it->second;
     }
-    PGK_CUDA(launch(kern, dim3(cfg.ctas), dim3(cfg.warps_per_cta * 32), smem, st,
+    epi.ahead = pdl_enabled();
+    PGK_CUDA(launch_waiting(kern, dim3(cfg.ctas), dim3(cfg.warps_per_cta * 32), smem, st,
                     (const uint16_t*)A, (const uint8_t*)B0, (const uint16_t*)S0, (const uint8_t*)B1,
                     (const uint16_t*)S1, (uint16_t*)C, K, N, cfg.rho, epi));
     return 0;
@@ -382,11 +384,11 @@ static int gemv_fp8_dispatch(const void* A, const void* B0, const void* S0, cons
         int block = 256;
         long grid = (warps * 32 + block - 1) / block;
         if (swiglu)
-            PGK_CUDA(launch(gemv_fp8_generic_kernel<2>, dim3((unsigned)grid), dim3(block), 0, st, a,
+            PGK_CUDA(launch_waiting(gemv_fp8_generic_kernel<2>, dim3((unsigned)grid), dim3(block), 0, st, a,
                             (const uint8_t*)B0, (const uint16_t*)S0, (const uint8_t*)B1,
                             (const uint16_t*)S1, c, M, K, N, epi));
         else
-            PGK_CUDA(launch(gemv_fp8_generic_kernel<1>, dim3((unsigned)grid), dim3(block), 0, st, a,
+            PGK_CUDA(launch_waiting(gemv_fp8_generic_kernel<1>, dim3((unsigned)grid), dim3(block), 0, st, a,
                             (const uint8_t*)B0, (const uint16_t*)S0, (const uint8_t*)nullptr,
                             (const uint16_t*)nullptr, c, M, K, N, epi));
         return 0;

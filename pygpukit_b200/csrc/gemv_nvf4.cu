@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(512) gemv_nvf4_kernel(Nvf4Params p) {
     float* red_f = reinterpret_cast<float*>(smem_raw + kNvf4Hdr);  // aliases a_s after the main loop
     __shared__ unsigned s_ticket;
 
+    if (!p.epi.ahead) griddep_wait();
     const int K = p.K, N = p.N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, wpc = blockDim.x >> 5;
     const int g = blockIdx.x / p.KS, ks = blockIdx.x % p.KS;
@@ -361,7 +362,8 @@ static int launch_nvf4(Nvf4Params p, cudaStream_t st) {
     p.bpc = cfg.bpc;
     p.ws = g_ws;
     p.counters = g_counters;
-    PGK_CUDA(launch(kern, dim3(G * cfg.KS), dim3(cfg.wpc * 32), cfg.smem, st, p));
+    p.epi.ahead = pdl_enabled();
+    PGK_CUDA(launch_waiting(kern, dim3(G * cfg.KS), dim3(cfg.wpc * 32), cfg.smem, st, p));
     return 0;
 }
 
@@ -395,7 +397,7 @@ static int nvf4_dispatch(const void* A, const void* Bd, const void* Bs, void* C,
     if (!fast) {
         GemvEpilogue epi = {(const uint16_t*)bias, (const uint16_t*)residual};
         long tot = (long)M * N;
-        PGK_CUDA(launch(gemv_nvf4_generic_kernel, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, st,
+        PGK_CUDA(launch_waiting(gemv_nvf4_generic_kernel, dim3((unsigned)((tot + 255) / 256)), dim3(256), 0, st,
                         (const uint16_t*)A, (const uint8_t*)Bd, (const uint8_t*)Bs, (uint16_t*)C, M, K, N,
                         alpha, epi));
         return 0;
@@ -499,7 +501,8 @@ static int launch_nvf4_noalloc(Nvf4Params p, cudaStream_t st) {
     // the array keeps the last call's contents: the counters must start at zero (the partials are overwritten before
     // they are read)
     if (KS > 1) PGK_CUDA(cudaMemsetAsync(p.counters, 0, (size_t)G * sizeof(unsigned), st));
-    PGK_CUDA(launch(kern, dim3(G * KS), dim3(wpc * 32), smem, st, p));
+    p.epi.ahead = pdl_enabled();
+    PGK_CUDA(launch_waiting(kern, dim3(G * KS), dim3(wpc * 32), smem, st, p));
     return 0;
 }
 

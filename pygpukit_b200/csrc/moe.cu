@@ -557,7 +557,7 @@ static int launch_moe_nvf4(const void* A, int a_stride, const void* Bd0, const v
         const int kb = K >> 5;
         while (ks > 1 && kb / ks < kMoeNvf4Warps) --ks;
     }
-    PGK_CUDA(launch(moe_grouped_gemv_nvf4_kernel<NMAT>, dim3(tiles, M, ks), dim3(kMoeNvf4Warps * 32), smem,
+    PGK_CUDA(launch_waiting(moe_grouped_gemv_nvf4_kernel<NMAT>, dim3(tiles, M, ks), dim3(kMoeNvf4Warps * 32), smem,
                     (cudaStream_t)stream, (const uint16_t*)A, (const uint8_t*)Bd0, (const uint8_t*)Bs0, (const uint8_t*)Bd1,
                     (const uint8_t*)Bs1, (uint16_t*)C, row_expert_ids, K, N, a_stride, expert_offset, num_local_experts,
                     ws, cnt));
@@ -584,32 +584,32 @@ int pgk_moe_topk(const void* logits, void* values, int32_t* indices, int num_tok
                 "moe_topk_with_indices failed: unsupported num_experts=%d k=%d", num_experts, k);
     if (num_tokens <= 0) return 0;
     unsigned g = nblk((size_t)num_tokens * 32, 128);
-    if (dtype == 0) PGK_CUDA(launch(moe_topk_kernel<0>, dim3(g), dim3(128), 0, ST(stream), logits, values, indices, num_tokens, num_experts, k));
-    else if (dtype == 1) PGK_CUDA(launch(moe_topk_kernel<1>, dim3(g), dim3(128), 0, ST(stream), logits, values, indices, num_tokens, num_experts, k));
-    else if (dtype == 2) PGK_CUDA(launch(moe_topk_kernel<2>, dim3(g), dim3(128), 0, ST(stream), logits, values, indices, num_tokens, num_experts, k));
+    if (dtype == 0) PGK_CUDA(launch_waiting(moe_topk_kernel<0>, dim3(g), dim3(128), 0, ST(stream), logits, values, indices, num_tokens, num_experts, k));
+    else if (dtype == 1) PGK_CUDA(launch_waiting(moe_topk_kernel<1>, dim3(g), dim3(128), 0, ST(stream), logits, values, indices, num_tokens, num_experts, k));
+    else if (dtype == 2) PGK_CUDA(launch_waiting(moe_topk_kernel<2>, dim3(g), dim3(128), 0, ST(stream), logits, values, indices, num_tokens, num_experts, k));
     else { set_error("moe_topk_with_indices failed: unsupported dtype code %d", dtype); return 1; }
     return 0;
 }
 int pgk_moe_softmax_topk(void* values, int num_tokens, int k, int dtype, void* stream) {
     if (num_tokens <= 0) return 0;
     unsigned g = nblk(num_tokens, 128);
-    if (dtype == 0) PGK_CUDA(launch(moe_softmax_topk_kernel<0>, dim3(g), dim3(128), 0, ST(stream), values, num_tokens, k));
-    else if (dtype == 1) PGK_CUDA(launch(moe_softmax_topk_kernel<1>, dim3(g), dim3(128), 0, ST(stream), values, num_tokens, k));
-    else if (dtype == 2) PGK_CUDA(launch(moe_softmax_topk_kernel<2>, dim3(g), dim3(128), 0, ST(stream), values, num_tokens, k));
+    if (dtype == 0) PGK_CUDA(launch_waiting(moe_softmax_topk_kernel<0>, dim3(g), dim3(128), 0, ST(stream), values, num_tokens, k));
+    else if (dtype == 1) PGK_CUDA(launch_waiting(moe_softmax_topk_kernel<1>, dim3(g), dim3(128), 0, ST(stream), values, num_tokens, k));
+    else if (dtype == 2) PGK_CUDA(launch_waiting(moe_softmax_topk_kernel<2>, dim3(g), dim3(128), 0, ST(stream), values, num_tokens, k));
     else { set_error("moe_softmax_topk failed: unsupported dtype code %d", dtype); return 1; }
     return 0;
 }
 int pgk_moe_compute_permutation(const int32_t* expert_indices, int32_t* expert_counts, int32_t* expert_offsets,
                                 int32_t* permute_indices, int32_t* reverse_perm, int num_tokens, int num_experts,
                                 int k, void* stream) {
-    PGK_CUDA(launch(moe_permutation_kernel, dim3(1), dim3(256), 0, ST(stream), expert_indices, expert_counts,
+    PGK_CUDA(launch_waiting(moe_permutation_kernel, dim3(1), dim3(256), 0, ST(stream), expert_indices, expert_counts,
                     expert_offsets, permute_indices, reverse_perm, num_tokens * k, num_experts));
     return 0;
 }
 int pgk_moe_expand_expert_offsets(const int32_t* expert_offsets, int32_t* row_expert_ids, int num_experts,
                                   int m_total, void* stream) {
     if (m_total <= 0) return 0;
-    PGK_CUDA(launch(moe_expand_offsets_kernel, dim3(nblk(m_total, 128)), dim3(128), 0, ST(stream), expert_offsets,
+    PGK_CUDA(launch_waiting(moe_expand_offsets_kernel, dim3(nblk(m_total, 128)), dim3(128), 0, ST(stream), expert_offsets,
                     row_expert_ids, num_experts, m_total));
     return 0;
 }
@@ -617,14 +617,14 @@ int pgk_moe_gather(const void* hidden, const int32_t* permute_indices, void* gat
                    int hidden_size, int k, void* stream) {
     int rows = num_tokens * k;
     if (rows <= 0) return 0;
-    PGK_CUDA(launch(moe_gather_kernel, dim3(rows), dim3(256), 0, ST(stream), (const uint16_t*)hidden, permute_indices,
+    PGK_CUDA(launch_waiting(moe_gather_kernel, dim3(rows), dim3(256), 0, ST(stream), (const uint16_t*)hidden, permute_indices,
                     (uint16_t*)gathered, rows, hidden_size, k));
     return 0;
 }
 int pgk_moe_scatter(const void* expert_out, const void* router_weights, const int32_t* reverse_perm, void* output,
                     int num_tokens, int hidden_size, int k, void* stream) {
     if (num_tokens <= 0) return 0;
-    PGK_CUDA(launch(moe_scatter_kernel, dim3(num_tokens), dim3(256), 0, ST(stream), (const uint16_t*)expert_out,
+    PGK_CUDA(launch_waiting(moe_scatter_kernel, dim3(num_tokens), dim3(256), 0, ST(stream), (const uint16_t*)expert_out,
                     (const uint16_t*)router_weights, reverse_perm, (uint16_t*)output, num_tokens, hidden_size, k));
     return 0;
 }
@@ -641,7 +641,7 @@ int pgk_moe_grouped_gemv_fp8_ex(const void* A, int a_stride, const void* B_enk, 
     bool clean;
     if (int rc = moe_fp8_clean(B_enk, num_local_experts, N, K, stream, &clean)) return rc;
     auto kern = clean ? moe_grouped_gemv_fp8_kernel<true> : moe_grouped_gemv_fp8_kernel<false>;
-    PGK_CUDA(launch(kern, dim3(nblk(warps * 32, 256)), dim3(256), 0, ST(stream),
+    PGK_CUDA(launch_waiting(kern, dim3(nblk(warps * 32, 256)), dim3(256), 0, ST(stream),
                     (const uint16_t*)A, (const uint8_t*)B_enk, (const uint16_t*)S, (uint16_t*)C, row_expert_ids, M, K, N,
                     a_stride, expert_offset, num_local_experts));
     return 0;
@@ -681,7 +681,7 @@ int pgk_moe_route_t1(const void* logits, void* weights, int32_t* indices, int32_
                      int k, void* stream) {
     PGK_REQUIRE(num_experts >= 1 && num_experts <= 512 && k >= 1 && k <= num_experts && k <= 32,
                 "moe_route_t1 failed: unsupported num_experts=%d k=%d", num_experts, k);
-    PGK_CUDA(launch(moe_route_t1_kernel, dim3(1), dim3(32), 0, ST(stream), (const uint16_t*)logits, (uint16_t*)weights,
+    PGK_CUDA(launch_waiting(moe_route_t1_kernel, dim3(1), dim3(32), 0, ST(stream), (const uint16_t*)logits, (uint16_t*)weights,
                     indices, row_expert_ids, num_experts, k));
     return 0;
 }
@@ -694,7 +694,7 @@ int pgk_moe_gateup_fp8_t1(const void* x, const void* Bg_enk, const void* Sg, con
     if (int rc = moe_fp8_clean(Bg_enk, num_local_experts, N, K, stream, &cg)) return rc;
     if (int rc = moe_fp8_clean(Bu_enk, num_local_experts, N, K, stream, &cu)) return rc;
     auto kern = (cg && cu) ? moe_gateup_fp8_t1_kernel<true> : moe_gateup_fp8_t1_kernel<false>;
-    PGK_CUDA(launch(kern, dim3(nblk(warps * 32, 256)), dim3(256), 0, ST(stream), (const uint16_t*)x,
+    PGK_CUDA(launch_waiting(kern, dim3(nblk(warps * 32, 256)), dim3(256), 0, ST(stream), (const uint16_t*)x,
                     (const uint8_t*)Bg_enk, (const uint16_t*)Sg, (const uint8_t*)Bu_enk, (const uint16_t*)Su,
                     (uint16_t*)act, row_expert_ids, k, K, N, expert_offset, num_local_experts));
     return 0;
@@ -707,7 +707,7 @@ int pgk_moe_down_combine_fp8_t1(const void* act, const void* Bd_enk, const void*
     bool clean;
     if (int rc = moe_fp8_clean(Bd_enk, num_local_experts, N, K, stream, &clean)) return rc;
     auto kern = clean ? moe_down_combine_fp8_t1_kernel<true> : moe_down_combine_fp8_t1_kernel<false>;
-    PGK_CUDA(launch(kern, dim3((N + cols - 1) / cols), dim3(cols * k * 32), 0, ST(stream),
+    PGK_CUDA(launch_waiting(kern, dim3((N + cols - 1) / cols), dim3(cols * k * 32), 0, ST(stream),
                     (const uint16_t*)act, (const uint8_t*)Bd_enk, (const uint16_t*)Sd, (const uint16_t*)router_weights,
                     row_expert_ids, (const uint16_t*)residual, (uint16_t*)out, k, K, N, cols, expert_offset,
                     num_local_experts));
@@ -715,7 +715,7 @@ int pgk_moe_down_combine_fp8_t1(const void* act, const void* Bd_enk, const void*
 }
 int pgk_moe_combine_t1(const void* expert_out, const void* router_weights, const void* residual, void* out,
                        int hidden_size, int k, void* stream) {
-    PGK_CUDA(launch(moe_combine_t1_kernel, dim3(nblk(hidden_size, 256)), dim3(256), 0, ST(stream),
+    PGK_CUDA(launch_waiting(moe_combine_t1_kernel, dim3(nblk(hidden_size, 256)), dim3(256), 0, ST(stream),
                     (const uint16_t*)expert_out, (const uint16_t*)router_weights, (const uint16_t*)residual,
                     (uint16_t*)out, hidden_size, k));
     return 0;

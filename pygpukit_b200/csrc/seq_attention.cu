@@ -233,6 +233,8 @@ __device__ __forceinline__ float block_sum_256(float v, float* red) {
 // (k + b_k) / rms(all of k) * (w_off + w_k) as the KEY row, head by head
 template <typename TC>
 __global__ void __launch_bounds__(256) mixer_prep_all_kernel(PrepAllArgs a) {
+    griddep_wait();
+    griddep_launch();
     __shared__ float red[8];
     const int t = blockIdx.x;
     float* q = a.proj + (size_t)t * a.ld;
@@ -1081,8 +1083,8 @@ int pgk_seq_mixer_prep_all(float* proj, int ld, int tokens, int heads, int kv_he
     if (tokens <= 0) return 0;
     PrepAllArgs a{proj, ld, heads, kv_heads, dim, k_off, q_bias, k_bias, q_weight, k_weight, weight_offset, eps, k_cache, v_cache,
                   table, max_pages, page_size, slot, pos};
-    if (cache_dtype == 2) PGK_CUDA(launch(mixer_prep_all_kernel<uint16_t>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
-    else PGK_CUDA(launch(mixer_prep_all_kernel<float>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    if (cache_dtype == 2) PGK_CUDA(launch_waiting(mixer_prep_all_kernel<uint16_t>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    else PGK_CUDA(launch_waiting(mixer_prep_all_kernel<float>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 int pgk_seq_decode_heads_per_block(void) { return DPAIRS_MAX; }

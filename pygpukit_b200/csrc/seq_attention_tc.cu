@@ -141,6 +141,7 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     tc_fence_after();
     const uint32_t tmem = *tmem_slot;
     griddep_wait();
+    griddep_launch();
     const int4 tile = a.tiles[blockIdx.x];
     const int t0 = tile.x, nq = tile.y, slot = tile.z, pos0 = tile.w, D = a.D, Dv = a.Dv, HB = a.HB;
     const int rep = a.H / a.G, hsplit = (rep + HB - 1) / HB;
@@ -695,7 +696,7 @@ int launch_form(const TcAttnArgs& p, const CUtensorMap& kmap, const CUtensorMap&
         configured = true;
     }
     const int rep = p.a.H / p.a.G, hsplit = (rep + p.a.HB - 1) / p.a.HB;
-    PGK_CUDA(launch(seq_attention_tc_kernel<CAP, SLOPE, PROB>, dim3(tiles, p.a.G * hsplit, p.a.splits), dim3(A_THREADS), smem, st, kmap, vmap, p));
+    PGK_CUDA(launch_waiting(seq_attention_tc_kernel<CAP, SLOPE, PROB>, dim3(tiles, p.a.G * hsplit, p.a.splits), dim3(A_THREADS), smem, st, kmap, vmap, p));
     return 0;
 }
 

@@ -211,6 +211,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         asm volatile("prefetch.tensormap [%0];" :: "l"(&amap) : "memory");
     }
     griddep_wait();
+    griddep_launch();
     if (p.g.group_off && warp == 2) {            // tiles before every group
         int run = 0;
         for (int e0 = 0; e0 < p.batch; e0 += 32) {
@@ -390,6 +391,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
     }
     griddep_wait();
+    griddep_launch();
     const int m0 = p.rpb ? (int)blockIdx.z * p.rpb : 0, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z;
     const int rows = z < 0 ? 0 : min(p.rpb ? p.rpb : TC_DIRECT_ROWS, p.g.M - m0);      // no matrix: nothing to do, the same in the cluster
     tc_fence_before();
@@ -596,11 +598,10 @@ cudaError_t launch_clustered(const void* kernel, dim3 grid, size_t smem, int clu
     at[n].id = cudaLaunchAttributeClusterDimension;
     at[n].val.clusterDim.x = cluster; at[n].val.clusterDim.y = 1; at[n].val.clusterDim.z = 1;
     ++n;
-    if (pdl_enabled()) {
-        at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[n].val.programmaticStreamSerializationAllowed = 1;
-        ++n;
-    }
+    // both kernels wait before they touch anything (see launch_waiting)
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
     cfg.attrs = at; cfg.numAttrs = n;
     count_launch();
     return cudaLaunchKernelExC(&cfg, kernel, args);
@@ -703,7 +704,7 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
     const bool vec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
     int gy = (chunks + 255) / 256;
     if (gy > 8) gy = 8;
-    cudaError_t e = launch(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, a, (uint16_t*)abuf, batch, kpr, vec);
+    cudaError_t e = launch_waiting(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, a, (uint16_t*)abuf, batch, kpr, vec);
     if (e == cudaSuccess) {
         const int sms = sm_count();
         const long long tiles = (long long)batch * p.mt * p.nt;

@@ -85,6 +85,8 @@ __device__ __forceinline__ void latent_row(const LatentPrepArgs& a, int t, float
 
 template <typename TC>
 __global__ void __launch_bounds__(256) latent_prep_kernel(LatentPrepArgs a) {
+    griddep_wait();
+    griddep_launch();
     __shared__ float red[8];
     latent_row<TC>(a, blockIdx.x, red);
 }
@@ -119,7 +121,11 @@ __device__ __forceinline__ void rope_tails(const RopeHeadsArgs& a, int t, int pa
     }
 }
 
-__global__ void __launch_bounds__(256) rope_heads_kernel(RopeHeadsArgs a) { rope_tails(a, blockIdx.x, 0, 1); }
+__global__ void __launch_bounds__(256) rope_heads_kernel(RopeHeadsArgs a) {
+    griddep_wait();
+    griddep_launch();
+    rope_tails(a, blockIdx.x, 0, 1);
+}
 
 // blocks (t, 0 .. parts - 1): query tails; block (t, parts), when there is one: the cache row
 template <typename TC>
@@ -143,8 +149,8 @@ int pgk_seq_latent_prep(float* proj, int ld, int tokens, int q_rank, int kv_off,
     if (tokens <= 0) return 0;
     LatentPrepArgs a{proj, ld, q_rank, rank, rot, rot_dims, kv_off, q_weight, c_weight, weight_offset, eps, inv_freq, k_cache,
                      table, max_pages, page_size, slot, pos, 1.f};
-    if (cache_dtype == 2) PGK_CUDA(launch(latent_prep_kernel<uint16_t>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
-    else PGK_CUDA(launch(latent_prep_kernel<float>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    if (cache_dtype == 2) PGK_CUDA(launch_waiting(latent_prep_kernel<uint16_t>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    else PGK_CUDA(launch_waiting(latent_prep_kernel<float>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 
@@ -154,7 +160,7 @@ int pgk_seq_rope_heads(const float* src, int lds, int src_head, int src_off, flo
                 "seq_rope_heads failed: %d heads, rotated part %d of which %d turn", heads, rot, rot_dims);
     if (tokens <= 0 || rot == 0) return 0;
     RopeHeadsArgs a{src, lds, src_head, src_off, dst, ldd, dst_head, dst_off, heads, rot, rot_dims, inv_freq, pos, 1.f};
-    PGK_CUDA(launch(rope_heads_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    PGK_CUDA(launch_waiting(rope_heads_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 

@@ -16,6 +16,8 @@ template <> __device__ __forceinline__ float wload<uint16_t>(const uint16_t* p) 
 
 template <typename TW>
 __global__ void __launch_bounds__(256) embed_rows_kernel(const TW* table, const int* tok, float* x, int W, int vocab, float scale) {
+    griddep_wait();
+    griddep_launch();
     const int t = blockIdx.x;
     int id = tok[t];
     id = id < 0 ? 0 : (id >= vocab ? vocab - 1 : id);
@@ -98,6 +100,8 @@ struct RmsArgs {
 };
 
 __global__ void __launch_bounds__(256) rms_norm_rows_kernel(RmsArgs a) {
+    griddep_wait();
+    griddep_launch();
     extern __shared__ float y[];
     __shared__ float red[8];
     const int t = blockIdx.x;
@@ -130,6 +134,8 @@ struct RmsSeamArgs {
 };
 
 __global__ void __launch_bounds__(256) rms_seam_kernel(RmsSeamArgs a) {
+    griddep_wait();
+    griddep_launch();
     extern __shared__ float row[];
     __shared__ float red[8];
     const int t = blockIdx.x;
@@ -339,6 +345,8 @@ __global__ void __launch_bounds__(1024) rms_add_norm_kernel(RmsAddNormArgs a) {
 template <typename TW>
 __global__ void __launch_bounds__(256) embed_norm_rows_kernel(const TW* table, const int* tok, const float* w, float off, float eps,
                                                               float* x, float* keep, int W, int vocab) {
+    griddep_wait();
+    griddep_launch();
     extern __shared__ float row[];
     __shared__ float red[8];
     const int t = blockIdx.x;
@@ -470,8 +478,8 @@ int pgk_embed_rows_scaled_f32(const void* table, int wdt, const int32_t* tokens,
                               void* stream) {
     PGK_REQUIRE(wdt == 0 || wdt == 2, "embed_rows_f32 failed: table must be float32 (0) or bfloat16 (2), got %d", wdt);
     if (n <= 0) return 0;
-    if (wdt == 2) PGK_CUDA(launch(embed_rows_kernel<uint16_t>, dim3(n, (width + 1023) / 1024), dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)table, tokens, x, width, vocab, scale));
-    else PGK_CUDA(launch(embed_rows_kernel<float>, dim3(n, (width + 1023) / 1024), dim3(256), 0, (cudaStream_t)stream, (const float*)table, tokens, x, width, vocab, scale));
+    if (wdt == 2) PGK_CUDA(launch_waiting(embed_rows_kernel<uint16_t>, dim3(n, (width + 1023) / 1024), dim3(256), 0, (cudaStream_t)stream, (const uint16_t*)table, tokens, x, width, vocab, scale));
+    else PGK_CUDA(launch_waiting(embed_rows_kernel<float>, dim3(n, (width + 1023) / 1024), dim3(256), 0, (cudaStream_t)stream, (const float*)table, tokens, x, width, vocab, scale));
     return 0;
 }
 
@@ -504,7 +512,7 @@ int pgk_rms_norm_rows_f32(const float* x, const int32_t* src_rows, const float* 
         PGK_CUDA(cudaFuncSetAttribute(rms_norm_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         configured = true;
     }
-    PGK_CUDA(launch(rms_norm_rows_kernel, dim3(rows), dim3(256), smem, (cudaStream_t)stream, a));
+    PGK_CUDA(launch_waiting(rms_norm_rows_kernel, dim3(rows), dim3(256), smem, (cudaStream_t)stream, a));
     return 0;
 }
 
@@ -519,7 +527,7 @@ int pgk_rms_norm_seam_f32(const float* y, const float* weight1, float offset1, f
         PGK_CUDA(cudaFuncSetAttribute(rms_seam_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         configured = true;
     }
-    PGK_CUDA(launch(rms_seam_kernel, dim3(rows), dim3(256), smem, (cudaStream_t)stream, a));
+    PGK_CUDA(launch_waiting(rms_seam_kernel, dim3(rows), dim3(256), smem, (cudaStream_t)stream, a));
     return 0;
 }
 
@@ -570,8 +578,8 @@ int pgk_embed_norm_rows_f32(const void* table, int wdt, const int32_t* tokens, c
         PGK_CUDA(cudaFuncSetAttribute(embed_norm_rows_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         configured = true;
     }
-    if (wdt == 2) PGK_CUDA(launch(embed_norm_rows_kernel<uint16_t>, dim3(n), dim3(256), smem, (cudaStream_t)stream, (const uint16_t*)table, tokens, weight, weight_offset, eps, x, keep, width, vocab));
-    else PGK_CUDA(launch(embed_norm_rows_kernel<float>, dim3(n), dim3(256), smem, (cudaStream_t)stream, (const float*)table, tokens, weight, weight_offset, eps, x, keep, width, vocab));
+    if (wdt == 2) PGK_CUDA(launch_waiting(embed_norm_rows_kernel<uint16_t>, dim3(n), dim3(256), smem, (cudaStream_t)stream, (const uint16_t*)table, tokens, weight, weight_offset, eps, x, keep, width, vocab));
+    else PGK_CUDA(launch_waiting(embed_norm_rows_kernel<float>, dim3(n), dim3(256), smem, (cudaStream_t)stream, (const float*)table, tokens, weight, weight_offset, eps, x, keep, width, vocab));
     return 0;
 }
 

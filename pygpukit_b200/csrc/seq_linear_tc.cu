@@ -388,9 +388,9 @@ int linear_tc(const float* proj, int ld, int q_off, int k_off, int v_off, float*
     PGK_REQUIRE(err, "seq_linear_attention_chunks failed: no pinned host memory");
     LinTcArgs a{proj, ld, q_off, k_off, v_off, out, ldo, state, decay, (const int4*)seqs, H, D, Dv, begin, end, (end - begin + LT - 1) / LT, ws, err};
     const dim3 grid(a.chunks, n_seqs, H);
-    PGK_CUDA(launch(linear_tc_update_kernel, grid, dim3(256), L_SMEM, st, a));
-    PGK_CUDA(launch(linear_tc_scan_kernel, dim3((unsigned)((D * Dv + 511) / 512), H, n_seqs), dim3(128), 0, st, a));
-    PGK_CUDA(launch(linear_tc_output_kernel, grid, dim3(256), L_SMEM, st, a));
+    PGK_CUDA(launch_waiting(linear_tc_update_kernel, grid, dim3(256), L_SMEM, st, a));
+    PGK_CUDA(launch_waiting(linear_tc_scan_kernel, dim3((unsigned)((D * Dv + 511) / 512), H, n_seqs), dim3(128), 0, st, a));
+    PGK_CUDA(launch_waiting(linear_tc_output_kernel, grid, dim3(256), L_SMEM, st, a));
     return 0;
 }
 

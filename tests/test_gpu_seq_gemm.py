@@ -413,3 +413,36 @@ def test_idle_work_memory_goes_back():
         assert before - free_bytes() <= 32 << 20
     plain()
     assert (c.to_numpy() == 0).all()
+
+
+@pytest.mark.parametrize("M", [1, 8, 40, 300])
+def test_products_see_weights_and_rows_written_by_the_launch_before(M):
+    """Launches are brought to the SMs while the one before drains: weights and activations that the kernel just before has written are
+    the ones that the product reads, in every form (streaming GEMV, few rows, many rows), call after call without a wait."""
+    from pygpukit_b200 import llm
+    from pygpukit_b200._lib import api
+    K, N, rounds = 1024, 2048, 6
+    rng = np.random.default_rng(M)
+    W = [gk.from_numpy(rng.standard_normal((N, K)).astype(np.float32)) for _ in range(rounds)]
+    X = [gk.from_numpy(rng.standard_normal((M, K)).astype(np.float32)) for _ in range(rounds)]
+
+    def run(wait):
+        w, x, xb = gk.zeros((N, K), gk.bfloat16), gk.zeros((M, K), gk.float32), gk.zeros((M, K), gk.bfloat16)
+        rows, gemv = [gk.zeros((M, N), gk.float32) for _ in range(rounds)], [gk.zeros((M, N), gk.bfloat16) for _ in range(rounds)]
+        layer = llm.LinearRows(w)
+        for i in range(rounds):
+            api.cast(X[i].device_ptr, x.device_ptr, M * K, 0, 0, None)
+            api.cast(W[i].device_ptr, w.device_ptr, N * K, 0, 2, None)
+            if wait:
+                api.device_sync()
+            layer.forward(x.device_ptr, K, M, rows[i].device_ptr, N)
+            if M <= 8:
+                api.cast(X[i].device_ptr, xb.device_ptr, M * K, 0, 2, None)
+                api.cast(W[rounds - 1 - i].device_ptr, w.device_ptr, N * K, 0, 2, None)
+                if wait:
+                    api.device_sync()
+                api.gemv_bf16(xb.device_ptr, w.device_ptr, gemv[i].device_ptr, M, K, N, None)
+        return [a.to_numpy() for a in rows + gemv]
+
+    for a, b in zip(run(True), run(False)):
+        assert np.array_equal(a, b)
