@@ -110,7 +110,9 @@ inline cudaError_t launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_
 // For kernels whose every block executes griddep_wait() before it touches global memory: they may always be brought to the SMs while
 // the kernel before them drains, which hides the launch (2 ... 4 us of a kernel with a large block); whoever comes after them finds
 // everything before them finished, since they do not finish earlier themselves.  What a kernel reads AHEAD of its wait (weights, see
-// griddep_wait) it reads ahead only under pdl_enabled(); otherwise its first act is the wait.
+// griddep_wait) it reads ahead only under pdl_enabled(); otherwise its first act is the wait.  Measured (us a pass, plain launches
+// -> these): one FP8 GEMV of 6144 x 4096 10.2 -> 8.2, attention layer of one token 30.7 -> 25.2, five launches of a mixture of experts
+// 32.8 -> 22.0, decode step of eight requests 453 -> 436.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_waiting(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     return launch_as(true, kernel, grid, block, smem, stream, args...);

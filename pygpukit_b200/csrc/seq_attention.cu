@@ -48,6 +48,8 @@ struct PrepArgs {
 // units: H query heads, G key heads, G value heads; one warp each, four per block
 template <typename TC>
 __global__ void __launch_bounds__(128) mixer_prep_kernel(PrepArgs a) {
+    griddep_wait();
+    griddep_launch();
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int u = blockIdx.y * 4 + warp;
     if (u >= a.H + 2 * a.G) return;
@@ -982,8 +984,8 @@ int pgk_seq_mixer_prep(float* proj, int ld, int tokens, int heads, int kv_heads,
     if (tokens <= 0) return 0;
     PrepArgs a{proj, ld, heads, kv_heads, dim, vdim, q_weight, k_weight, eps, v_mode, lam, v_first, k_cache, v_cache, table,
                max_pages, page_size, slot, pos};
-    if (cache_dtype == 2) PGK_CUDA(launch(mixer_prep_kernel<uint16_t>, dim3(tokens, (heads + 2 * kv_heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
-    else PGK_CUDA(launch(mixer_prep_kernel<float>, dim3(tokens, (heads + 2 * kv_heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
+    if (cache_dtype == 2) PGK_CUDA(launch_waiting(mixer_prep_kernel<uint16_t>, dim3(tokens, (heads + 2 * kv_heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
+    else PGK_CUDA(launch_waiting(mixer_prep_kernel<float>, dim3(tokens, (heads + 2 * kv_heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
     return 0;
 }
 

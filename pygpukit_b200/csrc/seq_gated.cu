@@ -113,6 +113,8 @@ __device__ __forceinline__ void warp_argmax(float& v, int& i) {
 constexpr int ROUTE_WARPS = 4;       // tokens per block, a warp each
 
 __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_biased_kernel(RouteBiasArgs a) {
+    griddep_wait();
+    griddep_launch();
     extern __shared__ float sm[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t = blockIdx.x * ROUTE_WARPS + warp;
@@ -313,6 +315,8 @@ __device__ __forceinline__ float combine_gate(const CombineArgs& a, int t) {
 
 template <bool VEC>
 __global__ void __launch_bounds__(256) moe_combine_rows_kernel(CombineArgs a) {
+    griddep_wait();
+    griddep_launch();
     __shared__ float wk[CTOP];
     __shared__ long long pk[CTOP];
     const int t = blockIdx.x;
@@ -720,7 +724,7 @@ int pgk_moe_route_biased(const float* logits, int ld, int tokens, int outputs, i
     RouteBiasArgs a{logits, ld, tokens, outputs, real_experts, top, renorm ? 1 : 0, bias, idx, mat, weights, rank, counts};
     const size_t smem = (size_t)ROUTE_WARPS * 2 * outputs * 4;
     PGK_REQUIRE(smem <= 48 * 1024, "moe_route_biased failed: too many router outputs (%d)", outputs);
-    PGK_CUDA(launch(moe_route_biased_kernel, dim3((tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), smem,
+    PGK_CUDA(launch_waiting(moe_route_biased_kernel, dim3((tokens + ROUTE_WARPS - 1) / ROUTE_WARPS), dim3(ROUTE_WARPS * 32), smem,
                     (cudaStream_t)stream, a));
     return 0;
 }
@@ -765,8 +769,8 @@ int pgk_moe_combine_rows_f32(const float* parts, const int32_t* inv, const int32
     const uintptr_t all = (uintptr_t)a.parts | (uintptr_t)a.self_rows | (uintptr_t)a.shared | (uintptr_t)a.out;
     const bool vec = a.W % 4 == 0 && all % 16 == 0 && top <= 8;
     const int threads = a.W < 1024 ? (a.W / 4 + 31) / 32 * 32 : 256;
-    if (vec) PGK_CUDA(launch(moe_combine_rows_kernel<true>, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, a));
-    else PGK_CUDA(launch(moe_combine_rows_kernel<false>, dim3(rows), dim3(256), 0, (cudaStream_t)stream, a));
+    if (vec) PGK_CUDA(launch_waiting(moe_combine_rows_kernel<true>, dim3(rows), dim3(threads), 0, (cudaStream_t)stream, a));
+    else PGK_CUDA(launch_waiting(moe_combine_rows_kernel<false>, dim3(rows), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 

@@ -471,6 +471,8 @@ constexpr int SKM = 4, SK_WARPS = 4;
 
 template <int SKN>
 __global__ void __launch_bounds__(SK_WARPS * 32) gemm_skinny_f32_kernel(GemmArgs a) {
+    griddep_wait();
+    griddep_launch();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m0 = (blockIdx.x * SK_WARPS + warp) * SKM, n0 = blockIdx.y * SKN;
     if (m0 >= a.M) return;
@@ -531,8 +533,8 @@ int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const vo
     cudaStream_t st = (cudaStream_t)stream;
     if (wdt == 0 && epilogue == 0 && !group_off && !a_rows && N <= 64) {        // router logits: few columns, float32 weights
         const int gx = (M + SK_WARPS * SKM - 1) / (SK_WARPS * SKM);
-        if (N <= 4) PGK_CUDA(launch(gemm_skinny_f32_kernel<4>, dim3(gx), dim3(SK_WARPS * 32), 0, st, a));
-        else PGK_CUDA(launch(gemm_skinny_f32_kernel<8>, dim3(gx, (N + 7) / 8), dim3(SK_WARPS * 32), 0, st, a));
+        if (N <= 4) PGK_CUDA(launch_waiting(gemm_skinny_f32_kernel<4>, dim3(gx), dim3(SK_WARPS * 32), 0, st, a));
+        else PGK_CUDA(launch_waiting(gemm_skinny_f32_kernel<8>, dim3(gx, (N + 7) / 8), dim3(SK_WARPS * 32), 0, st, a));
         return 0;
     }
     const int bound = group_off ? total_rows : M;

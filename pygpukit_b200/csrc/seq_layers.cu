@@ -54,6 +54,8 @@ struct NormArgs {
 constexpr int TOPMAX = 64;          // (token, slot) rows staged in shared memory; beyond that they are re-read
 
 __global__ void __launch_bounds__(256) combine_norm_kernel(NormArgs a) {
+    griddep_wait();
+    griddep_launch();
     extern __shared__ float y[];
     __shared__ float red[8];
     __shared__ float wk[TOPMAX];
@@ -453,6 +455,8 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(RouteArgs a
 // perm[row] = token, inv[t * top + k] = row
 __global__ void __launch_bounds__(1024) moe_lists_kernel(int* counts, int* offsets, const int* idx, const int* rank, int* perm,
                                                         int* inv, int E, int n, int top) {
+    griddep_wait();
+    griddep_launch();
     if (threadIdx.x == 0) {
         int acc = 0;
         for (int e = 0; e < E; ++e) { offsets[e] = acc; acc += counts[e]; counts[e] = 0; }
@@ -496,7 +500,7 @@ int pgk_combine_layernorm_f32(const float* base, const int32_t* src_rows, const 
         PGK_CUDA(cudaFuncSetAttribute(combine_norm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
         configured = true;
     }
-    PGK_CUDA(launch(combine_norm_kernel, dim3(rows), dim3(256), smem, (cudaStream_t)stream, a));
+    PGK_CUDA(launch_waiting(combine_norm_kernel, dim3(rows), dim3(256), smem, (cudaStream_t)stream, a));
     return 0;
 }
 
@@ -602,7 +606,7 @@ int pgk_moe_route_grouped(const float* logits, int ld, int tokens, int experts, 
 int pgk_moe_row_lists(int32_t* counts, int32_t* offsets, const int32_t* idx, const int32_t* rank, int32_t* perm, int32_t* inv,
                       int experts, int tokens, int top, void* stream) {
     if (tokens <= 0) return 0;
-    PGK_CUDA(launch(moe_lists_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, counts, offsets, idx, rank, perm, inv, experts,
+    PGK_CUDA(launch_waiting(moe_lists_kernel, dim3(1), dim3(1024), 0, (cudaStream_t)stream, counts, offsets, idx, rank, perm, inv, experts,
                     tokens * top, top));
     return 0;
 }

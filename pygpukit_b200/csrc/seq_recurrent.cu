@@ -74,6 +74,8 @@ __global__ void __launch_bounds__(256) causal_conv_rows_kernel(ConvArgs a) {
 constexpr int CTAPS = 4, CROWS = 4;
 
 __global__ void __launch_bounds__(256) causal_conv_many_kernel(ConvArgs a) {
+    griddep_wait();
+    griddep_launch();
     const int t0 = blockIdx.x * CROWS, c = blockIdx.y * 256 + threadIdx.x;
     if (c >= a.W) return;
     const int ring = a.taps - 1, W = a.W;
@@ -172,6 +174,8 @@ __global__ void __launch_bounds__(128) linear_prep_kernel(LinPrepArgs a) {
 constexpr int LIN_TURNS = 4096;                           // angles that shared memory holds
 
 __global__ void __launch_bounds__(256) linear_prep_many_kernel(LinPrepArgs a) {
+    griddep_wait();
+    griddep_launch();
     extern __shared__ float2 turn[];                      // [rot_dims / 2] (sine, cosine)
     const int t = blockIdx.x, lane = threadIdx.x & 31, half = a.rot_dims / 2;
     const int pos = half ? a.pos[t] : 0;
@@ -480,6 +484,8 @@ struct LinFinishArgs {
 };
 
 __global__ void __launch_bounds__(256) linear_finish_kernel(LinFinishArgs a) {
+    griddep_wait();
+    griddep_launch();
     __shared__ float red[8];
     __shared__ float inv_s[256];
     const int t = blockIdx.x, n = a.H * a.Dv, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -537,7 +543,7 @@ int pgk_causal_conv_rows_ex_f32(const float* h, int ldh, float* u, int ldu, cons
                activation ? 1 : 0};
     // four rows per thread from 256 rows on (2000 rows: 38 -> 24 us); fewer leave SMs idle
     if (rows >= 256 && taps <= CTAPS)
-        PGK_CUDA(launch(causal_conv_many_kernel, dim3((rows + CROWS - 1) / CROWS, (width + 255) / 256), dim3(256), 0, (cudaStream_t)stream, a));
+        PGK_CUDA(launch_waiting(causal_conv_many_kernel, dim3((rows + CROWS - 1) / CROWS, (width + 255) / 256), dim3(256), 0, (cudaStream_t)stream, a));
     else
         PGK_CUDA(launch(causal_conv_rows_kernel, dim3(rows, (width + 255) / 256), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
@@ -566,7 +572,7 @@ int pgk_seq_linear_prep(float* proj, int ld, int tokens, int heads, int dim, int
     if (heads > 8 && rot_dims / 2 <= LIN_TURNS) {
         // a unit per warp while that fills the SMs no more than once, then two blocks per token (angles twice instead of six times)
         const int all = (3 * heads + 7) / 8, groups = (long long)tokens * all <= 8 * sm_count() ? all : 2;
-        PGK_CUDA(launch(linear_prep_many_kernel, dim3(tokens, groups), dim3(256), (size_t)(rot_dims / 2) * sizeof(float2), (cudaStream_t)stream, a));
+        PGK_CUDA(launch_waiting(linear_prep_many_kernel, dim3(tokens, groups), dim3(256), (size_t)(rot_dims / 2) * sizeof(float2), (cudaStream_t)stream, a));
     } else
         PGK_CUDA(launch(linear_prep_kernel, dim3(tokens, (3 * heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
     return 0;
@@ -637,7 +643,7 @@ int pgk_seq_linear_finish(float* o, int ldo, const float* gate_rows, int ldg, in
                 "seq_linear_finish failed: invalid arguments");
     if (tokens <= 0) return 0;
     LinFinishArgs a{o, ldo, gate_rows, ldg, gate_off, weight, heads, vdim, per_head ? 1 : 0, gate_act, eps, mult};
-    PGK_CUDA(launch(linear_finish_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    PGK_CUDA(launch_waiting(linear_finish_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 

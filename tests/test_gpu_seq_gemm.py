@@ -419,8 +419,6 @@ def test_idle_work_memory_goes_back():
 def test_products_see_weights_and_rows_written_by_the_launch_before(M):
     """Launches are brought to the SMs while the one before drains: weights and activations that the kernel just before has written are
     the ones that the product reads, in every form (streaming GEMV, few rows, many rows), call after call without a wait."""
-    from pygpukit_b200 import llm
-    from pygpukit_b200._lib import api
     K, N, rounds = 1024, 2048, 6
     rng = np.random.default_rng(M)
     W = [gk.from_numpy(rng.standard_normal((N, K)).astype(np.float32)) for _ in range(rounds)]
