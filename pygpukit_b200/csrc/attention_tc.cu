@@ -369,7 +369,10 @@ int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, 
                 "sdpa_causal_fixed_cache failed: cuTensorMapEncodeTiled refused the operands");
     if (p.splits > 1) {
         void* ws = nullptr;
-        if (int rc = scratch_alloc(&ws, (size_t)q_len * hq * p.splits * (M_D + 4) * sizeof(float), st)) return rc;
+        if (scratch_alloc(&ws, (size_t)q_len * hq * p.splits * (M_D + 4) * sizeof(float), st)) {
+            set_error("");                                // no room for the records: one range
+            p.splits = 1;
+        }
         p.ws = (float*)ws;
     }
     cudaError_t e = launch_waiting(sdpa_prompt_kernel, dim3(qtiles, n_kv * p.hsplit, p.splits), dim3(M_THREADS), M_SMEM, st, kmap, vmap, p);

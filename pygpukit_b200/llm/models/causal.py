@@ -247,7 +247,8 @@ class CausalTransformerModel:
         slab = self.buffers.max_batch_size
         if len(input_ids) > slab and self._long_portions():
             hidden = self._prompt(list(input_ids), start)
-            return hidden, (start + len(input_ids) if use_cache else None)
+            if hidden is not None:
+                return hidden, (start + len(input_ids) if use_cache else None)
         for i in range(0, len(input_ids), slab):
             ids = input_ids[i:i + slab]
             hidden = self._decode_step_fixed_cache_batch(ids, start + i, start + i + len(ids))
@@ -271,7 +272,7 @@ class CausalTransformerModel:
 
     def _prompt(self, ids: list[int], start: int) -> GPUArray:
         """`ids` through all layers, PROMPT_ROWS rows at a time; returns the final-norm hidden of the last slab of `max_batch_size`
-        rows, like the slabs would."""
+        rows, like the slabs would; None, and nothing done, when there is no room for the portion's arrays."""
         slab, n = self.buffers.max_batch_size, len(ids)
         if start + n > self._max_seq:
             raise ValueError(f"context_len {start + n} exceeds the fixed cache ({self._max_seq})")
@@ -279,7 +280,10 @@ class CausalTransformerModel:
         rows = min(portion, n)
         if self._prompt_bufs is None or self._prompt_bufs.max_seq_len < rows:
             self._prompt_bufs = None
-            self._prompt_bufs = PrefillBuffers.for_rows(self.config, rows)
+            try:
+                self._prompt_bufs = PrefillBuffers.for_rows(self.config, rows)
+            except RuntimeError:                     # out of device memory
+                return None
         b, hidden = self._prompt_bufs, None
         for i in range(0, n, portion):
             part = ids[i:i + portion]
