@@ -126,6 +126,8 @@ inline cudaError_t launch_waiting(void (*kernel)(KArgs...), dim3 grid, dim3 bloc
 // kernel before the predecessor has completed and flushed: code placed before griddep_wait() may read
 // anything that was last written two or more kernels back (weights, the device-side position counters,
 // KV-cache rows of earlier steps), never the predecessor's outputs.
+// A kernel that allocates tensor memory lets no thread execute launch_dependents before a barrier of the block behind the allocation: a
+// dependent block that had taken the columns first would hold them until this grid has finished, and this grid would wait for them.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

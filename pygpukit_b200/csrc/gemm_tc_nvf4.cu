@@ -115,7 +115,6 @@ gemm_nvf4_tc_kernel(N4Params p) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     griddep_wait();
-    griddep_launch();
 #pragma unroll
     for (int d = 0; d < RAW; ++d) {
         if (conv && d < nkb) issue_acts(kb0 + d, d);
@@ -126,6 +125,7 @@ gemm_nvf4_tc_kernel(N4Params p) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    griddep_launch();                                  // tensor memory is held
     const uint32_t tmem_d = tmem_base_s;
     constexpr uint32_t idesc = umma_idesc_bf16(NB);
     // converter role of this thread: k chunk c (8 k = 4 byte rows), columns 4 n4 .. 4 n4 + 3

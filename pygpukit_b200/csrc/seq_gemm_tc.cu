@@ -211,7 +211,6 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
         asm volatile("prefetch.tensormap [%0];" :: "l"(&amap) : "memory");
     }
     griddep_wait();
-    griddep_launch();
     if (p.g.group_off && warp == 2) {            // tiles before every group
         int run = 0;
         for (int e0 = 0; e0 < p.batch; e0 += 32) {
@@ -232,6 +231,7 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    griddep_launch();                            // tensor memory is held
     const uint32_t tmem = tmem_base_s;
     const int total = p.g.group_off ? pre[p.batch] : p.batch * p.mt * p.nt;
     const int rank = p.splits > 1 ? (int)cluster_rank() : 0;
@@ -391,12 +391,12 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
     }
     griddep_wait();
-    griddep_launch();
     const int m0 = p.rpb ? (int)blockIdx.z * p.rpb : 0, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z;
     const int rows = z < 0 ? 0 : min(p.rpb ? p.rpb : TC_DIRECT_ROWS, p.g.M - m0);      // no matrix: nothing to do, the same in the cluster
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    griddep_launch();                            // tensor memory is held
     const uint32_t tmem = tmem_base_s;
     if (p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");       // this block runs
     float v[16];

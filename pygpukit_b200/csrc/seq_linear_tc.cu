@@ -100,7 +100,6 @@ __global__ void __launch_bounds__(256, 1) linear_tc_update_kernel(const __grid_c
     __shared__ float pw[LT + 1];
     LinBlock b;
     griddep_wait();
-    griddep_launch();
     if (!lin_block(a, b)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t ks = (smem_u32(smem) + 1023u) & ~1023u, vs = ks + L_OPERAND;
@@ -108,6 +107,7 @@ __global__ void __launch_bounds__(256, 1) linear_tc_update_kernel(const __grid_c
     if (tid == 0) { mbar_init(&done, 1); mbar_fence_init(); }
     if (tid <= LT) pw[tid] = powf(b.dec, (float)tid);
     __syncthreads();
+    griddep_launch();                              // tensor memory is held
     const float* kp = a.proj + (size_t)b.r0 * a.ld + a.k_off + (size_t)b.h * a.D;
     const float* vp = a.proj + (size_t)b.r0 * a.ld + a.v_off + (size_t)b.h * a.Dv;
     const int vw = (a.Dv + 63) & ~63, N = (a.Dv + 15) & ~15;
@@ -199,7 +199,6 @@ __global__ void __launch_bounds__(256, 1) linear_tc_output_kernel(const __grid_c
     __shared__ float pw[LT + 1];
     LinBlock b;
     griddep_wait();
-    griddep_launch();
     if (!lin_block(a, b)) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t r1 = (smem_u32(smem) + 1023u) & ~1023u, r2 = r1 + L_OPERAND;
@@ -210,6 +209,7 @@ __global__ void __launch_bounds__(256, 1) linear_tc_output_kernel(const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
+    griddep_launch();
     const float* qp = a.proj + (size_t)b.r0 * a.ld + a.q_off + (size_t)b.h * a.D;
     const float* kp = a.proj + (size_t)b.r0 * a.ld + a.k_off + (size_t)b.h * a.D;
     const float* vp = a.proj + (size_t)b.r0 * a.ld + a.v_off + (size_t)b.h * a.Dv;
