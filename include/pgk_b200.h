@@ -76,6 +76,7 @@ int pgk_event_elapsed_ms(void* start, void* stop, float* ms);
 /* CUDA-graph capture of a decode step: native/core/cuda_graph.cpp, used by
  * llm/decode/m1_graph.py:248-457 */
 int pgk_graph_begin(void* stream);
+int pgk_stream_capturing(void* stream, int* capturing);
 int pgk_graph_end(void* stream, void** graph_exec);
 int pgk_graph_launch(void* graph_exec, void* stream);
 int pgk_graph_destroy(void* graph_exec);

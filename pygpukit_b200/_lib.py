@@ -36,7 +36,7 @@ _SIGS = {
     "pgk_stream_create": [C.POINTER(vp)], "pgk_stream_destroy": [vp], "pgk_stream_sync": [vp],
     "pgk_event_create": [C.POINTER(vp)], "pgk_event_destroy": [vp], "pgk_event_record": [vp, vp],
     "pgk_event_sync": [vp], "pgk_event_elapsed_ms": [vp, vp, C.POINTER(f32)],
-    "pgk_graph_begin": [vp], "pgk_graph_end": [vp, C.POINTER(vp)], "pgk_graph_launch": [vp, vp],
+    "pgk_graph_begin": [vp], "pgk_stream_capturing": [vp, C.POINTER(C.c_int)], "pgk_graph_end": [vp, C.POINTER(vp)], "pgk_graph_launch": [vp, vp],
     "pgk_graph_destroy": [vp],
     "pgk_set_pdl": [i32], "pgk_flush_l2": [vp],
     "pgk_gemv_fp8_bf16": [vp, vp, vp, vp, i32, i32, i32, vp],

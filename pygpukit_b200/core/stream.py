@@ -57,6 +57,13 @@ def use_stream(stream: "Stream | None"):
         _current = prev
 
 
+def is_capturing(handle) -> bool:
+    """What is enqueued on this stream is recorded into a graph and does not run."""
+    out = C.c_int(0)
+    api.stream_capturing(handle, C.byref(out))
+    return out.value != 0
+
+
 def default_stream():
     return None
 

@@ -380,6 +380,12 @@ int pgk_graph_begin(void* stream) {
     PGK_CUDA(cudaStreamBeginCapture(S(stream), cudaStreamCaptureModeThreadLocal));
     return 0;
 }
+int pgk_stream_capturing(void* stream, int* capturing) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    PGK_CUDA(cudaStreamIsCapturing(S(stream), &cs));
+    *capturing = cs != cudaStreamCaptureStatusNone;
+    return 0;
+}
 int pgk_graph_end(void* stream, void** graph_exec) {
     cudaGraph_t g = nullptr;
     PGK_CUDA(cudaStreamEndCapture(S(stream), &g));

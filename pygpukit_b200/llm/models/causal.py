@@ -23,7 +23,7 @@ from ..._lib import api
 from ...core.array import GPUArray
 from ...core.dtypes import bfloat16, int32
 from ...core.factory import from_numpy
-from ...core.stream import CudaGraph, Stream, current_stream_handle as _st, use_stream
+from ...core.stream import CudaGraph, Stream, current_stream_handle as _st, is_capturing, use_stream
 from ..buffers import DecodeBuffers, PrefillBuffers
 from ..config import ModelSpec, TransformerConfig
 from ..layers.block import TransformerBlock
@@ -144,15 +144,22 @@ class CausalTransformerModel:
         return self._buffers
 
     # ------------------------------------------------------------------ pieces
+    def _enter(self, stream) -> None:
+        """Every step works on the same arrays and none waits for its end: what is about to be enqueued on `stream` comes after the last
+        step, which may still run on another stream (streams have no order among each other)."""
+        if self._last_stream is not None and self._last_stream[0] is stream:
+            return
+        if is_capturing(stream):
+            return
+        api.device_sync()
+        self._last_stream = (stream,)
+
     def _embed(self, token_ids: list[int] | None, M: int, start_position: int, b: DecodeBuffers) -> GPUArray:
         hidden = b.hidden if b.hidden.shape[0] == M else b.hidden.slice_rows(M)
         if token_ids is not None:
             ids = np.asarray(token_ids, np.int32)
-            stream = _st()
-            if self._last_stream is None or self._last_stream[0] is not stream:
-                api.device_sync()                # the step before ran on another stream, on the same arrays
-                self._last_stream = (stream,)
-            api.upload(b.token_buf.device_ptr, ids.ctypes.data_as(C.c_void_p), ids.nbytes, stream)
+            self._enter(_st())
+            api.upload(b.token_buf.device_ptr, ids.ctypes.data_as(C.c_void_p), ids.nbytes, _st())
         self._embed_rows(hidden, M, start_position, None, b)
         return hidden
 
@@ -299,7 +306,7 @@ class CausalTransformerModel:
         """One greedy token entirely on the device: reads token_buf / position_buf / context_buf,
         writes the sampled token to next_token AND token_buf, then advances position / context."""
         b = self.buffers
-        self._last_stream = (_st(),)
+        self._enter(_st())
         if getattr(self, "_num_sequences", 1) > 1:
             return self._decode_step_device_multi()
         step = self.step_program()
@@ -369,6 +376,7 @@ class CausalTransformerModel:
         if len(toks) != S or len(pos) != S:
             raise ValueError(f"decode state needs {S} tokens / positions")
         st = np.array(pos + [p + 1 for p in pos] + toks, np.int32)
+        self._enter(_st())
         api.memcpy_h2d(b.state_buf.device_ptr, st.ctypes.data_as(C.c_void_p), st.nbytes, _st())
         api.stream_sync(_st()) if _st() is not None else api.device_sync()
 
@@ -395,8 +403,8 @@ class CausalTransformerModel:
         arr[2 * S:3 * S] = toks
         b = self.buffers
         sh = self._graph_stream.handle
+        self._enter(sh)
         api.memcpy_h2d(b.state_buf.device_ptr, pin, 12 * S, sh)
-        self._last_stream = (sh,)
         self._graph.replay(self._graph_stream)
         api.memcpy_d2h(pin.value + 12 * S, b.next_token.device_ptr, 4 * S, sh)
         api.stream_sync(sh)
@@ -418,7 +426,7 @@ class CausalTransformerModel:
 
     def decode_graph_replay(self) -> None:
         assert self._graph is not None, "Call init_decode_graph first"
-        self._last_stream = (self._graph_stream.handle,)
+        self._enter(self._graph_stream.handle)
         self._graph.replay(self._graph_stream)
 
     # ------------------------------------------------------------------ generation
@@ -490,6 +498,7 @@ class CausalTransformerModel:
     def snapshot_kv_cache(self) -> list[tuple[np.ndarray, np.ndarray]]:
         """Every layer's K / V cache on the host (causal.py:1003-1015): BF16 bit patterns, [sequences x n_kv, max_seq,
         head_dim].  The speculative / Jacobi paths here do not need it (lookahead pointers); kept for callers that do."""
+        self._enter(_st())
         return [(blk.attn._k_cache.to_numpy().copy(), blk.attn._v_cache.to_numpy().copy()) for blk in self.blocks]
 
     def restore_kv_cache(self, snapshot: list[tuple[np.ndarray, np.ndarray]]) -> None:
@@ -497,6 +506,7 @@ class CausalTransformerModel:
         a captured decode graph stays valid."""
         if len(snapshot) != len(self.blocks):
             raise ValueError(f"snapshot holds {len(snapshot)} layers, the model has {len(self.blocks)}")
+        self._enter(_st())
         for blk, (k_np, v_np) in zip(self.blocks, snapshot):
             blk.attn._k_cache.copy_from_numpy(np.ascontiguousarray(k_np, np.uint16))
             blk.attn._v_cache.copy_from_numpy(np.ascontiguousarray(v_np, np.uint16))

@@ -406,3 +406,45 @@ def test_long_prompt_portions_equal_slabs(n, monkeypatch):
     assert np.linalg.norm(a - b) <= 10 * 2.0 ** -9 * np.linalg.norm(b)
     for x, y in zip(ka, kb):
         assert np.linalg.norm(x - y) <= 10 * 2.0 ** -9 * np.linalg.norm(y)
+
+
+def test_captured_steps_follow_an_unfinished_prompt():
+    """Prompts do not wait for their end and captured steps run on a stream of their own: a step right behind a prompt, and a prompt right
+    behind steps, give what they give when each is waited for.  A caller may record a step into a graph of its own at any time."""
+    from pygpukit_b200._lib import api
+    from pygpukit_b200.core.stream import CudaGraph, Stream
+    model = llm.build_random_model("tiny-qwen3", "fp8", max_seq=1280, seed=7, std=0.05)
+    rng = np.random.default_rng(5)
+    prompts = [[int(t) for t in rng.integers(0, model.config.vocab_size, n)] for n in (1100, 700)]
+
+    def run(wait):
+        model.init_decode(1280, max_batch_size=16)
+        model.init_decode_graph()
+        out = []
+        for p in prompts:
+            model.prefill(p[:-1])
+            if wait:
+                api.device_sync()
+            tok = model.decode_step_host(p[-1], len(p) - 1)
+            out.append((tok, model.buffers.logits.to_numpy().copy()))
+            model.decode_graph_replay()
+            if wait:
+                api.device_sync()
+        api.device_sync()
+        return out, [k for kv in model.snapshot_kv_cache() for k in kv]
+
+    (a, ka), (b, kb) = run(True), run(False)
+    for (t, x), (u, y) in zip(a, b):
+        assert t == u and np.array_equal(x, y)
+    assert all(np.array_equal(x, y) for x, y in zip(ka, kb))
+    model.prefill(prompts[0])
+    side, g = Stream(), CudaGraph()
+    with g.capture(side):
+        model.decode_step_device()
+    model.set_decode_state(7, 1100)
+    g.replay(side)
+    side.synchronize()
+    first = int(model.buffers.next_token.to_numpy()[0])
+    model.set_decode_state(7, 1100)
+    model.decode_step_device()
+    assert int(model.buffers.next_token.to_numpy()[0]) == first
