@@ -14,10 +14,33 @@ import ctypes as C
 from .._lib import api
 
 _current = None  # ctypes void* handle or None (default stream)
+_open = False    # the current stream has work that its callers may take for complete (see `leave_open`)
 
 
 def current_stream_handle():
     return _current
+
+
+def leave_open() -> None:
+    """For work that used to be waited for: it is left running on the current stream, whose order everything enqueued there keeps; a
+    change of the current stream (streams have no order among each other) or a capture waits for it first."""
+    global _open
+    _open = True
+
+
+def settle() -> None:
+    """Wait for what `leave_open` left running."""
+    global _open
+    if _open:
+        _open = False
+        api.stream_sync(_current)
+
+
+def _switch(handle) -> None:
+    global _current
+    if handle is not _current:
+        settle()
+    _current = handle
 
 
 class Stream:
@@ -30,14 +53,16 @@ class Stream:
         api.stream_sync(self.handle)
 
     def __enter__(self) -> "Stream":
-        global _current
         self._prev = _current
-        _current = self.handle
+        _switch(self.handle)
         return self
 
     def __exit__(self, *exc) -> None:
         global _current
-        _current = self._prev
+        try:
+            _switch(self._prev)
+        finally:                                 # also when the work that was waited for has failed
+            _current = self._prev
 
     def __del__(self) -> None:
         try:
@@ -50,11 +75,14 @@ class Stream:
 def use_stream(stream: "Stream | None"):
     global _current
     prev = _current
-    _current = stream.handle if stream is not None else None
+    _switch(stream.handle if stream is not None else None)
     try:
         yield
     finally:
-        _current = prev
+        try:
+            _switch(prev)
+        finally:
+            _current = prev
 
 
 def is_capturing(handle) -> bool:
@@ -120,6 +148,7 @@ class CudaGraph:
     def capture(self, stream: Stream):
         self._stream = stream
         with use_stream(stream):
+            settle()
             api.graph_begin(stream.handle)
             try:
                 yield self

@@ -22,7 +22,7 @@ import numpy as np
 from ..._lib import api
 from ...core.array import GPUArray
 from ...core.dtypes import float32, int32
-from ...core.stream import CudaGraph, Stream, current_stream_handle as _st
+from ...core.stream import CudaGraph, Stream, current_stream_handle as _st, leave_open
 from ..buffers import RowBuffers
 from ..config import LayeredConfig
 from ..layers.linear import LinearRows
@@ -234,7 +234,9 @@ class LayeredCausalModel:
 
     def step_device(self, entries, end=()) -> tuple[GPUArray | None, int]:
         """Run one ragged batch; returns (float32 logits [n_want, vocab] on the device or None, n_want).  `end` names
-        the requests whose cache is given back after the step."""
+        the requests whose cache is given back after the step.  The step runs in the order of the current stream and is not waited for: what
+        reads its results there (`to_numpy`, the library's operators) finds them.  Decode steps are also complete for whoever makes another
+        stream the current one; a prompt, and any call that names a stream by its handle, needs a wait or an event of the caller's own."""
         if self.cache is None:
             self.init_cache()
         V = self.config.vocab_size
@@ -271,6 +273,7 @@ class LayeredCausalModel:
                         self._forward(ctx)
                     self._graphs[key] = g
                 api.graph_launch(g._exec, stream)      # in the caller's order, like an eager step
+                leave_open()
         for seq_id in end:
             self.cache.release(seq_id)
         return (self._out if ctx.n_want else None), ctx.n_want
@@ -291,7 +294,7 @@ class LayeredCausalModel:
         self.cache.release(seq_id)
 
     def residual_rows(self, n: int) -> np.ndarray:
-        """The first n rows of the residual stream as the last step left them (debugging aid)."""
+        """The first n rows of the residual stream as the last step left them (debugging aid; read on the stream of that step)."""
         return self._buf.x.to_numpy()[:n].copy()
 
     # ------------------------------------------------------------------ generation

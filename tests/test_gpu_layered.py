@@ -558,3 +558,29 @@ def test_steps_do_not_wait_and_keep_their_order():
         with CudaGraph().capture(s1):
             m.step_device([("new", [1, 2, 3], [0])])
     api.device_sync()
+
+
+def test_decode_steps_are_complete_for_other_streams():
+    """Logits and residual rows of a replayed decode step, read behind the `use_stream` block that ran it (or inside one that did not), are
+    those of a step that is waited for."""
+    from pygpukit_b200.core.stream import Stream, use_stream
+
+    def run(side, read):
+        cfg, _, m = make("mixed_stack")
+        p = tokens(cfg, 64, seed=4)
+        with use_stream(side):
+            m.step([(0, p, [])])
+            for i in range(3):                           # eager, captured, replayed
+                m.step([(0, [i], [0])])
+        kept = []
+        for i in range(12):
+            with use_stream(side):
+                out, _ = m.step_device([(0, [i], [0])])
+            with use_stream(read):
+                kept += [out.to_numpy()[:1].copy(), m.residual_rows(1)]
+        return kept
+
+    s = Stream()
+    want = run(None, None)
+    for side, read in ((s, None), (None, s), (s, s), (s, Stream())):
+        assert all(np.array_equal(x, y) for x, y in zip(want, run(side, read)))

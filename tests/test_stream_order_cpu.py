@@ -72,3 +72,54 @@ def test_a_recorded_step_neither_waits_nor_counts(model):
     assert calls(m) == []
     m._embed([1], 1, 0, m._buffers)
     assert calls(m) == ["upload", "embed"]
+
+
+def test_work_left_open_is_waited_for_when_the_stream_changes(monkeypatch):
+    """A replayed decode step is not waited for on its own stream, and complete for everyone else: a change of the current stream, in
+    either direction, and a capture wait for it -- once, and not where nothing was left open."""
+    log = []
+
+    class Api:
+        def __getattr__(self, name):
+            return lambda *a: log.append((name, *a[:1]))
+
+    monkeypatch.setattr(streams, "api", Api())
+    s, t = SimpleNamespace(handle=object()), SimpleNamespace(handle=object())
+    with streams.use_stream(s):
+        pass
+    assert log == []
+    streams.leave_open()
+    with streams.use_stream(None):
+        assert log == []
+        with streams.use_stream(s):
+            assert log == [("stream_sync", None)]
+            streams.leave_open()
+            with streams.use_stream(s):
+                assert len(log) == 1
+            with streams.use_stream(t):
+                assert log[1:] == [("stream_sync", s.handle)]
+            streams.leave_open()
+        assert log[2:] == [("stream_sync", s.handle)]
+    assert len(log) == 3
+    with streams.use_stream(s):
+        streams.leave_open()
+        with streams.CudaGraph().capture(s):
+            assert log[3:] == [("stream_sync", s.handle), ("graph_begin", s.handle)]
+    assert log[5] == ("graph_end", s.handle)
+
+
+def test_a_wait_that_fails_leaves_the_right_stream_current(monkeypatch):
+    def fail(*a):
+        raise RuntimeError("ran out")
+
+    monkeypatch.setattr(streams, "api", SimpleNamespace(stream_sync=fail))
+    s = SimpleNamespace(handle=object())
+    streams.leave_open()
+    with pytest.raises(RuntimeError, match="ran out"):
+        with streams.use_stream(s):
+            raise AssertionError("not entered")
+    assert streams.current_stream_handle() is None
+    with pytest.raises(RuntimeError, match="ran out"):
+        with streams.use_stream(s):
+            streams.leave_open()
+    assert streams.current_stream_handle() is None and not streams._open
