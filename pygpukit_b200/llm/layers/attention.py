@@ -186,6 +186,12 @@ class Attention:
     def get_confirmed_pos(self) -> int:
         return self._confirmed_pos
 
+    @property
+    def serves_many_rows(self) -> bool:
+        """Portions of more than 64 rows have a kernel of their own (pgk_sdpa_decode: heads of 128, up to 128 query heads a KV head).  The
+        decode kernel, which serves all others, reads the whole context for every four rows and takes 16384 groups of four."""
+        return self.head_dim == 128 and self.num_kv_groups <= 128
+
     # ---- decode
     def attend(self, x: GPUArray, position: int, context_len: int, *, qkv_buf: GPUArray | None = None,
                attn_buf: GPUArray | None = None, pos_buf: GPUArray | None = None,

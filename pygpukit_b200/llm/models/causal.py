@@ -26,6 +26,7 @@ from ...core.factory import from_numpy
 from ...core.stream import CudaGraph, Stream, current_stream_handle as _st, is_capturing, use_stream
 from ..buffers import DecodeBuffers, PrefillBuffers
 from ..config import ModelSpec, TransformerConfig
+from ..layers.attention import Attention
 from ..layers.block import TransformerBlock
 from ..layers.linear import LinearFP8, can_fuse_norm
 from ..layers.mlp import MLP
@@ -265,12 +266,14 @@ class CausalTransformerModel:
     PROMPT_ROWS = 512                # tokens per portion: the products are near their rate, the buffers 30 ... 60 MB for 8B ... 70B models
 
     def _long_portions(self) -> bool:
-        """True when every layer serves portions of more than 64 rows on the tensor cores (FP8 projections, silu MLP without biases on
-        gate and up, one GPU); other prompts run in slabs of `max_batch_size` rows."""
+        """True when every layer serves portions of more than 64 rows on the tensor cores (FP8 projections, heads of 128, silu MLP without
+        biases on gate and up, one GPU); other prompts run in slabs of `max_batch_size` rows."""
         if self.tp > 1:
             return False
         for blk in self.blocks:
             if type(blk) is not TransformerBlock or blk.comm is not None or type(blk.mlp) is not MLP or not blk.mlp._fp8_pair():
+                return False
+            if type(blk.attn) is not Attention or not blk.attn.serves_many_rows:
                 return False
             lin = (blk.attn.qkv_proj, blk.attn.o_proj, blk.mlp.gate_proj, blk.mlp.up_proj, blk.mlp.down_proj)
             if not all(isinstance(p, LinearFP8) and p.uses_tensor_cores(65) for p in lin):

@@ -387,16 +387,20 @@ def test_multi_sequence_decode_matches_single_sequence_runs(name, fmt, S):
         assert same >= 8, f"sequence {s}: only {same} identical tokens"
 
 
-@pytest.mark.parametrize("n", [17, 65, 130, 600])
-def test_long_prompt_portions_equal_slabs(n, monkeypatch):
-    """A prompt in portions of up to 512 rows and the same in slabs of 16: the hidden rows that come back are the last slab's (same count),
-    the caches and hidden rows agree within BF16 sums in another order, and decoding goes on from either."""
-    model = llm.build_random_model("tiny-qwen3", "fp8", max_seq=640, seed=7, std=0.05)
+@pytest.mark.parametrize("name,n", [("tiny-qwen3", 17), ("tiny-qwen3", 65), ("tiny-qwen3", 130), ("tiny-qwen3", 600), ("small-llama", 600)])
+def test_long_prompt_portions_equal_slabs(name, n, monkeypatch):
+    """A prompt in portions of up to 512 rows (heads of 128; heads of 64 have none) and the same in slabs of 16: the hidden rows that come
+    back are the last slab's (same count), the caches and hidden rows agree within BF16 sums in another order."""
+    model = llm.build_random_model(name, "fp8", max_seq=640, seed=7, std=0.05)
+    portions = []
+    prompt_rows = type(model)._prompt
+    monkeypatch.setattr(type(model), "_prompt", lambda self, ids, start: portions.append(prompt_rows(self, ids, start)) or portions[-1])
     rng = np.random.default_rng(n)
     prompt = [int(t) for t in rng.integers(0, model.config.vocab_size, n)]
     model.init_decode(640, max_batch_size=16)
     a, past = model(prompt, use_cache=True)
     a, ka = f32(a.to_numpy()), [f32(k) for kv in model.snapshot_kv_cache() for k in kv]
+    assert len(portions) == (model.config.head_dim == 128) and None not in portions
     monkeypatch.setattr(type(model), "_long_portions", lambda self: False)
     model.init_decode(640, max_batch_size=16)
     b, past2 = model(prompt, use_cache=True)

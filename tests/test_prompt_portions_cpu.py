@@ -1,0 +1,37 @@
+"""Which prompts run in portions of 512 rows, and what a feed-forward calls: the Python side of the FP8 path, without a GPU."""
+import pytest
+
+from pygpukit_b200.core.array import GPUArray
+from pygpukit_b200.core.dtypes import bfloat16, uint8
+from pygpukit_b200.llm.config import TransformerConfig
+from pygpukit_b200.llm.layers import mlp as mlp_module
+from pygpukit_b200.llm.layers.attention import Attention
+from pygpukit_b200.llm.layers.block import TransformerBlock
+from pygpukit_b200.llm.layers.linear import LinearFP8
+from pygpukit_b200.llm.layers.mlp import MLP
+from pygpukit_b200.llm.models.causal import CausalTransformerModel
+
+
+def array(*shape, dtype=bfloat16):
+    return GPUArray(shape, dtype, ptr=256)               # never read
+
+
+def fp8(n, k):
+    return LinearFP8(array(n, k, dtype=uint8), array(-(-n // 128), -(-k // 128)))
+
+
+def model(heads, kv_heads, dim):
+    c = TransformerConfig(vocab_size=256, hidden_size=256, num_layers=1, num_heads=heads, num_kv_heads=kv_heads, intermediate_size=512, _head_dim=dim,
+                          norm_eps=1e-6, rope_theta=1e4, max_position_embeddings=64, tie_word_embeddings=False)
+    attn = Attention(None, None, None, fp8(256, heads * dim), c, qkv_proj=fp8((heads + 2 * kv_heads) * dim, 256))
+    mlp = MLP(c, gate_proj=fp8(512, 256), up_proj=fp8(512, 256), down_proj=fp8(256, 512))
+    m = object.__new__(CausalTransformerModel)
+    m.comm, m.blocks = None, [TransformerBlock(None, attn, None, mlp)]
+    return m
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,portions", [(4, 2, 128, True), (128, 1, 128, True), (256, 2, 128, True), (129, 1, 128, False), (4, 2, 64, False),
+                                                         (8, 4, 32, False), (2, 1, 256, False)])
+def test_long_portions_need_attention_for_many_rows(heads, kv_heads, dim, portions):
+    """Other heads keep their slabs: their kernel reads the context for every four rows and refuses more than 16384 groups of four."""
+    assert model(heads, kv_heads, dim)._long_portions() is portions
