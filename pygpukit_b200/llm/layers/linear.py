@@ -92,6 +92,11 @@ class LinearBF16:
 Linear = LinearBF16
 
 
+def raw_codes_asked() -> bool:
+    """PGK_TC_IMPL=2: batches of up to 64 rows multiply the FP8 codes themselves (pgk_gemv_fp8_bf16 reads the variable once)."""
+    return os.environ.get("PGK_TC_IMPL", "1").strip() == "2"
+
+
 class LinearFP8:
     """y = x dequant(W)^T + b; W = E4M3 codes [out, in] + bf16 scale_inv [out/128, in/128]
     (layers/linear.py:101-260)."""
@@ -126,8 +131,8 @@ class LinearFP8:
 
     def uses_tensor_cores(self, M: int) -> bool:
         """True when a batch of M rows is served by the tcgen05 GEMMs (pgk_gemm_fp8_bf16_tc; above 64 rows the kernel of
-        gemm_tc_rows.cu) instead of the CUDA-core GEMV: M >= TC_MIN_M and 128-aligned shapes."""
-        return (TC_MIN_M <= M <= 65536 and self.in_features % 128 == 0 and self.out_features % 128 == 0
+        gemm_tc_rows.cu) instead of the CUDA-core GEMV: M >= TC_MIN_M and 128-aligned shapes.  The kernel of PGK_TC_IMPL=2 ends at 64."""
+        return (TC_MIN_M <= M <= (64 if raw_codes_asked() else 65536) and self.in_features % 128 == 0 and self.out_features % 128 == 0
                 and os.environ.get("PGK_TC", "1") != "0")
 
     def _dequantize_cpu(self) -> np.ndarray:

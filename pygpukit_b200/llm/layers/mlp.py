@@ -18,7 +18,7 @@ from ...core.factory import from_numpy
 from ...core.stream import current_stream_handle as _st
 from ...ops.elementwise import mul
 from ...ops.nn import gelu, silu
-from .linear import LinearBF16, LinearFP8, LinearNVF4, can_fuse_norm
+from .linear import LinearBF16, LinearFP8, LinearNVF4, can_fuse_norm, raw_codes_asked
 
 if TYPE_CHECKING:
     from ..config import TransformerConfig
@@ -87,7 +87,8 @@ class MLP:
         M, K, I = x.shape[0], x.shape[1], self.intermediate_size
         if out is None:
             out = GPUArray((M, I), bfloat16)
-        if self._fp8_pair() and self.gate_proj.uses_tensor_cores(M) and self.up_proj.uses_tensor_cores(M):
+        if (self._fp8_pair() and self.gate_proj.uses_tensor_cores(M) and self.up_proj.uses_tensor_cores(M)
+                and not raw_codes_asked()):
             # from TC_MIN_M rows on: both products, silu and mul in one launch, with the layer path's roundings
             if norm is not None:
                 xs = self._scratch.get(("x", M))
@@ -100,7 +101,8 @@ class MLP:
             return out
         if (self.gate_up_proj is None and isinstance(self.gate_proj, LinearFP8) and isinstance(self.up_proj, LinearFP8)
                 and self.gate_proj.uses_tensor_cores(M) and self.up_proj.uses_tensor_cores(M)):
-            # products with a bias: gate and up one after the other, then silu -> mul with the layer path's two roundings
+            # products with a bias, or of the codes themselves: gate and up one after the other, then silu -> mul with the layer path's
+            # two roundings
             if norm is not None:
                 xs = self._scratch.get(("x", M))
                 if xs is None:

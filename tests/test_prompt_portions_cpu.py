@@ -35,3 +35,29 @@ def model(heads, kv_heads, dim):
 def test_long_portions_need_attention_for_many_rows(heads, kv_heads, dim, portions):
     """Other heads keep their slabs: their kernel reads the context for every four rows and refuses more than 16384 groups of four."""
     assert model(heads, kv_heads, dim)._long_portions() is portions
+
+
+class Calls(list):
+    def __getattr__(self, name):
+        return lambda *a: self.append(name)
+
+
+@pytest.mark.parametrize("impl,rows,products,fused", [(None, 16, 0, 1), ("1", 64, 0, 1), ("2", 16, 2, 0), ("2", 64, 2, 0), (None, 200, 0, 1), ("2", 200, 0, 1)])
+def test_the_other_product_serves_gate_and_up_too(monkeypatch, impl, rows, products, fused):
+    """PGK_TC_IMPL=2 selects the product of the codes themselves (up to 64 rows), which has no form for gate and up together; prompts keep
+    their slabs then."""
+    from pygpukit_b200.llm.layers import linear as linear_module
+    monkeypatch.delenv("PGK_TC_IMPL", raising=False)
+    if impl is not None:
+        monkeypatch.setenv("PGK_TC_IMPL", impl)
+    m = model(4, 2, 128)
+    calls = Calls()
+    monkeypatch.setattr(mlp_module, "api", calls)
+    monkeypatch.setattr(linear_module, "api", calls)
+    monkeypatch.setattr(mlp_module, "silu", lambda x, out: out)
+    monkeypatch.setattr(mlp_module, "mul", lambda x, y, out: out)
+    mlp = m.blocks[0].mlp
+    mlp._scratch[rows] = (array(rows, 512), array(rows, 512))
+    mlp.gate_up_act(array(rows, 256), out=array(rows, 512))
+    assert (calls.count("gemv_fp8_bf16_ex"), calls.count("gemv_fp8_swiglu_bf16")) == (products, fused)
+    assert m._long_portions() is (impl != "2")
