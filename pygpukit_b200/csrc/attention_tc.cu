@@ -8,7 +8,9 @@
 //   * A operands sit in tensor memory, where an MMA of 128 columns takes 77 cycles (110 with A in shared memory): the queries all along,
 //     the weights written there by the warps that form them, which also saves their way through shared memory;
 //   * a weight is float32: three BF16 terms, cut off and not rounded, that together hold its 24 bits, enter the product one after the
-//     other.  None of a weight's terms is zero (2^-126 stands in), so that an infinite value gives infinity, as in float32;
+//     other.  The second and third are never zero (2^-126 stands in), so that an infinite value gives infinity, as in float32;
+//   * a masked key's weight is zero, and zero times an infinite or NaN value is NaN: rows that came out NaN in a range with keys behind
+//     their own last one are summed again over their own keys, in float32 on the ordinary units;
 //   * the scores of tile i + 1 are multiplied while tile i's weights are formed; the first two terms lie where its scores were;
 //   * eight warps, a lane a row, two warps a row (64 keys each); a row's reference moves only when its maximum has grown by LAZY (log2
 //     units): the outputs in tensor memory are rescaled then;
@@ -36,7 +38,8 @@ constexpr uint32_t M_O = 0, M_Q = 128, M_S = 192, M_LO = 448;      // TMEM colum
 constexpr float M_LAZY = 8.f;
 
 struct PromptAttnParams {
-    const uint16_t* Q; uint16_t* out;
+    const uint16_t* Q; const uint16_t* K; const uint16_t* V; uint16_t* out;
+    int max_seq;
     long q_sh, q_st, o_sh, o_st;
     int hq, n_kv, q_len, context_len;
     int HB, QB, hsplit, splits;
@@ -56,6 +59,35 @@ __device__ __forceinline__ bool all_wait(int* err, uint32_t bar, uint32_t parity
 }
 // the upper halves of two words: two float32 values cut off to BF16
 __device__ __forceinline__ uint32_t cut2(float lo, float hi) { return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632); }
+
+// 16 elements of one row's sum over keys [from, to), by a warp: q, k and v are the row's query and the first rows of its keys and values
+__device__ __forceinline__ void sum_again(const uint16_t* q, const uint16_t* k, const uint16_t* v, int from, int to, float scale_log2, float neg, float (&o)[16]) {
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[e] = 0.f;
+#pragma unroll 1
+    for (int j = from + (int)(threadIdx.x & 31); j < to; j += 32) {
+        float s = 0.f;
+#pragma unroll 1
+        for (int i = 0; i < M_D; i += 8) {
+            const uint4 a = ld_act16(q + i), b = ld_act16(k + (size_t)j * M_D + i);
+            s = fmaf(bf16lo(a.x), bf16lo(b.x), s); s = fmaf(bf16hi(a.x), bf16hi(b.x), s);
+            s = fmaf(bf16lo(a.y), bf16lo(b.y), s); s = fmaf(bf16hi(a.y), bf16hi(b.y), s);
+            s = fmaf(bf16lo(a.z), bf16lo(b.z), s); s = fmaf(bf16hi(a.z), bf16hi(b.z), s);
+            s = fmaf(bf16lo(a.w), bf16lo(b.w), s); s = fmaf(bf16hi(a.w), bf16hi(b.w), s);
+        }
+        const float w = ex2f(fmaf(s, scale_log2, neg));
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const uint4 x = ld_act16(v + (size_t)j * M_D + 8 * i);
+            o[8 * i] = fmaf(w, bf16lo(x.x), o[8 * i]); o[8 * i + 1] = fmaf(w, bf16hi(x.x), o[8 * i + 1]);
+            o[8 * i + 2] = fmaf(w, bf16lo(x.y), o[8 * i + 2]); o[8 * i + 3] = fmaf(w, bf16hi(x.y), o[8 * i + 3]);
+            o[8 * i + 4] = fmaf(w, bf16lo(x.z), o[8 * i + 4]); o[8 * i + 5] = fmaf(w, bf16hi(x.z), o[8 * i + 5]);
+            o[8 * i + 6] = fmaf(w, bf16lo(x.w), o[8 * i + 6]); o[8 * i + 7] = fmaf(w, bf16hi(x.w), o[8 * i + 7]);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 16; ++e) o[e] = warp_sum(o[e]);
+}
 
 __global__ void __launch_bounds__(M_THREADS, 1)
 sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_constant__ CUtensorMap vmap, const __grid_constant__ PromptAttnParams p) {
@@ -275,6 +307,8 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         const float inv = p.splits > 1 ? 1.f : (l > 0.f || l != l ? 1.f / l : 0.f);
         float* rec = p.splits > 1 ? p.ws + (((size_t)t * p.hq + h) * p.splits + blockIdx.z) * (M_D + 4) : nullptr;
         if (rec && live && half == 0) { rec[0] = m; rec[1] = l; }
+        const int from = tbeg * M_KEYS, end = min(p.context_len, (tbeg + n) * M_KEYS);
+        const size_t kv = (size_t)g * p.max_seq * M_D;
 #pragma unroll 1
         for (int c = 0; c < 64; c += 16) {
             float o[16];
@@ -283,6 +317,20 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
             else {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) o[e] = 0.f;
+            }
+            bool none = false;
+#pragma unroll
+            for (int e = 0; e < 16; ++e) none |= o[e] != o[e];
+            uint32_t rows = __ballot_sync(0xffffffffu, live && none && limit + 1 < end);
+#pragma unroll 1
+            while (rows) {
+                const int s = __ffs(rows) - 1, r = quad * 32 + s, sh = r / p.QB, sq = r - sh * p.QB;
+                rows &= rows - 1;
+                float x[16];
+                sum_again(p.Q + (size_t)(g * rep + h0 + sh) * p.q_sh + (size_t)(q0 + sq) * p.q_st, p.K + kv, p.V + kv + half * 64 + c, from, pos0 + sq + 1,
+                          p.scale_log2, __shfl_sync(0xffffffffu, neg, s), x);
+#pragma unroll
+                for (int e = 0; e < 16; ++e) o[e] = lane == s ? x[e] : o[e];
             }
             if (live && rec) {
 #pragma unroll
@@ -345,7 +393,8 @@ int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, 
         configured = true;
     }
     PromptAttnParams p = {};
-    p.Q = (const uint16_t*)Q; p.out = (uint16_t*)out;
+    p.Q = (const uint16_t*)Q; p.K = (const uint16_t*)K; p.V = (const uint16_t*)V; p.out = (uint16_t*)out;
+    p.max_seq = max_seq;
     p.q_sh = q_sh; p.q_st = q_st; p.o_sh = o_sh; p.o_st = o_st;
     p.hq = hq; p.n_kv = n_kv; p.q_len = q_len; p.context_len = context_len;
     p.scale_log2 = scale_log2;

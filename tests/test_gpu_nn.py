@@ -550,19 +550,21 @@ def test_rope_sdpa_decode_infinite_value_rows(ctx):
                                                (260, 515, 8, 8), (40, 3000, 16, 4), (20, 9000, 4, 1)])
 def test_prompt_attention_on_tensor_cores_against_float64(q_len, ctx, hq, n_kv):
     """Many query rows over the fixed cache: rows that do not fill a block, ragged groups, key ranges (in records and beyond 64 tiles), the edges
-    of key tiles, an infinite value that the first rows do not see, rows behind the context that hold NaN.  Scores are float32 sums of
-    128 exact products and weights float32, so beside the output's rounding (2^-8) only a few 1e-6 of the largest value can be off."""
+    of key tiles, an infinite value and a NaN that the first rows do not see, rows behind the context that hold NaN.  Scores are float32 sums
+    of 128 exact products and weights float32, so beside the output's rounding (2^-8) only a few 1e-6 of the largest value can be off."""
     rng = np.random.default_rng(q_len + ctx)
     max_seq, width = ctx + 5, (hq + 2 * n_kv) * 128
     qkv, K, V = rand_bf16(rng, (q_len, width)), rand_bf16(rng, (n_kv, max_seq, 128)), rand_bf16(rng, (n_kv, max_seq, 128))
     K[:, ctx:], V[:, ctx:] = 0x7FC0, 0x7FC0
     V[0, ctx - 1, 7] = 0x7F80                                # the last key: only the last query sees it
+    sees = ctx - q_len + np.arange(q_len) >= ctx - q_len // 2
+    V[0, ctx - q_len // 2, 70] = 0x7FC0
     gq, gk_, gv, out = gk.from_numpy(qkv), gk.from_numpy(K), gk.from_numpy(V), gk.zeros((q_len, hq * 128), gk.bfloat16)
     api.sdpa_decode(gq.device_ptr, gk_.device_ptr, gv.device_ptr, out.device_ptr, hq, n_kv, q_len, 128, max_seq, ctx, None, 0.0, 128, width, 128, hq * 128, 2,
                     None)
     got = f32(out.to_numpy()).astype(np.float64).reshape(q_len, hq, 128)
     rep = hq // n_kv
-    assert np.isposinf(got[-1, :rep, 7]).all()
+    assert np.isposinf(got[-1, :rep, 7]).all() and np.isnan(got[sees][:, :rep, 70]).all()
     q = f32(qkv).astype(np.float64)[:, :hq * 128].reshape(q_len, hq, 128)
     for h in range(hq):
         g = h // rep
@@ -570,10 +572,10 @@ def test_prompt_attention_on_tensor_cores_against_float64(q_len, ctx, hq, n_kv):
         s = q[:, h] @ k.T / np.sqrt(128.0)
         s[np.arange(ctx)[None, :] > ctx - q_len + np.arange(q_len)[:, None]] = -np.inf
         p = np.exp(s - s.max(-1, keepdims=True))
-        if g == 0:                                           # masked weights times the infinite value: its column is looked at above only
-            v[ctx - 1, 7] = 0.0
+        if g == 0:                                           # rows that see them are looked at above
+            v[ctx - 1, 7] = v[ctx - q_len // 2, 70] = 0.0
         ref = p @ v / p.sum(-1, keepdims=True)
         d = np.abs(got[:, h] - ref) - (2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(v).max())
         if g == 0:
-            d[:, 7] = 0.0
+            d[-1, 7] = d[sees, 70] = 0.0
         assert (d <= 0).all()
