@@ -351,7 +351,8 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
     if (warp == M_SOFT + 1) tmem_dealloc(tmem, 512);
 }
 
-// a warp per (query, head): the records of its key ranges in their order
+// a warp per (query, head): the records of its key ranges in their order.  A range in which the row sees no key has m = -inf and l = 0; one
+// whose scores are all NaN has m = -inf and l = NaN, and the row becomes NaN as it does in one range.
 __global__ void __launch_bounds__(256) sdpa_prompt_fold_kernel(const __grid_constant__ PromptAttnParams p) {
     griddep_wait();
     griddep_launch();
@@ -364,10 +365,9 @@ __global__ void __launch_bounds__(256) sdpa_prompt_fold_kernel(const __grid_cons
     float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int s = 0; s < p.splits; ++s) {
         const float* r = rec + s * (M_D + 4);
-        const float m = __ldcg(r), w = m == -INFINITY ? 0.f : exp2f(m - M);
-        if (w == 0.f) continue;
+        const float m = __ldcg(r), l = __ldcg(r + 1), w = m == -INFINITY ? l - l : exp2f(m - M);
         const float4 v = __ldcg((const float4*)(r + 4 + lane * 4));
-        L = fmaf(w, __ldcg(r + 1), L);
+        L = fmaf(w, l, L);
         o.x = fmaf(w, v.x, o.x); o.y = fmaf(w, v.y, o.y); o.z = fmaf(w, v.z, o.z); o.w = fmaf(w, v.w, o.w);
     }
     const float inv = L > 0.f || L != L ? 1.f / L : 0.f;

@@ -579,3 +579,25 @@ def test_prompt_attention_on_tensor_cores_against_float64(q_len, ctx, hq, n_kv):
         if g == 0:
             d[-1, 7] = d[sees, 70] = 0.0
         assert (d <= 0).all()
+
+
+@pytest.mark.parametrize("q_len,ctx,hq,n_kv", [(16, 40, 2, 2), (32, 600, 4, 2), (20, 9000, 4, 1), (300, 2600, 2, 1)])
+def test_prompt_attention_of_nan_queries_and_keys(q_len, ctx, hq, n_kv):
+    """A query of NaN, and a query that sees a key of NaN, give NaN however many key ranges there are; all other rows keep their values."""
+    rng = np.random.default_rng(q_len + ctx)
+    width = (hq + 2 * n_kv) * 128
+    qkv, K, V = rand_bf16(rng, (q_len, width)), rand_bf16(rng, (n_kv, ctx, 128)), rand_bf16(rng, (n_kv, ctx, 128))
+
+    def run():
+        out, a = gk.zeros((q_len, hq * 128), gk.bfloat16), [gk.from_numpy(x) for x in (qkv, K, V)]
+        api.sdpa_decode(*(x.device_ptr for x in a), out.device_ptr, hq, n_kv, q_len, 128, ctx, ctx, None, 0.0, 128, width, 128, hq * 128, 2, None)
+        return f32(out.to_numpy()).reshape(q_len, hq, 128)
+
+    clean = run()
+    assert np.isfinite(clean).all()
+    qkv[3, 128:256] = 0x7FC0                                 # head 1 of query 3
+    K[0, ctx - 5, 11] = 0x7FC0                               # the last five queries see it
+    got, nan = run(), np.zeros((q_len, hq), bool)
+    nan[3, 1], nan[q_len - 5:, :hq // n_kv] = True, True
+    assert np.isnan(got[nan]).all()
+    assert np.array_equal(got[~nan], clean[~nan])
