@@ -265,6 +265,9 @@ int pgk_sdpa_decode(const void* Q, const void* K, const void* V, void* out, int 
                     int n_kv, int q_len, int head_dim, int max_seq, int context_len,
                     const int32_t* ctx_buf, float scale, long q_stride_h, long q_stride_t,
                     long o_stride_h, long o_stride_t, int dtype, void* stream);
+/* plan[3]: queries of a block, key ranges and queries of a launch that pgk_sdpa_decode takes for many query rows on a device of `sms` SMs
+ * (BF16, heads of 128; reads no device) */
+int pgk_sdpa_prompt_plan(int n_heads_q, int n_kv, int q_len, int context_len, int sms, int32_t* plan);
 /* The whole decode attention bracket of ONE new token in one launch (bf16, head_dim 128): per-head
  * QK-RMSNorm (gamma NULL = off) -> RoPE at *pos_buf (or pos) from f32 tables -> K/V row written into the
  * un-expanded cache -> split-KV attention over the first *ctx_buf (or context_len) positions, new row

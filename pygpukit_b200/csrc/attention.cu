@@ -32,7 +32,7 @@ namespace pgk {
 bool sdpa_prompt_ok(const void* Q, const void* K, const void* V, const void* out, int hq, int n_kv, int q_len, int max_seq, int context_len, long q_sh, long q_st,
                     long o_sh, long o_st);
 int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, int n_kv, int q_len, int max_seq, int context_len, float scale_log2, long q_sh,
-                long q_st, long o_sh, long o_st, cudaStream_t st);
+                long q_st, long o_sh, long o_st, cudaStream_t st, bool* no_room);
 // From 16 queries over 32 keys on (us, here / there, 32 / 8 heads: 16 over 16 8.0 / 10.3, 20 over 100 12.6 / 10.4, 64 over 64 16.6 / 10.4); fewer rows
 // leave most of a block of 128 empty.
 constexpr int kPromptRows = 16, kPromptKeys = 32;
@@ -991,9 +991,12 @@ int pgk_sdpa_decode(const void* Q, const void* K, const void* V, void* out, int 
     PGK_REQUIRE(((uintptr_t)K % 16 == 0) && ((uintptr_t)V % 16 == 0), "sdpa_causal_fixed_cache failed: K/V must be 16-byte aligned");
     if (scale <= 0.f) scale = 1.0f / sqrtf((float)head_dim);   // sdpa_causal.inl:464-467
     if (dtype == 2 && head_dim == 128 && !ctx_buf && q_len >= kPromptRows && context_len >= kPromptKeys &&
-        sdpa_prompt_ok(Q, K, V, out, n_heads_q, n_kv, q_len, max_seq, context_len, q_stride_h, q_stride_t, o_stride_h, o_stride_t))
-        return sdpa_prompt(Q, K, V, out, n_heads_q, n_kv, q_len, max_seq, context_len, scale * 1.4426950408889634f, q_stride_h, q_stride_t, o_stride_h,
-                           o_stride_t, (cudaStream_t)stream);
+        sdpa_prompt_ok(Q, K, V, out, n_heads_q, n_kv, q_len, max_seq, context_len, q_stride_h, q_stride_t, o_stride_h, o_stride_t)) {
+        bool no_room = false;
+        const int rc = sdpa_prompt(Q, K, V, out, n_heads_q, n_kv, q_len, max_seq, context_len, scale * 1.4426950408889634f, q_stride_h, q_stride_t, o_stride_h,
+                                   o_stride_t, (cudaStream_t)stream, &no_room);
+        if (!no_room) return rc;
+    }
     SdpaParams p = {};
     p.Q = Q; p.K = K; p.V = V; p.out = out;
     p.hq = n_heads_q; p.n_kv = n_kv; p.q_len = q_len; p.max_seq = max_seq; p.context_len = context_len;

@@ -43,8 +43,9 @@ struct PromptAttnParams {
     long q_sh, q_st, o_sh, o_st;
     int hq, n_kv, q_len, context_len;
     int HB, QB, hsplit, splits;
+    int t0, t1;                                    // the launch's queries
     float scale_log2;
-    float* ws;                                     // splits > 1: records (m, l, -, -, o[128]) [query][head][split]
+    float* ws;                                     // splits > 1: records (m, l, -, -, o[128]) [query - t0][head][split]
     int* err;
 };
 
@@ -116,7 +117,7 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
     griddep_launch();
 
     const int rep = p.hq / p.n_kv, g = blockIdx.y / p.hsplit, part = blockIdx.y - g * p.hsplit, h0 = part * p.HB, nh = min(p.HB, rep - h0);
-    const int q0 = (int)(gridDim.x - 1 - blockIdx.x) * p.QB, nq = min(p.QB, p.q_len - q0), pos0 = p.context_len - p.q_len + q0;
+    const int q0 = p.t0 + (int)(gridDim.x - 1 - blockIdx.x) * p.QB, nq = min(p.QB, p.t1 - q0), pos0 = p.context_len - p.q_len + q0;
     const int ntile = (pos0 + nq - 1) / M_KEYS + 1, per = (ntile + p.splits - 1) / p.splits;
     const int tbeg = (int)blockIdx.z * per, n = max(0, min(ntile, tbeg + per) - tbeg);
     // row r: head r / QB, query r % QB
@@ -305,7 +306,7 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
         l = wmax[0][0][row] + wmax[0][1][row];
         const int h = g * rep + h0 + rh, t = q0 + rq;
         const float inv = p.splits > 1 ? 1.f : (l > 0.f || l != l ? 1.f / l : 0.f);
-        float* rec = p.splits > 1 ? p.ws + (((size_t)t * p.hq + h) * p.splits + blockIdx.z) * (M_D + 4) : nullptr;
+        float* rec = p.splits > 1 ? p.ws + (((size_t)(t - p.t0) * p.hq + h) * p.splits + blockIdx.z) * (M_D + 4) : nullptr;
         if (rec && live && half == 0) { rec[0] = m; rec[1] = l; }
         const int from = tbeg * M_KEYS, end = min(p.context_len, (tbeg + n) * M_KEYS);
         const size_t kv = (size_t)g * p.max_seq * M_D;
@@ -357,8 +358,8 @@ __global__ void __launch_bounds__(256) sdpa_prompt_fold_kernel(const __grid_cons
     griddep_wait();
     griddep_launch();
     const int lane = threadIdx.x & 31, i = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (i >= p.q_len * p.hq) return;
-    const int t = i / p.hq, h = i - t * p.hq;
+    if (i >= (p.t1 - p.t0) * p.hq) return;
+    const int t = p.t0 + i / p.hq, h = i % p.hq;
     const float* rec = p.ws + (size_t)i * p.splits * (M_D + 4);
     float M = -INFINITY, L = 0.f;
     for (int s = 0; s < p.splits; ++s) M = fmaxf(M, __ldcg(rec + s * (M_D + 4)));
@@ -385,8 +386,36 @@ bool sdpa_prompt_ok(const void* Q, const void* K, const void* V, const void* out
            hq / n_kv <= 128 && tma_encode_fn() != nullptr;
 }
 
+struct PromptPlan { int HB, QB, hsplit, splits, ranges, rows; };       // ranges: the fewest splits that the sums allow
+
+// Key ranges until the blocks fill the SMs, four tiles (a record costs what half a tile does) at least in each and 64 at most: a range's
+// sums stay in the tensor cores' accumulators, which cut off (over 32768 keys in one range the error against float64 was 1.665e-3, in
+// ranges of 8192 it is that of the float32 kernel, 1.661e-3: BF16 outputs).  Records take up to kRecordBytes (512 queries of 64 heads over
+// 131072 keys would have 277 MB); more queries go one launch after the other, each with blocks for all SMs.
+constexpr size_t kRecordBytes = 64ull << 20;
+static PromptPlan prompt_plan(int hq, int n_kv, int q_len, int context_len, int sms) {
+    PromptPlan p;
+    const int rep = hq / n_kv;
+    p.HB = rep < 16 ? rep : 16;
+    p.QB = M_ROWS / p.HB;
+    p.hsplit = (rep + p.HB - 1) / p.HB;
+    const long long blocks = (long long)((q_len + p.QB - 1) / p.QB) * n_kv * p.hsplit;
+    const int ntile = (context_len + M_KEYS - 1) / M_KEYS;
+    p.splits = (int)(sms / blocks);
+    if (p.splits > ntile / 4) p.splits = ntile / 4;
+    p.ranges = (ntile + 63) / 64;
+    if (p.splits < p.ranges) p.splits = p.ranges;
+    p.rows = q_len;
+    if (p.splits > 1) {
+        const size_t fit = kRecordBytes / ((size_t)hq * p.splits * (M_D + 4) * sizeof(float)) / p.QB * p.QB;
+        if (fit < (size_t)q_len) p.rows = fit > (size_t)p.QB ? (int)fit : (p.QB < q_len ? p.QB : q_len);
+    }
+    return p;
+}
+
+// `no_room`: nothing was done, the records of the ranges that the sums need do not fit the device
 int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, int n_kv, int q_len, int max_seq, int context_len, float scale_log2, long q_sh,
-                long q_st, long o_sh, long o_st, cudaStream_t st) {
+                long q_st, long o_sh, long o_st, cudaStream_t st, bool* no_room) {
     static bool configured = false;
     if (!configured) {
         PGK_CUDA(cudaFuncSetAttribute(sdpa_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)M_SMEM));
@@ -398,39 +427,47 @@ int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, 
     p.q_sh = q_sh; p.q_st = q_st; p.o_sh = o_sh; p.o_st = o_st;
     p.hq = hq; p.n_kv = n_kv; p.q_len = q_len; p.context_len = context_len;
     p.scale_log2 = scale_log2;
-    const int rep = hq / n_kv;
-    p.HB = rep < 16 ? rep : 16;
-    p.QB = M_ROWS / p.HB;
-    p.hsplit = (rep + p.HB - 1) / p.HB;
+    const PromptPlan plan = prompt_plan(hq, n_kv, q_len, context_len, sm_count());
+    p.HB = plan.HB; p.QB = plan.QB; p.hsplit = plan.hsplit; p.splits = plan.splits;
     p.err = wait_word(kWaitAttention);
     PGK_REQUIRE(p.err, "sdpa_causal_fixed_cache failed: no pinned host memory");
-    // key ranges until the blocks fill the SMs, four tiles (a record costs what half a tile does) at least in each and 64 at most: a range's
-    // sums stay in the tensor cores' accumulators, which cut off (over 32768 keys in one range the error against float64 was 1.665e-3, in
-    // ranges of 8192 it is that of the float32 kernel, 1.661e-3: BF16 outputs)
-    const int qtiles = (q_len + p.QB - 1) / p.QB, blocks = qtiles * n_kv * p.hsplit, ntile = (context_len + M_KEYS - 1) / M_KEYS;
-    p.splits = sm_count() / blocks;
-    if (p.splits > ntile / 4) p.splits = ntile / 4;
-    if (p.splits < (ntile + 63) / 64) p.splits = (ntile + 63) / 64;
     CUtensorMap kmap, vmap;
     const uint64_t dims[3] = {M_D, (uint64_t)context_len, (uint64_t)n_kv}, strides[2] = {M_D * 2, (uint64_t)max_seq * M_D * 2};
     const uint32_t box[3] = {64, M_KEYS, 1};
     PGK_REQUIRE(tma_map_bf16_3d(&kmap, K, dims, strides, box) && tma_map_bf16_3d(&vmap, V, dims, strides, box),
                 "sdpa_causal_fixed_cache failed: cuTensorMapEncodeTiled refused the operands");
+    int rows = plan.rows;
     if (p.splits > 1) {
         void* ws = nullptr;
-        if (scratch_alloc(&ws, (size_t)q_len * hq * p.splits * (M_D + 4) * sizeof(float), st)) {
-            set_error("");                                // no room for the records: one range
-            p.splits = 1;
-        }
+        const int rc = scratch_alloc(&ws, (size_t)rows * hq * p.splits * (M_D + 4) * sizeof(float), st);
+        if (rc == (int)cudaErrorMemoryAllocation) {
+            set_error("");
+            if (plan.ranges > 1) { *no_room = true; return 0; }
+            p.splits = 1;                                 // the ranges were to fill the SMs only
+            rows = q_len;
+        } else if (rc)
+            return rc;
         p.ws = (float*)ws;
     }
-    cudaError_t e = launch_waiting(sdpa_prompt_kernel, dim3(qtiles, n_kv * p.hsplit, p.splits), dim3(M_THREADS), M_SMEM, st, kmap, vmap, p);
-    if (p.splits > 1) {
-        if (e == cudaSuccess) e = launch_waiting(sdpa_prompt_fold_kernel, dim3((q_len * hq + 7) / 8), dim3(256), 0, st, p);
-        if (int rc = scratch_free(p.ws, st)) return rc;
+    cudaError_t e = cudaSuccess;
+    for (int t = 0; e == cudaSuccess && t < q_len; t += rows) {
+        p.t0 = t;
+        p.t1 = t + rows < q_len ? t + rows : q_len;
+        e = launch_waiting(sdpa_prompt_kernel, dim3((p.t1 - t + p.QB - 1) / p.QB, n_kv * p.hsplit, p.splits), dim3(M_THREADS), M_SMEM, st, kmap, vmap, p);
+        if (e == cudaSuccess && p.splits > 1)
+            e = launch_waiting(sdpa_prompt_fold_kernel, dim3(((p.t1 - t) * hq + 7) / 8), dim3(256), 0, st, p);
     }
+    if (int rc = scratch_free(p.ws, st)) return rc;
     PGK_CUDA(e);
     return 0;
 }
 
 }  // namespace pgk
+
+extern "C" int pgk_sdpa_prompt_plan(int n_heads_q, int n_kv, int q_len, int context_len, int sms, int32_t* plan) {
+    PGK_REQUIRE(n_kv > 0 && n_heads_q % n_kv == 0 && n_heads_q / n_kv > 0 && n_heads_q / n_kv <= 128 && q_len > 0 && context_len >= q_len && sms > 0,
+                "sdpa_prompt_plan failed: %d / %d heads, %d queries over %d keys", n_heads_q, n_kv, q_len, context_len);
+    const pgk::PromptPlan p = pgk::prompt_plan(n_heads_q, n_kv, q_len, context_len, sms);
+    plan[0] = p.QB; plan[1] = p.splits; plan[2] = p.rows;
+    return 0;
+}

@@ -2,6 +2,8 @@
 oracle and the reference's own CUDA kernels.  Tolerances: bit-exact for copies and index work,
 <= 1 bf16 ulp for elementwise f32 math (fast-math exp/rsqrt in the reference build),
 1e-2 relative for attention (north_star, BF16)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -601,3 +603,58 @@ def test_prompt_attention_of_nan_queries_and_keys(q_len, ctx, hq, n_kv):
     nan[3, 1], nan[q_len - 5:, :hq // n_kv] = True, True
     assert np.isnan(got[nan]).all()
     assert np.array_equal(got[~nan], clean[~nan])
+
+
+def test_prompt_attention_in_several_launches_against_float64():
+    """Queries whose records exceed what one launch may have go one launch after the other: rows on both sides of the cut."""
+    q_len, ctx, hq, n_kv = 400, 17000, 128, 8
+    plan = (C.c_int32 * 3)()
+    api.sdpa_prompt_plan(hq, n_kv, q_len, ctx, 148, plan)
+    assert plan[1] == 3 and 0 < plan[2] < q_len
+    rng = np.random.default_rng(1)
+    q, K, V = rand_bf16(rng, (q_len, hq * 128)), rand_bf16(rng, (n_kv, ctx, 128)), rand_bf16(rng, (n_kv, ctx, 128))
+    out, a = gk.zeros((q_len, hq * 128), gk.bfloat16), [gk.from_numpy(x) for x in (q, K, V)]
+    api.sdpa_decode(*(x.device_ptr for x in a), out.device_ptr, hq, n_kv, q_len, 128, ctx, ctx, None, 0.0, 128, hq * 128, 128, hq * 128, 2, None)
+    got = f32(out.to_numpy()).reshape(q_len, hq, 128)
+    assert np.isfinite(got).all()
+    rows = np.array([0, 1, plan[2] - 1, plan[2], plan[2] + 1, q_len - 1])
+    qf = f32(q).astype(np.float64).reshape(q_len, hq, 128)
+    for h in (0, 77, 127):
+        k, v = f32(K[h // 16]).astype(np.float64), f32(V[h // 16]).astype(np.float64)
+        s = qf[rows, h] @ k.T / np.sqrt(128.0)
+        s[np.arange(ctx)[None] > ctx - q_len + rows[:, None]] = -np.inf
+        p = np.exp(s - s.max(-1, keepdims=True))
+        ref = p @ v / p.sum(-1, keepdims=True)
+        assert (np.abs(got[rows, h] - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5 * np.abs(v).max()).all()
+
+
+@pytest.mark.parametrize("q_len,ctx", [(20, 4000), (20, 9000)])
+def test_prompt_attention_without_room_for_records(q_len, ctx):
+    """A full device: ranges that were to fill the SMs become one, and where the sums need ranges the kernel of few rows serves the call."""
+    hq, n_kv = 4, 1
+    rng = np.random.default_rng(ctx)
+    a = [gk.from_numpy(rand_bf16(rng, s)) for s in ((q_len, hq * 128), (n_kv, ctx, 128), (n_kv, ctx, 128))]
+
+    def run(rows, out):
+        before = api.launch_count()
+        api.sdpa_decode(*(x.device_ptr for x in a), out.device_ptr, hq, n_kv, rows, 128, ctx, ctx, None, 0.0, 128, hq * 128, 128, hq * 128, 2, None)
+        return api.launch_count() - before
+
+    want, got = (gk.zeros((q_len, hq * 128), gk.bfloat16) for _ in range(2))
+    assert run(8, want) == 1                                 # the other kernel and its memory
+    assert run(q_len, want) == 2
+    api.device_sync()
+    full, size = [], 1 << 36
+    while size >= 1 << 20:
+        try:
+            full.append(gk.empty((size,), gk.uint8))
+        except RuntimeError:
+            size //= 2
+    try:
+        assert run(q_len, got) == 1
+        x = f32(got.to_numpy())
+    finally:
+        full.clear()
+    ref = f32(want.to_numpy())
+    assert (np.abs(x - ref) <= 2.0 ** -7 * np.abs(ref) + 1e-5).all()      # one step of BF16: float32 sums in another order, rounded
+    assert run(q_len, got) == 2
