@@ -240,6 +240,12 @@ def check(rc: int) -> None:
 class _Api:
     """lib.<fn>(...) with automatic error checking: `api.gemv_fp8_bf16(...)`."""
 
+    def mem_trim(self) -> None:
+        """Idle memory goes back to the device: that of Python objects, then the library's own."""
+        from .core import idle
+        idle.give_back()
+        check(load().pgk_mem_trim())
+
     def __getattr__(self, name: str):
         fn = getattr(load(), "pgk_" + name, None)
         if fn is None:

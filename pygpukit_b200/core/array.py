@@ -12,7 +12,7 @@ from typing import Any
 import numpy as np
 
 from .._lib import api
-from . import dtypes as _dt
+from . import dtypes as _dt, idle
 from .dtypes import DataType
 from .stream import current_stream_handle
 
@@ -26,7 +26,12 @@ class GPUArray:
         self._source_ref = source
         if ptr is None:
             h = C.c_void_p()
-            api.malloc(C.byref(h), max(1, self.nbytes))
+            try:
+                api.malloc(C.byref(h), max(1, self.nbytes))
+            except RuntimeError as e:
+                if not idle.out_of_memory(e) or not idle.give_back():
+                    raise
+                api.malloc(C.byref(h), max(1, self.nbytes))
             self._ptr = int(h.value)
             self._owner = True
         else:

@@ -20,6 +20,7 @@ import os
 import numpy as np
 
 from ..._lib import api
+from ...core import idle
 from ...core.array import GPUArray
 from ...core.dtypes import bfloat16, int32
 from ...core.factory import from_numpy
@@ -280,7 +281,7 @@ class CausalTransformerModel:
                 return False
         return True
 
-    def _prompt(self, ids: list[int], start: int) -> GPUArray:
+    def _prompt(self, ids: list[int], start: int) -> GPUArray | None:
         """`ids` through all layers, PROMPT_ROWS rows at a time; returns the final-norm hidden of the last slab of `max_batch_size`
         rows, like the slabs would; None, and nothing done, when there is no room for the portion's arrays."""
         slab, n = self.buffers.max_batch_size, len(ids)
@@ -288,13 +289,16 @@ class CausalTransformerModel:
             raise ValueError(f"context_len {start + n} exceeds the fixed cache ({self._max_seq})")
         portion = max(1, self.PROMPT_ROWS // slab) * slab                    # its ends are slabs' ends
         rows = min(portion, n)
-        if self._prompt_bufs is None or self._prompt_bufs.max_seq_len < rows:
-            self._prompt_bufs = None
+        b = self._prompt_bufs                    # held by this call, whoever asks for idle memory meanwhile
+        if b is None or b.max_seq_len < rows:
+            b = self._prompt_bufs = None
             try:
-                self._prompt_bufs = PrefillBuffers.for_rows(self.config, rows)
-            except RuntimeError:                     # out of device memory
+                b = self._prompt_bufs = PrefillBuffers.for_rows(self.config, rows)
+            except RuntimeError as e:
+                if not idle.out_of_memory(e):
+                    raise
                 return None
-        b, hidden = self._prompt_bufs, None
+            idle.register(self)
         for i in range(0, n, portion):
             part = ids[i:i + portion]
             hidden = self._embed(part, len(part), start + i, b)
@@ -303,6 +307,11 @@ class CausalTransformerModel:
         width = hidden.shape[1]
         tail = GPUArray((last, width), bfloat16, ptr=hidden.device_ptr + 2 * width * (m - last), source=hidden)
         return self._final(tail, self.buffers)
+
+    def give_back(self) -> bool:
+        """The arrays of long prompts, which the next one makes anew."""
+        held, self._prompt_bufs = self._prompt_bufs, None
+        return held is not None
 
     # ------------------------------------------------------------------ device-resident step
     def decode_step_device(self) -> None:

@@ -1,6 +1,8 @@
 """End-to-end parity of the decode path against the CPU restatement of the reference's step
 (oracle/model.py): logits within 1e-2 relative (BF16 bar of BASELINE.json), greedy tokens identical,
 graph replay == eager, for FP8 / NVF4 / BF16 weights, QK-norm on/off, dense and MoE."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -452,3 +454,34 @@ def test_captured_steps_follow_an_unfinished_prompt():
     model.set_decode_state(7, 1100)
     model.decode_step_device()
     assert int(model.buffers.next_token.to_numpy()[0]) == first
+
+
+def test_long_prompts_without_room_and_what_they_leave(monkeypatch):
+    """Without room for a portion's arrays a prompt runs in slabs; they stay for the next prompt, and go back on request."""
+    from pygpukit_b200._lib import api
+    from pygpukit_b200.llm.buffers import PrefillBuffers
+    model = llm.build_random_model("small-qwen3", "fp8", max_seq=1024, seed=7, std=0.05)
+    prompt = [int(t) for t in np.random.default_rng(1).integers(0, model.config.vocab_size, 900)]
+
+    def run():
+        model.init_decode(1024, max_batch_size=16)
+        return model.prefill(prompt).to_numpy()
+
+    run()
+    api.mem_trim()
+    free, used = (C.c_size_t() for _ in range(2))
+    api.mem_info(C.byref(free), C.byref(used))
+    before = free.value
+    a = run()
+    api.mem_trim()
+    api.mem_info(C.byref(free), C.byref(used))
+    assert abs(before - free.value) <= 2 << 20               # 512 rows have 4.7 MB (the decode arrays are new ones of the same size)
+
+    def full(*a):
+        raise RuntimeError("cudaMalloc(ptr, bytes) failed: out of memory (runtime.cu:303)")
+
+    monkeypatch.setattr(PrefillBuffers, "for_rows", classmethod(full))
+    b = run()
+    monkeypatch.setattr(type(model), "_long_portions", lambda self: False)
+    c = run()
+    assert np.array_equal(b, c) and np.linalg.norm(f32(a) - f32(b)) <= 10 * 2.0 ** -9 * np.linalg.norm(f32(b))

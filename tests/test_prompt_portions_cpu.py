@@ -61,3 +61,48 @@ def test_the_other_product_serves_gate_and_up_too(monkeypatch, impl, rows, produ
     mlp.gate_up_act(array(rows, 256), out=array(rows, 512))
     assert (calls.count("gemv_fp8_bf16_ex"), calls.count("gemv_fp8_swiglu_bf16")) == (products, fused)
     assert m._long_portions() is (impl != "2")
+
+
+def test_arrays_of_a_portion(monkeypatch):
+    """No room is no error, anything else is; the arrays stay for the next prompt, and go when idle memory is asked for or an allocation
+    would fail without them."""
+    from types import SimpleNamespace
+    from pygpukit_b200.core import array as array_module, idle
+    from pygpukit_b200.llm.models import causal
+    m, room, freed = model(4, 2, 128), [1 << 20], []
+
+    def malloc(out, n):
+        if n > room[0]:
+            raise RuntimeError("cudaMalloc(ptr, bytes) failed: out of memory (runtime.cu:303)")
+        room[0] -= n
+        out._obj.value = 4096
+        out._obj.size = n
+
+    def free(ptr):
+        freed.append(ptr)
+        room[0] = 1 << 20
+
+    api = SimpleNamespace(malloc=malloc, free=free)
+    monkeypatch.setattr(array_module, "api", api)
+    m.config = m.blocks[0].attn.config
+    m._buffers, m._max_seq, m._prompt_bufs = SimpleNamespace(max_batch_size=16), 4096, None
+    m._embed = lambda part, n, start, b: array(n, 256)
+    m._layers = lambda *a: None
+    m._final = lambda tail, b: tail
+    ids = list(range(40))
+    assert m._prompt(ids, 0).shape == (8, 256)
+    kept = m._prompt_bufs
+    assert kept is not None and m._prompt(ids, 0).shape == (8, 256) and m._prompt_bufs is kept and not freed
+    kept = None
+    x = GPUArray(((1 << 20) - 256,), uint8)                  # fits once the arrays are given back
+    assert freed == [4096] and m._prompt_bufs is None
+    assert m._prompt(ids, 0) is None                         # no room: slabs
+    del x
+    assert m._prompt(ids, 0) is not None and idle.give_back() and m._prompt_bufs is None and not idle.give_back()
+
+    def fault(out, n):
+        raise RuntimeError("cudaMalloc(ptr, bytes) failed: an illegal memory access was encountered (runtime.cu:303)")
+
+    api.malloc = fault
+    with pytest.raises(RuntimeError, match="illegal"):
+        m._prompt(ids, 0)
