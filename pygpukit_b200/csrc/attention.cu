@@ -68,13 +68,6 @@ template <> __device__ __forceinline__ void st_elem<0>(void* p, size_t i, float 
 template <> __device__ __forceinline__ void st_elem<1>(void* p, size_t i, float v) { ((__half*)p)[i] = __float2half_rn(v); }
 template <> __device__ __forceinline__ void st_elem<2>(void* p, size_t i, float v) { ((__nv_bfloat16*)p)[i] = __float2bfloat16_rn(v); }
 
-__device__ __forceinline__ uint4 ldg_kv(const void* p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-
 struct SdpaParams {
     const void* Q; const void* K; const void* V; void* out;
     int hq, n_kv, q_len, max_seq, context_len;
@@ -562,10 +555,10 @@ rope_sdpa_mma_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_cons
         const float* cs = p.cos_t + (size_t)pos * HD;
         const float* sn = p.sin_t + (size_t)pos * HD;
 #pragma unroll
-        for (int i = 0; i < 2; ++i) { rc[i] = __ldg(cs + lane + 32 * i); rs[i] = __ldg(sn + lane + 32 * i); }
+        for (int i = 0; i < 2; ++i) { rc[i] = cs[lane + 32 * i]; rs[i] = sn[lane + 32 * i]; }
         if (my_gamma) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) rg[i] = bf16_bits_to_f32(__ldg(my_gamma + lane + 32 * i));
+            for (int i = 0; i < 4; ++i) rg[i] = bf16_bits_to_f32(my_gamma[lane + 32 * i]);
         }
     }
     griddep_wait();

@@ -154,18 +154,21 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
     return r;
 }
 
-// streaming loads: read-only path, do not allocate in L1, evict-first in L2 (weights are
-// touched once per token).  sm_100a has 256-bit global loads.
+// What a kernel that is launched as a dependent reads may have been written by the kernel before, whose lifetime overlaps its own:
+// weights, too, unless pdl_enabled().  So no such kernel loads through the read-only path (.nc, __ldg), which is for what nobody writes
+// meanwhile, and no pointer that it loads through is __restrict__, which lets the compiler choose that path and move the load ahead
+// of griddep_wait; a pointer that is only stored through may be.
+
+// streaming loads: do not allocate in L1, evict-first in L2 (weights are touched once per token).  sm_100a has 256-bit global loads.
 struct alignas(32) u32x8 { uint32_t v[8]; };
 __device__ __forceinline__ u32x8 ldg_stream256(const void* p) {
     u32x8 r;
-    asm volatile("ld.global.nc.L1::no_allocate.L2::evict_first.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm volatile("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]),
                    "=r"(r.v[6]), "=r"(r.v[7]) : "l"(p));
     return r;
 }
-// activations written by the kernel just before this one (programmatic dependent launch: this kernel's lifetime
-// overlaps its producer's, so the read-only .nc path is formally off limits for them): coherent, L2-cached loads
+// activations written by the kernel just before this one: coherent, L2-cached loads
 __device__ __forceinline__ uint4 ld_act16(const void* p) {
     uint4 v;
     asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
@@ -178,7 +181,7 @@ __device__ __forceinline__ uint16_t ld_act2(const uint16_t* p) {
 }
 __device__ __forceinline__ uint4 ldg_stream(const void* p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }

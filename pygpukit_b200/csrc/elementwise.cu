@@ -47,60 +47,53 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 // ---------------------------------------------------------------- RMSNorm / LayerNorm
 // rmsnorm_*_kernel norm_kernels.cuh:375-585: y = x * rsqrt(mean(x^2)+eps) * gamma (left to right).
 template <int DT, bool RESIDUAL>
-__global__ void rmsnorm_kernel(const void* __restrict__ x, const void* __restrict__ res,
-                               const void* __restrict__ gamma, void* __restrict__ y, int features, float eps) {
+__global__ void rmsnorm_kernel(const void* x, const void* res,
+                               const void* gamma, void* __restrict__ y, int features, float eps) {
     __shared__ float red[32];
     griddep_wait();
     griddep_launch();
     const size_t base = (size_t)blockIdx.x * features;
-    // thread t owns elements t, t + bs, ... (the reference's partial sums); up to 32 of them are loaded
-    // up front (all loads in flight at once) and kept in registers for the second pass
-    constexpr int MAXE = 32;
-    float xv[MAXE];
+    // Thread t owns elements t, t + bs, ... (the reference's partial sums).  Latency bounds it: GRP elements are loaded ahead of their sums
+    // and stores (no load passes a store), and read again for the second pass: kept in registers meanwhile, they left an SM three blocks
+    // (us, kept -> here: 1 row of 4096 6.2 -> 4.1, 512 rows 12.3 -> 6.2, 2000 rows 22.6 -> 14.3; 2000 rows of 12288 47.6 -> 36.9).
+    constexpr int GRP = 8;
     const int bs = blockDim.x;
-    const bool cached = features <= bs * MAXE;
+    auto row = [&](float (&v)[GRP], int i0) {
+#pragma unroll
+        for (int j = 0; j < GRP; ++j) {
+            const int i = i0 + j * bs;
+            v[j] = i < features ? Elem<DT>::ld(x, base + i) : 0.f;
+        }
+        if (RESIDUAL) {
+#pragma unroll
+            for (int j = 0; j < GRP; ++j)
+                if (i0 + j * bs < features) v[j] += Elem<DT>::ld(res, base + i0 + j * bs);   // fused_kernels.cuh:36-220 keeps the sum in f32
+        }
+    };
     float ss = 0.f;
-    if (cached) {
+    for (int i0 = threadIdx.x; i0 < features; i0 += GRP * bs) {
+        float v[GRP];
+        row(v, i0);
 #pragma unroll
-        for (int e = 0; e < MAXE; ++e) {
-            const int i = threadIdx.x + e * bs;
-            xv[e] = 0.f;
-            if (i < features) {
-                xv[e] = Elem<DT>::ld(x, base + i);
-                if (RESIDUAL) xv[e] += Elem<DT>::ld(res, base + i);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < MAXE; ++e)
-            if (threadIdx.x + e * bs < features) ss = fmaf(xv[e], xv[e], ss);
-    } else {
-        for (int i = threadIdx.x; i < features; i += bs) {
-            float v = Elem<DT>::ld(x, base + i);
-            if (RESIDUAL) v += Elem<DT>::ld(res, base + i);   // fused_kernels.cuh:36-220 keeps the sum in f32
-            ss = fmaf(v, v, ss);
-        }
+        for (int j = 0; j < GRP; ++j)
+            if (i0 + j * bs < features) ss = fmaf(v[j], v[j], ss);
     }
-    float tot = block_sum(ss, red);
-    float inv = rsqrtf(tot / (float)features + eps);
-    if (cached) {
+    const float inv = rsqrtf(block_sum(ss, red) / (float)features + eps);
+    for (int i0 = threadIdx.x; i0 < features; i0 += GRP * bs) {
+        float v[GRP], g[GRP];
+        row(v, i0);
 #pragma unroll
-        for (int e = 0; e < MAXE; ++e) {
-            const int i = threadIdx.x + e * bs;
-            if (i < features) Elem<DT>::st(y, base + i, xv[e] * inv * Elem<DT>::ld(gamma, i));
-        }
-    } else {
-        for (int i = threadIdx.x; i < features; i += bs) {
-            float v = Elem<DT>::ld(x, base + i);
-            if (RESIDUAL) v += Elem<DT>::ld(res, base + i);
-            Elem<DT>::st(y, base + i, v * inv * Elem<DT>::ld(gamma, i));
-        }
+        for (int j = 0; j < GRP; ++j) g[j] = i0 + j * bs < features ? Elem<DT>::ld(gamma, i0 + j * bs) : 0.f;
+#pragma unroll
+        for (int j = 0; j < GRP; ++j)
+            if (i0 + j * bs < features) Elem<DT>::st(y, base + i0 + j * bs, v[j] * inv * g[j]);
     }
 }
 
 // layernorm_*_kernel norm_kernels.cuh:32-330: mean, var = mean((x-mean)^2), (x-mean)*rsqrt(var+eps)*g+b
 template <int DT>
-__global__ void layernorm_kernel(const void* __restrict__ x, const void* __restrict__ gamma,
-                                 const void* __restrict__ beta, void* __restrict__ y, int features, float eps) {
+__global__ void layernorm_kernel(const void* x, const void* gamma,
+                                 const void* beta, void* __restrict__ y, int features, float eps) {
     __shared__ float red[32];
     griddep_wait();
     griddep_launch();
@@ -126,8 +119,8 @@ __global__ void layernorm_kernel(const void* __restrict__ x, const void* __restr
 // rope_*_kernel / rope_*_f32table_kernel elementwise_kernels.cuh:82-366.  One thread per
 // (position, head, d < hd/2) of q then k.
 template <int DT, int TDT>
-__global__ void rope_kernel(void* __restrict__ q, void* __restrict__ k, const void* __restrict__ cs,
-                            const void* __restrict__ sn, int seq, int hq, int hk, int hd) {
+__global__ void rope_kernel(void* q, void* k, const void* cs,
+                            const void* sn, int seq, int hq, int hk, int hd) {
     griddep_wait();
     griddep_launch();
     const int half = hd >> 1;
@@ -157,7 +150,7 @@ __device__ __forceinline__ float gelu_f(float x) {                              
 }
 
 template <int DT, int OP>
-__global__ void unary_kernel(const void* __restrict__ x, void* __restrict__ y, size_t n) {
+__global__ void unary_kernel(const void* x, void* __restrict__ y, size_t n) {
     griddep_wait();
     griddep_launch();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -169,7 +162,7 @@ __global__ void unary_kernel(const void* __restrict__ x, void* __restrict__ y, s
 // add: f32 add then one rounding (elementwise/elementwise_kernels.cuh:55-60);
 // mul: exact f32 product then rounding; swiglu: silu_f32(g)*u one rounding (fused_kernels.cuh:233-247)
 template <int DT, int OP>
-__global__ void binary_kernel(const void* __restrict__ a, const void* __restrict__ b, void* __restrict__ c, size_t n) {
+__global__ void binary_kernel(const void* a, const void* b, void* __restrict__ c, size_t n) {
     griddep_wait();
     griddep_launch();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -186,7 +179,7 @@ __global__ void binary_kernel(const void* __restrict__ a, const void* __restrict
 // in-place native-precision add/mul (__hadd/__hmul: one rounding of the exact result),
 // elementwise_kernels.cuh:370-470
 template <int DT, int OP>
-__global__ void binary_inplace_kernel(void* __restrict__ a, const void* __restrict__ b, size_t n) {
+__global__ void binary_inplace_kernel(void* a, const void* b, size_t n) {
     griddep_wait();
     griddep_launch();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -200,7 +193,7 @@ __global__ void binary_inplace_kernel(void* __restrict__ a, const void* __restri
 
 // bias_add_*_kernel elementwise_kernels.cuh:22-75: f32 add, one rounding
 template <int DT>
-__global__ void bias_add_kernel(void* __restrict__ x, const void* __restrict__ bias, size_t n, int features) {
+__global__ void bias_add_kernel(void* x, const void* bias, size_t n, int features) {
     griddep_wait();
     griddep_launch();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -209,7 +202,7 @@ __global__ void bias_add_kernel(void* __restrict__ x, const void* __restrict__ b
 }
 
 template <int SDT, int DDT>
-__global__ void cast_kernel(const void* __restrict__ s, void* __restrict__ d, size_t n) {
+__global__ void cast_kernel(const void* s, void* __restrict__ d, size_t n) {
     griddep_wait();
     griddep_launch();
     size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -219,9 +212,9 @@ __global__ void cast_kernel(const void* __restrict__ s, void* __restrict__ d, si
 // GPT-2 input: hidden[t] = wte[token[t]] + wpe[pos + t], one rounding (models/causal.py:137-146 adds the
 // two rows on the host in the storage dtype); token ids and the position may live in device buffers.
 template <int DT>
-__global__ void embedding_pos_kernel(const void* __restrict__ wte, const void* __restrict__ wpe, void* __restrict__ out,
-                                     int H, const int32_t* __restrict__ token_buf, int n_tokens, int pos,
-                                     const int32_t* __restrict__ pos_buf) {
+__global__ void embedding_pos_kernel(const void* wte, const void* wpe, void* __restrict__ out,
+                                     int H, const int32_t* token_buf, int n_tokens, int pos,
+                                     const int32_t* pos_buf) {
     griddep_wait();
     griddep_launch();
     const int p0 = pos_buf ? *pos_buf : pos;
@@ -234,8 +227,8 @@ __global__ void embedding_pos_kernel(const void* __restrict__ wte, const void* _
 
 // ---------------------------------------------------------------- gather / argmax / layout
 // embedding_lookup(_ptr,_batch) embedding_kernels.cuh:27-165: row copy; token id from host or device
-__global__ void embedding_kernel(const uint8_t* __restrict__ table, uint8_t* __restrict__ out, size_t row_bytes,
-                                 int token, const int32_t* __restrict__ token_buf, int n_tokens) {
+__global__ void embedding_kernel(const uint8_t* table, uint8_t* __restrict__ out, size_t row_bytes,
+                                 int token, const int32_t* token_buf, int n_tokens) {
     griddep_wait();
     griddep_launch();
     const size_t vec = row_bytes >> 4;
@@ -244,7 +237,7 @@ __global__ void embedding_kernel(const uint8_t* __restrict__ table, uint8_t* __r
         const uint4* src = reinterpret_cast<const uint4*>(table + (size_t)tok * row_bytes);
         uint4* dst = reinterpret_cast<uint4*>(out + (size_t)t * row_bytes);
         for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < vec; i += (size_t)gridDim.x * blockDim.x)
-            dst[i] = __ldg(src + i);
+            dst[i] = src[i];
         if (blockIdx.x == 0)
             for (size_t i = (vec << 4) + threadIdx.x; i < row_bytes; i += blockDim.x)
                 out[(size_t)t * row_bytes + i] = table[(size_t)tok * row_bytes + i];
@@ -253,7 +246,7 @@ __global__ void embedding_kernel(const uint8_t* __restrict__ table, uint8_t* __r
 
 // sample_argmax_*_kernel sampling_kernels.cuh:55-200: first maximum wins (np.argmax)
 template <int DT>
-__global__ void argmax_kernel(const void* __restrict__ x, int32_t* __restrict__ out, int n) {
+__global__ void argmax_kernel(const void* x, int32_t* __restrict__ out, int n) {
     __shared__ float sv[32];
     __shared__ int si[32];
     griddep_wait();
@@ -281,7 +274,7 @@ __global__ void argmax_kernel(const void* __restrict__ x, int32_t* __restrict__ 
 // gate/up columns interleaved in groups of 8 ([g0..g7, u0..u7, g8..], the fused NVF4 MLP tensor): out[m, j] =
 // bf16( bf16(silu(g)) * u ) -- silu_bf16_kernel then mul_inplace_bf16_kernel of the reference (activation_kernels.cuh:164-171,
 // elementwise_kernels.cuh:429-438), two roundings
-__global__ void swiglu_interleaved8_kernel(const uint16_t* __restrict__ gu, uint16_t* __restrict__ out, int M, int I) {
+__global__ void swiglu_interleaved8_kernel(const uint16_t* gu, uint16_t* __restrict__ out, int M, int I) {
     griddep_wait();
     griddep_launch();
     const size_t total = (size_t)M * I;
@@ -296,7 +289,7 @@ __global__ void swiglu_interleaved8_kernel(const uint16_t* __restrict__ gu, uint
 }
 // one CTA per row of a [rows, n] matrix (greedy tokens of a decode batch); out2 (optional) receives the same tokens
 template <int DT>
-__global__ void argmax_rows_kernel(const void* __restrict__ x, int32_t* __restrict__ out, int32_t* __restrict__ out2, int n) {
+__global__ void argmax_rows_kernel(const void* x, int32_t* __restrict__ out, int32_t* __restrict__ out2, int n) {
     __shared__ float sv[32];
     __shared__ int si[32];
     griddep_wait();
@@ -327,7 +320,7 @@ __global__ void argmax_rows_kernel(const void* __restrict__ x, int32_t* __restri
 
 // transpose_3d_021: [d0,d1,d2] -> [d1,d0,d2]
 template <typename T>
-__global__ void transpose021_kernel(const T* __restrict__ in, T* __restrict__ out, int d0, int d1, int d2) {
+__global__ void transpose021_kernel(const T* in, T* __restrict__ out, int d0, int d1, int d2) {
     griddep_wait();
     griddep_launch();
     size_t n = (size_t)d0 * d1 * d2;
@@ -341,9 +334,9 @@ __global__ void transpose021_kernel(const T* __restrict__ in, T* __restrict__ ou
 
 // kv_cache_update(_gqa)(_ptr) / kv_cache_prefill_gqa kv_cache_kernels.cuh:176-421.
 // new_kv [seq, n_kv, hd] -> cache [heads_out, max_seq, hd]; heads_out = G * n_kv replicates.
-__global__ void kv_update_kernel(const uint8_t* __restrict__ new_kv, uint8_t* __restrict__ cache, int seq, int n_kv,
+__global__ void kv_update_kernel(const uint8_t* new_kv, uint8_t* __restrict__ cache, int seq, int n_kv,
                                  int heads_out, size_t row_bytes, int max_seq, int pos,
-                                 const int32_t* __restrict__ pos_buf) {
+                                 const int32_t* pos_buf) {
     griddep_wait();
     griddep_launch();
     const int p0 = pos_buf ? *pos_buf : pos;
@@ -360,9 +353,9 @@ __global__ void kv_update_kernel(const uint8_t* __restrict__ new_kv, uint8_t* __
         dst[v] = src[v];
     }
 }
-__global__ void kv_update_bytes_kernel(const uint8_t* __restrict__ new_kv, uint8_t* __restrict__ cache, int seq,
+__global__ void kv_update_bytes_kernel(const uint8_t* new_kv, uint8_t* __restrict__ cache, int seq,
                                        int n_kv, int heads_out, size_t row_bytes, int max_seq, int pos,
-                                       const int32_t* __restrict__ pos_buf) {
+                                       const int32_t* pos_buf) {
     griddep_wait();
     griddep_launch();
     const int p0 = pos_buf ? *pos_buf : pos;
@@ -381,11 +374,11 @@ __global__ void kv_update_bytes_kernel(const uint8_t* __restrict__ new_kv, uint8
 // pos+m) -> in-place store (q, k) and K/V cache write.  Rounds to bf16 after the norm and after
 // the rotation exactly like rmsnorm -> rope_inplace_f32table -> kv_cache_update_gqa
 // (layers/attention.py:326-351).
-__global__ void qk_norm_rope_kv_kernel(uint16_t* __restrict__ qkv, const uint16_t* __restrict__ qg,
-                                       const uint16_t* __restrict__ kg, float eps, const float* __restrict__ cs,
-                                       const float* __restrict__ sn, uint16_t* __restrict__ kc,
+__global__ void qk_norm_rope_kv_kernel(uint16_t* qkv, const uint16_t* qg,
+                                       const uint16_t* kg, float eps, const float* cs,
+                                       const float* sn, uint16_t* __restrict__ kc,
                                        uint16_t* __restrict__ vc, int M, int hq, int hkv, int hd, int max_seq,
-                                       int pos, const int32_t* __restrict__ pos_buf) {
+                                       int pos, const int32_t* pos_buf) {
     griddep_wait();
     griddep_launch();
     const int lane = threadIdx.x & 31;

@@ -87,8 +87,8 @@ gemm_fp8_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     // the block's scales are weights: staged before the dependency wait
     const size_t scales = (size_t)(blockIdx.y >> (PAIR ? 1 : 0)) * nkb_total + kb0;
     for (int i = tid; i < nkb; i += F_THREADS) {
-        sc_s[i] = bf16_bits_to_f32(__ldg(p.S + scales + i));
-        if (PAIR) sc_s[kTcMaxKb + i] = bf16_bits_to_f32(__ldg(p.S1 + scales + i));
+        sc_s[i] = bf16_bits_to_f32(p.S[scales + i]);
+        if (PAIR) sc_s[kTcMaxKb + i] = bf16_bits_to_f32(p.S1[scales + i]);
     }
     if (warp == F_WARPS + 1) tmem_alloc(&tmem_base_s, TMEM_COLS);
     if (tid == 0) {

@@ -277,8 +277,8 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
 #pragma unroll 1
             for (int it = 0; it < nkb; ++it) {
                 if ((it & 31) == 0) {
-                    s0 = __ldg(p.S0 + scales + min(it + lane, nkb - 1));
-                    if (PAIR) s1 = __ldg(p.S1 + scales + min(it + lane, nkb - 1));
+                    s0 = p.S0[scales + min(it + lane, nkb - 1)];
+                    if (PAIR) s1 = p.S1[scales + min(it + lane, nkb - 1)];
                 }
                 uint32_t bits = __shfl_sync(0xffffffffu, s0, it & 31);
                 if (PAIR) {

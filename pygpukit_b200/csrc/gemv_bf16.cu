@@ -22,8 +22,8 @@
 namespace pgk {
 
 template <int M>
-__device__ __forceinline__ void stage_activations_bf16(const uint16_t* __restrict__ A, int K, uint16_t* a_s,
-                                                       const uint16_t* __restrict__ gamma = nullptr, float eps = 0.f) {
+__device__ __forceinline__ void stage_activations_bf16(const uint16_t* A, int K, uint16_t* a_s,
+                                                       const uint16_t* gamma = nullptr, float eps = 0.f) {
     const int nvec = K >> 3, nchunk = K >> 4;
     float rinv[M];
 #pragma unroll
@@ -36,7 +36,7 @@ __device__ __forceinline__ void stage_activations_bf16(const uint16_t* __restric
         uint4* dst = reinterpret_cast<uint4*>(a_s + (size_t)m * K);
         for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
             uint4 v = ld_act16(src + j);
-            if (gamma) v = norm8_bf16(v, __ldg(gv + j), rinv[m]);
+            if (gamma) v = norm8_bf16(v, gv[j], rinv[m]);
             dst[(j & 1) * nchunk + (j >> 1)] = v;
         }
     }
@@ -51,7 +51,7 @@ struct ArgmaxOut {
 
 template <int M, bool ARGMAX>
 __global__ void __launch_bounds__(512)
-gemv_bf16_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B, uint16_t* __restrict__ C,
+gemv_bf16_kernel(const uint16_t* A, const uint16_t* B, uint16_t* __restrict__ C,
                  int K, int N, int rho, GemvEpilogue epi, ArgmaxOut am) {
     constexpr int U = 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -139,7 +139,7 @@ gemv_bf16_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B,
 }
 
 template <bool ARGMAX>
-__global__ void gemv_bf16_generic_kernel(const uint16_t* __restrict__ A, const uint16_t* __restrict__ B,
+__global__ void gemv_bf16_generic_kernel(const uint16_t* A, const uint16_t* B,
                                          uint16_t* __restrict__ C, int M, int K, int N, GemvEpilogue epi) {
     griddep_wait();
     griddep_launch();

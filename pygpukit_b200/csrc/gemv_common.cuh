@@ -84,7 +84,7 @@ __device__ __forceinline__ void xchg_finish(const GemvXchg& x, unsigned seq, uns
 // threads, thread t folds elements t, t+bs, ... with fma, a shuffle tree per warp, then a tree over
 // the warp totals.  `scratch` needs bs floats of shared memory; every thread returns the same value,
 // so fused and unfused paths give bit-identical normalised activations.
-__device__ __forceinline__ float row_inv_rms_ref_order(const uint16_t* __restrict__ row, int K, float eps,
+__device__ __forceinline__ float row_inv_rms_ref_order(const uint16_t* row, int K, float eps,
                                                        float* scratch) {
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
     const int bs = min(256, (K + 31) & ~31), nw = bs >> 5;
@@ -128,9 +128,9 @@ __device__ __forceinline__ uint4 norm8_bf16(const uint4& x, const uint4& g, floa
 // per-lane 16-byte reads (lane = chunk) are bank-conflict free.
 // PLANES = false keeps the natural k order (used by the column-parallel NVF4 kernel).
 template <int M, bool PLANES = true>
-__device__ __forceinline__ void stage_activations_f16_3pass(const uint16_t* __restrict__ A, int K,
+__device__ __forceinline__ void stage_activations_f16_3pass(const uint16_t* A, int K,
                                                             __half* a_s, float* inv_s, uint32_t* red,
-                                                            const uint16_t* __restrict__ gamma = nullptr,
+                                                            const uint16_t* gamma = nullptr,
                                                             float eps = 0.f) {
     const int tid = threadIdx.x, nthr = blockDim.x;
     const int nvec = K >> 3;  // 16-byte vectors per row
@@ -148,7 +148,7 @@ __device__ __forceinline__ void stage_activations_f16_3pass(const uint16_t* __re
         const uint4* src = reinterpret_cast<const uint4*>(A + (size_t)m * K);
         for (int j = tid; j < nvec; j += nthr) {
             uint4 v = ld_act16(src + j);
-            if (gamma) v = norm8_bf16(v, __ldg(gv + j), rinv[m]);
+            if (gamma) v = norm8_bf16(v, gv[j], rinv[m]);
             uint32_t t = __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu),
                                   __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
             mx[m] = max(mx[m], max(t & 0xffffu, t >> 16));
@@ -179,7 +179,7 @@ __device__ __forceinline__ void stage_activations_f16_3pass(const uint16_t* __re
         uint4* dst = reinterpret_cast<uint4*>(a_s + (size_t)m * K);
         for (int j = tid; j < nvec; j += nthr) {
             uint4 v = ld_act16(src + j);
-            if (gamma) v = norm8_bf16(v, __ldg(gv + j), rinv[m]);
+            if (gamma) v = norm8_bf16(v, gv[j], rinv[m]);
             uint4 o;
             __half2 h;
             h = __floats2half2_rn(bf16lo(v.x) * mult[m], bf16hi(v.x) * mult[m]); o.x = *reinterpret_cast<uint32_t*>(&h);
@@ -209,9 +209,9 @@ __device__ __forceinline__ uint4 bf16x8_to_f16x8_scaled(const uint4& v, float mu
 // `red`, and the f16 planes are written last.  Same arithmetic, hence the same bits, as the 3-pass version.
 //   red[0 .. 63]   : per-warp maxima (m * 16 + warp)      red[64 .. 71] : per-virtual-warp sums of squares
 template <int M, bool PLANES = true>
-__device__ __forceinline__ void stage_activations_f16(const uint16_t* __restrict__ A, int K,
+__device__ __forceinline__ void stage_activations_f16(const uint16_t* A, int K,
                                                       __half* a_s, float* inv_s, uint32_t* red,
-                                                      const uint16_t* __restrict__ gamma = nullptr,
+                                                      const uint16_t* gamma = nullptr,
                                                       float eps = 0.f) {
     constexpr int VY = 8;
     const int tid = threadIdx.x, nthr = blockDim.x;
@@ -234,7 +234,7 @@ __device__ __forceinline__ void stage_activations_f16(const uint16_t* __restrict
             const int j = tid + e * nthr;
             if (j < nvec) {
                 v[e] = ld_act16(src + j);
-                if (gamma) g[e] = __ldg(gv + j);
+                if (gamma) g[e] = gv[j];
             }
         }
         if (gamma) {

@@ -41,7 +41,7 @@ template <> struct ColVec<16> {
 template <> struct ColVec<8> {
     uint32_t w[2];
     __device__ __forceinline__ void load(const uint8_t* p) {
-        asm volatile("ld.global.nc.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
+        asm volatile("ld.global.L1::no_allocate.v2.u32 {%0,%1}, [%2];" : "=r"(w[0]), "=r"(w[1]) : "l"(p));
     }
 };
 
@@ -240,8 +240,8 @@ __global__ void __launch_bounds__(512) gemv_nvf4_kernel(Nvf4Params p) {
 
 // Generic fallback (any K / N / alignment): one thread per (m, column), serial over K in the
 // reference's own order (nvf4_kernels.cu:19-73).
-__global__ void gemv_nvf4_generic_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ Bd,
-                                         const uint8_t* __restrict__ Bs, uint16_t* __restrict__ C, int M,
+__global__ void gemv_nvf4_generic_kernel(const uint16_t* A, const uint8_t* Bd,
+                                         const uint8_t* Bs, uint16_t* __restrict__ C, int M,
                                          int K, int N, float alpha, GemvEpilogue epi) {
     griddep_wait();
     griddep_launch();

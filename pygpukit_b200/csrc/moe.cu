@@ -21,7 +21,7 @@ template <> __device__ __forceinline__ void mst<2>(void* p, size_t i, float v) {
 // topk_with_indices_*_kernel topk_kernels.cuh:69-186: k passes of strict '>' argmax (lowest
 // index wins ties).  One warp per token: lane-strided scan + (value, index) shuffle reduce.
 template <int DT>
-__global__ void moe_topk_kernel(const void* __restrict__ logits, void* __restrict__ values,
+__global__ void moe_topk_kernel(const void* logits, void* __restrict__ values,
                                 int32_t* __restrict__ indices, int T, int E, int k) {
     griddep_wait();
     griddep_launch();
@@ -52,7 +52,7 @@ __global__ void moe_topk_kernel(const void* __restrict__ logits, void* __restric
 
 // softmax_topk_*_kernel topk_kernels.cuh:192-256, in place, one thread per token
 template <int DT>
-__global__ void moe_softmax_topk_kernel(void* __restrict__ values, int T, int k) {
+__global__ void moe_softmax_topk_kernel(void* values, int T, int k) {
     griddep_wait();
     griddep_launch();
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -68,32 +68,44 @@ __global__ void moe_softmax_topk_kernel(void* __restrict__ values, int T, int k)
 }
 
 // count/offsets/permute/reverse in one single-CTA kernel (T*k <= 512 at decode), ascending order.
-__global__ void moe_permutation_kernel(const int32_t* __restrict__ expert_indices, int32_t* __restrict__ counts,
-                                       int32_t* __restrict__ offsets, int32_t* __restrict__ permute,
+__global__ void moe_permutation_kernel(const int32_t* expert_indices, int32_t* __restrict__ counts,
+                                       int32_t* offsets, int32_t* __restrict__ permute,
                                        int32_t* __restrict__ reverse, int total, int E) {
+    constexpr int STAGED = 4096, COUNTED = 1024;  // choices and experts that shared memory holds
+    __shared__ int32_t staged[STAGED], first[COUNTED];
     griddep_wait();
     griddep_launch();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        int c = 0;
-        for (int i = 0; i < total; ++i) c += (expert_indices[i] == e);
-        counts[e] = c;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int off = 0;
-        for (int e = 0; e < E; ++e) { offsets[e] = off; off += counts[e]; }
-        offsets[E] = off;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < E; e += blockDim.x) {
-        int p = offsets[e];
-        for (int i = 0; i < total; ++i)
-            if (expert_indices[i] == e) { permute[p] = i; reverse[i] = p; ++p; }
-    }
+    auto fill = [&](const int32_t* chosen, int32_t* at) {         // at: counts, then the offsets before each expert
+        for (int e = threadIdx.x; e < E; e += blockDim.x) {
+            int c = 0;
+#pragma unroll 8
+            for (int i = 0; i < total; ++i) c += (chosen[i] == e);
+            at[e] = counts[e] = c;
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int off = 0;
+            for (int e = 0; e < E; ++e) { const int c = at[e]; at[e] = offsets[e] = off; off += c; }
+            offsets[E] = off;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < E; e += blockDim.x) {
+            int p = at[e];
+#pragma unroll 8
+            for (int i = 0; i < total; ++i)
+                if (chosen[i] == e) { permute[p] = i; reverse[i] = p; ++p; }
+        }
+    };
+    if (total <= STAGED && E <= COUNTED) {
+        for (int i = threadIdx.x; i < total; i += blockDim.x) staged[i] = expert_indices[i];
+        __syncthreads();
+        fill(staged, first);
+    } else
+        fill(expert_indices, offsets);
 }
 
 // expand_expert_offsets_kernel moe_kernels.cuh:236-259
-__global__ void moe_expand_offsets_kernel(const int32_t* __restrict__ offsets, int32_t* __restrict__ row_ids, int E,
+__global__ void moe_expand_offsets_kernel(const int32_t* offsets, int32_t* __restrict__ row_ids, int E,
                                           int m_total) {
     griddep_wait();
     griddep_launch();
@@ -105,29 +117,43 @@ __global__ void moe_expand_offsets_kernel(const int32_t* __restrict__ offsets, i
 }
 
 // gather_hidden_states_* permute_kernels.cuh:95-182: gathered[p] = hidden[permute[p] / k]
-__global__ void moe_gather_kernel(const uint16_t* __restrict__ hidden, const int32_t* __restrict__ permute,
+__global__ void moe_gather_kernel(const uint16_t* hidden, const int32_t* permute,
                                   uint16_t* __restrict__ gathered, int rows, int H, int k) {
     griddep_wait();
     griddep_launch();
     for (int p = blockIdx.x; p < rows; p += gridDim.x) {
         const uint16_t* src = hidden + (size_t)(permute[p] / k) * H;
-        for (int i = threadIdx.x; i < H; i += blockDim.x) gathered[(size_t)p * H + i] = src[i];
+        constexpr int U = 8;                      // loads ahead of the stores, which no load passes
+        for (int i0 = threadIdx.x; i0 < H; i0 += U * blockDim.x) {
+            uint16_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + u * blockDim.x < H) v[u] = src[i0 + u * blockDim.x];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (i0 + u * blockDim.x < H) gathered[(size_t)p * H + i0 + u * blockDim.x] = v[u];
+        }
     }
 }
 
 // scatter_with_reverse_perm_kernel permute_kernels.cuh:218-242: f32 sum over slots 0..k-1
-__global__ void moe_scatter_kernel(const uint16_t* __restrict__ expert_out, const uint16_t* __restrict__ weights,
-                                   const int32_t* __restrict__ reverse, uint16_t* __restrict__ out, int T, int H, int k) {
+__global__ void moe_scatter_kernel(const uint16_t* expert_out, const uint16_t* weights,
+                                   const int32_t* reverse, uint16_t* __restrict__ out, int T, int H, int k) {
     griddep_wait();
     griddep_launch();
     for (int t = blockIdx.x; t < T; t += gridDim.x)
-        for (int h = threadIdx.x; h < H; h += blockDim.x) {
-            float sum = 0.f;
+        for (int h0 = threadIdx.x; h0 < H; h0 += 4 * blockDim.x) {
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
             for (int s = 0; s < k; ++s) {
-                int f = t * k + s;
-                sum = fmaf(bf16_bits_to_f32(weights[f]), bf16_bits_to_f32(expert_out[(size_t)reverse[f] * H + h]), sum);
+                const float w = bf16_bits_to_f32(weights[t * k + s]);
+                const uint16_t* row = expert_out + (size_t)reverse[t * k + s] * H;
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (h0 + u * blockDim.x < H) sum[u] = fmaf(w, bf16_bits_to_f32(row[h0 + u * blockDim.x]), sum[u]);
             }
-            out[(size_t)t * H + h] = f32_to_bf16_bits(sum);
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (h0 + u * blockDim.x < H) out[(size_t)t * H + h0 + u * blockDim.x] = f32_to_bf16_bits(sum[u]);
         }
 }
 
@@ -135,7 +161,7 @@ __global__ void moe_scatter_kernel(const uint16_t* __restrict__ expert_out, cons
 // 128 k), then a warp sum: 128-bit weight loads, exact f32 products, lane-strided 16-k chunks.  Every
 // expert GEMV below goes through this one function, so fused and unfused forms agree bit for bit.
 template <int NB, bool CLEAN>
-__device__ __forceinline__ void fp8_rows_dot(const uint16_t* __restrict__ arow, const uint8_t* const (&brow)[NB],
+__device__ __forceinline__ void fp8_rows_dot(const uint16_t* arow, const uint8_t* const (&brow)[NB],
                                              const uint16_t* const (&srow)[NB], int K, int lane, float (&acc)[NB]) {
 #pragma unroll
     for (int b = 0; b < NB; ++b) acc[b] = 0.f;
@@ -185,9 +211,9 @@ __device__ __forceinline__ void fp8_rows_dot(const uint16_t* __restrict__ arow, 
 // One warp per (m, n): 128-bit weight loads, exact f32 products (bf16 activation x decoded
 // e4m3), scale per 128-k block.  K % 16 == 0 fast path, scalar tail otherwise.
 template <bool CLEAN>
-__global__ void moe_grouped_gemv_fp8_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ B,
-                                            const uint16_t* __restrict__ S, uint16_t* __restrict__ C,
-                                            const int32_t* __restrict__ row_ids, int M, int K, int N,
+__global__ void moe_grouped_gemv_fp8_kernel(const uint16_t* A, const uint8_t* B,
+                                            const uint16_t* S, uint16_t* __restrict__ C,
+                                            const int32_t* row_ids, int M, int K, int N,
                                             int a_stride, int expert_offset, int num_local) {
     griddep_wait();
     griddep_launch();
@@ -213,7 +239,7 @@ __global__ void moe_grouped_gemv_fp8_kernel(const uint16_t* __restrict__ A, cons
 // router logits, then softmax over the selected values in slot order -- the arithmetic of topk_with_indices +
 // softmax_topk (topk_kernels.cuh:111-147,222-256), statement for statement.  Lane j < k returns expert j and its
 // bf16 weight bits.
-__device__ __forceinline__ void moe_route_warp(const uint16_t* __restrict__ logits, int E, int k, int lane, int& my_idx,
+__device__ __forceinline__ void moe_route_warp(const uint16_t* logits, int E, int k, int lane, int& my_idx,
                                                uint16_t& my_w) {
     constexpr int MAXPL = 16;
     float loc[MAXPL];
@@ -262,12 +288,12 @@ constexpr int kMoeNvf4Warps = 16;   // 512 threads: 128 registers per thread (32
 // B200 and removed; numbers in profiles/r01_bench_qwen3-30b-a3b_*.json and DESIGN.md.)
 template <int NMAT>
 __global__ void __launch_bounds__(kMoeNvf4Warps * 32)
-moe_grouped_gemv_nvf4_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ Bd0,
-                             const uint8_t* __restrict__ Bs0, const uint8_t* __restrict__ Bd1,
-                             const uint8_t* __restrict__ Bs1, uint16_t* __restrict__ C,
-                             const int32_t* __restrict__ row_expert_ids, int K, int N, int a_stride,
-                             int expert_offset, int num_local, float* __restrict__ split_ws,
-                             unsigned* __restrict__ split_cnt) {
+moe_grouped_gemv_nvf4_kernel(const uint16_t* A, const uint8_t* Bd0,
+                             const uint8_t* Bs0, const uint8_t* Bd1,
+                             const uint8_t* Bs1, uint16_t* __restrict__ C,
+                             const int32_t* row_expert_ids, int K, int N, int a_stride,
+                             int expert_offset, int num_local, float* split_ws,
+                             unsigned* split_cnt) {
     extern __shared__ __align__(16) unsigned char moe_smem[];
     __shared__ unsigned s_ticket;
     float* a_s = reinterpret_cast<float*>(moe_smem);                  // [K]
@@ -287,7 +313,15 @@ moe_grouped_gemv_nvf4_kernel(const uint16_t* __restrict__ A, const uint8_t* __re
         }
         return;
     }
-    for (int k = threadIdx.x; k < K; k += blockDim.x) a_s[k] = bf16_bits_to_f32(A[(size_t)r * a_stride + k]);
+    for (int k0 = threadIdx.x; k0 < K; k0 += 4 * kMoeNvf4Warps * 32) {
+        uint16_t v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u * kMoeNvf4Warps * 32 < K) v[u] = A[(size_t)r * a_stride + k0 + u * kMoeNvf4Warps * 32];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u * kMoeNvf4Warps * 32 < K) a_s[k0 + u * kMoeNvf4Warps * 32] = bf16_bits_to_f32(v[u]);
+    }
     __syncthreads();
     const uint8_t* bdp[2] = {Bd0 + (size_t)e * (K >> 1) * N, NMAT == 2 ? Bd1 + (size_t)e * (K >> 1) * N : nullptr};
     const uint8_t* bsp[2] = {Bs0 + (size_t)e * ((K + 31) >> 5) * N, NMAT == 2 ? Bs1 + (size_t)e * ((K + 31) >> 5) * N : nullptr};
@@ -311,10 +345,10 @@ moe_grouped_gemv_nvf4_kernel(const uint16_t* __restrict__ A, const uint8_t* __re
             for (int m = 0; m < NMAT; ++m) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i)
-                    w[m][i] = CPL == 4 ? __ldg(reinterpret_cast<const uint32_t*>(bdp[m] + (size_t)(blk * 16 + i) * N + c))
-                                       : (uint32_t)__ldg(bdp[m] + (size_t)(blk * 16 + i) * N + c);
-                sw[m] = CPL == 4 ? __ldg(reinterpret_cast<const uint32_t*>(bsp[m] + (size_t)blk * N + c))
-                                 : (uint32_t)__ldg(bsp[m] + (size_t)blk * N + c);
+                    w[m][i] = CPL == 4 ? *reinterpret_cast<const uint32_t*>(bdp[m] + (size_t)(blk * 16 + i) * N + c)
+                                       : (uint32_t)bdp[m][(size_t)(blk * 16 + i) * N + c];
+                sw[m] = CPL == 4 ? *reinterpret_cast<const uint32_t*>(bsp[m] + (size_t)blk * N + c)
+                                 : (uint32_t)bsp[m][(size_t)blk * N + c];
             }
 #pragma unroll
             for (int m = 0; m < NMAT; ++m) {
@@ -346,7 +380,7 @@ moe_grouped_gemv_nvf4_kernel(const uint16_t* __restrict__ A, const uint8_t* __re
                     if (c + j >= N) break;
                     uint32_t b[16];
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) b[i] = __ldg(bdp[m] + (size_t)(blk * 16 + i) * N + c + j);
+                    for (int i = 0; i < 16; ++i) b[i] = bdp[m][(size_t)(blk * 16 + i) * N + c + j];
 #pragma unroll
                     for (int i = 0; i < 16; ++i) {
                         part[j] = fmaf(a_s[blk * 32 + 2 * i], e2m1_to_f32(b[i] & 0xf), part[j]);
@@ -416,7 +450,7 @@ moe_grouped_gemv_nvf4_kernel(const uint16_t* __restrict__ A, const uint8_t* __re
 // the generic kernels above, statement for statement (tests compare the two bit for bit).
 
 // top-k (strict '>', lowest index wins) + softmax over the selected logits + row ids, one warp.
-__global__ void moe_route_t1_kernel(const uint16_t* __restrict__ logits, uint16_t* __restrict__ weights,
+__global__ void moe_route_t1_kernel(const uint16_t* logits, uint16_t* __restrict__ weights,
                                     int32_t* __restrict__ indices, int32_t* __restrict__ row_ids, int E, int k) {
     griddep_wait();
     griddep_launch();
@@ -430,10 +464,10 @@ __global__ void moe_route_t1_kernel(const uint16_t* __restrict__ logits, uint16_
 // gate and up GEMVs of the k routed experts + silu + multiply in one launch: one warp per (slot, n)
 // reads x once for both weight rows.  act = bf16(bf16(silu(bf16 gate)) * bf16 up), the three-launch form.
 template <bool CLEAN>
-__global__ void moe_gateup_fp8_t1_kernel(const uint16_t* __restrict__ x, const uint8_t* __restrict__ Bg,
-                                         const uint16_t* __restrict__ Sg, const uint8_t* __restrict__ Bu,
-                                         const uint16_t* __restrict__ Su, uint16_t* __restrict__ act,
-                                         const int32_t* __restrict__ row_ids, int R, int K, int N, int expert_offset,
+__global__ void moe_gateup_fp8_t1_kernel(const uint16_t* x, const uint8_t* Bg,
+                                         const uint16_t* Sg, const uint8_t* Bu,
+                                         const uint16_t* Su, uint16_t* __restrict__ act,
+                                         const int32_t* row_ids, int R, int K, int N, int expert_offset,
                                          int num_local) {
     griddep_wait();
     griddep_launch();
@@ -463,9 +497,9 @@ __global__ void moe_gateup_fp8_t1_kernel(const uint16_t* __restrict__ x, const u
 // down GEMV of the k routed experts + weighted combine in slot order (+ residual): CTA = cols x k
 // warps, warp (c, s) owns expert row n0+c of slot s; the k rounded results meet in shared memory.
 template <bool CLEAN>
-__global__ void moe_down_combine_fp8_t1_kernel(const uint16_t* __restrict__ act, const uint8_t* __restrict__ Bd,
-                                               const uint16_t* __restrict__ Sd, const uint16_t* __restrict__ weights,
-                                               const int32_t* __restrict__ row_ids, const uint16_t* __restrict__ residual,
+__global__ void moe_down_combine_fp8_t1_kernel(const uint16_t* act, const uint8_t* Bd,
+                                               const uint16_t* Sd, const uint16_t* weights,
+                                               const int32_t* row_ids, const uint16_t* residual,
                                                uint16_t* __restrict__ out, int k, int K, int N, int cols,
                                                int expert_offset, int num_local) {
     __shared__ float part_s[32];
@@ -501,8 +535,8 @@ __global__ void moe_down_combine_fp8_t1_kernel(const uint16_t* __restrict__ act,
 }
 
 // scatter with identity row order (+ residual) for the formats without a fused down kernel
-__global__ void moe_combine_t1_kernel(const uint16_t* __restrict__ expert_out, const uint16_t* __restrict__ weights,
-                                      const uint16_t* __restrict__ residual, uint16_t* __restrict__ out, int H, int k) {
+__global__ void moe_combine_t1_kernel(const uint16_t* expert_out, const uint16_t* weights,
+                                      const uint16_t* residual, uint16_t* __restrict__ out, int H, int k) {
     griddep_wait();
     griddep_launch();
     const int h = blockIdx.x * blockDim.x + threadIdx.x;

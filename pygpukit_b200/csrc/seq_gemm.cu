@@ -469,8 +469,9 @@ int launch_few(const GemmArgs& a, int wdt, int rows_per_block, cudaStream_t st, 
 // 2048, 4 / 16 / 64 columns 14.5 / 25.2 / 84 -> 12.8 / 14.5 / 28.8; two rows per warp 16.4 / 22.7 / 45.2).  The sums' order is that of one warp per row.
 constexpr int SKM = 4, SK_WARPS = 4;
 
+// (One block per SM as the stated least: without it the compiler keeps to 96 registers and half the loads in flight, 14.4 -> 18.5 us at 18 columns.)
 template <int SKN>
-__global__ void __launch_bounds__(SK_WARPS * 32) gemm_skinny_f32_kernel(GemmArgs a) {
+__global__ void __launch_bounds__(SK_WARPS * 32, 1) gemm_skinny_f32_kernel(GemmArgs a) {
     griddep_wait();
     griddep_launch();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -491,9 +492,9 @@ __global__ void __launch_bounds__(SK_WARPS * 32) gemm_skinny_f32_kernel(GemmArgs
     for (int k = lane; k < a.K; k += 32) {
         float xv[SKM], wv[SKN];
 #pragma unroll
-        for (int i = 0; i < SKM; ++i) xv[i] = __ldg(x[i] + k);
+        for (int i = 0; i < SKM; ++i) xv[i] = x[i][k];
 #pragma unroll
-        for (int j = 0; j < SKN; ++j) wv[j] = __ldg(w[j] + k);
+        for (int j = 0; j < SKN; ++j) wv[j] = w[j][k];
 #pragma unroll
         for (int i = 0; i < SKM; ++i)
 #pragma unroll

@@ -42,3 +42,33 @@ def test_tensor_memory_is_held_before_dependents_may_start(where, name, body):
     head = body[:body.index("griddep_launch()")]
     assert "tmem_alloc(" in head, f"{where}: {name} lets its dependents start before it holds its tensor memory"
     assert "__syncthreads()" in head[head.rindex("tmem_alloc("):]
+
+
+def dependents():
+    """Files whose kernels are always launched as dependents, and the headers they share.  (fp8_scan_codes_kernel is launched plainly.)"""
+    sources = [f for f in sorted(CSRC.glob("*.cu")) if re.search(r"launch_waiting\(|ProgrammaticStreamSerialization", strip(f.read_text(encoding="utf-8")))]
+    return sources + [CSRC / "common.cuh", CSRC / "gemv_common.cuh", CSRC / "tc_common.cuh", CSRC / "tma.cuh"]
+
+
+def test_dependent_kernels_do_not_load_through_the_read_only_path():
+    """Their lifetime overlaps that of the kernel which writes what they read."""
+    assert len(dependents()) > 15
+    for f in dependents():
+        text = strip(f.read_text(encoding="utf-8"))
+        for name, _, body in kernels(f):
+            if name == "fp8_scan_codes_kernel":
+                text = text.replace(body, "")
+        assert "__ldg(" not in text and "global.nc" not in text, f.name
+
+
+@pytest.mark.parametrize("where,name,params", [(f.name, n, p) for f in dependents() for n, p, b in kernels(f) if "griddep_wait" in b and "__restrict__" in p],
+                         ids=lambda x: x if len(x) < 40 else "")
+def test_dependent_kernels_load_through_plain_pointers(where, name, params):
+    """__restrict__ lets the compiler move a load ahead of the wait: only pointers that a kernel stores through may have it."""
+    body = next(b for n, p, b in kernels(CSRC / where) if n == name and p == params)
+    assert not re.search(r"const\s+\w+\s*\*\s*__restrict__", params)
+    for p in re.findall(r"\*\s*__restrict__\s+(\w+)", params):
+        uses = re.findall(r"[^;{}]*\b%s\b[^;{}]*" % p, body)
+        assert uses
+        for use in uses:                                     # `p[...] = x`, `*p = x`, a store helper, or a pointer that is stored through
+            assert re.search(r"\b(st|mst<DT>)\(%s\b|\b%s\[.*\]\s*=[^=]|\*%s\s*=[^=]|(?:uint4|uint16_t)\* ?dst\w*\s*=" % (p, p, p), use) or re.fullmatch(r"\s*if \(%s\).*" % p, use), (name, use)

@@ -658,3 +658,60 @@ def test_prompt_attention_without_room_for_records(q_len, ctx):
     ref = f32(want.to_numpy())
     assert (np.abs(x - ref) <= 2.0 ** -7 * np.abs(ref) + 1e-5).all()      # one step of BF16: float32 sums in another order, rounded
     assert run(q_len, got) == 2
+
+
+def test_row_operators_see_what_the_launch_before_wrote():
+    """Launches are brought to the SMs while the one before drains: every operator's rows, weights, indices and counts are written by the
+    launch just before it, call after call without a wait, and come out as when each launch is waited for."""
+    M, H, E, k, rounds, bf = 64, 4096, 8, 2, 5, 2
+    rng = np.random.default_rng(8)
+    gammas = [gk.from_numpy(rng.uniform(0.5, 1.5, H).astype(np.float32)) for _ in range(rounds)]
+    tables = [gk.from_numpy(rng.standard_normal((H, H)).astype(np.float32)) for _ in range(2)]
+    start = gk.from_numpy(rand_bf16(rng, (M, H)))
+
+    def run(wait):
+        g, table = gk.zeros((H,), gk.bfloat16), gk.zeros((H, H), gk.bfloat16)
+        a, b, c, e = (gk.zeros((M, H), gk.bfloat16) for _ in range(4))
+        wide, cache = gk.zeros((M, H), gk.float32), gk.zeros((32, M, 128), gk.bfloat16)
+        tok = gk.zeros((M,), gk.int32)
+        logits, values = gk.zeros((M, E), gk.bfloat16), gk.zeros((M, k), gk.bfloat16)
+        idx, perm, rev, ids = (gk.zeros((M * k,), gk.int32) for _ in range(4))
+        counts, offsets, gathered = gk.zeros((E,), gk.int32), gk.zeros((E + 1,), gk.int32), gk.zeros((M * k, H), gk.bfloat16)
+        d = {n: x.device_ptr for n, x in locals().items() if isinstance(x, gk.GPUArray)}
+        api.memcpy_d2d(d["a"], start.device_ptr, start.nbytes, None)
+        for i in range(rounds):
+            steps = [("cast", gammas[i].device_ptr, d["g"], H, 0, bf), ("rmsnorm", d["a"], d["g"], d["b"], M, H, 1e-5, bf),
+                     ("silu", d["b"], d["c"], M * H, bf), ("mul_inplace", d["c"], d["b"], M * H, bf), ("add", d["c"], d["a"], d["e"], M * H, bf),
+                     ("cast", gammas[-1 - i].device_ptr, d["g"], H, 0, bf), ("bias_add_inplace", d["e"], d["g"], M, H, bf),
+                     ("cast", d["e"], d["wide"], M * H, bf, 0), ("rmsnorm", d["wide"], gammas[i].device_ptr, d["wide"], M, H, 1e-5, 0),
+                     ("cast", d["wide"], d["a"], M * H, 0, bf), ("argmax_rows", d["a"], d["tok"], None, M, H, bf),
+                     ("cast", tables[i % 2].device_ptr, d["table"], H * H, 0, bf), ("embedding_lookup_ptr", d["table"], d["b"], H, d["tok"], M, 2),
+                     ("add_inplace", d["a"], d["b"], M * H, bf), ("kv_cache_update", d["a"], d["cache"], M, 32, 32, 128, M, 0, None, 2),
+                     ("transpose_021", d["cache"], d["c"], 32, M, 128, 2), ("swiglu", d["c"], d["a"], d["e"], M * H, bf),
+                     ("gemv_bf16", d["e"], d["table"], d["logits"], M, H, E), ("moe_topk", d["logits"], d["values"], d["idx"], M, E, k, bf),
+                     ("moe_softmax_topk", d["values"], M, k, bf), ("moe_compute_permutation", d["idx"], d["counts"], d["offsets"], d["perm"], d["rev"], M, E, k),
+                     ("moe_expand_expert_offsets", d["offsets"], d["ids"], E, M * k), ("moe_gather", d["e"], d["perm"], d["gathered"], M, H, k),
+                     ("moe_scatter", d["gathered"], d["values"], d["rev"], d["a"], M, H, k)]
+            for name, *args in steps:
+                getattr(api, name)(*args, None)
+                if wait:
+                    api.device_sync()
+        return [x.to_numpy() for x in (a, b, c, e, wide, cache, tok, logits, values, idx, perm, rev, ids, counts, offsets, gathered)]
+
+    want = run(True)
+    assert np.isfinite(f32(want[0])).all() and len(set(want[9])) > 1
+    for _ in range(3):
+        assert all(np.array_equal(x, y) for x, y in zip(want, run(False)))
+
+
+@pytest.mark.parametrize("tokens,experts,k", [(1, 8, 2), (512, 128, 8), (513, 128, 8), (64, 1024, 4), (64, 1025, 4), (1400, 1500, 3)])
+def test_permutation_of_many_choices_and_experts(tokens, experts, k):
+    """Choices and offsets in shared memory and, beyond 4096 choices or 1024 experts, in the arrays themselves."""
+    n, rng = tokens * k, np.random.default_rng(tokens)
+    ids = rng.integers(0, experts, n).astype(np.int32)
+    gi, counts, offsets, perm, rev = gk.from_numpy(ids), gk.zeros((experts,), gk.int32), gk.zeros((experts + 1,), gk.int32), gk.zeros((n,), gk.int32), gk.zeros((n,), gk.int32)
+    api.moe_compute_permutation(*(a.device_ptr for a in (gi, counts, offsets, perm, rev)), tokens, experts, k, None)
+    want = np.argsort(ids, kind="stable")
+    assert np.array_equal(counts.to_numpy(), np.bincount(ids, minlength=experts))
+    assert np.array_equal(offsets.to_numpy(), np.concatenate([[0], np.cumsum(np.bincount(ids, minlength=experts))]))
+    assert np.array_equal(perm.to_numpy(), want) and np.array_equal(rev.to_numpy()[want], np.arange(n))
