@@ -117,7 +117,7 @@ int pgk_gemv_fp8_swiglu_bf16(const void* A, const void* Wg_nk, const void* Sg, c
 int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void* S, void* C, int M, int K, int N,
                          const void* bias, const void* residual, void* stream);
 
-/* 1 in *out once a wait of the FP8 tensor-core GEMM ran out in this process (its results are then undefined), else 0.  The next call
+/* 1 in *out once a wait of the FP8 tensor-core GEMMs ran out in this process (its results are then undefined), else 0.  The next call
  * that synchronises (pgk_stream_sync, pgk_device_sync, pgk_event_sync) has failed or fails for it. */
 int pgk_gemm_fp8_wait_error(int* out);
 /* The same contract with NO CUDA-core work on the weight stream: raw E4M3 tiles by TMA (cp.async.bulk.tensor, 2-D tensor
@@ -800,7 +800,8 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
                      long long c_batch, int M, int N, int K, int batch, int epilogue, float p0, float p1, const float* col_scale,
                      const void* aux, int aux_dtype, const int32_t* aux_rows, int aux_ld, int aux_off, int rows_per_block,
                      void* stream);
-/* the same for the tensor-core prompt attention (2: its shared memory was not where it needs it) */
+/* the same for the tensor-core kernels of attention over the paged and the fixed cache and of linear attention (2: its shared memory was
+ * not where it needs it) */
 int pgk_seq_attention_wait_error(int* out);
 /* 1 when the tensor-core attention serves such rows of an aligned cache whose requests have at most `positions` positions (pages x page
  * size), else 0: single_query 2 and prompts then take the float32 kernels */

@@ -429,7 +429,7 @@ int sdpa_prompt(const void* Q, const void* K, const void* V, void* out, int hq, 
     p.scale_log2 = scale_log2;
     const PromptPlan plan = prompt_plan(hq, n_kv, q_len, context_len, sm_count());
     p.HB = plan.HB; p.QB = plan.QB; p.hsplit = plan.hsplit; p.splits = plan.splits;
-    p.err = wait_word(kWaitAttention);
+    p.err = wait_word(kWaitPrompt);
     PGK_REQUIRE(p.err, "sdpa_causal_fixed_cache failed: no pinned host memory");
     CUtensorMap kmap, vmap;
     const uint64_t dims[3] = {M_D, (uint64_t)context_len, (uint64_t)n_kv}, strides[2] = {M_D * 2, (uint64_t)max_seq * M_D * 2};

@@ -430,5 +430,6 @@ extern "C" int pgk_gemm_fp8_bf16_tc(const void* A, const void* B_nk, const void*
 extern "C" int pgk_gemm_fp8_wait_error(int* out) {
     PGK_CUDA(cudaDeviceSynchronize());
     *out = pgk::wait_raised(pgk::kWaitFp8);
+    if (*out == 0) *out = pgk::wait_raised(pgk::kWaitFp8Rows);
     return 0;
 }

@@ -488,7 +488,7 @@ int launch_f8rows(F8RowsParams p, const void* A, const void* B0, const void* B1,
     p.mrows = plan.mrows;
     p.m_tiles = (p.M + p.mrows - 1) / p.mrows;
     p.ahead = pdl_enabled();
-    p.err = wait_word(kWaitFp8);
+    p.err = wait_word(kWaitFp8Rows);
     PGK_REQUIRE(p.err, "gemm_fp8 failed: no pinned host memory");
     PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_fp8 failed: the driver does not export cuTensorMapEncodeTiled");
     CUtensorMap wmap, umap, amap;

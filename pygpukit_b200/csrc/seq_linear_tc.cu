@@ -384,7 +384,7 @@ int linear_tc(const float* proj, int ld, int q_off, int k_off, int v_off, float*
         PGK_CUDA(cudaFuncSetAttribute(linear_tc_output_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L_SMEM));
         configured = true;
     }
-    int* err = wait_word(kWaitAttention);
+    int* err = wait_word(kWaitLinear);
     PGK_REQUIRE(err, "seq_linear_attention_chunks failed: no pinned host memory");
     LinTcArgs a{proj, ld, q_off, k_off, v_off, out, ldo, state, decay, (const int4*)seqs, H, D, Dv, begin, end, (end - begin + LT - 1) / LT, ws, err};
     const dim3 grid(a.chunks, n_seqs, H);
