@@ -30,6 +30,17 @@ from ..layers.norm import RowNorm
 from ..paged_cache import PagedKVCache
 
 
+def token_ids(tokens: list) -> np.ndarray:
+    """int(t) of every token, as int32."""
+    try:
+        out = np.asarray(tokens, np.int32)
+        if out.ndim == 1:
+            return out
+    except (TypeError, ValueError):
+        pass
+    return np.asarray([int(t) for t in tokens], np.int32)       # arrays of one element, tensors of a device, and what else int() takes
+
+
 class StepContext:
     """Device-side description of one ragged batch (one int32 upload per step)."""
 
@@ -58,11 +69,7 @@ class StepContext:
         first, rows, slot_of, pos_of = desc.T
         of_row = np.repeat(np.arange(len(seqs)), rows)          # sequence of every row
         within = np.arange(row, dtype=np.int32) - first[of_row]
-        try:
-            tok = np.asarray(toks, np.int32)
-        except (TypeError, ValueError):                         # anything else that int() takes
-            tok = np.asarray([int(t) for t in toks], np.int32)
-        parts = [tok, slot_of[of_row], pos_of[of_row] + within, np.asarray(want_rows, np.int32)]
+        parts = [token_ids(toks), slot_of[of_row], pos_of[of_row] + within, np.asarray(want_rows, np.int32)]
         off = {"tok": 0, "slot": self.T, "pos": 2 * self.T, "want": 3 * self.T}
         cur = 3 * self.T + self.n_want
         self._rows_off = {}

@@ -1,6 +1,8 @@
 """CPU tests of the layered family's host side: config parsing and registry, the page pool (slots and pages
 that are freed and handed out again, growth, truncation), gate/up interleaving, and the NumPy oracle's own
 mechanisms on hand-made cases (so that the oracle the GPU tests lean on is itself pinned)."""
+import warnings
+
 import numpy as np
 import pytest
 
@@ -127,3 +129,20 @@ def test_oracle_attention_prefers_the_standout_key_only_inside_the_chunk():
     assert o[8, 0, 0] > 0.99 and o[8, 0, 1] == 0.0
     o = R.attention_core(q, k, v, scale=1.0, softcap=0.0, chunk=0)
     assert o[8, 0, 1] > 0.99
+
+
+def test_token_ids_are_what_int_makes_of_them():
+    from pygpukit_b200.llm.models.layered import token_ids
+
+    class Id:
+        def __int__(self):
+            return 9
+
+    for tokens in ([1, 2, 3], list(np.arange(4)), [np.int64(7)], [True, 2.0], ["12"], [np.array([5]), np.array([6])], [np.array(5), 6], [Id(), 1], [np.array([[4]])]):
+        with warnings.catch_warnings():
+            warnings.simplefilter("ignore")                  # int() of arrays with one element
+            got = token_ids(tokens)
+            assert got.dtype == np.int32 and got.tolist() == [int(t) for t in tokens]
+    for bad, error in ((["a"], ValueError), ([None], TypeError), ([[1]], TypeError), ([2 ** 31], OverflowError), ([np.array([1, 2])], TypeError)):
+        with pytest.raises(error):
+            token_ids(bad)
