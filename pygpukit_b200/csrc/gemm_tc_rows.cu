@@ -34,9 +34,11 @@ namespace {
 
 constexpr int P_BK = 128;                          // k block = FP8 scale block
 // Warpgroups: two for sums and outputs, two for the conversion, one for copies of codes, copies of activations and the MMAs of two
-// products.  Registers: 256 x 184 + 256 x 40 + 128 x 32 = 640 x 96, the block's at launch.
+// products.  Registers: 256 x 184 + 256 x 40 + 128 x 32 = 640 x 96, the block's at launch (f8rows_config asks for it: with fewer, the
+// warps that want more would wait without end).
 constexpr int P_SUMS = 8, P_CONV = 8;
 constexpr int P_THREADS = (P_SUMS + P_CONV + 4) * 32;
+constexpr int P_SUMS_REGS = 184, P_CONV_REGS = 40, P_REST_REGS = 32, P_REGS = P_SUMS * 32 * P_SUMS_REGS + P_CONV * 32 * P_CONV_REGS + 4 * 32 * P_REST_REGS;
 constexpr int P_CODES_WARP = P_SUMS + P_CONV, P_ROWS_WARP = P_CODES_WARP + 1, P_MMA_WARP = P_CODES_WARP + 2;
 constexpr int P_HALF = 128;                        // activation rows of one product
 constexpr int P_CODES = 4, P_ROWS = 5, P_ACCS = 3;
@@ -122,7 +124,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
     // ahead: whoever has passed ready(g - 2) knows that g - 5, the slot's last user, is read, so no wait takes an older phase for its own.
     auto rows_of = [&](int item) { return min(p.mrows, p.M - (item % p.m_tiles) * p.mrows); };
     if (warp >= P_CODES_WARP) {
-    registers_down<32>();
+    registers_down<P_REST_REGS>();
     if (warp == P_CODES_WARP) {
         // ---------------- codes; weights, so the first ones leave before the dependency wait
         if (elect_one()) {
@@ -220,7 +222,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
     }
     } else if (warp >= P_SUMS) {
         // ---------------- codes -> TMEM
-        registers_down<40>();
+        registers_down<P_CONV_REGS>();
         griddep_wait();
         griddep_launch();
         const int row = (warp & 3) * 32 + lane, kh = (warp - P_SUMS) >> 2;
@@ -258,7 +260,7 @@ gemm_fp8_rows_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_cons
         }
     } else {
         // ---------------- sums and outputs
-        registers_up<184>();
+        registers_up<P_SUMS_REGS>();
         griddep_wait();
         griddep_launch();
         const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane;
@@ -413,6 +415,10 @@ cudaError_t f8rows_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int 
     if (!configured) {
         const cudaError_t e = cudaFuncSetAttribute(gemm_fp8_rows_kernel<PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P_SMEM);
         if (e != cudaSuccess) return e;
+        cudaFuncAttributes fa;
+        const cudaError_t f = cudaFuncGetAttributes(&fa, gemm_fp8_rows_kernel<PAIR>);
+        if (f != cudaSuccess) return f;
+        if (fa.numRegs * P_THREADS < P_REGS) return cudaErrorInvalidConfiguration;
         configured = true;
     }
     cfg->blockDim = dim3(P_THREADS);

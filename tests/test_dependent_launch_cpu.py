@@ -72,3 +72,17 @@ def test_dependent_kernels_load_through_plain_pointers(where, name, params):
         assert uses
         for use in uses:                                     # `p[...] = x`, `*p = x`, a store helper, or a pointer that is stored through
             assert re.search(r"\b(st|mst<DT>)\(%s\b|\b%s\[.*\]\s*=[^=]|\*%s\s*=[^=]|(?:uint4|uint16_t)\* ?dst\w*\s*=" % (p, p, p), use) or re.fullmatch(r"\s*if \(%s\).*" % p, use), (name, use)
+
+
+def test_register_shares_of_a_block_fit_its_launch():
+    """setmaxnreg.inc waits until the block has the registers that others of its warps gave up: a kernel that asks for shares adds them up,
+    fits an SM with them, and refuses to launch where the compiler gave the block fewer."""
+    for f in sorted(CSRC.glob("*.cu")):
+        text = strip(f.read_text(encoding="utf-8"))
+        if "setmaxnreg" not in text:
+            continue
+        names = {n: int(eval(v, {}, {})) for n, v in re.findall(r"\b(P_\w+) = ([0-9]+)(?=[,;])", text)}
+        total = 32 * (names["P_SUMS"] * names["P_SUMS_REGS"] + names["P_CONV"] * names["P_CONV_REGS"] + 4 * names["P_REST_REGS"])
+        assert total <= 65536 and total % (32 * (names["P_SUMS"] + names["P_CONV"] + 4)) == 0
+        assert re.search(r"numRegs \* P_THREADS < P_REGS\) return cudaErrorInvalidConfiguration", text), f.name
+        assert not re.search(r"registers_(?:up|down)<\d", text)
