@@ -92,9 +92,12 @@ class LinearBF16:
 Linear = LinearBF16
 
 
+# PGK_TC_IMPL=2: batches of up to 64 rows multiply the FP8 codes themselves (read once, as pgk_gemv_fp8_bf16 does)
+_RAW_CODES = os.environ.get("PGK_TC_IMPL", "1").strip() == "2"
+
+
 def raw_codes_asked() -> bool:
-    """PGK_TC_IMPL=2: batches of up to 64 rows multiply the FP8 codes themselves (pgk_gemv_fp8_bf16 reads the variable once)."""
-    return os.environ.get("PGK_TC_IMPL", "1").strip() == "2"
+    return _RAW_CODES
 
 
 class LinearFP8:

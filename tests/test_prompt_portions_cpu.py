@@ -1,4 +1,8 @@
 """Which prompts run in portions of 512 rows, and what a feed-forward calls: the Python side of the FP8 path, without a GPU."""
+import os
+import subprocess
+import sys
+
 import pytest
 
 from pygpukit_b200.core.array import GPUArray
@@ -47,9 +51,11 @@ def test_the_other_product_serves_gate_and_up_too(monkeypatch, impl, rows, produ
     """PGK_TC_IMPL=2 selects the product of the codes themselves (up to 64 rows), which has no form for gate and up together; prompts keep
     their slabs then."""
     from pygpukit_b200.llm.layers import linear as linear_module
-    monkeypatch.delenv("PGK_TC_IMPL", raising=False)
-    if impl is not None:
-        monkeypatch.setenv("PGK_TC_IMPL", impl)
+    asked = "import os, sys; sys.path.insert(0, os.getcwd()); from pygpukit_b200.llm.layers.linear import raw_codes_asked; print(raw_codes_asked())"
+    env = {k: v for k, v in os.environ.items() if k != "PGK_TC_IMPL"} | ({} if impl is None else {"PGK_TC_IMPL": impl})
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    assert subprocess.run([sys.executable, "-c", asked], env=env, cwd=root, capture_output=True, text=True).stdout.strip() == str(impl == "2")
+    monkeypatch.setattr(linear_module, "_RAW_CODES", impl == "2")
     m = model(4, 2, 128)
     calls = Calls()
     monkeypatch.setattr(mlp_module, "api", calls)
