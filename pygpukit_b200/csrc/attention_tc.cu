@@ -49,11 +49,6 @@ struct PromptAttnParams {
     int* err;
 };
 
-__device__ __forceinline__ float ex2f(float x) {
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ bool all_wait(int* err, uint32_t bar, uint32_t parity) {
     const bool ok = bar_wait(err, bar, parity);
     return __all_sync(0xffffffffu, ok);
@@ -76,7 +71,7 @@ __device__ __forceinline__ void sum_again(const uint16_t* q, const uint16_t* k, 
             s = fmaf(bf16lo(a.z), bf16lo(b.z), s); s = fmaf(bf16hi(a.z), bf16hi(b.z), s);
             s = fmaf(bf16lo(a.w), bf16lo(b.w), s); s = fmaf(bf16hi(a.w), bf16hi(b.w), s);
         }
-        const float w = ex2f(fmaf(s, scale_log2, neg));
+        const float w = ex2(fmaf(s, scale_log2, neg));
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             const uint4 x = ld_act16(v + (size_t)j * M_D + 8 * i);
@@ -270,7 +265,7 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
                 uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
-                    float a = ex2f(s[c + 2 * e] + neg), b = ex2f(s[c + 2 * e + 1] + neg);
+                    float a = ex2(s[c + 2 * e] + neg), b = ex2(s[c + 2 * e + 1] + neg);
                     l += a + b;
                     hi[e] = cut2(a, b);
                     a = fmaxf(a - bf16lo(hi[e]), tiny);

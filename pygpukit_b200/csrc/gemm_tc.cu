@@ -53,16 +53,6 @@ struct F8TcParams {
     int* err;                                     // raised when a bounded wait runs out
 };
 
-// four e4m3 codes (one 32-bit word) -> four bf16 (two packed words), exact.  (The bits moved by integer instructions and a product
-// with 2^120 for the bias are slower, 55 -> 63 us at 14336 x 14336; with no conversion at all it would be 43.)
-__device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {
-    const uint32_t h0 = e4m3x2_to_f16x2_lo(w), h1 = e4m3x2_to_f16x2_hi(w);
-    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
-    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
-    lo = pack_bf16x2(f0.x, f0.y);
-    hi = pack_bf16x2(f1.x, f1.y);
-}
-
 // PAIR: a tile is 64 rows of a gate and 64 of an up matrix, by turns of 16, so that a lane's partner is 16 lanes on; C = silu(gate) * up
 template <int NB, bool PAIR>
 __global__ void __launch_bounds__(F_THREADS, 2)

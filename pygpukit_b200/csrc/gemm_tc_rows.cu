@@ -56,13 +56,6 @@ struct F8RowsParams {
     int* err;
 };
 
-__device__ __forceinline__ void e4m3x4_to_bf16x4(uint32_t w, uint32_t& lo, uint32_t& hi) {       // exact
-    const uint32_t h0 = e4m3x2_to_f16x2_lo(w), h1 = e4m3x2_to_f16x2_hi(w);
-    const float2 f0 = __half22float2(*reinterpret_cast<const __half2*>(&h0));
-    const float2 f1 = __half22float2(*reinterpret_cast<const __half2*>(&h1));
-    lo = pack_bf16x2(f0.x, f0.y);
-    hi = pack_bf16x2(f1.x, f1.y);
-}
 // two float32 products and sums, each rounded once, by one instruction
 __device__ __forceinline__ void fma2(float& a0, float& a1, float s, float v0, float v1) {
     asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %2};\n\tmov.b64 c, {%3, %4};\n\tfma.rn.f32x2 a, b, c, a;\n\tmov.b64 {%0, %1}, a;\n\t}"

@@ -81,11 +81,6 @@ template <typename F> __device__ __forceinline__ float reduce16(float (&v)[16], 
     }
     return f(v[0], __shfl_xor_sync(0xffffffffu, v[0], 16));
 }
-__device__ __forceinline__ float ex2(float x) {          // 2^x to 2 units, 0 below 2^-126
-    float r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
 __device__ __forceinline__ float max_nan(float a, float b) {       // NaN if either is
     float r;
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
