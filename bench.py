@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""bench.py -- decode tokens/s of the B200 decode hot path (BASELINE.json metric), one JSON line.
+"""bench.py -- decode tokens/s of the B200 decode hot path, one JSON line.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--model llama3-70b] [--format nvf4] [--context 8192] [--batch 1] [--configs all|none]
@@ -8,13 +8,13 @@ A "step" is one greedy decode step (one token per sequence) of the named model a
 -> all layers (fused RMSNorm, W8A16/NVF4 GEMV, QK-norm + RoPE + KV write, split-KV attention, SwiGLU GEMV,
 residual GEMVs) -> final norm -> lm_head GEMV + argmax.
 
-Default workload = BASELINE.json configs[4], north_star's scaling target: Llama-3-70B NVF4 weights, BF16
+Default workload: Llama-3-70B NVF4 weights, BF16
 activations, batch 1, 8k context.  It fits ONE B200 (36 GB of weights), so the same workload is measured at every
-N (tensor parallel, strong scaling) and the driver's 1 -> 8 GPU curve measures the claim itself.  The other
-single-GPU configurations of BASELINE.json ride in the `configs` object of the same line (each with tokens/s and
-the step's HBM roofline fraction): Llama-3-8B FP8 @4k (north_star's >= 70 % target), Qwen3-8B w8a16 @4k
-(configs[1]), Llama-3-8B FP8 @32k at 1 / 8 sequences and @16k at 64 sequences (configs[2]; 64 x 32k of KV cache is
-275 GB and does not fit one B200), Qwen3-30B-A3B NVF4 (configs[3]).
+N (tensor parallel, strong scaling).  The other
+single-GPU configurations ride in the `configs` object of the same line (each with tokens/s and
+the step's HBM roofline fraction): Llama-3-8B FP8 @4k, Qwen3-8B w8a16 @4k,
+Llama-3-8B FP8 @32k at 1 / 8 sequences and @16k at 64 sequences (64 x 32k of KV cache is
+275 GB and does not fit one B200), Qwen3-30B-A3B NVF4.
 
   value   device-timed tokens/s: K replays of the one-graph step with every input resident in HBM
           (CUDA events on the launching stream, barrier + sync on both sides, max over ranks).
@@ -27,7 +27,7 @@ the step's HBM roofline fraction): Llama-3-8B FP8 @4k (north_star's >= 70 % targ
           MEASURED_PEAKS.json hbm_gbs.
   cpu_baseline   oracle/oracle.c (the C restatement of the reference kernels, OpenMP, all host threads) running
           REAL decoder layers of the same shapes on the host for a bounded time; plus, as `config1_reference`,
-          BASELINE.json configs[0] through the reference package itself (oracle/ref_gpt2_cpu.py).
+          GPT-2 small through the reference package itself (oracle/ref_gpt2_cpu.py).
   --impl reference   the CPU arm: K + W real steps, each `layers_per_step` decoder layers + the matching share of
           the lm_head, so that the K timed steps are whole tokens' worth of work; nothing is extrapolated.
 N > 1 (torchrun): tensor-parallel over N GPUs (strong scaling: the same token stream, weights sharded).
@@ -74,7 +74,7 @@ if ROOT not in sys.path:
 import numpy as np  # noqa: E402
 
 FMT_NAME = {"fp8": "w8a16 FP8-E4M3 128x128 block-scaled", "nvf4": "NVF4 (E2M1, UE4M3 scale per 32)", "bf16": "bf16"}
-# (key, model, format, context, batch): the other single-GPU configurations of BASELINE.json
+# (key, model, format, context, batch): the other single-GPU configurations
 SUB_CONFIGS = [
     ("llama3-8b:fp8:4k", "llama3-8b", "fp8", 4096, 1),
     ("qwen3-8b:fp8:4k", "qwen3-8b", "fp8", 4096, 1),
@@ -277,7 +277,7 @@ def cpu_decode_sample(model_name: str, fmt: str, context: int, budget_s: float =
 
 
 def gpt2_reference_cpu(prompt_len: int = 16, new_tokens: int = 8) -> dict:
-    """BASELINE.json configs[0] through the reference package on its CPU backend (separate process: it sets the
+    """GPT-2 small through the reference package on its CPU backend (separate process: it sets the
     reference's global backend).  Bounded: the reference's NumPy path runs ~1 token/s and the full 128 + 128 run takes
     minutes, so the default sample is a short prompt + a few greedy tokens, decode timed apart from the prompt pass."""
     try:

@@ -324,7 +324,7 @@ int pgk_moe_grouped_gemv_nvf4_ex(const void* A, int a_stride, const void* B_data
                                  const int32_t* row_expert_ids, int M, int K, int N, int expert_offset,
                                  int num_local_experts, void* stream);
 
-/* ------------------------------------------------------------------ token sampling on the device (SURVEY 8f-4)
+/* ------------------------------------------------------------------ token sampling on the device
  * sample_token (llm/sampling.py:11-63: temperature -> softmax -> top-k -> top-p -> argmax / draw in index order) for one
  * row of bf16 logits; replaces the D2H of the logits + NumPy that generate() does per token (models/causal.py:62-71) and
  * the reference's sample_token_gpu (ops/sampling.py:11-41 -> native/ops/sampling/sampling.cu:336-362), whose top-k kernel

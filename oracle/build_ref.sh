@@ -3,7 +3,7 @@
 # under /root/reference (nothing is copied into this repo) with the reference's build flags
 # (native/CMakeLists.txt:122: -O3 --use_fast_math --expt-relaxed-constexpr) plus the harness
 # oracle/ref_harness.cu -> oracle/_ref/libref_cuda.so.  Skipped (exit 0) when the reference
-# tree is not mounted (e.g. on the GPU box, which uses the prebuilt .so).
+# tree is not mounted (the prebuilt .so is used there).
 set -euo pipefail
 HERE="$(cd "$(dirname "$0")" && pwd)"
 REF="${PGK_REFERENCE:-/root/reference}"
@@ -33,7 +33,7 @@ nvcc -gencode arch=compute_100a,code=sm_100a -shared -o "$OUT/libref_cuda.so" "$
 echo "built $OUT/libref_cuda.so"
 # The reference's pure-Python package, as it lies, for bench.py's config-1 CPU leg (GPT-2 small through the
 # reference's own CausalTransformerModel.generate on its CPUSimulationBackend).  oracle/_ref/ is git-ignored
-# (never part of this repo's history) but travels to the GPU box, where /root/reference does not exist.
+# (never part of this repo's history) but travels to where the reference's sources are not.
 if [ -d "$REF/src/pygpukit" ]; then
   rm -rf "$OUT/pysrc"; mkdir -p "$OUT/pysrc"
   cp -r "$REF/src/pygpukit" "$OUT/pysrc/pygpukit"

@@ -3,7 +3,7 @@
 Follows `DecodeM1.step` (src/pygpukit/llm/decode/m1.py:40-121) -> `Attention.forward_fixed_cache`
 (llm/layers/attention.py:279-370) -> `_mlp_forward_zero_alloc` (llm/models/causal.py:489-514) ->
 `MoELayer.__call__` (llm/layers/moe.py:153-318), calling the per-kernel restatements of oracle.c in
-the reference's order so that every rounding point of SURVEY.md Appendix A.1 is reproduced:
+the reference's order so that every rounding point is reproduced:
 rmsnorm -> q/k/v GEMV -> [QK-norm] -> RoPE (f32 tables) -> KV write -> SDPA -> o GEMV -> add_inplace
 -> rmsnorm -> gate GEMV -> silu -> up GEMV -> mul_inplace -> down GEMV -> add_inplace -> ... ->
 final rmsnorm -> lm_head -> argmax (first maximum).  lm_head uses the BF16 GEMV restatement

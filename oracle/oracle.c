@@ -1,14 +1,14 @@
 /*
  * oracle.c -- CPU restatement of PyGPUkit's decode hot path (TEST INFRASTRUCTURE).
  *
- * This file is the *checker*, never the product: only tests/, __graft_entry__.smoke()
+ * This file is the oracle, never the product: only tests/, __graft_entry__.smoke()
  * and bench.py's cpu_baseline / --impl reference legs may load it.  The shipped path
  * (pygpukit_b200/) never imports, links or executes anything under oracle/.
  *
  * Every function restates one reference CUDA kernel in plain C, keeping the
  * reference's accumulation ORDER (lane-strided partial sums + shfl_down tree, serial-K,
  * ...) so that results are deterministic and as close to the reference kernels as a
- * CPU can get.  File:line citations are relative to /root/reference.
+ * CPU can get.  File:line citations are relative to the reference's root.
  *
  * Parity pin: (1) tests/golden/*.npz generated from the reference's own Python CPU
  * functions (llm/quant.py, ops/nn/*.py _cpu branches, llm/layers/rope.py,

@@ -1,4 +1,4 @@
-"""TEST / BENCH INFRASTRUCTURE -- BASELINE.json configs[0] on the host cores, through the REFERENCE package itself.
+"""TEST / BENCH INFRASTRUCTURE -- GPT-2 small on the host cores, through the REFERENCE package itself.
 
 GPT-2 small (124M, random init, FP32), 128-token prompt + 128 greedy tokens through the reference's own
 `CausalTransformerModel.generate` (src/pygpukit/llm/models/causal.py:179-255) on its `CPUSimulationBackend`
@@ -89,7 +89,7 @@ def run(prompt_len: int = 128, new_tokens: int = 128, seed: int = 0) -> dict:
             "sample": f"GPT-2 small (124M) random-init FP32 through the reference package's "
                       f"CausalTransformerModel.generate on CPUSimulationBackend (NumPy): {new_tokens} greedy decode tokens "
                       f"after a {prompt_len}-token prompt (prompt pass {t_prompt:.1f} s timed separately and excluded; "
-                      f"BASELINE.json configs[0] is 128 + 128 tokens, which takes ~260 s on 8 cores, so the bench runs "
+                      f"the whole workload is 128 + 128 tokens, which takes ~260 s on 8 cores, so the bench runs "
                       f"this bounded sample of it); package from {root}"}
 
 

@@ -8,7 +8,7 @@
 // scores in shared memory, fails past 12k context) and the FP16-only two-kernel
 // flash_decoding (flash_decoding.cuh:75-377).
 //
-// Design (HBM-bound; DESIGN.md "sdpa_decode"):
+// Design (HBM-bound):
 //   * the cache is read in its UN-expanded [n_kv, max_seq, hd] form: one CTA serves all
 //     G = Hq/n_kv query heads of a KV head (in row tiles of RT), so K/V bytes are fetched
 //     once per group instead of G times (the reference stores and reads the expanded copy).
@@ -383,8 +383,8 @@ static int launch_sdpa(SdpaParams p, cudaStream_t st) {
 
 
 // ---------------------------------------------------------------------------------------------------
-// Fused decode bracket + attention for the q_len == 1, bf16, head_dim 128 case (every config of
-// BASELINE.json): [QK-RMSNorm] -> RoPE -> K/V cache write -> split-KV attention in ONE launch.
+// Fused decode bracket + attention for the q_len == 1, bf16, head_dim 128 case (the benchmark
+// models): [QK-RMSNorm] -> RoPE -> K/V cache write -> split-KV attention in ONE launch.
 // Replaces the chain rmsnorm(q), rmsnorm(k), rope_inplace_f32table, kv_cache_update_gqa x2,
 // sdpa_causal_fixed_cache_ptr of layers/attention.py:326-368 with the same rounding points (q/k rounded
 // to bf16 after the norm and after the rotation, probabilities and the output accumulator in f32).
@@ -416,7 +416,7 @@ struct RopeSdpaParams {
 // ---------------------------------------------------------------------------------------------------------------
 // The score and P.V products run on the tensor cores (mma.sync m16n8k16)
 // and the K/V tiles fetched by tensor-map TMA (cp.async.bulk.tensor.4d, SWIZZLE_128B) so that ldmatrix
-// reads them without bank conflicts.  Decode attention is HBM / latency bound; the CUDA-core loop of round 1 spent 450
+// reads them without bank conflicts.  Decode attention is HBM / latency bound; a CUDA-core loop spent 450
 // issue slots per warp per 64 positions (unpacking V, 15 shuffles of the score reduce-scatter), which bounded the long
 // contexts and the multi-sequence batches.  Here a warp owns 16 positions of a 64-position tile:
 //     S[8 heads (+8 zero rows), 16 pos]  = Q[16, 128] . K^T      16 MMAs, B fragments by ldmatrix from the swizzled tile
@@ -429,7 +429,7 @@ struct RopeSdpaParams {
 // One CTA = 4 consumer warps + 1 TMA producer warp, 2 CTAs per SM; up to 8 query heads per CTA, so a GQA group of 8
 // (Llama-3-70B, Qwen3-30B-A3B) reads its K/V once instead of twice.  Stages: 2 x 32 KB for one sequence -- measured:
 // with 3 stages the two CTAs need 202 KB of shared memory, the SM is switched to its largest carve-out, and the GEMVs
-// that FOLLOW in the step run 8 % slower on the 28 KB of L1 that leaves them (profiles/r02_attn_mma_carveout.txt) --
+// that FOLLOW in the step run 8 % slower on the 28 KB of L1 that leaves them --
 // and 3 x 32 KB for multi-sequence batches, where attention is most of the step.
 constexpr int kMW = 4;                          // consumer warps
 constexpr int kMTile = 64;                      // KV positions per stage

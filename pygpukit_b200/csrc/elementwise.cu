@@ -1,7 +1,7 @@
 // elementwise.cu -- the small ops that bracket the GEMVs in a decode step: RMSNorm /
 // LayerNorm, RoPE, SiLU/GELU, add/mul, bias, cast, embedding gather, argmax, transpose,
 // KV-cache write, and the fused QK-norm + RoPE + KV-write bracket.
-// All f32 math with the reference's rounding points (SURVEY.md Appendix A.1); file:line
+// All f32 math with the reference's rounding points; file:line
 // citations of the reference kernels are on each op.
 #include "common.cuh"
 #include "../../include/pgk_b200.h"

@@ -5,7 +5,7 @@
 //
 // replaces gemv_fp8_warp_reduce_vec4_batched_kernel (fp8_opt.cuh:220-295) and the mma.sync path of
 // pygpukit_w8a16_gemm_sm120 (w8a16_gemm.cu:104-339); on this repo's own path it supersedes gemm_tc.cu, whose converter
-// warps turned every weight byte into BF16 on the CUDA cores (measured 1.2-1.9 TB/s of weight stream, DESIGN.md).
+// warps turned every weight byte into BF16 on the CUDA cores (measured 1.2-1.9 TB/s of weight stream).
 //
 // Design: NO CUDA-core work on the weight stream.
 //   * a pre-kernel (fp8_act_terms_kernel) scales every activation row by a power of two (max |a| -> [128, 256)) and

@@ -5,7 +5,7 @@
 // replaces gemv_fp8_warp_reduce_vec4_kernel / _batched_kernel
 // (native/ops/matmul/gemv/w8a16_bf16/sm120/fp8_opt.cuh:133-295).
 //
-// Design (HBM-bound; see DESIGN.md "gemv_fp8"):
+// Design (HBM-bound):
 //   * one wave: every warp of the grid is resident at once and owns `rho` consecutive
 //     weight rows; the host picks (warps/CTA, CTAs/SM) so that N / (rho * warps) ~ 1.
 //   * weights stream with 256-bit ld.global.L1::no_allocate.L2::evict_first loads, four
@@ -30,11 +30,10 @@
 
 namespace pgk {
 
-// gemm_tc.cu: tcgen05 skinny GEMM for 16 <= M <= 64
+// gemm_tc.cu: tcgen05 GEMM for PGK_TC_MIN_M (5) <= M <= 64, and its form for a gate and an up matrix
 bool gemm_fp8_tc_eligible(int M, int K, int N, const void* A, const void* B);
 int gemm_fp8_tc(const void* A, const void* B_nk, const void* S, void* C, int M, int K, int N, const void* bias,
                 const void* residual, cudaStream_t st);
-
 int gemm_fp8_tc_pair(const void* A, const void* Wg, const void* Sg, const void* Wu, const void* Su, void* C, int M, int K, int N, cudaStream_t st);
 
 // gemm_tc_rows.cu: the same for M > 64; B1: gate and up matrix, silu(gate) * up
@@ -102,7 +101,7 @@ static const bool g_free_hook_registered = (set_free_hook(fp8_codes_forget), tru
 // NMAT = 1: plain GEMV; NMAT = 2: gate/up pair with SiLU*up epilogue.
 //
 // One group (U x 256-bit loads per lane) in flight per warp, up to 16 warps per CTA.  (A register double-buffered
-// form was measured slower on B200 -- 168 registers cap the CTA at 12 warps -- see profiles/r01_*; removed.)
+// form was measured slower on B200 -- 168 registers cap the CTA at 12 warps; removed.)
 // XCHG: the tensor-parallel form with the all-reduce inside (a separate instantiation: the plain kernel pays nothing for it)
 template <int M, int NMAT, bool XCHG = false>
 __global__ void __launch_bounds__(512)
@@ -347,8 +346,9 @@ static bool tp_active_fp8() {
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static bool aligned32(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 31) == 0; }
 
-// Dispatch over M (activation rows).  M > 4 is processed in slabs of <= 4 rows (weights are
-// re-read once per slab; the tcgen05 skinny GEMM takes over for M >= 16, see gemm_w8a16_tc.cu).
+// Dispatch over M (activation rows).  From PGK_TC_MIN_M (5) rows on shapes in multiples of 128 go to the tcgen05 products: gemm_tc.cu
+// to 64 rows, gemm_tc_rows.cu above (gemm_tc_f8.cu to 64 under PGK_TC_IMPL=2).  Other shapes run in slabs of up to 4 rows (2 for gate and
+// up), each of which reads the weights again; weights with the codes 0x7F / 0xFF and odd shapes take the generic kernel.
 static int gemv_fp8_dispatch(const void* A, const void* B0, const void* S0, const void* B1,
                              const void* S1, void* C, int M, int K, int N, const void* bias,
                              const void* residual, bool swiglu, cudaStream_t st, const void* gamma = nullptr,

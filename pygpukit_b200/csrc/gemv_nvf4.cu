@@ -7,7 +7,7 @@
 // replaces gemv_nvf4_bf16_kernel(_unrolled) (native/ops/matmul/gemv/w4a16_bf16/sm120/
 // nvf4_kernels.cu:19-233), which walks K serially with one thread per column.
 //
-// Design (see DESIGN.md "gemv_nvf4"):
+// Design:
 //   * the reference layout is N-contiguous, so lanes own COLS consecutive columns (one
 //     128-bit / 64-bit load = COLS bytes = COLS columns x 2 k) and K is split three ways:
 //     over the 16 byte-rows of a scale block (in flight together), over the warps of a CTA
@@ -404,7 +404,7 @@ static int nvf4_dispatch(const void* A, const void* Bd, const void* Bs, void* C,
     }
     // decode batch >= 5: the tensor-core GEMM reads the weights once for all rows (PGK_TC=0 keeps the slabs of four rows)
     static const bool tc_on = !(getenv("PGK_TC") && atoi(getenv("PGK_TC")) == 0);
-    // measured crossover (profiles/r02_batch_nvf4_*.txt): five rows are still faster as 4 + 1 on the CUDA cores
+    // measured crossover: five rows are still faster as 4 + 1 on the CUDA cores
     if (tc_on && !swiglu && !gamma && M >= gemm_fp8_tc_min_m() + 1 && gemm_nvf4_tc_shape_ok(M, K, N, A, Bd, Bs))
         return gemm_nvf4_tc(A, Bd, Bs, C, M, K, N, alpha, bias, residual, st);
     if (int rc = ensure_workspace(st)) return rc;

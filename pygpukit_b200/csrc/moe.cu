@@ -285,7 +285,7 @@ constexpr int kMoeNvf4Warps = 16;   // 512 threads: 128 registers per thread (32
 // NMAT = 1: C[r, :] = A[r, :] . B[e]      NMAT = 2 (decode gate/up pair): C[r, :] = bf16(bf16(silu(g)) * u) with
 // g = bf16(A . Bg[e]), u = bf16(A . Bu[e]) -- the rounding points of gate GEMV -> silu -> up GEMV -> mul_inplace.
 // (A 32-column CTA form with byte loads and a form that recomputed the routing in every warp were measured slower on
-// B200 and removed; numbers in profiles/r01_bench_qwen3-30b-a3b_*.json and DESIGN.md.)
+// B200 and removed.)
 template <int NMAT>
 __global__ void __launch_bounds__(kMoeNvf4Warps * 32)
 moe_grouped_gemv_nvf4_kernel(const uint16_t* A, const uint8_t* Bd0,

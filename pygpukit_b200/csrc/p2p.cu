@@ -1,6 +1,6 @@
 // p2p.cu -- one-shot all-reduce (+ residual add) over NVLink peer memory for the row-parallel layers of the
-// tensor-parallel decode step (net-new: the reference is single-GPU; SURVEY.md section 8e names this as the
-// replacement of the NCCL all-reduce, whose ~10 us latency per 16 KB message dominates a batch-1 step).
+// tensor-parallel decode step (net-new: the reference is single-GPU; it replaces the
+// NCCL all-reduce, whose ~10 us latency per 16 KB message dominates a batch-1 step).
 //
 //   hidden[M,H] <- bf16( hidden + bf16( sum_r partial_r[M,H] ) )        r = 0 .. world-1, fixed order
 //

@@ -1,4 +1,4 @@
-// sampling.cu -- temperature / top-k / top-p token sampling on the device (SURVEY.md 8f-4).
+// sampling.cu -- temperature / top-k / top-p token sampling on the device.
 //
 // Semantics: pygpukit.llm.sampling.sample_token (llm/sampling.py:11-63), the function generate() calls:
 //   x = logits / T;  p = softmax(x);  top-k: keep the k largest p, renormalise;  top-p: keep the largest p until their

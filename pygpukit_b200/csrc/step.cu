@@ -5,7 +5,7 @@
 // replaces the launch sequence of DecodeM1.step (src/pygpukit/llm/decode/m1.py:40-121) and, on this repo's own
 // path, the 5-launches-per-layer graph of llm/models/causal.py::decode_step_device.
 //
-// Design (HBM-bound; DESIGN.md "step program"):
+// Design (HBM-bound):
 //   * grid = one CTA per SM, 16 consumer warps + 1 producer warp.  The producer walks the SAME op list as the
 //     consumers and streams every byte the CTA will need (weight rows, K/V tiles) into a ring of 8 KB shared-memory
 //     slots with cp.async.bulk (TMA) completing on per-slot mbarriers.  Weights and old KV rows are

@@ -1,6 +1,6 @@
 """pygpukit_b200.llm -- layers, model and decode strategies of the decode hot path (names of
 pygpukit/llm/__init__.py, pinned upstream by tests/test_llm_unified.py:198-239).  The tokenizer, chat templates, the lazy / streaming
-loaders and the weight-repacking pool are out of scope (SURVEY.md section 8); the legacy aliases of
+loaders and the weight-repacking pool are out of scope; the legacy aliases of
 models/causal.py:1496-1501 are provided."""
 from .buffers import DecodeBuffers, PrefillBuffers, RowBuffers
 from .config import (GPT2_SPEC, LLAMA_SPEC, MIXTRAL_SPEC, MODEL_SPECS, QWEN2_SPEC, QWEN3_MOE_SPEC, QWEN3_SPEC,

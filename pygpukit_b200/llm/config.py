@@ -1,7 +1,7 @@
 """Model configuration (mirror of pygpukit/llm/config.py:20-615).
 
 `ModelSpec` here keeps only the architecture flags the decode path reads (the reference's HF
-tensor-name patterns belong to checkpoint loading, which is out of scope: SURVEY.md section 8f-3);
+tensor-name patterns belong to checkpoint loading, llm/loader.py);
 `TransformerConfig` has the reference's fields, defaults and derived properties
 (config.py:440-510) plus `tp_size` / `tp_rank` for the net-new tensor-parallel path.
 """
@@ -187,7 +187,7 @@ class Qwen3Config:
                                  norm_eps=self.rms_norm_eps, rope_theta=self.rope_theta)
 
 
-# ---- the shapes BASELINE.json's configs name (SURVEY.md section 8 header)
+# ---- the shapes of the benchmark models
 def named_config(name: str, max_seq: int = 4096, tp_size: int = 1, tp_rank: int = 0) -> tuple[TransformerConfig, ModelSpec]:
     """(config, spec) of a benchmark model: 'gpt2', 'qwen3-8b', 'llama3-8b', 'llama3-70b', 'qwen3-30b-a3b'
     (and 'tiny-*' variants used by the tests)."""

@@ -2,7 +2,7 @@
 
 Same constructor, attributes (`q_proj/k_proj/v_proj/o_proj`, `q_norm/k_norm`, `_k_cache/_v_cache`,
 `_max_cache_len`, lookahead bookkeeping) and methods (`init_fixed_cache`, `forward_fixed_cache`,
-`forward_fixed_cache_batch`) as the reference.  What changes underneath (SURVEY.md A.4):
+`forward_fixed_cache_batch`) as the reference.  What changes underneath:
   * q/k/v weights are concatenated row-wise into ONE projection for every weight format (rows are
     independent, so results equal the three separate GEMVs the reference runs for FP8,
     attention.py:315-319);

@@ -3,7 +3,7 @@
 LinearBF16 / LinearFP8 keep the reference's constructor arguments, attributes (`weight`,
 `weight_fp8`, `scale_inv`, `bias`, `in_features`, `out_features`, `_use_gemv`) and call
 signature `layer(x, *, out=None)`; LinearNVF4 is net-new (the reference has NVF4 kernels but no
-NVF4 layer).  Differences, all on the dispatch side (SURVEY.md A.4):
+NVF4 layer).  Differences, all on the dispatch side:
   * every batch size 1..64 goes to the weight-streaming GEMV family of libpgk_b200.so, which
     reads the weights once for all rows -- there is no [K,N] transposed copy, no cuBLASLt matmul,
     no CPU dequantisation fallback;

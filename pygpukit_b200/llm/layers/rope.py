@@ -1,6 +1,6 @@
 """RoPE tables (host, NumPy float32) -- must be bit-identical to the reference's
-llm/layers/rope.py:13-24 because token parity at long context depends on the table rounding
-(SURVEY.md Appendix A.3): float32 inverse frequencies, float32 positions, outer product,
+llm/layers/rope.py:13-24 because token parity at long context depends on the table rounding:
+float32 inverse frequencies, float32 positions, outer product,
 cos/sin, each duplicated across the two halves of head_dim."""
 from __future__ import annotations
 

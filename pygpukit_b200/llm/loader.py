@@ -1,4 +1,4 @@
-"""Checkpoint loading for the decode path (mirror of pygpukit/llm/loader.py:132-612; SURVEY.md section 8f-3).
+"""Checkpoint loading for the decode path (mirror of pygpukit/llm/loader.py:132-612).
 
 `load_model_from_safetensors(path, dtype="bfloat16", spec=None)` keeps the reference's entry point: it opens a
 `model.safetensors` file or a `model.safetensors.index.json` shard index, detects the family from the tensor names

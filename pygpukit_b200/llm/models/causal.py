@@ -63,7 +63,7 @@ class CausalTransformerModel:
         self._graph_stream: Stream | None = None
         self._gathered_logits: GPUArray | None = None
         # one-launch step kernel (llm/step_program.py), built on first use when the model fits it.  Opt-in: PGK_STEP=1 or
-        # `use_step_program = True`.  Measured on B200 (DESIGN.md "step program"): its ring streams the BF16 lm_head at the
+        # `use_step_program = True`.  Measured on B200: its ring streams the BF16 lm_head at the
         # HBM peak, but an op boundary inside the kernel (device-side grid barrier + re-staging the activation vector)
         # costs ~7 us against ~3.3 us for a programmatic-dependent-launch boundary, and the CUDA-core dequantisation of the
         # FP8 / NVF4 rows runs at about the HBM rate, so it cannot catch up -- the per-op launches stay the default.
@@ -88,8 +88,8 @@ class CausalTransformerModel:
 
     def init_decode(self, max_seq_len: int, max_batch_size: int = 1, num_sequences: int = 1) -> DecodeBuffers:
         """Allocate the fixed KV caches (all layers), the shared RoPE tables and the step buffers.
-        num_sequences = S > 1: S independent sequences decode together (one row each per step; continuous batching,
-        SURVEY.md section 8f-2): every layer holds S cache regions, position / context are arrays of S."""
+        num_sequences = S > 1: S independent sequences decode together (one row each per step; continuous
+        batching): every layer holds S cache regions, position / context are arrays of S."""
         S = max(1, int(num_sequences))
         if S > 1:
             a0 = self.blocks[0].attn
@@ -551,7 +551,7 @@ class CausalTransformerModel:
                 return
             last = self._decode_step_fixed_cache(nxt, len(tokens) - 1, len(tokens))
 
-    # ------------------------------------------------------------------ self-speculative decode (SURVEY 8f-4)
+    # ------------------------------------------------------------------ self-speculative decode
     def set_lookahead_confirmed_pos(self, pos: int) -> None:
         """Tokens 0 .. pos-1 are committed in every layer's cache (causal.py:1204-1211)."""
         for blk in self.blocks:
@@ -624,7 +624,7 @@ class CausalTransformerModel:
         stats = {"draft_count": len(draft), "accepted_count": sum(1 for a, d in zip(accepted, draft) if a == d)}
         return accepted, stats
 
-    # ------------------------------------------------------------------ Jacobi decode (SURVEY 8f-4)
+    # ------------------------------------------------------------------ Jacobi decode
     def _argmax_tokens(self, hidden: GPUArray, scratch: GPUArray) -> list[int]:
         """greedy token of every row of final-normed hidden states: lm_head + row argmax on the device"""
         M = hidden.shape[0]
@@ -689,7 +689,7 @@ class CausalTransformerModel:
 
     # ------------------------------------------------------------------ accounting
     def weight_bytes_per_token(self) -> int:
-        """Algorithmic weight bytes one decode token streams on this rank (SURVEY.md 8d)."""
+        """Algorithmic weight bytes one decode token streams on this rank."""
         return sum(blk.weight_bytes for blk in self.blocks) + self._head.nbytes + self.final_norm.weight.nbytes
 
     def kv_bytes_per_token(self, context_len: int) -> int:
@@ -699,7 +699,7 @@ class CausalTransformerModel:
 
 GPT2Model = CausalTransformerModel
 LlamaModel = CausalTransformerModel
-QwenModel = CausalTransformerModel   # named by BASELINE.json's north_star; absent upstream
+QwenModel = CausalTransformerModel   # absent upstream
 
 __all__ = ["CausalTransformerModel", "GPT2Model", "LlamaModel", "QwenModel"]
 _ = from_numpy

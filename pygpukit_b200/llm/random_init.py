@@ -1,5 +1,5 @@
 """Random-init models of the benchmark shapes (net-new; the reference only loads checkpoints,
-llm/loader.py:132-612, which is out of scope -- SURVEY.md section 8f-3).
+llm/loader.py:132-612).
 
 BF16 masters N(0, std^2) are drawn on the device (pgk_fill_normal_bf16) and quantised there
 (pgk_quantize_bf16_to_fp8_block / the bit-exact pgk_quantize_bf16_to_nvf4), so an 8B..70B model is
@@ -160,7 +160,7 @@ def build_random_model(name: str = "qwen3-8b", weight_format: str = "fp8", max_s
 
 def _gpt2(name: str, config: TransformerConfig, spec: ModelSpec, weight_format: str, seed: int, std: float,
           world: int, shards: int) -> CausalTransformerModel:
-    """GPT-2 family (BASELINE.json configs[0]): LayerNorm with bias, biased q/k/v/o and fc1/fc2, GELU, learned
+    """GPT-2 family: LayerNorm with bias, biased q/k/v/o and fc1/fc2, GELU, learned
     positions, tied lm_head -- BF16 weights on one GPU (the reference runs it in FP32/FP16; there is no quantised
     GPT-2 checkpoint format upstream)."""
     if weight_format != "bf16" or world > 1 or shards > 1:

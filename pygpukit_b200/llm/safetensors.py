@@ -1,5 +1,5 @@
 """safetensors reader / writer in pure Python + NumPy (mirror of pygpukit/llm/safetensors.py; the reference's
-reader is its Rust mmap loader rust/pygpukit-core/src/llm/tensor_loader.rs, which is out of scope -- SURVEY.md 8f-3).
+reader is its Rust mmap loader rust/pygpukit-core/src/llm/tensor_loader.rs).
 
 File format: 8-byte little-endian header length, a JSON header {name: {dtype, shape, data_offsets}}, then the raw
 tensor bytes.  Tensors are memory-mapped; `tensor(name)` returns a NumPy view (BF16 and FP8 as uint16 / uint8 bit

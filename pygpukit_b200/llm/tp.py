@@ -1,5 +1,5 @@
 """Tensor parallelism for the decode path (net-new: the reference is single-GPU,
-docs/scheduler.md:358; SURVEY.md section 8e).
+docs/scheduler.md:358).
 
 One process per GPU.  Megatron-style sharding decided at weight-creation time:
   column-parallel  q/k/v (heads split), gate/up (intermediate split)   -> no communication

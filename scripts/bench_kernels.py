@@ -1,4 +1,4 @@
-"""Per-kernel achieved HBM GB/s for the decode GEMV family (run on the GPU box).
+"""Per-kernel achieved HBM GB/s for the decode GEMV family (needs a GPU).
 
 Each kernel cycles through a ring of distinct weight buffers larger than L2 (126 MB) so every
 launch streams from HBM; timing = CUDA events around `iters` back-to-back launches."""

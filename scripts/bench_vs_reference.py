@@ -1,6 +1,6 @@
 """Kernel against kernel on the same B200: the REFERENCE's own CUDA kernels (oracle/_ref/libref_cuda.so, compiled
-in place from /root/reference by oracle/build_ref.sh for sm_100a with the reference's flags) next to ours, on the
-shapes of BASELINE.json's configs (SURVEY.md section 8d "Reference-on-B200 baseline").
+in place from the reference's sources by oracle/build_ref.sh for sm_100a with the reference's flags) next to ours, on the
+shapes of the benchmark models.
 
 Timing as src/pygpukit/benchmark/base.py:31-60 prescribes (warm-up, then CUDA events around back-to-back launches on
 the default stream), every launch on a different weight set so the stream comes from HBM (ring >> 126 MB L2).
@@ -18,7 +18,7 @@ from pygpukit_b200._lib import api  # noqa: E402
 from pygpukit_b200.core.stream import CudaEvent, event_elapsed_ms  # noqa: E402
 
 if not refcuda.available():
-    print(json.dumps({"unavailable": "oracle/_ref/libref_cuda.so missing (build it where /root/reference is mounted)"}))
+    print(json.dumps({"unavailable": "oracle/_ref/libref_cuda.so missing (oracle/build_ref.sh builds it from the reference's sources)"}))
     sys.exit(0)
 api.set_pdl(0)                       # plain back-to-back launches on both sides
 refcuda.set_sync(False)

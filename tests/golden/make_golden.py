@@ -1,5 +1,5 @@
 """Generate golden vectors from the REFERENCE's own Python CPU code (run in the build container,
-where /root/reference is mounted; the GPU box only sees the committed .npz).
+where /root/reference is mounted; elsewhere only the committed .npz is seen).
 
     python tests/golden/make_golden.py
 

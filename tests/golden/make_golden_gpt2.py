@@ -1,4 +1,4 @@
-"""Golden run of BASELINE.json configs[0]'s shape of workload (GPT-2, random init, greedy decode on the
+"""Golden run of a small decode workload (GPT-2, random init, greedy decode on the
 reference's NumPy/CPU backend) at test size: the REFERENCE's own CausalTransformerModel.generate on
 CPUSimulationBackend (FP32), in the build container where /root/reference is mounted.
 

@@ -1,5 +1,5 @@
 """Golden vectors for token sampling, produced by the REFERENCE's own function (run in the build container, where
-/root/reference exists; the GPU box only sees the committed .npz):
+/root/reference exists; elsewhere only the committed .npz is seen):
 
     python tests/golden/make_golden_sampling.py
 

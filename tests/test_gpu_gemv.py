@@ -1,6 +1,6 @@
 """GPU parity: weight-only-quantised GEMV family through the C ABI vs the CPU oracle and vs the
 reference's own CUDA kernels (oracle/_ref/libref_cuda.so) on identical seeded inputs.
-Tolerance (north_star): 2e-3 relative for f32-accumulate GEMV outputs (metric of the reference's
+Tolerance: 2e-3 relative for f32-accumulate GEMV outputs (metric of the reference's
 own tests: max|d|/max|ref|); dequantisation / quantisation bit-exact."""
 import numpy as np
 import pytest
@@ -56,7 +56,7 @@ def test_gemm_fp8_tc_vs_oracle(K, N, M):
     """Decode batch (1..)5..64 on tcgen05 (pgk_gemm_fp8_bf16_tc, reached through gemv_fp8_bf16_batched) vs the
     oracle's FP8 GEMV (f32 weights x bf16 activations).  The block scale is folded into the activations and
     rounded to BF16 (the reference's M >= 16 path rounds weight*scale to BF16 instead, w8a16_gemm.cu:104-339):
-    BF16-operand tolerance 1e-2 (north_star); and the slab GEMV (PGK_TC=0 semantics, M rows in slabs of 4)
+    BF16-operand tolerance 1e-2; and the slab GEMV (PGK_TC=0 semantics, M rows in slabs of 4)
     must agree with it to the same bar."""
     if K * N * M > 4096 * 4096 * 16 * 2:
         pytest.skip("oracle time")
@@ -261,7 +261,7 @@ def test_gemv_nvf4_vs_oracle(K, N, M):
 @pytest.mark.parametrize("K,N", [(8192, 1024), (2048, 768), (768, 2048), (1024, 7168), (4096, 512), (96, 40)])
 @pytest.mark.parametrize("M", [5, 8, 16, 32, 64])
 def test_gemv_nvf4_batched_vs_oracle(K, N, M):
-    """NVF4 decode batch 5..64 (batch 1-32) vs the oracle's serial-K restatement of
+    """NVF4 decode batch 5..64 vs the oracle's serial-K restatement of
     gemv_nvf4_bf16_kernel (nvf4_kernels.cu:79-200), row by row.  128-aligned shapes go to the tcgen05 GEMM
     (E2M1 x UE4M3 is exact in BF16, the activations are BF16: exact products, f32 accumulation in TMEM -- the
     f32-accumulate bar 2e-3 applies); the others stay on the CUDA-core GEMV in slabs of 4 rows."""

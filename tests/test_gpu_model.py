@@ -1,5 +1,5 @@
 """End-to-end parity of the decode path against the CPU restatement of the reference's step
-(oracle/model.py): logits within 1e-2 relative (BF16 bar of BASELINE.json), greedy tokens identical,
+(oracle/model.py): logits within 1e-2 relative (BF16), greedy tokens identical,
 graph replay == eager, for FP8 / NVF4 / BF16 weights, QK-norm on/off, dense and MoE."""
 import ctypes as C
 
@@ -14,7 +14,7 @@ from tests.util import f32, rel_err
 pytestmark = pytest.mark.gpu
 
 MAX_SEQ = 160
-N_NEW = 128            # north_star: greedy tokens identical for the first 128 steps
+N_NEW = 128            # greedy tokens identical for the first 128 steps
 
 
 def _build(name, fmt, **kw):
@@ -80,7 +80,7 @@ def test_greedy_tokens_match_oracle(name, fmt, pdl):
 
 
 def _real_width(family: str):
-    """Full hidden size / heads / intermediate size of a BASELINE.json model with 2 layers and a 4096-token vocabulary,
+    """Full hidden size / heads / intermediate size of a benchmark model with 2 layers and a 4096-token vocabulary,
     so the CPU oracle finishes: the shapes every kernel of the step sees are the real ones."""
     from pygpukit_b200.llm.config import named_config
     cfg, spec = named_config(family, max_seq=MAX_SEQ)
@@ -92,7 +92,7 @@ def _real_width(family: str):
                                               ("qwen3-30b-a3b", "nvf4", 128), ("qwen3-30b-a3b", "fp8", 64),
                                               ("llama3-70b", "nvf4", 32)])
 def test_greedy_tokens_match_oracle_real_width(family, fmt, n_new):
-    """One real-width case per model family of BASELINE.json (128 greedy steps; fewer for the widest model, whose
+    """One real-width case per model family of the benchmark (128 greedy steps; fewer for the widest model, whose
     oracle needs ~1.5 s per token on 8 cores), graph replay with PDL on -- the mode bench.py measures."""
     from pygpukit_b200._lib import api
     cfg, spec = _real_width(family)
@@ -244,7 +244,7 @@ def test_moe_decode_form_equals_generic_pipeline(fmt, offset, wide):
             assert np.any(outs[0] != 0)
 
 
-# ---------------------------------------------------------------------------- GPT-2 (BASELINE.json configs[0] family)
+# ---------------------------------------------------------------------------- GPT-2
 def _gpt2_tiny_model():
     """The tiny GPT-2 of tests/golden/gpt2_tiny.py assembled through the reference's constructors
     (Attention with biases, GELU MLP, LayerNorm, learned positions, tied lm_head), BF16 on the GPU."""
@@ -328,7 +328,7 @@ def test_gpt2_position_table_bound():
 
 
 def test_gpt2_small_full_size_graph_equals_eager():
-    """BASELINE.json configs[0] at its full size on the GPU path: GPT-2 small (124M, random init), 128-token prompt +
+    """The GPU path at its full size: GPT-2 small (124M, random init), 128-token prompt +
     128 greedy tokens; the device-resident graph replay and the eager per-op path give the same tokens."""
     model = llm.build_random_model("gpt2", "bf16", max_seq=1024, seed=3, std=0.02)
     assert model.config.num_layers == 12 and model.config.hidden_size == 768 and model.position_embed.shape == (1024, 768)
@@ -344,7 +344,7 @@ def test_gpt2_small_full_size_graph_equals_eager():
 
 @pytest.mark.parametrize("name,fmt,S", [("small-qwen3", "fp8", 3), ("small-qwen3", "nvf4", 3), ("small-qwen3", "fp8", 8)])
 def test_multi_sequence_decode_matches_single_sequence_runs(name, fmt, S):
-    """Multi-sequence decode (SURVEY.md section 8f-2; replaces the reference's unused paged_attention.cuh:46-283 /
+    """Multi-sequence decode (replaces the reference's unused paged_attention.cuh:46-283 /
     continuous_batching.cuh:70-245): S independent sequences with different prompt lengths decode together -- one row
     per sequence through every linear layer, ONE attention launch per layer over the S cache regions with per-sequence
     positions -- and must produce the tokens each sequence produces when it decodes alone (the split-KV fold order and,

@@ -1,7 +1,7 @@
 """GPU parity: norm / RoPE / KV-cache / attention / glue / MoE routing through the C ABI vs the CPU
 oracle and the reference's own CUDA kernels.  Tolerances: bit-exact for copies and index work,
 <= 1 bf16 ulp for elementwise f32 math (fast-math exp/rsqrt in the reference build),
-1e-2 relative for attention (north_star, BF16)."""
+1e-2 relative for attention (BF16)."""
 import ctypes as C
 
 import numpy as np
@@ -197,7 +197,7 @@ def test_oracle_vs_reference_cuda_attention():
 
 @pytest.mark.parametrize("H,Hkv", [(32, 8), (64, 8)])
 def test_sdpa_decode_vs_oracle_32k(H, Hkv):
-    """BASELINE.json configs[2]'s attention at its full size: bf16, head_dim 128, one query token over a 32 768-token
+    """Decode attention at its full size: bf16, head_dim 128, one query token over a 32 768-token
     cache (Llama-3-8B 32/8 heads, Llama-3-70B 64/8), against oracle.c's restatement of sdpa_causal_bf16_kernel
     (attention_kernels.cuh:259-370, OpenMP over heads) on the GQA-expanded cache the reference reads.  BF16 bar 1e-2;
     the context also comes from device memory (_ptr form) and, one token short of the cache, exercises a ragged tail."""

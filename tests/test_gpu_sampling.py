@@ -1,4 +1,4 @@
-"""pgk_sample_token_bf16 (temperature / top-k / top-p sampling on the device, SURVEY 8f-4) against oracle/sampling.py, the
+"""pgk_sample_token_bf16 (temperature / top-k / top-p sampling on the device) against oracle/sampling.py, the
 restatement of pygpukit.llm.sampling.sample_token that tests/test_sampling_oracle.py pins to the reference's own outputs.
 
 Exact comparison on the golden cases (tie-free logits: every cut is unambiguous); on vocabulary-sized random logits,

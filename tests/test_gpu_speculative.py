@@ -1,4 +1,4 @@
-"""Self-speculative decode (SURVEY 8f-4; causal.py:1036-1235, decode/speculative.py): the early layers draft, the full
+"""Self-speculative decode (causal.py:1036-1235, decode/speculative.py): the early layers draft, the full
 model verifies in one batched pass.  Whatever the draft proposes, the emitted tokens are the full model's greedy tokens:
 they are checked against the oracle's greedy continuation with the tie rule of tests/test_gpu_model.py (the batched
 verification pass sums attention in a different order than single steps, so only BF16-resolution ties may differ)."""

@@ -1,6 +1,6 @@
 """GPU parity of the one-launch step kernel (csrc/step.cu, pgk_step_*): every GEMV-type op as a ONE-op program
 must be bit-identical to the per-op entry point it mirrors (same per-row instruction sequence); the NVF4
-row-packed op and the attention op are held to the oracle with the north_star tolerances (2e-3 f32-accumulate
+row-packed op and the attention op are held to the oracle with the oracle's tolerances (2e-3 f32-accumulate
 GEMV, 1e-2 BF16 attention); whole models decode the oracle's greedy tokens through it."""
 import numpy as np
 import pytest
@@ -148,7 +148,7 @@ def _attn_case(rng, hq, n_kv, max_seq, pos, qk_norm):
 @pytest.mark.parametrize("qk_norm", [False, True])
 def test_step_attention_vs_per_op_kernel(hq, n_kv, pos, qk_norm):
     """The attention op (QK-norm + RoPE + KV write + split-KV attention + fold) against pgk_rope_sdpa_decode on the same
-    inputs: same rounding points, different split / fold order -> BF16 outputs within 1e-2 of max (north_star), most
+    inputs: same rounding points, different split / fold order -> BF16 outputs within 1e-2 of max, most
     elements equal; the K/V rows written to the cache are bit-identical."""
     if pos > 1000 and (hq, n_kv) not in ((32, 8), (8, 1)):
         pytest.skip("long contexts on two head layouts")

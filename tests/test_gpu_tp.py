@@ -1,4 +1,4 @@
-"""Tensor-parallel token parity on real GPUs at N = 2 / 4 / 8 (SURVEY.md section 8e): dense FP8, dense NVF4,
+"""Tensor-parallel token parity on real GPUs at N = 2 / 4 / 8: dense FP8, dense NVF4,
 MoE FP8 / NVF4 (experts sharded, un-combined rows exchanged), and a case with more ranks than KV heads (KV heads
 replicated).  Each world size runs ONE torchrun job over all of its cases (tests/tp_worker.py); a test per case
 reads its line.  Self-skips when the box has fewer GPUs than ranks."""

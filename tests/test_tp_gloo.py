@@ -1,6 +1,6 @@
 """Host-side tensor-parallel logic on CPU: two processes over `gloo` (no GPU, no NCCL).
 
-Covers what pygpukit_b200/llm/tp.py decides on the host for N > 1 (SURVEY.md section 8e): the shard plan
+Covers what pygpukit_b200/llm/tp.py decides on the host for N > 1: the shard plan
 partitions every sharded tensor exactly once, the NCCL-id exchange over torch.distributed delivers rank 0's
 payload, a row-parallel layer's partial sums all-reduce to the unsharded product, and the 8-byte-per-rank
 greedy combine picks np.argmax's token (first maximum wins)."""

@@ -1,11 +1,11 @@
-"""Tensor-parallel parity worker (SURVEY.md section 8e "Parity under TP"); launched by tests/test_gpu_tp.py as
+"""Tensor-parallel parity worker; launched by tests/test_gpu_tp.py as
 
     python -m torch.distributed.run --nnodes=1 --nproc-per-node N --master-addr 127.0.0.1 --master-port P \
         tests/tp_worker.py name:format:steps[:layers] [more cases ...]
 
 Every rank builds its shard of the random-init model (piece `rank` of N); rank 0 additionally builds the SAME
 global model in one process (`shards=N` concatenates the N pieces).  Both decode greedily from the same prompt.
-The all-reduce changes the summation order of the row-parallel projections, so the check is north_star's:
+The all-reduce changes the summation order of the row-parallel projections, so the check is:
 identical greedy tokens for `steps` steps, unless the single-GPU top-2 logit margin at the first divergence is
 below 2^-5 (a tie at BF16 logit resolution).  Rank 0 prints one JSON line per case; exit code 1 on a real mismatch."""
 import json

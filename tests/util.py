@@ -1,4 +1,4 @@
-"""Shared synthetic-data helpers for the tests (seeded, SURVEY.md section 8d)."""
+"""Shared synthetic-data helpers for the tests (seeded)."""
 import numpy as np
 
 from pygpukit_b200.core.dtypes import bf16_bits_to_f32, f32_to_bf16_bits
