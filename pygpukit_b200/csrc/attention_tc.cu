@@ -314,10 +314,10 @@ sdpa_prompt_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_consta
 #pragma unroll
                 for (int e = 0; e < 16; ++e) o[e] = 0.f;
             }
-            bool none = false;
+            bool nan = false;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) none |= o[e] != o[e];
-            uint32_t rows = __ballot_sync(0xffffffffu, live && none && limit + 1 < end);
+            for (int e = 0; e < 16; ++e) nan |= o[e] != o[e];
+            uint32_t rows = __ballot_sync(0xffffffffu, live && nan && limit + 1 < end);
 #pragma unroll 1
             while (rows) {
                 const int s = __ffs(rows) - 1, r = quad * 32 + s, sh = r / p.QB, sq = r - sh * p.QB;
