@@ -157,7 +157,7 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 // What a kernel that is launched as a dependent reads may have been written by the kernel before, whose lifetime overlaps its own:
 // weights, too, unless pdl_enabled().  So no such kernel loads through the read-only path (.nc, __ldg), which is for what nobody writes
 // meanwhile, and no pointer that it loads through is __restrict__, which lets the compiler choose that path and move the load ahead
-// of griddep_wait; a pointer that is only stored through may be.
+// of griddep_wait; a pointer that is only stored through may be.  Kernels that are dependents under pdl_enabled() only read weights so.
 
 // streaming loads: do not allocate in L1, evict-first in L2 (weights are touched once per token).  sm_100a has 256-bit global loads.
 struct alignas(32) u32x8 { uint32_t v[8]; };

@@ -49,7 +49,7 @@ struct F8Params {
 };
 
 // ---- activation rows -> two E4M3 terms, in the B operand's shared-memory image (one CTA per padded row)
-__global__ void __launch_bounds__(256) fp8_act_terms_kernel(const uint16_t* __restrict__ A, uint8_t* __restrict__ img,
+__global__ void __launch_bounds__(256) fp8_act_terms_kernel(const uint16_t* A, uint8_t* __restrict__ img,
                                                             float* __restrict__ unshift, int M, int K, int mpad) {
     __shared__ uint32_t red[8];
     griddep_wait();
@@ -251,7 +251,7 @@ gemm_fp8_f8mma_kernel(const __grid_constant__ CUtensorMap wmap, F8Params p) {
 #pragma unroll
         for (int m = 0; m < MP; ++m) {
             if (m >= p.M) break;
-            const float x0 = acc[m] * __ldg(p.unshift + m);
+            const float x0 = acc[m] * p.unshift[m];
             if (p.splits == 1) {
                 float x = x0;
                 const size_t o = (size_t)m * p.N + n;

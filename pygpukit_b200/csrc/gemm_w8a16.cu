@@ -17,7 +17,7 @@ namespace pgk {
 constexpr int kGW = 8;   // warps per CTA (K split)
 template <int MT>
 __global__ void __launch_bounds__(kGW * 32)
-w8a16_gemm_kn_kernel(const uint16_t* __restrict__ A, const uint8_t* __restrict__ B, const uint16_t* __restrict__ S,
+w8a16_gemm_kn_kernel(const uint16_t* A, const uint8_t* __restrict__ B, const uint16_t* __restrict__ S,
                      uint16_t* __restrict__ C, int M, int K, int N) {
     __shared__ float red[kGW][MT][128];
     griddep_wait();

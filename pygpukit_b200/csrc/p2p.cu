@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(1024) p2p_ll_allreduce_add_kernel(P2pLLParams 
 // greedy token of a vocabulary-sharded lm_head: every rank publishes (its best logit, global index) as two LL words and
 // takes the maximum of all keys (identical on every rank; the lowest index wins ties) -- 16 bytes per rank instead of
 // an all-gather of the logits
-__global__ void p2p_ll_argmax_kernel(const uint16_t* __restrict__ logits, int32_t* token_buf, int vocab_offset, P2pLLParams p) {
+__global__ void p2p_ll_argmax_kernel(const uint16_t* logits, int32_t* token_buf, int vocab_offset, P2pLLParams p) {
     griddep_wait();
     griddep_launch();
     if (threadIdx.x != 0) return;

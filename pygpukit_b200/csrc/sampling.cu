@@ -55,12 +55,12 @@ __device__ __forceinline__ float smp_key_value(uint32_t k) {          // inverse
 // eight consecutive logits of (warp, iteration, lane); positions >= V read as -inf and are flagged by their index
 __device__ __forceinline__ void smp_load8(const SmpParams& p, int base, uint32_t (&b)[8]) {
     if (base + 8 <= p.V) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(p.logits + base));
+        const uint4 v = *reinterpret_cast<const uint4*>(p.logits + base);
         b[0] = v.x & 0xffffu; b[1] = v.x >> 16; b[2] = v.y & 0xffffu; b[3] = v.y >> 16;
         b[4] = v.z & 0xffffu; b[5] = v.z >> 16; b[6] = v.w & 0xffffu; b[7] = v.w >> 16;
     } else {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) b[q] = (base + q < p.V) ? (uint32_t)__ldg(p.logits + base + q) : 0xff80u;
+        for (int q = 0; q < 8; ++q) b[q] = (base + q < p.V) ? (uint32_t)p.logits[base + q] : 0xff80u;
     }
 }
 
@@ -164,7 +164,7 @@ __device__ __forceinline__ void smp_foreach(const SmpParams& p, F f) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const int base = base0 + (i0 + j) * 256;
-            if (i0 + j < p.iters && base + 8 <= p.V) v[j] = __ldg(reinterpret_cast<const uint4*>(p.logits + base));
+            if (i0 + j < p.iters && base + 8 <= p.V) v[j] = *reinterpret_cast<const uint4*>(p.logits + base);
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(256) gla_scan_kernel(ChunkArgs p) {
 #pragma unroll
         for (int i = 0; i < B; ++i) {
             add[i] = c + i < n ? __ldcg(u + (size_t)(c + i) * step) : 0.f;
-            dec[i] = c + i < n ? __ldg(dc + (size_t)(c + i) * step) : 0.f;
+            dec[i] = c + i < n ? dc[(size_t)(c + i) * step] : 0.f;
         }
 #pragma unroll
         for (int i = 0; i < B; ++i)
@@ -397,7 +397,7 @@ __device__ __forceinline__ void stage_transposed(const float* src, size_t ld, in
         for (int d0 = dl; d0 < D; d0 += 8 * B) {
             float r[B];
 #pragma unroll
-            for (int b = 0; b < B; ++b) r[b] = (in && d0 + 8 * b < D) ? __ldg(row + d0 + 8 * b) : 0.f;
+            for (int b = 0; b < B; ++b) r[b] = (in && d0 + 8 * b < D) ? row[d0 + 8 * b] : 0.f;
 #pragma unroll
             for (int b = 0; b < B; ++b)
                 if (d0 + 8 * b < D) dst[at_dt<MC>(d0 + 8 * b, t)] = r[b] * mult;

@@ -390,7 +390,7 @@ __device__ __forceinline__ void stage_transposed(const float* src, int ld, int n
 #pragma unroll
         for (int b = 0; b < B; ++b) {
             const int u = u0 + 8 * b, d = (u % nd) * 8 + dl, t = (u / nd) * 4 + tl;
-            r[b] = (d < D && t < nc) ? __ldg(src + (size_t)t * ld + d) : 0.f;
+            r[b] = (d < D && t < nc) ? src[(size_t)t * ld + d] : 0.f;
         }
 #pragma unroll
         for (int b = 0; b < B; ++b) {
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(256, 2) mlstm_output_kernel(ChunkArgs p) {
         for (int s = q; s <= t; s += 4) x += At[s * MP + t];
         if (has_state)
 #pragma unroll 8
-            for (int d = q; d < D; d += 4) y = fmaf(Qt[d * MP + t], __ldg(Nc + d), y);
+            for (int d = q; d < D; d += 4) y = fmaf(Qt[d * MP + t], Nc[d], y);
         x = fmaf(y, win[t], x);
         x += __shfl_xor_sync(0xffffffffu, x, 1);
         x += __shfl_xor_sync(0xffffffffu, x, 2);

@@ -61,6 +61,15 @@ def test_dependent_kernels_do_not_load_through_the_read_only_path():
         assert "__ldg(" not in text and "global.nc" not in text, f.name
 
 
+def test_other_kernels_read_only_weights_through_the_read_only_path():
+    """Kernels that are dependents under set_pdl alone: weights are older than the launch before, rows are not."""
+    weights = {"gemm_tc_f8.cu": ["p.S"], "gemm_w8a16.cu": ["reinterpret_cast<const uint32_t*>(B"], "gemv_fp8.cu": ["reinterpret_cast<const uint4*>(B)"],
+               "seq_gla.cu": ["wp", "a.w2"], "step.cu": ["gv", "(t ? sj.S1", "gamma", "cs", "sn"]}
+    for f in sorted([*CSRC.glob("*.cu"), *CSRC.glob("*.cuh")]):
+        for arg in re.findall(r"__ldg\(([^;]*)", strip(f.read_text(encoding="utf-8"))):
+            assert any(arg.startswith(w) for w in weights.get(f.name, [])), (f.name, arg)
+
+
 @pytest.mark.parametrize("where,name,params", [(f.name, n, p) for f in dependents() for n, p, b in kernels(f) if "griddep_wait" in b and "__restrict__" in p],
                          ids=lambda x: x if len(x) < 40 else "")
 def test_dependent_kernels_load_through_plain_pointers(where, name, params):
