@@ -16,33 +16,18 @@
 // reduced to [-pi, pi] in double (positions reach thousands, where a float32 product has lost four digits), sine and cosine
 // in float32.  Dimensions from `rot_dims` on pass unchanged.
 #include "common.cuh"
+#include "seq_rows.cuh"
 #include "../../include/pgk_b200.h"
 
 using namespace pgk;
 
 namespace {
 
-template <typename TC> __device__ __forceinline__ void cstore(TC* p, float v);
-template <> __device__ __forceinline__ void cstore<float>(float* p, float v) { *p = v; }
-template <> __device__ __forceinline__ void cstore<uint16_t>(uint16_t* p, float v) { *p = f32_to_bf16_bits(v); }
-
 __device__ __forceinline__ void angle_sincos(int pos, double inv_freq, float& sn, float& cs) {
     const double a = (double)pos * inv_freq;
     const double two_pi = 6.283185307179586476925286766559;
     const float r = (float)(a - two_pi * rint(a / two_pi));
     sincosf(r, &sn, &cs);
-}
-
-__device__ __forceinline__ float block_sum_256(float v, float* red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    v = warp_sum(v);
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) s += red[i];
-    return s;
 }
 
 struct LatentPrepArgs {
@@ -55,40 +40,77 @@ struct LatentPrepArgs {
     float mult;                                       // factor on cosine and sine
 };
 
-template <typename TC>
-__device__ __forceinline__ void latent_row(const LatentPrepArgs& a, int t, float* red) {
+// What bounds a row is its chain of loads: both latents, their weights, the position's way to its cache row and the angles go out together and
+// are held in registers (B200, us, ranks 768 and 512, one element per access and two barriers -> here: 2000 tokens 14.5 -> 11.5, 8 tokens 8.2 ->
+// 3.8).  VEC: 16-byte accesses; up to 2048 elements of a latent are held, longer ones are read again.
+template <typename TC, bool VEC>
+__device__ __forceinline__ void latent_row(const LatentPrepArgs& a, int t, float (*red)[32]) {
+    constexpr int G = 2;
     float* dq = a.proj + (size_t)t * a.ld;
     const float* dkv = dq + a.kv_off;
-    float sq = 0.f, sc = 0.f;
-    for (int i = threadIdx.x; i < a.q_rank; i += blockDim.x) sq = fmaf(dq[i], dq[i], sq);
-    for (int i = threadIdx.x; i < a.rank; i += blockDim.x) sc = fmaf(dkv[i], dkv[i], sc);
-    sq = block_sum_256(sq, red);
-    sc = block_sum_256(sc, red);
-    const float iq = a.q_rank > 0 ? 1.f / sqrtf(sq / (float)a.q_rank + a.eps) : 0.f;
-    const float ic = 1.f / sqrtf(sc / (float)a.rank + a.eps);
-    for (int i = threadIdx.x; i < a.q_rank; i += blockDim.x) dq[i] = dq[i] * iq * (a.w_off + a.qw[i]);
-    const int pos = a.pos[t], slot = a.slot[t];
+    const int pos = a.pos[t], slot = a.slot[t], half = a.rot_dims / 2;
+    const bool held = a.q_rank <= 4 * G * 256 && a.rank <= 4 * G * 256;
+    const float* kr = dkv + a.rank;
+    const int pair = 255 - (int)threadIdx.x;              // the last threads turn: the first ones have most of the latents
+    float sn = 0.f, cs = 0.f, u = 0.f, v = 0.f;
+    if (pair < half) {
+        u = kr[2 * pair]; v = kr[2 * pair + 1];
+        angle_sincos(pos, a.inv_freq[pair], sn, cs);
+    }
+    float x[4 * G], y[4 * G], w[4 * G], z[4 * G], sq = 0.f, sc = 0.f;
+    if (held) {
+        row_load<VEC, G>(x, dq, a.q_rank);
+        row_load<VEC, G>(y, dkv, a.rank);
+        row_load<VEC, G>(w, a.qw, a.q_rank);
+        row_load<VEC, G>(z, a.cw, a.rank);
+        sq = square_sum(x);
+        sc = square_sum(y);
+    } else {
+        for (int i = threadIdx.x; i < a.q_rank; i += blockDim.x) sq = fmaf(dq[i], dq[i], sq);
+        for (int i = threadIdx.x; i < a.rank; i += blockDim.x) sc = fmaf(dkv[i], dkv[i], sc);
+    }
     const int page = a.table[(size_t)slot * a.max_pages + pos / a.PS], r = pos % a.PS;
     TC* dst = (TC*)a.kc + ((size_t)page * a.PS + r) * (a.rank + a.rot);
-    for (int i = threadIdx.x; i < a.rank; i += blockDim.x) cstore<TC>(dst + i, dkv[i] * ic * (a.w_off + a.cw[i]));
-    const float* kr = dkv + a.rank;
-    for (int i = threadIdx.x; i < a.rot_dims / 2; i += blockDim.x) {
-        float sn, cs;
-        angle_sincos(pos, a.inv_freq[i], sn, cs);
-        sn *= a.mult; cs *= a.mult;
-        const float u = kr[2 * i], v = kr[2 * i + 1];
-        cstore<TC>(dst + a.rank + 2 * i, u * cs - v * sn);
-        cstore<TC>(dst + a.rank + 2 * i + 1, v * cs + u * sn);
+    row_sums(sq, sc, red);
+    const float iq = a.q_rank > 0 ? 1.f / sqrtf(row_total(red[0]) / (float)a.q_rank + a.eps) : 0.f;
+    const float ic = 1.f / sqrtf(row_total(red[1]) / (float)a.rank + a.eps);
+    if (held) {
+#pragma unroll
+        for (int j = 0; j < 4 * G; ++j) { x[j] = x[j] * iq * (a.w_off + w[j]); y[j] = y[j] * ic * (a.w_off + z[j]); }
+        row_store<VEC, G>(dq, x, a.q_rank);
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (VEC) {
+                const float v[4] = {y[4 * g], y[4 * g + 1], y[4 * g + 2], y[4 * g + 3]};
+                const int i = row_at<VEC, G>(g, 0);
+                if (i < a.rank) store4(dst + i, v);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { const int i = row_at<VEC, G>(g, e); if (i < a.rank) store1(dst + i, y[4 * g + e]); }
+            }
+        }
+    } else {
+        for (int i = threadIdx.x; i < a.q_rank; i += blockDim.x) dq[i] = dq[i] * iq * (a.w_off + a.qw[i]);
+        for (int i = threadIdx.x; i < a.rank; i += blockDim.x) store1(dst + i, dkv[i] * ic * (a.w_off + a.cw[i]));
     }
-    for (int i = a.rot_dims + threadIdx.x; i < a.rot; i += blockDim.x) cstore<TC>(dst + a.rank + i, kr[i]);
+    for (int i = pair; i < half; i += 256) {
+        if (i != pair) {
+            u = kr[2 * i]; v = kr[2 * i + 1];
+            angle_sincos(pos, a.inv_freq[i], sn, cs);
+        }
+        sn *= a.mult; cs *= a.mult;
+        store1(dst + a.rank + 2 * i, u * cs - v * sn);
+        store1(dst + a.rank + 2 * i + 1, v * cs + u * sn);
+    }
+    for (int i = a.rot_dims + threadIdx.x; i < a.rot; i += blockDim.x) store1(dst + a.rank + i, kr[i]);
 }
 
-template <typename TC>
+template <typename TC, bool VEC>
 __global__ void __launch_bounds__(256) latent_prep_kernel(LatentPrepArgs a) {
     griddep_wait();
     griddep_launch();
-    __shared__ float red[8];
-    latent_row<TC>(a, blockIdx.x, red);
+    __shared__ float red[2][32];
+    latent_row<TC, VEC>(a, blockIdx.x, red);
 }
 
 struct RopeHeadsArgs {
@@ -128,11 +150,16 @@ __global__ void __launch_bounds__(256) rope_heads_kernel(RopeHeadsArgs a) {
 }
 
 // blocks (t, 0 .. parts - 1): query tails; block (t, parts), when there is one: the cache row
-template <typename TC>
+template <typename TC, bool VEC>
 __global__ void __launch_bounds__(256) latent_prep_heads_kernel(LatentPrepArgs p, RopeHeadsArgs a, int parts) {
-    __shared__ float red[8];
+    __shared__ float red[2][32];
     if ((int)blockIdx.y < parts) rope_tails(a, blockIdx.x, blockIdx.y, parts);
-    else latent_row<TC>(p, blockIdx.x, red);
+    else latent_row<TC, VEC>(p, blockIdx.x, red);
+}
+
+// whether the latents of every token and their cache rows keep 16-byte (bfloat16 cache: 8-byte) boundaries
+bool latent_vec(const LatentPrepArgs& a) {
+    return a.ld % 4 == 0 && a.kv_off % 4 == 0 && a.q_rank % 4 == 0 && a.rot % 4 == 0 && row_vec(a.rank, {a.proj, a.qw, a.cw, a.kc});
 }
 
 }  // namespace
@@ -149,8 +176,9 @@ int pgk_seq_latent_prep(float* proj, int ld, int tokens, int q_rank, int kv_off,
     if (tokens <= 0) return 0;
     LatentPrepArgs a{proj, ld, q_rank, rank, rot, rot_dims, kv_off, q_weight, c_weight, weight_offset, eps, inv_freq, k_cache,
                      table, max_pages, page_size, slot, pos, 1.f};
-    if (cache_dtype == 2) PGK_CUDA(launch_waiting(latent_prep_kernel<uint16_t>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
-    else PGK_CUDA(launch_waiting(latent_prep_kernel<float>, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
+    const auto kernel = cache_dtype == 2 ? (latent_vec(a) ? latent_prep_kernel<uint16_t, true> : latent_prep_kernel<uint16_t, false>)
+                                         : (latent_vec(a) ? latent_prep_kernel<float, true> : latent_prep_kernel<float, false>);
+    PGK_CUDA(launch_waiting(kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
 
@@ -180,8 +208,9 @@ int pgk_seq_latent_prep_heads(float* proj, int ld, int tokens, int q_head, int q
     const int parts = rot == 0 ? 0 : (tokens <= 32 ? (heads * rot / 2 + 255) / 256 : 1);
     const dim3 grid(tokens, parts + (rank > 0 ? 1 : 0));
     if (grid.y == 0) return 0;
-    if (cache_dtype == 2) PGK_CUDA(launch(latent_prep_heads_kernel<uint16_t>, grid, dim3(256), 0, (cudaStream_t)stream, p, a, parts));
-    else PGK_CUDA(launch(latent_prep_heads_kernel<float>, grid, dim3(256), 0, (cudaStream_t)stream, p, a, parts));
+    const auto kernel = cache_dtype == 2 ? (latent_vec(p) ? latent_prep_heads_kernel<uint16_t, true> : latent_prep_heads_kernel<uint16_t, false>)
+                                         : (latent_vec(p) ? latent_prep_heads_kernel<float, true> : latent_prep_heads_kernel<float, false>);
+    PGK_CUDA(launch(kernel, grid, dim3(256), 0, (cudaStream_t)stream, p, a, parts));
     return 0;
 }
 

@@ -17,6 +17,7 @@
 //   linear_finish      the heads' outputs divided by their root mean square (over all heads with a weight, or head by head
 //                      without one), times sigmoid or silu of the gate columns, times a constant.
 #include "common.cuh"
+#include "seq_rows.cuh"
 #include "../../include/pgk_b200.h"
 
 namespace pgk {
@@ -68,35 +69,62 @@ __global__ void __launch_bounds__(256) causal_conv_rows_kernel(ConvArgs a) {
     if (tail_row) rout[(size_t)(p % ring) * W + c] = hv;
 }
 
-// Many rows and at most CTAPS taps: a thread takes CROWS consecutive rows of its column, their inputs loaded once and all together
-// -- a block per row waits for its slot, then for its inputs, and reads each of them once per tap (a linear-attention
-// prompt of 2000 tokens: 38 -> 24 us).  Sums, rings and their order as above.
+// Many rows and at most CTAPS taps: a thread takes CROWS consecutive rows of its V columns, their inputs loaded once and all together
+// -- a block per row waits for its slot, then for its inputs, and reads each of them once per tap.  Four columns per thread where rows
+// allow 16-byte accesses: the taps of a column and the slots of the rows are read for four of them (a linear-attention prompt of 2000
+// tokens, width 2048: a block per row 38 us, V = 1 25.4, V = 4 12.7).  Sums, rings and their order as above.
 constexpr int CTAPS = 4, CROWS = 4;
 
-__global__ void __launch_bounds__(256) causal_conv_many_kernel(ConvArgs a) {
+template <int V> __device__ __forceinline__ void cols_load(float (&v)[V], const float* p) {
+    if constexpr (V == 4) *(float4*)v = *(const float4*)p;
+    else v[0] = *p;
+}
+template <int V> __device__ __forceinline__ void cols_store(float* p, const float (&v)[V]) {
+    if constexpr (V == 4) *(float4*)p = *(const float4*)v;
+    else *p = v[0];
+}
+
+template <int V>
+__global__ void __launch_bounds__(128) causal_conv_many_kernel(ConvArgs a) {
     griddep_wait();
     griddep_launch();
-    const int t0 = blockIdx.x * CROWS, c = blockIdx.y * 256 + threadIdx.x;
+    const int t0 = blockIdx.x * CROWS, c = (blockIdx.y * 128 + threadIdx.x) * V;
     if (c >= a.W) return;
     const int ring = a.taps - 1, W = a.W;
     const bool twice = a.parity != nullptr;
     constexpr int BACK = CTAPS - 1;
-    float hv[CROWS + BACK], wk[CTAPS], out[CROWS];
+    float hv[CROWS + BACK][V], wk[CTAPS][V], out[CROWS][V];
     int sl[CROWS + 2 * BACK], ps[CROWS], pr[CROWS];
 #pragma unroll
     for (int j = 0; j < CROWS + 2 * BACK; ++j) {
         const int t = t0 - BACK + j;
         const bool in = t >= 0 && t < a.T;
         sl[j] = in ? a.slot[t] : -1;
-        if (j < CROWS + BACK) hv[j] = in ? a.h[(size_t)t * a.ldh + c] : 0.f;
+        if (j < CROWS + BACK) {
+            if (in) cols_load<V>(hv[j], a.h + (size_t)t * a.ldh + c);
+            else {
+#pragma unroll
+                for (int e = 0; e < V; ++e) hv[j][e] = 0.f;
+            }
+        }
     }
 #pragma unroll
     for (int r = 0; r < CROWS; ++r) {
         ps[r] = t0 + r < a.T ? a.pos[t0 + r] : 0;
         pr[r] = twice && t0 + r < a.T ? a.parity[t0 + r] & 1 : 0;
     }
+    if (V == 4 && a.taps == CTAPS) {                      // the weights of four columns are sixteen neighbours
 #pragma unroll
-    for (int k = 0; k < CTAPS; ++k) wk[k] = k < a.taps ? a.w[(size_t)c * a.taps + a.taps - 1 - k] : 0.f;
+        for (int e = 0; e < V; ++e) {
+            const float4 w = *(const float4*)(a.w + (size_t)(c + e) * CTAPS);
+            wk[3][e] = w.x; wk[2][e] = w.y; wk[1][e] = w.z; wk[0][e] = w.w;
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < CTAPS; ++k)
+#pragma unroll
+            for (int e = 0; e < V; ++e) wk[k][e] = k < a.taps ? a.w[(size_t)(c + e) * a.taps + a.taps - 1 - k] : 0.f;
+    }
 #pragma unroll
     for (int r = 0; r < CROWS; ++r) {
         const int t = t0 + r, s = sl[r + BACK], p = ps[r];
@@ -104,27 +132,34 @@ __global__ void __launch_bounds__(256) causal_conv_many_kernel(ConvArgs a) {
         const float* rin = a.state + ((size_t)s * (twice ? 2 : 1) + pr[r]) * ring * W;
         float* rout = a.state + ((size_t)s * 2 + (pr[r] ^ 1)) * ring * W;
         const bool last_row = twice && (t + 1 >= a.T || sl[r + BACK + 1] != s);
-        float acc = fmaf(wk[0], hv[r + BACK], a.residual ? hv[r + BACK] : 0.f);
+        float acc[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) acc[e] = fmaf(wk[0][e], hv[r + BACK][e], a.residual ? hv[r + BACK][e] : 0.f);
 #pragma unroll
         for (int k = 1; k < CTAPS; ++k) {
             if (k >= a.taps || k > p) break;
             const bool instep = t - k >= 0 && sl[r + BACK - k] == s;
-            const float v = instep ? hv[r + BACK - k] : rin[(size_t)((p - k) % ring) * W + c];
-            acc = fmaf(wk[k], v, acc);
-            if (last_row && k < ring && !instep) rout[(size_t)((p - k) % ring) * W + c] = v;
+            float v[V];
+#pragma unroll
+            for (int e = 0; e < V; ++e) v[e] = hv[r + BACK - k][e];
+            if (!instep) cols_load<V>(v, rin + (size_t)((p - k) % ring) * W + c);
+#pragma unroll
+            for (int e = 0; e < V; ++e) acc[e] = fmaf(wk[k][e], v[e], acc[e]);
+            if (last_row && k < ring && !instep) cols_store<V>(rout + (size_t)((p - k) % ring) * W + c, v);
         }
-        out[r] = a.act ? silu_f(acc) : acc;
+#pragma unroll
+        for (int e = 0; e < V; ++e) out[r][e] = a.act ? silu_f(acc[e]) : acc[e];
         if (twice && ring > 0) {
             int behind = -1;                              // slot of row t + ring
 #pragma unroll
             for (int k = 1; k < CTAPS; ++k)
                 if (k == ring) behind = sl[r + BACK + k];
-            if (t + ring >= a.T || behind != s) rout[(size_t)(p % ring) * W + c] = hv[r + BACK];
+            if (t + ring >= a.T || behind != s) cols_store<V>(rout + (size_t)(p % ring) * W + c, hv[r + BACK]);
         }
     }
 #pragma unroll
     for (int r = 0; r < CROWS; ++r)
-        if (t0 + r < a.T) a.u[(size_t)(t0 + r) * a.ldu + c] = out[r];
+        if (t0 + r < a.T) cols_store<V>(a.u + (size_t)(t0 + r) * a.ldu + c, out[r]);
 }
 
 // seqs [n][4] = (first row, rows, slot, first position); block x = sequence * ring + i: the i-th last row of the sequence
@@ -171,31 +206,72 @@ __global__ void __launch_bounds__(128) linear_prep_kernel(LinPrepArgs a) {
 // Many heads: the warps of a token's gridDim.y blocks take the units in turn, and the token's angles (a product in float64 and a sine
 // pair each) are taken once per block instead of once per head (2000 tokens, us: 16 heads of 128 36 -> 26, 32 85 -> 57).  With few heads
 // the barrier costs more than that (five 13.6 -> 15.5), and so does a test for the table's end in one kernel for both (32 heads of 64 42 -> 34 instead of 29).
+// VEC: four neighbouring elements per access (2000 tokens, 16 heads of 128 without a rotation: 31.4 -> 20.0 us).
 constexpr int LIN_TURNS = 4096;                           // angles that shared memory holds
 
+__device__ __forceinline__ void act4(float (&v)[4], bool act, float sc) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = (act ? silu_f(v[e]) : v[e]) * sc;
+}
+
+template <bool VEC>
 __global__ void __launch_bounds__(256) linear_prep_many_kernel(LinPrepArgs a) {
     griddep_wait();
     griddep_launch();
     extern __shared__ float2 turn[];                      // [rot_dims / 2] (sine, cosine)
     const int t = blockIdx.x, lane = threadIdx.x & 31, half = a.rot_dims / 2;
-    const int pos = half ? a.pos[t] : 0;
-    for (int i = threadIdx.x; i < half; i += 256) {
-        float sn, cs;
-        rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
-        turn[i] = make_float2(sn, cs);
+    if (half) {
+        const int pos = a.pos[t];
+        for (int i = threadIdx.x; i < half; i += 256) {
+            float sn, cs;
+            rope_angle_sincos(pos, a.inv_freq[i], sn, cs);
+            turn[i] = make_float2(sn, cs);
+        }
+        __syncthreads();
     }
-    __syncthreads();
     float* row = a.proj + (size_t)t * a.ld;
     for (int u = blockIdx.y * 8 + (threadIdx.x >> 5); u < 3 * a.H; u += 8 * gridDim.y) {
         if (u >= 2 * a.H) {
             if (!a.act) break;
             float* v = row + a.v_off + (size_t)(u - 2 * a.H) * a.Dv;
-            for (int d = lane; d < a.Dv; d += 32) v[d] = silu_f(v[d]);
+            if (VEC) {
+                for (int d = lane * 4; d < a.Dv; d += 128) {
+                    float x[4];
+                    *(float4*)x = *(const float4*)(v + d);
+                    act4(x, true, 1.f);
+                    store4(v + d, x);
+                }
+            } else
+                for (int d = lane; d < a.Dv; d += 32) v[d] = silu_f(v[d]);
             continue;
         }
         const bool is_k = u >= a.H;
         float* x = row + (is_k ? a.k_off + (size_t)(u - a.H) * a.D : a.q_off + (size_t)u * a.D);
         const float sc = is_k ? a.k_scale : 1.f;
+        if (VEC) {
+            for (int i = lane * 4; i < half; i += 128) {
+                float p0[4], p1[4], y0[4], y1[4];
+                *(float4*)p0 = *(const float4*)(x + i);
+                *(float4*)p1 = *(const float4*)(x + i + half);
+                act4(p0, a.act, 1.f);
+                act4(p1, a.act, 1.f);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float sn = turn[i + e].x, cs = turn[i + e].y;
+                    y0[e] = (p0[e] * cs - p1[e] * sn) * sc;
+                    y1[e] = (p1[e] * cs + p0[e] * sn) * sc;
+                }
+                store4(x + i, y0);
+                store4(x + i + half, y1);
+            }
+            for (int d = 2 * half + lane * 4; d < a.D; d += 128) {
+                float v[4];
+                *(float4*)v = *(const float4*)(x + d);
+                act4(v, a.act, sc);
+                store4(x + d, v);
+            }
+            continue;
+        }
         for (int i = lane; i < half; i += 32) {
             float p0 = x[i], p1 = x[i + half];
             if (a.act) { p0 = silu_f(p0); p1 = silu_f(p1); }
@@ -528,6 +604,29 @@ __global__ void __launch_bounds__(256) linear_finish_kernel(LinFinishArgs a) {
     }
 }
 
+// The norm over all heads with the row in registers: outputs, gates and weights go out together (2000 rows of 2048: 19.7 -> 11.0 us).
+template <bool VEC, int G>
+__global__ void __launch_bounds__(ROW_THREADS) linear_finish_row_kernel(LinFinishArgs a) {
+    griddep_wait();
+    griddep_launch();
+    __shared__ float red[32];
+    const int t = blockIdx.x, n = a.H * a.Dv;
+    float* o = a.o + (size_t)t * a.ldo;
+    float v[4 * G], g[4 * G], w[4 * G];
+    row_load<VEC, G>(v, o, n);
+    if (a.gate_act) row_load<VEC, G>(g, a.gate + (size_t)t * a.ldg + a.g_off, n);
+    if (a.w) row_load<VEC, G>(w, a.w, n);
+    const float inv = 1.f / sqrtf(row_sum(square_sum(v), red) / (float)n + a.eps);
+#pragma unroll
+    for (int j = 0; j < 4 * G; ++j) {
+        v[j] *= inv;
+        if (a.w) v[j] *= w[j];
+        if (a.gate_act == 1) v[j] *= sigmoid_f(g[j]); else if (a.gate_act == 2) v[j] *= silu_f(g[j]);
+        v[j] *= a.mult;
+    }
+    row_store<VEC, G>(o, v, n);
+}
+
 }  // namespace
 
 extern "C" {
@@ -541,10 +640,13 @@ int pgk_causal_conv_rows_ex_f32(const float* h, int ldh, float* u, int ldu, cons
     if (rows <= 0) return 0;
     ConvArgs a{h, u, weight, state, slot, pos, taps > 1 ? parity : nullptr, rows, width, taps, ldh, ldu, residual ? 1 : 0,
                activation ? 1 : 0};
-    // four rows per thread from 256 rows on (2000 rows: 38 -> 24 us); fewer leave SMs idle
-    if (rows >= 256 && taps <= CTAPS)
-        PGK_CUDA(launch_waiting(causal_conv_many_kernel, dim3((rows + CROWS - 1) / CROWS, (width + 255) / 256), dim3(256), 0, (cudaStream_t)stream, a));
-    else
+    // four rows per thread from 256 rows on; fewer leave SMs idle
+    if (rows >= 256 && taps <= CTAPS) {
+        const bool vec = ldh % 4 == 0 && ldu % 4 == 0 && row_vec(width, {h, u, weight, state});
+        const int cols = vec ? 4 : 1;
+        const auto kernel = vec ? causal_conv_many_kernel<4> : causal_conv_many_kernel<1>;
+        PGK_CUDA(launch_waiting(kernel, dim3((rows + CROWS - 1) / CROWS, (width + 128 * cols - 1) / (128 * cols)), dim3(128), 0, (cudaStream_t)stream, a));
+    } else
         PGK_CUDA(launch(causal_conv_rows_kernel, dim3(rows, (width + 255) / 256), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }
@@ -572,7 +674,9 @@ int pgk_seq_linear_prep(float* proj, int ld, int tokens, int heads, int dim, int
     if (heads > 8 && rot_dims / 2 <= LIN_TURNS) {
         // a unit per warp while that fills the SMs no more than once, then two blocks per token (angles twice instead of six times)
         const int all = (3 * heads + 7) / 8, groups = (long long)tokens * all <= 8 * sm_count() ? all : 2;
-        PGK_CUDA(launch_waiting(linear_prep_many_kernel, dim3(tokens, groups), dim3(256), (size_t)(rot_dims / 2) * sizeof(float2), (cudaStream_t)stream, a));
+        const bool vec = ld % 4 == 0 && vdim % 4 == 0 && rot_dims % 8 == 0 && (q_off | k_off | v_off) % 4 == 0 && row_vec(dim, {proj});
+        const auto kernel = vec ? linear_prep_many_kernel<true> : linear_prep_many_kernel<false>;
+        PGK_CUDA(launch_waiting(kernel, dim3(tokens, groups), dim3(256), (size_t)(rot_dims / 2) * sizeof(float2), (cudaStream_t)stream, a));
     } else
         PGK_CUDA(launch(linear_prep_kernel, dim3(tokens, (3 * heads + 3) / 4), dim3(128), 0, (cudaStream_t)stream, a));
     return 0;
@@ -643,6 +747,14 @@ int pgk_seq_linear_finish(float* o, int ldo, const float* gate_rows, int ldg, in
                 "seq_linear_finish failed: invalid arguments");
     if (tokens <= 0) return 0;
     LinFinishArgs a{o, ldo, gate_rows, ldg, gate_off, weight, heads, vdim, per_head ? 1 : 0, gate_act, eps, mult};
+    const int n = heads * vdim;
+    if (!per_head && n <= 4 * ROW_G2 * ROW_THREADS) {
+        const bool vec = ldo % 4 == 0 && ldg % 4 == 0 && gate_off % 4 == 0 && row_vec(n, {o, gate_rows, weight}), wide = n > 4 * ROW_G * ROW_THREADS;
+        const auto kernel = vec ? (wide ? linear_finish_row_kernel<true, ROW_G2> : linear_finish_row_kernel<true, ROW_G>)
+                                : (wide ? linear_finish_row_kernel<false, ROW_G2> : linear_finish_row_kernel<false, ROW_G>);
+        PGK_CUDA(launch_waiting(kernel, dim3(tokens), dim3(row_threads(n, wide ? ROW_G2 : ROW_G)), 0, (cudaStream_t)stream, a));
+        return 0;
+    }
     PGK_CUDA(launch_waiting(linear_finish_kernel, dim3(tokens), dim3(256), 0, (cudaStream_t)stream, a));
     return 0;
 }

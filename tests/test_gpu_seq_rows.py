@@ -19,10 +19,10 @@ def i32(a):
 
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 @pytest.mark.parametrize("rows,twice", [((256,), False), ((1, 258, 2, 3), True), ((130, 131), True), ((5, 1, 1, 300), False)])
-def test_convolution_over_many_rows_equals_portions(rows, twice, taps):
+def test_convolution_over_many_rows_equals_portions(rows, twice, taps, width=300):
     """one launch of 256 rows and more against the same rows in launches of fewer (the kernel of a row per block): the same bits in
     rows and rings, sequences that start, continue and end anywhere in a thread's four rows"""
-    W, S = 300, len(rows)
+    W, S = width, len(rows)
     rng = np.random.default_rng(sum(rows) + taps)
     ring, first = max(1, taps - 1), [0 if s % 2 == 0 else 7 for s in range(S)]
     h, w = rng.standard_normal((sum(rows), W)), f32(rng.standard_normal((W, taps)))
@@ -165,3 +165,171 @@ def test_linear_attention_chunks_with_an_infinite_value():
     keep = np.ones_like(a, bool)
     keep[150:, 7] = False
     assert np.isfinite(b[keep]).all() and np.abs(b - a)[keep].max() <= 1e-5 * np.abs(a).max()
+
+
+_HELD = []
+
+
+def _held(a):
+    """the address of an operand that lives until the next test"""
+    _HELD.append(a)
+    return a.device_ptr
+
+
+@pytest.fixture(autouse=True)
+def _let_go():
+    yield
+    gk.synchronize()
+    _HELD.clear()
+
+
+def _close(got, ref, terms):
+    """float32 arithmetic of a row kernel: sums in some order (a block's: up to 20 additions in a row beside the elements of a thread) and a
+    handful of roundings behind them, of magnitudes `terms`"""
+    assert (np.abs(got - ref) <= 2.0 ** -24 * 48 * (np.abs(terms) + 1.0)).all()
+
+
+@pytest.mark.parametrize("W", [1, 63, 256, 260, 2048, 4095, 4096, 4097, 4100, 8192, 8193, 8196])
+@pytest.mark.parametrize("rows", [1, 5])
+def test_norms_of_rows_of_any_width(rows, W):
+    """the forms by width (two and four groups of four per thread, shared memory beyond) and by alignment"""
+    rng = np.random.default_rng(W)
+    x, y, d = (rng.standard_normal((rows, W)).astype(np.float32) for _ in range(3))
+    w, g, b = (rng.standard_normal(W).astype(np.float32) for _ in range(3))
+    X, Y, D = (v.astype(np.float64) for v in (x, y, d))
+    rms = lambda v, k: v / np.sqrt((v * v).mean(1, keepdims=True) + 1e-5) * k
+    xs, out = f32(x), f32(y)
+    api.rms_norm_rows_f32(xs.device_ptr, None, _held(f32(d)), xs.device_ptr, _held(f32(w)), 0.5, 1e-5, out.device_ptr, rows, W, 1, None)
+    _close(xs.to_numpy(), X + D, X)
+    _close(out.to_numpy(), Y + rms(X + D, 0.5 + w), 4 * (np.abs(Y) + np.abs(rms(X + D, 0.5 + w))))
+    xs, h = f32(x), gk.from_numpy(np.full((rows, W), 7.0, np.float32))
+    api.rms_norm_seam_f32(_held(f32(y)), _held(f32(w)), 1.0, xs.device_ptr, _held(f32(d)), _held(f32(g)), 0.0, 1e-5, h.device_ptr, rows, W, None)
+    s = X + rms(Y, 1.0 + w) + D
+    _close(xs.to_numpy(), s, 8 * np.abs(rms(Y, 1.0 + w)) + np.abs(X))
+    _close(h.to_numpy(), rms(s, g), 40 * np.abs(rms(s, g)) + 8)
+    top = 3
+    parts, inv, wt = rng.standard_normal((rows * top, W)).astype(np.float32), rng.permutation(rows * top).reshape(rows, top), rng.random((rows, top)).astype(np.float32)
+    out = f32(y)
+    api.combine_layernorm_f32(_held(f32(x)), None, _held(f32(parts)), _held(i32(inv)), _held(f32(wt)), top, _held(f32(g)), _held(f32(b)),
+                              1e-5, out.device_ptr, rows, W, 1, None)
+    s = X + (wt[..., None].astype(np.float64) * parts.astype(np.float64)[inv]).sum(1)
+    c = s - s.mean(1, keepdims=True)
+    n = c / np.sqrt((c * c).mean(1, keepdims=True) + 1e-5)
+    if W > 1:
+        _close(out.to_numpy(), Y + n * g + b, 16 * (np.abs(n * g) + np.abs(g)) + np.abs(Y) + np.abs(b))
+    table, toks = rng.standard_normal((9, W)).astype(np.float32), rng.integers(0, 9, rows)
+    xs, keep = f32(x), f32(x)
+    api.embed_norm_rows_f32(_held(f32(table)), 0, _held(i32(toks)), _held(f32(w)), 1.0, 1e-5, xs.device_ptr, keep.device_ptr, rows, W, 9, None)
+    ref = rms(table.astype(np.float64)[toks], 1.0 + w)
+    _close(xs.to_numpy(), ref, 4 * ref)
+    assert np.array_equal(xs.to_numpy(), keep.to_numpy())
+
+
+@pytest.mark.parametrize("H,G,D,Dv,pad", [(1, 1, 128, 128, 0), (32, 4, 128, 64, 4), (45, 9, 96, 100, 0), (6, 2, 4, 8, 1), (4, 2, 132, 128, 0)])
+@pytest.mark.parametrize("T", [3, 400])
+def test_heads_and_cache_rows_of_a_projection(H, G, D, Dv, pad, T):
+    """several heads of a warp, heads that leave lanes idle, rows off 16-byte boundaries and heads too long for a lane's four elements; values recorded
+    and mixed.  Queries and the float32 cache against float64."""
+    rng = np.random.default_rng(H * D + T)
+    PS, pages = 16, T // 16 + 1
+    ld = (H + G) * D + G * Dv + pad
+    x = rng.standard_normal((T, ld)).astype(np.float32)
+    qw, kw = (rng.standard_normal(D).astype(np.float32) for _ in range(2))
+    first = rng.standard_normal((T, G * Dv)).astype(np.float32)
+    table = rng.permutation(pages).astype(np.int32)
+    X = x.astype(np.float64)
+    qk = X[:, :(H + G) * D].reshape(T, H + G, D)
+    qk = qk / np.sqrt((qk * qk).mean(2, keepdims=True) + 1e-6) * np.where(np.arange(H + G)[:, None] < H, qw, kw)
+    for mode in (0, 1, 2):
+        p, kc, vc, vf = f32(x), gk.zeros((pages * G * PS * D,), gk.float32), gk.zeros((pages * G * PS * Dv,), gk.float32), f32(first)
+        api.seq_mixer_prep(p.device_ptr, ld, T, H, G, D, Dv, _held(f32(qw)), _held(f32(kw)), 1e-6, mode, 0.25, vf.device_ptr, kc.device_ptr,
+                           vc.device_ptr, 0, _held(i32(table)), pages, PS, _held(i32(np.zeros(T))), _held(i32(np.arange(T))), None)
+        v = X[:, (H + G) * D:(H + G) * D + G * Dv]
+        if mode == 2:
+            v = 0.75 * v + 0.25 * first.astype(np.float64)
+        rows = lambda c, n: c.to_numpy().reshape(pages, G, PS, n)[table].transpose(0, 2, 1, 3).reshape(pages * PS, G, n)[:T]
+        got = p.to_numpy()
+        _close(got[:, :H * D], qk[:, :H].reshape(T, -1), 4 * qk[:, :H].reshape(T, -1))
+        _close(rows(kc, D), qk[:, H:], 4 * qk[:, H:])
+        _close(rows(vc, Dv), v.reshape(T, G, Dv), 4 * v.reshape(T, G, Dv))
+        assert np.array_equal(got[:, H * D:], x[:, H * D:])
+        assert mode != 1 or np.array_equal(vf.to_numpy(), x[:, (H + G) * D:(H + G) * D + G * Dv])
+
+
+@pytest.mark.parametrize("H,G,D,pad", [(4, 2, 64, 0), (16, 8, 128, 3), (32, 4, 128, 0), (33, 2, 128, 0), (3, 1, 30, 0)])
+def test_whole_projection_norm(H, G, D, pad):
+    rng = np.random.default_rng(H * D)
+    T, PS, pages, off = 9, 4, 3, H * D + pad
+    ld = off + G * D + pad
+    x = rng.standard_normal((T, ld)).astype(np.float32)
+    qb, qw = (rng.standard_normal(H * D).astype(np.float32) for _ in range(2))
+    kb, kw = (rng.standard_normal(G * D).astype(np.float32) for _ in range(2))
+    p, kc, vc = f32(x), gk.zeros((pages * G * PS * D,), gk.float32), gk.zeros((pages * G * PS * D,), gk.float32)
+    api.seq_mixer_prep_all(p.device_ptr, ld, T, H, G, D, off, _held(f32(qb)), _held(f32(kb)), _held(f32(qw)), _held(f32(kw)), 1.0, 1e-6,
+                           kc.device_ptr, vc.device_ptr, 0, _held(i32(np.arange(pages))), pages, PS, _held(i32(np.zeros(T))), _held(i32(np.arange(T))), None)
+    q, k = x[:, :H * D].astype(np.float64) + qb, x[:, off:off + G * D].astype(np.float64) + kb
+    rms = lambda v: v / np.sqrt((v * v).mean(1, keepdims=True) + 1e-6)
+    rows = lambda c: c.to_numpy().reshape(pages, G, PS, D).transpose(0, 2, 1, 3).reshape(pages * PS, G * D)[:T]
+    _close(p.to_numpy()[:, :H * D], rms(q) * (1.0 + qw), 4 * np.abs(rms(q)) * (1 + np.abs(qw)))
+    _close(rows(kc), rms(k) * (1.0 + kw), 4 * np.abs(rms(k)) * (1 + np.abs(kw)))
+    _close(rows(vc), k, 2 * np.abs(k))
+
+
+@pytest.mark.parametrize("qr,rank,rot,turn,pad", [(768, 512, 64, 64, 0), (0, 256, 64, 32, 1), (2052, 512, 8, 8, 0), (512, 2100, 64, 64, 0), (30, 18, 6, 4, 0), (64, 64, 520, 516, 0)])
+def test_latents_and_their_cache_rows(qr, rank, rot, turn, pad):
+    rng = np.random.default_rng(qr + rank)
+    T, PS, pages = 9, 4, 3
+    ld = qr + rank + rot + pad
+    x = rng.standard_normal((T, ld)).astype(np.float32)
+    qw, cw = rng.standard_normal(max(1, qr)).astype(np.float32), rng.standard_normal(rank).astype(np.float32)
+    freq, pos = 10000.0 ** (-np.arange(turn // 2) / (turn // 2)), np.arange(T)
+    p, kc = f32(x), gk.zeros((pages * PS * (rank + rot),), gk.float32)
+    api.seq_latent_prep(p.device_ptr, ld, T, qr, qr, rank, rot, turn, _held(f32(qw)) if qr else None, _held(f32(cw)), 1.0, 1e-6, _held(gk.from_numpy(freq)),
+                        kc.device_ptr, 0, _held(i32(np.arange(pages))), pages, PS, _held(i32(np.zeros(T))), _held(i32(pos)), None)
+    X = x.astype(np.float64)
+    rms = lambda v: v / np.sqrt((v * v).mean(1, keepdims=True) + 1e-6)
+    q, c, r = X[:, :qr], rms(X[:, qr:qr + rank]) * (1.0 + cw), X[:, qr + rank:qr + rank + rot].copy()
+    a = pos[:, None] * freq
+    u, v = r[:, 0:turn:2].copy(), r[:, 1:turn:2].copy()
+    r[:, 0:turn:2], r[:, 1:turn:2] = u * np.cos(a) - v * np.sin(a), v * np.cos(a) + u * np.sin(a)
+    got, rows = p.to_numpy(), kc.to_numpy().reshape(pages * PS, rank + rot)[:T]
+    if qr:
+        _close(got[:, :qr], rms(q) * (1.0 + qw), 4 * np.abs(rms(q)) * (1 + np.abs(qw)))
+    _close(rows, np.concatenate([c, r], 1), 4 * np.abs(np.concatenate([c, np.abs(r) + 1], 1)))
+    assert np.array_equal(got[:, qr:], x[:, qr:])
+
+
+@pytest.mark.parametrize("T,top,E", [(1, 1, 1), (2000, 4, 18), (37, 8, 513), (4100, 2, 64)])
+def test_rows_of_every_expert(T, top, E):
+    rng = np.random.default_rng(T)
+    idx = rng.integers(0, E, (T, top)).astype(np.int32)
+    counts, rank = np.bincount(idx.ravel(), minlength=E), np.zeros(T * top, np.int64)
+    for e in range(E):
+        m = idx.ravel() == e
+        rank[m] = rng.permutation(m.sum())
+    cd, off, perm, inv = i32(counts), i32(np.zeros(E + 1)), i32(np.zeros(T * top)), i32(np.zeros(T * top))
+    api.moe_row_lists(cd.device_ptr, off.device_ptr, _held(i32(idx)), _held(i32(rank)), perm.device_ptr, inv.device_ptr, E, T, top, None)
+    first = np.concatenate([[0], np.cumsum(counts)])
+    row = first[idx.ravel()] + rank
+    assert np.array_equal(off.to_numpy(), first) and np.array_equal(inv.to_numpy(), row) and (cd.to_numpy() == 0).all()
+    assert np.array_equal(perm.to_numpy()[row], np.arange(T * top) // top)
+
+
+@pytest.mark.parametrize("taps", [3, 4])
+def test_convolution_of_single_columns(taps):
+    """rows whose width leaves no 16-byte boundaries"""
+    test_convolution_over_many_rows_equals_portions((1, 258, 2, 3), True, taps, width=301)
+
+
+@pytest.mark.parametrize("H,Dv,pad", [(16, 128, 0), (3, 7, 1), (33, 128, 0), (64, 128, 4), (65, 128, 0)])
+@pytest.mark.parametrize("act", [0, 1, 2])
+def test_output_norm_and_gate_over_all_heads(H, Dv, pad, act):
+    rng = np.random.default_rng(H + Dv)
+    T, n = 5, H * Dv
+    o, g, w = rng.standard_normal((T, n + pad)).astype(np.float32), rng.standard_normal((T, n + 2 * pad)).astype(np.float32), rng.standard_normal(n).astype(np.float32)
+    od = f32(o)
+    api.seq_linear_finish(od.device_ptr, n + pad, _held(f32(g)), n + 2 * pad, pad, _held(f32(w)), T, H, Dv, 0, act, 1e-5, 0.5, None)
+    x, z = o[:, :n].astype(np.float64), g[:, pad:pad + n].astype(np.float64)
+    ref = x / np.sqrt((x * x).mean(1, keepdims=True) + 1e-5) * w * 0.5 * (1.0 if act == 0 else (1 if act == 1 else z) / (1 + np.exp(-z)))
+    _close(od.to_numpy()[:, :n], ref, 4 * ref)
+    assert np.array_equal(od.to_numpy()[:, n:], o[:, n:])
