@@ -182,7 +182,7 @@ static int launch_bf16(const uint16_t* A, const uint16_t* B, uint16_t* C, int K,
             int occ[17] = {0};
             for (int wpc = 2; wpc <= 16; ++wpc)
                 PGK_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ[wpc], kern, wpc * 32, smem));
-            it = cache.emplace(key, pick_gemv_cfg(N, occ)).first;
+            it = cache.emplace(key, pick_gemv_cfg(N, 2.0 * K, occ)).first;
         }
         cfg = it->second;
     }

@@ -11,23 +11,27 @@ struct GemvCfg {
     int rho;  // rows per warp
 };
 
-// Pick (warps per CTA, CTAs) such that all CTAs are co-resident (one wave) and the rows
-// divide evenly over the warps.  max_ctas_per_sm[wpc] comes from the occupancy calculator.
-inline GemvCfg pick_gemv_cfg(int n_rows, const int* max_ctas_per_sm /* index = warps per CTA, 1..16 */) {
+// Pick (warps per CTA, CTAs) such that all CTAs are co-resident (one wave): the count of warps whose rows take the least time.  A warp has
+// one group of 4 KB in flight and waits for each -- 1.0 us from its request to the next --, an SM draws 39 bytes per ns when all do, and
+// the warps walk ceil(rows / warps) rows one after the other.  The model meets what was measured for 2 to 16 warps an SM within 10 % (us, one row of
+// FP8: 4992 x 10496 2 warps 56, 6 21.6, 10 17.3, 12 14.9, 16 16.0; 6144 x 4096 4 warps 15.0, 10 10.0, 14 8.6, 16 9.1); choosing by how evenly rows
+// divide alone took 2 warps an SM for 39 x 128 rows (one row 4992 x 10496 56 -> 14.9, three 6784 x 1792 31 -> 10.7).
+inline GemvCfg pick_gemv_cfg(int n_rows, double row_bytes, const int* max_ctas_per_sm /* index = warps per CTA, 1..16 */) {
     const int sms = sm_count();
     GemvCfg best = {8, sms, (n_rows + sms * 8 - 1) / (sms * 8)};
-    double best_score = -1.0;
+    double best_cost = 1e30;
+    const double groups = (double)(long)((row_bytes + 4095.0) / 4096.0);
     for (int wpc = 2; wpc <= 16; ++wpc) {
         for (int c = 1; c <= max_ctas_per_sm[wpc]; ++c) {
-            int W = wpc * c;
-            long total = (long)sms * W;
-            int rho = (int)((n_rows + total - 1) / total);
-            double eff = (double)n_rows / ((double)rho * (double)total);
-            // prefer high efficiency; tie-break toward more resident warps (bytes in flight)
-            // and fewer, larger CTAs (less activation staging)
-            double score = eff + 0.0004 * (W > 40 ? 40 : W) - 0.0002 * c;
-            if (score > best_score) {
-                best_score = score;
+            const int W = wpc * c;
+            const long total = (long)sms * W;
+            const int rho = (int)((n_rows + total - 1) / total);
+            const double turn = W * row_bytes / 39e3;
+            // ties go to more warps where memory bounds (32768 x 4096 in BF16 42.6 -> 40.5), to fewer where the wait does, which leaves few rows on
+            // more SMs (128 x 2048 6.9 -> 4.3), and to fewer, larger CTAs (less activation staging)
+            const double cost = rho * (turn > groups ? turn * (1.0 - 0.0004 * (W > 40 ? 40 : W)) : groups * (1.0 + 0.0004 * W)) * (1.0 + 0.0002 * c);
+            if (cost < best_cost) {
+                best_cost = cost;
                 best = {wpc, sms * c, rho};
             }
         }

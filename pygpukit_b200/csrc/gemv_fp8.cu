@@ -317,7 +317,7 @@ static int launch_fp8_kern(Kern kern, int maxw, int M, const void* A, const void
                 occ[wpc] = nb;
             }
             PGK_REQUIRE(occ[4] > 0, "gemv_fp8_bf16 failed: kernel does not fit (K=%d, M=%d)", K, M);
-            it = cache.emplace(key, pick_gemv_cfg(N, occ)).first;
+            it = cache.emplace(key, pick_gemv_cfg(N, (B1 ? 2.0 : 1.0) * K, occ)).first;
         }
         cfg = it->second;
     }
