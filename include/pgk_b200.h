@@ -146,10 +146,12 @@ int pgk_gemv_nvf4_bf16_ex(const void* A, const void* B_data, const void* B_scale
 /* Decode batch 5..64 on the tensor cores: E2M1 x UE4M3 has <= 6 significant bits, so the converter warps write EXACT BF16
  * weight tiles (E2M1 conversion, multiply by the scale) and one tcgen05.mma.kind::f16 per 16 k computes exact products with
  * F32 accumulation in TMEM -- the FP32-accumulate class of the GEMV, weights read once for all M rows.  Needs
- * 1 <= M <= 64, K % 128 == 0, N % 128 == 0; pgk_gemv_nvf4_bf16(_ex) dispatch here for M >= 5.  Replaces the per-row use of
+ * 1 <= M <= 64, K % 128 == 0, N % 128 == 0; pgk_gemv_nvf4_bf16(_ex) and, with the activation, pgk_gemv_nvf4_swiglu_bf16 dispatch here for M >= 5.  Replaces the per-row use of
  * gemv_nvf4_bf16_kernel (nvf4_kernels.cu:79-233) and the CUTLASS NVF4 GEMM of gemm/w4a16_bf16/sm120/nvf4_cutlass.cu. */
 int pgk_gemm_nvf4_bf16_tc(const void* A, const void* B_data, const void* B_scale, void* C, int M, int K, int N,
                           float alpha, const void* bias, const void* residual, void* stream);
+/* Waits of that kernel that ran out so far (0: none), after a device synchronisation. */
+int pgk_gemm_nvf4_wait_error(int* out);
 /* out[M,I] = bf16(bf16(silu(g)) * u) from a [M, 2I] tensor whose columns are gate/up interleaved in groups of 8 (the
  * fused NVF4 MLP layout below): the epilogue of the batched (tensor-core) gate/up projection */
 int pgk_swiglu_interleaved8_bf16(const void* gate_up, void* out, int M, int I, void* stream);
@@ -351,6 +353,21 @@ int pgk_moe_gateup_fp8_t1(const void* x, const void* Bg_enk, const void* Sg, con
 int pgk_moe_gateup_nvf4_t1(const void* x, const void* Bg_data, const void* Bg_scale, const void* Bu_data,
                            const void* Bu_scale, void* act, const int32_t* row_expert_ids, int k, int K, int N,
                            int expert_offset, int num_local_experts, void* stream);
+/* A few dozen tokens (2 ... 64) through NVF4 experts, the arithmetic of the row-by-row entry points above with the products on the tensor
+ * cores.  route_rows: top-k and softmax of bf16 logits [tokens, E] as pgk_moe_topk + pgk_moe_softmax_topk, weights [tokens, k]; active [1 + E] = (how
+ * many experts have rows, which); first [E + 1] = the first row of each in the experts'
+ * order; only experts expert_offset ... + num_local_experts - 1, whose matrices are here, are listed, and the rows of others are not written; row_token [tokens k]; inv [tokens k] = row of every
+ * (token, slot).  tokens * k <= 1024, E <= 512, k <= 32. */
+int pgk_moe_route_rows(const void* logits, void* weights, int32_t* active, int32_t* first, int32_t* row_token, int32_t* inv, int tokens, int num_experts,
+                       int k, int expert_offset, int num_local_experts, void* stream);
+int pgk_moe_experts_gateup_nvf4(const void* x, const void* Bg_data, const void* Bg_scale, const void* Bu_data, const void* Bu_scale, void* act,
+                                const int32_t* active, const int32_t* first, const int32_t* row_token, int tokens, int k, int K, int N, int experts,
+                                int expert_offset, int num_local_experts, void* stream);
+int pgk_moe_experts_down_nvf4(const void* act, const void* B_data, const void* B_scale, void* C, const int32_t* active, const int32_t* first,
+                              int tokens, int k, int K, int N, int experts, int expert_offset, int num_local_experts, void* stream);
+/* out[t] = sum over slots of weight x row inv[t, slot] (+ residual) */
+int pgk_moe_combine_rows_bf16(const void* expert_rows, const void* router_weights, const int32_t* inv, const void* residual, void* out, int tokens, int hidden,
+                              int k, void* stream);
 int pgk_moe_down_combine_fp8_t1(const void* act, const void* Bd_enk, const void* Sd, const void* router_weights,
                                 const int32_t* row_expert_ids, const void* residual, void* out, int k, int K, int N,
                                 int expert_offset, int num_local_experts, void* stream);

@@ -48,6 +48,11 @@ _SIGS = {
     "pgk_gemv_nvf4_swiglu_bf16": [vp, vp, vp, vp, i32, i32, i32, vp],
     "pgk_quantize_bf16_to_nvf4": [vp, vp, vp, i32, i32, vp],
     "pgk_gemm_nvf4_bf16_tc": [vp, vp, vp, vp, i32, i32, i32, f32, vp, vp, vp],
+    "pgk_gemm_nvf4_wait_error": [C.POINTER(i32)],
+    "pgk_moe_route_rows": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp],
+    "pgk_moe_experts_gateup_nvf4": [vp, vp, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp],
+    "pgk_moe_experts_down_nvf4": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, vp],
+    "pgk_moe_combine_rows_bf16": [vp, vp, vp, vp, vp, i32, i32, i32, vp],
     "pgk_swiglu_interleaved8_bf16": [vp, vp, i32, i32, vp],
     "pgk_gemv_bf16": [vp, vp, vp, i32, i32, i32, vp],
     "pgk_gemv_bf16_ex": [vp, vp, vp, i32, i32, i32, vp, vp, vp],

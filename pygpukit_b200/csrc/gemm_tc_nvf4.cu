@@ -1,338 +1,454 @@
-// gemm_tc_nvf4.cu -- NVF4 (W4A16) skinny GEMM for decode batch 5..64 on the 5th-gen tensor cores (tcgen05 + TMEM).
+// gemm_tc_nvf4.cu -- NVF4 (W4A16) products of a few dozen rows on the 5th-gen tensor cores (tcgen05 + TMEM + TMA).
 //
 //   C[M,N] = alpha * A[M,K] . dequant(Bd[K/2,N], Bs[K/32,N])     Bd: two E2M1 nibbles per byte (low = even k),
 //                                                                 Bs: UE4M3 scale per (32 k, column), 1 <= M <= 64
 //
 // replaces the batched use of gemv_nvf4_bf16_kernel (native/ops/matmul/gemv/w4a16_bf16/sm120/nvf4_kernels.cu:79-233: one
 // launch per row, weights re-read M times) and the role of the CUTLASS NVF4 GEMM the reference cannot build here
-// (native/ops/matmul/gemm/w4a16_bf16/sm120/nvf4_cutlass.cu).  On this repo's own path it replaces the slabs of four rows of
-// gemv_nvf4.cu (weights re-read ceil(M/4) times) for M >= 5.
+// (native/ops/matmul/gemm/w4a16_bf16/sm120/nvf4_cutlass.cu).  Forms: plain; a gate/up matrix interleaved by eight columns with silu(gate) * up;
+// the experts of a mixture -- gate and up matrices with silu(gate) * up over gathered rows, and the down product of the sorted rows.
 //
-// Design: same weight-streaming pipeline as gemm_tc.cu (FP8).  The one difference is the dequantisation: an E2M1 value
-// (<= 2 significant bits) times a UE4M3 scale (4 significant bits) has at most 6 significant bits and lies in
-// [2^-8, 2880], so nibble x scale is EXACT in BF16 -- the converter warps write exact BF16 weight tiles, the
-// activations go to the tensor cores as they are (BF16), and ONE tcgen05.mma.kind::f16 per 16 k computes exact
-// products with F32 accumulation in TMEM: the same FP32-accumulate class as the CUDA-core GEMV, no hi/lo split and no
-// block-scaled MMA (whose UE4M3 decoding would not reproduce the reference's "exponent 0 is normal" table,
-// nvf4.cuh:65-115).
-//   * a CTA owns 128 weight columns (MMA M = 128, one TMEM lane per column) and a k range (split-K over gridDim.y);
-//     the batch is the MMA N (16 / 32 / 64 TMEM columns).
-//   * per 128-wide k block: 64 byte rows x 128 B of nibbles + 4 x 128 B of scales stream global -> shared memory with
-//     cp.async in full 128-byte lines (ring of raw blocks, requested before the dependency wait), thread (k chunk c,
-//     column quad) gathers the four bytes of a column with byte permutes, cvt e2m1x2 -> f16x2, multiplied by the scale (exact
-//     in F16) -> BF16x2, and stores the 16-byte k chunk into the canonical no-swizzle K-major core-matrix layout;
-//     fence.proxy.async; a dedicated warp issues the 8 MMAs of the block and commits to the stage's mbarrier.
+// What bounds it: the conversion of the nibbles -- three instructions a weight, 590 issue slots of an SM per block of 128 columns x 128 k, where
+// the block's way from HBM is 360 cycles; 890 are seen.  What follows from that, as in gemm_tc.cu:
+//   * transposed, D^T[n, m]: a TMEM lane per weight column, the batch is the MMA's N (16 / 32 / 64); the weights are the MMA's A operand in
+//     TENSOR MEMORY, whose 32-bit element (lane, column) is a pair of neighbouring k -- exactly one byte of Bd.  A thread reads the bytes of
+//     its column one by one (a warp's 32 bytes lie side by side), puts their bits where BF16 has them and multiplies by the scale: an E2M1
+//     value has two significant bits, a UE4M3 scale four, the product is exact;
+//   * the nibble's exponent goes into BF16's own as it is, which makes it 2^-126 of its value -- its subnormal 0.5 a subnormal of BF16 --, and the
+//     scale's exponent brings it back up to a factor 2^8 (480 x 2^126 would not fit BF16), which the sums are multiplied by at the end;
+//   * TMA brings codes, scales and activations (128-byte swizzle) into a ring; eight warps convert, one copies, one issues the MMAs; two blocks
+//     per SM hide each other's start and end; K is cut over a cluster that pushes its partial rows to their owners' shared memory: no work memory;
+//   * experts: a block per (slice of k, column tile, expert that has rows); the rows of an expert are at most the tokens of the call.  Gate
+//     and up fetch their rows by token (gathering copies of four rows), down finds them in the experts' order.
+// Measured on B200 (us, a pass of a feed-forward or mixture; conversion into shared memory and a launch for the activation, experts row by row ->
+// here): 19 rows 2176 / 17280 72 -> 37, 28 rows 5376 / 3200 56 -> 27, 9 rows 6656 / 4864 74 -> 36; 45 tokens through 128 experts of 1792 /
+// 896, eight each, 498 -> 176, 13 through eight of 3200 / 1920, two each, 154 -> 53.  37888 x 8192 alone: 60 (16 rows), 66 (64 rows), 2.7 TB/s.
 #include "common.cuh"
+#include "gemv_common.cuh"
 #include "tc_common.cuh"
+#include "tma.cuh"
 #include "../../include/pgk_b200.h"
+
+#include <cmath>
+#include <initializer_list>
 
 namespace pgk {
 
-constexpr int kN4BK = 128;          // k per block (64 byte rows, 4 scale rows)
-constexpr int kN4Threads = 512;     // 16 converter warps (+ one MMA-issuing warp)
-constexpr int kN4Stages = 2;        // BF16 operand stages
-constexpr int kN4RawW = 64 * 128 + 4 * 128;   // raw bytes of one weight block (nibbles + scales)
-__host__ __device__ constexpr int n4_raw_depth(int nb) { return nb <= 16 ? 8 : (nb <= 32 ? 6 : 4); }
+namespace {
+
+constexpr int Q_BK = 128;                         // k per block: 64 rows of codes, 4 of scales
+constexpr int Q_WARPS = 8;                        // conversion and output; one more for the copies, one for the MMAs
+constexpr int Q_THREADS = (Q_WARPS + 2) * 32;
+constexpr uint32_t Q_CODES = 64 * 128, Q_SCALES = 4 * 128;
+constexpr int Q_MAX_TILES = 8192;
+enum { Q_PLAIN, Q_SWIGLU, Q_GATEUP, Q_DOWN };     // the two last: experts
+// 16 rows leave room for a third block per SM, with one converted block in tensor memory instead of three (us, 896 x 75776: 22.3 -> 20.8, 8192 x
+// 18944 42.0 -> 40.5; 32 rows the same or slower)
+__host__ __device__ constexpr int q_stages(int nb) { return nb <= 16 ? 5 : (nb <= 32 ? 6 : 4); }
+__host__ __device__ constexpr int q_bufs(int nb) { return nb <= 16 ? 1 : 3; }                        // converted blocks in tensor memory
+__host__ __device__ constexpr int q_blocks(int nb) { return nb <= 16 ? 3 : 2; }                      // blocks per SM
+__host__ __device__ constexpr uint32_t q_stage_bytes(int nb) { return (uint32_t)nb * 256 + Q_CODES + 1024; }
+__host__ __device__ constexpr size_t q_smem(int nb) { return (size_t)q_stages(nb) * q_stage_bytes(nb) + 1024; }
 
 struct N4Params {
-    const uint16_t* A; const uint8_t* Bd; const uint8_t* Bs; uint16_t* C;
-    const uint16_t* bias; const uint16_t* residual;
-    int M, K, N, splits;
+    uint16_t* C; const uint16_t* bias; const uint16_t* residual;
+    int M, K, N, splits, kper;                    // N: columns of one matrix
     float alpha;
-    float* ws; unsigned* counters;
+    const int* active; const int* first; const int* token;        // experts that have rows (their number first), first row of each, token of each row
+    int offset;                                   // the expert whose matrix comes first
+    int ahead;                                    // the first codes are read before the kernel before has finished
+    int* err;                                     // raised when a bounded wait runs out
 };
 
-template <int BYTE>
-__device__ __forceinline__ uint32_t e2m1_pair_scaled_bf16x2(uint32_t q, __half2 s2) {
-    const uint32_t h = e2m1x2_to_f16x2<BYTE>(q);
-    const __half2 p = __hmul2(*reinterpret_cast<const __half2*>(&h), s2);      // exact: <= 6 significant bits
-    const float2 f = __half22float2(p);
-    return pack_bf16x2(f.x, f.y);                                               // exact: fits BF16
+__device__ __forceinline__ uint32_t lds_u8(uint32_t at) {
+    uint32_t v;
+    asm volatile("ld.shared.u8 %0, [%1];" : "=r"(v) : "r"(at));
+    return v;
+}
+// a byte's two E2M1 values as BF16 times 2^-126: low nibble in the lower half
+__device__ __forceinline__ uint32_t e2m1x2_to_bf16x2(uint32_t b) {
+    return ((b * 0x00040040u) & 0x01c001c0u) | ((b * 0x01001000u) & 0x80008000u);
+}
+__device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
+    uint32_t r;
+    asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+    return r;
+}
+// UE4M3 (bit 7 ignored, exponent 0 is normal) times 2^118, twice
+__device__ __forceinline__ uint32_t ue4m3_to_bf16x2(uint32_t s) { return (((s & 0x7fu) << 4) + 0x7700u) * 0x00010001u; }
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c0, const int* rows, uint32_t bar) {
+    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                 :: "r"(dst), "l"(map), "r"(c0), "r"(rows[0]), "r"(rows[1]), "r"(rows[2]), "r"(rows[3]), "r"(bar) : "memory");
 }
 
-template <int NB>
-__global__ void __launch_bounds__(kN4Threads + 32, 1)
-gemm_nvf4_tc_kernel(N4Params p) {
-    constexpr int NW = kN4Threads / 32;
-    constexpr int RAW = n4_raw_depth(NB);
-    constexpr int AI = (NB / 2 + NW - 1) / NW;             // activation items per thread per k block
-    constexpr uint32_t A_STAGE = kTcRows * kN4BK * 2;      // 32 KB of BF16 weights
-    constexpr uint32_t B_STAGE = NB * kN4BK * 2;           // BF16 activation tile
-    constexpr uint32_t TMEM_COLS = NB < 32 ? 32 : NB;
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ __align__(8) uint64_t mma_bar[kN4Stages];
+template <int NB, int FORM>
+__global__ void __launch_bounds__(Q_THREADS, q_blocks(NB))
+gemm_nvf4_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap smap, const __grid_constant__ CUtensorMap umap,
+                    const __grid_constant__ CUtensorMap tmap, const __grid_constant__ CUtensorMap amap, const __grid_constant__ N4Params p) {
+    constexpr bool EXPERTS = FORM == Q_GATEUP || FORM == Q_DOWN, TWO = FORM == Q_GATEUP;
+    constexpr int STAGES = q_stages(NB), COLS = NB / 2, TILE = TWO ? 64 : 128;       // TILE: columns of one matrix
+    constexpr uint32_t STAGE = q_stage_bytes(NB), ACTS = NB * 256, TMEM_COLS = NB <= 16 ? 128 : 256;
+    constexpr int Q_BUFS = q_bufs(NB);
+    static_assert(NB + 64 * Q_BUFS <= (int)TMEM_COLS && q_blocks(NB) * (int)TMEM_COLS <= 512, "blocks per SM");
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES], ready_bar[Q_BUFS], free_bar[Q_BUFS];
     __shared__ uint32_t tmem_base_s;
-    __shared__ unsigned s_ticket;
+    __shared__ int token_s[TWO ? NB : 1];
+    const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+    const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
+    const uint32_t ready = smem_u32(ready_bar), freed = smem_u32(free_bar);
+    int* const err = p.err;
+    const int rank = blockIdx.x, n0 = blockIdx.y * TILE, nkb_total = p.K / Q_BK;
+    const int kb0 = rank * p.kper, nkb = max(0, min(nkb_total, kb0 + p.kper) - kb0);
 
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int tile = blockIdx.x, split = blockIdx.y;
-    const int n0 = tile * kTcRows;
-    const int nkb_total = p.K / kN4BK;
-    const int per = (nkb_total + p.splits - 1) / p.splits;
-    const int kb0 = split * per, kb1 = min(nkb_total, kb0 + per);
-    const int nkb = max(0, kb1 - kb0);
-    const int rr = lane & 7, piece = lane >> 3;
-    const bool conv = warp < NW;
-
-    if (warp == 0) tmem_alloc(&tmem_base_s, TMEM_COLS);
+    int z = 0, row0 = 0, rows = min(NB, p.M);
+    if (EXPERTS || !p.ahead) griddep_wait();
+    if constexpr (EXPERTS) {
+        if ((int)blockIdx.z >= p.active[0]) return;       // the same in the whole cluster
+        z = p.active[1 + blockIdx.z];
+        row0 = p.first[z];
+        rows = min(NB, p.first[z + 1] - row0);
+        z -= p.offset;
+        if (TWO && tid < NB) token_s[tid] = p.token[row0 + min(tid, rows - 1)];
+    }
+    if (warp == Q_WARPS + 1) tmem_alloc(&tmem_base_s, TMEM_COLS);
     if (tid == 0) {
-#pragma unroll
-        for (int s = 0; s < kN4Stages; ++s) mbar_init(&mma_bar[s], 1);
+        for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+        for (int b = 0; b < Q_BUFS; ++b) { mbar_init(&ready_bar[b], Q_WARPS); mbar_init(&free_bar[b], 1); }
         mbar_fence_init();
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
+        asm volatile("prefetch.tensormap [%0];" :: "l"(&amap) : "memory");
     }
-    unsigned char* raw_w = smem + (size_t)kN4Stages * (A_STAGE + B_STAGE);
-    unsigned char* raw_a = raw_w + (size_t)RAW * kN4RawW;
-    // weights: 64 rows x 128 B of nibbles (one 16-byte piece per thread) + 4 rows x 128 B of scales (threads 0..31)
-    auto issue_weights = [&](int kb, int rs) {
-        unsigned char* dst0 = raw_w + (size_t)rs * kN4RawW;
-        {
-            const int j = tid >> 3, pc = tid & 7;
-            const uint8_t* src = p.Bd + (size_t)(kb * 64 + j) * p.N + n0 + pc * 16;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_u32(dst0 + j * 128 + pc * 16)), "l"(src) : "memory");
-        }
-        if (tid < 32) {
-            const int j = tid >> 3, pc = tid & 7;
-            const uint8_t* src = p.Bs + (size_t)(kb * 4 + j) * p.N + n0 + pc * 16;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(smem_u32(dst0 + 64 * 128 + j * 128 + pc * 16)), "l"(src) : "memory");
-        }
-    };
-    auto issue_acts = [&](int kb, int rs) {
-#pragma unroll
-        for (int i = 0; i < AI; ++i) {
-            const int m = (i * NW + warp) * 2 + (lane >> 4), pc = lane & 15;    // 2 rows x 256 B per warp request
-            if (m < NB) {
-                const bool ok = m < p.M;                       // rows past the batch are zero-filled (src-size 0)
-                const uint16_t* src = p.A + (ok ? (size_t)m * p.K + (size_t)kb * kN4BK + pc * 8 : 0);
-                const uint32_t dst = smem_u32(raw_a + (size_t)rs * (NB * kN4BK * 2) + m * 256 + ((pc ^ (m & 7)) * 16));
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
-            }
-        }
-    };
-    // group order as in gemm_tc.cu: W0..W(D-1) | A0..A(D-1) | (W_D, A_D) | ...
-#pragma unroll
-    for (int d = 0; d < RAW; ++d) {
-        if (conv && d < nkb) issue_weights(kb0 + d, d);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    griddep_wait();
-#pragma unroll
-    for (int d = 0; d < RAW; ++d) {
-        if (conv && d < nkb) issue_acts(kb0 + d, d);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    }
-    asm volatile("cp.async.wait_group %0;" :: "n"(RAW - 1) : "memory");       // block 0 (weights + slab) landed
-
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    griddep_launch();                                  // tensor memory is held
-    const uint32_t tmem_d = tmem_base_s;
-    constexpr uint32_t idesc = umma_idesc_bf16(NB);
-    // converter role of this thread: k chunk c (8 k = 4 byte rows), columns 4 n4 .. 4 n4 + 3
-    const int c = tid >> 5, n4 = tid & 31;
+    const uint32_t tmem = tmem_base_s, tmem_w = tmem + NB;       // the sums, then blocks of weights (64 columns each)
 
-    for (int it = 0; it < nkb; ++it) {
-        const int st = it & 1, kb = kb0 + it, rs = it % RAW;
-        unsigned char* a_s = smem + (size_t)st * (A_STAGE + B_STAGE);
-        unsigned char* b_s = a_s + A_STAGE;
-        const unsigned char* rw = raw_w + (size_t)rs * kN4RawW;
-        const unsigned char* ra = raw_a + (size_t)rs * (NB * kN4BK * 2);
-        if (conv) {
-            uint32_t w[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const uint32_t*>(rw + (4 * c + i) * 128 + 4 * n4);
-            const uint32_t sw = *reinterpret_cast<const uint32_t*>(rw + 64 * 128 + (c >> 2) * 128 + 4 * n4);
-            uint4 aq[AI];
-#pragma unroll
-            for (int i = 0; i < AI; ++i) {
-                const int q = i * NW + warp;                      // NB/2 items: row group q>>2, 64-byte quarter q&3
-                if (q < NB / 2) {
-                    const int m = 8 * (q >> 2) + rr, pc = (q & 3) * 4 + piece;
-                    aq[i] = *reinterpret_cast<const uint4*>(ra + m * 256 + ((pc ^ rr) * 16));
+    if (warp == Q_WARPS) {
+        // ---------------- copies; the first weights leave before the dependency wait
+        if (elect_one()) {
+            const uint64_t once = l2_evict_first();
+            const int quads = TWO ? (rows + 3) / 4 : 0;
+            const uint32_t bytes = Q_CODES + Q_SCALES + (TWO ? (uint32_t)quads * 1024u : ACTS);
+            auto weights = [&](int it, uint32_t s) {
+                const uint32_t at = ring + s * STAGE + ACTS, bar = full + 8u * s;
+                mbar_expect_tx(bar, bytes);
+                tma_load_3d_hint(at, &wmap, n0, (kb0 + it) * 64, z, bar, once);
+                tma_load_3d_hint(at + Q_CODES, &smap, n0, (kb0 + it) * 4, z, bar, once);
+                if constexpr (TWO) {
+                    tma_load_3d_hint(at + Q_CODES / 2, &umap, n0, (kb0 + it) * 64, z, bar, once);
+                    tma_load_3d_hint(at + Q_CODES + Q_SCALES / 2, &tmap, n0, (kb0 + it) * 4, z, bar, once);
                 }
-            }
-            // the MMAs that read this BF16 stage two iterations ago must have completed
-            if (it >= kN4Stages) mbar_wait(&mma_bar[st], (uint32_t)(((it >> 1) - 1) & 1));
-            // weights: the four bytes of one column (k 8c .. 8c+7) x its block scale -> eight exact BF16 = one 16-byte k chunk
+            };
+            auto acts = [&](int it, uint32_t s) {
+                const uint32_t at = ring + s * STAGE, bar = full + 8u * s;
 #pragma unroll
-            for (int i2 = 0; i2 < 4; ++i2) {
-                const int col = (i2 + (n4 >> 1)) & 3;             // rotated so that a quarter warp stores to 8 bank groups
-                const uint32_t sel = (uint32_t)col | ((uint32_t)(4 + col) << 4);
-                const uint32_t q = __byte_perm(__byte_perm(w[0], w[1], sel), __byte_perm(w[2], w[3], sel), 0x5410);
-                const uint32_t sb = (sw >> (8 * col)) & 0x7fu;    // UE4M3 (bit 7 ignored, exponent 0 is normal) as F16 bits
-                const uint32_t s16 = (sb << 7) + 0x2000u;
-                const uint32_t s32 = s16 | (s16 << 16);
-                const __half2 s2 = *reinterpret_cast<const __half2*>(&s32);
-                uint4 o;
-                o.x = e2m1_pair_scaled_bf16x2<0>(q, s2);
-                o.y = e2m1_pair_scaled_bf16x2<1>(q, s2);
-                o.z = e2m1_pair_scaled_bf16x2<2>(q, s2);
-                o.w = e2m1_pair_scaled_bf16x2<3>(q, s2);
-                const int n = 4 * n4 + col;
-                *reinterpret_cast<uint4*>(a_s + (size_t)c * (kTcRows * 16) + (size_t)n * 16) = o;
-            }
-            // activations: plain copy of the k chunk into the canonical layout
-#pragma unroll
-            for (int i = 0; i < AI; ++i) {
-                const int q = i * NW + warp;
-                if (q < NB / 2) {
-                    const int cc = (q & 3) * 4 + piece;
-                    *reinterpret_cast<uint4*>(b_s + (size_t)cc * (NB * 16) + (size_t)(q >> 2) * 128 + rr * 16) = aq[i];
+                for (int c = 0; c < 2; ++c) {
+                    if constexpr (TWO) {
+                        for (int q = 0; q < quads; ++q)
+                            tma_gather4(at + (uint32_t)c * (NB * 128u) + (uint32_t)q * 512u, &amap, (kb0 + it) * Q_BK + c * 64, token_s + 4 * q, bar);
+                    } else
+                        tma_load_2d(at + (uint32_t)c * (NB * 128u), &amap, (kb0 + it) * Q_BK + c * 64, row0, bar);
                 }
+            };
+            const int first = min(nkb, STAGES);
+            for (int it = 0; it < first; ++it) weights(it, (uint32_t)it);
+            griddep_wait();
+            griddep_launch();
+            for (int it = 0; it < first; ++it) acts(it, (uint32_t)it);
+            RingPos r;
+            r.round = 1;
+            int it = first;
+            for (; it < nkb; ++it, r.next(STAGES)) {
+                if (!bar_wait(err, empty + 8u * r.s, r.round ^ 1u)) break;
+                weights(it, r.s);
+                acts(it, r.s);
             }
-            fence_proxy_async();          // generic-proxy smem writes -> visible to the tensor core (async proxy)
-            asm volatile("cp.async.wait_group %0;" :: "n"(RAW - 2) : "memory");   // this thread's part of block it+1 landed
+            for (int j = max(0, it - STAGES); j < it; ++j)    // whoever gave up: do not leave with copies in flight
+                bar_wait(err, full + 8u * (uint32_t)(j % STAGES), (uint32_t)((j / STAGES) & 1));
+        } else {
+            griddep_wait();
+            griddep_launch();
         }
-        __syncthreads();                  // BF16 stage complete; raw slot `rs` fully read; block it+1 visible to all
-        if (conv) {
-            if (it + RAW < nkb) { issue_weights(kb + RAW, rs); issue_acts(kb + RAW, rs); }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        } else if (lane == 0) {           // the MMA warp
+        __syncwarp();
+    } else if (warp == Q_WARPS + 1) {
+        // ---------------- MMAs
+        griddep_wait();
+        griddep_launch();
+        if (elect_one()) {
+            constexpr uint32_t idesc = umma_idesc_bf16(NB);
+            RingPos r, w;
+            for (int it = 0; it < nkb; ++it, r.next(STAGES), w.next(Q_BUFS)) {
+                if (!bar_wait(err, full + 8u * r.s, r.round) || !bar_wait(err, ready + 8u * w.s, w.round)) break;
+                tc_fence_after();
+                const uint32_t a_s = ring + r.s * STAGE;
+#pragma unroll
+                for (int ks = 0; ks < Q_BK / 16; ++ks)
+                    umma_bf16_ta(tmem, tmem_w + w.s * 64u + (uint32_t)ks * 8u, desc_sw128(a_s + (uint32_t)(ks >> 2) * (NB * 128u)) + (uint64_t)((ks & 3) * 2), idesc,
+                                 (it > 0 || ks > 0) ? 1u : 0u);
+                umma_commit(&free_bar[w.s]);
+                umma_commit(&empty_bar[r.s]);
+            }
+        }
+        __syncwarp();
+    } else {
+        // ---------------- codes -> TMEM
+        griddep_wait();
+        griddep_launch();
+        const int quad = warp & 3, half = warp >> 2, col = quad * 32 + lane;
+        const uint32_t lanes = (uint32_t)(quad * 32) << 16;
+        // where the thread's column starts in a stage: rows of TILE bytes, the second matrix behind the first
+        const uint32_t code_at = ACTS + (TWO ? (uint32_t)(quad >> 1) * (Q_CODES / 2) : 0u) + (uint32_t)(col & (TILE - 1)) + (uint32_t)half * (32 * TILE);
+        const uint32_t scale_at = ACTS + Q_CODES + (TWO ? (uint32_t)(quad >> 1) * (Q_SCALES / 2) : 0u) + (uint32_t)(col & (TILE - 1)) + (uint32_t)half * (2 * TILE);
+        bool ok = true;
+        RingPos r, w;
+        for (int it = 0; it < nkb; ++it, r.next(STAGES), w.next(Q_BUFS)) {
+            const uint32_t st = ring + r.s * STAGE;
+            ok = ok && bar_wait(err, full + 8u * r.s, r.round);
+            __syncwarp();
+            uint32_t b[32], s[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) s[h] = lds_u8(st + scale_at + (uint32_t)(h * TILE));
+#pragma unroll
+            for (int i = 0; i < 32; ++i) b[i] = lds_u8(st + code_at + (uint32_t)(i * TILE));
+            if (it >= Q_BUFS) {                               // the products that read this buffer are done
+                ok = ok && bar_wait(err, freed + 8u * w.s, w.round ^ 1u);
+                __syncwarp();
+                tc_fence_after();
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {                     // 32 k: 16 columns and a scale
+                uint32_t o[16];
+                const uint32_t sc = ue4m3_to_bf16x2(s[h]);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) o[i] = mul_bf16x2(e2m1x2_to_bf16x2(b[16 * h + i]), sc);
+                tmem_st16u(tmem_w + lanes + w.s * 64u + (uint32_t)(half * 32 + h * 16), o);
+            }
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&ready_bar[w.s]);
+        }
+        if (nkb > 0) {                                        // products complete in order: the last one's end is everyone's
+            const int last = nkb - 1;
+            ok = ok && bar_wait(err, freed + 8u * (uint32_t)(last % Q_BUFS), (uint32_t)((last / Q_BUFS) & 1));
+            __syncwarp();
             tc_fence_after();
-            const uint32_t a_addr = smem_u32(a_s), b_addr = smem_u32(b_s);
-#pragma unroll
-            for (int ks = 0; ks < kN4BK / 16; ++ks) {
-                const uint64_t da = umma_desc(a_addr + ks * 2 * (kTcRows * 16), kTcRows * 16, 128);
-                const uint64_t db = umma_desc(b_addr + ks * 2 * (NB * 16), NB * 16, 128);
-                umma_bf16(tmem_d, da, db, idesc, (it > 0 || ks > 0) ? 1u : 0u);
-            }
-            umma_commit(&mma_bar[st]);
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // ---- epilogue
-    if (nkb > 0) {
-        const int last = nkb - 1;
-        mbar_wait(&mma_bar[last & 1], (uint32_t)((last >> 1) & 1));
-    }
-    tc_fence_after();
-    const int row = 32 * (warp & 3) + lane;                 // TMEM lane = weight column of the tile
-    const int n = n0 + row;
-    const size_t tile_ws = ((size_t)tile * p.splits + split) * (size_t)NB * kTcRows;
-    if (warp < 4) {
-#pragma unroll
-        for (int cb = 0; cb < NB; cb += 16) {
-            float v[16];
-            if (nkb > 0) tmem_ld16(tmem_d + ((uint32_t)(32 * warp) << 16) + cb, v);
+
+    // ---------------- outputs: row m of the partial sums goes to block m % splits of the cluster, which adds them in the order of the ranks
+    const int slots = (rows + p.splits - 1) / p.splits;
+    __syncthreads();
+    if (p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");     // every ring is free
+    const int quad = warp & 3, half = warp >> 2;
+    if (warp < Q_WARPS) {
+        int owner = half * COLS % p.splits, slot = half * COLS / p.splits;
+#pragma unroll 1
+        for (int c0 = 0; c0 < COLS; c0 += 8) {
+            float v[8];
+            if (nkb > 0) tmem_ld8(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(half * COLS + c0), v);
             else {
 #pragma unroll
-                for (int j = 0; j < 16; ++j) v[j] = 0.f;
+                for (int j = 0; j < 8; ++j) v[j] = 0.f;
             }
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const int m = cb + j;
-                if (m >= p.M) continue;
-                if (p.splits == 1) {
-                    float x = p.alpha * v[j];
-                    const size_t o = (size_t)m * p.N + n;
-                    if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[n]);
-                    p.C[o] = p.residual ? hadd_bf16_bits(x, p.residual[o]) : f32_to_bf16_bits(x);
-                } else {
-                    __stcg(p.ws + tile_ws + (size_t)m * kTcRows + row, v[j]);
+            for (int j = 0; j < 8; ++j) {
+                if (half * COLS + c0 + j < rows) {
+                    const uint32_t to = ring + (uint32_t)((rank * slots + slot) * kTcRows + quad * 32 + lane) * 4u;
+                    uint32_t remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(to), "r"(owner));
+                    asm volatile("st.shared::cluster.f32 [%0], %1;" :: "r"(remote), "f"(v[j]) : "memory");
                 }
+                if (++owner == p.splits) { owner = 0; ++slot; }
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem_d, TMEM_COLS);
-    if (p.splits == 1) return;
-    if (tid == 0) {
-        __threadfence();
-        s_ticket = atomicAdd(p.counters + tile, 1u);
-        __threadfence();
-    }
-    __syncthreads();
-    if (s_ticket != (unsigned)(p.splits - 1)) return;
-    // last CTA of the tile: fold the split-K partials in split order (deterministic), then the epilogue
-    if (conv) {
-        const int r = tid & (kTcRows - 1), half = tid >> 7;
-        const float* base = p.ws + (size_t)tile * p.splits * NB * kTcRows;
-        const int nn = n0 + r;
-        for (int m = half; m < p.M; m += kN4Threads / kTcRows) {
-            float x = 0.f;
-            for (int s0 = 0; s0 < p.splits; s0 += 8) {
-                float v[8];
-#pragma unroll
-                for (int u = 0; u < 8; ++u)
-                    v[u] = (s0 + u < p.splits) ? __ldcg(base + ((size_t)(s0 + u) * NB + m) * kTcRows + r) : 0.f;
-#pragma unroll
-                for (int u = 0; u < 8; ++u) x += v[u];
-            }
-            x *= p.alpha;
-            const size_t o = (size_t)m * p.N + nn;
-            if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[nn]);
+    if (warp == Q_WARPS + 1) tmem_dealloc(tmem, TMEM_COLS);
+    if (p.splits > 1) asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp >= Q_WARPS) return;
+    const int parts = nkb_total > 0 ? (nkb_total + p.kper - 1) / p.kper : 0;              // blocks that had any k
+    const float* part = (const float*)(smem + (ring - smem_u32(smem)));
+    const float alpha = p.alpha * 256.f;
+    // a thread's column of the output; PAIRED: the gate's column in the partial rows, the up value `other` columns on
+    constexpr bool PAIRED = FORM == Q_SWIGLU || FORM == Q_GATEUP;
+    constexpr int OUT = PAIRED ? 64 : 128, OTHER = FORM == Q_SWIGLU ? 8 : 64;
+    const int oc = tid & (OUT - 1), c = FORM == Q_SWIGLU ? (oc >> 3) * 16 + (oc & 7) : oc;
+    const int n = FORM == Q_SWIGLU ? n0 / 2 + oc : n0 + oc, ldc = FORM == Q_SWIGLU ? p.N / 2 : p.N;
+    for (int slot = tid / OUT; slot * p.splits + rank < rows; slot += Q_WARPS * 32 / OUT) {
+        const int m = slot * p.splits + rank;
+        float x = 0.f, u = 0.f;
+        for (int s = 0; s < parts; ++s) {
+            x += part[(s * slots + slot) * kTcRows + c];
+            if (PAIRED) u += part[(s * slots + slot) * kTcRows + c + OTHER];
+        }
+        x *= alpha;
+        const size_t o = (size_t)(row0 + m) * ldc + n;
+        if constexpr (PAIRED) p.C[o] = f32_to_bf16_bits(round_bf16(silu_ref(round_bf16(x))) * round_bf16(u * alpha));
+        else {
+            if (p.bias) x = round_bf16(x) + bf16_bits_to_f32(p.bias[n]);
             p.C[o] = p.residual ? hadd_bf16_bits(x, p.residual[o]) : f32_to_bf16_bits(x);
         }
     }
-    if (tid == 0) p.counters[tile] = 0;
 }
 
-static float* g_n4_ws = nullptr;
-static unsigned* g_n4_cnt = nullptr;
-static const size_t kN4WsBytes = 96ull << 20;
-static const int kN4MaxTiles = 8192;
+template <int NB, int FORM>
+cudaError_t n4_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int splits) {
+    static bool configured = false;
+    if (!configured) {
+        const cudaError_t e = cudaFuncSetAttribute(gemm_nvf4_tc_kernel<NB, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)q_smem(NB));
+        if (e != cudaSuccess) return e;
+        configured = true;
+    }
+    cfg->blockDim = dim3(Q_THREADS);
+    cfg->dynamicSmemBytes = q_smem(NB);
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = splits; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg->attrs = at;
+    cfg->numAttrs = 1;
+    return cudaSuccess;
+}
 
-template <int NB>
-static int launch_n4(N4Params p, cudaStream_t st) {
-    const int tiles = p.N / kTcRows, nkb = p.K / kN4BK;
+// Blocks that the device holds at one time in clusters of s, counted as in gemm_tc.cu
+int n4_held(int s) {
+    static int held[9] = {};
+    if (held[s] == 0) {
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute at[2];
+        int n = 0;
+        cfg.gridDim = dim3(s, 64);
+        if (n4_config<64, Q_PLAIN>(&cfg, at, s) != cudaSuccess || cudaOccupancyMaxActiveClusters(&n, gemm_nvf4_tc_kernel<64, Q_PLAIN>, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            n = 0;
+        }
+        held[s] = n > 0 ? n * s : -1;
+    }
+    return held[s];
+}
+
+// Blocks per tile: a k block takes 450 cycles of the SM that converts it and 600 at least from one to the next in a block; start and
+// end cost 6000 cycles, half of it hidden where two blocks share an SM, an exchange 2000 more.
+int n4_splits(long long tiles, int nkb) {
     const int sms = sm_count();
-    int splits = 1;
-    double best = -1.0;
-    for (int s = 1; s <= 12 && s * 2 <= (nkb < 2 ? 2 : nkb); ++s) {
-        const long ctas = (long)tiles * s;
-        const long waves = (ctas + sms - 1) / sms;
-        const int per = (nkb + s - 1) / s;
-        const double t = (double)waves * (per + 2.0);      // whole waves; ~2 blocks of fixed cost per CTA
-        const double score = 1.0 / t - 1e-6 * s;
-        if (score > best) { best = score; splits = s; }
+    int best = 1;
+    double best_cost = 1e30;
+    for (int s = 1; s <= 8; ++s) {
+        if (s > 1 && (nkb < 2 * s || n4_held(s) <= 0)) continue;
+        const double blocks = (double)tiles * s;
+        const int held = s == 1 ? 2 * sms : n4_held(s);
+        const double rounds = (double)(long long)((blocks + held - 1) / held), per_sm = blocks <= sms ? 1.0 : fmin(2.0, blocks / sms);
+        const double cost = rounds * ((nkb + s - 1) / s) * fmax(per_sm * 450.0, 600.0) + 6000.0 + (rounds - 1.0) * 3000.0 + (s > 1 ? 2000.0 : 0.0);
+        if (cost < best_cost * 0.999) { best_cost = cost; best = s; }
     }
-    while (splits > 1 && (size_t)tiles * splits * NB * kTcRows * sizeof(float) > kN4WsBytes) --splits;
-    if (!g_n4_ws) {
-        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-        cudaStreamIsCapturing(st, &cs);
-        PGK_REQUIRE(cs == cudaStreamCaptureStatusNone,
-                    "gemm_nvf4_tc failed: first call must happen outside graph capture (workspace allocation)");
-        PGK_CUDA(cudaMalloc(&g_n4_ws, kN4WsBytes));
-        PGK_CUDA(cudaMalloc(&g_n4_cnt, kN4MaxTiles * sizeof(unsigned)));
-        PGK_CUDA(cudaMemset(g_n4_cnt, 0, kN4MaxTiles * sizeof(unsigned)));
-    }
-    p.splits = splits;
-    p.ws = g_n4_ws;
-    p.counters = g_n4_cnt;
-    constexpr size_t kSmem = (size_t)kN4Stages * (kTcRows * kN4BK * 2 + NB * kN4BK * 2) +
-                             (size_t)n4_raw_depth(NB) * (kN4RawW + NB * kN4BK * 2);
-    static bool attr_set = false;
-    if (!attr_set) {
-        PGK_CUDA(cudaFuncSetAttribute(gemm_nvf4_tc_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
-        attr_set = true;
-    }
-    PGK_CUDA(launch(gemm_nvf4_tc_kernel<NB>, dim3(tiles, splits), dim3(kN4Threads + 32), kSmem, st, p));
+    return best;
+}
+
+struct N4Operands { const void* A; int a_rows; const void* Bd; const void* Bs; const void* Ud; const void* Us; int matrices; int slots; long long tiles; };
+
+template <int NB, int FORM>
+int launch_n4(N4Params p, const N4Operands& b, cudaStream_t st) {
+    constexpr bool TWO = FORM == Q_GATEUP;
+    const int tiles = p.N / (TWO ? 64 : kTcRows), nkb = p.K / Q_BK;
+    p.splits = n4_splits(b.tiles, nkb);
+    p.kper = (nkb + p.splits - 1) / p.splits;
+    p.ahead = pdl_enabled();
+    p.err = wait_word(kWaitNvf4);
+    PGK_REQUIRE(p.err, "gemm_nvf4_tc failed: no pinned host memory");
+    PGK_REQUIRE(tma_encode_fn() != nullptr, "gemm_nvf4_tc failed: the driver does not export cuTensorMapEncodeTiled");
+    CUtensorMap wmap, smap, umap, tmap, amap;
+    const uint32_t cols = TWO ? 64 : kTcRows;
+    const uint64_t E = (uint64_t)b.matrices, N = (uint64_t)p.N, K = (uint64_t)p.K;
+    PGK_REQUIRE(tma_map_bytes_3d(&wmap, b.Bd, {N, K / 2, E}, {cols, 64, 1}) && tma_map_bytes_3d(&smap, b.Bs, {N, K / 32, E}, {cols, 4, 1}) &&
+                tma_map_bytes_3d(&umap, TWO ? b.Ud : b.Bd, {N, K / 2, E}, {cols, 64, 1}) && tma_map_bytes_3d(&tmap, TWO ? b.Us : b.Bs, {N, K / 32, E}, {cols, 4, 1}) &&
+                tma_map_bf16_2d(&amap, b.A, K, (uint64_t)b.a_rows, K * 2, 64, TWO ? 1 : NB), "gemm_nvf4_tc failed: cuTensorMapEncodeTiled refused the operands");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[2];
+    PGK_CUDA((n4_config<NB, FORM>(&cfg, at, p.splits)));
+    cfg.gridDim = dim3(p.splits, tiles, b.slots);
+    cfg.stream = st;
+    at[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // see launch_waiting
+    at[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    count_launch();
+    PGK_CUDA(cudaLaunchKernelEx(&cfg, gemm_nvf4_tc_kernel<NB, FORM>, wmap, smap, umap, tmap, amap, p));
     return 0;
 }
 
+template <int FORM> int launch_n4_rows(const N4Params& p, const N4Operands& b, cudaStream_t st) {
+    if (p.M <= 16) return launch_n4<16, FORM>(p, b, st);
+    if (p.M <= 32) return launch_n4<32, FORM>(p, b, st);
+    return launch_n4<64, FORM>(p, b, st);
+}
+
+}  // namespace
+
 bool gemm_nvf4_tc_shape_ok(int M, int K, int N, const void* A, const void* Bd, const void* Bs) {
-    return M >= 1 && M <= 64 && K % kN4BK == 0 && K >= kN4BK && N % kTcRows == 0 && N / kTcRows <= kN4MaxTiles &&
+    return M >= 1 && M <= 64 && K % Q_BK == 0 && K >= Q_BK && N % kTcRows == 0 && N / kTcRows <= Q_MAX_TILES &&
            ((uintptr_t)A % 16 == 0) && ((uintptr_t)Bd % 16 == 0) && ((uintptr_t)Bs % 16 == 0);
 }
 
+// swiglu: the columns are eight of a gate matrix and eight of an up matrix by turns, C = silu(gate) * up [M, N / 2]
 int gemm_nvf4_tc(const void* A, const void* Bd, const void* Bs, void* C, int M, int K, int N, float alpha, const void* bias,
-                 const void* residual, cudaStream_t st) {
+                 const void* residual, bool swiglu, cudaStream_t st) {
     PGK_REQUIRE(gemm_nvf4_tc_shape_ok(M, K, N, A, Bd, Bs),
                 "gemm_nvf4_tc failed: needs 1 <= M <= 64, K %% 128 == 0, N %% 128 == 0 and 16-byte aligned pointers (M=%d K=%d N=%d)",
                 M, K, N);
     N4Params p = {};
-    p.A = (const uint16_t*)A; p.Bd = (const uint8_t*)Bd; p.Bs = (const uint8_t*)Bs; p.C = (uint16_t*)C;
-    p.bias = (const uint16_t*)bias; p.residual = (const uint16_t*)residual;
+    p.C = (uint16_t*)C; p.bias = (const uint16_t*)bias; p.residual = (const uint16_t*)residual;
     p.M = M; p.K = K; p.N = N; p.alpha = alpha;
-    if (M <= 16) return launch_n4<16>(p, st);
-    if (M <= 32) return launch_n4<32>(p, st);
-    return launch_n4<64>(p, st);
+    const N4Operands b{A, M, Bd, Bs, nullptr, nullptr, 1, 1, N / kTcRows};
+    return swiglu ? launch_n4_rows<Q_SWIGLU>(p, b, st) : launch_n4_rows<Q_PLAIN>(p, b, st);
 }
 
 }  // namespace pgk
 
+using namespace pgk;
+
 extern "C" int pgk_gemm_nvf4_bf16_tc(const void* A, const void* B_data, const void* B_scale, void* C, int M, int K, int N,
                                      float alpha, const void* bias, const void* residual, void* stream) {
-    return pgk::gemm_nvf4_tc(A, B_data, B_scale, C, M, K, N, alpha, bias, residual, (cudaStream_t)stream);
+    return gemm_nvf4_tc(A, B_data, B_scale, C, M, K, N, alpha, bias, residual, false, (cudaStream_t)stream);
+}
+
+extern "C" int pgk_gemm_nvf4_wait_error(int* out) {
+    PGK_CUDA(cudaDeviceSynchronize());
+    *out = wait_raised(kWaitNvf4);
+    return 0;
+}
+
+/* The experts of `tokens` rows (pgk_moe_route_rows says who gets which): gate and up over the tokens' rows, act[r] = silu(gate) * up in the experts'
+ * order, and the down product of those rows.  K, N and the matrices as in pgk_moe_grouped_gemv_nvf4.  k is cut by how many experts there are, not by
+ * how many are held, so that a row's bits do not depend on the ranks. */
+static int experts_ok(const char* what, int tokens, int k, int K, int N, int held, std::initializer_list<const void*> ptrs) {
+    uintptr_t all = 0;
+    for (const void* q : ptrs) all |= (uintptr_t)q;
+    PGK_REQUIRE(tokens >= 1 && tokens <= 64 && k >= 1 && held >= 1 && K % Q_BK == 0 && K >= Q_BK && N % kTcRows == 0 && N / 64 <= 65535 && all % 16 == 0,
+                "%s failed: needs 1 <= tokens <= 64, K and N in multiples of 128 and 16-byte aligned pointers (tokens=%d K=%d N=%d)", what, tokens, K, N);
+    return 0;
+}
+// experts that have rows, as many as there may be and as there are in the mean: what the launch holds room for, what its k is cut by
+static int expert_slots(int tokens, int k, int experts) { return experts < tokens * k ? experts : tokens * k; }
+static long long expert_tiles(int tokens, int k, int experts, int tiles) {
+    const double used = experts * (1.0 - pow(1.0 - fmin(1.0, (double)k / experts), tokens));
+    return (long long)(used * tiles + 0.5);
+}
+
+extern "C" int pgk_moe_experts_gateup_nvf4(const void* x, const void* Bg_data, const void* Bg_scale, const void* Bu_data, const void* Bu_scale, void* act,
+                                           const int32_t* active, const int32_t* first, const int32_t* row_token, int tokens, int k, int K, int N, int experts,
+                                           int expert_offset, int num_local_experts, void* stream) {
+    if (int rc = experts_ok("moe_experts_gateup_nvf4", tokens, k, K, N, num_local_experts, {x, Bg_data, Bg_scale, Bu_data, Bu_scale})) return rc;
+    N4Params p = {};
+    p.C = (uint16_t*)act; p.M = tokens; p.K = K; p.N = N; p.alpha = 1.f;
+    p.active = active; p.first = first; p.token = row_token; p.offset = expert_offset;
+    const N4Operands b{x, tokens, Bg_data, Bg_scale, Bu_data, Bu_scale, num_local_experts, expert_slots(tokens, k, num_local_experts), expert_tiles(tokens, k, experts, N / 64)};
+    return launch_n4_rows<Q_GATEUP>(p, b, (cudaStream_t)stream);
+}
+extern "C" int pgk_moe_experts_down_nvf4(const void* act, const void* B_data, const void* B_scale, void* C, const int32_t* active, const int32_t* first,
+                                         int tokens, int k, int K, int N, int experts, int expert_offset, int num_local_experts, void* stream) {
+    if (int rc = experts_ok("moe_experts_down_nvf4", tokens, k, K, N, num_local_experts, {act, B_data, B_scale})) return rc;
+    N4Params p = {};
+    p.C = (uint16_t*)C; p.M = tokens; p.K = K; p.N = N; p.alpha = 1.f;
+    p.active = active; p.first = first; p.offset = expert_offset;
+    const N4Operands b{act, tokens * k, B_data, B_scale, nullptr, nullptr, num_local_experts, expert_slots(tokens, k, num_local_experts), expert_tiles(tokens, k, experts, N / kTcRows)};
+    return launch_n4_rows<Q_DOWN>(p, b, (cudaStream_t)stream);
 }

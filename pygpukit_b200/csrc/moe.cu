@@ -461,6 +461,115 @@ __global__ void moe_route_t1_kernel(const uint16_t* logits, uint16_t* __restrict
     if (lane < k) { indices[lane] = idx; row_ids[lane] = idx; weights[lane] = w; }
 }
 
+// ---------------------------------------------------------------------------------------------
+// A few dozen tokens whose experts run as products (gemm_tc_nvf4.cu).  One block routes them all: a warp per token chooses and weighs
+// (moe_route_warp), then the (token, slot) entries are ranked within their experts in ascending order -- 32 entries at a time by who
+// has the same expert, the 32s by a walk of one thread per expert -- and the experts that have rows are listed.  What bounds it is the
+// chain of barriers; four launches did this before (21 us for 30 tokens of 64 experts, eight each).
+constexpr int kRouteTokens = 64, kRouteEntries = 1024, kRouteExperts = 512;
+
+__global__ void __launch_bounds__(1024) moe_route_rows_kernel(const uint16_t* logits, uint16_t* weights, int32_t* active, int32_t* first, int32_t* row_token,
+                                                              int32_t* inv, int T, int E, int k, int offset, int held) {
+    __shared__ uint16_t expert_s[kRouteEntries], from_s[kRouteEntries], rank_s[kRouteEntries], seen_s[kRouteEntries / 32][kRouteExperts];
+    __shared__ int32_t first_s[kRouteExperts];
+    griddep_wait();
+    griddep_launch();
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n = T * k, groups = (n + 31) / 32;
+    for (int t = warp; t < T; t += 32) {
+        int idx;
+        uint16_t w;
+        moe_route_warp(logits + (size_t)t * E, E, k, lane, idx, w);
+        // slots without a choice of their own (fewer finite logits than slots) name expert 0 again: they share its row
+        const unsigned same = __match_any_sync(0xffffffffu, lane < k ? idx : -1 - lane);
+        if (lane < k) { expert_s[t * k + lane] = (uint16_t)idx; from_s[t * k + lane] = (uint16_t)(t * k + __ffs(same) - 1); weights[t * k + lane] = w; }
+    }
+    for (int i = tid; i < groups * kRouteExperts / 2; i += 1024) ((uint32_t*)seen_s)[i] = 0u;
+    __syncthreads();
+    if (warp < groups) {
+        const int i = warp * 32 + lane;
+        const bool own = i < n && from_s[i] == i;
+        const int e = own ? expert_s[i] : kRouteExperts + lane;                                 // nobody's entries match nothing
+        const unsigned same = __match_any_sync(0xffffffffu, e), before = same & ((1u << lane) - 1u);
+        if (own) {
+            rank_s[i] = (uint16_t)__popc(before);
+            if (!before) seen_s[warp][e] = (uint16_t)__popc(same);
+        }
+    }
+    __syncthreads();
+    int count = 0;
+    if (tid < E)
+        for (int g = 0; g < groups; ++g) { const int c = seen_s[g][tid]; seen_s[g][tid] = (uint16_t)count; count += c; }
+    if (tid < kRouteExperts) first_s[tid] = count;
+    __syncthreads();
+    if (warp == 0) {
+        int rows = 0, used = 0;
+        for (int e0 = 0; e0 < E; e0 += 32) {
+            const int e = e0 + lane, c = e < E ? first_s[e] : 0;
+            int inc = c;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += up;
+            }
+            const bool here = c > 0 && e >= offset && e - offset < held;          // another rank's rows are not listed
+            const unsigned has = __ballot_sync(0xffffffffu, here);
+            if (e < E) first_s[e] = first[e] = rows + inc - c;
+            if (here) active[1 + used + __popc(has & ((1u << lane) - 1u))] = e;
+            rows += __shfl_sync(0xffffffffu, inc, 31);
+            used += __popc(has);
+        }
+        if (lane == 0) { active[0] = used; first[E] = rows; }
+    }
+    __syncthreads();
+    if (tid < n) {
+        const int e = expert_s[tid], i = from_s[tid], r = first_s[e] + seen_s[i >> 5][e] + rank_s[i];
+        if (i == tid) row_token[r] = tid / k;
+        inv[tid] = r;
+    }
+}
+
+// out[t] = sum over the slots, in their order, of weight x the expert's row (+ residual): eight columns per thread, four rows in flight
+__global__ void __launch_bounds__(128) moe_combine_rows_bf16_kernel(const uint16_t* rows, const uint16_t* weights, const int32_t* inv, const uint16_t* residual,
+                                                                    uint16_t* out, int H, int k) {
+    __shared__ float w_s[32];
+    __shared__ int32_t r_s[32];
+    griddep_wait();
+    griddep_launch();
+    const int t = blockIdx.x, c = (blockIdx.y * 128 + threadIdx.x) * 8;
+    if (threadIdx.x < k) {
+        w_s[threadIdx.x] = bf16_bits_to_f32(weights[t * k + threadIdx.x]);
+        r_s[threadIdx.x] = inv[t * k + threadIdx.x];
+    }
+    __syncthreads();
+    if (c >= H) return;
+    uint4 res = make_uint4(0u, 0u, 0u, 0u);
+    if (residual) res = ld_act16(residual + (size_t)t * H + c);
+    float sum[8] = {};
+    for (int s0 = 0; s0 < k; s0 += 4) {
+        uint4 v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) if (s0 + j < k) v[j] = ld_act16(rows + (size_t)r_s[s0 + j] * H + c);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            if (s0 + j >= k) break;
+            const uint32_t u[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                sum[2 * q] = fmaf(w_s[s0 + j], bf16lo(u[q]), sum[2 * q]);
+                sum[2 * q + 1] = fmaf(w_s[s0 + j], bf16hi(u[q]), sum[2 * q + 1]);
+            }
+        }
+    }
+    uint32_t o[4];
+    const uint32_t r[4] = {res.x, res.y, res.z, res.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        o[q] = pack_bf16x2(sum[2 * q], sum[2 * q + 1]);
+        if (residual) o[q] = pack_bf16x2(bf16lo(o[q]) + bf16lo(r[q]), bf16hi(o[q]) + bf16hi(r[q]));
+    }
+    *(uint4*)(out + (size_t)t * H + c) = make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // gate and up GEMVs of the k routed experts + silu + multiply in one launch: one warp per (slot, n)
 // reads x once for both weight rows.  act = bf16(bf16(silu(bf16 gate)) * bf16 up), the three-launch form.
 template <bool CLEAN>
@@ -707,6 +816,25 @@ int pgk_moe_gateup_nvf4_t1(const void* x, const void* Bg_data, const void* Bg_sc
     PGK_REQUIRE(K % 32 == 0 && K >= 32, "moe_gateup_nvf4_t1 failed: K=%d must be a multiple of 32", K);
     return launch_moe_nvf4<2>(x, 0, Bg_data, Bg_scale, Bu_data, Bu_scale, act, row_expert_ids, k, K, N, expert_offset,
                               num_local_experts, stream);
+    return 0;
+}
+
+/* ---- a few dozen tokens: see moe_route_rows_kernel ---- */
+int pgk_moe_route_rows(const void* logits, void* weights, int32_t* active, int32_t* first, int32_t* row_token, int32_t* inv, int tokens, int num_experts,
+                       int k, int expert_offset, int num_local_experts, void* stream) {
+    PGK_REQUIRE(num_experts >= 1 && num_experts <= kRouteExperts && k >= 1 && k <= num_experts && k <= 32 && tokens >= 1 && tokens <= kRouteTokens &&
+                tokens * k <= kRouteEntries, "moe_route_rows failed: %d tokens, %d of %d experts", tokens, k, num_experts);
+    PGK_CUDA(launch_waiting(moe_route_rows_kernel, dim3(1), dim3(1024), 0, ST(stream), (const uint16_t*)logits, (uint16_t*)weights, active, first, row_token, inv,
+                            tokens, num_experts, k, expert_offset, num_local_experts));
+    return 0;
+}
+int pgk_moe_combine_rows_bf16(const void* expert_rows, const void* router_weights, const int32_t* inv, const void* residual, void* out, int tokens, int hidden,
+                              int k, void* stream) {
+    const uintptr_t all = (uintptr_t)expert_rows | (uintptr_t)residual | (uintptr_t)out;
+    PGK_REQUIRE(k >= 1 && k <= 32 && hidden % 8 == 0 && all % 16 == 0, "moe_combine_rows_bf16 failed: k=%d hidden=%d", k, hidden);
+    if (tokens <= 0) return 0;
+    PGK_CUDA(launch_waiting(moe_combine_rows_bf16_kernel, dim3(tokens, (hidden + 1023) / 1024), dim3(128), 0, ST(stream), (const uint16_t*)expert_rows,
+                            (const uint16_t*)router_weights, inv, (const uint16_t*)residual, (uint16_t*)out, hidden, k));
     return 0;
 }
 

@@ -42,6 +42,13 @@ inline bool tma_map_bytes_2d(CUtensorMap* m, const void* base, uint64_t cols, ui
     return tma_encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), d, s, b, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
                            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
+// bytes [.][rows][cols], no swizzle
+inline bool tma_map_bytes_3d(CUtensorMap* m, const void* base, const uint64_t (&dims)[3], const uint32_t (&box)[3]) {
+    const cuuint64_t d[3] = {dims[0], dims[1], dims[2]}, s[2] = {dims[0], dims[0] * dims[1]};
+    const cuuint32_t b[3] = {box[0], box[1], box[2]}, one[3] = {1, 1, 1};
+    return tma_encode_fn()(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), d, s, b, one, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 #ifdef __CUDACC__
 __device__ __forceinline__ void tma_load_2d(uint32_t smem_dst, const CUtensorMap* map, int c0, int c1, uint32_t bar) {

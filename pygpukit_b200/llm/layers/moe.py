@@ -94,7 +94,7 @@ class MoELayer:
                 "reverse": GPUArray((R,), int32), "row_ids": GPUArray((R,), int32),
                 "gathered": GPUArray((R, H), bfloat16), "act": GPUArray((R, I), bfloat16),
                 "up": GPUArray((R, I), bfloat16), "down": GPUArray((R, H), bfloat16),
-                "combine": GPUArray((T, H), bfloat16),
+                "combine": GPUArray((T, H), bfloat16), "active": GPUArray((E + 1,), int32), "row_token": GPUArray((R,), int32),
             }
             self._bufs[T] = b
         return b
@@ -124,6 +124,8 @@ class MoELayer:
         self.gate.forward(x, out=b["logits"])
         if T == 1 and _DECODE_FORM and k <= 32:
             return self._forward_t1(x, b, out, residual, st, comm if tp else None)
+        if self._as_products(x):
+            return self._forward_products(x, b, out, residual, st, comm if tp else None)
         api.moe_topk(b["logits"].device_ptr, b["weights"].device_ptr, b["indices"].device_ptr, T, E, k, 2, st)
         api.moe_softmax_topk(b["weights"].device_ptr, T, k, 2, st)
         api.moe_compute_permutation(b["indices"].device_ptr, b["counts"].device_ptr, b["offsets"].device_ptr,
@@ -144,6 +146,35 @@ class MoELayer:
                         T, H, k, st)
         if residual is not None:
             api.add(target.device_ptr, residual.device_ptr, y.device_ptr, T * H, 2, st)
+        return y
+
+    def _as_products(self, x: GPUArray) -> bool:
+        """True when the experts of x's tokens run as tensor-core products: NVF4 matrices of multiples of 128 that copies can fetch."""
+        T = x.shape[0]
+        if self.format != "nvf4" or any(p % 16 for p in [x.device_ptr] + [a.device_ptr for n in ("gate", "up", "down") for a in self._w[n]]):
+            return False
+        return (2 <= T <= 64 and self.hidden_size % 128 == 0 and self.intermediate_size % 128 == 0 and self.num_experts <= 512
+                and self.num_experts_per_tok <= 32 and T * self.num_experts_per_tok <= 1024 and os.environ.get("PGK_TC", "1") != "0")
+
+    def _forward_products(self, x: GPUArray, b: dict, out: GPUArray | None, residual: GPUArray | None, st,
+                          comm=None) -> GPUArray:
+        """Routing with the experts' row lists, gate/up with silu and mul, down, weighted sum: four launches, every expert's weights read
+        once whatever the tokens that chose it.  The roundings are those of the row-by-row pipeline; rows of remote experts are zeros."""
+        T, H, I, E, k = x.shape[0], self.hidden_size, self.intermediate_size, self.num_experts, self.num_experts_per_tok
+        (wg, sg), (wu, su), (wd, sd) = self._w["gate"], self._w["up"], self._w["down"]
+        off, nl = self.expert_offset, self.num_local_experts
+        active, first, inv = b["active"].device_ptr, b["offsets"].device_ptr, b["reverse"].device_ptr
+        api.moe_route_rows(b["logits"].device_ptr, b["weights"].device_ptr, active, first, b["row_token"].device_ptr, inv, T, E, k, off, nl, st)
+        api.moe_experts_gateup_nvf4(x.device_ptr, wg.device_ptr, sg.device_ptr, wu.device_ptr, su.device_ptr, b["act"].device_ptr, active, first,
+                                    b["row_token"].device_ptr, T, k, H, I, E, off, nl, st)
+        if nl < E:
+            api.memset(b["down"].device_ptr, 0, b["down"].nbytes, st)
+        api.moe_experts_down_nvf4(b["act"].device_ptr, wd.device_ptr, sd.device_ptr, b["down"].device_ptr, active, first, T, k, I, H, E, off, nl, st)
+        if comm is not None:
+            comm.allreduce_rows(b["down"])
+        y = out if out is not None else GPUArray((T, H), bfloat16)
+        api.moe_combine_rows_bf16(b["down"].device_ptr, b["weights"].device_ptr, inv, residual.device_ptr if residual is not None else None,
+                                  y.device_ptr, T, H, k, st)
         return y
 
     def _forward_t1(self, x: GPUArray, b: dict, out: GPUArray | None, residual: GPUArray | None, st,
