@@ -138,6 +138,67 @@ gemv_bf16_kernel(const uint16_t* A, const uint16_t* B, uint16_t* __restrict__ C,
     }
 }
 
+// Five rows and more: the slabs of four read the weights again for each, and a matrix of few columns (router logits) leaves a warp to walk a
+// whole row.  Here a block has 16 rows x 8 NT columns; its 16 warps take 32 k each by turns, both operands straight from memory in pieces
+// of eight k per lane -- which k an MMA's lane names is free as long as both operands agree -- and add up through shared memory in the
+// order of the warps.  Exact products, float32 sums (mma.sync).  B200, us, slabs -> here: 15 x 3456 -> 128 29.2 -> 4.3, 64 x 4096 -> 8 117 -> 4.3.
+constexpr int kRowsWarps = 16;
+
+template <int NT>
+__global__ void __launch_bounds__(kRowsWarps * 32) gemm_bf16_rows_kernel(const uint16_t* A, const uint16_t* B, uint16_t* C, int M, int K, int N,
+                                                                         GemvEpilogue epi) {
+    __shared__ float part[kRowsWarps][16][8 * NT + 1];
+    griddep_wait();
+    griddep_launch();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3, m0 = blockIdx.y * 16, n0 = blockIdx.x * 8 * NT;
+    const uint16_t* a0 = A + (size_t)min(m0 + g, M - 1) * K + t * 8;          // rows and columns beyond the edge repeat the last one
+    const uint16_t* a1 = A + (size_t)min(m0 + g + 8, M - 1) * K + t * 8;
+    const uint16_t* b[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) b[j] = B + (size_t)min(n0 + j * 8 + g, N - 1) * K + t * 8;
+    float acc[NT][4] = {};
+    constexpr int U = NT == 1 ? 4 : 2;
+    for (int k0 = warp * 32; k0 < K; k0 += U * kRowsWarps * 32) {
+        uint4 x0[U], x1[U], w[U][NT];
+        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * kRowsWarps * 32;
+            const bool in = k + t * 8 < K;                                    // K is a multiple of eight
+            x0[u] = in ? ld_act16(a0 + k) : zero;
+            x1[u] = in ? ld_act16(a1 + k) : zero;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) w[u][j] = in ? ld_act16(b[j] + k) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                             : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
+                             : "r"(x0[u].x), "r"(x1[u].x), "r"(x0[u].y), "r"(x1[u].y), "r"(w[u][j].x), "r"(w[u][j].y));
+                asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                             : "+f"(acc[j][0]), "+f"(acc[j][1]), "+f"(acc[j][2]), "+f"(acc[j][3])
+                             : "r"(x0[u].z), "r"(x1[u].z), "r"(x0[u].w), "r"(x1[u].w), "r"(w[u][j].z), "r"(w[u][j].w));
+            }
+    }
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) part[warp][g + (e >> 1) * 8][j * 8 + 2 * t + (e & 1)] = acc[j][e];
+    __syncthreads();
+    for (int i = threadIdx.x; i < 16 * 8 * NT; i += kRowsWarps * 32) {
+        const int r = i / (8 * NT), c = i - r * 8 * NT, m = m0 + r, n = n0 + c;
+        if (m >= M || n >= N) continue;
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < kRowsWarps; ++q) v += part[q][r][c];
+        const size_t o = (size_t)m * N + n;
+        if (epi.bias) v = round_bf16(v) + bf16_bits_to_f32(epi.bias[n]);
+        C[o] = epi.residual ? hadd_bf16_bits(v, epi.residual[o]) : f32_to_bf16_bits(v);
+    }
+}
+
 template <bool ARGMAX>
 __global__ void gemv_bf16_generic_kernel(const uint16_t* A, const uint16_t* B,
                                          uint16_t* __restrict__ C, int M, int K, int N, GemvEpilogue epi) {
@@ -220,6 +281,22 @@ static int bf16_dispatch(const void* A, const void* B, void* C, int M, int K, in
         long warps = (long)N * M;
         PGK_CUDA(launch_waiting(gemv_bf16_generic_kernel<false>, dim3((unsigned)((warps * 32 + 255) / 256)), dim3(256),
                         0, st, a, b, c, M, K, N, epi));
+        return 0;
+    }
+    // up to four rows get the bits of one row alone; a norm in front of more runs as a launch of its own, so that both ways give the same bits
+    if (M >= 5 && N <= 4096) {
+        void* normed = nullptr;
+        if (gamma) {
+            if (const int rc = scratch_alloc(&normed, (size_t)M * K * 2, st)) return rc;
+            if (pgk_rmsnorm(A, gamma, normed, M, K, eps, 2, st)) { scratch_free(normed, st); return 1; }
+            a = (const uint16_t*)normed;
+        }
+        GemvEpilogue epi = {(const uint16_t*)bias, (const uint16_t*)residual};
+        const int wide = (N + 31) / 32 * ((M + 15) / 16) >= sm_count();
+        const auto kernel = wide ? gemm_bf16_rows_kernel<4> : gemm_bf16_rows_kernel<1>;
+        const cudaError_t e = launch_waiting(kernel, dim3((N + (wide ? 31 : 7)) / (wide ? 32 : 8), (M + 15) / 16), dim3(kRowsWarps * 32), 0, st, a, b, c, M, K, N, epi);
+        if (normed) if (const int rc = scratch_free(normed, st)) return rc;
+        PGK_CUDA(e);
         return 0;
     }
     int max_m = 4;
