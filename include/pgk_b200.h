@@ -822,6 +822,10 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
 int pgk_seq_attention_wait_error(int* out);
 /* 1 when the tensor-core attention serves such rows of an aligned cache whose requests have at most `positions` positions (pages x page
  * size), else 0: single_query 2 and prompts then take the float32 kernels */
+/* Decoding (one query per request) with a request's keys cut over a cluster of blocks: how many, 0 where that kernel does not serve the layer.  The
+ * entry points below take it as `splits` with single_query = 3, no workspace and no tickets.  same_rows: the values are a prefix of the key rows. */
+int pgk_seq_attention_few_plan(int dim, int vdim, int k_ld, int v_ld, int same_rows, int heads, int kv_heads, int cache_dtype, int page_size,
+                               int requests, int keys);
 int pgk_seq_attention_tensor(int dim, int vdim, int k_ld, int v_ld, int heads, int kv_heads, int cache_dtype, long long positions);
 int pgk_seq_decode_heads_per_block(void);
 int pgk_seq_heads_per_block(int heads, int kv_heads);

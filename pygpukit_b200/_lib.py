@@ -190,13 +190,13 @@ _SIGS = {
 }
 _RESTYPE = {"pgk_last_error": C.c_char_p, "pgk_launch_count": i64, "pgk_launch_count_reset": None,
             "pgk_sdpa_workspace_bytes": sz, "pgk_p2p_handle_bytes": sz, "pgk_p2p_ready": i32,
-            "pgk_p2p_max_bytes": sz, "pgk_sm_count": i32, "pgk_seq_attention_tensor": i32, "pgk_seq_heads_per_block": i32, "pgk_seq_queries_per_tile": i32,
+            "pgk_p2p_max_bytes": sz, "pgk_sm_count": i32, "pgk_seq_attention_tensor": i32, "pgk_seq_attention_few_plan": i32, "pgk_seq_heads_per_block": i32, "pgk_seq_queries_per_tile": i32,
             "pgk_seq_decode_heads_per_block": i32, "pgk_seq_linear_value_slice": i32, "pgk_seq_linear_chunk_tokens": i32,
             "pgk_seq_mlstm_chunk_tokens": i32, "pgk_seq_mlstm_fused_finish": i32, "pgk_seq_mlstm_gate_floats": sz,
             "pgk_seq_gla_chunk_tokens": i32, "pgk_seq_gla_fused_finish": i32}
 _EXTRA = {"pgk_last_error": [], "pgk_launch_count": [], "pgk_launch_count_reset": [],
           "pgk_sdpa_workspace_bytes": [i32, i32, i32, i32], "pgk_p2p_handle_bytes": [], "pgk_p2p_ready": [], "pgk_p2p_max_bytes": [],
-          "pgk_sm_count": [], "pgk_seq_attention_tensor": [i32, i32, i32, i32, i32, i32, i32, C.c_longlong], "pgk_seq_heads_per_block": [i32, i32], "pgk_seq_queries_per_tile": [i32, i32],
+          "pgk_sm_count": [], "pgk_seq_attention_few_plan": [i32] * 11, "pgk_seq_attention_tensor": [i32, i32, i32, i32, i32, i32, i32, C.c_longlong], "pgk_seq_heads_per_block": [i32, i32], "pgk_seq_queries_per_tile": [i32, i32],
           "pgk_seq_decode_heads_per_block": [], "pgk_seq_linear_value_slice": [i32, i32, i32, i32], "pgk_seq_linear_chunk_tokens": [],
           "pgk_seq_mlstm_chunk_tokens": [], "pgk_seq_mlstm_fused_finish": [i32], "pgk_seq_mlstm_gate_floats": [i32, i32],
           "pgk_seq_gla_chunk_tokens": [i32, i32], "pgk_seq_gla_fused_finish": [i32]}

@@ -53,6 +53,7 @@ SOURCES = {
     "seq_gemm_tc.cu": [],
     "seq_attention.cu": [],
     "seq_attention_tc.cu": [],
+    "seq_attention_few.cu": [],
     "seq_layers.cu": [],
     "seq_latent.cu": [],
     "seq_recurrent.cu": [],
@@ -66,7 +67,7 @@ SOURCES = {
 COMPONENTS = {
     "core": ["runtime.cu"],
     # token-major float32-activation models on the paged cache (llm/models/layered.py)
-    "seq": ["runtime.cu", "seq_gemm.cu", "seq_gemm_tc.cu", "seq_attention.cu", "seq_attention_tc.cu", "seq_layers.cu", "seq_latent.cu", "seq_recurrent.cu",
+    "seq": ["runtime.cu", "seq_gemm.cu", "seq_gemm_tc.cu", "seq_attention.cu", "seq_attention_tc.cu", "seq_attention_few.cu", "seq_layers.cu", "seq_latent.cu", "seq_recurrent.cu",
             "seq_linear_tc.cu",
             "seq_gated.cu", "seq_mlstm.cu", "seq_gla.cu"],
 }

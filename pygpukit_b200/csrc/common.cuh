@@ -46,7 +46,7 @@ int  scratch_free(void* ptr, cudaStream_t st);
 
 // The word that a kernel raises when one of its bounded waits runs out: host memory that every device reaches, so that looking at it
 // costs a load.  Every call that synchronises with the device looks (wait_check) and fails once for each raised word.
-enum WaitKind { kWaitRows, kWaitFp8, kWaitFp8Rows, kWaitNvf4, kWaitAttention, kWaitPrompt, kWaitLinear, kWaitProbe, kWaitKinds };      // one per source file
+enum WaitKind { kWaitRows, kWaitFp8, kWaitFp8Rows, kWaitNvf4, kWaitAttention, kWaitFew, kWaitPrompt, kWaitLinear, kWaitProbe, kWaitKinds };      // one per source file
 int* wait_word(WaitKind kind);           // NULL when no such memory can be had
 int  wait_check();
 int  wait_raised(WaitKind kind);         // the word's value, whether or not a call has failed for it yet

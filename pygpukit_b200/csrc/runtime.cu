@@ -249,7 +249,7 @@ int* wait_word(WaitKind kind) {
     return w + kind;
 }
 int wait_check() {
-    static const char* const what[kWaitKinds] = {"gemm_rows", "gemm_fp8_tc", "gemm_fp8_rows", "gemm_nvf4_tc", "seq_attention", "sdpa_causal_fixed_cache",
+    static const char* const what[kWaitKinds] = {"gemm_rows", "gemm_fp8_tc", "gemm_fp8_rows", "gemm_nvf4_tc", "seq_attention", "seq_attention_decode", "sdpa_causal_fixed_cache",
                                                   "seq_linear_attention_chunks", "wait_probe"};
     int* w = g_wait_words.load(std::memory_order_acquire);
     if (!w) return 0;

@@ -1157,7 +1157,7 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
     PGK_REQUIRE(weight_mode == 0 || (weight_mode == 1 && !sinks), "seq_attention failed: weight mode %d", weight_mode);
     PGK_REQUIRE(cache_dtype == 0 || cache_dtype == 2, "seq_attention failed: the cache is float32 (0) or bfloat16 (2), got %d", cache_dtype);
     PGK_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && vdim > 0, "seq_attention failed: invalid head layout");
-    PGK_REQUIRE(splits >= 1 && splits <= 64 && (splits == 1 || (workspace && tickets)),
+    PGK_REQUIRE(splits >= 1 && splits <= 64 && (splits == 1 || single_query == 3 || (workspace && tickets)),
                 "seq_attention failed: 1..64 key slices, more than one needs the workspace and the tickets");
     PGK_REQUIRE(gate_mode >= 0 && gate_mode <= 2 && (gate_mode == 0 || gate_rows), "seq_attention failed: gate mode %d", gate_mode);
     PGK_REQUIRE(k_ld >= dim && v_ld >= vdim && chunk >= 0 && window >= 0, "seq_attention failed: row strides %d / %d below the head sizes", k_ld, v_ld);
@@ -1175,6 +1175,13 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
     a.scale = scale; a.cap = softcap; a.splits = splits; a.ws = workspace; a.tickets = tickets;
     a.pool = pool; a.pool_rows = pool_rows; a.pk = k_pool; a.pv = v_pool; a.o_inv_freq = out_inv_freq; a.o_pairs = out_pairs;
     PGK_REQUIRE(!a.valias || pool == 0, "seq_attention failed: pooled blocks keep their values in an array of their own");
+    if (single_query == 3) {                 // the kernel of few queries, `splits` blocks share a request's keys
+        bool served = false;
+        a.splits = 1;
+        if (cache_dtype == 2)
+            if (const int rc = seq_attention_few(a, n_tiles, splits, (cudaStream_t)stream, &served)) return rc;
+        if (served) return 0;
+    }
     if (single_query && single_query != 2)  // every tile holds one query: the decoding kernel (2: the tensor cores where they can serve)
         return cache_dtype == 2 ? launch_attn_decode_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
                                 : launch_attn_decode_nv<float>(a, n_tiles, (cudaStream_t)stream);

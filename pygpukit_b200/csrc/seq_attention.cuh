@@ -48,4 +48,8 @@ __device__ __forceinline__ float distance_term(float slope, float slope2, bool l
 // not fit its copies or the on-chip memory.
 int seq_attention_tc(const AttnArgs& a, int tiles, cudaStream_t st, bool* served);
 
+// Decoding (seq_attention_few.cu): bfloat16 cache, softmax weights, windows, chunks, distance terms, sinks, gates; `cluster` blocks share a
+// request's keys.
+int seq_attention_few(const AttnArgs& a, int tiles, int cluster, cudaStream_t st, bool* served);
+
 }  // namespace pgk

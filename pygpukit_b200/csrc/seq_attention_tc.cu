@@ -753,7 +753,7 @@ extern "C" int pgk_seq_attention_tensor(int dim, int vdim, int k_ld, int v_ld, i
 extern "C" int pgk_seq_attention_wait_error(int* out) {
     PGK_CUDA(cudaDeviceSynchronize());
     *out = 0;
-    for (pgk::WaitKind k : {pgk::kWaitAttention, pgk::kWaitPrompt, pgk::kWaitLinear})
+    for (pgk::WaitKind k : {pgk::kWaitAttention, pgk::kWaitFew, pgk::kWaitPrompt, pgk::kWaitLinear})
         if (*out == 0) *out = pgk::wait_raised(k);
     return 0;
 }

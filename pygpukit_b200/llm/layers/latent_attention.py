@@ -28,7 +28,7 @@ from ...core.factory import from_numpy
 from ...core.stream import current_stream_handle as _st
 from ..config import LatentMixerSpec
 from .linear import LinearRows
-from .paged_attention import TENSOR, key_slices
+from .paged_attention import few_decode, key_slices, launch_form
 
 
 class LatentAttentionMixer:
@@ -69,8 +69,10 @@ class LatentAttentionMixer:
         return self.down.nbytes + (self.q_up.nbytes if self.q_up is not None else 0) + self.k_absorb.nbytes + self.v_up.nbytes + self.o_proj.nbytes
 
     def key_slices(self, ctx) -> int:
-        return key_slices(ctx, self.spec.heads, 1, 0, self.spec.window, self.queries_per_tile, self.heads_per_block, self.decode_heads_per_block,
-                          tensor_dims=(self.row, self.spec.kv_rank, self.row, self.row))
+        dims = (self.row, self.spec.kv_rank, self.row, self.row)
+        few = few_decode(ctx, self.spec.heads, 1, 0, self.spec.window, self.queries_per_tile, dims, True)
+        return few or key_slices(ctx, self.spec.heads, 1, 0, self.spec.window, self.queries_per_tile, self.heads_per_block, self.decode_heads_per_block,
+                                 tensor_dims=dims)
 
     def forward(self, ctx, x: GPUArray, out: GPUArray, cache_index: int | None = None, out_scale: int | None = None) -> None:
         """x [T, W] (the block's normed rows) -> out [T, W]: stored, or out += out_scale * result when out_scale (device
@@ -96,9 +98,8 @@ class LatentAttentionMixer:
         # q~_h = Wuk_h^T q_h^nope for every head: product h reads columns h * hd .. of the queries, writes columns h * row .. of qa
         self.k_absorb.forward_seq(q_ptr, ldq, T, qa.device_ptr, H * row, epilogue=0, batch=H, a_batch=hd, c_batch=row)
         tiles_ptr, n_tiles = ctx.tiles(self.queries_per_tile)
-        form, ws, tickets = self.key_slices(ctx), None, None
-        splits = form % TENSOR
-        if splits > 1:
+        (splits, single), ws, tickets = launch_form(self.key_slices(ctx), ctx.decode_only), None, None
+        if splits > 1 and single != 3:
             ws = ctx.workspace(T * H * splits * (R + 2)).device_ptr
             tickets = b.tickets.device_ptr
         head_gate = s.out_gate and s.gate_per_head                     # a gate per element waits for the values
@@ -107,7 +108,7 @@ class LatentAttentionMixer:
                              lat.device_ptr, H * R, kc.device_ptr, kc.device_ptr, row, row, cache.dtype_code,
                              cache.table_dev.device_ptr, cache.pool.max_pages, cache.page_size, tiles_ptr, n_tiles, None,
                              self.sinks.device_ptr if self.sinks is not None else None, H, 1, row, R, 0, s.window, s.scale, 0.0,
-                             splits, ws, tickets, (2 if form >= TENSOR else 1) if ctx.decode_only else 0, _st())
+                             splits, ws, tickets, single, _st())
         gated = s.out_gate and not s.gate_per_head
         self.v_up.forward_seq(lat.device_ptr, H * R, T, vo.device_ptr, H * s.vdim, epilogue=10 if gated else 0, batch=H, a_batch=R,
                               c_batch=s.vdim, aux=(proj.device_ptr, 0, None, ld, g_off) if gated else None)

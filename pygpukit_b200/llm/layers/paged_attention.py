@@ -37,6 +37,7 @@ from .linear import LinearRows
 
 
 TENSOR = 256                 # added to a number of key slices (at most 64): decoding runs on the tensor cores
+FEW = 1024                   # added to a number of blocks per request (at most 16): decoding runs on the kernel of few queries
 
 
 def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_per_tile: int, heads_per_block: int,
@@ -73,6 +74,24 @@ def key_slices(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_
     if n_tiles * kv_heads * rep > 4096:          # one arrival counter per (tile, head block)
         return 1 + tensor
     return min(64, 1 << (want - 1).bit_length()) + tensor
+
+
+def few_decode(ctx, heads: int, kv_heads: int, chunk: int, window: int, queries_per_tile: int, dims: "tuple[int, int, int, int]", same_rows: bool) -> int:
+    """FEW + blocks per request where decoding belongs on the kernel of few queries (seq_attention_few.cu: value rows of 136 to 512), else 0.  A block
+    takes its tiles of 128 keys one after the other, a request has 16 blocks at most: up to six tiles a block it is the faster one (us, best number of key
+    slices / here: eight requests over 2000 keys 43.0 / 28.6, over 8192 69.6 / 67.6; one over 2000 40.9 / 22.5, over 16384 58 / 67.6)."""
+    if not ctx.decode_only:
+        return 0
+    cache, keys, n = ctx.cache, ctx.max_keys(chunk, window), ctx.tiles(queries_per_tile)[1]
+    blocks = api.seq_attention_few_plan(*dims, 1 if same_rows else 0, heads, kv_heads, cache.dtype_code, cache.page_size, n, keys)
+    return FEW + blocks if blocks and -(-keys // 128) <= 6 * blocks else 0
+
+
+def launch_form(form: int, decode_only: bool) -> tuple[int, int]:
+    """(key slices or blocks per request, the launch's single_query) of a form"""
+    if not decode_only:
+        return form, 0
+    return (form - FEW, 3) if form >= FEW else (form % TENSOR, 2 if form >= TENSOR else 1)
 
 
 def _tensor_decode(ctx, n_tiles: int, heads: int, kv_heads: int, rows: int, keys: int, dim: int, vdim: int, key_row: int, value_row: int) -> bool:
@@ -166,6 +185,10 @@ class PagedAttentionMixer:
 
     def key_slices(self, ctx) -> int:
         s = self.spec
+        if s.weights == "softmax" and not (s.pool or s.rot_values or s.keep_first):
+            few = few_decode(ctx, s.heads, s.kv_heads, s.chunk, s.window, self.queries_per_tile, (s.dim, s.vdim, s.dim, s.vdim), False)
+            if few:
+                return few
         return key_slices(ctx, s.heads, s.kv_heads, s.chunk, s.window, self.queries_per_tile, self.heads_per_block,
                           self.decode_heads_per_block, s.keep_first, s.pool, None if s.pool or s.rot_values else (s.dim, s.vdim, s.dim, s.vdim))
 
@@ -222,9 +245,8 @@ class PagedAttentionMixer:
                                cache.dtype_code, cache.table_dev.device_ptr, cache.pool.max_pages, cache.page_size,
                                ctx.slot_ptr, ctx.pos_ptr, _st())
         tiles_ptr, n_tiles = ctx.tiles(self.queries_per_tile)
-        form, ws, tickets = self.key_slices(ctx), None, None
-        splits = form % TENSOR
-        if splits > 1:
+        (splits, single), ws, tickets = launch_form(self.key_slices(ctx), ctx.decode_only), None, None
+        if splits > 1 and single != 3:
             ws = ctx.workspace(T * s.heads * splits * (s.vdim + 2)).device_ptr
             tickets = ctx.buf.tickets.device_ptr
         gate_mode = 0 if not s.out_gate else (2 if s.gate_per_head else 1)
@@ -238,7 +260,7 @@ class PagedAttentionMixer:
                               self.weight_bias.device_ptr if self.weight_bias is not None else None, self.out_mult, s.pool,
                               cache.pool_rows(ci), cache.pk[ci].device_ptr if s.pool else None,
                               cache.pv[ci].device_ptr if s.pool else None, self.v_inv_freq.device_ptr if s.rot_values else None,
-                              self.pairs, splits, ws, tickets, (2 if form >= TENSOR else 1) if ctx.decode_only else 0, _st())
+                              self.pairs, splits, ws, tickets, single, _st())
 
 
-__all__ = ["PagedAttentionMixer", "key_slices"]
+__all__ = ["PagedAttentionMixer", "key_slices", "few_decode", "launch_form"]
