@@ -393,14 +393,14 @@ __global__ void __launch_bounds__(FEW_MAX_WARPS * 32) gemm_few_rows_kernel(GemmA
 }
 
 // The tcgen05 form (seq_gemm_tc.cu) takes 10 us from the rounding of the rows to its last store, little more for more work; the tiles
-// below 4 us and 18 ns per k in a wave, again for every further wave.  Above 16 rows (which need no rounding pass) the line lies
+// below 4 us and 18 ns per k in a wave, again for every further wave.  Beyond the kernel of few rows (few_rows_pay), which needs no rounding pass, the line lies
 // where the two meet, by the tiles there are (us, tiles -> tcgen05): K = 64 5.2 -> 10.3 for one tile or 128, 12.4 -> 15.1 for 1024,
 // 42 -> 35 for 4608; K = 256 9.3 -> 10.4 for 128, 11.4 -> 10.5 for 256; K = 320 10.4 -> 10.4 for 32; K = 512 14.4 -> 12.4 for 4.  Groups: by
 // the tiles that have rows, groups of the mean length taken, and a little for the grid's empty ones: 32 tiles K = 384 10.4 -> 12.5, K =
 // 512 12.5 -> 12.5; 512 tiles K = 192 14.7 -> 16.5, K = 256 18.6 -> 16.5.
 inline bool many_tc_pays(const GemmArgs& a, int groups, int max_rows, int rows) {
     const double nt = (a.N + BN - 1) / BN;
-    if (!a.group_off) return a.M <= 16 || a.K * ((double)groups * ((a.M + BM - 1) / BM) * nt + 512.0) >= 180000.0;
+    if (!a.group_off) return few_rows_pay(a.M, a.N, a.K, groups) || a.K * ((double)groups * ((a.M + BM - 1) / BM) * nt + 512.0) >= 180000.0;
     const int mean = (rows + groups - 1) / groups;
     const double live = (double)groups * ((mean + BM - 1) / BM) * nt, grid = (double)groups * ((max_rows + BM - 1) / BM) * nt;
     return a.K * (2.0 * live + 0.25 * grid + 1000.0) >= 500000.0;

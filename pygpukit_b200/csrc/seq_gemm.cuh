@@ -39,7 +39,15 @@ __device__ __forceinline__ float silu_f(float z) { return z / (1.f + expf(-z)); 
 // bound of the longest group.  *served is false, and nothing is launched, when the operands do not fit its copies.
 int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_rows, cudaStream_t st, bool* served);
 
-// The same for at most 16 rows, in one launch without work memory: `batch` products over the same rows, or blocks of rows_per_block
+// Where the kernel of few rows is faster than the rounding pass and the product of many rows: up to 32 rows, for which the weights are read once, and blocks of
+// 32 that read them again out of L2 while the device has room for all of them at one time (us, many rows -> few, 24 rows: 512 x 512 8.9 -> 6.1, 2048 x
+// 2048 19.1 -> 7.2, 8192 x 2048 26.9 -> 13.9, 2048 x 32768 27.2 -> 21.5; 2048 x 2048, 64 / 128 / 192 rows 20.1 -> 10.7, 23.2 -> 14.6, 13.3 -> 16.5; 8192 x 2048, 64
+// / 128 rows 27.4 -> 23.4, 30.2 -> 47.0; 192 rows 1024 x 1024 10.5 -> 9.7, 512 x 4096 8.8 -> 7.6, 2048 x 8192 15.2 -> 30.6).
+inline bool few_rows_pay(int M, int N, int K, int batch) {
+    return M <= 32 || (M <= 256 && (double)batch * N * K * ((M + 31) / 32) <= 16777216.0);
+}
+
+// The same for few rows, in one launch without work memory: `batch` products over the same rows, or blocks of rows_per_block (at most 32)
 // rows that share the matrix a.row_group names.
 int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, cudaStream_t st, bool* served);
 

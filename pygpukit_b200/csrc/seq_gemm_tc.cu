@@ -14,7 +14,7 @@
 //   * few tiles: a cluster of 2 ... 8 blocks shares a tile, each with a part of k, and the partial sums meet in shared memory
 //     (distributed loads, added in the order of the ranks), so that all SMs pull on the weights.  How k is cut follows from the number
 //     of rows, too: the bits of a row are those of the tiles only where it is not cut, and may differ between a whole prompt and its parts;
-//   * up to 16 rows (decoding): a kernel of its own (gemm_few_tc_kernel), one launch without work memory.
+//   * up to 32 rows (decoding), and blocks of them while a product is small: a kernel of its own (gemm_few_tc_kernel), one launch without work memory.
 // Measured on B200, 2000 x 9216 x 2048: 573 us on the 64 x 64 tiles of seq_gemm.cu (132 TFLOP/s), 6 + 59 us here (1.27 PFLOP/s in
 // the product); 8000 gathered rows over 16 experts, 4096 x 2048 and 2048 x 2048: 1510 -> 262 us for both.
 #include "seq_gemm.cuh"
@@ -33,10 +33,10 @@ constexpr int TC_MAX_GROUPS = 512;
 constexpr uint32_t TC_W_BYTES = kTcRows * TBK * 2;
 constexpr uint32_t TC_RING_BYTES = 200 * 1024;
 constexpr int TC_MAX_STAGES = 10;
-constexpr int TC_DIRECT_ROWS = 16;         // rows whose activations the kernel rounds itself
-constexpr int FEW_STAGES = 5;
-constexpr uint32_t FEW_STAGE_BYTES = TC_W_BYTES + TC_DIRECT_ROWS * TBK * 2;
-constexpr uint32_t FEW_SMEM = FEW_STAGES * FEW_STAGE_BYTES + 1024;      // with 16 KB of partial rows: two blocks per SM
+constexpr int TC_DIRECT_ROWS = 32;         // rows whose activations the kernel rounds itself, in blocks of 16 or 32
+__host__ __device__ constexpr int few_stages(int r) { return r == 16 ? 5 : 4; }
+__host__ __device__ constexpr uint32_t few_stage_bytes(int r) { return TC_W_BYTES + (uint32_t)r * TBK * 2; }
+__host__ __device__ constexpr uint32_t few_smem(int r) { return few_stages(r) * few_stage_bytes(r) + 1024; }      // with the partial rows: two blocks per SM
 
 struct TcArgs {
     GemmArgs g;
@@ -349,18 +349,20 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
     if (warp == 1) tmem_dealloc(tmem, 512);
 }
 
-// ---------------------------------------------------------------- at most 16 rows
+// ---------------------------------------------------------------- up to 32 rows, and blocks of 32
 // One tile of `th` weight rows (or a share of its k) per block, two blocks per SM: the next block's start -- barriers, TMEM,
 // the first copies' way from HBM, 5000 cycles -- hides behind the other's stream.  No work memory: the epilogue warps, idle until
 // the tile is done, round the float32 rows into the stages, eight k blocks per fence (a fence also waits for loads in flight).
 // A cluster that shares a tile along k pushes its partial rows to their owners' shared memory, one barrier, and every block
-// finishes its rows.  Measured at 8 rows, against a warp per column pair (gemm_few_rows_kernel): see few_tc_pays.
+// finishes its rows.  Measured at 8 rows, against a warp per column pair (gemm_few_rows_kernel): see few_tc_pays.  R: rows of the accumulator, 16 or 32;
+// more rows than that are blocks of 32 side by side (see few_rows_pay).
 // The weights are marked first to leave L2: at the default they push out what the small kernels in between keep reading (norm
 // weights, page tables, rows), which then cost 4 us more each: a decode step of 0.5 GB of weights 598 -> 536 us.  Rows that name the same
 // matrix read it at nearly the same time and lose nothing (64 rows of 4096 x 2048, all of one matrix 72.1 us, 73.6 without the mark).
 struct FewArgs {
     GemmArgs g;
     int epi, th, nkb, kper, splits, rpb, avec;
+    int blocks;          // blocks of R rows that share a matrix, one behind the other in grid.z
     int* err;
 };
 
@@ -373,12 +375,15 @@ __device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* ro
     return v;
 }
 
+template <int R>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ FewArgs p) {
+    constexpr int FEW_STAGES = few_stages(R);
+    constexpr uint32_t FEW_STAGE_BYTES = few_stage_bytes(R);
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) uint64_t full_bar[FEW_STAGES], empty_bar[FEW_STAGES], done_bar;
     __shared__ uint32_t tmem_base_s;
-    __shared__ float part[TC_DIRECT_ROWS * 2 * kTcRows];               // partial rows: [rank][row slot][128], at most 16 + 7 rows
+    __shared__ float part[(R + 7) * kTcRows];                          // partial rows: [rank][row slot][128]
     const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const uint32_t ring = (smem_u32(smem) + 1023u) & ~1023u, full = smem_u32(full_bar), empty = smem_u32(empty_bar);
     const int rank = blockIdx.x, n0 = blockIdx.y * p.th, kb0 = rank * p.kper, kb1 = min(p.nkb, kb0 + p.kper);
@@ -391,8 +396,8 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
     }
     griddep_wait();
-    const int m0 = p.rpb ? (int)blockIdx.z * p.rpb : 0, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z;
-    const int rows = z < 0 ? 0 : min(p.rpb ? p.rpb : TC_DIRECT_ROWS, p.g.M - m0);      // no matrix: nothing to do, the same in the cluster
+    const int m0 = p.rpb ? (int)blockIdx.z * p.rpb : (int)blockIdx.z % p.blocks * R, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z / p.blocks;
+    const int rows = z < 0 ? 0 : min(p.rpb ? p.rpb : R, p.g.M - m0);      // no matrix: nothing to do, the same in the cluster
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -419,7 +424,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
     } else if (rows > 0 && warp == 1) {
         if (elect_one()) {
             RingPos r;
-            constexpr uint32_t idesc = umma_idesc_bf16(TC_DIRECT_ROWS);
+            constexpr uint32_t idesc = umma_idesc_bf16(R);
             for (int kb = kb0; kb < kb1; ++kb, r.next(FEW_STAGES)) {
                 if (!bar_wait(p.err, full + 8u * r.s, r.round)) break;
                 tc_fence_after();
@@ -434,9 +439,9 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         }
         __syncwarp();
     } else if (rows > 0) {
-        // this thread's row and four columns of every k block
-        constexpr int DEPTH = 8;
-        const int et = tid - 64, r = et >> 4, c4 = et & 15;
+        // this thread's row and C groups of four columns of every k block
+        constexpr int C = R / 16, DEPTH = 8 / C, GROUP = 4 / C;
+        const int et = tid - 64, r = et / (16 / C), c4 = et % (16 / C) * C;
         const float* row = nullptr;
         if (r < rows) row = p.g.A + (size_t)(p.rpb ? 0 : z) * p.g.a_z + (size_t)(p.g.a_rows ? p.g.a_rows[m0 + r] : m0 + r) * p.g.lda;
         const uint32_t at = ring + TC_W_BYTES + (uint32_t)r * 128u + (uint32_t)(((c4 >> 1) ^ (r & 7)) << 4) + (uint32_t)(c4 & 1) * 8u;
@@ -444,54 +449,61 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         bool ok = true;
         for (int kb = kb0; kb < kb1; kb += DEPTH) {
             const int nb = min(DEPTH, kb1 - kb);
-            float4 v[DEPTH];
+            float4 v[DEPTH][C];
 #pragma unroll
-            for (int d = 0; d < DEPTH; ++d) v[d] = direct_load(p.g, d < nb ? row : nullptr, (kb + d) * TBK + c4 * 4, p.avec);
+            for (int d = 0; d < DEPTH; ++d)
+#pragma unroll
+                for (int c = 0; c < C; ++c) v[d][c] = direct_load(p.g, d < nb ? row : nullptr, (kb + d) * TBK + (c4 + c) * 4, p.avec);
             // hand over in groups that the ring can hold: a group's stages are free before any of them is written
 #pragma unroll
-            for (int d0 = 0; d0 < DEPTH; d0 += 4) {
+            for (int d0 = 0; d0 < DEPTH; d0 += GROUP) {
                 if (d0 >= nb) break;
                 RingPos h = f;
 #pragma unroll
-                for (int d = d0; d < d0 + 4; ++d) {
+                for (int d = d0; d < d0 + GROUP; ++d) {
                     if (d >= nb) break;
                     ok = ok && bar_wait(p.err, empty + 8u * f.s, f.round ^ 1u);
-                    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(at + f.s * FEW_STAGE_BYTES), "r"(pack_bf16x2(v[d].x, v[d].y)),
-                                 "r"(pack_bf16x2(v[d].z, v[d].w)) : "memory");
+                    if constexpr (C == 1)
+                        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" :: "r"(at + f.s * FEW_STAGE_BYTES), "r"(pack_bf16x2(v[d][0].x, v[d][0].y)),
+                                     "r"(pack_bf16x2(v[d][0].z, v[d][0].w)) : "memory");
+                    else
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(at + f.s * FEW_STAGE_BYTES), "r"(pack_bf16x2(v[d][0].x, v[d][0].y)),
+                                     "r"(pack_bf16x2(v[d][0].z, v[d][0].w)), "r"(pack_bf16x2(v[d][C - 1].x, v[d][C - 1].y)), "r"(pack_bf16x2(v[d][C - 1].z, v[d][C - 1].w)) : "memory");
                     f.next(FEW_STAGES);
                 }
                 fence_proxy_async();
                 __syncwarp();
                 if (lane == 0)
-                    for (int d = d0; d < min(d0 + 4, nb); ++d, h.next(FEW_STAGES)) mbar_arrive(&full_bar[h.s]);
+                    for (int d = d0; d < min(d0 + GROUP, nb); ++d, h.next(FEW_STAGES)) mbar_arrive(&full_bar[h.s]);
             }
         }
-        const int quad = warp & 3, col = n0 + quad * 32 + lane;
-        if (warp < 6) {                                   // four warps drain: lane = output column, v = the rows
+        const int quad = warp & 3, col = n0 + quad * 32 + lane, first = (warp - 2) / 4 * 16;
+        if (first < R) {                                  // four warps drain 16 rows: lane = output column, v = the rows
             bar_wait(p.err, smem_u32(&done_bar), 0);
             __syncwarp();
             tc_fence_after();
-            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16), v);
-            if (p.splits == 1) {
+            tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)first, v);
+            if (p.splits == 1 && first < rows) {
                 GemmArgs a = p.g;
                 a.N = min(a.N, n0 + p.th);
                 if (!p.rpb) {
                     a.C += (size_t)z * a.c_z;
                     if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)z * a.c_z;
                 }
-                epilogue_rows<16>(a, p.epi, v, m0, rows, col, lane);
+                epilogue_rows<16>(a, p.epi, v, m0 + first, rows - first, col, lane);
             }
         }
     }
     if (p.splits > 1) {
-        const int quad = warp & 3, col = n0 + quad * 32 + lane, slots = (rows + p.splits - 1) / p.splits;
+        const int quad = warp & 3, col = n0 + quad * 32 + lane, slots = (rows + p.splits - 1) / p.splits, first = (warp - 2) / 4 * 16;
+        const bool drains = warp >= 2 && first < R;
         __syncwarp();
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");                       // so do the others
-        if (rows > 0 && warp >= 2 && warp < 6) {          // row j belongs to block j % splits
-            int owner = 0, slot = 0;
+        if (rows > 0 && drains) {                         // row j belongs to block j % splits
+            int owner = first % p.splits, slot = first / p.splits;
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                if (j < rows) {
+                if (first + j < rows) {
                     const uint32_t to = smem_u32(part) + (uint32_t)((rank * slots + slot) * kTcRows + quad * 32 + lane) * 4u;
                     uint32_t remote;
                     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(to), "r"(owner));
@@ -502,7 +514,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         }
         __syncwarp();
         cluster_arrive_wait();
-        if (rows > 0 && warp >= 2 && warp < 6) {
+        if (rows > 0 && drains) {
             const int parts = (p.nkb + p.kper - 1) / p.kper;          // blocks that had any k
             GemmArgs a = p.g;
             a.N = min(a.N, n0 + p.th);
@@ -510,7 +522,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
                 a.C += (size_t)z * a.c_z;
                 if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)z * a.c_z;
             }
-            for (int j = rank, slot = 0; j < rows; j += p.splits, ++slot) {
+            for (int slot = first / 16, j = rank + slot * p.splits; j < rows; j += R / 16 * p.splits, slot += R / 16) {
                 float sum[1] = {0.f};
                 for (int s = 0; s < parts; ++s) sum[0] += part[(s * slots + slot) * kTcRows + quad * 32 + lane];
                 epilogue_rows<1>(a, p.epi, sum, m0 + j, 1, col, lane);
@@ -554,14 +566,14 @@ int clusters_held(int s) {
     static int held[9] = {};
     if (held[s] == 0) {
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(s, 64); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = FEW_SMEM;
+        cfg.gridDim = dim3(s, 64); cfg.blockDim = dim3(TC_THREADS); cfg.dynamicSmemBytes = few_smem(16);
         cudaLaunchAttribute at[1];
         at[0].id = cudaLaunchAttributeClusterDimension;
         at[0].val.clusterDim.x = s; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(gemm_few_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FEW_SMEM) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, gemm_few_tc_kernel, &cfg) != cudaSuccess) {
+        if (cudaFuncSetAttribute(gemm_few_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(16)) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, gemm_few_tc_kernel<16>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
         }
@@ -620,8 +632,9 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
     *served = false;
     const bool own = a.row_group != nullptr, many = own || batch > 1;
     if (a.K % 8 || a.K < TBK || (uintptr_t)a.W % 16 || (many && (a.w_stride % 8 || a.w_stride <= 0)) || !tma_encode_fn()) return 0;
-    if (a.group_off || (own ? rows_per_block : a.M) > TC_DIRECT_ROWS || (own && batch > 1) || a.M <= 0) return 0;
-    const int zs = own ? (a.M + rows_per_block - 1) / rows_per_block : batch;
+    if (a.group_off || (own && (rows_per_block > TC_DIRECT_ROWS || batch > 1)) || a.M <= 0) return 0;
+    const int R = (own ? rows_per_block : a.M) <= 16 ? 16 : TC_DIRECT_ROWS, blocks = own ? 1 : (a.M + R - 1) / R;
+    const int zs = own ? (a.M + rows_per_block - 1) / rows_per_block : batch * blocks;
     if (zs > 65535) return 0;
     FewArgs p{};
     p.g = a;
@@ -633,6 +646,7 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
     p.splits = plan.splits;
     p.kper = (p.nkb + p.splits - 1) / p.splits;
     p.rpb = own ? rows_per_block : 0;
+    p.blocks = blocks;
     p.avec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
     p.err = wait_word(kWaitRows);
     PGK_REQUIRE(p.err, "gemm_rows failed: no pinned host memory");
@@ -640,11 +654,13 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
     if (!weight_map(&wmap, a, own ? 1u << 20 : (uint64_t)batch, many, p.th)) return 0;      // row groups name matrices that exist
     static bool configured = false;
     if (!configured) {
-        PGK_CUDA(cudaFuncSetAttribute(gemm_few_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FEW_SMEM));
+        PGK_CUDA(cudaFuncSetAttribute(gemm_few_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(16)));
+        PGK_CUDA(cudaFuncSetAttribute(gemm_few_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(32)));
         configured = true;
     }
     void* args[] = {&wmap, &p};
-    const cudaError_t e = launch_clustered((const void*)gemm_few_tc_kernel, dim3(p.splits, (a.N + p.th - 1) / p.th, zs), FEW_SMEM, p.splits, st, args);
+    const cudaError_t e = launch_clustered(R == 16 ? (const void*)gemm_few_tc_kernel<16> : (const void*)gemm_few_tc_kernel<32>,
+                                           dim3(p.splits, (a.N + p.th - 1) / p.th, zs), few_smem(R), p.splits, st, args);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_few_tc", __FILE__, __LINE__);
     *served = true;
     return 0;
@@ -657,7 +673,7 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
     if (a.group_off && batch > TC_MAX_GROUPS) return 0;
     if (rows <= 0) return 0;
     const bool grouped = a.group_off != nullptr;
-    if (!grouped && a.M <= TC_DIRECT_ROWS) return gemm_few_tc(a, epilogue, batch, a.M, st, served);
+    if (!grouped && few_rows_pay(a.M, a.N, a.K, batch)) return gemm_few_tc(a, epilogue, batch, a.M, st, served);
     TcArgs p{};
     p.g = a;
     p.epi = epilogue;

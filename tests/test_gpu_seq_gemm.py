@@ -444,3 +444,10 @@ def test_products_see_weights_and_rows_written_by_the_launch_before(M):
 
     for a, b in zip(run(True), run(False)):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("M,N,K", [(17, 200, 520), (31, 129, 72), (32, 2048, 2048), (33, 130, 456), (64, 2048, 2048), (65, 2056, 2048), (255, 72, 1000), (256, 512, 1024),
+                                   (257, 512, 1024), (128, 24, 8192)])
+def test_blocks_of_few_rows(M, N, K):
+    """accumulators of 32 rows, blocks of them whose last one is not full, k cut over a cluster, and sizes beside the line to the product of many rows"""
+    test_rows(M, N, K)
