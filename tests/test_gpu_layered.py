@@ -584,3 +584,17 @@ def test_decode_steps_are_complete_for_other_streams():
     want = run(None, None)
     for side, read in ((s, None), (None, s), (s, s), (s, Stream())):
         assert all(np.array_equal(x, y) for x, y in zip(want, run(side, read)))
+
+
+@pytest.mark.parametrize("requests", [9, 20, 33])
+def test_decode_steps_of_many_requests_replay_as_they_run(requests):
+    """captured steps of up to 32 requests, their work memory included, against single launches: the same logits"""
+    outs = []
+    for graphs in (False, True):
+        cfg, _, m = make("mixed_stack")
+        m.use_graphs = graphs
+        m.init_cache(max_tokens=64 * 2 * requests, slots=requests)
+        m.step([(r, tokens(cfg, 3 + r % 5, seed=r), []) for r in range(requests)])
+        outs.append([m.step([(r, [t], [0]) for r, t in enumerate(tokens(cfg, requests, seed=100 + i))]) for i in range(5)])
+        assert bool(m._graphs) == (graphs and requests <= 32)
+    assert all(np.array_equal(a, b) for a, b in zip(*outs))
