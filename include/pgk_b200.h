@@ -521,6 +521,8 @@ int pgk_gemm_rows_f32(const float* A, int lda, const int32_t* a_rows, const void
 int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
                         float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows, int total_rows,
                         int epilogue, float scale, float cap, void* stream);
+/* In both, and in pgk_gemm_seq_f32 with rows_per_block 0: wdt 2 + 16: the rows of A are bfloat16 (lda in elements), 2 + 32: those of C, which
+ * is only written; 2 + 48: both.  For rows between two products, which round what they read: the same results. */
 /* the same for a bounded wait inside those products */
 int pgk_gemm_rows_wait_error(int* out);
 /* the same product for few rows (decoding): blocks of rows_per_block (<= 8) consecutive rows share the matrix

@@ -76,10 +76,6 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
 }
 // UE4M3 (bit 7 ignored, exponent 0 is normal) times 2^118, twice
 __device__ __forceinline__ uint32_t ue4m3_to_bf16x2(uint32_t s) { return (((s & 0x7fu) << 4) + 0x7700u) * 0x00010001u; }
-__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, int c0, const int* rows, uint32_t bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cta.global.tile::gather4.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                 :: "r"(dst), "l"(map), "r"(c0), "r"(rows[0]), "r"(rows[1]), "r"(rows[2]), "r"(rows[3]), "r"(bar) : "memory");
-}
 
 template <int NB, int FORM>
 __global__ void __launch_bounds__(Q_THREADS, q_blocks(NB))
@@ -146,7 +142,7 @@ gemm_nvf4_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
                 for (int c = 0; c < 2; ++c) {
                     if constexpr (TWO) {
                         for (int q = 0; q < quads; ++q)
-                            tma_gather4(at + (uint32_t)c * (NB * 128u) + (uint32_t)q * 512u, &amap, (kb0 + it) * Q_BK + c * 64, token_s + 4 * q, bar);
+                            tma_gather4(at + (uint32_t)c * (NB * 128u) + (uint32_t)q * 512u, &amap, (kb0 + it) * Q_BK + c * 64, token_s[4 * q], token_s[4 * q + 1], token_s[4 * q + 2], token_s[4 * q + 3], bar);
                     } else
                         tma_load_2d(at + (uint32_t)c * (NB * 128u), &amap, (kb0 + it) * Q_BK + c * 64, row0, bar);
                 }

@@ -23,21 +23,27 @@ using namespace pgk;
 
 namespace {
 
+// What a caller asks of the rows beside the weights' type: bfloat16 A (16) and C (32), for bfloat16 weights, many rows and a C that is only written.
+struct Rows16 {
+    int wdt, a16, c16;
+    explicit Rows16(int dt) : wdt(dt & 15), a16(dt >> 4 & 1), c16(dt >> 5 & 1) {}
+};
+
 template <int EPI>
 __device__ __forceinline__ void store_pair(const GemmArgs& a, int row, int col, float c0, float c1) {
     // (row, col) and (row, col + 1), col even
     if (EPI == 1) {
-        if (col + 1 < a.N) a.C[(size_t)row * a.ldc + (col >> 1)] = silu_f(c0) * c1;
+        if (col + 1 < a.N) put(a, (size_t)row * a.ldc + (col >> 1), silu_f(c0) * c1);
         return;
     }
     if (EPI == 7) {
-        if (col + 1 < a.N) a.C[(size_t)row * a.ldc + (col >> 1)] = gelu_tanh_f(c0) * c1;
+        if (col + 1 < a.N) put(a, (size_t)row * a.ldc + (col >> 1), gelu_tanh_f(c0) * c1);
         return;
     }
     if (EPI == 3) {          // scale = alpha, cap = limit
         if (col + 1 < a.N) {
             const float g = fminf(c0, a.cap), u = fminf(fmaxf(c1, -a.cap), a.cap);
-            a.C[(size_t)row * a.ldc + (col >> 1)] = g / (1.f + expf(-a.scale * g)) * (u + 1.f);
+            put(a, (size_t)row * a.ldc + (col >> 1), g / (1.f + expf(-a.scale * g)) * (u + 1.f));
         }
         return;
     }
@@ -56,19 +62,20 @@ __device__ __forceinline__ void store_pair(const GemmArgs& a, int row, int col, 
         if (col < a.N) c0 *= 1.f / (1.f + expf(-g[0]));
         if (col + 1 < a.N) c1 *= 1.f / (1.f + expf(-g[1]));
     }
-    float* p = a.C + (size_t)row * a.ldc + col;
+    const size_t at = (size_t)row * a.ldc + col;
     if (EPI == 4) {
+        float* p = a.C + at;
         if (col < a.N) p[0] = fmaf(a.colv[col], c0, p[0]);
         if (col + 1 < a.N) p[1] = fmaf(a.colv[col + 1], c1, p[1]);
         return;
     }
     if (EPI == 5) {
-        if (col < a.N) p[0] = gelu_tanh_f(c0) * aux_at(a, row, col);
-        if (col + 1 < a.N) p[1] = gelu_tanh_f(c1) * aux_at(a, row, col + 1);
+        if (col < a.N) put(a, at, gelu_tanh_f(c0) * aux_at(a, row, col));
+        if (col + 1 < a.N) put(a, at + 1, gelu_tanh_f(c1) * aux_at(a, row, col + 1));
         return;
     }
-    if (col < a.N) p[0] = c0;
-    if (col + 1 < a.N) p[1] = c1;
+    if (col < a.N) put(a, at, c0);
+    if (col + 1 < a.N) put(a, at + 1, c1);
 }
 
 constexpr int BM = 64, BN = 64, BK = 32;
@@ -85,11 +92,12 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
 }
 
 // ---------------------------------------------------------------- many rows, bfloat16 weights: tensor cores
-template <int EPI>
+template <int EPI, bool R16>
 __global__ void __launch_bounds__(128) gemm_rows_bf16_kernel(GemmArgs a) {
+    if (!R16) a.a16 = a.c16 = 0;
     const int e = blockIdx.z;
-    a.A += (size_t)e * a.a_z;
-    a.C += (size_t)e * a.c_z;
+    move_a(a, e * a.a_z);
+    move_c(a, e * a.c_z);
     if (EPI == 10) a.aux = (const float*)a.aux + (size_t)e * a.c_z;
     const int m_begin = a.group_off ? a.group_off[e] : 0;
     const int m_end = a.group_off ? a.group_off[e + 1] : a.M;
@@ -107,7 +115,7 @@ __global__ void __launch_bounds__(128) gemm_rows_bf16_kernel(GemmArgs a) {
         rows[tid] = r < m_end ? (a.a_rows ? a.a_rows[r] : r) : -1;
     }
     __syncthreads();
-    const bool avec = (a.K % 4 == 0) && (a.lda % 4 == 0) && (((uintptr_t)a.A & 15) == 0);
+    const bool avec = (a.K % 4 == 0) && (a.lda % 4 == 0) && (((uintptr_t)a.A & (a.a16 ? 7 : 15)) == 0);
     const bool wvec = (a.K % 8 == 0) && (((uintptr_t)W & 15) == 0);
 
     float4 ra[4];
@@ -118,13 +126,13 @@ __global__ void __launch_bounds__(128) gemm_rows_bf16_kernel(GemmArgs a) {
             const int idx = tid + i * 128, r = idx >> 3, c = (idx & 7) * 4, gr = rows[r], k = k0 + c;
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (gr >= 0) {
-                const float* p = a.A + (size_t)gr * a.lda + k;
-                if (avec && k + 3 < a.K) v = *(const float4*)p;
+                const size_t p = (size_t)gr * a.lda + k;
+                if (avec && k + 3 < a.K) v = a_at4(a, p);
                 else {
-                    if (k < a.K) v.x = p[0];
-                    if (k + 1 < a.K) v.y = p[1];
-                    if (k + 2 < a.K) v.z = p[2];
-                    if (k + 3 < a.K) v.w = p[3];
+                    if (k < a.K) v.x = a_at(a, p);
+                    if (k + 1 < a.K) v.y = a_at(a, p + 1);
+                    if (k + 2 < a.K) v.z = a_at(a, p + 2);
+                    if (k + 3 < a.K) v.w = a_at(a, p + 3);
                 }
             }
             ra[i] = v;
@@ -205,6 +213,7 @@ __global__ void __launch_bounds__(128) gemm_rows_bf16_kernel(GemmArgs a) {
 template <int EPI>
 __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(GemmArgs a) {
     const int e = blockIdx.z;
+    a.a16 = a.c16 = 0;
     a.A += (size_t)e * a.a_z;
     a.C += (size_t)e * a.c_z;
     if (EPI == 10) a.aux = (const float*)a.aux + (size_t)e * a.c_z;
@@ -291,6 +300,7 @@ __global__ void __launch_bounds__(FEW_MAX_WARPS * 32) gemm_few_rows_kernel(GemmA
     extern __shared__ __align__(16) float xs[];                 // [rows][K]
     const int r0 = blockIdx.y * rows_per_block;
     const int nr = min(rows_per_block, a.M - r0);
+    a.a16 = a.c16 = 0;
     const int grp = a.row_group ? a.row_group[r0] : (int)blockIdx.z;
     if (grp < 0) return;                                        // a row without a matrix (its output is formed elsewhere)
     a.A += (size_t)blockIdx.z * a.a_z;
@@ -417,7 +427,8 @@ int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream
         if (served) return 0;
     }
     dim3 grid((a.N + BN - 1) / BN, (max_rows + BM - 1) / BM, groups);
-    if (wdt == 2) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI>, grid, dim3(128), 0, st, a));
+    if (a.a16 || a.c16) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI, true>, grid, dim3(128), 0, st, a));
+    else if (wdt == 2) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI, false>, grid, dim3(128), 0, st, a));
     else PGK_CUDA(launch(gemm_rows_f32_kernel<EPI>, grid, dim3(128), 0, st, a));
     return 0;
 }
@@ -523,14 +534,16 @@ int pgk_gemm_rows_f32(const float* A, int lda, const int32_t* a_rows, const void
 int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const void* W, int wdt, long long w_group_stride,
                         float* C, int ldc, int M, int N, int K, const int32_t* group_off, int groups, int max_rows, int total_rows,
                         int epilogue, float scale, float cap, void* stream) {
-    PGK_REQUIRE(wdt == 0 || wdt == 2, "gemm_rows_f32 failed: weights must be float32 (0) or bfloat16 (2), got %d", wdt);
+    const Rows16 dt(wdt);
+    PGK_REQUIRE(wdt == 0 || (wdt & ~48) == 2, "gemm_rows_f32 failed: weights must be float32 (0) or bfloat16 (2), got %d", wdt);
+    wdt = dt.wdt;
     PGK_REQUIRE(N > 0 && K > 0 && M >= 0, "gemm_rows_f32 failed: invalid shape M=%d N=%d K=%d", M, N, K);
     PGK_REQUIRE((epilogue >= 0 && epilogue <= 2) || (epilogue >= 6 && epilogue <= 9), "gemm_rows_f32 failed: unknown epilogue %d", epilogue);
     PGK_REQUIRE((epilogue != 1 && epilogue != 7) || N % 2 == 0, "gemm_rows_f32 failed: the gate/up epilogue needs an even N");
     const int G = group_off ? groups : 1;
     const int rows = group_off ? max_rows : M;
     if (rows <= 0 || G <= 0) return 0;
-    GemmArgs a{A, a_rows, W, C, group_off, nullptr, w_group_stride, lda, ldc, M, N, K, scale, cap, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0};
+    GemmArgs a{A, a_rows, W, C, group_off, nullptr, w_group_stride, lda, ldc, M, N, K, scale, cap, nullptr, nullptr, nullptr, 0, 0, 0, 0, 0, dt.a16, dt.c16};
     cudaStream_t st = (cudaStream_t)stream;
     if (wdt == 0 && epilogue == 0 && !group_off && !a_rows && N <= 64) {        // router logits: few columns, float32 weights
         const int gx = (M + SK_WARPS * SKM - 1) / (SK_WARPS * SKM);
@@ -571,7 +584,6 @@ int pgk_gemm_few_rows_f32(const float* A, int lda, const int32_t* a_rows, const 
     return launch_few<2>(a, wdt, rows_per_block, st);
 }
 
-
 /* The general form: `batch` independent products (A columns a_batch apart, matrices w_batch apart, C columns c_batch apart)
  * over the same M rows, every epilogue.  rows_per_block > 0 selects the few-row kernel (M <= 8 rows share one pass over the
  * weights), 0 the tiled kernel. */
@@ -579,7 +591,11 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
                      long long c_batch, int M, int N, int K, int batch, int epilogue, float p0, float p1, const float* col_scale,
                      const void* aux, int aux_dtype, const int32_t* aux_rows, int aux_ld, int aux_off, int rows_per_block,
                      void* stream) {
-    PGK_REQUIRE(wdt == 0 || wdt == 2, "gemm_seq_f32 failed: weights must be float32 (0) or bfloat16 (2), got %d", wdt);
+    const Rows16 dt(wdt);
+    PGK_REQUIRE(wdt == 0 || (wdt & ~48) == 2, "gemm_seq_f32 failed: weights must be float32 (0) or bfloat16 (2), got %d", wdt);
+    PGK_REQUIRE(wdt < 16 || rows_per_block == 0, "gemm_seq_f32 failed: bfloat16 rows need the form of many rows");
+    PGK_REQUIRE(!dt.c16 || epilogue != 4, "gemm_seq_f32 failed: the scaled-accumulate epilogue adds to float32 rows");
+    wdt = dt.wdt;
     PGK_REQUIRE(N > 0 && K > 0 && M >= 0 && batch >= 1, "gemm_seq_f32 failed: invalid shape M=%d N=%d K=%d batch=%d", M, N, K, batch);
     PGK_REQUIRE(epilogue >= 0 && epilogue <= 10, "gemm_seq_f32 failed: unknown epilogue %d", epilogue);
     PGK_REQUIRE((epilogue != 1 && epilogue != 3 && epilogue != 7) || N % 2 == 0, "gemm_seq_f32 failed: a gate/up epilogue needs an even N");
@@ -589,7 +605,7 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
     PGK_REQUIRE(rows_per_block >= 0 && rows_per_block <= RMAX, "gemm_seq_f32 failed: 0..%d rows per block", RMAX);
     PGK_REQUIRE(rows_per_block == 0 || (size_t)rows_per_block * K * 4 <= 200 * 1024, "gemm_seq_f32 failed: %d rows of K=%d do not fit shared memory", rows_per_block, K);
     if (M == 0) return 0;
-    GemmArgs a{A, nullptr, W, C, nullptr, nullptr, w_batch, lda, ldc, M, N, K, p0, p1, col_scale, aux, aux_rows, aux_ld, aux_off, aux_dtype, a_batch, c_batch};
+    GemmArgs a{A, nullptr, W, C, nullptr, nullptr, w_batch, lda, ldc, M, N, K, p0, p1, col_scale, aux, aux_rows, aux_ld, aux_off, aux_dtype, a_batch, c_batch, dt.a16, dt.c16};
     cudaStream_t st = (cudaStream_t)stream;
     if (rows_per_block > 0) {
         switch (epilogue) {

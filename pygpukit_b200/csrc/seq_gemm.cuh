@@ -21,7 +21,22 @@ struct GemmArgs {
     const int* aux_rows;
     int aux_ld, aux_off, aux_dt;
     long long a_z, c_z;       // batches: elements between the A columns / C columns of consecutive products
+    int a16, c16;             // A / C are bfloat16 rows: what one product leaves and only the next one reads
 };
+
+__device__ __forceinline__ void move_a(GemmArgs& a, long long n) { a.A = a.a16 ? (const float*)((const uint16_t*)a.A + n) : a.A + n; }
+__device__ __forceinline__ void move_c(GemmArgs& a, long long n) { a.C = a.c16 ? (float*)((uint16_t*)a.C + n) : a.C + n; }
+__device__ __forceinline__ void put(const GemmArgs& a, size_t at, float v) {
+    if (a.c16) ((uint16_t*)a.C)[at] = f32_to_bf16_bits(v);
+    else a.C[at] = v;
+}
+__device__ __forceinline__ float a_at(const GemmArgs& a, size_t at) { return a.a16 ? bf16_bits_to_f32(((const uint16_t*)a.A)[at]) : a.A[at]; }
+// four elements from an even multiple of four on (16-byte float32, 8-byte bfloat16 loads)
+__device__ __forceinline__ float4 a_at4(const GemmArgs& a, size_t at) {
+    if (!a.a16) return *(const float4*)(a.A + at);
+    const uint2 v = *(const uint2*)((const uint16_t*)a.A + at);
+    return make_float4(bf16lo(v.x), bf16hi(v.x), bf16lo(v.y), bf16hi(v.y));
+}
 
 __device__ __forceinline__ float gelu_tanh_f(float z) {
     return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));

@@ -51,25 +51,25 @@ struct TcArgs {
     int* err;            // raised when a bounded wait runs out (never, unless a copy or a product is lost)
 };
 
-// ---------------------------------------------------------------- activations -> bfloat16 rows [r][batch][K]
+// ---------------------------------------------------------------- activations -> bfloat16 rows [r][batch][K] (rows that are bfloat16 already stay where they are)
 // Memory: reads 4 and writes 2 bytes per element; 16-byte accesses both ways.  2000 x 2048: 4.0 us warm, 6.0 us from HBM.
 __global__ void __launch_bounds__(256) rows_to_bf16_kernel(GemmArgs a, uint16_t* out, int batch, int kpr, bool vec) {
     griddep_wait();
     griddep_launch();
     const int r = blockIdx.x;
     if (a.group_off && r >= a.group_off[batch]) return;
-    const float* src = a.A + (size_t)(a.a_rows ? a.a_rows[r] : r) * a.lda;
+    const size_t src = (size_t)(a.a_rows ? a.a_rows[r] : r) * a.lda;
     const int nb = a.group_off ? 1 : batch, chunks = nb * kpr;                 // chunks of eight elements
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < chunks; c += gridDim.y * blockDim.x) {
         const int b = nb == 1 ? 0 : c / kpr, k = (c - b * kpr) * 8;
-        const float* p = src + (size_t)b * a.a_z + k;
+        const size_t p = src + (size_t)b * a.a_z + k;
         float v[8];
         if (vec) {
-            *(float4*)&v[0] = *(const float4*)p;
-            *(float4*)&v[4] = *(const float4*)(p + 4);
+            *(float4*)&v[0] = a_at4(a, p);
+            *(float4*)&v[4] = a_at4(a, p + 4);
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = p[j];
+            for (int j = 0; j < 8; ++j) v[j] = a_at(a, p + j);
         }
         uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
         *(uint4*)(out + ((size_t)r * nb + b) * a.K + k) = o;
@@ -124,10 +124,10 @@ __device__ __forceinline__ Tile tile_at(const TcArgs& p, const int* pre, int t) 
 template <int R, typename F>
 __device__ __forceinline__ void store_rows(const GemmArgs& a, const float (&v)[R], int row, int left, int col, F f) {
     if (col >= a.N) return;
-    float* p = a.C + (size_t)row * a.ldc + col;
+    const size_t at = (size_t)row * a.ldc + col;
 #pragma unroll
     for (int j = 0; j < R; ++j)
-        if (j < left) p[(size_t)j * a.ldc] = f(v[j], j);
+        if (j < left) put(a, at + (size_t)j * a.ldc, f(v[j], j));
 }
 // pairs (2j, 2j + 1) of columns sit in neighbouring lanes: the even lane finishes the even rows, the odd lane the odd ones
 template <int R, typename F>
@@ -135,7 +135,7 @@ __device__ __forceinline__ void store_pairs(const GemmArgs& a, const float (&v)[
     const bool odd = lane & 1;
     if constexpr (R == 1) {
         const float second = __shfl_xor_sync(0xffffffffu, v[0], 1);
-        if (!odd && col + 1 < a.N && left > 0) a.C[(size_t)row * a.ldc + (col >> 1)] = f(v[0], second);
+        if (!odd && col + 1 < a.N && left > 0) put(a, (size_t)row * a.ldc + (col >> 1), f(v[0], second));
         return;
     } else {
 #pragma unroll
@@ -143,7 +143,7 @@ __device__ __forceinline__ void store_pairs(const GemmArgs& a, const float (&v)[
             const float got = __shfl_xor_sync(0xffffffffu, odd ? v[j] : v[j + 1], 1);
             const float first = odd ? got : v[j], second = odd ? v[j + 1] : got;
             const int jj = odd ? j + 1 : j;
-            if ((col | 1) < a.N && jj < left) a.C[(size_t)(row + jj) * a.ldc + (col >> 1)] = f(first, second);
+            if ((col | 1) < a.N && jj < left) put(a, (size_t)(row + jj) * a.ldc + (col >> 1), f(first, second));
         }
     }
 }
@@ -193,6 +193,7 @@ __device__ __forceinline__ void epilogue_rows(const GemmArgs& a, int epi, const 
 }
 
 // ---------------------------------------------------------------- the product
+template <bool R16>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ CUtensorMap amap, const __grid_constant__ TcArgs p) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -295,8 +296,9 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             const int col = w.n0 + quad * 32 + lane;
             if (p.splits == 1) {
                 GemmArgs a = p.g;
+                if (!R16) a.c16 = 0;
                 if (!a.group_off) {
-                    a.C += (size_t)w.z * a.c_z;
+                    move_c(a, w.z * a.c_z);
                     if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)w.z * a.c_z;
                 }
                 for (int c = half * 16; c < w.rows; c += 32) {
@@ -326,8 +328,9 @@ gemm_rows_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_const
             const Tile w = tile_at(p, pre, first);
             const int ew = warp - 2, quad = warp & 3, half = ew >> 2, col = w.n0 + quad * 32 + lane;
             GemmArgs a = p.g;
+            if (!R16) a.c16 = 0;
             if (!a.group_off) {
-                a.C += (size_t)w.z * a.c_z;
+                move_c(a, w.z * a.c_z);
                 if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)w.z * a.c_z;
             }
             const int parts = (p.nkb + per - 1) / per;            // blocks that had any k
@@ -366,16 +369,22 @@ struct FewArgs {
     int* err;
 };
 
-__device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* row, int k, bool vec) {
+__device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* row, int k, bool vec, bool a16) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (row && k < a.K) {                        // K is a multiple of eight
-        if (vec) v = *(const float4*)(row + k);
+        if (a16) {
+            const uint16_t* h = (const uint16_t*)row + k;
+            uint2 u;
+            if (vec) u = *(const uint2*)h;
+            else u = make_uint2(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16);
+            v = make_float4(bf16lo(u.x), bf16hi(u.x), bf16lo(u.y), bf16hi(u.y));
+        } else if (vec) v = *(const float4*)(row + k);
         else { v.x = row[k]; v.y = row[k + 1]; v.z = row[k + 2]; v.w = row[k + 3]; }
     }
     return v;
 }
 
-template <int R>
+template <int R, bool R16>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ FewArgs p) {
     constexpr int FEW_STAGES = few_stages(R);
@@ -396,7 +405,8 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         asm volatile("prefetch.tensormap [%0];" :: "l"(&wmap) : "memory");
     }
     griddep_wait();
-    const int m0 = p.rpb ? (int)blockIdx.z * p.rpb : (int)blockIdx.z % p.blocks * R, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z / p.blocks;
+    int m0 = p.rpb ? (int)blockIdx.z * p.rpb : 0, z = p.rpb ? p.g.row_group[m0] : (int)blockIdx.z;
+    if (p.blocks > 1) { m0 = z % p.blocks * R; z /= p.blocks; }
     const int rows = z < 0 ? 0 : min(p.rpb ? p.rpb : R, p.g.M - m0);      // no matrix: nothing to do, the same in the cluster
     tc_fence_before();
     __syncthreads();
@@ -443,7 +453,10 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         constexpr int C = R / 16, DEPTH = 8 / C, GROUP = 4 / C;
         const int et = tid - 64, r = et / (16 / C), c4 = et % (16 / C) * C;
         const float* row = nullptr;
-        if (r < rows) row = p.g.A + (size_t)(p.rpb ? 0 : z) * p.g.a_z + (size_t)(p.g.a_rows ? p.g.a_rows[m0 + r] : m0 + r) * p.g.lda;
+        if (r < rows) {
+            const size_t off = (size_t)(p.rpb ? 0 : z) * p.g.a_z + (size_t)(p.g.a_rows ? p.g.a_rows[m0 + r] : m0 + r) * p.g.lda;
+            row = R16 && p.g.a16 ? (const float*)((const uint16_t*)p.g.A + off) : p.g.A + off;
+        }
         const uint32_t at = ring + TC_W_BYTES + (uint32_t)r * 128u + (uint32_t)(((c4 >> 1) ^ (r & 7)) << 4) + (uint32_t)(c4 & 1) * 8u;
         RingPos f;
         bool ok = true;
@@ -453,7 +466,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
 #pragma unroll
             for (int d = 0; d < DEPTH; ++d)
 #pragma unroll
-                for (int c = 0; c < C; ++c) v[d][c] = direct_load(p.g, d < nb ? row : nullptr, (kb + d) * TBK + (c4 + c) * 4, p.avec);
+                for (int c = 0; c < C; ++c) v[d][c] = direct_load(p.g, d < nb ? row : nullptr, (kb + d) * TBK + (c4 + c) * 4, p.avec, R16 && p.g.a16);
             // hand over in groups that the ring can hold: a group's stages are free before any of them is written
 #pragma unroll
             for (int d0 = 0; d0 < DEPTH; d0 += GROUP) {
@@ -477,17 +490,18 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
                     for (int d = d0; d < min(d0 + GROUP, nb); ++d, h.next(FEW_STAGES)) mbar_arrive(&full_bar[h.s]);
             }
         }
-        const int quad = warp & 3, col = n0 + quad * 32 + lane, first = (warp - 2) / 4 * 16;
-        if (first < R) {                                  // four warps drain 16 rows: lane = output column, v = the rows
+        const int quad = warp & 3, col = n0 + quad * 32 + lane, first = R > 16 ? (warp - 2) / 4 * 16 : 0;
+        if (warp < 2 + R / 4) {                                // four warps drain 16 rows: lane = output column, v = the rows
             bar_wait(p.err, smem_u32(&done_bar), 0);
             __syncwarp();
             tc_fence_after();
             tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)first, v);
             if (p.splits == 1 && first < rows) {
                 GemmArgs a = p.g;
+                if (!R16) a.c16 = 0;
                 a.N = min(a.N, n0 + p.th);
                 if (!p.rpb) {
-                    a.C += (size_t)z * a.c_z;
+                    move_c(a, z * a.c_z);
                     if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)z * a.c_z;
                 }
                 epilogue_rows<16>(a, p.epi, v, m0 + first, rows - first, col, lane);
@@ -495,8 +509,8 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         }
     }
     if (p.splits > 1) {
-        const int quad = warp & 3, col = n0 + quad * 32 + lane, slots = (rows + p.splits - 1) / p.splits, first = (warp - 2) / 4 * 16;
-        const bool drains = warp >= 2 && first < R;
+        const int quad = warp & 3, col = n0 + quad * 32 + lane, slots = (rows + p.splits - 1) / p.splits, first = R > 16 ? (warp - 2) / 4 * 16 : 0;
+        const bool drains = warp >= 2 && warp < 2 + R / 4;
         __syncwarp();
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");                       // so do the others
         if (rows > 0 && drains) {                         // row j belongs to block j % splits
@@ -517,9 +531,10 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         if (rows > 0 && drains) {
             const int parts = (p.nkb + p.kper - 1) / p.kper;          // blocks that had any k
             GemmArgs a = p.g;
+            if (!R16) a.c16 = 0;
             a.N = min(a.N, n0 + p.th);
             if (!p.rpb) {
-                a.C += (size_t)z * a.c_z;
+                move_c(a, z * a.c_z);
                 if (p.epi == 10) a.aux = (const float*)a.aux + (size_t)z * a.c_z;
             }
             for (int slot = first / 16, j = rank + slot * p.splits; j < rows; j += R / 16 * p.splits, slot += R / 16) {
@@ -572,8 +587,8 @@ int clusters_held(int s) {
         at[0].val.clusterDim.x = s; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
         cfg.attrs = at; cfg.numAttrs = 1;
         int n = 0;
-        if (cudaFuncSetAttribute(gemm_few_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(16)) != cudaSuccess ||
-            cudaOccupancyMaxActiveClusters(&n, gemm_few_tc_kernel<16>, &cfg) != cudaSuccess) {
+        if (cudaFuncSetAttribute(gemm_few_tc_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(16)) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, gemm_few_tc_kernel<16, false>, &cfg) != cudaSuccess) {
             cudaGetLastError();
             n = 0;
         }
@@ -647,20 +662,21 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
     p.kper = (p.nkb + p.splits - 1) / p.splits;
     p.rpb = own ? rows_per_block : 0;
     p.blocks = blocks;
-    p.avec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
+    p.avec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % (a.a16 ? 8 : 16) == 0;
     p.err = wait_word(kWaitRows);
     PGK_REQUIRE(p.err, "gemm_rows failed: no pinned host memory");
     CUtensorMap wmap;
     if (!weight_map(&wmap, a, own ? 1u << 20 : (uint64_t)batch, many, p.th)) return 0;      // row groups name matrices that exist
     static bool configured = false;
+    const void* const kernels[2][2] = {{(const void*)gemm_few_tc_kernel<16, false>, (const void*)gemm_few_tc_kernel<16, true>},
+                                       {(const void*)gemm_few_tc_kernel<32, false>, (const void*)gemm_few_tc_kernel<32, true>}};
     if (!configured) {
-        PGK_CUDA(cudaFuncSetAttribute(gemm_few_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(16)));
-        PGK_CUDA(cudaFuncSetAttribute(gemm_few_tc_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(32)));
+        for (int r = 0; r < 4; ++r)
+            PGK_CUDA(cudaFuncSetAttribute(kernels[r >> 1][r & 1], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem(r >> 1 ? 32 : 16)));
         configured = true;
     }
     void* args[] = {&wmap, &p};
-    const cudaError_t e = launch_clustered(R == 16 ? (const void*)gemm_few_tc_kernel<16> : (const void*)gemm_few_tc_kernel<32>,
-                                           dim3(p.splits, (a.N + p.th - 1) / p.th, zs), few_smem(R), p.splits, st, args);
+    const cudaError_t e = launch_clustered(kernels[R / 16 - 1][a.a16 || a.c16], dim3(p.splits, (a.N + p.th - 1) / p.th, zs), few_smem(R), p.splits, st, args);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_few_tc", __FILE__, __LINE__);
     *served = true;
     return 0;
@@ -674,6 +690,7 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
     if (rows <= 0) return 0;
     const bool grouped = a.group_off != nullptr;
     if (!grouped && few_rows_pay(a.M, a.N, a.K, batch)) return gemm_few_tc(a, epilogue, batch, a.M, st, served);
+    const bool direct = a.a16 && a.lda % 8 == 0 && a.a_z % 8 == 0 && (uintptr_t)a.A % 16 == 0 && !a.a_rows;
     TcArgs p{};
     p.g = a;
     p.epi = epilogue;
@@ -702,38 +719,49 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
 
     const int nb = grouped ? 1 : batch;
     void* abuf = nullptr;
-    const size_t bytes = (size_t)rows * nb * a.K * 2;
-    if (scratch_alloc(&abuf, bytes, st)) {        // no room for the copy: the tiles of seq_gemm.cu need none
-        set_error("");
-        return 0;
-    }
     CUtensorMap wmap, amap;
+    bool described = weight_map(&wmap, a, (uint64_t)batch, batch > 1, kTcRows);
     const uint64_t ad[3] = {(uint64_t)a.K, (uint64_t)nb, (uint64_t)rows};
-    const uint64_t as[2] = {(uint64_t)a.K * 2, (uint64_t)nb * a.K * 2};
     const uint32_t ab[3] = {TBK, 1, (uint32_t)p.abox};
-    if (!weight_map(&wmap, a, (uint64_t)batch, batch > 1, kTcRows) || !tma_map_bf16_3d(&amap, abuf, ad, as, ab)) {
-        scratch_free(abuf, st);
+    cudaError_t e = cudaSuccess;
+    if (direct) {                                 // rows as the product before left them: fetched where they are
+        const uint64_t as[2] = {(uint64_t)(nb > 1 ? a.a_z : a.lda) * 2, (uint64_t)a.lda * 2};
+        described = described && tma_map_bf16_3d(&amap, a.A, ad, as, ab);
+    } else {
+        const size_t bytes = (size_t)rows * nb * a.K * 2;
+        if (scratch_alloc(&abuf, bytes, st)) {    // no room for the copy: the tiles of seq_gemm.cu need none
+            set_error("");
+            return 0;
+        }
+        const uint64_t as[2] = {(uint64_t)a.K * 2, (uint64_t)nb * a.K * 2};
+        described = described && tma_map_bf16_3d(&amap, abuf, ad, as, ab);
+    }
+    if (!described) {
+        if (abuf) scratch_free(abuf, st);
         set_error("gemm_rows failed: the copies of a %d x %d x %d product cannot be described", rows, a.N, a.K);
         return 1;
     }
-    const int kpr = a.K / 8, chunks = nb * kpr;
-    const bool vec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % 16 == 0;
-    int gy = (chunks + 255) / 256;
-    if (gy > 8) gy = 8;
-    cudaError_t e = launch_waiting(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, a, (uint16_t*)abuf, batch, kpr, vec);
+    if (!direct) {
+        const int kpr = a.K / 8, chunks = nb * kpr;
+        const bool vec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % (a.a16 ? 8 : 16) == 0;
+        int gy = (chunks + 255) / 256;
+        if (gy > 8) gy = 8;
+        e = launch_waiting(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, a, (uint16_t*)abuf, batch, kpr, vec);
+    }
     if (e == cudaSuccess) {
         const int sms = sm_count();
         const long long tiles = (long long)batch * p.mt * p.nt;
         const int grid = grouped ? sms : (p.splits > 1 ? (int)(tiles * p.splits) : (int)(tiles < sms ? tiles : sms));
         static bool configured = false;
         if (!configured) {
-            e = cudaFuncSetAttribute(gemm_rows_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_RING_BYTES + 1024);
+            e = cudaFuncSetAttribute(gemm_rows_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_RING_BYTES + 1024);
+            if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_rows_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_RING_BYTES + 1024);
             configured = e == cudaSuccess;
         }
         void* args[] = {&wmap, &amap, &p};
-        if (e == cudaSuccess) e = launch_clustered((const void*)gemm_rows_tc_kernel, dim3(grid), TC_RING_BYTES + 1024, p.splits, st, args);
+        if (e == cudaSuccess) e = launch_clustered(a.c16 ? (const void*)gemm_rows_tc_kernel<true> : (const void*)gemm_rows_tc_kernel<false>, dim3(grid), TC_RING_BYTES + 1024, p.splits, st, args);
     }
-    const int rc = scratch_free(abuf, st);
+    const int rc = abuf ? scratch_free(abuf, st) : 0;
     if (e != cudaSuccess) return cuda_fail(e, "gemm_rows_tc", __FILE__, __LINE__);
     *served = rc == 0;
     return rc;

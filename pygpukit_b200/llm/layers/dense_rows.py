@@ -33,14 +33,15 @@ class GatedDenseRows:
     def forward(self, ctx, h_ptr: int, out_ptr: int, out_scale: int | None = None) -> None:
         sp, T = self.spec, ctx.T
         W, act = self.gate_up.in_features, ctx.buf.shared_act
+        h16 = self.gate_up.hands_over(T, self.down)
         if sp.activation in ("silu", "gelu_tanh"):
-            self.gate_up.forward_seq(h_ptr, W, T, act.device_ptr, sp.ff, epilogue=1 if sp.activation == "silu" else 7)
+            self.gate_up.forward_seq(h_ptr, W, T, act.device_ptr, sp.ff, epilogue=1 if sp.activation == "silu" else 7, out16=h16)
         else:
-            self.gate_up.forward_seq(h_ptr, W, T, act.device_ptr, sp.ff, epilogue=3, p0=sp.alpha, p1=sp.limit)
+            self.gate_up.forward_seq(h_ptr, W, T, act.device_ptr, sp.ff, epilogue=3, p0=sp.alpha, p1=sp.limit, out16=h16)
         if out_scale is None:
-            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=0)
+            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=0, x16=h16)
         else:
-            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=4, col_scale=out_scale)
+            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=4, col_scale=out_scale, x16=h16)
 
 
 class ActivatedRows:
@@ -60,11 +61,12 @@ class ActivatedRows:
     def forward(self, ctx, h_ptr: int, out_ptr: int, out_scale: int | None = None) -> None:
         sp, T = self.spec, ctx.T
         W, act = self.up.in_features, ctx.buf.shared_act
-        self.up.forward_seq(h_ptr, W, T, act.device_ptr, sp.ff, epilogue=self.EPILOGUES[sp.activation])
+        h16 = self.up.hands_over(T, self.down)
+        self.up.forward_seq(h_ptr, W, T, act.device_ptr, sp.ff, epilogue=self.EPILOGUES[sp.activation], out16=h16)
         if out_scale is None:
-            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=0)
+            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=0, x16=h16)
         else:
-            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=4, col_scale=out_scale)
+            self.down.forward_seq(act.device_ptr, sp.ff, T, out_ptr, self.down.out_features, epilogue=4, col_scale=out_scale, x16=h16)
 
 
 class SquaredReluRows(ActivatedRows):

@@ -110,13 +110,14 @@ class LatentAttentionMixer:
                              self.sinks.device_ptr if self.sinks is not None else None, H, 1, row, R, 0, s.window, s.scale, 0.0,
                              splits, ws, tickets, single, _st())
         gated = s.out_gate and not s.gate_per_head
+        h16 = self.v_up.hands_over(T, self.o_proj)
         self.v_up.forward_seq(lat.device_ptr, H * R, T, vo.device_ptr, H * s.vdim, epilogue=10 if gated else 0, batch=H, a_batch=R,
-                              c_batch=s.vdim, aux=(proj.device_ptr, 0, None, ld, g_off) if gated else None)
+                              c_batch=s.vdim, aux=(proj.device_ptr, 0, None, ld, g_off) if gated else None, out16=h16)
         if out_scale is None:
-            self.o_proj.forward_seq(vo.device_ptr, H * s.vdim, T, out.device_ptr, self.o_proj.out_features, epilogue=0)
+            self.o_proj.forward_seq(vo.device_ptr, H * s.vdim, T, out.device_ptr, self.o_proj.out_features, epilogue=0, x16=h16)
         else:
             self.o_proj.forward_seq(vo.device_ptr, H * s.vdim, T, out.device_ptr, self.o_proj.out_features, epilogue=4,
-                                    col_scale=out_scale)
+                                    col_scale=out_scale, x16=h16)
 
     def _prep_with_query_latent(self, ctx, proj: GPUArray, ld: int, qup: GPUArray, qa: GPUArray, kc: GPUArray) -> None:
         """norms, cache row, query up-projection, rotated query tails"""

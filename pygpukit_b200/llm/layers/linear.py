@@ -280,8 +280,14 @@ class LinearRows:
     def nbytes(self) -> int:
         return self.weight.nbytes
 
-    def forward(self, x_ptr: int, ldx: int, rows: int, out_ptr: int, ldo: int, a_rows: int | None = None) -> None:
-        """out[r] = x[a_rows[r] or r] . W^T for `rows` rows (device pointers; a_rows: int32 device array or None)."""
+    def hands_over(self, rows: int, after: "LinearRows") -> int:
+        """Rows that this product writes and only `after` reads stay in bfloat16 when `after` would round them to it (the same bits, half the bytes
+        and no pass of its own for the rounding): the `out16` of this product and the `x16` of the other."""
+        return 1 if rows > self.FEW and self.wdt == 2 and after.wdt == 2 else 0
+
+    def forward(self, x_ptr: int, ldx: int, rows: int, out_ptr: int, ldo: int, a_rows: int | None = None, x16: int = 0, out16: int = 0) -> None:
+        """out[r] = x[a_rows[r] or r] . W^T for `rows` rows (device pointers; a_rows: int32 device array or None).  x16 / out16: the rows of x /
+        out are bfloat16 (more rows than FEW, bfloat16 weights)."""
         N, K = self.out_features, self.in_features
         if rows <= self.FEW and K <= self.FEW_MAX_K:
             # rows of one block share the streamed weights; their activations must fit shared memory
@@ -289,12 +295,12 @@ class LinearRows:
             api.gemm_few_rows_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt, 0, out_ptr, ldo, rows, N, K, None,
                                   per_block, self.epilogue, self.scale, self.cap, _st())
         else:
-            api.gemm_rows_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt, 0, out_ptr, ldo, rows, N, K, None, 1,
+            api.gemm_rows_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt + 16 * x16 + 32 * out16, 0, out_ptr, ldo, rows, N, K, None, 1,
                               rows, self.epilogue, self.scale, self.cap, _st())
 
     def forward_seq(self, x_ptr: int, ldx: int, rows: int, out_ptr: int, ldo: int, *, epilogue: int | None = None,
                     p0: float | None = None, p1: float | None = None, col_scale: int | None = None, aux: tuple | None = None,
-                    batch: int = 1, a_batch: int = 0, c_batch: int = 0) -> None:
+                    batch: int = 1, a_batch: int = 0, c_batch: int = 0, x16: int = 0, out16: int = 0) -> None:
         """The general product (pgk_gemm_seq_f32).  epilogue 3: clamped gate/up pairs (p0 = alpha, p1 = limit); 4: out +=
         col_scale * product (col_scale: device pointer of [N] floats); 5: gelu_tanh(product) * aux entry, aux = (table
         pointer, dtype code, row-index pointer, row stride, column offset); 10: product * sigmoid(aux element of the same row and
@@ -304,16 +310,16 @@ class LinearRows:
         epi = self.epilogue if epilogue is None else epilogue
         per_block = max(1, min(rows, self.FEW_SMEM_FLOATS // K)) if rows <= self.FEW and K <= self.FEW_MAX_K else 0
         ax = aux or (None, 0, None, 0, 0)
-        api.gemm_seq_f32(x_ptr, ldx, a_batch, self.weight.device_ptr, self.wdt, N * K if batch > 1 else 0, out_ptr, ldo, c_batch,
+        api.gemm_seq_f32(x_ptr, ldx, a_batch, self.weight.device_ptr, self.wdt + 16 * x16 + 32 * out16, N * K if batch > 1 else 0, out_ptr, ldo, c_batch,
                          rows, N, K, batch, epi, self.scale if p0 is None else p0, self.cap if p1 is None else p1, col_scale,
                          ax[0], ax[1], ax[2], ax[3], ax[4], per_block, _st())
 
     def forward_grouped(self, x_ptr: int, ldx: int, out_ptr: int, ldo: int, a_rows: int | None, group_off: int,
-                        max_rows: int, rows: int = -1) -> None:
+                        max_rows: int, rows: int = -1, x16: int = 0, out16: int = 0) -> None:
         """Rows sorted by group: run g = rows group_off[g] .. group_off[g + 1] uses matrix g.  rows: a bound on all groups'
         rows together (-1: not known; the product then runs on the general tiles)."""
         N, K = self.out_features, self.in_features
-        api.gemm_groups_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt, N * K, out_ptr, ldo, 0, N, K, group_off,
+        api.gemm_groups_f32(x_ptr, ldx, a_rows, self.weight.device_ptr, self.wdt + 16 * x16 + 32 * out16, N * K, out_ptr, ldo, 0, N, K, group_off,
                             self.groups, max_rows, rows, self.epilogue, self.scale, self.cap, _st())
 
     def forward_per_row(self, x_ptr: int, ldx: int, rows: int, out_ptr: int, ldo: int, a_rows: int | None,

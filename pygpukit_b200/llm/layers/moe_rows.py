@@ -73,15 +73,15 @@ class GroupedRouterMoE:
         else:
             api.moe_row_lists(b.moe_counts.device_ptr, b.moe_off.device_ptr, b.moe_idx.device_ptr, b.moe_rank.device_ptr,
                               b.moe_perm.device_ptr, b.moe_inv.device_ptr, self.stack, T, top, _st())
-            self.gate_up.forward_grouped(x.device_ptr, W, b.moe_act.device_ptr, ff, b.moe_perm.device_ptr,
-                                         b.moe_off.device_ptr, T, T * top)
-            self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T, T * top)
+            h16 = self.gate_up.hands_over(T, self.down)
+            self.gate_up.forward_grouped(x.device_ptr, W, b.moe_act.device_ptr, ff, b.moe_perm.device_ptr, b.moe_off.device_ptr, T, T * top, out16=h16)
+            self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T, T * top, x16=h16)
             inv = b.moe_inv.device_ptr
         base = None
         if self.shared_gate_up is not None:
-            fs = self.shared_gate_up.out_cols
-            self.shared_gate_up.forward(x.device_ptr, W, T, b.shared_act.device_ptr, fs)
-            self.shared_down.forward(b.shared_act.device_ptr, fs, T, shared_out.device_ptr, W)
+            fs, h16 = self.shared_gate_up.out_cols, self.shared_gate_up.hands_over(T, self.shared_down)
+            self.shared_gate_up.forward(x.device_ptr, W, T, b.shared_act.device_ptr, fs, out16=h16)
+            self.shared_down.forward(b.shared_act.device_ptr, fs, T, shared_out.device_ptr, W, x16=h16)
             base = shared_out.device_ptr
         return base, b.moe_parts.device_ptr, inv, b.moe_w.device_ptr, top
 
@@ -159,15 +159,15 @@ class BiasedRouterMoE:
             api.moe_row_lists(b.moe_counts.device_ptr, b.moe_off.device_ptr, b.moe_idx.device_ptr, b.moe_rank.device_ptr,
                               b.moe_perm.device_ptr, b.moe_inv.device_ptr, max(R, self.stack), T, top, _st())
             if sp.experts > 0:
-                self.gate_up.forward_grouped(x.device_ptr, W, b.moe_act.device_ptr, ff, b.moe_perm.device_ptr,
-                                             b.moe_off.device_ptr, T, T * top)
-                self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T, T * top)
+                h16 = self.gate_up.hands_over(T, self.down)
+                self.gate_up.forward_grouped(x.device_ptr, W, b.moe_act.device_ptr, ff, b.moe_perm.device_ptr, b.moe_off.device_ptr, T, T * top, out16=h16)
+                self.down.forward_grouped(b.moe_act.device_ptr, ff, b.moe_parts.device_ptr, W, None, b.moe_off.device_ptr, T, T * top, x16=h16)
             inv = b.moe_inv.device_ptr
         shared = None
         if self.shared_gate_up is not None:
-            fs = self.shared_gate_up.out_cols
-            self.shared_gate_up.forward(x.device_ptr, W, T, b.shared_act.device_ptr, fs)
-            self.shared_down.forward(b.shared_act.device_ptr, fs, T, b.y2.device_ptr, W)
+            fs, h16 = self.shared_gate_up.out_cols, self.shared_gate_up.hands_over(T, self.shared_down)
+            self.shared_gate_up.forward(x.device_ptr, W, T, b.shared_act.device_ptr, fs, out16=h16)
+            self.shared_down.forward(b.shared_act.device_ptr, fs, T, b.y2.device_ptr, W, x16=h16)
             shared = b.y2.device_ptr
         return {"mode": "experts", "parts": b.moe_parts.device_ptr, "inv": inv, "mat": mat.device_ptr if sp.router == "biased" else None,
                 "w": b.moe_w.device_ptr, "top": top, "self_rows": x.device_ptr, "shared": shared,

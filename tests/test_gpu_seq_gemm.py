@@ -451,3 +451,52 @@ def test_products_see_weights_and_rows_written_by_the_launch_before(M):
 def test_blocks_of_few_rows(M, N, K):
     """accumulators of 32 rows, blocks of them whose last one is not full, k cut over a cluster, and sizes beside the line to the product of many rows"""
     test_rows(M, N, K)
+
+
+# rows of few (17, 200 x 512), of tcgen05 (600, 300 x 2048, cut k and not), of the tiles (short k, k no multiple of 8, unaligned rows)
+@pytest.mark.parametrize("M,N,K,batch,pad", [(17, 136, 520, 1, 0), (200, 512, 256, 2, 4), (600, 1034, 512, 1, 8), (300, 128, 2048, 3, 8), (300, 130, 2048, 1, 3),
+                                             (70, 64, 40, 2, 0), (70, 66, 44, 1, 1), (40, 64, 203, 1, 0)])
+@pytest.mark.parametrize("epi", [0, 1, 3, 5, 6, 8, 10])
+def test_bfloat16_rows_between_products(M, N, K, batch, pad, epi):
+    """rows of A as the product would round them, and C rounded as the next product would: the bits of float32 rows"""
+    A, W = operands(M + N, M, N, K * 1, batch)
+    lda, F = K + pad, N // 2 if epi in (1, 3, 7) else N
+    A = np.pad(A, ((0, 0), (0, pad)))
+    rng = np.random.default_rng(5)
+    table = gk.from_numpy(rng.standard_normal((M, F * batch + 3)).astype(np.float32))
+    rows = gk.from_numpy(np.arange(M, dtype=np.int32))
+    a32, a16, w = gk.from_numpy(A), dev_w(bf16(A)), dev_w(W)
+
+    def run(x16, out16):
+        c = gk.from_numpy(np.zeros((M, F * batch + 2), np.uint16 if out16 else np.float32))
+        api.gemm_seq_f32((a16 if x16 else a32).device_ptr, lda, 0, w.device_ptr, 2 + 16 * x16 + 32 * out16, N * K if batch > 1 else 0, c.device_ptr,
+                         F * batch + 2, F if batch > 1 else 0, M, N, K, batch, epi, 1.5, 2.0, None, table.device_ptr, 0, rows.device_ptr, F * batch + 3, 1, 0, None)
+        return c.to_numpy()
+
+    want = run(0, 0)
+    assert np.array_equal(run(1, 0), want)
+    assert np.array_equal(run(0, 1), bf16(want).view(np.uint32) >> 16) and np.array_equal(run(1, 1), bf16(want).view(np.uint32) >> 16)
+    no_wait_error()
+
+
+@pytest.mark.parametrize("counts,N,K", [([30, 0, 70, 1, 9], 130, 72), ([300, 16, 0, 17, 257, 1], 256, 128), ([700, 3, 254, 130], 384, 1032), ([0, 0, 5], 64, 200),
+                                        ([1] * 40, 96, 2048), ([3, 129] * 20, 64, 97)])
+@pytest.mark.parametrize("gather", [False, True])
+def test_bfloat16_rows_of_groups(counts, N, K, gather):
+    E, R = len(counts), sum(counts)
+    A, W = operands(R + N, R, N, K, E)
+    off, src = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32), np.random.default_rng(R).integers(0, R, R + 9).astype(np.int32)
+    src[R:] = 1 << 30                                    # rows behind the last group name nothing
+    a32, a16, w, o, s = gk.from_numpy(A), dev_w(bf16(A)), dev_w(W), gk.from_numpy(off), gk.from_numpy(src)
+    lin = llm.LinearRows(w, epilogue=1)
+
+    def run(x16, out16):
+        c = gk.from_numpy(np.zeros((R, N // 2), np.uint16 if out16 else np.float32))
+        lin.forward_grouped((a16 if x16 else a32).device_ptr, K, c.device_ptr, N // 2, s.device_ptr if gather else None, o.device_ptr, max(counts),
+                            R + (9 if gather else 0), x16=x16, out16=out16)
+        return c.to_numpy()
+
+    want = run(0, 0)
+    assert np.array_equal(run(1, 0), want)
+    assert np.array_equal(run(0, 1), bf16(want).view(np.uint32) >> 16) and np.array_equal(run(1, 1), bf16(want).view(np.uint32) >> 16)
+    no_wait_error()
