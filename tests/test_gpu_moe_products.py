@@ -113,3 +113,31 @@ def test_slots_without_a_finite_choice_share_a_row():
     layer._as_products = lambda x: False
     ref = f32(layer.forward(x).to_numpy())
     assert np.isfinite(got).all() and np.linalg.norm(got - ref) <= 2.0 ** -8 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("E,k", [(1, 1), (8, 8), (128, 8), (129, 32), (512, 6)])
+def test_routing_of_unusual_logits(E, k):
+    """ties, zeros of either sign, infinities, NaN, values at the limit of what is chosen, and fewer candidates than slots"""
+    rng = np.random.default_rng(E)
+    for case in range(6):
+        z = np.round(rng.standard_normal(E) * 2) / 2 if case else np.full(E, np.nan)
+        if case == 1:
+            z = np.where(rng.random(E) < 0.5, 0.0, -0.0)
+        if case == 2:
+            z[rng.random(E) < 0.9] = -np.inf
+        if case == 3:
+            z[rng.random(E) < 0.5] = np.nan
+        if case == 4:
+            z = np.where(rng.random(E) < 0.8, -1e30, -9e29)
+        bits = (np.asarray(z, np.float32).view(np.uint32) >> 16).astype(np.uint16)
+        v = (bits.astype(np.uint32) << 16).view(np.float32)
+        left, ids, vals = {e: v[e] for e in range(E) if v[e] > np.float32(-1e30)}, [], []
+        for _ in range(k):
+            e = min(left, key=lambda i: (-left[i], i)) if left else 0
+            ids.append(e)
+            vals.append(left.pop(e) if left else np.float32(-1e30))
+        zd, wd, idd, rd = gk.from_numpy(bits), gk.from_numpy(np.zeros(k, np.uint16)), gk.from_numpy(np.full(k, -1, np.int32)), gk.from_numpy(np.full(k, -1, np.int32))
+        api.moe_route_t1(zd.device_ptr, wd.device_ptr, idd.device_ptr, rd.device_ptr, E, k, None)
+        assert idd.to_numpy().tolist() == ids and rd.to_numpy().tolist() == ids
+        ex = np.exp(np.asarray(vals, np.float64) - max(vals))
+        assert np.abs((wd.to_numpy().astype(np.uint32) << 16).view(np.float32) - ex / ex.sum()).max() <= 2.0 ** -8
