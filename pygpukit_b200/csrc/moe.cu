@@ -312,15 +312,7 @@ moe_grouped_gemv_nvf4_kernel(const uint16_t* A, const uint8_t* Bd0,
     griddep_launch();
     const int r = blockIdx.y, col0 = blockIdx.x * TILE;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int e = row_expert_ids[r] - expert_offset;
-    const int c = col0 + lane * CPL;
-    if (e < 0 || e >= num_local) {
-        if (warp == 0 && c < N) {
-#pragma unroll
-            for (int j = 0; j < CPL; ++j) if (c + j < N) C[(size_t)r * N + c + j] = 0;
-        }
-        return;
-    }
+    const int id = row_expert_ids[r];                                 // its way and that of the row are one
     for (int k0 = threadIdx.x; k0 < K; k0 += 4 * kMoeNvf4Warps * 32) {
         uint16_t v[4];
 #pragma unroll
@@ -329,6 +321,15 @@ moe_grouped_gemv_nvf4_kernel(const uint16_t* A, const uint8_t* Bd0,
 #pragma unroll
         for (int u = 0; u < 4; ++u)
             if (k0 + u * kMoeNvf4Warps * 32 < K) a_s[k0 + u * kMoeNvf4Warps * 32] = bf16_bits_to_f32(v[u]);
+    }
+    const int e = id - expert_offset;
+    const int c = col0 + lane * CPL;
+    if (e < 0 || e >= num_local) {
+        if (warp == 0 && c < N) {
+#pragma unroll
+            for (int j = 0; j < CPL; ++j) if (c + j < N) C[(size_t)r * N + c + j] = 0;
+        }
+        return;
     }
     __syncthreads();
     const uint8_t* bdp[2] = {Bd0 + (size_t)e * (K >> 1) * N, NMAT == 2 ? Bd1 + (size_t)e * (K >> 1) * N : nullptr};
@@ -659,6 +660,7 @@ __global__ void moe_combine_t1_kernel(const uint16_t* expert_out, const uint16_t
     const int h = blockIdx.x * blockDim.x + threadIdx.x;
     if (h >= H) return;
     float sum = 0.f;
+#pragma unroll 8
     for (int s = 0; s < k; ++s)
         sum = fmaf(bf16_bits_to_f32(weights[s]), bf16_bits_to_f32(expert_out[(size_t)s * H + h]), sum);
     uint16_t o = f32_to_bf16_bits(sum);
