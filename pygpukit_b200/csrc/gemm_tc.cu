@@ -298,9 +298,8 @@ cudaError_t f8tc_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* at, int sp
     return cudaSuccess;
 }
 
-// Blocks that the device holds at one time in clusters of s, as cudaOccupancyMaxActiveClusters counts them (clusters do not cross its
-// processing clusters).  For kernels that allocate tensor memory it answers with one block per SM, while two were seen to run together:
-// plans of several blocks per tile are charged rounds that they may not take.
+// Blocks that the device holds at one time in clusters of s, one per SM, as cudaOccupancyMaxActiveClusters counts them (for kernels that allocate
+// tensor memory; two per SM run together all the same).
 int f8tc_held(int s) {
     static int held[9] = {};
     if (held[s] == 0) {
@@ -317,27 +316,31 @@ int f8tc_held(int s) {
     return held[s];
 }
 
-// Blocks per tile: an SM draws 24 bytes of weights per cycle when all do (HBM), and needs 600 cycles at least from one k block of a
-// block to its next; start and end cost 6000 cycles, half of it hidden where two blocks share an SM, an exchange 2000 more.
-int f8tc_splits(int tiles, int nkb) {
-    const int sms = sm_count();
+// Blocks per tile, by what a launch takes (us, a fit of 22 matrices of 1 ... 200 MB, 6 ... 64 rows, 1 ... 8 blocks per tile, within 10 % but for 2 %
+// of them): 5 ... 6.5 for its start and end, 1.5 ... 2.4 for an exchange and 2.5 ... 5 for every further wave; per k block 0.41 ... 0.47 (16 ... 64 rows) while an SM has one block, 0.64 ... 0.78
+// once some have two, a tenth more when all do.  The device holds two blocks per SM, in clusters some less for each of its processing
+// clusters; what is left over follows in a wave of its own.  64 rows, the k blocks of HBM traffic alone as the line before -> this one: 14336 x 14336
+// 62 -> 52, 10752 x 11776 47 -> 32, 11776 x 4352 23 -> 19, 14336 x 4096 21.5 -> 19, 5120 x 10240 25 -> 20, 4096 x 6144 16 -> 14.
+double f8tc_time(int nb, int tiles, int nkb, int s) {
+    const int sms = sm_count(), c = nb <= 16 ? 0 : (nb <= 32 ? 1 : 2);
+    const double one[3] = {0.41, 0.425, 0.465}, some[3] = {0.64, 0.68, 0.775}, all[3] = {0.72, 0.74, 0.84}, ends[3] = {4.9, 5.4, 6.3}, again[3] = {2.5, 3.5, 5.0};
+    const int per = (nkb + s - 1) / s, blocks = tiles * s, held = s == 1 ? 2 * sms : 2 * sms - 5 * s, alone = f8tc_held(s);
+    auto wave = [&](int n) { return per * (n <= alone ? one[c] : some[c] + (all[c] - some[c]) * fmax(0, n - sms) / sms); };
+    const int waves = blocks / held, rest = blocks - waves * held;
+    const double full = waves * wave(held) + (rest > 0 ? wave(rest) : 0.0);
+    return ends[c] + (s > 1 ? 1.2 + 0.15 * s : 0.0) + full + again[c] * (waves - (rest > 0 ? 0 : 1));
+}
+int f8tc_splits(int nb, int tiles, int nkb) {
     int best = 1;
-    double best_cost = 1e30;
-    for (int s = 1; s <= 8; ++s) {
-        if (s > 1 && (nkb < 2 * s || f8tc_held(s) <= 0)) continue;
-        const int blocks = tiles * s;
-        const int held = s == 1 ? 2 * sms : f8tc_held(s);
-        const double rounds = (double)((blocks + held - 1) / held), per_sm = blocks <= sms ? 1.0 : fmin(2.0, (double)blocks / sms);
-        const double cost = rounds * ((nkb + s - 1) / s) * fmax(per_sm * F_W_BYTES / 24.0, 600.0) + 6000.0 + (rounds - 1.0) * 3000.0 + (s > 1 ? 2000.0 : 0.0);
-        if (cost < best_cost * 0.999) { best_cost = cost; best = s; }
-    }
+    for (int s = 2; s <= 8; ++s)
+        if (nkb >= 2 * s && f8tc_held(s) > 0 && f8tc_time(nb, tiles, nkb, s) < f8tc_time(nb, tiles, nkb, best) * 0.999) best = s;
     return best;
 }
 
 template <int NB, bool PAIR>
 int launch_f8tc(F8TcParams p, const void* A, const void* B, const void* B1, cudaStream_t st) {
     const int tiles = p.N / (PAIR ? kTcRows / 2 : kTcRows), nkb = p.K / kTcBK;
-    p.splits = f8tc_splits(tiles, nkb);
+    p.splits = f8tc_splits(NB, tiles, nkb);
     p.kper = (nkb + p.splits - 1) / p.splits;
     p.ahead = pdl_enabled();
     p.err = wait_word(kWaitFp8);
