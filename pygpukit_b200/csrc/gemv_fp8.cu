@@ -396,7 +396,6 @@ static int gemv_fp8_dispatch(const void* A, const void* B0, const void* S0, cons
     // rows per slab limited by shared memory (M*K*2 bytes) and registers
     int max_m = 4;
     while (max_m > 1 && (size_t)max_m * K * 2 + 1024 > 200 * 1024) max_m >>= 1;
-    if (swiglu && max_m > 2) max_m = 2;
     for (int m0 = 0; m0 < M;) {
         int mt = M - m0;
         if (mt > max_m) mt = max_m;
@@ -408,7 +407,9 @@ static int gemv_fp8_dispatch(const void* A, const void* B0, const void* S0, cons
         int rc = 0;
         if (swiglu) {
             if (mt == 1) rc = launch_fp8<1, 2>(am, B0, S0, B1, S1, cm, K, N, epi, st);
-            else         rc = launch_fp8<2, 2>(am, B0, S0, B1, S1, cm, K, N, epi, st);
+            else if (mt == 2) rc = launch_fp8<2, 2>(am, B0, S0, B1, S1, cm, K, N, epi, st);
+            else if (mt == 3) rc = launch_fp8<3, 2>(am, B0, S0, B1, S1, cm, K, N, epi, st);
+            else              rc = launch_fp8<4, 2>(am, B0, S0, B1, S1, cm, K, N, epi, st);
         } else {
             if (mt == 1 && tp_active_fp8()) rc = launch_fp8<1, 1, true>(am, B0, S0, nullptr, nullptr, cm, K, N, epi, st);
             else if (mt == 1) rc = launch_fp8<1, 1>(am, B0, S0, nullptr, nullptr, cm, K, N, epi, st);

@@ -550,3 +550,21 @@ def test_gemm_fp8_swiglu_many_rows_against_float64(M, K, N):
     api.gemv_fp8_swiglu_bf16(*(x.device_ptr for x in arrs), out.device_ptr, M, K, N, None)
     got = f32(out.to_numpy()).astype(np.float64)
     assert (np.abs(got - s * u) <= es * np.abs(u) + (np.abs(s) + es) * eu + 2.0 ** -8 * np.abs(s * u) + 1e-30).all()
+
+
+@pytest.mark.parametrize("K,N", [(1408, 200), (4096, 1024), (512, 7), (33024, 64)])
+@pytest.mark.parametrize("M", [2, 3, 4])
+def test_gemv_fp8_swiglu_rows_have_the_bits_of_one_row(M, K, N):
+    """gate and up of up to four rows in one pass over the weights (K = 33024: two rows, then the rest)"""
+    rng = np.random.default_rng(M * K)
+    (g, sg), (u, su) = (rand_fp8_weights(rng, N, K) for _ in range(2))
+    w = [gk.from_numpy(a) for a in (g, sg, u, su)]
+    x = rand_bf16(rng, (M, K))
+    out, one = gk.empty((M, N), gk.bfloat16), gk.empty((1, N), gk.bfloat16)
+    gx = gk.from_numpy(x)
+    api.gemv_fp8_swiglu_bf16(gx.device_ptr, *(a.device_ptr for a in w), out.device_ptr, M, K, N, None)
+    got = out.to_numpy()
+    for m in range(M):
+        xm = gk.from_numpy(x[m:m + 1])
+        api.gemv_fp8_swiglu_bf16(xm.device_ptr, *(a.device_ptr for a in w), one.device_ptr, 1, K, N, None)
+        assert np.array_equal(got[m], one.to_numpy()[0])
