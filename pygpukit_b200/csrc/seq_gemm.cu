@@ -416,11 +416,35 @@ inline bool many_tc_pays(const GemmArgs& a, int groups, int max_rows, int rows) 
     return a.K * (2.0 * live + 0.25 * grid + 1000.0) >= 500000.0;
 }
 
+inline bool off_boundaries(const GemmArgs& a, int matrices) {
+    return a.K % 8 != 0 || (uintptr_t)a.W % 16 != 0 || (matrices > 1 && a.w_stride % 8 != 0);
+}
+// Bringing the matrices to boundaries first (pad_weights) takes 2 us and 0.9 us per million elements, the tcgen05 form then what it takes; the kernels
+// for any K cost (us, before -> with it): tiles 36 ns per k and more, from 160 on always slower (9 rows 600 x 300 14.5 -> 8.3, 768 x 1004 39 -> 8.6, 5664 x 3574 236 ->
+// 29; 3500 rows 1536 x 2668 399 -> 47, 5664 x 3574 2137 -> 197); a warp per column pair 4 ns per k, 2 more for every further row (a third of that where K is
+// a multiple of four), or 2.5 us per million elements (one row 768 x 1004 6.4 -> 8.9, 1536 x 2668 20.5 -> 10.6, 5664 x 3574 56 -> 27; eight rows 600 x 300 7.1 -> 8.4, 1024 x 746
+// 16.6 -> 8.7).
+inline bool pad_pays(const GemmArgs& a, int matrices) {
+    if (a.M > RMAX) return a.K >= 160;
+    const double m = (double)matrices * a.N * a.K * 1e-6, chain = a.K * (0.004 + 0.0019 * (a.M - 1) * (a.K % 4 ? 1.0 : 0.3));
+    return a.K >= 64 && 4.5 + (chain > 2.45 * m ? chain : 2.45 * m) > 1.05 * (8.5 + 0.92 * m);
+}
+
 // bfloat16 weights go to the tcgen05 form wherever it is faster and its copies can fetch the operands; `rows` bounds the rows of
 // A (-1: the groups' total is not known here).  The tiles below serve what is left: short k, K no multiple of 8, matrices off
 // 16-byte boundaries, groups without a bound.
 template <int EPI>
 int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream_t st, int rows = -1) {
+    if (wdt == 2 && !a.group_off && off_boundaries(a, groups) && pad_pays(a, groups)) {
+        GemmArgs b;
+        bool done = false;
+        if (const int rc = pad_weights(a, groups, st, &b, &done)) return rc;
+        if (done) {
+            bool served = false;
+            const int rc = gemm_rows_tc(b, EPI, groups, rows, max_rows, st, &served), rf = scratch_free((void*)b.W, st);
+            if (rc || rf || served) return rc ? rc : rf;
+        }
+    }
     if (wdt == 2 && rows >= 0 && many_tc_pays(a, groups, max_rows, rows)) {
         bool served = false;
         if (const int rc = gemm_rows_tc(a, EPI, groups, rows, max_rows, st, &served)) return rc;
@@ -464,6 +488,16 @@ inline bool few_tc_pays(const GemmArgs& a, int rows_per_block, int batch) {
 
 template <int EPI>
 int launch_few(const GemmArgs& a, int wdt, int rows_per_block, cudaStream_t st, int batch = 1) {
+    if (wdt == 2 && !a.row_group && a.M <= rows_per_block && off_boundaries(a, batch) && pad_pays(a, batch)) {
+        GemmArgs b;
+        bool done = false;
+        if (const int rc = pad_weights(a, batch, st, &b, &done)) return rc;
+        if (done) {
+            bool served = false;
+            const int rc = gemm_few_tc(b, EPI, batch, a.M, st, &served), rf = scratch_free((void*)b.W, st);
+            if (rc || rf || served) return rc ? rc : rf;
+        }
+    }
     if (wdt == 2 && few_tc_pays(a, rows_per_block, batch)) {
         bool served = false;
         if (const int rc = gemm_few_tc(a, EPI, batch, rows_per_block, st, &served)) return rc;

@@ -22,6 +22,7 @@ struct GemmArgs {
     int aux_ld, aux_off, aux_dt;
     long long a_z, c_z;       // batches: elements between the A columns / C columns of consecutive products
     int a16, c16;             // A / C are bfloat16 rows: what one product leaves and only the next one reads
+    int ka;                   // elements of a row of A where the matrices were brought to a multiple of eight by zeros, K more (0: K)
 };
 
 __device__ __forceinline__ void move_a(GemmArgs& a, long long n) { a.A = a.a16 ? (const float*)((const uint16_t*)a.A + n) : a.A + n; }
@@ -61,6 +62,10 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
 inline bool few_rows_pay(int M, int N, int K, int batch) {
     return M <= 32 || (M <= 256 && (double)batch * N * K * ((M + 31) / 32) <= 16777216.0);
 }
+
+// Matrices whose rows the copies cannot fetch, brought to 16-byte boundaries in work memory: *b is the product on them.  *done is false, and nothing is
+// launched, without room for them.
+int pad_weights(const GemmArgs& a, int matrices, cudaStream_t st, GemmArgs* b, bool* done);
 
 // The same for few rows, in one launch without work memory: `batch` products over the same rows, or blocks of rows_per_block (at most 32)
 // rows that share the matrix a.row_group names.

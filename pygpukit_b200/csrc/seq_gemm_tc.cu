@@ -64,16 +64,47 @@ __global__ void __launch_bounds__(256) rows_to_bf16_kernel(GemmArgs a, uint16_t*
         const int b = nb == 1 ? 0 : c / kpr, k = (c - b * kpr) * 8;
         const size_t p = src + (size_t)b * a.a_z + k;
         float v[8];
-        if (vec) {
+        if (vec && k + 8 <= a.ka) {
             *(float4*)&v[0] = a_at4(a, p);
             *(float4*)&v[4] = a_at4(a, p + 4);
         } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) v[j] = a_at(a, p + j);
+            for (int j = 0; j < 8; ++j) v[j] = k + j < a.ka ? a_at(a, p + j) : 0.f;
         }
         uint4 o = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
         *(uint4*)(out + ((size_t)r * nb + b) * a.K + k) = o;
     }
+}
+
+// ---------------------------------------------------------------- matrices whose rows start anywhere -> rows of a multiple of 16 bytes, zeros behind them
+// Memory: reads and writes 2 bytes per element.  A row starts on a word or half a word behind one: four or five words per eight elements, single elements
+// at the matrices' two ends and behind a row's.  5664 x 3574 (40 MB): 15 us.
+__global__ void __launch_bounds__(256) pad_weights_kernel(const uint16_t* W, uint16_t* out, int K, int N, int kpr, long long stride, long long total) {
+    griddep_wait();
+    griddep_launch();
+    const long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (i >= total) return;
+    const long long row = i / kpr;
+    const int k = (int)(i - row * kpr) * 8, m = (int)(row / N), n = (int)(row - (long long)m * N);
+    const uint16_t* p = W + m * stride + (long long)n * K + k;
+    const bool half = ((uintptr_t)p & 2) != 0, ends = (n == 0 && k == 0) || (n == N - 1 && k + 9 > K);
+    uint32_t o[4];
+    if (k + 8 <= K && !ends) {
+        const uint32_t* q = (const uint32_t*)(p - (half ? 1 : 0));
+        uint32_t w[5];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = q[j];
+        w[4] = half ? q[4] : 0u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = half ? __funnelshift_r(w[j], w[j + 1], 16) : w[j];
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t lo = k + 2 * j < K ? p[2 * j] : 0u, hi = k + 2 * j + 1 < K ? p[2 * j + 1] : 0u;
+            o[j] = lo | hi << 16;
+        }
+    }
+    *(uint4*)(out + i * 8) = make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // ---------------------------------------------------------------- small pieces
@@ -369,22 +400,31 @@ struct FewArgs {
     int* err;
 };
 
-__device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* row, int k, bool vec, bool a16) {
+// ODD: bfloat16 rows, or rows that end within the matrix's (K is a multiple of eight, ka any number)
+template <bool ODD>
+__device__ __forceinline__ float4 direct_load(const GemmArgs& a, const float* row, int k, bool vec) {
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (row && k < a.K) {                        // K is a multiple of eight
-        if (a16) {
-            const uint16_t* h = (const uint16_t*)row + k;
-            uint2 u;
-            if (vec) u = *(const uint2*)h;
-            else u = make_uint2(h[0] | (uint32_t)h[1] << 16, h[2] | (uint32_t)h[3] << 16);
-            v = make_float4(bf16lo(u.x), bf16hi(u.x), bf16lo(u.y), bf16hi(u.y));
-        } else if (vec) v = *(const float4*)(row + k);
-        else { v.x = row[k]; v.y = row[k + 1]; v.z = row[k + 2]; v.w = row[k + 3]; }
+    if (!ODD) {
+        if (row && k < a.K) {
+            if (vec) v = *(const float4*)(row + k);
+            else { v.x = row[k]; v.y = row[k + 1]; v.z = row[k + 2]; v.w = row[k + 3]; }
+        }
+        return v;
     }
-    return v;
+    if (!row || k >= a.ka) return v;
+    const uint16_t* h = (const uint16_t*)row + k;
+    if (vec && k + 4 <= a.ka) {
+        if (!a.a16) return *(const float4*)(row + k);
+        const uint2 u = *(const uint2*)h;
+        return make_float4(bf16lo(u.x), bf16hi(u.x), bf16lo(u.y), bf16hi(u.y));
+    }
+    float e[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) e[j] = k + j < a.ka ? (a.a16 ? bf16_bits_to_f32(h[j]) : row[k + j]) : 0.f;
+    return make_float4(e[0], e[1], e[2], e[3]);
 }
 
-template <int R, bool R16>
+template <int R, bool ODD>
 __global__ void __launch_bounds__(TC_THREADS, 2)
 gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_constant__ FewArgs p) {
     constexpr int FEW_STAGES = few_stages(R);
@@ -455,7 +495,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         const float* row = nullptr;
         if (r < rows) {
             const size_t off = (size_t)(p.rpb ? 0 : z) * p.g.a_z + (size_t)(p.g.a_rows ? p.g.a_rows[m0 + r] : m0 + r) * p.g.lda;
-            row = R16 && p.g.a16 ? (const float*)((const uint16_t*)p.g.A + off) : p.g.A + off;
+            row = ODD && p.g.a16 ? (const float*)((const uint16_t*)p.g.A + off) : p.g.A + off;
         }
         const uint32_t at = ring + TC_W_BYTES + (uint32_t)r * 128u + (uint32_t)(((c4 >> 1) ^ (r & 7)) << 4) + (uint32_t)(c4 & 1) * 8u;
         RingPos f;
@@ -466,7 +506,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
 #pragma unroll
             for (int d = 0; d < DEPTH; ++d)
 #pragma unroll
-                for (int c = 0; c < C; ++c) v[d][c] = direct_load(p.g, d < nb ? row : nullptr, (kb + d) * TBK + (c4 + c) * 4, p.avec, R16 && p.g.a16);
+                for (int c = 0; c < C; ++c) v[d][c] = direct_load<ODD>(p.g, d < nb ? row : nullptr, (kb + d) * TBK + (c4 + c) * 4, p.avec);
             // hand over in groups that the ring can hold: a group's stages are free before any of them is written
 #pragma unroll
             for (int d0 = 0; d0 < DEPTH; d0 += GROUP) {
@@ -498,7 +538,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
             tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)first, v);
             if (p.splits == 1 && first < rows) {
                 GemmArgs a = p.g;
-                if (!R16) a.c16 = 0;
+                if (!ODD) a.c16 = 0;
                 a.N = min(a.N, n0 + p.th);
                 if (!p.rpb) {
                     move_c(a, z * a.c_z);
@@ -531,7 +571,7 @@ gemm_few_tc_kernel(const __grid_constant__ CUtensorMap wmap, const __grid_consta
         if (rows > 0 && drains) {
             const int parts = (p.nkb + p.kper - 1) / p.kper;          // blocks that had any k
             GemmArgs a = p.g;
-            if (!R16) a.c16 = 0;
+            if (!ODD) a.c16 = 0;
             a.N = min(a.N, n0 + p.th);
             if (!p.rpb) {
                 move_c(a, z * a.c_z);
@@ -643,6 +683,27 @@ bool weight_map(CUtensorMap* m, const GemmArgs& a, uint64_t matrices, bool many,
 
 }  // namespace
 
+int pad_weights(const GemmArgs& a, int matrices, cudaStream_t st, GemmArgs* b, bool* done) {
+    *done = false;
+    const int kpr = (a.K + 7) / 8;
+    const long long total = (long long)matrices * a.N * kpr;
+    void* buf = nullptr;
+    if (total > (1LL << 38) || scratch_alloc(&buf, (size_t)total * 16, st)) {
+        set_error("");
+        return 0;
+    }
+    *b = a;
+    b->W = buf; b->K = kpr * 8; b->ka = a.K; b->w_stride = (long long)a.N * kpr * 8;
+    const cudaError_t e = launch_waiting(pad_weights_kernel, dim3((unsigned)((total + 255) / 256)), dim3(256), 0, st, (const uint16_t*)a.W, (uint16_t*)buf, a.K, a.N, kpr,
+                                         a.w_stride, total);
+    if (e != cudaSuccess) {
+        scratch_free(buf, st);
+        return cuda_fail(e, "pad_weights", __FILE__, __LINE__);
+    }
+    *done = true;
+    return 0;
+}
+
 int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, cudaStream_t st, bool* served) {
     *served = false;
     const bool own = a.row_group != nullptr, many = own || batch > 1;
@@ -653,6 +714,7 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
     if (zs > 65535) return 0;
     FewArgs p{};
     p.g = a;
+    if (!a.ka) p.g.ka = a.K;
     p.epi = epilogue;
     p.nkb = (a.K + TBK - 1) / TBK;
     const FewPlan plan = few_plan(a.N, zs, p.nkb);
@@ -676,7 +738,7 @@ int gemm_few_tc(const GemmArgs& a, int epilogue, int batch, int rows_per_block, 
         configured = true;
     }
     void* args[] = {&wmap, &p};
-    const cudaError_t e = launch_clustered(kernels[R / 16 - 1][a.a16 || a.c16], dim3(p.splits, (a.N + p.th - 1) / p.th, zs), few_smem(R), p.splits, st, args);
+    const cudaError_t e = launch_clustered(kernels[R / 16 - 1][a.a16 || a.c16 || p.g.ka != a.K], dim3(p.splits, (a.N + p.th - 1) / p.th, zs), few_smem(R), p.splits, st, args);
     if (e != cudaSuccess) return cuda_fail(e, "gemm_few_tc", __FILE__, __LINE__);
     *served = true;
     return 0;
@@ -690,9 +752,10 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
     if (rows <= 0) return 0;
     const bool grouped = a.group_off != nullptr;
     if (!grouped && few_rows_pay(a.M, a.N, a.K, batch)) return gemm_few_tc(a, epilogue, batch, a.M, st, served);
-    const bool direct = a.a16 && a.lda % 8 == 0 && a.a_z % 8 == 0 && (uintptr_t)a.A % 16 == 0 && !a.a_rows;
+    const bool direct = a.a16 && (!a.ka || a.ka == a.K) && a.lda % 8 == 0 && a.a_z % 8 == 0 && (uintptr_t)a.A % 16 == 0 && !a.a_rows;
     TcArgs p{};
     p.g = a;
+    if (!a.ka) p.g.ka = a.K;
     p.epi = epilogue;
     p.batch = batch;
     p.err = wait_word(kWaitRows);
@@ -746,7 +809,7 @@ int gemm_rows_tc(const GemmArgs& a, int epilogue, int batch, int rows, int max_r
         const bool vec = a.lda % 4 == 0 && a.a_z % 4 == 0 && (uintptr_t)a.A % (a.a16 ? 8 : 16) == 0;
         int gy = (chunks + 255) / 256;
         if (gy > 8) gy = 8;
-        e = launch_waiting(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, a, (uint16_t*)abuf, batch, kpr, vec);
+        e = launch_waiting(rows_to_bf16_kernel, dim3(rows, gy), dim3(chunks >= 256 ? 256 : (chunks + 31) / 32 * 32), 0, st, p.g, (uint16_t*)abuf, batch, kpr, vec);
     }
     if (e == cudaSuccess) {
         const int sms = sm_count();

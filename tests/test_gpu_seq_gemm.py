@@ -500,3 +500,34 @@ def test_bfloat16_rows_of_groups(counts, N, K, gather):
     assert np.array_equal(run(1, 0), want)
     assert np.array_equal(run(0, 1), bf16(want).view(np.uint32) >> 16) and np.array_equal(run(1, 1), bf16(want).view(np.uint32) >> 16)
     no_wait_error()
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 2000, 2050), (2, 900, 3001), (4, 1024, 746), (7, 514, 1007), (8, 130, 843), (8, 6000, 1004), (9, 64, 161), (17, 300, 163), (33, 130, 1001),
+                                   (200, 70, 167), (300, 515, 514), (1000, 256, 1002)])
+@pytest.mark.parametrize("off", [0, 1, 2])
+def test_matrices_off_the_boundaries(M, N, K, off):
+    """k of any number, matrices from any element on: brought to boundaries first, for one row up; what lies around the matrix is not read into a sum"""
+    A, W = operands(M + N, M, N, K)
+    ref, tol = product(A, W[0])
+    around = np.full(N * K + 16, np.inf, np.float32)
+    around[off:off + N * K] = W[0].ravel()
+    w, a, c = dev_w(around), gk.from_numpy(np.pad(A, ((0, 0), (0, 1)), constant_values=np.inf)), gk.from_numpy(np.full((M, N), 7.0, np.float32))
+    if M <= 8:
+        api.gemm_few_rows_f32(a.device_ptr, K + 1, None, w.device_ptr + 2 * off, 2, 0, c.device_ptr, N, M, N, K, None, M, 0, 1.0, 0.0, None)
+    else:
+        api.gemm_rows_f32(a.device_ptr, K + 1, None, w.device_ptr + 2 * off, 2, 0, c.device_ptr, N, M, N, K, None, 1, M, 0, 1.0, 0.0, None)
+    assert (np.abs(c.to_numpy() - ref) <= tol + 1e-6).all()
+    no_wait_error()
+
+
+@pytest.mark.parametrize("M", [3, 20, 300])
+def test_batches_off_the_boundaries(M):
+    """products side by side whose matrices start anywhere"""
+    batch, N, K = 3, 66, 1101
+    A, W = operands(M, M, N, K * 1, batch)
+    a, w, c = gk.from_numpy(A), dev_w(W), gk.from_numpy(np.zeros((M, batch * N), np.float32))
+    api.gemm_seq_f32(a.device_ptr, K, 0, w.device_ptr, 2, N * K, c.device_ptr, batch * N, N, M, N, K, batch, 0, 1.0, 0.0, None, None, 0, None, 0, 0, M if M <= 8 else 0, None)
+    for b in range(batch):
+        ref, tol = product(A, W[b])
+        assert (np.abs(c.to_numpy()[:, b * N:(b + 1) * N] - ref) <= tol + 1e-6).all()
+    no_wait_error()
