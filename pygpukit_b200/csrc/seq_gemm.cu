@@ -210,8 +210,13 @@ __global__ void __launch_bounds__(128) gemm_rows_bf16_kernel(GemmArgs a) {
 }
 
 // ---------------------------------------------------------------- many rows, float32 weights: FMAs, summed in k order
-template <int EPI>
+// Tiles of 8 TM x 64; a thread has TM rows and two pairs of columns.  What bounds small products is a tile's walk over k, one slab after the other: a slab
+// is fetched into registers while the one before is multiplied, and tiles of 16 rows (TM = 2) put products of few tiles on all SMs (us, one slab of 16 at
+// a time and 64 rows -> here: 983 x 256 x 1650 230 -> 77, 101 x 802 x 212 33 -> 10.5, 1000 x 3000 x 2048 658 -> 437).  Every sum goes over k in
+// order, whatever the tile.
+template <int EPI, int TM>
 __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(GemmArgs a) {
+    constexpr int TR = 8 * TM, FK = 32, LA = TR * FK / 128, LW = BN * FK / 128;
     const int e = blockIdx.z;
     a.a16 = a.c16 = 0;
     a.A += (size_t)e * a.a_z;
@@ -219,52 +224,70 @@ __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(GemmArgs a) {
     if (EPI == 10) a.aux = (const float*)a.aux + (size_t)e * a.c_z;
     const int m_begin = a.group_off ? a.group_off[e] : 0;
     const int m_end = a.group_off ? a.group_off[e + 1] : a.M;
-    const int m0 = m_begin + blockIdx.y * BM;
+    const int m0 = m_begin + blockIdx.y * TR;
     if (m0 >= m_end) return;
     const int n0 = blockIdx.x * BN;
     const float* W = (const float*)a.W + (size_t)e * a.w_stride;
-    constexpr int FK = 16;
-    __shared__ float As[FK][BM + 4];
-    __shared__ float Ws[FK][BN + 4];
-    __shared__ int rows[BM];
-    const int tid = threadIdx.x;
-    if (tid < BM) {
+    __shared__ __align__(8) float As[2][FK][TR + 2];
+    __shared__ __align__(8) float Ws[2][FK][BN + 2];
+    __shared__ int rows[TR];
+    const int tid = threadIdx.x, lk = tid & 31, lr = tid >> 5;            // loads: k of the slab, every fourth row
+    if (tid < TR) {
         const int r = m0 + tid;
         rows[tid] = r < m_end ? (a.a_rows ? a.a_rows[r] : r) : -1;
     }
     __syncthreads();
-    const int ty = tid >> 4, tx = tid & 15;          // 8 rows x 4 columns per thread
-    float acc[8][4] = {};
-    for (int k0 = 0; k0 < a.K; k0 += FK) {
+    float ra[LA], rw[LW];
+    auto fetch = [&](int k0) {
+        const int k = k0 + lk;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int idx = tid + i * 128, r = idx >> 4, c = idx & 15, k = k0 + c;
-            const int gr = rows[r];
-            As[c][r] = (gr >= 0 && k < a.K) ? a.A[(size_t)gr * a.lda + k] : 0.f;
-            const int n = n0 + r;
-            Ws[c][r] = (n < a.N && k < a.K) ? W[(size_t)n * a.K + k] : 0.f;
+        for (int i = 0; i < LA; ++i) {
+            const int gr = rows[lr + 4 * i];
+            ra[i] = gr >= 0 && k < a.K ? a.A[(size_t)gr * a.lda + k] : 0.f;
         }
-        __syncthreads();
 #pragma unroll
+        for (int i = 0; i < LW; ++i) {
+            const int n = n0 + lr + 4 * i;
+            rw[i] = n < a.N && k < a.K ? W[(size_t)n * a.K + k] : 0.f;
+        }
+    };
+    auto stash = [&](int b) {
+#pragma unroll
+        for (int i = 0; i < LA; ++i) As[b][lk][lr + 4 * i] = ra[i];
+#pragma unroll
+        for (int i = 0; i < LW; ++i) Ws[b][lk][lr + 4 * i] = rw[i];
+    };
+    const int ty = tid >> 4, tx = tid & 15;          // rows TM ty ..., columns 2 tx, 2 tx + 1 and 32 further on
+    float acc[TM][4] = {};
+    fetch(0);
+    stash(0);
+    __syncthreads();
+    for (int k0 = 0, b = 0; k0 < a.K; k0 += FK, b ^= 1) {
+        const bool more = k0 + FK < a.K;
+        if (more) fetch(k0 + FK);
+#pragma unroll 8
         for (int k = 0; k < FK; ++k) {
-            float av[8], wv[4];
+            float av[TM];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) av[i] = As[k][ty * 8 + i];
+            for (int i = 0; i < TM; i += 2) *(float2*)&av[i] = *(const float2*)&As[b][k][ty * TM + i];
+            const float2 w0 = *(const float2*)&Ws[b][k][2 * tx], w1 = *(const float2*)&Ws[b][k][32 + 2 * tx];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) wv[j] = Ws[k][tx * 4 + j];
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], wv[j], acc[i][j]);
+            for (int i = 0; i < TM; ++i) {
+                acc[i][0] = fmaf(av[i], w0.x, acc[i][0]);
+                acc[i][1] = fmaf(av[i], w0.y, acc[i][1]);
+                acc[i][2] = fmaf(av[i], w1.x, acc[i][2]);
+                acc[i][3] = fmaf(av[i], w1.y, acc[i][3]);
+            }
         }
+        if (more) stash(b ^ 1);
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int r = m0 + ty * 8 + i;
+    for (int i = 0; i < TM; ++i) {
+        const int r = m0 + ty * TM + i;
         if (r >= m_end) continue;
-        store_pair<EPI>(a, r, n0 + tx * 4, acc[i][0], acc[i][1]);
-        store_pair<EPI>(a, r, n0 + tx * 4 + 2, acc[i][2], acc[i][3]);
+        store_pair<EPI>(a, r, n0 + 2 * tx, acc[i][0], acc[i][1]);
+        store_pair<EPI>(a, r, n0 + 32 + 2 * tx, acc[i][2], acc[i][3]);
     }
 }
 
@@ -453,7 +476,8 @@ int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream
     dim3 grid((a.N + BN - 1) / BN, (max_rows + BM - 1) / BM, groups);
     if (a.a16 || a.c16) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI, true>, grid, dim3(128), 0, st, a));
     else if (wdt == 2) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI, false>, grid, dim3(128), 0, st, a));
-    else PGK_CUDA(launch(gemm_rows_f32_kernel<EPI>, grid, dim3(128), 0, st, a));
+    else if ((long long)grid.x * grid.y * grid.z >= sm_count()) PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 8>, grid, dim3(128), 0, st, a));
+    else PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 2>, dim3(grid.x, (max_rows + 15) / 16, groups), dim3(128), 0, st, a));
     return 0;
 }
 

@@ -531,3 +531,24 @@ def test_batches_off_the_boundaries(M):
         ref, tol = product(A, W[b])
         assert (np.abs(c.to_numpy()[:, b * N:(b + 1) * N] - ref) <= tol + 1e-6).all()
     no_wait_error()
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 66, 31), (16, 128, 32), (17, 130, 33), (64, 70, 100), (101, 802, 212), (1000, 700, 65), (1025, 1000, 40)])
+@pytest.mark.parametrize("epi", [0, 6, 7])
+def test_float32_rows_sum_in_the_order_of_k(M, N, K, epi):
+    """(more than 64 columns: up to there the router's kernel serves plain products) both tile heights: every sum is the chain of fused multiply-adds over k (float64 products rounded once per step), bit for bit without an activation"""
+    A, W = operands(M + N, M, N, K)
+    W = W[0] + np.float32(1e-4)
+    F = N // 2 if epi == 7 else N
+    a, w, c = gk.from_numpy(A), gk.from_numpy(W), gk.from_numpy(np.zeros((M, F), np.float32))
+    api.gemm_rows_f32(a.device_ptr, K, None, w.device_ptr, 0, 0, c.device_ptr, F, M, N, K, None, 1, M, epi, 1.0, 0.0, None)
+    z = np.zeros((M, N), np.float32)
+    for k in range(K):                                   # a float64 product of float32 is exact, its sum with z rounds twice at worst: half a unit in 2^-29 of all cases
+        z = (A[:, k:k + 1].astype(np.float64) * W[:, k].astype(np.float64) + z).astype(np.float32)
+    got = c.to_numpy()
+    if epi == 0:
+        assert (got != z).mean() < 1e-4 and np.allclose(got, z, rtol=1e-6, atol=1e-6)
+    else:
+        z = z.astype(np.float64)
+        ref = np.maximum(z, 0) ** 2 if epi == 6 else gelu_tanh(z[:, 0::2]) * z[:, 1::2]
+        assert np.allclose(got, ref, rtol=2e-5, atol=2e-6)
