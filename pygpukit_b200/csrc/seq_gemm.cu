@@ -210,13 +210,14 @@ __global__ void __launch_bounds__(128) gemm_rows_bf16_kernel(GemmArgs a) {
 }
 
 // ---------------------------------------------------------------- many rows, float32 weights: FMAs, summed in k order
-// Tiles of 8 TM x 64; a thread has TM rows and two pairs of columns.  What bounds small products is a tile's walk over k, one slab after the other: a slab
-// is fetched into registers while the one before is multiplied, and tiles of 16 rows (TM = 2) put products of few tiles on all SMs (us, one slab of 16 at
-// a time and 64 rows -> here: 983 x 256 x 1650 230 -> 77, 101 x 802 x 212 33 -> 10.5, 1000 x 3000 x 2048 658 -> 437).  Every sum goes over k in
-// order, whatever the tile.
+// Tiles of 8 TM x 64; a thread has TM rows and four columns and reads four k of each at once.  What bounds small products is a tile's walk over k, one
+// slab after the other: slabs are on their way in registers while one is multiplied -- two with the lower tiles, whose slabs take less than
+// a load's way; with TM = 8 one, the registers of a second cost more --, and lower tiles put products of few tiles on all SMs (us, one slab of 16 at
+// a time and 64 rows -> here: 983 x 256 x 1650 230 -> 56, 101 x 802 x 212 33 -> 10.4, 700 x 700 x 700 99 -> 35, 1000 x 3000 x 2048 658 -> 372; copies by
+// cp.async, which an SM takes 16 bytes a cycle of, 60, 8.5, 38 and 418).  Every sum goes over k in order, whatever the tile.
 template <int EPI, int TM>
 __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(GemmArgs a) {
-    constexpr int TR = 8 * TM, FK = 32, LA = TR * FK / 128, LW = BN * FK / 128;
+    constexpr int TR = 8 * TM, FK = 32, AHEAD = TM == 8 ? 1 : 2, LD = FK + 4, L4 = FK / 4, LR = 128 / L4, LA = TR / LR, LW = BN / LR;
     const int e = blockIdx.z;
     a.a16 = a.c16 = 0;
     a.A += (size_t)e * a.a_z;
@@ -228,66 +229,92 @@ __global__ void __launch_bounds__(128) gemm_rows_f32_kernel(GemmArgs a) {
     if (m0 >= m_end) return;
     const int n0 = blockIdx.x * BN;
     const float* W = (const float*)a.W + (size_t)e * a.w_stride;
-    __shared__ __align__(8) float As[2][FK][TR + 2];
-    __shared__ __align__(8) float Ws[2][FK][BN + 2];
-    __shared__ int rows[TR];
-    const int tid = threadIdx.x, lk = tid & 31, lr = tid >> 5;            // loads: k of the slab, every fourth row
-    if (tid < TR) {
-        const int r = m0 + tid;
-        rows[tid] = r < m_end ? (a.a_rows ? a.a_rows[r] : r) : -1;
+    __shared__ __align__(16) float As[2][TR][LD];
+    __shared__ __align__(16) float Ws[2][BN][LD];
+    const int tid = threadIdx.x, lk = tid % L4 * 4, lr = tid / L4;        // loads: four k of the slab, every LR-th row
+    const bool avec = a.lda % 4 == 0 && ((uintptr_t)a.A & 15) == 0, wvec = a.K % 4 == 0 && ((uintptr_t)W & 15) == 0;
+    const float *pa[LA], *pw[LW];                                         // rows beyond the edge: none
+#pragma unroll
+    for (int i = 0; i < LA; ++i) {
+        const int r = m0 + lr + LR * i;
+        pa[i] = r < m_end ? a.A + (size_t)(a.a_rows ? a.a_rows[r] : r) * a.lda + lk : nullptr;
     }
-    __syncthreads();
-    float ra[LA], rw[LW];
-    auto fetch = [&](int k0) {
-        const int k = k0 + lk;
 #pragma unroll
-        for (int i = 0; i < LA; ++i) {
-            const int gr = rows[lr + 4 * i];
-            ra[i] = gr >= 0 && k < a.K ? a.A[(size_t)gr * a.lda + k] : 0.f;
-        }
-#pragma unroll
-        for (int i = 0; i < LW; ++i) {
-            const int n = n0 + lr + 4 * i;
-            rw[i] = n < a.N && k < a.K ? W[(size_t)n * a.K + k] : 0.f;
-        }
+    for (int i = 0; i < LW; ++i) pw[i] = n0 + lr + LR * i < a.N ? W + (size_t)(n0 + lr + LR * i) * a.K + lk : nullptr;
+    float4 ra[AHEAD][LA], rw[AHEAD][LW];
+    auto four = [&](const float* p, int k, bool vec) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (!p) return v;
+        if (vec && k + lk + 4 <= a.K) return *(const float4*)(p + k);
+        if (k + lk < a.K) v.x = p[k];
+        if (k + lk + 1 < a.K) v.y = p[k + 1];
+        if (k + lk + 2 < a.K) v.z = p[k + 2];
+        if (k + lk + 3 < a.K) v.w = p[k + 3];
+        return v;
     };
-    auto stash = [&](int b) {
+    auto fetch = [&](float4 (&ra)[LA], float4 (&rw)[LW], int k0) {
 #pragma unroll
-        for (int i = 0; i < LA; ++i) As[b][lk][lr + 4 * i] = ra[i];
+        for (int i = 0; i < LA; ++i) ra[i] = four(pa[i], k0, avec);
 #pragma unroll
-        for (int i = 0; i < LW; ++i) Ws[b][lk][lr + 4 * i] = rw[i];
+        for (int i = 0; i < LW; ++i) rw[i] = four(pw[i], k0, wvec);
     };
-    const int ty = tid >> 4, tx = tid & 15;          // rows TM ty ..., columns 2 tx, 2 tx + 1 and 32 further on
+    auto stash = [&](const float4 (&ra)[LA], const float4 (&rw)[LW], int b) {
+#pragma unroll
+        for (int i = 0; i < LA; ++i) *(float4*)&As[b][lr + LR * i][lk] = ra[i];
+#pragma unroll
+        for (int i = 0; i < LW; ++i) *(float4*)&Ws[b][lr + LR * i][lk] = rw[i];
+    };
+    const int ty = tid >> 4, tx = tid & 15;          // rows ty + 8 i, columns tx + 16 j: no two lanes of a quarter warp share a bank
     float acc[TM][4] = {};
-    fetch(0);
-    stash(0);
-    __syncthreads();
-    for (int k0 = 0, b = 0; k0 < a.K; k0 += FK, b ^= 1) {
-        const bool more = k0 + FK < a.K;
-        if (more) fetch(k0 + FK);
-#pragma unroll 8
-        for (int k = 0; k < FK; ++k) {
-            float av[TM];
+    auto multiply = [&](int b) {
+#pragma unroll 2
+        for (int k = 0; k < FK; k += 4) {
+            float4 av[TM], wv[4];
 #pragma unroll
-            for (int i = 0; i < TM; i += 2) *(float2*)&av[i] = *(const float2*)&As[b][k][ty * TM + i];
-            const float2 w0 = *(const float2*)&Ws[b][k][2 * tx], w1 = *(const float2*)&Ws[b][k][32 + 2 * tx];
+            for (int i = 0; i < TM; ++i) av[i] = *(const float4*)&As[b][ty + 8 * i][k];
 #pragma unroll
-            for (int i = 0; i < TM; ++i) {
-                acc[i][0] = fmaf(av[i], w0.x, acc[i][0]);
-                acc[i][1] = fmaf(av[i], w0.y, acc[i][1]);
-                acc[i][2] = fmaf(av[i], w1.x, acc[i][2]);
-                acc[i][3] = fmaf(av[i], w1.y, acc[i][3]);
-            }
+            for (int j = 0; j < 4; ++j) wv[j] = *(const float4*)&Ws[b][tx + 16 * j][k];
+#pragma unroll
+            for (int i = 0; i < TM; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    acc[i][j] = fmaf(av[i].x, wv[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].y, wv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].z, wv[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(av[i].w, wv[j].w, acc[i][j]);
+                }
         }
-        if (more) stash(b ^ 1);
-        __syncthreads();
+    };
+    fetch(ra[0], rw[0], 0);
+    if (AHEAD == 2 && FK < a.K) fetch(ra[AHEAD - 1], rw[AHEAD - 1], FK);
+    stash(ra[0], rw[0], 0);
+    __syncthreads();
+    for (int k0 = 0; k0 < a.K; k0 += 2 * FK) {       // slabs k0 and k0 + FK
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int k = k0 + q * FK, from = AHEAD == 2 ? q ^ 1 : 0;
+            if (k >= a.K) break;
+            if (k + AHEAD * FK < a.K) fetch(ra[AHEAD == 2 ? q : 0], rw[AHEAD == 2 ? q : 0], k + AHEAD * FK);
+            multiply(q);
+            if (k + FK < a.K) stash(ra[from], rw[from], q ^ 1);
+            __syncthreads();
+        }
     }
+    // neighbouring columns, as the epilogue wants them, meet in shared memory
+    float* const out = &Ws[0][0][0];                 // [TR][BN + 2]
+    static_assert(TR * (BN + 2) <= 2 * BN * LD);
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) out[(ty + 8 * i) * (BN + 2) + tx + 16 * j] = acc[i][j];
+    __syncthreads();
 #pragma unroll
     for (int i = 0; i < TM; ++i) {
-        const int r = m0 + ty * TM + i;
+        const int r = m0 + ty + 8 * i;
         if (r >= m_end) continue;
-        store_pair<EPI>(a, r, n0 + 2 * tx, acc[i][0], acc[i][1]);
-        store_pair<EPI>(a, r, n0 + 32 + 2 * tx, acc[i][2], acc[i][3]);
+        const float* v = out + (ty + 8 * i) * (BN + 2) + 2 * tx;
+        store_pair<EPI>(a, r, n0 + 2 * tx, v[0], v[1]);
+        store_pair<EPI>(a, r, n0 + 32 + 2 * tx, v[32], v[33]);
     }
 }
 
@@ -476,8 +503,16 @@ int launch_many(const GemmArgs& a, int wdt, int groups, int max_rows, cudaStream
     dim3 grid((a.N + BN - 1) / BN, (max_rows + BM - 1) / BM, groups);
     if (a.a16 || a.c16) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI, true>, grid, dim3(128), 0, st, a));
     else if (wdt == 2) PGK_CUDA(launch(gemm_rows_bf16_kernel<EPI, false>, grid, dim3(128), 0, st, a));
-    else if ((long long)grid.x * grid.y * grid.z >= sm_count()) PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 8>, grid, dim3(128), 0, st, a));
-    else PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 2>, dim3(grid.x, (max_rows + 15) / 16, groups), dim3(128), 0, st, a));
+    else {
+        // the highest tiles when lower ones would not fit the SMs at one time (1000 x 3000 x 2048 493 -> 372, 700 x 1500 x 800 101 -> 58; 151 x 1830 x 2003, 145
+        // tiles of 32 rows, 66 against 95 and 84 with 64 and 16), the lowest when not half of them have one (64 x 512 x 400 16.6 -> 14.5)
+        const long long low = (long long)grid.x * ((max_rows + 31) / 32) * groups;
+        const int tm = low > sm_count() ? 8 : (2 * low >= sm_count() ? 4 : 2);
+        grid.y = (max_rows + 8 * tm - 1) / (8 * tm);
+        if (tm == 8) PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 8>, grid, dim3(128), 0, st, a));
+        else if (tm == 4) PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 4>, grid, dim3(128), 0, st, a));
+        else PGK_CUDA(launch(gemm_rows_f32_kernel<EPI, 2>, grid, dim3(128), 0, st, a));
+    }
     return 0;
 }
 
