@@ -137,10 +137,14 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     const uint32_t tmem = *tmem_slot;
     griddep_wait();
     griddep_launch();
-    const int4 tile = a.tiles[blockIdx.x];
+    // blocks start in the order of their numbers: a request's last queries, which see the most keys, first, so that none of the long ones starts when the
+    // others end (16 heads over latent rows, 2000 tokens, 1000 blocks of 1 to 16 tiles 465 -> 440 us;
+    // 32 / 4 heads of 128 in chunks of 1024, 2000 blocks 192 -> 173)
+    const int nth = (int)(blockIdx.y * gridDim.x + blockIdx.x), block = nth / (int)gridDim.y, part = nth - block * (int)gridDim.y;
+    const int4 tile = a.tiles[(int)gridDim.x - 1 - block];
     const int t0 = tile.x, nq = tile.y, slot = tile.z, pos0 = tile.w, D = a.D, Dv = a.Dv, HB = a.HB;
     const int rep = a.H / a.G, hsplit = (rep + HB - 1) / HB;
-    const int g = blockIdx.y / hsplit, hpart = blockIdx.y - g * hsplit;
+    const int g = part / hsplit, hpart = part - g * hsplit;
     const int hb0 = g * rep + hpart * HB, nh = min(HB, rep - hpart * HB);
     const int live = min(AR, nq * HB);                   // rows that a query has
 
