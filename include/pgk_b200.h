@@ -711,7 +711,8 @@ int pgk_seq_mixer_prep_rot_ex2(float* proj, int ld, int tokens, int heads, int k
                                void* stream);
 /* pgk_seq_attention_ex2 with pooled blocks (pool > 0, needs a window: beside its window a query at i sees the pooled key and
  * value of every block that ends at or before i - window, in the same softmax) and outputs turned back by the query's position
- * (out_inv_freq [vdim / 2], out_pairs as in the preparation) in front of the gate. */
+ * (out_inv_freq [vdim / 2], out_pairs as in the preparation) in front of the gate. cache_dtype 18: a
+ * bfloat16 cache and bfloat16 outputs, for rows that a product reads (prompt tiles, sizes that pgk_seq_attention_tensor serves). */
 int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_rows, int ldg, int gate_off, int gate_mode,
                           float* out, int ldo, const void* k_cache, const void* v_cache, int k_ld, int v_ld, int cache_dtype,
                           const int32_t* table, int max_pages, int page_size, const int32_t* tiles, int n_tiles,

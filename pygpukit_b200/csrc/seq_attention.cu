@@ -1155,6 +1155,9 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
                 "seq_attention failed: kept first positions need a window and no chunks");
     PGK_REQUIRE(!slopes2 || slopes, "seq_attention failed: the logarithmic distance term needs both per-head vectors");
     PGK_REQUIRE(weight_mode == 0 || (weight_mode == 1 && !sinks), "seq_attention failed: weight mode %d", weight_mode);
+    const int out16 = cache_dtype == 18;
+    if (out16) cache_dtype = 2;
+    PGK_REQUIRE(!out16 || (single_query == 0 && pool == 0 && !out_inv_freq), "seq_attention failed: bfloat16 outputs come from prompt tiles and plain heads");
     PGK_REQUIRE(cache_dtype == 0 || cache_dtype == 2, "seq_attention failed: the cache is float32 (0) or bfloat16 (2), got %d", cache_dtype);
     PGK_REQUIRE(heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && dim > 0 && vdim > 0, "seq_attention failed: invalid head layout");
     PGK_REQUIRE(splits >= 1 && splits <= 64 && (splits == 1 || single_query == 3 || (workspace && tickets)),
@@ -1173,7 +1176,7 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
     a.H = heads; a.G = kv_heads; a.D = dim; a.Dv = vdim; a.chunk = chunk;
     a.HB = pgk_seq_heads_per_block(heads, kv_heads); a.gate = gate_mode;
     a.scale = scale; a.cap = softcap; a.splits = splits; a.ws = workspace; a.tickets = tickets;
-    a.pool = pool; a.pool_rows = pool_rows; a.pk = k_pool; a.pv = v_pool; a.o_inv_freq = out_inv_freq; a.o_pairs = out_pairs;
+    a.pool = pool; a.pool_rows = pool_rows; a.pk = k_pool; a.pv = v_pool; a.o_inv_freq = out_inv_freq; a.o_pairs = out_pairs; a.out16 = out16;
     PGK_REQUIRE(!a.valias || pool == 0, "seq_attention failed: pooled blocks keep their values in an array of their own");
     if (single_query == 3) {                 // the kernel of few queries, `splits` blocks share a request's keys
         bool served = false;
@@ -1190,6 +1193,7 @@ int pgk_seq_attention_ex3(const float* q, int ldq, int q_off, const float* gate_
         if (const int rc = seq_attention_tc(a, n_tiles, (cudaStream_t)stream, &served)) return rc;
         if (served) return 0;
     }
+    PGK_REQUIRE(!out16, "seq_attention failed: bfloat16 outputs need heads and a cache that the tensor cores serve (pgk_seq_attention_tensor)");
     if (single_query)
         return cache_dtype == 2 ? launch_attn_decode_nv<uint16_t>(a, n_tiles, (cudaStream_t)stream)
                                 : launch_attn_decode_nv<float>(a, n_tiles, (cudaStream_t)stream);

@@ -28,6 +28,7 @@ struct AttnArgs {
     const void* pk; const void* pv;     // [pages][G][pool_rows][D] / [Dv], dense rows
     const double* o_inv_freq;           // [Dv / 2] or NULL: pair m of an output (elements m and m + Dv / 2, or 2m and 2m + 1
     int o_pairs;                        // with o_pairs) turns by -position * o_inv_freq[m]
+    int out16;                          // bfloat16 outputs (tensor cores): rows that only a product reads, which rounds them so
 };
 
 __device__ __forceinline__ float gate_logit(const AttnArgs& a, size_t t, int h, int dv) {

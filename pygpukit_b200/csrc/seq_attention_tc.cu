@@ -601,7 +601,9 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
                     if (a.splits > 1) a.ws[((t * a.H + h) * a.splits + blockIdx.z) * (Dv + 2) + 2 + dv] = v;
                     else {
                         if (gated) v *= 1.f / (1.f + expf(-gz[e]));
-                        a.out[t * a.ldo + (size_t)h * Dv + dv] = v;
+                        const size_t to = t * a.ldo + (size_t)h * Dv + dv;
+                        if (a.out16) ((uint16_t*)a.out)[to] = f32_to_bf16_bits(v);
+                        else a.out[to] = v;
                     }
                 }
             }
@@ -676,13 +678,20 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
             if (row[q] < 0) continue;
             const int ro = rowo[row[q]], dv = 2 * (i0 + q * A_THREADS - row[q] * half_dv), h = hb0 + (ro & 0xffff);
             const size_t t = t0 + (ro >> 16);
-            float* dst = a.out + t * a.ldo + (size_t)h * Dv + dv;
+            const size_t to = t * a.ldo + (size_t)h * Dv + dv;
             if (a.gate) {
                 o[q].x *= 1.f / (1.f + expf(-gate_logit(a, t, h, dv)));
                 o[q].y *= 1.f / (1.f + expf(-gate_logit(a, t, h, dv + 1)));
             }
-            dst[0] = o[q].x * a.out_mult;
-            dst[1] = o[q].y * a.out_mult;
+            o[q].x *= a.out_mult;
+            o[q].y *= a.out_mult;
+            if (a.out16) {
+                ((uint16_t*)a.out)[to] = f32_to_bf16_bits(o[q].x);
+                ((uint16_t*)a.out)[to + 1] = f32_to_bf16_bits(o[q].y);
+            } else {
+                a.out[to] = o[q].x;
+                a.out[to + 1] = o[q].y;
+            }
         }
     }
 }

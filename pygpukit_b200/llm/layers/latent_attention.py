@@ -28,7 +28,7 @@ from ...core.factory import from_numpy
 from ...core.stream import current_stream_handle as _st
 from ..config import LatentMixerSpec
 from .linear import LinearRows
-from .paged_attention import few_decode, key_slices, launch_form
+from .paged_attention import few_decode, key_slices, launch_form, rounded_outputs
 
 
 class LatentAttentionMixer:
@@ -102,17 +102,18 @@ class LatentAttentionMixer:
         if splits > 1 and single != 3:
             ws = ctx.workspace(T * H * splits * (R + 2)).device_ptr
             tickets = b.tickets.device_ptr
+        r16 = rounded_outputs(ctx, single, self.v_up, (row, R, row, row), H, 1)
         head_gate = s.out_gate and s.gate_per_head                     # a gate per element waits for the values
         g_off = s.q_cols + s.kv_cols
         api.seq_attention_ex(qa.device_ptr, H * row, 0, proj.device_ptr, ld, g_off, 2 if head_gate else 0,
-                             lat.device_ptr, H * R, kc.device_ptr, kc.device_ptr, row, row, cache.dtype_code,
+                             lat.device_ptr, H * R, kc.device_ptr, kc.device_ptr, row, row, cache.dtype_code + 16 * r16,
                              cache.table_dev.device_ptr, cache.pool.max_pages, cache.page_size, tiles_ptr, n_tiles, None,
                              self.sinks.device_ptr if self.sinks is not None else None, H, 1, row, R, 0, s.window, s.scale, 0.0,
                              splits, ws, tickets, single, _st())
         gated = s.out_gate and not s.gate_per_head
         h16 = self.v_up.hands_over(T, self.o_proj)
         self.v_up.forward_seq(lat.device_ptr, H * R, T, vo.device_ptr, H * s.vdim, epilogue=10 if gated else 0, batch=H, a_batch=R,
-                              c_batch=s.vdim, aux=(proj.device_ptr, 0, None, ld, g_off) if gated else None, out16=h16)
+                              c_batch=s.vdim, aux=(proj.device_ptr, 0, None, ld, g_off) if gated else None, x16=r16, out16=h16)
         if out_scale is None:
             self.o_proj.forward_seq(vo.device_ptr, H * s.vdim, T, out.device_ptr, self.o_proj.out_features, epilogue=0, x16=h16)
         else:

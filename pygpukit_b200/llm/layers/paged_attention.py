@@ -107,6 +107,15 @@ def _tensor_decode(ctx, n_tiles: int, heads: int, kv_heads: int, rows: int, keys
     return vdim <= 128 or n_tiles * heads * keys * (dim + vdim) >= (1 << 27 if rows > 16 else 1 << 26)
 
 
+def rounded_outputs(ctx, single: int, after, dims, heads: int, kv_heads: int) -> int:
+    """1 when the attention of a step's prompt rows may leave its outputs in bfloat16, as the product `after`, their only reader, rounds them: the
+    tensor cores serve it (dims: key, value sizes and their rows in the cache), more rows than a product of few takes."""
+    c = ctx.cache
+    if ctx.T <= after.FEW or ctx.decode_only or single or after.wdt != 2 or c.dtype_code != 2:
+        return 0
+    return api.seq_attention_tensor(dims[0], dims[1], dims[2], dims[3], heads, kv_heads, 2, c.pool.max_pages * c.page_size)
+
+
 class PagedAttentionMixer:
     def __init__(self, spec: AttentionMixerSpec, layer: int, qkvg: "LinearRows | None", o_proj: "LinearRows | None",
                  q_norm: "GPUArray | None", k_norm: "GPUArray | None", eps: float, v_role: int = 0, v_lambda: float = 0.0,
@@ -203,16 +212,17 @@ class PagedAttentionMixer:
         ld = self.proj_cols
         self.qkvg.forward(x.device_ptr, W, T, proj.device_ptr, ld)
         ldo = s.heads * s.vdim
-        self.attend(ctx, proj.device_ptr, ld, attn.device_ptr, ldo, cache_index)
+        r16 = self.attend(ctx, proj.device_ptr, ld, attn.device_ptr, ldo, cache_index, after=self.o_proj)
         if out_scale is None:
-            self.o_proj.forward(attn.device_ptr, ldo, T, out.device_ptr, self.o_proj.out_features)
+            self.o_proj.forward(attn.device_ptr, ldo, T, out.device_ptr, self.o_proj.out_features, x16=r16)
         else:
             self.o_proj.forward_seq(attn.device_ptr, ldo, T, out.device_ptr, self.o_proj.out_features, epilogue=4,
-                                    col_scale=out_scale)
+                                    col_scale=out_scale, x16=r16)
 
-    def attend(self, ctx, proj_ptr: int, ld: int, attn_ptr: int, ldo: int, cache_index: int | None = None) -> None:
+    def attend(self, ctx, proj_ptr: int, ld: int, attn_ptr: int, ldo: int, cache_index: int | None = None, after=None) -> int:
         """Everything between the two matrix products: proj_ptr points at this mixer's [q | k | v | gate] columns inside
-        rows of stride ld; the heads' outputs go to attn_ptr (row stride ldo)."""
+        rows of stride ld; the heads' outputs go to attn_ptr (row stride ldo).  after: the product that alone reads them; returns 1 when they
+        are bfloat16 for it."""
         s, T = self.spec, ctx.T
         cache = ctx.cache
         ci = self.layer if cache_index is None else cache_index
@@ -249,9 +259,12 @@ class PagedAttentionMixer:
         if splits > 1 and single != 3:
             ws = ctx.workspace(T * s.heads * splits * (s.vdim + 2)).device_ptr
             tickets = ctx.buf.tickets.device_ptr
+        r16 = 0
+        if after is not None and not s.pool and not s.rot_values:
+            r16 = rounded_outputs(ctx, single, after, (s.dim, s.vdim, s.dim, s.vdim), s.heads, s.kv_heads)
         gate_mode = 0 if not s.out_gate else (2 if s.gate_per_head else 1)
         api.seq_attention_ex3(proj_ptr, ld, 0, proj_ptr, ld, self.q_cols + self.k_cols + self.v_cols, gate_mode,
-                              attn_ptr, ldo, kc.device_ptr, vc.device_ptr, s.dim, s.vdim, cache.dtype_code,
+                              attn_ptr, ldo, kc.device_ptr, vc.device_ptr, s.dim, s.vdim, cache.dtype_code + 16 * r16,
                               cache.table_dev.device_ptr, cache.pool.max_pages, cache.page_size, tiles_ptr, n_tiles,
                               self.slopes.device_ptr if self.slopes is not None else None,
                               self.slopes2.device_ptr if self.slopes2 is not None else None,
@@ -261,6 +274,7 @@ class PagedAttentionMixer:
                               cache.pool_rows(ci), cache.pk[ci].device_ptr if s.pool else None,
                               cache.pv[ci].device_ptr if s.pool else None, self.v_inv_freq.device_ptr if s.rot_values else None,
                               self.pairs, splits, ws, tickets, single, _st())
+        return r16
 
 
-__all__ = ["PagedAttentionMixer", "key_slices", "few_decode", "launch_form"]
+__all__ = ["PagedAttentionMixer", "key_slices", "few_decode", "launch_form", "rounded_outputs"]

@@ -598,3 +598,21 @@ def test_decode_steps_of_many_requests_replay_as_they_run(requests):
         outs.append([m.step([(r, [t], [0]) for r, t in enumerate(tokens(cfg, requests, seed=100 + i))]) for i in range(5)])
         assert bool(m._graphs) == (graphs and requests <= 32)
     assert all(np.array_equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("portion", [9, 40, 300])
+def test_outputs_left_in_bfloat16_have_the_bits_of_the_rounding_product(portion, monkeypatch):
+    """attention outputs and gate/up rows that only the next product reads: rounded where they are formed or where they are read, the same logits"""
+    from pygpukit_b200.llm.layers import linear, paged_attention
+    outs, used = [], []
+    seen = paged_attention.rounded_outputs
+    for apart in (False, True):
+        cfg, _, m = make("mixed_stack", dtype="bfloat16")
+        if apart:
+            monkeypatch.setattr(paged_attention, "rounded_outputs", lambda *a: 0)
+            monkeypatch.setattr(linear.LinearRows, "hands_over", lambda *a: 0)
+        else:
+            monkeypatch.setattr(paged_attention, "rounded_outputs", lambda *a: used.append(seen(*a)) or used[-1])
+        m.init_cache(max_tokens=2048, slots=2)
+        outs.append(m.step([(0, tokens(cfg, portion, seed=1), [portion - 1]), (1, tokens(cfg, 5, seed=2), [4])]))
+    assert any(used) and np.array_equal(outs[0], outs[1])
