@@ -22,8 +22,8 @@
 //   * the copies start beside the queries' conversion, an edge tile's zeros are written while the next pair of chunks arrives, the
 //     outputs leave four rows at a time in a short loop (code that runs once per block costs its fetch), and rows that no query
 //     has are left out: what decoding, one tile per block, spends its time on.
-// Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 191 us; 16 heads over latent rows
-// of 576 / 512 5097 -> 471 us.  Decoding, 8 requests: latent rows over 2000 keys 129 -> 50 us, 16 / 4 heads of 128 over 1024 65 -> 24
+// Measured on B200, 2000 tokens: 32 / 4 heads of 128 in chunks of 1024 with cap and slopes 1336 -> 186 us; 16 heads over latent rows
+// of 576 / 512 5097 -> 445 us.  Decoding, 8 requests: latent rows over 2000 keys 129 -> 50 us, 16 / 4 heads of 128 over 1024 65 -> 24
 // us.  (Weights reach 2^LAZY before their reference moves: sums of values above 2^120 may overflow.)  Against float64 the errors are the float32 kernel's or smaller (rms 4.7e-8 -> 3.3e-8 at heads of
 // 128).
 #include "seq_attention.cuh"
@@ -138,8 +138,8 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     griddep_wait();
     griddep_launch();
     // blocks start in the order of their numbers: a request's last queries, which see the most keys, first, so that none of the long ones starts when the
-    // others end (16 heads over latent rows, 2000 tokens, 1000 blocks of 1 to 16 tiles 465 -> 440 us;
-    // 32 / 4 heads of 128 in chunks of 1024, 2000 blocks 192 -> 173)
+    // others end (16 heads over latent rows, 2000 tokens, 1000 blocks of 1 to 16 tiles 466 -> 445 us;
+    // 32 / 4 heads of 128 in chunks of 1024, 2000 blocks 195 -> 186)
     const int nth = (int)(blockIdx.y * gridDim.x + blockIdx.x), block = nth / (int)gridDim.y, part = nth - block * (int)gridDim.y;
     const int4 tile = a.tiles[(int)gridDim.x - 1 - block];
     const int t0 = tile.x, nq = tile.y, slot = tile.z, pos0 = tile.w, D = a.D, Dv = a.Dv, HB = a.HB;
