@@ -570,11 +570,12 @@ int launch_few(const GemmArgs& a, int wdt, int rows_per_block, cudaStream_t st, 
 // A 64 x 64 tile would leave all but one tile column empty and the grid a handful of blocks.  Here a warp owns SKM rows and SKN
 // columns and walks K with a lane per element; the partial sums meet in a warp reduction.  Plain epilogue only.  Latency bounds it: a
 // warp per column group instead of one for all columns, addresses that need no test (us, one warp per row group -> here: 2000 rows of
-// 2048, 4 / 16 / 64 columns 14.5 / 25.2 / 84 -> 12.8 / 14.5 / 28.8; two rows per warp 16.4 / 22.7 / 45.2).  The sums' order is that of one warp per row.
+// 2048, 4 / 16 / 64 columns 14.5 / 25.2 / 84 -> 12.8 / 14.5 / 28.8; two rows per warp 16.4 / 22.7 / 45.2).  Where rows keep 16-byte
+// boundaries a lane takes four k at once (18 columns 16.6 -> 10.3, 40 rows of 64 columns 8.0 -> 5.7): chains of the same length over other k.
 constexpr int SKM = 4, SK_WARPS = 4;
 
 // (One block per SM as the stated least: without it the compiler keeps to 96 registers and half the loads in flight, 14.4 -> 18.5 us at 18 columns.)
-template <int SKN>
+template <int SKN, bool VEC>
 __global__ void __launch_bounds__(SK_WARPS * 32, 1) gemm_skinny_f32_kernel(GemmArgs a) {
     griddep_wait();
     griddep_launch();
@@ -592,6 +593,25 @@ __global__ void __launch_bounds__(SK_WARPS * 32, 1) gemm_skinny_f32_kernel(GemmA
     for (int i = 0; i < SKM; ++i)
 #pragma unroll
         for (int j = 0; j < SKN; ++j) acc[i][j] = 0.f;
+    if (VEC) {                                            // a lane takes four k at a time
+#pragma unroll 2
+        for (int k = lane * 4; k < a.K; k += 128) {
+            float4 xv[SKM], wv[SKN];
+#pragma unroll
+            for (int i = 0; i < SKM; ++i) xv[i] = *(const float4*)(x[i] + k);
+#pragma unroll
+            for (int j = 0; j < SKN; ++j) wv[j] = *(const float4*)(w[j] + k);
+#pragma unroll
+            for (int i = 0; i < SKM; ++i)
+#pragma unroll
+                for (int j = 0; j < SKN; ++j) {
+                    acc[i][j] = fmaf(xv[i].x, wv[j].x, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].y, wv[j].y, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].z, wv[j].z, acc[i][j]);
+                    acc[i][j] = fmaf(xv[i].w, wv[j].w, acc[i][j]);
+                }
+        }
+    } else {
 #pragma unroll 4
     for (int k = lane; k < a.K; k += 32) {
         float xv[SKM], wv[SKN];
@@ -603,6 +623,7 @@ __global__ void __launch_bounds__(SK_WARPS * 32, 1) gemm_skinny_f32_kernel(GemmA
         for (int i = 0; i < SKM; ++i)
 #pragma unroll
             for (int j = 0; j < SKN; ++j) acc[i][j] = fmaf(xv[i], wv[j], acc[i][j]);
+    }
     }
 #pragma unroll
     for (int i = 0; i < SKM; ++i)
@@ -640,8 +661,10 @@ int pgk_gemm_groups_f32(const float* A, int lda, const int32_t* a_rows, const vo
     cudaStream_t st = (cudaStream_t)stream;
     if (wdt == 0 && epilogue == 0 && !group_off && !a_rows && N <= 64) {        // router logits: few columns, float32 weights
         const int gx = (M + SK_WARPS * SKM - 1) / (SK_WARPS * SKM);
-        if (N <= 4) PGK_CUDA(launch_waiting(gemm_skinny_f32_kernel<4>, dim3(gx), dim3(SK_WARPS * 32), 0, st, a));
-        else PGK_CUDA(launch_waiting(gemm_skinny_f32_kernel<8>, dim3(gx, (N + 7) / 8), dim3(SK_WARPS * 32), 0, st, a));
+        const bool vec = K % 4 == 0 && lda % 4 == 0 && (((uintptr_t)A | (uintptr_t)W) & 15) == 0;
+        const auto kernel = N <= 4 ? (vec ? gemm_skinny_f32_kernel<4, true> : gemm_skinny_f32_kernel<4, false>)
+                                   : (vec ? gemm_skinny_f32_kernel<8, true> : gemm_skinny_f32_kernel<8, false>);
+        PGK_CUDA(launch_waiting(kernel, dim3(gx, N <= 4 ? 1 : (N + 7) / 8), dim3(SK_WARPS * 32), 0, st, a));
         return 0;
     }
     const int bound = group_off ? total_rows : M;

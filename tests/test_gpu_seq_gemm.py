@@ -552,3 +552,15 @@ def test_float32_rows_sum_in_the_order_of_k(M, N, K, epi):
         z = z.astype(np.float64)
         ref = np.maximum(z, 0) ** 2 if epi == 6 else gelu_tanh(z[:, 0::2]) * z[:, 1::2]
         assert np.allclose(got, ref, rtol=2e-5, atol=2e-6)
+
+
+@pytest.mark.parametrize("M,N,K", [(9, 1, 1), (17, 4, 127), (30, 5, 128), (16, 18, 132), (33, 64, 260), (100, 8, 1023), (12, 17, 2048)])
+def test_router_logits_by_fours_and_one_by_one(M, N, K):
+    """float32 rows of few columns, k that is and is not a multiple of a lane's four and of a warp's 128; each lane adds ceil(K / 32) + 4 products, five
+    more sums join the lanes: so many half units of 2^-24, twice for products rounded into sums"""
+    A, W = operands(M + N, M, N, K)
+    W = W[0] + np.float32(1e-4)
+    a, w, c = gk.from_numpy(A), gk.from_numpy(W), gk.from_numpy(np.zeros((M, N), np.float32))
+    api.gemm_rows_f32(a.device_ptr, K, None, w.device_ptr, 0, 0, c.device_ptr, N, M, N, K, None, 1, M, 0, 1.0, 0.0, None)
+    ref, tol = A.astype(np.float64) @ W.astype(np.float64).T, (K / 32 + 10) * 2.0 ** -23 * (np.abs(A.astype(np.float64)) @ np.abs(W.astype(np.float64)).T)
+    assert (np.abs(c.to_numpy() - ref) <= tol).all()
