@@ -168,6 +168,7 @@ class LayeredCausalModel:
         self.use_graphs = os.environ.get("PGK_LAYERED_GRAPH", "1") != "0"
         self._graphs: dict = {}
         self._graph_warm: set = set()
+        self._graphs_of = 0                            # version of the cache's arrays that the captured steps read
         self._gstream: Stream | None = None            # captures
         self._last_stream: tuple | None = None         # the stream of the last step
         self._tile_sizes = {b.mixer.queries_per_tile for b in blocks if b.mixer.queries_per_tile}
@@ -180,26 +181,39 @@ class LayeredCausalModel:
         states = [tuple(getattr(self.blocks[li], "state_shapes", ())) for li, _ in self.runs]
         pools = [getattr(self.blocks[li].mixer.spec, "pool", 0) for li, _ in self.runs]
         self.cache = PagedKVCache(shapes, self.dtype, page_size, max_tokens, slots, state_shapes=states, pools=pools)
+        self._forget_graphs()
+        return self.cache
+
+    def _forget_graphs(self) -> None:
+        """An array that captured steps read or write is another one now: none of them runs again."""
         if self._graphs:
             api.device_sync()
         self._graphs.clear()
         self._graph_warm.clear()
-        return self.cache
 
     def _buffers(self, rows: int) -> RowBuffers:
         if self._buf is None or self._buf.rows < rows:
+            self._forget_graphs()
             self._buf = RowBuffers(self.config, max(rows, 2 * self._buf.rows if self._buf else 0))
         return self._buf
 
     def _workspace(self, n_floats: int) -> GPUArray:
         if self._ws is None or self._ws.size < n_floats:
+            self._forget_graphs()
             self._ws = GPUArray((max(1 << 20, 2 * n_floats),), float32)
         return self._ws
 
     def _meta_buffer(self, n: int) -> GPUArray:
         if self._meta is None or self._meta.size < n:
+            self._forget_graphs()
             self._meta = GPUArray((max(1024, 2 * n),), int32)
         return self._meta
+
+    def _logits(self, n: int) -> GPUArray:
+        if self._out is None or self._out.shape[0] < max(n, 1):
+            self._forget_graphs()
+            self._out = GPUArray((max(n, 16), self.config.vocab_size), float32)
+        return self._out
 
     # ------------------------------------------------------------------ the step
     def _forward(self, ctx: StepContext) -> None:
@@ -235,15 +249,14 @@ class LayeredCausalModel:
             self.lm_head.forward(xn.device_ptr, W, n, self._out.device_ptr, V)
 
     def _graph_key(self, ctx: StepContext):
-        """Decode steps (one token per request) replay a captured CUDA graph: the step's description
-        lives in device buffers whose addresses, and every launch shape, are fixed by this key."""
+        """Decode steps (one token per request) replay a captured CUDA graph: every launch shape is fixed by this key, and the arrays
+        -- the step's description lives in one of them -- stay the same ones as long as captured steps are kept (`_forget_graphs`)."""
         if not self.use_graphs or ctx.T > GRAPH_ROWS or not ctx.decode_only:
             return None
-        c = self.cache
-        arrays = tuple(a.device_ptr for a in c.k if a is not None)[:1] + tuple(a.device_ptr for st in c.state for a in st)[:1]
-        return (ctx.T, ctx.n_want, c.pool.max_pages, c.table_dev.device_ptr, arrays, id(ctx.buf),
-                self._meta.device_ptr, self._out.device_ptr, self._ws.device_ptr if self._ws is not None else 0,
-                tuple(blk.mixer.key_slices(ctx) for blk in self.blocks))
+        if self._graphs_of != self.cache.version:
+            self._forget_graphs()
+            self._graphs_of = self.cache.version
+        return (ctx.T, ctx.n_want, tuple(blk.mixer.key_slices(ctx) for blk in self.blocks))
 
     def step_device(self, entries, end=()) -> tuple[GPUArray | None, int]:
         """Run one ragged batch; returns (float32 logits [n_want, vocab] on the device or None, n_want).  `end` names
@@ -252,7 +265,6 @@ class LayeredCausalModel:
         stream the current one; a prompt, and any call that names a stream by its handle, needs a wait or an event of the caller's own."""
         if self.cache is None:
             self.init_cache()
-        V = self.config.vocab_size
         if not entries:                                # nothing to run: only give back what `end` names
             for seq_id in end:
                 self.cache.release(seq_id)
@@ -262,8 +274,7 @@ class LayeredCausalModel:
             api.device_sync()                          # the step before ran on another stream, on the same arrays
             self._last_stream = (stream,)
         ctx = StepContext(self, entries, self._tile_sizes, self._tops)
-        if self._out is None or self._out.shape[0] < max(ctx.n_want, 1):
-            self._out = GPUArray((max(ctx.n_want, 16), V), float32)
+        self._logits(ctx.n_want)
         key = self._graph_key(ctx)
         if key is None:
             self._forward(ctx)

@@ -23,6 +23,7 @@ front (`tokens_hint`) avoids both.
 from __future__ import annotations
 
 import heapq
+import itertools
 
 import numpy as np
 
@@ -31,6 +32,9 @@ from ..core.array import GPUArray
 from ..core.dtypes import bfloat16, float32, int32
 from ..core.factory import zeros
 from ..core.stream import current_stream_handle as _st
+
+
+_versions = itertools.count(1)
 
 
 class PagePool:
@@ -142,7 +146,9 @@ class PagedKVCache:
     (a layer that runs several times in a loop has one per run); vdim 0: the layer keeps one array whose rows serve as
     keys and, by a prefix, as values (latent attention) -- `v[i]` is then None; kv_heads 0: the layer has no pages at all.
     `state_shapes` = per cache the float32 elements per slot of each of its state arrays; `pools` = per cache the block size of
-    its pooled rows (0: none; `pk[i]`, `pv[i]` are then None)."""
+    its pooled rows (0: none; `pk[i]`, `pv[i]` are then None).
+    `version` names the device arrays that are in use: another number, never given before in this process, whenever any of them is
+    replaced.  (Their addresses name them no longer: freed memory comes back, for one array of a set and not for the next.)"""
 
     def __init__(self, layer_shapes: list[tuple[int, int, int]], dtype: str = "bfloat16", page_size: int = 64,
                  tokens_hint: int = 4096, slots: int = 8, state_shapes: "list[tuple] | None" = None,
@@ -192,6 +198,7 @@ class PagedKVCache:
         if copy_from is not None:
             api.device_sync()
         self.k, self.v, self.pk, self.pv = new
+        self.version = next(_versions)
         self._pages_dev = pages
 
     def _alloc_state(self, slots: int, copy_from) -> None:
@@ -207,6 +214,7 @@ class PagedKVCache:
         if copy_from is not None:
             api.device_sync()
         self.state = new
+        self.version = next(_versions)
         self._slots_dev = slots
 
     @property
@@ -236,6 +244,7 @@ class PagedKVCache:
         t = self.pool.table
         if self.table_dev.size != t.size:
             self.table_dev = GPUArray((t.size,), int32)
+            self.version = next(_versions)
         api.upload(self.table_dev.device_ptr, t.ctypes.data, t.nbytes, _st())       # a copy is taken: `t` may change at once
         self.pool.dirty = False
 

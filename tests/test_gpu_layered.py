@@ -600,6 +600,25 @@ def test_decode_steps_of_many_requests_replay_as_they_run(requests):
     assert all(np.array_equal(a, b) for a, b in zip(*outs))
 
 
+@pytest.mark.parametrize("hint", [2048, 64])
+def test_captured_steps_end_with_the_arrays_they_were_captured_on(hint):
+    """decode steps between prompts that outgrow the work arrays (and a small cache its pages) again and again: as without captured steps"""
+    outs = []
+    for graphs in (False, True):
+        cfg, _, m = make("mixed_stack")
+        m.use_graphs = graphs
+        m.init_cache(max_tokens=hint, slots=2)
+        m.step([(r, tokens(cfg, 3, seed=r), []) for r in range(2)])
+        out = []
+        for i, rows in enumerate((8, 16, 40, 100, 300)):
+            for j in range(3):
+                out.append(m.step([(r, tokens(cfg, 1, seed=100 * i + 10 * j + r), [0]) for r in range(2)]))
+            assert bool(m._graphs) == graphs
+            out.append(m.step([("p", tokens(cfg, rows, seed=50 + i), [rows - 1])], end=["p"]))
+        outs.append(out)
+    assert all(np.array_equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("portion", [9, 40, 300])
 def test_outputs_left_in_bfloat16_have_the_bits_of_the_rounding_product(portion, monkeypatch):
     """attention outputs and gate/up rows that only the next product reads: rounded where they are formed or where they are read, the same logits"""

@@ -1,0 +1,117 @@
+"""Which captured decode steps a layered model keeps, from the calls that it makes: no GPU."""
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+
+from pygpukit_b200.llm import paged_cache
+from pygpukit_b200.llm.models import layered
+
+
+class Array:
+    """a device array whose memory comes back at the address it had"""
+
+    def __init__(self, shape, dtype=None):
+        self.shape, self.size, self.device_ptr, self.nbytes = tuple(shape), int(np.prod(shape)), 4096, 4 * int(np.prod(shape))
+
+
+class Api:
+    def __init__(self):
+        self.calls = []
+
+    def __getattr__(self, name):
+        return lambda *a: self.calls.append(name)
+
+
+@pytest.fixture
+def model(monkeypatch):
+    api = Api()
+    monkeypatch.setattr(layered, "api", api)
+    monkeypatch.setattr(paged_cache, "api", api)
+    monkeypatch.setattr(layered, "GPUArray", Array)
+    monkeypatch.setattr(paged_cache, "GPUArray", Array)
+    monkeypatch.setattr(paged_cache, "zeros", Array)
+    # an object that takes the place, and so the identity, of the one before it
+    monkeypatch.setattr(layered, "RowBuffers", lambda config, rows, _one=SimpleNamespace(): vars(_one).update(rows=rows) or _one)
+    m = object.__new__(layered.LayeredCausalModel)
+    m.config, m.dtype, m.blocks, m.runs, m.trace_hook = SimpleNamespace(vocab_size=10), "bfloat16", [], [], None
+    m.use_graphs, m._graphs, m._graph_warm, m._gstream, m._last_stream = True, {}, set(), None, None
+    m._graphs_of, m._buf, m._meta, m._out, m._ws = 0, None, None, None, None
+    m._tile_sizes, m._tops = set(), set()
+    m.cache = paged_cache.PagedKVCache([(1, 8, 8)], tokens_hint=256, slots=4, state_shapes=[(8,)])
+    m.ran, m.captures = [], []
+    m._forward = lambda ctx: m.ran.append(ctx.T)
+
+    class Graph:
+        _exec = 1
+
+        def capture(self, stream):
+            import contextlib
+            m.captures.append(1)
+            return contextlib.nullcontext()
+
+    monkeypatch.setattr(layered, "CudaGraph", Graph)
+    monkeypatch.setattr(layered, "Stream", lambda: None)
+    m.api = api
+    return m
+
+
+def decode(m, ids, times=1):
+    for _ in range(times):
+        m.step_device([(i, [1], [0]) for i in ids])
+
+
+def start(m, ids, n=3):
+    m.step_device([(i, [1] * n, [n - 1]) for i in ids])
+
+
+def captured(m, ids):
+    """decode steps until one is replayed; another one of the same kind then is no new capture"""
+    for _ in range(40):
+        if m._graphs:
+            break
+        decode(m, ids)
+    n = len(m.captures)
+    decode(m, ids)
+    assert m._graphs and len(m.captures) == n
+
+
+def grow_rows(m):
+    m.step_device([("long", [1] * (m._buf.rows + 1), [])])
+
+
+def grow_pages(m):
+    ptrs = [a.device_ptr for a in m.cache.k]
+    m.step_device([("much", [1] * (m.cache.pool.free_pages * 64 + 1), [])])
+    assert [a.device_ptr for a in m.cache.k] == ptrs         # the fault's condition: the same address, another array
+
+
+def grow_slots(m):
+    start(m, [f"more{i}" for i in range(4)], 1)
+
+
+@pytest.mark.parametrize("grow", [grow_rows, grow_pages, grow_slots, lambda m: m._workspace(1 << 24), lambda m: m._meta_buffer(1 << 20),
+                                  lambda m: m._logits(100)], ids=["rows", "pages", "slots", "workspace", "description", "logits"])
+def test_no_captured_step_outlives_an_array_of_its_launches(model, grow):
+    """Addresses and identities of freed arrays come back; a captured step that names the arrays before must not."""
+    m = model
+    start(m, "ab")
+    captured(m, "ab")
+    replays = m.api.calls.count("graph_launch")
+    grow(m)
+    decode(m, "ab")
+    assert m.api.calls.count("graph_launch") == replays      # launched one by one, on the new arrays
+    captured(m, "ab")
+
+
+def test_captured_steps_stay_while_the_arrays_do(model):
+    m = model
+    start(m, "abc")
+    for ids in ("abc", "ab", "a"):
+        decode(m, ids, 5)
+    n = len(m.captures)
+    start(m, "d")
+    m.release("d")
+    for ids in ("abc", "ab", "a"):
+        decode(m, ids)
+    assert len(m.captures) == n
