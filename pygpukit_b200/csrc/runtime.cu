@@ -10,7 +10,6 @@
 #include <cstdarg>
 #include <cstring>
 #include <mutex>
-#include <unordered_map>
 
 namespace pgk {
 
@@ -180,51 +179,6 @@ static void upload_trim() {
         }
 }
 
-// ---- frees that do not wait.  cudaFree waits for the whole device: a caller that drops the array of the call before (the logits of a prompt)
-// could not launch ahead, and the device idled in each call.  Blocks of up to kLateBlock bytes wait instead, untouched and reused by nobody,
-// until the device is idle anyway (pgk_device_sync), their memory is asked for (pgk_mem_info, pgk_mem_trim, an allocation that fails), or
-// kLateBytes or kLateBlocks of them wait; cudaFree then takes them as ever (a prompt of 512 tokens and its logits: 427 -> 394 us).
-static constexpr size_t kLateBlock = 16ull << 20, kLateBytes = 64ull << 20;
-static constexpr int kLateBlocks = 512;
-static std::mutex g_late_mu;
-static std::unordered_map<void*, size_t> g_late_sizes;              // of blocks that may wait
-static void* g_late[kLateBlocks];
-static size_t g_late_bytes = 0;
-static int g_late_n = 0;
-
-static cudaError_t late_flush() {
-    void* blocks[kLateBlocks];
-    int n;
-    {
-        std::lock_guard<std::mutex> lk(g_late_mu);
-        n = g_late_n;
-        memcpy(blocks, g_late, n * sizeof(void*));
-        g_late_n = 0;
-        g_late_bytes = 0;
-    }
-    cudaError_t first = cudaSuccess;
-    for (int i = 0; i < n; ++i) {
-        const cudaError_t e = cudaFree(blocks[i]);
-        if (first == cudaSuccess) first = e;
-    }
-    return first;
-}
-static cudaError_t late_free(void* ptr) {
-    {
-        std::lock_guard<std::mutex> lk(g_late_mu);
-        const auto it = g_late_sizes.find(ptr);
-        const size_t bytes = it == g_late_sizes.end() ? kLateBytes + 1 : it->second;
-        if (it != g_late_sizes.end()) g_late_sizes.erase(it);
-        if (g_late_n < kLateBlocks && g_late_bytes + bytes <= kLateBytes) {
-            g_late[g_late_n++] = ptr;
-            g_late_bytes += bytes;
-            return cudaSuccess;
-        }
-    }
-    const cudaError_t e = cudaFree(ptr), f = late_flush();
-    return e != cudaSuccess ? e : f;
-}
-
 // ---- bounded waits
 static std::mutex g_wait_mu;
 static std::atomic<int*> g_wait_words{nullptr};
@@ -318,7 +272,6 @@ int pgk_device_props(int device, pgk_device_props_t* out) {
 int pgk_sm_count(void) { return sm_count(); }
 int pgk_device_sync(void) {
     PGK_CUDA(cudaDeviceSynchronize());
-    PGK_CUDA(late_flush());
     return wait_check();
 }
 int pgk_wait_probe(int limit_us, int32_t* ran_out, void* stream) {
@@ -329,13 +282,11 @@ int pgk_wait_probe(int limit_us, int32_t* ran_out, void* stream) {
     return 0;
 }
 int pgk_mem_info(size_t* free_bytes, size_t* total_bytes) {
-    PGK_CUDA(late_flush());
     PGK_CUDA(cudaMemGetInfo(free_bytes, total_bytes));
     return 0;
 }
 
 int pgk_mem_trim(void) {
-    late_flush();
     scratch_trim();
     upload_trim();
     cudaGetLastError();
@@ -345,24 +296,17 @@ int pgk_malloc(void** ptr, size_t bytes) {
     *ptr = nullptr;
     if (bytes == 0) bytes = 1;
     cudaError_t e = cudaMalloc(ptr, bytes);
-    if (e == cudaErrorMemoryAllocation) {                         // idle work memory counts as free
-        cudaGetLastError();
-        late_flush();
-        scratch_trim();
+    if (e == cudaErrorMemoryAllocation && scratch_trim()) {       // idle work memory counts as free
         cudaGetLastError();
         e = cudaMalloc(ptr, bytes);
     }
     PGK_CUDA(e);
-    if (bytes <= kLateBlock) {
-        std::lock_guard<std::mutex> lk(g_late_mu);
-        g_late_sizes[*ptr] = bytes;
-    }
     return 0;
 }
 int pgk_free(void* ptr) {
     if (ptr) {
         if (g_free_hook) g_free_hook(ptr);
-        PGK_CUDA(late_free(ptr));
+        PGK_CUDA(cudaFree(ptr));
     }
     return 0;
 }
