@@ -141,6 +141,50 @@ class StepContext:
 GRAPH_ROWS = 32
 
 
+class StepGraphs:
+    """Captured decode steps by what fixes their launches: the number of requests, of wanted rows, the key slices of each layer.  Up to 32
+    requests with contexts that grow make more of these than are kept, so the least recently used one leaves, and a step is captured only when
+    it has come often enough that replays can earn what a capture costs: 400 us, where a replayed step takes 30 ... 150 us less than single
+    launches.  That is the second time for the few steps of up to LinearRows.FEW requests, the fourth for others, and the 16th for all once
+    the room is used up: keys that change from step to step then cost no more than single launches."""
+    ROOM, SEEN = 64, 1024
+
+    def __init__(self):
+        self._kept: dict = {}                          # least recently used first
+        self._seen: dict = {}                          # times that steps without a graph have run, oldest first
+
+    def __len__(self) -> int:
+        return len(self._kept)
+
+    def get(self, key):
+        g = self._kept.pop(key, None)
+        if g is not None:
+            self._kept[key] = g
+        return g
+
+    def due(self, key) -> bool:
+        """Whether a step without a graph is captured now; counts it otherwise.  The first one always runs (kernel attributes, workspaces)."""
+        n = self._seen.pop(key, 0)
+        if n >= (15 if len(self._kept) >= self.ROOM else 1 if key[0] <= LinearRows.FEW else 3):
+            return True
+        self._seen[key] = n + 1
+        if len(self._seen) > self.SEEN:
+            del self._seen[next(iter(self._seen))]
+        return False
+
+    def make_room(self) -> None:
+        """Before a capture, with nothing running."""
+        while len(self._kept) >= self.ROOM:
+            del self._kept[next(iter(self._kept))]
+
+    def keep(self, key, graph) -> None:
+        self._kept[key] = graph
+
+    def clear(self) -> None:
+        self._kept.clear()
+        self._seen.clear()
+
+
 class LayeredCausalModel:
     def __init__(self, config: LayeredConfig, embed_tokens: GPUArray, blocks: list, final_norm, lm_head: LinearRows,
                  dtype: str = "bfloat16", embed_norm: RowNorm | None = None):
@@ -166,8 +210,7 @@ class LayeredCausalModel:
         self._out: GPUArray | None = None
         self._ws: GPUArray | None = None
         self.use_graphs = os.environ.get("PGK_LAYERED_GRAPH", "1") != "0"
-        self._graphs: dict = {}
-        self._graph_warm: set = set()
+        self._graphs = StepGraphs()
         self._graphs_of = 0                            # version of the cache's arrays that the captured steps read
         self._gstream: Stream | None = None            # captures
         self._last_stream: tuple | None = None         # the stream of the last step
@@ -189,7 +232,6 @@ class LayeredCausalModel:
         if self._graphs:
             api.device_sync()
         self._graphs.clear()
-        self._graph_warm.clear()
 
     def _buffers(self, rows: int) -> RowBuffers:
         if self._buf is None or self._buf.rows < rows:
@@ -280,22 +322,18 @@ class LayeredCausalModel:
             self._forward(ctx)
         else:
             g = self._graphs.get(key)
-            if g is None and key not in self._graph_warm:
-                self._graph_warm.add(key)              # first sight: run eagerly (kernel attributes, workspaces)
-                self._forward(ctx)
-                if self._graph_key(ctx) != key:        # the eager run grew a workspace: forget the stale key
-                    self._graph_warm.discard(key)
+            if g is None and not self._graphs.due(key):
+                self._forward(ctx)                     # an array that grows in it takes the count with it
             else:
                 if self._gstream is None:
                     self._gstream = Stream()
                 if g is None:
                     g = CudaGraph()
                     api.device_sync()
-                    if len(self._graphs) >= 64:
-                        self._graphs.clear()
+                    self._graphs.make_room()
                     with g.capture(self._gstream):
                         self._forward(ctx)
-                    self._graphs[key] = g
+                    self._graphs.keep(key, g)
                 api.graph_launch(g._exec, stream)      # in the caller's order, like an eager step
                 leave_open()
         for seq_id in end:

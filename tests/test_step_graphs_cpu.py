@@ -35,10 +35,10 @@ def model(monkeypatch):
     monkeypatch.setattr(layered, "RowBuffers", lambda config, rows, _one=SimpleNamespace(): vars(_one).update(rows=rows) or _one)
     m = object.__new__(layered.LayeredCausalModel)
     m.config, m.dtype, m.blocks, m.runs, m.trace_hook = SimpleNamespace(vocab_size=10), "bfloat16", [], [], None
-    m.use_graphs, m._graphs, m._graph_warm, m._gstream, m._last_stream = True, {}, set(), None, None
+    m.use_graphs, m._graphs, m._gstream, m._last_stream = True, layered.StepGraphs(), None, None
     m._graphs_of, m._buf, m._meta, m._out, m._ws = 0, None, None, None, None
     m._tile_sizes, m._tops = set(), set()
-    m.cache = paged_cache.PagedKVCache([(1, 8, 8)], tokens_hint=256, slots=4, state_shapes=[(8,)])
+    m.cache = paged_cache.PagedKVCache([(1, 8, 8)], tokens_hint=1 << 18, slots=40, state_shapes=[(8,)])
     m.ran, m.captures = [], []
     m._forward = lambda ctx: m.ran.append(ctx.T)
 
@@ -87,7 +87,7 @@ def grow_pages(m):
 
 
 def grow_slots(m):
-    start(m, [f"more{i}" for i in range(4)], 1)
+    start(m, [f"more{i}" for i in range(40)], 1)
 
 
 @pytest.mark.parametrize("grow", [grow_rows, grow_pages, grow_slots, lambda m: m._workspace(1 << 24), lambda m: m._meta_buffer(1 << 20),
@@ -115,3 +115,38 @@ def test_captured_steps_stay_while_the_arrays_do(model):
     for ids in ("abc", "ab", "a"):
         decode(m, ids)
     assert len(m.captures) == n
+
+
+def churn(m, period, steps):
+    """decode steps of kinds that come by turns: `period` of them, 9 to 32 requests and different key slices"""
+    ids = [f"r{i}" for i in range(32)]
+    start(m, ids, 1)
+    m._logits(32), m._meta_buffer(1 << 16)
+    m.blocks = [SimpleNamespace(mixer=SimpleNamespace(key_slices=lambda ctx: m.plan))]
+    m.plan = 0
+    for i in range(steps):
+        m.plan, n = divmod(i % period, 24)
+        decode(m, ids[:9 + n])
+
+
+@pytest.mark.parametrize("period", [24, 64, 65, 100, 300])
+def test_steps_whose_kind_changes_are_not_captured_again_and_again(model, period):
+    """What fits is captured once; what does not runs as single launches, a capture at most every sixteenth time of its kind."""
+    m = model
+    churn(m, period, 20 * period)
+    assert len(m._graphs) == min(period, 64)
+    assert len(m.captures) <= min(period, 64) + (period > 64) * 20 * period // 16
+
+
+def test_kinds_that_come_no_more_make_room(model):
+    m = model
+    churn(m, 64, 64 * 6)
+    assert len(m._graphs) == 64
+    n, ids = len(m.captures), [f"r{i}" for i in range(20)]
+    m.plan = 7                                               # contexts have grown
+    decode(m, ids, 16)
+    assert len(m.captures) == n + 1 and len(m._graphs) == 64
+    decode(m, ids, 50)
+    m.plan = 0
+    decode(m, ids)                                           # used last before that: still there
+    assert len(m.captures) == n + 1
