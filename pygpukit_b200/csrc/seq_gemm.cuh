@@ -64,7 +64,7 @@ inline bool few_rows_pay(int M, int N, int K, int batch) {
 }
 
 // Matrices whose rows the copies cannot fetch, brought to 16-byte boundaries in work memory: *b is the product on them.  *done is false, and nothing is
-// launched, without room for them.
+// launched, without room for them.  (Inside a capture the room is had when the graph is made or launched, and that call fails without it.)
 int pad_weights(const GemmArgs& a, int matrices, cudaStream_t st, GemmArgs* b, bool* done);
 
 // The same for few rows, in one launch without work memory: `batch` products over the same rows, or blocks of rows_per_block (at most 32)

@@ -20,6 +20,7 @@ import os
 import numpy as np
 
 from ..._lib import api
+from ...core import idle
 from ...core.array import GPUArray
 from ...core.dtypes import float32, int32
 from ...core.stream import CudaGraph, Stream, current_stream_handle as _st, leave_open
@@ -152,6 +153,7 @@ class StepGraphs:
     def __init__(self):
         self._kept: dict = {}                          # least recently used first
         self._seen: dict = {}                          # times that steps without a graph have run, oldest first
+        self._refused: set = set()
 
     def __len__(self) -> int:
         return len(self._kept)
@@ -164,6 +166,8 @@ class StepGraphs:
 
     def due(self, key) -> bool:
         """Whether a step without a graph is captured now; counts it otherwise.  The first one always runs (kernel attributes, workspaces)."""
+        if key in self._refused:
+            return False
         n = self._seen.pop(key, 0)
         if n >= (15 if len(self._kept) >= self.ROOM else 1 if key[0] <= LinearRows.FEW else 3):
             return True
@@ -180,9 +184,17 @@ class StepGraphs:
     def keep(self, key, graph) -> None:
         self._kept[key] = graph
 
+    def refuse(self, key) -> None:
+        """The device has no room for this step's graph: it stays with single launches."""
+        self._kept.pop(key, None)
+        if len(self._refused) >= self.SEEN:
+            self._refused.clear()
+        self._refused.add(key)
+
     def clear(self) -> None:
         self._kept.clear()
         self._seen.clear()
+        self._refused.clear()
 
 
 class LayeredCausalModel:
@@ -300,6 +312,30 @@ class LayeredCausalModel:
             self._graphs_of = self.cache.version
         return (ctx.T, ctx.n_want, tuple(blk.mixer.key_slices(ctx) for blk in self.blocks))
 
+    def _replay(self, key, g, ctx: StepContext, stream) -> bool:
+        """Launch the step's graph, captured first where there is none (g None).  Work memory of a graph is had when it is made or launched,
+        too late for a kernel that needs none to take the place of one that does: False, and nothing is launched, where the device has
+        no room for it."""
+        try:
+            if g is None:
+                if self._gstream is None:
+                    self._gstream = Stream()
+                g = CudaGraph()
+                api.device_sync()
+                self._graphs.make_room()
+                with g.capture(self._gstream):
+                    self._forward(ctx)
+                self._graphs.keep(key, g)
+            api.graph_launch(g._exec, stream)          # in the caller's order, like an eager step
+        except RuntimeError as e:
+            if not idle.out_of_memory(e):
+                raise
+            api.device_sync()                          # the graph may still run for the step before
+            self._graphs.refuse(key)
+            return False
+        leave_open()
+        return True
+
     def step_device(self, entries, end=()) -> tuple[GPUArray | None, int]:
         """Run one ragged batch; returns (float32 logits [n_want, vocab] on the device or None, n_want).  `end` names
         the requests whose cache is given back after the step.  The step runs in the order of the current stream and is not waited for: what
@@ -324,18 +360,8 @@ class LayeredCausalModel:
             g = self._graphs.get(key)
             if g is None and not self._graphs.due(key):
                 self._forward(ctx)                     # an array that grows in it takes the count with it
-            else:
-                if self._gstream is None:
-                    self._gstream = Stream()
-                if g is None:
-                    g = CudaGraph()
-                    api.device_sync()
-                    self._graphs.make_room()
-                    with g.capture(self._gstream):
-                        self._forward(ctx)
-                    self._graphs.keep(key, g)
-                api.graph_launch(g._exec, stream)      # in the caller's order, like an eager step
-                leave_open()
+            elif not self._replay(key, g, ctx, stream):
+                self._forward(ctx)
         for seq_id in end:
             self.cache.release(seq_id)
         return (self._out if ctx.n_want else None), ctx.n_want

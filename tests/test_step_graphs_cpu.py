@@ -17,10 +17,14 @@ class Array:
 
 class Api:
     def __init__(self):
-        self.calls = []
+        self.calls, self.fails = [], {}
 
     def __getattr__(self, name):
-        return lambda *a: self.calls.append(name)
+        def call(*a):
+            self.calls.append(name)
+            if name in self.fails:
+                raise RuntimeError(self.fails[name])
+        return call
 
 
 @pytest.fixture
@@ -48,6 +52,8 @@ def model(monkeypatch):
         def capture(self, stream):
             import contextlib
             m.captures.append(1)
+            if "graph_end" in api.fails:
+                raise RuntimeError(api.fails["graph_end"])
             return contextlib.nullcontext()
 
     monkeypatch.setattr(layered, "CudaGraph", Graph)
@@ -150,3 +156,22 @@ def test_kinds_that_come_no_more_make_room(model):
     m.plan = 0
     decode(m, ids)                                           # used last before that: still there
     assert len(m.captures) == n + 1
+
+
+@pytest.mark.parametrize("call", ["graph_end", "graph_launch"])
+def test_a_step_whose_graph_finds_no_room_runs_as_single_launches(model, call):
+    """The memory of a graph's own allocations is had when it is made or launched; single launches take other kernels where there is none."""
+    m = model
+    start(m, "ab")
+    m.api.fails = {call: "cudaGraph... failed: out of memory"}
+    before = len(m.ran)
+    decode(m, "ab", 10)
+    assert len(m.ran) - before == 10 + (call == "graph_launch") and len(m.captures) == 1 and not m._graphs     # (a capture runs the launches' code, too)
+    decode(m, "a", 10)
+    assert len(m.captures) == 2
+    m.api.fails = {}
+    grow_rows(m)
+    captured(m, "ab")                                        # another try once the arrays are others
+    m.api.fails = {"graph_launch": "an illegal address"}
+    with pytest.raises(RuntimeError, match="illegal"):
+        decode(m, "ab")
