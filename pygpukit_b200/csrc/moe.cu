@@ -537,7 +537,9 @@ __global__ void __launch_bounds__(1024) moe_route_rows_kernel(const uint16_t* lo
     }
 }
 
-// out[t] = sum over the slots, in their order, of weight x the expert's row (+ residual): eight columns per thread, four rows in flight
+// out[t] = sum over the slots, in their order, of weight x the expert's row (+ residual): eight columns per thread, four rows in flight.
+// VEC: a caller's rows (residual, out) by 16-byte accesses; else element by element, wherever they start
+template <bool VEC>
 __global__ void __launch_bounds__(128) moe_combine_rows_bf16_kernel(const uint16_t* rows, const uint16_t* weights, const int32_t* inv, const uint16_t* residual,
                                                                     uint16_t* out, int H, int k) {
     __shared__ float w_s[32];
@@ -552,7 +554,11 @@ __global__ void __launch_bounds__(128) moe_combine_rows_bf16_kernel(const uint16
     __syncthreads();
     if (c >= H) return;
     uint4 res = make_uint4(0u, 0u, 0u, 0u);
-    if (residual) res = ld_act16(residual + (size_t)t * H + c);
+    if (residual) {
+        const uint16_t* p = residual + (size_t)t * H + c;
+        if (VEC) res = ld_act16(p);
+        else res = make_uint4(p[0] | (uint32_t)p[1] << 16, p[2] | (uint32_t)p[3] << 16, p[4] | (uint32_t)p[5] << 16, p[6] | (uint32_t)p[7] << 16);
+    }
     float sum[8] = {};
     for (int s0 = 0; s0 < k; s0 += 4) {
         uint4 v[4];
@@ -576,7 +582,12 @@ __global__ void __launch_bounds__(128) moe_combine_rows_bf16_kernel(const uint16
         o[q] = pack_bf16x2(sum[2 * q], sum[2 * q + 1]);
         if (residual) o[q] = pack_bf16x2(bf16lo(o[q]) + bf16lo(r[q]), bf16hi(o[q]) + bf16hi(r[q]));
     }
-    *(uint4*)(out + (size_t)t * H + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    uint16_t* const dst = out + (size_t)t * H + c;
+    if (VEC) *(uint4*)dst = make_uint4(o[0], o[1], o[2], o[3]);
+    else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { dst[2 * q] = (uint16_t)o[q]; dst[2 * q + 1] = (uint16_t)(o[q] >> 16); }
+    }
 }
 
 // gate and up GEMVs of the k routed experts + silu + multiply in one launch: one warp per (slot, n)
@@ -840,10 +851,10 @@ int pgk_moe_route_rows(const void* logits, void* weights, int32_t* active, int32
 }
 int pgk_moe_combine_rows_bf16(const void* expert_rows, const void* router_weights, const int32_t* inv, const void* residual, void* out, int tokens, int hidden,
                               int k, void* stream) {
-    const uintptr_t all = (uintptr_t)expert_rows | (uintptr_t)residual | (uintptr_t)out;
-    PGK_REQUIRE(k >= 1 && k <= 32 && hidden % 8 == 0 && all % 16 == 0, "moe_combine_rows_bf16 failed: k=%d hidden=%d", k, hidden);
+    PGK_REQUIRE(k >= 1 && k <= 32 && hidden % 8 == 0 && (uintptr_t)expert_rows % 16 == 0, "moe_combine_rows_bf16 failed: k=%d hidden=%d", k, hidden);
     if (tokens <= 0) return 0;
-    PGK_CUDA(launch_waiting(moe_combine_rows_bf16_kernel, dim3(tokens, (hidden + 1023) / 1024), dim3(128), 0, ST(stream), (const uint16_t*)expert_rows,
+    const auto kernel = ((uintptr_t)residual | (uintptr_t)out) % 16 == 0 ? moe_combine_rows_bf16_kernel<true> : moe_combine_rows_bf16_kernel<false>;
+    PGK_CUDA(launch_waiting(kernel, dim3(tokens, (hidden + 1023) / 1024), dim3(128), 0, ST(stream), (const uint16_t*)expert_rows,
                             (const uint16_t*)router_weights, inv, (const uint16_t*)residual, (uint16_t*)out, hidden, k));
     return 0;
 }

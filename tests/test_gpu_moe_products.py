@@ -50,6 +50,22 @@ def test_products_equal_the_row_by_row_pipeline(T, E, k, H, I):
         assert np.linalg.norm(got - ref) <= 2.0 ** -8 * np.linalg.norm(ref)
 
 
+@pytest.mark.parametrize("T,E,k,H,I", [(2, 8, 2, 128, 128), (19, 16, 4, 1152, 128)])
+@pytest.mark.parametrize("at,res_at", [(1, 0), (0, 1), (4, 3)])
+def test_rows_off_16_byte_boundaries_are_taken(T, E, k, H, I, at, res_at):
+    """an output and a residual that start `at` elements behind a boundary: the bits of those on one, and nothing beside them is written"""
+    rng = np.random.default_rng(T + at)
+    layer = _layer(rng, E, k, H, I)
+    x, r = gk.from_numpy(rand_bf16(rng, (T, H))), rand_bf16(rng, (T, H))
+    room, res = gk.from_numpy(np.zeros(T * H + 16, np.uint16)), gk.from_numpy(np.concatenate([r.reshape(-1)[:8], r.reshape(-1), r.reshape(-1)[:8]])[8 - res_at:])
+    view = lambda a, n: gk.GPUArray((T, H), gk.bfloat16, ptr=a.device_ptr + 2 * n, source=a)
+    want = layer.forward(x, residual=gk.from_numpy(r)).to_numpy()
+    got = layer.forward(x, out=view(room, at), residual=view(res, res_at))
+    assert got.device_ptr % 16 == 2 * at and np.array_equal(got.to_numpy(), want)
+    room = room.to_numpy()
+    assert (room[:at] == 0).all() and (room[at + T * H:] == 0).all()
+
+
 @pytest.mark.parametrize("offset,held", [(0, 3), (5, 3), (2, 6)])
 def test_rows_of_experts_held_elsewhere_are_zeros(offset, held):
     """The rows of the experts that are here have the bits of the whole layer's, the others are zeros."""
