@@ -141,7 +141,10 @@ gemv_bf16_kernel(const uint16_t* A, const uint16_t* B, uint16_t* __restrict__ C,
 // Five rows and more: the slabs of four read the weights again for each, and a matrix of few columns (router logits) leaves a warp to walk a
 // whole row.  Here a block has 16 rows x 8 NT columns; its 16 warps take 32 k each by turns, both operands straight from memory in pieces
 // of eight k per lane -- which k an MMA's lane names is free as long as both operands agree -- and add up through shared memory in the
-// order of the warps.  Exact products, float32 sums (mma.sync).  B200, us, slabs -> here: 15 x 3456 -> 128 29.2 -> 4.3, 64 x 4096 -> 8 117 -> 4.3.
+// order of the warps.  Exact products, float32 sums (mma.sync).  B200, us, slabs -> here: 15 x 3456 -> 128 29.2 -> 4.3, 64 x 4096 -> 8 117 -> 4.3.  The
+// slabs, which read the weights once for every four rows, are slower for any number of them: K = N = 4096, 5 / 64 / 512 / 4096 rows, cold caches, 27.6 -> 18.5,
+// 200 -> 42, 1480 -> 168, 11549 -> 1166.  From 128 rows on the operands' way from L2 bounds it -- each block fetches its own --, and the tcgen05 product of the
+// token-major models is faster on the same sizes (128 / 512 / 4096 rows 25, 35, 117; N = 128 up to 1024 rows slower than here).
 constexpr int kRowsWarps = 16;
 
 template <int NT>
@@ -291,10 +294,15 @@ static int bf16_dispatch(const void* A, const void* B, void* C, int M, int K, in
             if (pgk_rmsnorm(A, gamma, normed, M, K, eps, 2, st)) { scratch_free(normed, st); return 1; }
             a = (const uint16_t*)normed;
         }
-        GemvEpilogue epi = {(const uint16_t*)bias, (const uint16_t*)residual};
-        const int wide = (N + 31) / 32 * ((M + 15) / 16) >= sm_count();
+        const bool wide = (long long)((N + 31) / 32) * ((M + 15) / 16) >= sm_count();
         const auto kernel = wide ? gemm_bf16_rows_kernel<4> : gemm_bf16_rows_kernel<1>;
-        const cudaError_t e = launch_waiting(kernel, dim3((N + (wide ? 31 : 7)) / (wide ? 32 : 8), (M + 15) / 16), dim3(kRowsWarps * 32), 0, st, a, b, c, M, K, N, epi);
+        cudaError_t e = cudaSuccess;
+        for (long long m0 = 0; m0 < M && e == cudaSuccess; m0 += 16 * 65535) {         // what a grid holds
+            const int rows = (int)(M - m0 < 16 * 65535 ? M - m0 : 16 * 65535);
+            const size_t at = (size_t)m0 * N;
+            GemvEpilogue epi = {(const uint16_t*)bias, residual ? (const uint16_t*)residual + at : nullptr};
+            e = launch_waiting(kernel, dim3((N + (wide ? 31 : 7)) / (wide ? 32 : 8), (rows + 15) / 16), dim3(kRowsWarps * 32), 0, st, a + (size_t)m0 * K, b, c + at, rows, K, N, epi);
+        }
         if (normed) if (const int rc = scratch_free(normed, st)) return rc;
         PGK_CUDA(e);
         return 0;

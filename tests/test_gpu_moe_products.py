@@ -98,6 +98,22 @@ def test_fused_gate_up_equals_product_and_activation(M, K, I):
     assert np.array_equal(one.to_numpy(), two.to_numpy())
 
 
+@pytest.mark.parametrize("bias,residual", [(False, False), (True, True)])
+def test_bf16_rows_beyond_a_grid(bias, residual):
+    """more blocks of 16 rows than a grid has places for"""
+    rng = np.random.default_rng(1)
+    M, K, N = 16 * 65535 + 21, 16, 3
+    A, B, bb, rr = rand_bf16(rng, (M, K)), rand_bf16(rng, (N, K)), rand_bf16(rng, (N,)), rand_bf16(rng, (M, N))
+    a, b, bd, rd, c = (gk.from_numpy(v) for v in (A, B, bb, rr, np.zeros((M, N), np.uint16)))
+    api.gemv_bf16_ex(a.device_ptr, b.device_ptr, c.device_ptr, M, K, N, bd.device_ptr if bias else None, rd.device_ptr if residual else None, None)
+    x, y = f32(A).astype(np.float64), f32(B).astype(np.float64)
+    ref = x @ y.T
+    s = ref + bias * f32(bb).astype(np.float64)
+    out = s + residual * f32(rr).astype(np.float64)
+    # as below: one rounding of the sum, one more behind the bias and one behind the residual
+    assert (np.abs(f32(c.to_numpy()) - out) <= 2.0 ** -7 * (np.abs(ref) + np.abs(s) + np.abs(out)) + 2.0 ** -20 * (np.abs(x) @ np.abs(y).T)).all()
+
+
 @pytest.mark.parametrize("M,K,N", [(5, 16, 1), (15, 3456, 128), (16, 512, 8), (17, 2048, 130), (64, 4096, 33), (64, 48, 4096), (33, 1040, 2048)])
 def test_bf16_rows_against_float64(M, K, N):
     """exact products, float32 sums of 32 k and over the 16 warps, one rounding to BF16 (and one more behind the bias)"""
