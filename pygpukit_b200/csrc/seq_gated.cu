@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_biased_kernel(Rout
         for (int e = lane; e < a.E; e += 32)
             if (c[e] > bv) { bv = c[e]; bi = e; }
         warp_argmax(bv, bi);
+        if (bi >= a.E) bi = k;                    // no score is a number: stay in range, another one each time
         __syncwarp();
         if (lane == 0) {
             c[bi] = -INFINITY;

@@ -559,6 +559,7 @@ __global__ void __launch_bounds__(ROUTE_WARPS * 32) moe_route_kernel(RouteArgs a
         for (int e = lane; e < a.E; e += 32)
             if (open[e] && s[e] > bv) { bv = s[e]; bi = e; }
         warp_argmax(bv, bi);
+        if (bi >= a.E) { bi = k; bv = s[k]; }     // no score is a number: stay in range, another one each time
         if (lane == 0) open[bi] = 0;
         __syncwarp();
         wsum += bv;

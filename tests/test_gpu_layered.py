@@ -149,6 +149,32 @@ def test_router_and_row_lists(E, top, gc, keep, wdt):
         assert o[flat[i]] <= v[i] < o[flat[i] + 1] and p[v[i]] == i // top
 
 
+@pytest.mark.parametrize("E,top,gc,keep", [(16, 4, 1, 1), (16, 3, 4, 2), (8, 8, 1, 1), (40, 5, 5, 2)])
+@pytest.mark.parametrize("router", ["grouped", "biased"])
+def test_routers_stay_in_range_where_logits_are_no_numbers(E, top, gc, keep, router):
+    """Tokens with NaN or infinite logits get weights of NaN and experts that there are, each once; the other tokens are as without them."""
+    rng = np.random.default_rng(E + top)
+    T, bad = 13, [2, 5, 12]
+    z = rng.standard_normal((T, E)).astype(np.float32)
+    good = z.copy()
+    z[2], z[5, 1], z[12, -1] = np.nan, np.nan, np.inf
+    got = []
+    for logits in (good, z):
+        idx, mat, rank, counts = (gk.from_numpy(np.full(n, v, np.int32)) for n, v in ((T * top, -9), (T * top, -9), (T * top, -9), (E, 0)))
+        wt, zd = gk.zeros((T * top,), gk.float32), f32(logits)
+        if router == "grouped":
+            api.moe_route_grouped(zd.device_ptr, E, T, E, top, gc, keep, idx.device_ptr, wt.device_ptr, rank.device_ptr, counts.device_ptr, None)
+        else:
+            api.moe_route_biased(zd.device_ptr, E, T, E, E - 2, top, None, 1, idx.device_ptr, mat.device_ptr, wt.device_ptr, rank.device_ptr,
+                                 counts.device_ptr, None)
+        got.append((idx.to_numpy().reshape(T, top), wt.to_numpy().reshape(T, top), counts.to_numpy()))
+    (i0, w0, _), (i1, w1, n1) = got
+    rest = [t for t in range(T) if t not in bad]
+    assert np.array_equal(i0[rest], i1[rest]) and np.array_equal(w0[rest], w1[rest])
+    assert (i1 >= 0).all() and (i1 < E).all() and all(len(set(i1[t])) == top for t in bad) and np.isnan(w1[bad]).all()
+    assert np.array_equal(n1, np.bincount(i1.reshape(-1), minlength=E))
+
+
 def test_combine_layernorm_with_and_without_parts():
     rng = np.random.default_rng(5)
     T, W, top = 6, 50, 3
