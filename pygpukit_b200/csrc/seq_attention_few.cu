@@ -34,6 +34,7 @@ struct FewAttnArgs {
     AttnArgs a;
     int nd, ndv;             // 64-element chunks of a key row and of a value row
     int hb, bp, cluster;     // heads per block, positions per copy, blocks per request
+    int qvec;                // queries by pairs
     int* err;
 };
 
@@ -146,7 +147,9 @@ seq_attention_few_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_
             float x[8];
 #pragma unroll
             for (int e = 0; e < 8; e += 2) {
-                const float2 v = r < nh && k8 * 8 < D ? *(const float2*)(q + (size_t)r * D + k8 * 8 + e) : make_float2(0.f, 0.f);
+                const float* const at = q + (size_t)r * D + k8 * 8 + e;
+                float2 v = make_float2(0.f, 0.f);
+                if (r < nh && k8 * 8 < D) v = p.qvec ? *(const float2*)at : make_float2(at[0], at[1]);
                 x[e] = v.x; x[e + 1] = v.y;
             }
             uint32_t t[4][3];
@@ -509,9 +512,10 @@ int seq_attention_few(const AttnArgs& a, int tiles, int cluster, cudaStream_t st
     *served = false;
     const bool alias = a.valias;
     if (!few_fits(a.D, a.Dv, a.kld, a.vld, alias, 2, a.PS) || cluster < 1 || cluster > W_CLUSTER || few_held(cluster) <= 0) return 0;
-    if (a.prob || a.pool || a.o_inv_freq || a.keep || (uintptr_t)a.kc % 16 || (uintptr_t)a.vc % 16 || (uintptr_t)a.proj % 8 || a.ld % 2 || a.q_off % 2) return 0;
+    if (a.prob || a.pool || a.o_inv_freq || a.keep || (uintptr_t)a.kc % 16 || (uintptr_t)a.vc % 16) return 0;
     FewAttnArgs p{};
     p.a = a;
+    p.qvec = (uintptr_t)a.proj % 8 == 0 && a.ld % 2 == 0 && a.q_off % 2 == 0;
     p.nd = (a.D + 63) / 64;
     p.ndv = (a.Dv + 63) / 64;
     const int rep = a.H / a.G;

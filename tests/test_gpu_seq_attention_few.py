@@ -39,6 +39,15 @@ def test_decoding(form, blocks):
     assert rms_new <= 1.5 * rms_old + 2.0 ** -24 * top
 
 
+@pytest.mark.parametrize("form", [0, 1, 5])
+def test_queries_at_odd_columns(form):
+    """rows of an odd stride (a layer's gate per head of an odd number of heads): the bits of rows on even ones"""
+    c = Case([(p, 1) for p in (0, 127, 300)], splits=2, single=3, **FORMS[form])
+    want = c.run(False)
+    c.q, c.ld = np.ascontiguousarray(np.pad(c.q, ((0, 0), (0, 1)))), c.ld + 1
+    assert c.ld % 2 and np.array_equal(c.run(False), want)
+
+
 def test_stale_rows_stay_outside():
     c = Case([(100, 1), (530, 1)], 8, 2, 128, 192, window=64, seed=4, single=3, splits=2)
     clean = c.run(False)
