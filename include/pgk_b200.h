@@ -153,7 +153,8 @@ int pgk_gemm_nvf4_bf16_tc(const void* A, const void* B_data, const void* B_scale
 /* Waits of that kernel that ran out so far (0: none), after a device synchronisation. */
 int pgk_gemm_nvf4_wait_error(int* out);
 /* out[M,I] = bf16(bf16(silu(g)) * u) from a [M, 2I] tensor whose columns are gate/up interleaved in groups of 8 (the
- * fused NVF4 MLP layout below): the epilogue of the batched (tensor-core) gate/up projection */
+ * fused NVF4 MLP layout below): what pgk_gemv_nvf4_swiglu_bf16 does within its product, as a step of its own for products that come
+ * without it (pgk_gemm_nvf4_bf16_tc) */
 int pgk_swiglu_interleaved8_bf16(const void* gate_up, void* out, int M, int I, void* stream);
 /* gate/up GEMV + SiLU*up on ONE fused weight tensor: Wgu_data u8 [K/2, 2I], Wgu_scale
  * [K/32, 2I] whose columns are gate/up interleaved in groups of 8
@@ -825,11 +826,11 @@ int pgk_gemm_seq_f32(const float* A, int lda, long long a_batch, const void* W, 
 int pgk_seq_attention_wait_error(int* out);
 /* 1 when the tensor-core attention serves such rows of an aligned cache whose requests have at most `positions` positions (pages x page
  * size), else 0: single_query 2 and prompts then take the float32 kernels */
+int pgk_seq_attention_tensor(int dim, int vdim, int k_ld, int v_ld, int heads, int kv_heads, int cache_dtype, long long positions);
 /* Decoding (one query per request) with a request's keys cut over a cluster of blocks: how many, 0 where that kernel does not serve the layer.  The
- * entry points below take it as `splits` with single_query = 3, no workspace and no tickets.  same_rows: the values are a prefix of the key rows. */
+ * pgk_seq_attention entry points take it as `splits` with single_query = 3, no workspace and no tickets.  same_rows: the values are a prefix of the key rows. */
 int pgk_seq_attention_few_plan(int dim, int vdim, int k_ld, int v_ld, int same_rows, int heads, int kv_heads, int cache_dtype, int page_size,
                                int requests, int keys);
-int pgk_seq_attention_tensor(int dim, int vdim, int k_ld, int v_ld, int heads, int kv_heads, int cache_dtype, long long positions);
 int pgk_seq_decode_heads_per_block(void);
 int pgk_seq_heads_per_block(int heads, int kv_heads);
 int pgk_seq_queries_per_tile(int heads, int kv_heads);

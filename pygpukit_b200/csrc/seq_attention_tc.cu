@@ -137,9 +137,9 @@ seq_attention_tc_kernel(const __grid_constant__ CUtensorMap kmap, const __grid_c
     const uint32_t tmem = *tmem_slot;
     griddep_wait();
     griddep_launch();
-    // blocks start in the order of their numbers: a request's last queries, which see the most keys, first, so that none of the long ones starts when the
-    // others end (16 heads over latent rows, 2000 tokens, 1000 blocks of 1 to 16 tiles 466 -> 445 us;
-    // 32 / 4 heads of 128 in chunks of 1024, 2000 blocks 195 -> 186)
+    // blocks start in the order of their numbers: the last request's last queries first, each request's from its last, which see the most keys, to its first,
+    // so that with one request none of the long ones starts when the others end (16 heads over latent rows, 2000 tokens, 1000 blocks of 1 to 16 tiles 466 -> 445 us;
+    // 32 / 4 heads of 128 in chunks of 1024, 2000 blocks 195 -> 186).  Which of several requests is the longest moves a prompt of 2 to 7 unequal ones by 1 % at most
     const int nth = (int)(blockIdx.y * gridDim.x + blockIdx.x), block = nth / (int)gridDim.y, part = nth - block * (int)gridDim.y;
     const int4 tile = a.tiles[(int)gridDim.x - 1 - block];
     const int t0 = tile.x, nq = tile.y, slot = tile.z, pos0 = tile.w, D = a.D, Dv = a.Dv, HB = a.HB;
