@@ -23,9 +23,9 @@ def test_dropped_arrays_go_back_when_memory_is_asked_for():
     before = _free()
     keep = [gk.empty((8 * MB,), gk.uint8) for _ in range(40)]
     assert before - _free() >= 300 * MB
-    del keep                                             # 320 MB, of which 64 MB may wait
+    del keep
     assert before - _free() <= 4 * MB
-    for _ in range(2000):                                # more blocks than may wait
+    for _ in range(2000):
         gk.empty((64,), gk.uint8)
     assert before - _free() <= 4 * MB
 

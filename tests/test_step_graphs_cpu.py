@@ -32,6 +32,7 @@ def model(monkeypatch):
     api = Api()
     monkeypatch.setattr(layered, "api", api)
     monkeypatch.setattr(paged_cache, "api", api)
+    monkeypatch.setattr(layered, "leave_open", lambda: None)         # process-wide state of the current stream
     monkeypatch.setattr(layered, "GPUArray", Array)
     monkeypatch.setattr(paged_cache, "GPUArray", Array)
     monkeypatch.setattr(paged_cache, "zeros", Array)
